@@ -78,6 +78,11 @@ NF4_API uint64_t nf4_kernel_launch_count(void);
  * Rust shim maps a non-zero status to anyhow::Error (src/lib.rs:16-32). */
 NF4_API int32_t nf4_device_status(int32_t *decode, int32_t *decode_split_k, int32_t *prefill);
 
+/* How many failures nf4_device_status and the `*_host` entry points have reported in this process.  A
+ * kernel that gave up may have left its workspace's flag words set: a host that keeps a workspace
+ * across calls clears its first 256 bytes again when this number has changed. */
+NF4_API uint64_t nf4_failure_count(void);
+
 /* Diagnostic: launches a one-thread kernel that waits on a barrier nobody signals, with the same
  * bounded wait the decode kernel uses and `limit_ns` (at most one second) as its limit.  The kernel
  * returns when the limit has passed and records the failure as the decode kernel would; the call

@@ -1,0 +1,75 @@
+"""The mirror's native host path: workspaces kept per thread and stream must serve calls of any mix of shapes."""
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+from gpu_util import DEV  # noqa: E402
+from unifur_b200 import _lib  # noqa: E402
+
+
+def layers():
+    from unifur_b200.quantize import PackedNf4Tensor
+
+    gen = torch.Generator(device=DEV).manual_seed(5)
+    out = []
+    # decode with an adapter, K in parts, strip kernel, split-K, prefill (its workspace is larger), K in parts again
+    for rows, k, n, r, layout, dt in ((4, 512, 256, 16, 0, torch.bfloat16), (3, 8192, 192, 8, 0, torch.bfloat16),
+                                      (2, 256, 320, 4, 1, torch.float32), (5, 320, 192, 8, 0, torch.bfloat16),
+                                      (40, 256, 192, 16, 0, torch.bfloat16), (16, 4352, 64, 64, 0, torch.bfloat16)):
+        rnd = lambda *s: torch.randn(*s, device=DEV, generator=gen)  # noqa: E731
+        a, b = ((r, k), (n, r)) if layout == 0 else ((k, r), (r, n))
+        out.append((rnd(rows, k).to(dt), PackedNf4Tensor.quantize(rnd(k * n) * 0.02), k, n, layout,
+                    (rnd(*a) * 0.05).to(dt), (rnd(*b) * 0.05).to(dt)))
+    return out
+
+
+def forward(x, p, k, n, layout, a, b):
+    from unifur_b200.quantize import linear_forward
+
+    return linear_forward(x, p, k, n, layout, lora_a=a, lora_b=b, lora_scale=1.5)
+
+
+@pytest.mark.parametrize("threads", [1, 3])
+def test_kept_workspaces_serve_any_mix_of_calls(threads):
+    cases = layers()
+    want = []
+    for c in cases:
+        _lib.host().release_workspaces()  # a fresh workspace for every reference result
+        want.append(forward(*c).cpu())
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(seed):
+        order = np.random.default_rng(seed).permutation(np.arange(len(cases)).repeat(6))
+        streams = [torch.cuda.Stream() for _ in range(2)]
+        got = []
+        for j, i in enumerate(order):
+            with torch.cuda.stream(streams[j % 2]):
+                got.append((i, forward(*cases[i])))
+        torch.cuda.synchronize()
+        bad.extend(i for i, y in got if not torch.equal(y.cpu(), want[i]))
+
+    ts = [threading.Thread(target=work, args=(t,)) for t in range(threads)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad
+    _lib.check(_lib.load().nf4_device_status(None, None, None))
+
+
+def test_forward_under_capture_replays_beside_eager_calls():
+    c = layers()[0]
+    want = forward(*c)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        y = forward(*c)
+    for _ in range(3):
+        g.replay()
+        again = forward(*c)
+    torch.cuda.synchronize()
+    assert torch.equal(y, want) and torch.equal(again, want)

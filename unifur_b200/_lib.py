@@ -69,6 +69,7 @@ SIGNATURES = {
     "nf4_last_error": (C.c_char_p, []),
     "nf4_kernel_launch_count": (_u64, []),
     "nf4_device_status": (_i32, [C.POINTER(_i32), C.POINTER(_i32), C.POINTER(_i32)]),
+    "nf4_failure_count": (_u64, []),
     "nf4_selftest_bounded_wait": (_i32, [_u64, C.POINTER(_u64)]),
     "nf4_selfcheck_code_selection": (_i32, [_u64, _u64, C.POINTER(_u64)]),
     "nf4_selfcheck_quantize_fast_path": (_i32, [_u64, _u64, _f32, C.POINTER(_u64)]),
@@ -140,6 +141,23 @@ def load() -> C.CDLL:
             fn.argtypes = args
         _lib = lib
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The native host path of the mirror (``csrc/host/host.cpp``); raises when it has not been built."""
+    global _host
+    if _host is None:
+        load()
+        try:
+            from . import _host as mod
+        except ImportError as e:
+            raise ImportError("unifur_b200/_host.so is missing or was built against another torch: build it with "
+                              "`python -m unifur_b200.build`") from e
+        _host = mod
+    return _host
 
 
 def last_error() -> str:

@@ -16,6 +16,7 @@ namespace nf4 {
 namespace {
 thread_local std::string t_last_error;
 std::atomic<uint64_t> g_launches{0};
+std::atomic<uint64_t> g_failures{0};  // failures of kernels reported to the host
 }  // namespace
 
 int32_t fail(int32_t code, const char *fmt, ...) {
@@ -162,6 +163,7 @@ int32_t flag_ptrs(int **out3) {
 int32_t report_flags(int *const *ptrs, const int *v) {
     for (int i = 0; i < 3; ++i)
         if (v[i]) NF4_CUDA_TRY(cudaMemset(ptrs[i], 0, sizeof(int)));
+    if (v[0] || v[1] || v[2]) g_failures.fetch_add(1, std::memory_order_relaxed);
     if (v[0] == 4)
         return fail(NF4_ERR_CUDA, "decode kernel: dynamic shared memory does not start where the kernel "
                                   "expects it; the launch produced no output");
@@ -317,6 +319,8 @@ int32_t nf4_device_status(int32_t *decode, int32_t *decode_split_k, int32_t *pre
     if (prefill) *prefill = v[2];
     return report_flags(ptrs, v);
 }
+
+uint64_t nf4_failure_count(void) { return g_failures.load(std::memory_order_relaxed); }
 
 int32_t nf4_selftest_bounded_wait(uint64_t limit_ns, uint64_t *waited_ns) {
     if (limit_ns == 0 || limit_ns > 1000000000ull)

@@ -1264,8 +1264,8 @@ WorkspaceLayout workspace_layout(uint64_t rows, uint64_t d_in, uint64_t d_out, u
                                  Extra extra = kPlain) {
     auto up = [](uint64_t v) { return (v + 255) / 256 * 256; };
     WorkspaceLayout w;
-    w.off_xh = 0;
-    w.off_scale = up(rows * d_in * 2);
+    w.off_xh = 256;  // the flag words at the start belong to the decode kernels and stay as they are
+    w.off_scale = w.off_xh + up(rows * d_in * 2);
     w.off_t = w.off_scale + up(rows * 4);
     w.off_flags = w.off_t + up(rows * 2ull * 64 * lora_chunks_of(lora_rank) * 2);
     const Sharing sh = share_tiles(rows, d_in, d_out);

@@ -17,7 +17,7 @@ from typing import Optional, Sequence, Tuple
 import torch
 
 from . import _lib
-from ._lib import DTYPE_BF16, DTYPE_F32, LAYOUT_IN_OUT, LAYOUT_OUT_IN, LinearArgs
+from ._lib import DTYPE_BF16, DTYPE_F32, LAYOUT_IN_OUT, LAYOUT_OUT_IN
 
 BLOCK_SIZE = 64  # src/quantize.rs:37
 
@@ -42,11 +42,6 @@ def nf4_levels() -> torch.Tensor:
     return torch.tensor(list(buf), dtype=torch.float32)
 
 
-def _flat_f32(values: torch.Tensor) -> torch.Tensor:
-    _require_cuda(values, "values")
-    return values.detach().to(torch.float32).contiguous().view(-1)
-
-
 class PackedNf4Tensor:
     """Packed 4-bit NF4 storage resident on the GPU (src/quantize.rs:248-400).
 
@@ -68,50 +63,23 @@ class PackedNf4Tensor:
     @staticmethod
     def quantize(values: torch.Tensor) -> "PackedNf4Tensor":
         """``PackedNf4Tensor::quantize`` (src/quantize.rs:262-279) on the device."""
-        v = _flat_f32(values)
-        n = v.numel()
-        dev = v.device
-        codes = torch.empty((n + 1) // 2, dtype=torch.uint8, device=dev)
-        absmax = torch.empty((n + BLOCK_SIZE - 1) // BLOCK_SIZE, dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
-            _lib.check(_lib.load().nf4_quantize_dev(_ptr(v), n, _ptr(codes), _ptr(absmax),
-                                                    _stream(dev)))
-        return PackedNf4Tensor(codes, n, absmax)
+        codes, absmax = _lib.host().quantize(values, False)
+        return PackedNf4Tensor(codes, values.numel(), absmax)
 
     @staticmethod
     def quantize_transposed(weight: torch.Tensor) -> "PackedNf4Tensor":
         """Packed NF4 of ``weight.t()`` flattened row-major, for a 2-D f32 or bf16 ``weight`` on
         the GPU, without materialising the transpose: the reference's checkpoint load path
         (``transpose2d`` + ``PackedNf4Tensor::quantize``, src/qwennet.rs:1375-1390, 1709-1711)."""
-        _require_cuda(weight, "weight")
-        if weight.dim() != 2 or weight.dtype not in (torch.float32, torch.bfloat16):
-            raise ValueError("weight must be a 2-D float32 or bfloat16 tensor")
-        w = weight.contiguous()
-        rows, cols = w.shape
-        n = rows * cols
-        dev = w.device
-        codes = torch.empty((n + 1) // 2, dtype=torch.uint8, device=dev)
-        absmax = torch.empty((n + BLOCK_SIZE - 1) // BLOCK_SIZE, dtype=torch.float32, device=dev)
-        lib = _lib.load()
-        ws_bytes = int(lib.nf4_quantize_transposed_workspace_bytes(rows, cols))
-        ws = torch.empty(max(ws_bytes, 16), dtype=torch.uint8, device=dev)
-        with torch.cuda.device(dev):
-            _lib.check(lib.nf4_quantize_transposed_dev(
-                _ptr(w), _lib.DTYPE_BF16 if w.dtype == torch.bfloat16 else _lib.DTYPE_F32, rows, cols,
-                _ptr(codes), _ptr(absmax), _ptr(ws), ws.numel(), _stream(dev)))
-        return PackedNf4Tensor(codes, n, absmax)
+        codes, absmax = _lib.host().quantize_transposed(weight)
+        return PackedNf4Tensor(codes, weight.numel(), absmax)
 
     def with_double_quantization(self) -> "PackedNf4Tensor":
         """src/quantize.rs:284-309; idempotent."""
         if self.is_double_quantized():
             return self
-        dev = self.codes.device
-        sc = torch.empty(max(self._num_blocks, 1), dtype=torch.uint8, device=dev)
-        sos = torch.empty(1, dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
-            _lib.check(_lib.load().nf4_double_quantize_dev(_ptr(self.absmax), self._num_blocks,
-                                                           _ptr(sc), _ptr(sos), _stream(dev)))
-        return PackedNf4Tensor(self.codes, self._len, None, sc[: self._num_blocks], sos)
+        sc, sos = _lib.host().double_quantize(self.absmax, self._num_blocks)
+        return PackedNf4Tensor(self.codes, self._len, None, sc, sos)
 
     # -- queries -----------------------------------------------------------------------
     def is_double_quantized(self) -> bool:
@@ -131,13 +99,7 @@ class PackedNf4Tensor:
 
     def dequantize(self) -> torch.Tensor:
         """src/quantize.rs:355-366: flat f32 device tensor of ``len()`` values."""
-        dev = self.codes.device
-        out = torch.empty(self._len, dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
-            _lib.check(_lib.load().nf4_dequantize_dev(
-                _ptr(self.codes), self._len, _ptr(self.absmax), _ptr(self.scale_codes),
-                _ptr(self.scale_of_scales), _ptr(out), _stream(dev)))
-        return out
+        return _lib.host().dequantize(self.codes, self._len, self.absmax, self.scale_codes, self.scale_of_scales, False)
 
     def resident_bytes(self) -> int:
         """src/quantize.rs:370-376."""
@@ -183,24 +145,12 @@ class Nf4Tensor:
 
     @staticmethod
     def quantize(values: torch.Tensor) -> "Nf4Tensor":
-        v = _flat_f32(values)
-        n = v.numel()
-        dev = v.device
-        codes = torch.empty(n, dtype=torch.uint8, device=dev)
-        absmax = torch.empty((n + BLOCK_SIZE - 1) // BLOCK_SIZE, dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
-            _lib.check(_lib.load().nf4_quantize_unpacked_dev(_ptr(v), n, _ptr(codes), _ptr(absmax),
-                                                             _stream(dev)))
-        return Nf4Tensor(codes, n, absmax)
+        codes, absmax = _lib.host().quantize(values, True)
+        return Nf4Tensor(codes, values.numel(), absmax)
 
     def with_double_quantization(self) -> "Nf4Tensor":
-        dev = self.codes.device
-        sc = torch.empty(max(self._num_blocks, 1), dtype=torch.uint8, device=dev)
-        sos = torch.empty(1, dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
-            _lib.check(_lib.load().nf4_double_quantize_dev(_ptr(self.absmax), self._num_blocks,
-                                                           _ptr(sc), _ptr(sos), _stream(dev)))
-        return Nf4Tensor(self.codes, self._len, self.absmax, sc[: self._num_blocks], sos)
+        sc, sos = _lib.host().double_quantize(self.absmax, self._num_blocks)
+        return Nf4Tensor(self.codes, self._len, self.absmax, sc, sos)
 
     def is_double_quantized(self) -> bool:
         return self.scale_codes is not None
@@ -215,14 +165,7 @@ class Nf4Tensor:
         return self._num_blocks
 
     def dequantize(self) -> torch.Tensor:
-        dev = self.codes.device
-        out = torch.empty(self._len, dtype=torch.float32, device=dev)
-        dq = self.is_double_quantized()
-        with torch.cuda.device(dev):
-            _lib.check(_lib.load().nf4_dequantize_unpacked_dev(
-                _ptr(self.codes), self._len, None if dq else _ptr(self.absmax),
-                _ptr(self.scale_codes), _ptr(self.scale_of_scales), _ptr(out), _stream(dev)))
-        return out
+        return _lib.host().dequantize(self.codes, self._len, self.absmax, self.scale_codes, self.scale_of_scales, True)
 
     def bits_per_value(self) -> float:
         """src/quantize.rs:190-200."""
@@ -235,17 +178,7 @@ class Nf4Tensor:
 
 def quantize_dequantize_tensor(tensor: torch.Tensor, double_quantization: bool) -> torch.Tensor:
     """src/quantize.rs:404-416: the error a frozen NF4 weight carries, same shape back."""
-    v = _flat_f32(tensor)
-    n = v.numel()
-    dev = v.device
-    lib = _lib.load()
-    out = torch.empty_like(v)
-    ws_bytes = int(lib.nf4_quantize_dequantize_workspace_bytes(n))
-    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
-    with torch.cuda.device(dev):
-        _lib.check(lib.nf4_quantize_dequantize_dev(_ptr(v), n, int(double_quantization), _ptr(out),
-                                                   _ptr(ws), ws_bytes, _stream(dev)))
-    return out.view(tensor.shape)
+    return _lib.host().quantize_dequantize(tensor, double_quantization)
 
 
 def quantize_module(module: torch.nn.Module, double_quantization: bool,
@@ -407,39 +340,10 @@ def qlora_merge(packed: "PackedNf4Tensor", d_in: int, d_out: int, a: torch.Tenso
     return out
 
 
-def _linear_args(lib, x2: torch.Tensor, packed: PackedNf4Tensor, d_in: int, d_out: int, layout: int, bias, lora_a,
-                 lora_b, lora_scale: float, out):
-    """The argument block of one forward, its output, and the tensors that must outlive the launch."""
-    dev = x2.device
-    rows = x2.shape[0]
-    rank = 0
-    if lora_a is not None:
-        rank = lora_a.shape[0] if layout == LAYOUT_OUT_IN else lora_a.shape[1]
-        lora_a = lora_a.to(x2.dtype).contiguous()
-        lora_b = lora_b.to(x2.dtype).contiguous()
-    y = out if out is not None else torch.empty(rows, d_out, dtype=x2.dtype, device=dev)
-    ws_bytes = int(lib.nf4_linear_workspace_bytes(rows, d_in, d_out, rank))
-    # the decode kernel's flag words at the start of the workspace must start at zero; the rest
-    # (tens of megabytes at prefill sizes) needs no initialisation
-    ws = torch.empty(max(ws_bytes, 256), dtype=torch.uint8, device=dev)
-    ws[:256].zero_()
-    bias32 = bias.to(torch.float32).contiguous() if bias is not None else None
-    a = LinearArgs()
-    a.struct_bytes = ctypes.sizeof(LinearArgs)
-    a.layout, a.io_dtype = layout, _io_dtype(x2)
-    a.rows, a.d_in, a.d_out = rows, d_in, d_out
-    a.x = x2.data_ptr()
-    a.packed = packed.codes.data_ptr()
-    a.absmax = packed.absmax.data_ptr() if not packed.is_double_quantized() else None
-    a.scale_codes = packed.scale_codes.data_ptr() if packed.is_double_quantized() else None
-    a.scale_of_scales = packed.scale_of_scales.data_ptr() if packed.is_double_quantized() else None
-    a.bias = bias32.data_ptr() if bias32 is not None else None
-    a.lora_a = lora_a.data_ptr() if rank else None
-    a.lora_b = lora_b.data_ptr() if rank else None
-    a.lora_rank, a.lora_scale = rank, float(lora_scale)
-    a.y, a.ldy = y.data_ptr(), y.stride(0)
-    a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
-    return a, y, (ws, bias32, lora_a, lora_b, x2)
+def _projection(packed: PackedNf4Tensor, d_out: int, bias, lora_a, lora_b, lora_scale: float) -> tuple:
+    """The operands of one projection in the order ``csrc/host/host.cpp`` takes them."""
+    return (packed.codes, packed.absmax, packed.scale_codes, packed.scale_of_scales, d_out, bias, lora_a, lora_b,
+            lora_scale)
 
 
 def linear_forward(x: torch.Tensor, packed: PackedNf4Tensor, d_in: int, d_out: int, layout: int,
@@ -452,15 +356,8 @@ def linear_forward(x: torch.Tensor, packed: PackedNf4Tensor, d_in: int, d_out: i
     (src/qwennet.rs:326-342).  ``layout`` selects ``W [d_out, d_in]`` (LAYOUT_OUT_IN, LoRA
     ``A [r, d_in]``, ``B [d_out, r]``) or the reference's ``W [d_in, d_out]``
     (LAYOUT_IN_OUT, ``A [d_in, r]``, ``B [r, d_out]``)."""
-    _require_cuda(x, "x")
-    lib = _lib.load()
-    dev = x.device
-    lead = x.shape[:-1]
-    x2 = x.contiguous().view(-1, d_in)
-    a, y, _alive = _linear_args(lib, x2, packed, d_in, d_out, layout, bias, lora_a, lora_b, lora_scale, out)
-    with torch.cuda.device(dev):
-        _lib.check(lib.nf4_linear_forward_dev(ctypes.byref(a), _stream(dev)))
-    return y.view(*lead, d_out) if out is None else y
+    return _lib.host().linear_forward(x, d_in, layout, packed.codes, packed.absmax, packed.scale_codes,
+                                      packed.scale_of_scales, d_out, bias, lora_a, lora_b, lora_scale, out)
 
 
 def linear_forward_grouped(x: torch.Tensor, d_in: int, layout: int, projections) -> list:
@@ -469,22 +366,9 @@ def linear_forward_grouped(x: torch.Tensor, d_in: int, layout: int, projections)
     ``d_out`` and optionally ``bias``, ``lora_a``, ``lora_b``, ``lora_scale``.  The outputs equal
     those of one ``linear_forward`` per projection, which is what the reference does
     (src/qwennet.rs:372-383 per projection)."""
-    _require_cuda(x, "x")
-    lib = _lib.load()
-    dev = x.device
-    lead = x.shape[:-1]
-    x2 = x.contiguous().view(-1, d_in)
-    block = (LinearArgs * len(projections))()
-    ys, alive = [], []
-    for i, pr in enumerate(projections):
-        a, y, keep = _linear_args(lib, x2, pr["packed"], d_in, pr["d_out"], layout, pr.get("bias"),
-                                  pr.get("lora_a"), pr.get("lora_b"), pr.get("lora_scale", 0.0), None)
-        block[i] = a
-        ys.append(y.view(*lead, pr["d_out"]))
-        alive.append(keep)
-    with torch.cuda.device(dev):
-        _lib.check(lib.nf4_linear_forward_grouped_dev(block, len(projections), _stream(dev)))
-    return ys
+    return _lib.host().linear_forward_grouped(x, d_in, layout, [
+        _projection(pr["packed"], pr["d_out"], pr.get("bias"), pr.get("lora_a"), pr.get("lora_b"),
+                    pr.get("lora_scale", 0.0)) for pr in projections])
 
 
 class QLoraLinear:

@@ -3,7 +3,6 @@
 :305-435) over the C ABI."""
 from __future__ import annotations
 
-import ctypes
 from typing import Optional
 
 import torch
@@ -106,37 +105,11 @@ class QloraLinear:
         bytes read in the other orientation (a ``[d_out, d_in]`` weight is a ``[d_in', d_out']``
         weight with ``d_in' = d_out``), with the adapter factors swapping roles; the two adapter
         gradients are small dense products.  All of it runs in ``nf4_qlora_backward_dev``."""
-        lib = _lib.load()
-        d_in, d_out = self.base.d_input(), self.base.d_output()
-        x2 = x.reshape(-1, d_in).contiguous()
-        g2 = grad_y.reshape(-1, d_out).to(x2.dtype).contiguous()
-        rows, dev = x2.shape[0], x2.device
-        la, lb = self.lora_a.to(x2.dtype).contiguous(), self.lora_b.to(x2.dtype).contiguous()
-        rank = la.shape[0] if self.base.layout == LAYOUT_OUT_IN else la.shape[1]
-        gx = torch.empty(rows, d_in, dtype=x2.dtype, device=dev)
-        ga, gb = torch.empty_like(la), torch.empty_like(lb)
-        ws = torch.empty(max(int(lib.nf4_qlora_backward_workspace_bytes(rows, d_in, d_out, rank)), 256),
-                         dtype=torch.uint8, device=dev)
-        ws[:256].zero_()   # the flag words; the rest needs no initialisation
-        pk = self.base.packed()
-        dq = pk.is_double_quantized()
-        a = _lib.LinearArgs()
-        a.struct_bytes = ctypes.sizeof(_lib.LinearArgs)
-        a.layout = self.base.layout
-        a.io_dtype = _lib.DTYPE_BF16 if x2.dtype == torch.bfloat16 else _lib.DTYPE_F32
-        a.rows, a.d_in, a.d_out = rows, d_in, d_out
-        a.x, a.packed = x2.data_ptr(), pk.codes.data_ptr()
-        a.absmax = None if dq else pk.absmax.data_ptr()
-        a.scale_codes = pk.scale_codes.data_ptr() if dq else None
-        a.scale_of_scales = pk.scale_of_scales.data_ptr() if dq else None
-        a.lora_a, a.lora_b, a.lora_rank, a.lora_scale = la.data_ptr(), lb.data_ptr(), rank, self.scaling
-        a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
-        vp = ctypes.c_void_p
-        with torch.cuda.device(dev):
-            _lib.check(lib.nf4_qlora_backward_dev(
-                ctypes.byref(a), vp(g2.data_ptr()), vp(gx.data_ptr()), vp(ga.data_ptr()), vp(gb.data_ptr()),
-                vp(torch.cuda.current_stream(dev).cuda_stream)))
-        return gx.reshape(x.shape), ga.to(self.lora_a.dtype), gb.to(self.lora_b.dtype)
+        base, pk = self.base, self.base.packed()
+        gx, ga, gb = _lib.host().qlora_backward(
+            x, grad_y, base.d_input(), base.layout, pk.codes, pk.absmax, pk.scale_codes, pk.scale_of_scales,
+            base.d_output(), None, self.lora_a, self.lora_b, self.scaling)
+        return gx, ga.to(self.lora_a.dtype), gb.to(self.lora_b.dtype)
 
     def resident_bytes(self) -> int:
         """src/qwennet.rs:362-366."""
@@ -253,13 +226,5 @@ class Nf4Embedding:
         if dtype not in (torch.float32, torch.bfloat16):
             raise ValueError("dtype must be float32 or bfloat16")
         p = self._packed
-        dev = p.codes.device
-        flat = ids.to(device=dev, dtype=torch.int64).contiguous().view(-1)
-        out = torch.empty(flat.numel(), self._d_model, dtype=dtype, device=dev)
-        ptr = lambda t: ctypes.c_void_p(t.data_ptr()) if t is not None else None
-        _lib.check(_lib.load().nf4_embedding_gather_dev(
-            ptr(p.codes), ptr(p.absmax), ptr(p.scale_codes), ptr(p.scale_of_scales),
-            self._n_embedding, self._d_model, ptr(flat), flat.numel(), ptr(out),
-            _lib.DTYPE_BF16 if dtype == torch.bfloat16 else _lib.DTYPE_F32,
-            ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)))
-        return out.view(*ids.shape, self._d_model)
+        return _lib.host().embedding(ids, p.codes, p.absmax, p.scale_codes, p.scale_of_scales, self._n_embedding,
+                                     self._d_model, dtype == torch.bfloat16)
