@@ -38,10 +38,14 @@ int32_t check_cuda(cudaError_t e, const char *what) {
     return fail(code, "%s: %s (%s)", what, cudaGetErrorName(e), cudaGetErrorString(e));
 }
 
-int32_t ensure_dynamic_smem(const void *kernel, int bytes) {
+namespace {
+// Sets an attribute of `kernel` on the current device unless it has been set there before: attributes
+// belong to the device a kernel is loaded on.
+int32_t set_once(const void *kernel, cudaFuncAttribute what, int value) {
     struct Done {
         const void *kernel;
         int device;
+        cudaFuncAttribute what;
     };
     static std::mutex mu;
     static Done done[256];
@@ -50,10 +54,19 @@ int32_t ensure_dynamic_smem(const void *kernel, int bytes) {
     NF4_CUDA_TRY(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lock(mu);
     for (int i = 0; i < n_done; ++i)
-        if (done[i].kernel == kernel && done[i].device == dev) return NF4_OK;
-    NF4_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    if (n_done < 256) done[n_done++] = Done{kernel, dev};
+        if (done[i].kernel == kernel && done[i].device == dev && done[i].what == what) return NF4_OK;
+    NF4_CUDA_TRY(cudaFuncSetAttribute(kernel, what, value));
+    if (n_done < 256) done[n_done++] = Done{kernel, dev, what};
     return NF4_OK;
+}
+}  // namespace
+
+int32_t ensure_dynamic_smem(const void *kernel, int bytes) {
+    return set_once(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+
+int32_t allow_large_clusters(const void *kernel) {
+    return set_once(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
 }
 
 void count_launch(uint64_t n) { g_launches.fetch_add(n, std::memory_order_relaxed); }

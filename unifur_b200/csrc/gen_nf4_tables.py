@@ -57,6 +57,9 @@ def threshold(i: int) -> np.float32:
     return unkey(hi)
 
 
+CELL_MARGIN = 2  # units of 2^-21 on either side of a threshold where the exact path decides (errors add up to < 1.4)
+
+
 def main():
     th = [threshold(i) for i in range(15)]
     lines = [
@@ -71,27 +74,26 @@ def main():
     lines.append("// the sixteen levels rounded to f16 (round to nearest even), as bit patterns")
     lines.append("#define NF4_LEVEL_F16_BITS_LIST \\")
     lines.append("  " + ", ".join("0x%04xu" % int(np.float16(l).view(np.uint16)) for l in LEVELS))
-    # 32 uniform cells over [-1, 1): cell c = [c/16 - 1, (c+1)/16 - 1) holds at most one threshold
-    # (they are >= 0.08 apart); entry = {that threshold or +inf, number of thresholds below the cell}
+    # 33 uniform cells of width 1/16 over [-1, 1]: a value v is rounded to n = round(64 v + 64) and
+    # belongs to cell n >> 2, so cell c is [(4c - 0.5) / 64 - 1, (4c + 3.5) / 64 - 1), which holds at most
+    # one threshold (they are >= 0.08 apart).  v itself enters as the bits of the f32 v * 2^21 + 1.5 * 2^23,
+    # which are 0x4b400000 + round(v * 2^21); the cell's word W is such that the top four bits of bits - W
+    # are the code and the low 28 bits are below 2 * MARGIN exactly when v is within MARGIN units of 2^-21 of
+    # the threshold.  Padded to 64 words; the last one (a NaN's bits index it) is always "within".
     cells = []
-    for c in range(32):
-        lo, hi = c / 16.0 - 1.0, (c + 1) / 16.0 - 1.0
+    for c in range(33):
+        lo, hi = (4 * c - 0.5) / 64.0 - 1.0, (4 * c + 3.5) / 64.0 - 1.0
         inside = [t for t in th if lo <= float(t) < hi]
         assert len(inside) <= 1
         base = sum(1 for t in th if float(t) < lo)
-        # one word per cell: the threshold with its low four mantissa bits replaced by `base`
-        # (a shift of at most 15 ulp < 9e-7, covered by the kernel's 3e-6 margin); a cell
-        # without a threshold carries a huge finite value so that the difference stays finite
-        tbits = int(np.float32(inside[0]).view(np.uint32)) if inside else 0x7f000000
-        word = (tbits & ~0xF) | base
-        if inside:
-            moved = abs(float(np.uint32(word).view(np.float32)) - float(inside[0]))
-            assert moved < 9e-7, moved
         # no threshold may sit within rounding distance of a cell edge
         for t in th:
             assert min(abs(float(t) - lo), abs(float(t) - hi)) > 1e-4
-        cells.append(word)
-    lines.append("// 32 uniform cells over [-1, 1): threshold inside the cell (or 1.7e38), low 4 bits = thresholds below the cell")
+        units = int(round(float(inside[0]) * 2 ** 21)) if inside else 1 << 26  # out of reach: never within, never above
+        cells.append((0x4B400000 + units - CELL_MARGIN - ((base + 1) << 28)) & 0xFFFFFFFF)
+    cells += [0x7FFFFFFF] * (64 - len(cells))
+    lines.append("// 33 cells of width 1/16 over [-1, 1], padded to 64 (see nf4_common.cuh: FastCodes)")
+    lines.append("#define NF4_CELL_MARGIN %d" % CELL_MARGIN)
     lines.append("#define NF4_CELL_TABLE_LIST \\")
     lines.append("  " + ", ".join("0x%08xu" % c for c in cells))
     lines.append("// thresholds as decimals: " + ", ".join(repr(float(t)) for t in th))

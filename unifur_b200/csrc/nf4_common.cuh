@@ -16,6 +16,8 @@ constexpr int kNumSMs = 148;            // B200
 int32_t fail(int32_t code, const char *fmt, ...);
 int32_t check_cuda(cudaError_t e, const char *what);
 void count_launch(uint64_t n = 1);
+// allows clusters of more than eight CTAs for `kernel` on the current device (once per kernel and device)
+int32_t allow_large_clusters(const void *kernel);
 
 #define NF4_CUDA_TRY(expr)                                         \
     do {                                                           \
@@ -90,39 +92,64 @@ __device__ __forceinline__ uint32_t code_of(float x, float absmax) {
 }
 
 // ---- fast code selection ------------------------------------------------------------------
-// Thirty-two uniform cells over [-1, 1); a cell holds at most one decision threshold.  One word
-// per cell: the f32 threshold inside the cell with its low four mantissa bits replaced by the
-// number of thresholds below the cell (the threshold moves by < 9e-7), or 1.7e38 | count for a
-// cell that holds none.
-static __device__ __constant__ const uint32_t c_cell_table[32] = {NF4_CELL_TABLE_LIST};
+// One word per cell of width 1/16 over [-1, 1] (gen_nf4_tables.py): the only decision threshold that
+// can lie in the cell and the number of thresholds below it, in the form FastCodes subtracts.
+constexpr int kCellWords = 64;  // padded: any masked index is inside
+static __device__ __constant__ const uint32_t c_cell_table[kCellWords] = {NF4_CELL_TABLE_LIST};
 
-// Code of x / absmax without the division, when that is provably safe.
-//   q = x * rcp with rcp = fl(1 / absmax) lies within 1.8e-7 of the correctly rounded quotient
-//   (|x| <= absmax, both roundings <= 2^-24 relative).  The cell of q names the only threshold
-//   that can matter; when q is more than 3e-6 away from the table's (slightly moved) copy of
-//   it, q and the exact quotient are on the same side of the true threshold and the code is
-//   `count + (q >= threshold)`.  Otherwise -- next to a threshold, NaN, or a scale outside
-//   [1e-30, 1e30] where rcp is not trustworthy (the caller starts `unsure` as true for those)
-//   -- the exact path decides.
-// `cells` is the table in shared memory (32 words, one bank each: no conflicts).  Cell rounding
-// can put q in a neighbouring cell only within 2e-6 of a cell edge, and no threshold is within
-// 1e-4 of an edge, so the count is unaffected.
 // Out of line on purpose: taken for a few values in a million, and inlining sixteen copies of
 // the division and the bisection doubles the quantize kernel's register count.
 static __device__ __noinline__ uint32_t code_of_exact(float x, float absmax) { return code_of(x, absmax); }
 
-// `unsure` is set (never cleared) when the value sits next to a threshold or is NaN; the caller
-// then redoes its values with code_of_exact.  Keeping the decision out of this function leaves
-// the common path branch-free.
-__device__ __forceinline__ uint32_t code_of_fast(float x, float rcp, const uint32_t *cells,
-                                                 bool &unsure) {
-    const float q = __fmul_rn(x, rcp);
-    int c = __float2int_rz(fmaf(q, 16.0f, 16.0f));  // NaN -> 0
-    c = min(max(c, 0), 31);
-    const uint32_t e = cells[c];
-    const float d = q - __uint_as_float(e);
-    unsure |= !(fabsf(d) > 3e-6f);
-    return (e & 15u) + (d >= 0.0f ? 1u : 0u);
+// Codes of up to eight values x / absmax without the division, where that is provably safe.
+//   u = bits of fma(x, 2^21 rcp, 1.5 * 2^23) = 0x4b400000 + the quotient in units of 2^-21, with rcp the
+//   hardware's reciprocal (within one ulp): within 0.88 units of the correctly rounded quotient (half
+//   for the rounding to units, a quarter for rcp, an eighth for the quotient; |x| <= absmax).  A second multiply-add leaves 4 * cell of the quotient in the low bits of its
+//   result; the cell's word W holds the only threshold that can matter and the count of those below,
+//   so that u - W has the code in its top four bits.  Unless the low 28 bits say that the quotient is
+//   within NF4_CELL_MARGIN (2) units of that threshold (rounded to units), the exact quotient is on the
+//   same side of it.
+//   Otherwise -- or for a NaN, or a scale outside [1e-30, 1e30] where rcp is not trustworthy -- the
+//   caller decides every value of the group with code_of_exact.  No threshold is within 1e-4 of a
+//   cell's edge, so it does not matter which of two neighbouring cells a value at an edge is given to.
+// What it costs.  Instruction issue bounds a quantizer that is not bound by memory, and the integer
+// pipe has half the rate of the FMA pipe: per value two multiply-adds, a mask, the table load, a
+// subtraction, a funnel shift that collects the code, and a mask and minimum for the nearest threshold;
+// 22 instructions per value with a conversion, a clamp and selects, 18 with a compare per threshold in f32.
+// `cells` is the table in shared memory (a bank per cell: no conflicts).
+struct FastCodes {
+    uint32_t codes = 0, nearest = 0xffffffffu;
+
+    // values are taken from the last (highest nibble) to the first; rcp = approx_rcp(absmax)
+    __device__ __forceinline__ void take(float x, float rcp_units, float rcp_cells, const uint32_t *cells) {
+        const uint32_t u = __float_as_uint(fmaf(x, rcp_units, 12582912.0f));
+        const uint32_t at = __float_as_uint(fmaf(x, rcp_cells, 12582912.0f + 64.0f)) & 0xfcu;
+        const uint32_t d = u - *reinterpret_cast<const uint32_t *>(reinterpret_cast<const char *>(cells) + at);
+        codes = __funnelshift_l(d, codes, 4);
+        nearest = min(nearest, d & 0x0fffffffu);
+    }
+    __device__ __forceinline__ bool sure() const { return nearest >= 2u * NF4_CELL_MARGIN; }
+};
+
+__device__ __forceinline__ float approx_rcp(float v) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// The eight codes of a group as nibbles, the first value in the lowest.
+__device__ __forceinline__ uint32_t codes_of_group(const float (&x)[8], float absmax, const uint32_t *cells) {
+    const float rcp = approx_rcp(absmax);
+    FastCodes f;
+    #pragma unroll
+    for (int i = 7; i >= 0; --i) f.take(x[i], rcp * 2097152.0f, rcp * 64.0f, cells);
+    uint32_t w = f.codes;
+    if (!f.sure() || !(absmax >= 1e-30f && absmax <= 1e30f)) {
+        w = 0;
+        #pragma unroll
+        for (int i = 0; i < 8; ++i) w |= code_of_exact(x[i], absmax) << (4 * i);
+    }
+    return w;
 }
 
 // Scale of a double-quantized block: divide first, then multiply (src/quantize.rs:348).

@@ -5,9 +5,11 @@
 // Layout: values and outputs are flat arrays; a thread owns 8 consecutive values
 // (one 32-byte sector of f32, one 32-bit word of nibbles), 8 lanes own one
 // 64-value block, a warp owns 4 blocks, and warps stride over the array.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
-#include "nf4_common.cuh"
+#include "kernels.cuh"
+#include "ptx.cuh"
 
 namespace nf4 {
 
@@ -16,6 +18,11 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kWarpsPerCta = kThreads / 32;
 
+// Copies the cell table of the fast code selection into shared memory (a barrier must follow).
+__device__ __forceinline__ void load_cells(uint32_t *cells) {
+    if (threadIdx.x < kCellWords) cells[threadIdx.x] = c_cell_table[threadIdx.x];
+}
+
 __device__ __forceinline__ float group8_max(float m) {
     m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
     m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
@@ -23,94 +30,117 @@ __device__ __forceinline__ float group8_max(float m) {
     return m;
 }
 
-// Full 64-blocks only: `nfull` blocks starting at values[0].  PACKED selects nibble
-// packing (two codes per byte) versus one code per byte.
-template <bool PACKED>
-__global__ void __launch_bounds__(kThreads, 8)
-quantize_full_kernel(const float4 *__restrict__ values, uint64_t nfull,
-                     uint8_t *__restrict__ codes, float *__restrict__ absmax) {
-    __shared__ uint32_t s_cells[32];
-    if (threadIdx.x < 32) s_cells[threadIdx.x] = c_cell_table[threadIdx.x];
-    __syncthreads();
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t warp = (uint64_t)blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
-    const uint64_t nwarps = (uint64_t)gridDim.x * kWarpsPerCta;
-    const uint64_t nchunks = (nfull + 3) / 4;  // one warp-chunk = 4 blocks
-    for (uint64_t chunk = warp; chunk < nchunks; chunk += nwarps) {
-        const uint64_t blk = chunk * 4 + (lane >> 3);
-        const bool live = blk < nfull;
-        const uint64_t g = chunk * 32 + lane;  // group of 8 values
-        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-        if (live) {
-            a = __ldcs(values + 2 * g);
-            b = __ldcs(values + 2 * g + 1);
-        }
-        float m = fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w))),
-                        fmaxf(fmaxf(fabsf(b.x), fabsf(b.y)), fmaxf(fabsf(b.z), fabsf(b.w))));
-        // fold from 0.0 with maxNum: NaNs drop out exactly as f32::max does
-        m = fmaxf(0.0f, m);
-        m = group8_max(m);
-        if (!live) continue;
-        // one exact reciprocal per thread; each value is then decided from x * rcp, and the
-        // whole group is redone exactly if any of its values lands next to a decision threshold
-        bool unsure = !(m >= 1e-30f && m <= 1e30f);
-        const float rcp = __fdiv_rn(1.0f, m);
-        uint32_t c0 = code_of_fast(a.x, rcp, s_cells, unsure),
-                 c1 = code_of_fast(a.y, rcp, s_cells, unsure),
-                 c2 = code_of_fast(a.z, rcp, s_cells, unsure),
-                 c3 = code_of_fast(a.w, rcp, s_cells, unsure),
-                 c4 = code_of_fast(b.x, rcp, s_cells, unsure),
-                 c5 = code_of_fast(b.y, rcp, s_cells, unsure),
-                 c6 = code_of_fast(b.z, rcp, s_cells, unsure),
-                 c7 = code_of_fast(b.w, rcp, s_cells, unsure);
-        if (unsure) {
-            c0 = code_of_exact(a.x, m); c1 = code_of_exact(a.y, m);
-            c2 = code_of_exact(a.z, m); c3 = code_of_exact(a.w, m);
-            c4 = code_of_exact(b.x, m); c5 = code_of_exact(b.y, m);
-            c6 = code_of_exact(b.z, m); c7 = code_of_exact(b.w, m);
-        }
-        if (PACKED) {
-            const uint32_t word = c0 | (c1 << 4) | (c2 << 8) | (c3 << 12) | (c4 << 16) |
-                                  (c5 << 20) | (c6 << 24) | (c7 << 28);
-            reinterpret_cast<uint32_t *>(codes)[g] = word;
-        } else {
-            uint2 w;
-            w.x = c0 | (c1 << 8) | (c2 << 16) | (c3 << 24);
-            w.y = c4 | (c5 << 8) | (c6 << 16) | (c7 << 24);
-            reinterpret_cast<uint2 *>(codes)[g] = w;
-        }
-        if ((lane & 7u) == 0) absmax[blk] = m;
+// fold of |v| from 0.0 with maxNum: NaNs drop out exactly as f32::max does
+__device__ __forceinline__ float absmax8(const float (&v)[8]) {
+    float m = 0.0f;
+    #pragma unroll
+    for (int i = 0; i < 8; ++i) m = fmaxf(m, fabsf(v[i]));
+    return m;
+}
+
+// Eight consecutive f32: one load / store of a whole sector per thread where the buffer is 32-byte
+// aligned (`wide`, the same for a whole launch), two of 16 bytes otherwise.
+__device__ __forceinline__ void ld8_stream(const float *p, float (&v)[8], bool wide) {
+    if (wide) {
+        asm volatile("ld.global.cs.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                     : "l"(p));
+    } else {
+        const float4 a = __ldcs(reinterpret_cast<const float4 *>(p)), b = __ldcs(reinterpret_cast<const float4 *>(p) + 1);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+        v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    }
+}
+__device__ __forceinline__ void st8_stream(float *p, const float (&v)[8], bool wide) {
+    if (wide) {
+        asm volatile("st.global.cs.v8.f32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};" ::"f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]),
+                     "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "l"(p)
+                     : "memory");
+    } else {
+        __stcs(reinterpret_cast<float4 *>(p), make_float4(v[0], v[1], v[2], v[3]));
+        __stcs(reinterpret_cast<float4 *>(p) + 1, make_float4(v[4], v[5], v[6], v[7]));
     }
 }
 
-// Generic path: any alignment, any length.  One warp per block, two values per lane.
-// Used for the ragged last block and for buffers that are not 16-byte aligned.
+// One code per byte from eight nibbles.
+__device__ __forceinline__ uint2 nibbles_to_bytes(uint32_t w) {
+    const uint32_t even = w & 0x0f0f0f0fu, odd = (w >> 4) & 0x0f0f0f0fu;
+    return make_uint2(__byte_perm(even, odd, 0x5140u), __byte_perm(even, odd, 0x7362u));
+}
+
+// One block of up to 64 values by a warp, two values per lane; a missing partner leaves its nibble 0.
+template <bool PACKED>
+__device__ __forceinline__ void quantize_block_by_warp(const float *values, uint32_t n, uint8_t *codes, float *absmax) {
+    const uint32_t lane = threadIdx.x & 31u, e0 = 2 * lane;
+    const bool h0 = e0 < n, h1 = e0 + 1 < n;
+    const float x0 = h0 ? values[e0] : 0.0f;
+    const float x1 = h1 ? values[e0 + 1] : 0.0f;
+    float m = fmaxf(0.0f, fmaxf(fabsf(x0), fabsf(x1)));
+    #pragma unroll
+    for (int s = 1; s < 32; s <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
+    const uint32_t c0 = h0 ? code_of_exact(x0, m) : 0u;
+    const uint32_t c1 = h1 ? code_of_exact(x1, m) : 0u;
+    if (PACKED) {
+        if (h0) codes[lane] = (uint8_t)(c0 | (c1 << 4));
+    } else {
+        if (h0) codes[e0] = (uint8_t)c0;
+        if (h1) codes[e0 + 1] = (uint8_t)c1;
+    }
+    if (lane == 0) *absmax = m;
+}
+
+// 16-byte aligned buffers.  PACKED selects nibble packing (two codes per byte) versus one code per byte.
+// `ngroups` groups of eight values make up the full 64-blocks; a ragged last block (`rest` values) is one
+// more warp's work in the same launch.
+// The loads of a warp's next chunk are in flight while it encodes one: without that a warp's 1 KB
+// arrives, is encoded and only then replaced, and half of the time went to waiting (4096 x 4096:
+// 17.6 us; 22.8 with the slower code selection).
+template <bool PACKED>
+__global__ void __launch_bounds__(kThreads, 6)
+quantize_full_kernel(const float *__restrict__ values, uint32_t ngroups, uint32_t rest,
+                     uint8_t *__restrict__ codes, float *__restrict__ absmax, bool wide) {
+    __shared__ uint32_t s_cells[kCellWords];
+    load_cells(s_cells);
+    __syncthreads();
+    ptx::pdl_wait();
+    ptx::pdl_launch_dependents();
+    // groups of eight values; eight neighbouring lanes hold a block, so a block's lanes are in range together
+    const uint32_t step = gridDim.x * kThreads;
+    uint32_t g = blockIdx.x * kThreads + threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31u;
+    float next[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (g < ngroups) ld8_stream(values + 8 * (uint64_t)g, next, wide);
+    while (g - lane < ngroups) {
+        float v[8];
+        #pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = next[i];
+        const uint32_t ahead = g + step;
+        if (ahead < ngroups) ld8_stream(values + 8 * (uint64_t)ahead, next, wide);
+        const float m = group8_max(absmax8(v));
+        if (g < ngroups) {
+            const uint32_t w = codes_of_group(v, m, s_cells);
+            if (PACKED) reinterpret_cast<uint32_t *>(codes)[g] = w;
+            else reinterpret_cast<uint2 *>(codes)[g] = nibbles_to_bytes(w);
+            if ((lane & 7u) == 0) absmax[g >> 3] = m;
+        }
+        g = ahead;
+    }
+    if (rest && blockIdx.x == gridDim.x - 1 && threadIdx.x < 32)
+        quantize_block_by_warp<PACKED>(values + 8 * (uint64_t)ngroups, rest, codes + (PACKED ? 4 : 8) * (uint64_t)ngroups,
+                                       absmax + ngroups / 8);
+}
+
+// Buffers that are not 16-byte aligned: a warp per block.
 template <bool PACKED>
 __global__ void __launch_bounds__(kThreads)
-quantize_generic_kernel(const float *__restrict__ values, uint64_t len, uint64_t first_block,
-                        uint64_t nblocks, uint8_t *__restrict__ codes,
+quantize_generic_kernel(const float *__restrict__ values, uint64_t len, uint64_t nblocks, uint8_t *__restrict__ codes,
                         float *__restrict__ absmax) {
-    const uint32_t lane = threadIdx.x & 31u;
     const uint64_t warp = (uint64_t)blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
     const uint64_t nwarps = (uint64_t)gridDim.x * kWarpsPerCta;
-    for (uint64_t i = warp; i < nblocks; i += nwarps) {
-        const uint64_t blk = first_block + i;
-        const uint64_t e0 = blk * kBlock + 2 * lane;
-        const bool h0 = e0 < len, h1 = e0 + 1 < len;
-        const float x0 = h0 ? values[e0] : 0.0f;
-        const float x1 = h1 ? values[e0 + 1] : 0.0f;
-        float m = fmaxf(0.0f, fmaxf(h0 ? fabsf(x0) : 0.0f, h1 ? fabsf(x1) : 0.0f));
-        #pragma unroll
-        for (int s = 1; s < 32; s <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
-        const uint32_t c0 = h0 ? code_of(x0, m) : 0u;
-        const uint32_t c1 = h1 ? code_of(x1, m) : 0u;  // a missing partner leaves the nibble 0
-        if (PACKED) {
-            if (h0) codes[e0 >> 1] = (uint8_t)(c0 | (c1 << 4));
-        } else {
-            if (h0) codes[e0] = (uint8_t)c0;
-            if (h1) codes[e0 + 1] = (uint8_t)c1;
-        }
-        if (lane == 0) absmax[blk] = m;
+    for (uint64_t blk = warp; blk < nblocks; blk += nwarps) {
+        const uint64_t left = len - blk * kBlock;
+        quantize_block_by_warp<PACKED>(values + blk * kBlock, left < kBlock ? (uint32_t)left : (uint32_t)kBlock,
+                                       codes + blk * (PACKED ? kBlock / 2 : kBlock), absmax + blk);
     }
 }
 
@@ -122,66 +152,53 @@ __device__ __forceinline__ float block_scale(const float *__restrict__ absmax,
     return absmax ? __ldg(absmax + blk) : dq_scale(__ldg(scale_codes + blk), sos);
 }
 
-// Full 64-blocks, 16-byte aligned buffers.  A lane reads the codes of eight consecutive values;
-// neighbouring lanes then swap halves so that the pair's two 128-bit stores each fill whole
-// 32-byte sectors (lane 2j writes values 16j..16j+3 and 16j+8..16j+11, lane 2j+1 the other two
-// quads).  Four such groups are in flight per thread to cover the load latency.
+// 16-byte aligned buffers.  A thread turns the codes of eight consecutive values into one 32-byte
+// sector of output; four such groups are in flight per thread to cover the load latency.  The last
+// len % 8 values go element by element.
 template <bool PACKED>
-__global__ void __launch_bounds__(kThreads, 8)
-dequantize_full_kernel(const uint8_t *__restrict__ codes, uint64_t nfull,
+__global__ void __launch_bounds__(kThreads, 7)
+dequantize_full_kernel(const uint8_t *__restrict__ codes, uint64_t len,
                        const float *__restrict__ absmax, const uint8_t *__restrict__ scale_codes,
-                       const float *__restrict__ scale_of_scales, float4 *__restrict__ out) {
+                       const float *__restrict__ scale_of_scales, float *__restrict__ out, bool wide) {
     constexpr int kInFlight = 4;
     __shared__ float s_levels[16];
     if (threadIdx.x < 16) s_levels[threadIdx.x] = __uint_as_float(c_level_bits[threadIdx.x]);
     __syncthreads();
+    ptx::pdl_wait();
+    ptx::pdl_launch_dependents();
     const float sos = scale_of_scales ? __ldg(scale_of_scales) : 0.0f;
-    const uint64_t ngroups = nfull * 8;  // 8 values per group; a multiple of 8, so lane pairs stay whole
+    const uint64_t ngroups = len / 8;  // 8 values per group
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x < (len & 7u)) {
+        const uint64_t e = 8 * ngroups + threadIdx.x;
+        const uint32_t c = PACKED ? (uint32_t)codes[e >> 1] >> (4 * (e & 1u)) : codes[e];
+        out[e] = __fmul_rn(s_levels[c & 15u], block_scale(absmax, scale_codes, sos, e / kBlock));
+    }
     const uint64_t stride = (uint64_t)gridDim.x * kThreads;
-    const uint32_t lane = threadIdx.x & 31u;
-    const bool odd = lane & 1u;
-    const uint64_t first = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
-    for (uint64_t g0 = first; g0 - lane < ngroups; g0 += stride * kInFlight) {
-        uint32_t lo[kInFlight], hi[kInFlight];  // codes of the first / second quad this lane stores
+    for (uint64_t g0 = (uint64_t)blockIdx.x * kThreads + threadIdx.x; g0 < ngroups; g0 += stride * kInFlight) {
+        uint2 w[kInFlight];
         float s[kInFlight];
         #pragma unroll
         for (int u = 0; u < kInFlight; ++u) {
             const uint64_t g = g0 + u * stride;
             const bool live = g < ngroups;
-            uint32_t a = 0, b = 0;  // codes of values 0..3 and 4..7 of the group
-            if (PACKED) {
-                const uint32_t w = live ? __ldcs(reinterpret_cast<const uint32_t *>(codes) + g) : 0u;
-                a = w & 0xffffu;
-                b = w >> 16;
-            } else {
-                const uint2 w = live ? __ldcs(reinterpret_cast<const uint2 *>(codes) + g)
-                                     : make_uint2(0u, 0u);
-                a = w.x;
-                b = w.y;
+            w[u] = make_uint2(0u, 0u);
+            if (live) {
+                if (PACKED) w[u].x = __ldcs(reinterpret_cast<const uint32_t *>(codes) + g);
+                else w[u] = __ldcs(reinterpret_cast<const uint2 *>(codes) + g);
             }
             s[u] = live ? block_scale(absmax, scale_codes, sos, g >> 3) : 0.0f;
-            const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
-            lo[u] = odd ? got : a;  // even: own first quad;   odd: partner's second quad
-            hi[u] = odd ? b : got;  // even: partner's first quad; odd: own second quad
         }
         #pragma unroll
         for (int u = 0; u < kInFlight; ++u) {
             const uint64_t g = g0 + u * stride;
             if (g >= ngroups) continue;
-            constexpr int kBits = PACKED ? 4 : 8;
-            float4 q0, q1;
-            q0.x = __fmul_rn(s_levels[(lo[u] >> (0 * kBits)) & 15u], s[u]);
-            q0.y = __fmul_rn(s_levels[(lo[u] >> (1 * kBits)) & 15u], s[u]);
-            q0.z = __fmul_rn(s_levels[(lo[u] >> (2 * kBits)) & 15u], s[u]);
-            q0.w = __fmul_rn(s_levels[(lo[u] >> (3 * kBits)) & 15u], s[u]);
-            q1.x = __fmul_rn(s_levels[(hi[u] >> (0 * kBits)) & 15u], s[u]);
-            q1.y = __fmul_rn(s_levels[(hi[u] >> (1 * kBits)) & 15u], s[u]);
-            q1.z = __fmul_rn(s_levels[(hi[u] >> (2 * kBits)) & 15u], s[u]);
-            q1.w = __fmul_rn(s_levels[(hi[u] >> (3 * kBits)) & 15u], s[u]);
-            // pair base = float4 index 2 * (g & ~1); even lane stores quads 0 and 2, odd 1 and 3
-            float4 *dst = out + 2 * (g & ~(uint64_t)1) + (odd ? 1 : 0);
-            __stcs(dst, q0);
-            __stcs(dst + 2, q1);
+            float v[8];
+            #pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const uint32_t word = PACKED || i < 4 ? w[u].x : w[u].y;
+                v[i] = __fmul_rn(s_levels[(word >> ((PACKED ? 4 * i : 8 * (i & 3)))) & 15u], s[u]);
+            }
+            st8_stream(out + 8 * g, v, wide);
         }
     }
 }
@@ -211,82 +228,72 @@ dequantize_generic_kernel(const uint8_t *__restrict__ codes, uint64_t len, uint6
 // src is [rows, cols] row-major (a PyTorch linear weight [out, in], bf16 or f32); the result is
 // the packed NF4 of its transpose [cols, rows] flattened row-major, i.e. element (c, r) at flat
 // index c * rows + r.  With rows % 64 == 0 a 64-block of the result is 64 consecutive r for one
-// c: a column segment of src.  One CTA takes a 64 x 64 tile of src through shared memory
-// (coalesced reads along c, conflict-free reads along r) and its eight warps quantize the tile's
-// 64 blocks with the same arithmetic as quantize_full_kernel.
-constexpr int kTTile = 64;
-constexpr int kTStride = kTTile + 1;  // floats between the tile's transposed rows (odd: spreads the banks)
+// c: a column segment of src.
+// Two lanes (kSplit) share a column of f32, or a pair of columns of bf16 (one 32-bit word per row):
+// each keeps 32 of the segment's 64 rows in registers, so a warp's load touches 64 bytes of two rows,
+// 32 loads are in flight per thread, a block's maximum is one shuffle and its codes leave as one sector.  No shared-memory transpose.  CTAs that are neighbours in launch order
+// take neighbouring row segments, so the sectors of an output line meet in the L2.
+// Bound by instruction issue (14 per value: half of them select the code) and the L2's tag lookups.
+// bf16 [14336, 4096]: 40 us; 92 through a 64 x 64 tile in shared memory with eight lanes per block; 49
+// with all 64 rows in one thread's registers (twenty warps per SM) and with sixteen rows per thread
+// (32-byte pieces of four rows per load: the L2 was busy with lookups).
+constexpr int kTThreads = 128;
+constexpr int kSplit = 2, kSplitRows = kBlock / kSplit, kSplitWords = 32 / kSplit;
+constexpr int kTWords = kTThreads / kSplit;  // words (columns or pairs) a CTA covers
 
 template <bool SRC_BF16>
-__global__ void __launch_bounds__(kThreads)
-quantize_transposed_kernel(const void *__restrict__ src, uint64_t rows, uint64_t cols,
-                           uint8_t *__restrict__ codes, float *__restrict__ absmax) {
-    __shared__ float s_t[kTTile * kTStride];  // s_t[c][r]
-    __shared__ uint32_t s_cells[32];
-    if (threadIdx.x < 32) s_cells[threadIdx.x] = c_cell_table[threadIdx.x];
-    const uint64_t tiles_c = (cols + kTTile - 1) / kTTile;
-    const uint64_t r0 = (blockIdx.x / tiles_c) * kTTile, c0 = (blockIdx.x % tiles_c) * kTTile;
-    // 256 threads: thread t reads row (t >> 4) + 16 i, columns 4 (t & 15) .. + 3
-    #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const uint64_t r = r0 + (threadIdx.x >> 4) + 16 * i;
-        const uint64_t c = c0 + 4 * (threadIdx.x & 15u);
-        float v[4] = {0.f, 0.f, 0.f, 0.f};
-        if (c + 3 < cols) {
-            if (SRC_BF16) {
-                const uint2 w = __ldcs(reinterpret_cast<const uint2 *>(
-                    static_cast<const __nv_bfloat16 *>(src) + r * cols + c));
-                v[0] = __uint_as_float(w.x << 16);
-                v[1] = __uint_as_float(w.x & 0xffff0000u);
-                v[2] = __uint_as_float(w.y << 16);
-                v[3] = __uint_as_float(w.y & 0xffff0000u);
-            } else {
-                const float4 w = __ldcs(reinterpret_cast<const float4 *>(
-                    static_cast<const float *>(src) + r * cols + c));
-                v[0] = w.x; v[1] = w.y; v[2] = w.z; v[3] = w.w;
-            }
-        } else {
-            for (int k = 0; k < 4; ++k)
-                if (c + k < cols)
-                    v[k] = SRC_BF16 ? __bfloat162float(static_cast<const __nv_bfloat16 *>(src)[r * cols + c + k])
-                                    : static_cast<const float *>(src)[r * cols + c + k];
-        }
-        const uint32_t rl = (threadIdx.x >> 4) + 16 * i, cl = 4 * (threadIdx.x & 15u);
-        #pragma unroll
-        for (int k = 0; k < 4; ++k) s_t[(cl + k) * kTStride + rl] = v[k];
-    }
+__global__ void __launch_bounds__(kTThreads, 7)
+quantize_transposed_kernel(const uint32_t *__restrict__ src, uint32_t segments, uint32_t words_per_row,
+                           uint8_t *__restrict__ codes, float *__restrict__ absmax, bool wide) {
+    __shared__ uint32_t s_cells[kCellWords];
+    load_cells(s_cells);
     __syncthreads();
-    // warp w quantizes the blocks of columns c0 + 8 w .. + 7, four at a time: lane l owns values
-    // 8 (l & 7) .. + 7 of block (l >> 3)
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    ptx::pdl_wait();
+    ptx::pdl_launch_dependents();
+    const uint32_t tile = blockIdx.x / segments, seg = blockIdx.x - tile * segments;
+    const uint32_t lane = threadIdx.x & 31u, part = lane / kSplitWords;  // which 32 rows
+    const uint32_t word = tile * kTWords + (threadIdx.x >> 5) * kSplitWords + lane % kSplitWords;
+    const bool in = word < words_per_row;  // (the lanes of a word agree)
+    const uint32_t *p = src + (uint64_t)(seg * kBlock + part * kSplitRows) * words_per_row + word;
+    uint32_t w[kSplitRows];
     #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-        const uint32_t cl = 8 * warp + 4 * half + (lane >> 3);
-        const uint64_t c = c0 + cl;
-        const float *sp = &s_t[cl * kTStride + 8 * (lane & 7u)];
-        const float4 a = make_float4(sp[0], sp[1], sp[2], sp[3]);
-        const float4 b = make_float4(sp[4], sp[5], sp[6], sp[7]);
-        float m = fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w))),
-                        fmaxf(fmaxf(fabsf(b.x), fabsf(b.y)), fmaxf(fabsf(b.z), fabsf(b.w))));
-        m = group8_max(fmaxf(0.0f, m));
-        if (c >= cols) continue;
-        bool unsure = !(m >= 1e-30f && m <= 1e30f);
-        const float rcp = __fdiv_rn(1.0f, m);
-        uint32_t q0 = code_of_fast(a.x, rcp, s_cells, unsure), q1 = code_of_fast(a.y, rcp, s_cells, unsure),
-                 q2 = code_of_fast(a.z, rcp, s_cells, unsure), q3 = code_of_fast(a.w, rcp, s_cells, unsure),
-                 q4 = code_of_fast(b.x, rcp, s_cells, unsure), q5 = code_of_fast(b.y, rcp, s_cells, unsure),
-                 q6 = code_of_fast(b.z, rcp, s_cells, unsure), q7 = code_of_fast(b.w, rcp, s_cells, unsure);
-        if (unsure) {
-            q0 = code_of_exact(a.x, m); q1 = code_of_exact(a.y, m); q2 = code_of_exact(a.z, m);
-            q3 = code_of_exact(a.w, m); q4 = code_of_exact(b.x, m); q5 = code_of_exact(b.y, m);
-            q6 = code_of_exact(b.z, m); q7 = code_of_exact(b.w, m);
+    for (int r = 0; r < kSplitRows; ++r, p += words_per_row) w[r] = in ? __ldcs(p) : 0u;
+    uint32_t mx = 0;  // both columns' maxima of |bf16| as a pair (NaNs drop out), or the f32 column's
+    auto larger = [&](uint32_t v) {
+        if (SRC_BF16) asm("max.bf16x2 %0, %0, %1;" : "+r"(mx) : "r"(v & 0x7fff7fffu));
+        else mx = __float_as_uint(fmaxf(__uint_as_float(mx), fabsf(__uint_as_float(v))));
+    };
+    #pragma unroll
+    for (int r = 0; r < kSplitRows; ++r) larger(w[r]);
+    #pragma unroll
+    for (int s = kSplitWords; s < 32; s <<= 1) larger(__shfl_xor_sync(0xffffffffu, mx, s));
+    if (!in) return;
+    constexpr int kCols = SRC_BF16 ? 2 : 1;
+    #pragma unroll 1  // (unrolled, both columns' values would be kept in registers at once)
+    for (int h = 0; h < kCols; ++h) {
+        const uint32_t half = h == 0 ? 0x1044u : 0x3244u;
+        auto value = [&](uint32_t bits) { return __uint_as_float(SRC_BF16 ? __byte_perm(bits, 0u, half) : bits); };
+        const float m = value(mx);
+        const uint64_t blk = (uint64_t)(word * kCols + h) * segments + seg;  // the block's number in the result
+        uint32_t out[kSplitRows / 8];
+        #pragma unroll
+        for (int g = 0; g < kSplitRows / 8; ++g) {
+            float v[8];
+            #pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = value(w[8 * g + i]);
+            out[g] = codes_of_group(v, m, s_cells);
         }
-        const uint64_t e = c * rows + r0 + 8 * (lane & 7u);  // flat index of this lane's first value
-        reinterpret_cast<uint32_t *>(codes)[e / 8] = q0 | (q1 << 4) | (q2 << 8) | (q3 << 12) | (q4 << 16) |
-                                                     (q5 << 20) | (q6 << 24) | (q7 << 28);
-        if ((lane & 7u) == 0) absmax[e / kBlock] = m;
+        uint32_t *dst = reinterpret_cast<uint32_t *>(codes + blk * (kBlock / 2) + part * (kSplitRows / 2));
+        if (wide) {
+            *reinterpret_cast<uint4 *>(dst) = make_uint4(out[0], out[1], out[2], out[3]);
+        } else {  // codes only 4-byte aligned
+            #pragma unroll
+            for (int g = 0; g < kSplitRows / 8; ++g) dst[g] = out[g];
+        }
+        if (part == 0) absmax[blk] = m;
     }
 }
+static_assert(kSplitRows == 32, "a lane stores four words of codes per block");
 
 // Any shape: the transpose written out as f32 (then quantized by the flat kernels).
 template <bool SRC_BF16>
@@ -319,76 +326,178 @@ transpose_to_f32_kernel(const void *__restrict__ src, uint64_t rows, uint64_t co
 // word and one block scale; other widths take the element-wise path.  An id outside
 // [0, n_embedding) yields a row of NaNs (the reference's gather would panic; a device kernel
 // must not trap).
+//
+// A warp takes a segment of 1024 consecutive elements of a row, four groups of eight per lane with
+// their loads in flight together; the row and segment come from one 32-bit division per warp (a
+// 64-bit division per group and one group in flight took 13.8 us for 4096 rows of 3584 in bf16).
+constexpr uint32_t kGatherGroups = 4;  // groups of eight per lane
 template <bool BF16>
 __global__ void __launch_bounds__(kThreads)
 embedding_gather_kernel(const uint8_t *__restrict__ codes, const float *__restrict__ absmax,
                         const uint8_t *__restrict__ scale_codes,
                         const float *__restrict__ scale_of_scales, uint64_t n_embedding,
-                        uint64_t d_model, const int64_t *__restrict__ ids, uint64_t n_ids,
-                        void *__restrict__ out) {
+                        uint32_t groups_per_row, const int64_t *__restrict__ ids, uint32_t segments,
+                        uint32_t work, void *__restrict__ out, bool wide) {
     __shared__ float s_levels[16];
     if (threadIdx.x < 16) s_levels[threadIdx.x] = __uint_as_float(c_level_bits[threadIdx.x]);
     __syncthreads();
+    ptx::pdl_wait();
+    ptx::pdl_launch_dependents();
+    const uint32_t item = blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+    if (item >= work) return;
+    const uint32_t t = item / segments, g0 = (item - t * segments) * (32 * kGatherGroups) + lane;
+    const int64_t id = __ldg(ids + t);
+    const bool known = id >= 0 && (uint64_t)id < n_embedding;
     const float sos = scale_of_scales ? __ldg(scale_of_scales) : 0.0f;
-    const float nan = __uint_as_float(0x7fc00000u);
-    const uint64_t stride = (uint64_t)gridDim.x * kThreads;
-    const uint64_t first = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
-    if ((d_model & 7u) == 0) {
-        const uint64_t groups_per_row = d_model / 8, total = n_ids * groups_per_row;
-        for (uint64_t i = first; i < total; i += stride) {
-            const uint64_t t = i / groups_per_row, gi = i - t * groups_per_row;
-            const int64_t id = __ldg(ids + t);
-            float v[8];
-            if (id < 0 || (uint64_t)id >= n_embedding) {
-                #pragma unroll
-                for (int k = 0; k < 8; ++k) v[k] = nan;
-            } else {
-                const uint64_t e = (uint64_t)id * d_model + gi * 8;  // a multiple of 8
-                const uint32_t w = __ldg(reinterpret_cast<const uint32_t *>(codes) + e / 8);
-                const float sc = block_scale(absmax, scale_codes, sos, e / kBlock);
-                #pragma unroll
-                for (int k = 0; k < 8; ++k) v[k] = __fmul_rn(s_levels[(w >> (4 * k)) & 15u], sc);
+    const uint64_t row = (uint64_t)(known ? id : 0) * groups_per_row;
+    uint32_t w[kGatherGroups];
+    float s[kGatherGroups];
+    #pragma unroll
+    for (uint32_t u = 0; u < kGatherGroups; ++u) {
+        const uint32_t g = g0 + 32 * u;
+        const bool in = known && g < groups_per_row;
+        w[u] = in ? __ldg(reinterpret_cast<const uint32_t *>(codes) + row + g) : 0u;
+        s[u] = in ? block_scale(absmax, scale_codes, sos, (row + g) >> 3) : __uint_as_float(0x7fc00000u);  // NaN
+    }
+    #pragma unroll
+    for (uint32_t u = 0; u < kGatherGroups; ++u) {
+        const uint32_t g = g0 + 32 * u;
+        if (g >= groups_per_row) continue;
+        float v[8];
+        #pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = __fmul_rn(s_levels[(w[u] >> (4 * k)) & 15u], s[u]);
+        const uint64_t at = (uint64_t)t * groups_per_row + g;
+        if (BF16) {
+            uint32_t o[4];
+            #pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
+                o[k] = *reinterpret_cast<const uint32_t *>(&h);
             }
-            if (BF16) {
-                uint32_t o[4];
-                #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
-                    o[k] = *reinterpret_cast<const uint32_t *>(&h);
-                }
-                reinterpret_cast<uint4 *>(out)[i] = make_uint4(o[0], o[1], o[2], o[3]);
-            } else {
-                float4 *dst = reinterpret_cast<float4 *>(out) + 2 * i;
-                __stcs(dst, make_float4(v[0], v[1], v[2], v[3]));
-                __stcs(dst + 1, make_float4(v[4], v[5], v[6], v[7]));
-            }
-        }
-    } else {
-        const uint64_t total = n_ids * d_model;
-        for (uint64_t i = first; i < total; i += stride) {
-            const uint64_t t = i / d_model, j = i - t * d_model;
-            const int64_t id = __ldg(ids + t);
-            float v = nan;
-            if (id >= 0 && (uint64_t)id < n_embedding) {
-                const uint64_t e = (uint64_t)id * d_model + j;
-                const uint32_t byte = __ldg(codes + (e >> 1));
-                const uint32_t c = (e & 1u) ? (byte >> 4) : (byte & 15u);
-                v = __fmul_rn(__uint_as_float(c_level_bits[c]), block_scale(absmax, scale_codes, sos, e / kBlock));
-            }
-            if (BF16) reinterpret_cast<__nv_bfloat16 *>(out)[i] = __float2bfloat16_rn(v);
-            else reinterpret_cast<float *>(out)[i] = v;
+            reinterpret_cast<uint4 *>(out)[at] = make_uint4(o[0], o[1], o[2], o[3]);
+        } else {
+            st8_stream(static_cast<float *>(out) + 8 * at, v, wide);
         }
     }
 }
 
-// ---- double quantization ------------------------------------------------------
+// Widths that are no multiple of eight: element by element.
+template <bool BF16>
+__global__ void __launch_bounds__(kThreads)
+embedding_gather_elements_kernel(const uint8_t *__restrict__ codes, const float *__restrict__ absmax,
+                                 const uint8_t *__restrict__ scale_codes,
+                                 const float *__restrict__ scale_of_scales, uint64_t n_embedding,
+                                 uint64_t d_model, const int64_t *__restrict__ ids, uint64_t n_ids,
+                                 void *__restrict__ out) {
+    const float sos = scale_of_scales ? __ldg(scale_of_scales) : 0.0f;
+    const uint64_t total = n_ids * d_model, stride = (uint64_t)gridDim.x * kThreads;
+    for (uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x; i < total; i += stride) {
+        const uint64_t t = i / d_model, j = i - t * d_model;
+        const int64_t id = __ldg(ids + t);
+        float v = __uint_as_float(0x7fc00000u);
+        if (id >= 0 && (uint64_t)id < n_embedding) {
+            const uint64_t e = (uint64_t)id * d_model + j;
+            const uint32_t byte = __ldg(codes + (e >> 1));
+            const uint32_t c = (e & 1u) ? (byte >> 4) : (byte & 15u);
+            v = __fmul_rn(__uint_as_float(c_level_bits[c]), block_scale(absmax, scale_codes, sos, e / kBlock));
+        }
+        if (BF16) reinterpret_cast<__nv_bfloat16 *>(out)[i] = __float2bfloat16_rn(v);
+        else reinterpret_cast<float *>(out)[i] = v;
+    }
+}
 
-// Pass 1: max over the (non-negative, never-NaN) block scales.  Their f32 bit patterns
-// order like unsigned integers, so one atomicMax on the bits per warp is exact.
+// ---- double quantization ------------------------------------------------------
+// c = round_half_away(s / max * 255) clamped to [0, 255]; 0 when max == 0 (src/quantize.rs:294-301).
+// A NaN quotient (inf / inf) casts to 0 as Rust's `as u8`.
+
+static __device__ __noinline__ uint32_t scale_code_exact(float s, float max_scale) {
+    if (max_scale == 0.0f) return 0u;
+    float q = roundf(__fmul_rn(__fdiv_rn(s, max_scale), 255.0f));
+    q = fminf(fmaxf(q, 0.0f), 255.0f);  // NaN -> 0 through fmaxf
+    return (uint32_t)q;
+}
+
+// The same without the division where that is safe: t = s * (255 / max) is within 1.2e-4 of the
+// reference's product, so unless it lies within 2.5e-4 of a half (or is NaN, or the largest scale is
+// outside the reciprocal's range) both round to the same integer.
+struct ScaleEncoder {
+    float max_scale, factor;
+    bool ranged;
+    __device__ explicit ScaleEncoder(float m)
+        : max_scale(m), factor(255.0f * approx_rcp(m)), ranged(m >= 1e-30f && m <= 1e30f) {}
+    __device__ __forceinline__ uint32_t four(const float4 &v) const {
+        const float s[4] = {v.x, v.y, v.z, v.w};
+        uint32_t c[4];
+        bool sure = ranged;
+        #pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float t = __fmul_rn(s[i], factor), r = t + 12582912.0f;  // t's nearest integer in the low mantissa bits
+            sure = sure && fabsf(t - (r - 12582912.0f)) < 0.49975f;
+            c[i] = __float_as_uint(r);
+        }
+        if (!sure) {
+            #pragma unroll
+            for (int i = 0; i < 4; ++i) c[i] = scale_code_exact(s[i], max_scale);
+        }
+        return __byte_perm(__byte_perm(c[0], c[1], 0x0040u), __byte_perm(c[2], c[3], 0x0040u), 0x5410u);
+    }
+};
+
+// Pass 1 for up to kClusterMaxBlocks scales: the maximum by one cluster of sixteen CTAs, whose results
+// meet in distributed shared memory, so that no word has to be cleared first.  Sixteen SMs with eight
+// 16-byte loads in flight per thread read 3.7 MB (the scales of 14336 x 4096 weights) from the L2 in
+// about 2 us.  (Both passes in one cluster: 16 us, the encoding is too much work for sixteen SMs.)
+constexpr int kClusterCtas = 16, kClusterThreads = 1024;
+constexpr uint64_t kClusterMaxBlocks = 1u << 20;
+
+__global__ void __launch_bounds__(kClusterThreads, 1)
+scale_max_cluster_kernel(const float4 *__restrict__ absmax4, const float *__restrict__ absmax, uint32_t nblocks,
+                         float *__restrict__ scale_of_scales) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    __shared__ float s_warp[kClusterThreads / 32];
+    __shared__ float s_cta[kClusterCtas];
+    const uint32_t rank = cluster.block_rank(), tid = threadIdx.x;
+    const uint32_t n4 = nblocks / 4;
+    constexpr uint32_t kStride = kClusterCtas * kClusterThreads, kInFlight = 8;
+    ptx::pdl_wait();
+    ptx::pdl_launch_dependents();
+    float m = 0.0f;
+    for (uint32_t i = rank * kClusterThreads + tid; i < n4; i += kStride * kInFlight) {
+        float4 v[kInFlight];
+        #pragma unroll
+        for (uint32_t u = 0; u < kInFlight; ++u)
+            v[u] = i + u * kStride < n4 ? __ldg(absmax4 + i + u * kStride) : make_float4(0.f, 0.f, 0.f, 0.f);
+        #pragma unroll
+        for (uint32_t u = 0; u < kInFlight; ++u) m = fmaxf(fmaxf(m, fmaxf(v[u].x, v[u].y)), fmaxf(v[u].z, v[u].w));
+    }
+    if (rank == 0 && 4 * n4 + tid < nblocks) m = fmaxf(m, __ldg(absmax + 4 * n4 + tid));
+    #pragma unroll
+    for (int s = 1; s < 32; s <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
+    if ((tid & 31u) == 0) s_warp[tid >> 5] = m;
+    __syncthreads();
+    if (tid < 32) {
+        m = s_warp[tid];
+        #pragma unroll
+        for (int s = 1; s < 32; s <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
+        if (tid == 0) cluster.map_shared_rank(s_cta, 0)[rank] = m;
+    }
+    cluster.sync();
+    if (rank == 0 && tid == 0) {
+        m = s_cta[0];
+        #pragma unroll
+        for (int r = 1; r < kClusterCtas; ++r) m = fmaxf(m, s_cta[r]);
+        *scale_of_scales = m;
+    }
+}
+
+// More scales, or unaligned ones.  Pass 1: max over the (non-negative, never-NaN) block scales.  Their
+// f32 bit patterns order like unsigned integers, so one atomicMax on the bits per warp is exact.
 __global__ void __launch_bounds__(kThreads)
 scale_max_kernel(const float *__restrict__ absmax, uint64_t nblocks, uint32_t *max_bits) {
     float m = 0.0f;
     const uint64_t stride = (uint64_t)gridDim.x * kThreads;
+    #pragma unroll 4
     for (uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x; i < nblocks; i += stride)
         m = fmaxf(m, __ldg(absmax + i));
     #pragma unroll
@@ -396,23 +505,23 @@ scale_max_kernel(const float *__restrict__ absmax, uint64_t nblocks, uint32_t *m
     if ((threadIdx.x & 31u) == 0) atomicMax(max_bits, __float_as_uint(m));
 }
 
-// Pass 2: c = round_half_away(s / max * 255) clamped to [0, 255]; 0 when max == 0
-// (src/quantize.rs:294-301).  A NaN quotient (inf / inf) casts to 0 as Rust's `as u8`.
+// Pass 2, four scales per thread; `whole`: both buffers allow words of four.
 __global__ void __launch_bounds__(kThreads)
 scale_encode_kernel(const float *__restrict__ absmax, uint64_t nblocks,
-                    const float *__restrict__ max_scale_ptr, uint8_t *__restrict__ scale_codes) {
+                    const float *max_scale_ptr, uint8_t *__restrict__ scale_codes, bool whole) {
+    ptx::pdl_wait();
+    ptx::pdl_launch_dependents();
     const float max_scale = *max_scale_ptr;
-    const uint64_t stride = (uint64_t)gridDim.x * kThreads;
-    for (uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x; i < nblocks; i += stride) {
-        uint32_t c = 0;
-        if (max_scale != 0.0f) {
-            float q = roundf(__fmul_rn(__fdiv_rn(__ldg(absmax + i), max_scale), 255.0f));
-            q = fminf(fmaxf(q, 0.0f), 255.0f);  // NaN -> 0 through fmaxf
-            c = (uint32_t)q;
-        }
-        scale_codes[i] = (uint8_t)c;
-    }
+    const uint64_t stride = (uint64_t)gridDim.x * kThreads, first = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
+    const uint64_t n4 = whole ? nblocks / 4 : 0;
+    const ScaleEncoder enc(max_scale);
+    for (uint64_t i = first; i < n4; i += stride)
+        reinterpret_cast<uint32_t *>(scale_codes)[i] = enc.four(__ldg(reinterpret_cast<const float4 *>(absmax) + i));
+    for (uint64_t i = 4 * n4 + first; i < nblocks; i += stride)
+        scale_codes[i] = (uint8_t)scale_code_exact(__ldg(absmax + i), max_scale);
 }
+
+inline bool aligned32(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 31u) == 0; }
 
 int grid_for(uint64_t work_items, int per_cta, int max_waves) {
     uint64_t ctas = (work_items + per_cta - 1) / per_cta;
@@ -422,27 +531,26 @@ int grid_for(uint64_t work_items, int per_cta, int max_waves) {
     return (int)ctas;
 }
 
+constexpr uint64_t kSliceBlocks = 1ull << 27;  // blocks one launch of a flat kernel takes
+
 template <bool PACKED>
 int32_t quantize_impl(const float *values, uint64_t len, uint8_t *codes, float *absmax,
                       cudaStream_t stream) {
     if (len == 0) return NF4_OK;
     if (!values || !codes || !absmax) return fail(NF4_ERR_INVALID_ARG, "nf4_quantize: null pointer");
     const uint64_t nblocks = (len + kBlock - 1) / kBlock;
-    const bool fast = aligned16(values) && aligned16(codes) && ((uintptr_t)absmax % 4 == 0);
-    uint64_t nfull = fast ? len / kBlock : 0;
-    if (nfull) {
-        const int grid = grid_for((nfull + 3) / 4, kWarpsPerCta, 8);
-        quantize_full_kernel<PACKED><<<grid, kThreads, 0, stream>>>(
-            reinterpret_cast<const float4 *>(values), nfull, codes, absmax);
-        count_launch();
+    if (aligned16(values) && aligned16(codes) && ((uintptr_t)absmax % 4 == 0)) {
+        for (uint64_t b0 = 0; b0 < nblocks; b0 += kSliceBlocks) {  // (32-bit positions in the kernel)
+            const uint64_t left = len - b0 * kBlock, n = left < kSliceBlocks * kBlock ? left : kSliceBlocks * kBlock;
+            count_launch();
+            NF4_TRY(launch_maybe_overlapped(quantize_full_kernel<PACKED>, dim3(grid_for((n + 7) / 8, kThreads, 6)), dim3(kThreads), 0,
+                                            stream, true, values + b0 * kBlock, (uint32_t)(n / kBlock * 8), (uint32_t)(n % kBlock),
+                                            codes + b0 * (PACKED ? kBlock / 2 : kBlock), absmax + b0, aligned32(values)));
+        }
+        return NF4_OK;
     }
-    if (nfull < nblocks) {
-        const uint64_t rest = nblocks - nfull;
-        const int grid = grid_for(rest, kWarpsPerCta, 8);
-        quantize_generic_kernel<PACKED><<<grid, kThreads, 0, stream>>>(values, len, nfull, rest,
-                                                                      codes, absmax);
-        count_launch();
-    }
+    quantize_generic_kernel<PACKED><<<grid_for(nblocks, kWarpsPerCta, 8), kThreads, 0, stream>>>(values, len, nblocks, codes, absmax);
+    count_launch();
     return check_cuda(cudaGetLastError(), "nf4_quantize launch");
 }
 
@@ -457,21 +565,14 @@ int32_t dequantize_impl(const uint8_t *codes, uint64_t len, const float *absmax,
                     "nf4_dequantize: give either absmax or scale_codes+scale_of_scales");
     if (scale_codes && !scale_of_scales)
         return fail(NF4_ERR_INVALID_ARG, "nf4_dequantize: scale_codes without scale_of_scales");
-    const bool fast = aligned16(codes) && aligned16(out);
-    const uint64_t nfull = fast ? len / kBlock : 0;
-    if (nfull) {
-        const int grid = grid_for(nfull * 8, kThreads, 8);
-        dequantize_full_kernel<PACKED><<<grid, kThreads, 0, stream>>>(
-            codes, nfull, absmax, scale_codes, scale_of_scales, reinterpret_cast<float4 *>(out));
+    if (aligned16(codes) && aligned16(out)) {
         count_launch();
+        return launch_maybe_overlapped(dequantize_full_kernel<PACKED>, dim3(grid_for(len / 8, kThreads, 7)), dim3(kThreads), 0, stream,
+                                       true, codes, len, absmax, scale_codes, scale_of_scales, out, aligned32(out));
     }
-    if (nfull * kBlock < len) {
-        const uint64_t rest = len - nfull * kBlock;
-        const int grid = grid_for(rest, kThreads, 8);
-        dequantize_generic_kernel<PACKED><<<grid, kThreads, 0, stream>>>(
-            codes, len, nfull * kBlock, absmax, scale_codes, scale_of_scales, out);
-        count_launch();
-    }
+    dequantize_generic_kernel<PACKED><<<grid_for(len, kThreads, 8), kThreads, 0, stream>>>(codes, len, 0, absmax, scale_codes,
+                                                                                         scale_of_scales, out);
+    count_launch();
     return check_cuda(cudaGetLastError(), "nf4_dequantize launch");
 }
 
@@ -504,17 +605,18 @@ int32_t quantize_transposed(const void *src, bool src_bf16, uint64_t rows, uint6
                             cudaStream_t stream) {
     if (rows == 0 || cols == 0) return NF4_OK;
     if (!src || !packed || !absmax) return fail(NF4_ERR_INVALID_ARG, "nf4_quantize_transposed: null pointer");
-    const bool fused = rows % kTTile == 0 && cols % 4 == 0 && aligned16(src) &&
+    const bool fused = rows % kBlock == 0 && cols % 4 == 0 && aligned16(src) &&
                        (reinterpret_cast<uintptr_t>(packed) & 3u) == 0;
     if (fused) {
-        const uint64_t tiles = (rows / kTTile) * ((cols + kTTile - 1) / kTTile);
-        if (tiles >= (1ull << 31)) return fail(NF4_ERR_UNSUPPORTED, "nf4_quantize_transposed: matrix too large");
-        if (src_bf16)
-            quantize_transposed_kernel<true><<<(unsigned)tiles, kThreads, 0, stream>>>(src, rows, cols, packed, absmax);
-        else
-            quantize_transposed_kernel<false><<<(unsigned)tiles, kThreads, 0, stream>>>(src, rows, cols, packed, absmax);
+        const uint64_t words = src_bf16 ? cols / 2 : cols;
+        const uint64_t ctas = rows / kBlock * ((words + kTWords - 1) / kTWords);
+        if (ctas >= (1ull << 31) || rows >= (1ull << 31) || cols >= (1ull << 31))
+            return fail(NF4_ERR_UNSUPPORTED, "nf4_quantize_transposed: matrix too large");
+        const uint32_t *w = static_cast<const uint32_t *>(src);
         count_launch();
-        return check_cuda(cudaGetLastError(), "nf4_quantize_transposed launch");
+        return launch_maybe_overlapped(src_bf16 ? quantize_transposed_kernel<true> : quantize_transposed_kernel<false>,
+                                       dim3((unsigned)ctas), dim3(kTThreads), 0, stream, true, w, (uint32_t)(rows / kBlock), (uint32_t)words, packed, absmax,
+                                       aligned16(packed));
     }
     // other shapes: transpose into the caller's workspace, then the flat quantizer
     const uint64_t need = rows * cols * sizeof(float);
@@ -545,14 +647,19 @@ int32_t embedding_gather(const uint8_t *packed, const float *absmax, const uint8
         return fail(NF4_ERR_INVALID_ARG, "nf4_embedding_gather: scale_codes without scale_of_scales");
     if ((d_model & 7u) == 0 && (!aligned16(out) || (reinterpret_cast<uintptr_t>(packed) & 3u)))
         return fail(NF4_ERR_INVALID_ARG, "nf4_embedding_gather: out must be 16-byte and packed 4-byte aligned");
-    const uint64_t work = (d_model & 7u) == 0 ? n_ids * (d_model / 8) : n_ids * d_model;
-    const int grid = grid_for(work, kThreads, 16);
-    if (out_bf16)
-        embedding_gather_kernel<true><<<grid, kThreads, 0, stream>>>(
-            packed, absmax, scale_codes, scale_of_scales, n_embedding, d_model, ids, n_ids, out);
-    else
-        embedding_gather_kernel<false><<<grid, kThreads, 0, stream>>>(
-            packed, absmax, scale_codes, scale_of_scales, n_embedding, d_model, ids, n_ids, out);
+    const uint64_t groups = d_model / 8, segments = (groups + 32 * kGatherGroups - 1) / (32 * kGatherGroups);
+    if ((d_model & 7u) == 0 && groups < (1ull << 31) && n_ids * segments < (1ull << 31)) {
+        const uint32_t work = (uint32_t)(n_ids * segments);
+        const unsigned grid = (work + kWarpsPerCta - 1) / kWarpsPerCta;
+        auto kernel = out_bf16 ? embedding_gather_kernel<true> : embedding_gather_kernel<false>;
+        NF4_TRY(launch_maybe_overlapped(kernel, dim3(grid), dim3(kThreads), 0, stream, true, packed, absmax, scale_codes,
+                                        scale_of_scales, n_embedding, (uint32_t)groups, ids, (uint32_t)segments, work, out,
+                                        aligned32(out)));
+    } else {
+        auto kernel = out_bf16 ? embedding_gather_elements_kernel<true> : embedding_gather_elements_kernel<false>;
+        kernel<<<grid_for(n_ids * d_model, kThreads, 16), kThreads, 0, stream>>>(packed, absmax, scale_codes, scale_of_scales,
+                                                                                n_embedding, d_model, ids, n_ids, out);
+    }
     count_launch();
     return check_cuda(cudaGetLastError(), "nf4_embedding_gather launch");
 }
@@ -560,17 +667,35 @@ int32_t embedding_gather(const uint8_t *packed, const float *absmax, const uint8
 int32_t double_quantize(const float *absmax, uint64_t nblocks, uint8_t *scale_codes,
                         float *scale_of_scales, cudaStream_t stream) {
     if (!scale_of_scales) return fail(NF4_ERR_INVALID_ARG, "nf4_double_quantize: null scale_of_scales");
-    NF4_CUDA_TRY(cudaMemsetAsync(scale_of_scales, 0, sizeof(float), stream));
-    if (nblocks == 0) return NF4_OK;
+    if (nblocks == 0) return check_cuda(cudaMemsetAsync(scale_of_scales, 0, sizeof(float), stream), "nf4_double_quantize");
     if (!absmax || !scale_codes)
         return fail(NF4_ERR_INVALID_ARG, "nf4_double_quantize: null pointer");
-    const int grid = grid_for(nblocks, kThreads * 4, 4);
-    scale_max_kernel<<<grid, kThreads, 0, stream>>>(absmax, nblocks,
-                                                    reinterpret_cast<uint32_t *>(scale_of_scales));
-    scale_encode_kernel<<<grid_for(nblocks, kThreads, 8), kThreads, 0, stream>>>(
-        absmax, nblocks, scale_of_scales, scale_codes);
+    const bool whole = aligned16(absmax) && (reinterpret_cast<uintptr_t>(scale_codes) & 3u) == 0;
+    if (aligned16(absmax) && nblocks <= kClusterMaxBlocks) {
+        NF4_TRY(allow_large_clusters(reinterpret_cast<const void *>(scale_max_cluster_kernel)));
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(kClusterCtas);
+        cfg.blockDim = dim3(kClusterThreads);
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = kClusterCtas;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
+        NF4_TRY(check_cuda(cudaLaunchKernelEx(&cfg, scale_max_cluster_kernel, reinterpret_cast<const float4 *>(absmax), absmax,
+                                              (uint32_t)nblocks, scale_of_scales), "nf4_double_quantize launch"));
+    } else {
+        NF4_CUDA_TRY(cudaMemsetAsync(scale_of_scales, 0, sizeof(float), stream));
+        scale_max_kernel<<<grid_for(nblocks, kThreads * 4, 4), kThreads, 0, stream>>>(
+            absmax, nblocks, reinterpret_cast<uint32_t *>(scale_of_scales));
+        NF4_CUDA_TRY(cudaGetLastError());
+    }
     count_launch(2);
-    return check_cuda(cudaGetLastError(), "nf4_double_quantize launch");
+    return launch_maybe_overlapped(scale_encode_kernel, dim3(grid_for(nblocks, kThreads * 4, 8)), dim3(kThreads), 0, stream, true,
+                                   absmax, nblocks, scale_of_scales, scale_codes, whole);
 }
 
 // ---- exhaustive self-check of the threshold bisection against the literal scan ----
@@ -595,20 +720,20 @@ selfcheck_codes_kernel(uint64_t first_bits, uint64_t count, unsigned long long *
 __global__ void __launch_bounds__(kThreads)
 selfcheck_fast_kernel(uint64_t first_bits, uint64_t count, float absmax,
                       unsigned long long *mismatches) {
-    __shared__ uint32_t s_cells[32];
-    if (threadIdx.x < 32) s_cells[threadIdx.x] = c_cell_table[threadIdx.x];
+    __shared__ uint32_t s_cells[kCellWords];
+    load_cells(s_cells);
     __syncthreads();
     const bool rcp_ok = absmax >= 1e-30f && absmax <= 1e30f;
-    const float rcp = __fdiv_rn(1.0f, absmax);
+    const float rcp = approx_rcp(absmax);
     unsigned long long bad = 0;
     const uint64_t stride = (uint64_t)gridDim.x * kThreads;
     for (uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x; i < count; i += stride) {
         const float x = __uint_as_float((uint32_t)(first_bits + i));
         if (fabsf(x) > absmax) continue;  // cannot occur inside a block whose absmax this is
         const uint32_t exact = absmax == 0.0f ? 7u : code_by_scan(__fdiv_rn(x, absmax));
-        bool unsure = !rcp_ok;
-        uint32_t got = code_of_fast(x, rcp, s_cells, unsure);
-        if (unsure) got = code_of_exact(x, absmax);
+        FastCodes f;
+        f.take(x, rcp * 2097152.0f, rcp * 64.0f, s_cells);
+        const uint32_t got = rcp_ok && f.sure() ? f.codes : code_of_exact(x, absmax);
         bad += got != exact;
     }
     if (bad) atomicAdd(mismatches, bad);
