@@ -119,6 +119,7 @@ struct Cfg {
 
 struct DecodeParams {
     const __nv_bfloat16 *x;
+    const float *absmax;   // read by the kernel where TMA does not bring the scales
     const uint8_t *scale_codes;
     const float *scale_of_scales;
     const float *bias;
@@ -207,15 +208,22 @@ __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t *p) {
     return v;
 }
 
+// How a launch gets its block scales.  d_in a multiple of 256 gives the scale rows a 16-byte pitch: f32
+// scales then come by TMA with the nibbles, u8 codes as one word per row and slice.  Other d_in (whole
+// blocks, but a pitch TMA does not take): lane t of a row's four lanes loads the scale of block t one
+// tile ahead and the four hand them round with shuffles.
+enum ScaleForm : int { kScalesTma = 0, kScalesU8Words = 1, kScalesF32 = 2, kScalesU8 = 3 };
+
 // One CTA's share of one forward.  `bid` of `nctas`: the CTA's number among the CTAs of this
 // forward (a launch can hold several forwards).  SPLIT: K is longer than a CTA's sixteen slices
 // and groups of CTAs multiply parts of it.  The descriptors and `p` are kernel parameters.
-template <int NT, bool DQ, bool SPLIT, bool PEERS = false>
+template <int NT, int SC, bool SPLIT, bool PEERS = false>
 __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const CUtensorMap *tm_scales,
                                             const DecodeParams &p, const uint32_t bid, const uint32_t nctas) {
     using C = Cfg;
     constexpr int kWarps = C::kWarps, kThreads = C::kThreads, SL = C::kSlices, kRing = C::kRing;
     constexpr int NC = SL * kSliceChunks;  // 64-blocks of K a warp owns
+    constexpr bool DQ = SC == kScalesU8Words || SC == kScalesU8, TMA_SCALES = SC == kScalesTma;
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     if (ptx::smem_addr(smem) != kWin0) {
@@ -225,7 +233,7 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
     }
     if (lane == 0) {  // the descriptors are on their way while the table is built
         ptx::prefetch_tmap(tm_codes);
-        if (!DQ) ptx::prefetch_tmap(tm_scales);
+        if (TMA_SCALES) ptx::prefetch_tmap(tm_scales);
     }
     float *red_s = reinterpret_cast<float *>(smem + C::kOffRed);
     float *t_s = reinterpret_cast<float *>(smem + C::kOffT);     // [SL][M][rank]
@@ -257,6 +265,9 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
     // parking place is zeroed once, so that the sums over the K-warps need not know)
     const uint32_t my_tiles = (nsl && rg < ntiles) ? (ntiles - rg + rw - 1) >> p.rw_shift : 0u;
     const uint32_t k0 = slice0 * kSliceK;
+    // blocks of this warp's slice that K still has (the last slice of a K that is no multiple of 256 is
+    // short: x reads as zero there, so whatever the table makes of the missing nibbles does not count)
+    const uint32_t have = p.nchunks > slice0 * kSliceChunks ? p.nchunks - slice0 * kSliceChunks : 0u;
 
     const uint32_t bar0 = kWin0 + C::kOffBars + warp * kRing * 8u;
     const uint32_t codes0 = kWin0 + C::kOffCodes + warp * kRing * C::kCodesTile;
@@ -271,10 +282,10 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
         const uint32_t slot = j & (kRing - 1);
         const int32_t row0 = (int32_t)(n0 + (rg + j * rw) * kTileRows);
         const uint32_t bar = bar0 + 8 * slot;
-        ptx::mbar_arrive_expect_tx(bar, DQ ? kCodesSlot : kCodesSlot + kScaleSlot);
+        ptx::mbar_arrive_expect_tx(bar, TMA_SCALES ? kCodesSlot + kScaleSlot : kCodesSlot);
         ptx::tma_load_2d(codes0 + slot * C::kCodesTile + sl * kCodesSlot, tm_codes,
                          (int32_t)((slice0 + sl) * 128u), row0, bar);
-        if (!DQ)
+        if (TMA_SCALES)
             ptx::tma_load_2d(scales0 + slot * C::kScaleTile + sl * kScaleSlot, tm_scales,
                              (int32_t)((slice0 + sl) * 4u), row0, bar);
     };
@@ -340,7 +351,7 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
         #pragma unroll
         for (int c = 0; c < kSliceChunks; ++c) {
             araw[c][0] = araw[c][1] = make_uint4(0, 0, 0, 0);
-            if (t_warp && h < nsl) {
+            if (t_warp && h < nsl && h * kSliceChunks + c < have) {
                 const uint4 *src = reinterpret_cast<const uint4 *>(
                     p.lora_a + (size_t)j * p.K + k0 + (h * kSliceChunks + c) * kChunk + 16 * t);
                 araw[c][0] = __ldg(src);
@@ -391,7 +402,7 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
         #pragma unroll
         for (int cc = 0; cc < 4; ++cc) {
             xr[cc][0] = xr[cc][1] = make_uint4(0, 0, 0, 0);
-            if (m < p.M && half < nsl) {
+            if (m < p.M && half < nsl && half * 4 + cc < have) {
                 const uint4 *src = reinterpret_cast<const uint4 *>(
                     p.x + (size_t)m * p.K + k0 + (half * 4 + cc) * kChunk + 16 * t);
                 // (x that other GPUs stored into while this kernel waited is read past the L1)
@@ -561,24 +572,27 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
     const uint32_t off_lo = (2 * g) * 128u + ((((t >> 1) ^ ((2 * g) & 7u))) << 4) + (t & 1u) * 8u;
     const uint32_t off_hi = (2 * g + 1) * 128u + ((((t >> 1) ^ ((2 * g + 1) & 7u))) << 4) + (t & 1u) * 8u;
 
-    // double-quantized scales come straight from global memory, one tile ahead
-    uint32_t dq_lo[SL], dq_hi[SL];
-    #pragma unroll
-    for (int sl = 0; sl < SL; ++sl) dq_lo[sl] = dq_hi[sl] = 0;
-    auto fetch_dq = [&](uint32_t j) {
-        if (DQ && j < my_tiles) {
-            const uint32_t row = n0 + (rg + j * rw) * kTileRows + 2 * g;
-            const uint32_t r_lo = min(row, p.N - 1), r_hi = min(row + 1, p.N - 1);
-            #pragma unroll
-            for (int sl = 0; sl < SL; ++sl) {
-                if ((uint32_t)sl < nsl) {
-                    dq_lo[sl] = __ldg(reinterpret_cast<const uint32_t *>(p.scale_codes + (size_t)r_lo * p.nchunks + (slice0 + sl) * 4u));
-                    dq_hi[sl] = __ldg(reinterpret_cast<const uint32_t *>(p.scale_codes + (size_t)r_hi * p.nchunks + (slice0 + sl) * 4u));
-                }
+    // scales that TMA does not bring come straight from global memory, one tile ahead
+    uint32_t sc_lo = 0, sc_hi = 0;  // of rows 2g and 2g + 1: a word of four codes, or block t's scale / code
+    static_assert(SL == 1, "one slice per warp");
+    auto fetch_scales = [&](uint32_t j) {
+        if (TMA_SCALES || j >= my_tiles) return;
+        const uint32_t row = n0 + (rg + j * rw) * kTileRows + 2 * g;
+        const size_t at_lo = (size_t)min(row, p.N - 1) * p.nchunks + slice0 * 4u, at_hi = (size_t)min(row + 1, p.N - 1) * p.nchunks + slice0 * 4u;
+        if (SC == kScalesU8Words) {
+            sc_lo = __ldg(reinterpret_cast<const uint32_t *>(p.scale_codes + at_lo));
+            sc_hi = __ldg(reinterpret_cast<const uint32_t *>(p.scale_codes + at_hi));
+        } else if (t < have) {
+            if (SC == kScalesF32) {
+                sc_lo = __float_as_uint(__ldg(p.absmax + at_lo + t));
+                sc_hi = __float_as_uint(__ldg(p.absmax + at_hi + t));
+            } else {
+                sc_lo = __ldg(p.scale_codes + at_lo + t);
+                sc_hi = __ldg(p.scale_codes + at_hi + t);
             }
         }
     };
-    fetch_dq(0);
+    fetch_scales(0);
 
     uint32_t use_j = 0;  // tiles consumed so far
 
@@ -613,11 +627,19 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
                         w1[c] = *reinterpret_cast<const uint2 *>(cs + (off_hi ^ ((uint32_t)c << 5)));
                     }
                     float s_lo[kSliceChunks], s_hi[kSliceChunks];
-                    if (DQ) {
+                    if (SC == kScalesU8Words) {
                         #pragma unroll
                         for (int c = 0; c < kSliceChunks; ++c) {
-                            s_lo[c] = __fmul_rn(dq_s[(dq_lo[sl] >> (8 * c)) & 0xffu], sos);
-                            s_hi[c] = __fmul_rn(dq_s[(dq_hi[sl] >> (8 * c)) & 0xffu], sos);
+                            s_lo[c] = __fmul_rn(dq_s[(sc_lo >> (8 * c)) & 0xffu], sos);
+                            s_hi[c] = __fmul_rn(dq_s[(sc_hi >> (8 * c)) & 0xffu], sos);
+                        }
+                    } else if (!TMA_SCALES) {
+                        const float lo = SC == kScalesF32 ? __uint_as_float(sc_lo) : __fmul_rn(dq_s[sc_lo], sos);
+                        const float hi = SC == kScalesF32 ? __uint_as_float(sc_hi) : __fmul_rn(dq_s[sc_hi], sos);
+                        #pragma unroll
+                        for (int c = 0; c < kSliceChunks; ++c) {
+                            s_lo[c] = __shfl_sync(0xffffffffu, lo, (lane & ~3u) | c);
+                            s_hi[c] = __shfl_sync(0xffffffffu, hi, (lane & ~3u) | c);
                         }
                     } else {
                         const uint8_t *ss = scales_ring + slot * C::kScaleTile + sl * kScaleSlot + g * 32u;
@@ -629,7 +651,7 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
                     if (sl + 1 == SL || (uint32_t)sl + 1 == nsl) {
                         // every lane holds the last of the tile in registers: refill the slot
                         ++use_j;
-                        fetch_dq(use_j);
+                        fetch_scales(use_j);
                         __syncwarp();
                         if (req_j < my_tiles) {
                             if (lane < nsl) request(req_j, lane);
@@ -840,11 +862,11 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
     }
 }
 
-template <int NT, bool DQ, bool SPLIT, bool PEERS>
+template <int NT, int SC, bool SPLIT, bool PEERS>
 __global__ void __launch_bounds__(Cfg::kThreads, 1)
 decode_kernel(const __grid_constant__ CUtensorMap tm_codes,
               const __grid_constant__ CUtensorMap tm_scales, const __grid_constant__ DecodeParams p) {
-    decode_body<NT, DQ, SPLIT, PEERS>(&tm_codes, &tm_scales, p, blockIdx.x, gridDim.x);
+    decode_body<NT, SC, SPLIT, PEERS>(&tm_codes, &tm_scales, p, blockIdx.x, gridDim.x);
 }
 
 // Waits (bounded) until `expected` CTAs of the ranks of a sharded layer have counted themselves in
@@ -877,12 +899,12 @@ struct GroupParams {
     uint32_t count;
 };
 
-template <int NT, bool DQ>
+template <int NT, int SC>
 __global__ void __launch_bounds__(Cfg::kThreads, 1)
 decode_group_kernel(const __grid_constant__ GroupParams gp) {
     uint32_t i = 0;
     while (i + 1 < gp.count && blockIdx.x >= gp.cta0[i + 1]) ++i;
-    decode_body<NT, DQ, false>(&gp.tm_codes[i], &gp.tm_scales[i], gp.p[i], blockIdx.x - gp.cta0[i],
+    decode_body<NT, SC, false>(&gp.tm_codes[i], &gp.tm_scales[i], gp.p[i], blockIdx.x - gp.cta0[i],
                                gp.cta0[i + 1] - gp.cta0[i]);
 }
 
@@ -963,6 +985,7 @@ int32_t make_map(CUtensorMap *map, CUtensorMapDataType dt, const void *base, uin
 struct Plan {
     DecodeParams p;
     uint32_t grid;
+    int scales;  // ScaleForm
 };
 
 // Fills the shape-dependent fields; false when the shape does not fit.
@@ -971,7 +994,7 @@ bool plan_shape(uint32_t M, uint32_t K, uint32_t N, uint32_t rank, uint32_t gran
     using C = Cfg;
     DecodeParams &p = pl.p;
     const uint32_t nt = M > 8 ? 2u : 1u;
-    p.kw = K / kSliceK;
+    p.kw = (K + kSliceK - 1) / kSliceK;
     p.kparts = (p.kw + kMaxSlices - 1) / kMaxSlices;
     p.part_slices = (p.kw + p.kparts - 1) / p.kparts;
     p.kwarps = (p.part_slices + C::kSlices - 1) / C::kSlices;
@@ -1020,15 +1043,17 @@ bool plan(const nf4_linear_args &a, Plan &pl, uint32_t max_ctas = 0) {
     if (max_ctas == 0) max_ctas = persistent_ctas();  // one CTA per SM, less what the host keeps free
     if (a.layout != NF4_LAYOUT_OUT_IN || a.io_dtype != NF4_DTYPE_BF16) return false;
     if (a.rows == 0 || a.rows > 16) return false;
-    // whole slices of four blocks: the scale rows then have a 16-byte pitch, which TMA needs
-    if (a.d_in % kSliceK != 0 || a.d_in > (uint64_t)kMaxParts * kMaxSlices * kSliceK) return false;
+    if (a.d_in % kChunk != 0 || a.d_in > (uint64_t)kMaxParts * kMaxSlices * kSliceK) return false;
     if (a.d_out >= (1ull << 31)) return false;
     const bool dq = a.scale_codes != nullptr;
     const uint32_t rank = a.lora_a ? a.lora_rank : 0;
     // LoRA-B rows move in a power-of-two number of 16-byte pieces
     if (rank != 0 && rank != 8 && rank != 16 && rank != 32 && rank != 64) return false;
-    const void *scales = dq ? (const void *)a.scale_codes : (const void *)a.absmax;
-    if (!aligned16(a.x) || !aligned16(a.packed) || !aligned16(scales)) return false;
+    if (!aligned16(a.x) || !aligned16(a.packed)) return false;
+    const bool whole_slices = a.d_in % kSliceK == 0;
+    if (dq) pl.scales = whole_slices && (reinterpret_cast<uintptr_t>(a.scale_codes) & 3u) == 0 ? kScalesU8Words : kScalesU8;
+    else pl.scales = whole_slices && aligned16(a.absmax) ? kScalesTma : kScalesF32;
+    if (reinterpret_cast<uintptr_t>(a.absmax) & 3u) return false;
     if (rank && (!aligned16(a.lora_a) || !aligned16(a.lora_b))) return false;
     if (reinterpret_cast<uintptr_t>(a.y) & (a.y_f32 ? 3u : 1u)) return false;
 
@@ -1042,6 +1067,7 @@ bool plan(const nf4_linear_args &a, Plan &pl, uint32_t max_ctas = 0) {
     if (!plan_shape(M, K, N, rank, gran, pl, max_ctas)) return false;
     p.wait_ns = 1000000000u;
     p.x = static_cast<const __nv_bfloat16 *>(a.x);
+    p.absmax = a.absmax;
     p.scale_codes = a.scale_codes;
     p.scale_of_scales = a.scale_of_scales;
     p.bias = a.bias;
@@ -1059,22 +1085,37 @@ bool plan(const nf4_linear_args &a, Plan &pl, uint32_t max_ctas = 0) {
     return true;
 }
 
-template <int NT, bool DQ, bool SPLIT, bool PEERS>
+template <int NT, int SC, bool SPLIT, bool PEERS>
 int32_t launch_as(const CUtensorMap &mc, const CUtensorMap &ms, const Plan &pl, cudaStream_t stream) {
     using C = Cfg;
-    NF4_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(decode_kernel<NT, DQ, SPLIT, PEERS>), (int)C::kSmemBytes));
+    NF4_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(decode_kernel<NT, SC, SPLIT, PEERS>), (int)C::kSmemBytes));
     count_launch();
-    return launch_maybe_overlapped(decode_kernel<NT, DQ, SPLIT, PEERS>, dim3(pl.grid), dim3(C::kThreads),
+    return launch_maybe_overlapped(decode_kernel<NT, SC, SPLIT, PEERS>, dim3(pl.grid), dim3(C::kThreads),
                                    C::kSmemBytes, stream, true, mc, ms, pl.p);
 }
 
-template <int NT, bool DQ>
+template <int NT, int SC>
 int32_t launch(const CUtensorMap &mc, const CUtensorMap &ms, const Plan &pl, cudaStream_t stream) {
-    if (pl.p.n_dest)
-        return pl.p.kparts > 1 ? launch_as<NT, DQ, true, true>(mc, ms, pl, stream)
-                               : launch_as<NT, DQ, false, true>(mc, ms, pl, stream);
-    return pl.p.kparts > 1 ? launch_as<NT, DQ, true, false>(mc, ms, pl, stream)
-                           : launch_as<NT, DQ, false, false>(mc, ms, pl, stream);
+    if (pl.p.n_dest) {
+        // (sharded layers: whole slices only, see decode_forward_scatter)
+        if constexpr (SC == kScalesTma || SC == kScalesU8Words)
+            return pl.p.kparts > 1 ? launch_as<NT, SC, true, true>(mc, ms, pl, stream)
+                                   : launch_as<NT, SC, false, true>(mc, ms, pl, stream);
+        else
+            return fail(NF4_ERR_UNSUPPORTED, "decode_forward_scatter: d_in must be a multiple of 256");
+    }
+    return pl.p.kparts > 1 ? launch_as<NT, SC, true, false>(mc, ms, pl, stream)
+                           : launch_as<NT, SC, false, false>(mc, ms, pl, stream);
+}
+
+template <int NT>
+int32_t launch_form(const CUtensorMap &mc, const CUtensorMap &ms, const Plan &pl, cudaStream_t stream) {
+    switch (pl.scales) {
+        case kScalesTma: return launch<NT, kScalesTma>(mc, ms, pl, stream);
+        case kScalesU8Words: return launch<NT, kScalesU8Words>(mc, ms, pl, stream);
+        case kScalesF32: return launch<NT, kScalesF32>(mc, ms, pl, stream);
+        default: return launch<NT, kScalesU8>(mc, ms, pl, stream);
+    }
 }
 
 // bytes of T in the workspace: a share per part of K (room for two where K is not split)
@@ -1086,7 +1127,6 @@ uint64_t t_bytes(uint64_t rows, uint32_t rank, uint32_t kparts) {
 // and, where K is split, for the parts' sums
 int32_t prepare(const nf4_linear_args &a, Plan &pl, void *scratch, CUtensorMap &mc, CUtensorMap &ms) {
     DecodeParams &p = pl.p;
-    const bool dq = a.scale_codes != nullptr;
     if (p.rank || p.kparts > 1 || p.signal || p.wait_on) {
         if (!scratch) return fail(NF4_ERR_INVALID_ARG, "decode_forward: this shape needs the workspace");
         p.flags = static_cast<uint32_t *>(scratch);
@@ -1095,7 +1135,7 @@ int32_t prepare(const nf4_linear_args &a, Plan &pl, void *scratch, CUtensorMap &
     }
     NF4_TRY(make_map(&mc, CU_TENSOR_MAP_DATA_TYPE_UINT8, a.packed, p.N, p.K / 2, p.K / 2, kTileRows, 128,
                      CU_TENSOR_MAP_SWIZZLE_128B));
-    if (dq) ms = mc;  // not used by the kernel
+    if (pl.scales != kScalesTma) ms = mc;  // not used by the kernel
     else
         NF4_TRY(make_map(&ms, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, a.absmax, p.N, p.nchunks,
                          (uint64_t)p.nchunks * 4, kTileRows, 4, CU_TENSOR_MAP_SWIZZLE_NONE));
@@ -1105,10 +1145,7 @@ int32_t prepare(const nf4_linear_args &a, Plan &pl, void *scratch, CUtensorMap &
 int32_t run(const nf4_linear_args &a, Plan &pl, void *scratch, cudaStream_t stream) {
     CUtensorMap mc, ms;
     NF4_TRY(prepare(a, pl, scratch, mc, ms));
-    const DecodeParams &p = pl.p;
-    const bool dq = a.scale_codes != nullptr;
-    if (p.M <= 8) return dq ? launch<1, true>(mc, ms, pl, stream) : launch<1, false>(mc, ms, pl, stream);
-    return dq ? launch<2, true>(mc, ms, pl, stream) : launch<2, false>(mc, ms, pl, stream);
+    return pl.p.M <= 8 ? launch_form<1>(mc, ms, pl, stream) : launch_form<2>(mc, ms, pl, stream);
 }
 
 }  // namespace
@@ -1120,9 +1157,9 @@ bool decode_supported(const nf4_linear_args &a) {
 
 uint64_t decode_workspace_bytes(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t lora_rank) {
     if (rows == 0 || rows > 16) return 0;
-    const uint64_t kw = d_in / kSliceK;
+    const uint64_t kw = (d_in + kSliceK - 1) / kSliceK;
     const uint32_t kparts = (uint32_t)((kw + kMaxSlices - 1) / kMaxSlices);
-    const bool split = d_in % kSliceK == 0 && kparts > 1 && kparts <= (uint32_t)kMaxParts;
+    const bool split = d_in % kChunk == 0 && kparts > 1 && kparts <= (uint32_t)kMaxParts;
     if (lora_rank == 0 && !split) return 0;
     uint64_t need = kFlagBytes + t_bytes(rows, lora_rank, split ? kparts : 1u);
     if (split) need += (uint64_t)kparts * rows * d_out * 4;  // the parts' sums
@@ -1139,13 +1176,23 @@ int32_t lora_t_small(const void *x, const void *a, uint32_t rows, uint32_t K, ui
                                    static_cast<const __nv_bfloat16 *>(a), K, rank, t_out);
 }
 
-template <int NT, bool DQ>
-int32_t launch_group(const GroupParams &gp, cudaStream_t stream) {
+template <int NT, int SC>
+int32_t launch_group_as(const GroupParams &gp, cudaStream_t stream) {
     using C = Cfg;
-    NF4_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(decode_group_kernel<NT, DQ>), (int)C::kSmemBytes));
+    NF4_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(decode_group_kernel<NT, SC>), (int)C::kSmemBytes));
     count_launch();
-    return launch_maybe_overlapped(decode_group_kernel<NT, DQ>, dim3(gp.cta0[gp.count]), dim3(C::kThreads),
+    return launch_maybe_overlapped(decode_group_kernel<NT, SC>, dim3(gp.cta0[gp.count]), dim3(C::kThreads),
                                    C::kSmemBytes, stream, true, gp);
+}
+
+template <int NT>
+int32_t launch_group(const GroupParams &gp, int scales, cudaStream_t stream) {
+    switch (scales) {
+        case kScalesTma: return launch_group_as<NT, kScalesTma>(gp, stream);
+        case kScalesU8Words: return launch_group_as<NT, kScalesU8Words>(gp, stream);
+        case kScalesF32: return launch_group_as<NT, kScalesF32>(gp, stream);
+        default: return launch_group_as<NT, kScalesU8>(gp, stream);
+    }
 }
 
 // Forwards that share x, rows, d_in and the scale form, as one launch; false (nothing launched,
@@ -1187,18 +1234,18 @@ int32_t decode_forward_grouped(const nf4_linear_args *a, uint32_t count, cudaStr
     }
     static thread_local GroupParams gp;
     gp.count = count;
+    int scales = 0;
     gp.cta0[0] = 0;
     for (uint32_t i = 0; i < count; ++i) {
         Plan pl;
-        if (!plan(a[i], pl, ctas[i])) return NF4_OK;
+        if (!plan(a[i], pl, ctas[i]) || (i && pl.scales != scales)) return NF4_OK;
+        scales = pl.scales;
         NF4_TRY(prepare(a[i], pl, a[i].workspace, gp.tm_codes[i], gp.tm_scales[i]));
         gp.p[i] = pl.p;
         gp.cta0[i + 1] = gp.cta0[i] + pl.grid;
     }
     *taken = true;
-    const bool dq = a[0].scale_codes != nullptr;
-    if (a[0].rows <= 8) return dq ? launch_group<1, true>(gp, stream) : launch_group<1, false>(gp, stream);
-    return dq ? launch_group<2, true>(gp, stream) : launch_group<2, false>(gp, stream);
+    return a[0].rows <= 8 ? launch_group<1>(gp, scales, stream) : launch_group<2>(gp, scales, stream);
 }
 
 // The forward of one rank's column shard, stored into every rank's output.  `dest`: the outputs
@@ -1207,7 +1254,7 @@ int32_t decode_forward_scatter(const nf4_linear_args &a, void *const *dest, uint
                                uint32_t rank, uint64_t ldy, bool signal, uint32_t *wait_on, uint32_t wait_expected,
                                cudaStream_t stream) {
     Plan pl;
-    if (world == 0 || world > 8 || rank >= world || !plan(a, pl))
+    if (world == 0 || world > 8 || rank >= world || a.d_in % kSliceK != 0 || !plan(a, pl))
         return fail(NF4_ERR_UNSUPPORTED, "decode_forward_scatter: decode shapes and up to eight ranks only");
     DecodeParams &p = pl.p;
     const size_t eb = a.y_f32 ? 4 : 2;
