@@ -156,41 +156,35 @@ __device__ __forceinline__ float block_scale(const float *__restrict__ absmax,
 // sector of output; four such groups are in flight per thread to cover the load latency.  The last
 // len % 8 values go element by element.
 template <bool PACKED>
-__global__ void __launch_bounds__(kThreads, 7)
-dequantize_full_kernel(const uint8_t *__restrict__ codes, uint64_t len,
+__global__ void __launch_bounds__(kThreads, 8)
+dequantize_full_kernel(const uint8_t *__restrict__ codes, uint32_t ngroups, uint32_t rest,
                        const float *__restrict__ absmax, const uint8_t *__restrict__ scale_codes,
                        const float *__restrict__ scale_of_scales, float *__restrict__ out, bool wide) {
-    constexpr int kInFlight = 4;
+    constexpr uint32_t kInFlight = 4;
     __shared__ float s_levels[16];
     if (threadIdx.x < 16) s_levels[threadIdx.x] = __uint_as_float(c_level_bits[threadIdx.x]);
     __syncthreads();
     ptx::pdl_wait();
     ptx::pdl_launch_dependents();
     const float sos = scale_of_scales ? __ldg(scale_of_scales) : 0.0f;
-    const uint64_t ngroups = len / 8;  // 8 values per group
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x < (len & 7u)) {
-        const uint64_t e = 8 * ngroups + threadIdx.x;
-        const uint32_t c = PACKED ? (uint32_t)codes[e >> 1] >> (4 * (e & 1u)) : codes[e];
-        out[e] = __fmul_rn(s_levels[c & 15u], block_scale(absmax, scale_codes, sos, e / kBlock));
-    }
-    const uint64_t stride = (uint64_t)gridDim.x * kThreads;
-    for (uint64_t g0 = (uint64_t)blockIdx.x * kThreads + threadIdx.x; g0 < ngroups; g0 += stride * kInFlight) {
+    const uint32_t stride = gridDim.x * kThreads;
+    for (uint32_t g0 = blockIdx.x * kThreads + threadIdx.x; g0 < ngroups; g0 += stride * kInFlight) {
         uint2 w[kInFlight];
         float s[kInFlight];
         #pragma unroll
-        for (int u = 0; u < kInFlight; ++u) {
-            const uint64_t g = g0 + u * stride;
-            const bool live = g < ngroups;
+        for (uint32_t u = 0; u < kInFlight; ++u) {
+            const uint32_t g = g0 + u * stride;
             w[u] = make_uint2(0u, 0u);
-            if (live) {
+            s[u] = 0.0f;
+            if (g < ngroups) {
                 if (PACKED) w[u].x = __ldcs(reinterpret_cast<const uint32_t *>(codes) + g);
                 else w[u] = __ldcs(reinterpret_cast<const uint2 *>(codes) + g);
+                s[u] = block_scale(absmax, scale_codes, sos, g >> 3);
             }
-            s[u] = live ? block_scale(absmax, scale_codes, sos, g >> 3) : 0.0f;
         }
         #pragma unroll
-        for (int u = 0; u < kInFlight; ++u) {
-            const uint64_t g = g0 + u * stride;
+        for (uint32_t u = 0; u < kInFlight; ++u) {
+            const uint32_t g = g0 + u * stride;
             if (g >= ngroups) continue;
             float v[8];
             #pragma unroll
@@ -198,8 +192,13 @@ dequantize_full_kernel(const uint8_t *__restrict__ codes, uint64_t len,
                 const uint32_t word = PACKED || i < 4 ? w[u].x : w[u].y;
                 v[i] = __fmul_rn(s_levels[(word >> ((PACKED ? 4 * i : 8 * (i & 3)))) & 15u], s[u]);
             }
-            st8_stream(out + 8 * g, v, wide);
+            st8_stream(out + 8 * (uint64_t)g, v, wide);
         }
+    }
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x < rest) {
+        const uint64_t e = 8 * (uint64_t)ngroups + threadIdx.x;
+        const uint32_t c = PACKED ? (uint32_t)codes[e >> 1] >> (4 * (e & 1u)) : codes[e];
+        out[e] = __fmul_rn(s_levels[c & 15u], block_scale(absmax, scale_codes, sos, e / kBlock));
     }
 }
 
@@ -566,9 +565,15 @@ int32_t dequantize_impl(const uint8_t *codes, uint64_t len, const float *absmax,
     if (scale_codes && !scale_of_scales)
         return fail(NF4_ERR_INVALID_ARG, "nf4_dequantize: scale_codes without scale_of_scales");
     if (aligned16(codes) && aligned16(out)) {
-        count_launch();
-        return launch_maybe_overlapped(dequantize_full_kernel<PACKED>, dim3(grid_for(len / 8, kThreads, 7)), dim3(kThreads), 0, stream,
-                                       true, codes, len, absmax, scale_codes, scale_of_scales, out, aligned32(out));
+        for (uint64_t b0 = 0; b0 * kBlock < len; b0 += kSliceBlocks) {  // (32-bit positions in the kernel)
+            const uint64_t left = len - b0 * kBlock, n = left < kSliceBlocks * kBlock ? left : kSliceBlocks * kBlock;
+            count_launch();
+            NF4_TRY(launch_maybe_overlapped(dequantize_full_kernel<PACKED>, dim3(grid_for(n / 8, kThreads, 8)), dim3(kThreads), 0,
+                                            stream, true, codes + b0 * (PACKED ? kBlock / 2 : kBlock), (uint32_t)(n / 8),
+                                            (uint32_t)(n % 8), absmax ? absmax + b0 : nullptr, scale_codes ? scale_codes + b0 : nullptr,
+                                            scale_of_scales, out + b0 * kBlock, aligned32(out)));
+        }
+        return NF4_OK;
     }
     dequantize_generic_kernel<PACKED><<<grid_for(len, kThreads, 8), kThreads, 0, stream>>>(codes, len, 0, absmax, scale_codes,
                                                                                          scale_of_scales, out);
