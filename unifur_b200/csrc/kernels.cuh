@@ -111,6 +111,11 @@ int32_t decode2_forward(const nf4_linear_args &a, cudaStream_t stream);
 uint64_t generic_workspace_bytes(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t lora_rank);
 int32_t generic_forward(const nf4_linear_args &a, cudaStream_t stream);
 
+// in_out_strips.cu: NF4_LAYOUT_IN_OUT at few rows (sixteen per launch), d_out a multiple of 64, f32 arithmetic
+bool strips_supported(const nf4_linear_args &a);
+uint64_t strips_workspace_bytes(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t lora_rank);
+int32_t strips_forward(const nf4_linear_args &a, cudaStream_t stream);
+
 // f32_rows.cu: f32 tensors, NF4_LAYOUT_OUT_IN, rows <= 16: rows split into bf16 halves for the decode kernels
 bool f32_rows_supported(const nf4_linear_args &a);
 uint64_t f32_rows_workspace_bytes(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t lora_rank);

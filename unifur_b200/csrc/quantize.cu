@@ -18,6 +18,11 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kWarpsPerCta = kThreads / 32;
 
+// End of a kernel that writes weights.  The forward kernels ask for weights before they wait for the
+// kernel ahead of them (programmatic launches), so these kernels let their successor start no sooner
+// than their CTAs end, with what they wrote visible by then.
+__device__ __forceinline__ void publish_weight() { __threadfence(); }
+
 // Copies the cell table of the fast code selection into shared memory (a barrier must follow).
 __device__ __forceinline__ void load_cells(uint32_t *cells) {
     if (threadIdx.x < kCellWords) cells[threadIdx.x] = c_cell_table[threadIdx.x];
@@ -103,7 +108,6 @@ quantize_full_kernel(const float *__restrict__ values, uint32_t ngroups, uint32_
     load_cells(s_cells);
     __syncthreads();
     ptx::pdl_wait();
-    ptx::pdl_launch_dependents();
     // groups of eight values; eight neighbouring lanes hold a block, so a block's lanes are in range together
     const uint32_t step = gridDim.x * kThreads;
     uint32_t g = blockIdx.x * kThreads + threadIdx.x;
@@ -128,6 +132,7 @@ quantize_full_kernel(const float *__restrict__ values, uint32_t ngroups, uint32_
     if (rest && blockIdx.x == gridDim.x - 1 && threadIdx.x < 32)
         quantize_block_by_warp<PACKED>(values + 8 * (uint64_t)ngroups, rest, codes + (PACKED ? 4 : 8) * (uint64_t)ngroups,
                                        absmax + ngroups / 8);
+    publish_weight();
 }
 
 // Buffers that are not 16-byte aligned: a warp per block.
@@ -248,7 +253,6 @@ quantize_transposed_kernel(const uint32_t *__restrict__ src, uint32_t segments, 
     load_cells(s_cells);
     __syncthreads();
     ptx::pdl_wait();
-    ptx::pdl_launch_dependents();
     const uint32_t tile = blockIdx.x / segments, seg = blockIdx.x - tile * segments;
     const uint32_t lane = threadIdx.x & 31u, part = lane / kSplitWords;  // which 32 rows
     const uint32_t word = tile * kTWords + (threadIdx.x >> 5) * kSplitWords + lane % kSplitWords;
@@ -291,6 +295,7 @@ quantize_transposed_kernel(const uint32_t *__restrict__ src, uint32_t segments, 
         }
         if (part == 0) absmax[blk] = m;
     }
+    publish_weight();
 }
 static_assert(kSplitRows == 32, "a lane stores four words of codes per block");
 
@@ -509,7 +514,6 @@ __global__ void __launch_bounds__(kThreads)
 scale_encode_kernel(const float *__restrict__ absmax, uint64_t nblocks,
                     const float *max_scale_ptr, uint8_t *__restrict__ scale_codes, bool whole) {
     ptx::pdl_wait();
-    ptx::pdl_launch_dependents();
     const float max_scale = *max_scale_ptr;
     const uint64_t stride = (uint64_t)gridDim.x * kThreads, first = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
     const uint64_t n4 = whole ? nblocks / 4 : 0;
@@ -518,6 +522,7 @@ scale_encode_kernel(const float *__restrict__ absmax, uint64_t nblocks,
         reinterpret_cast<uint32_t *>(scale_codes)[i] = enc.four(__ldg(reinterpret_cast<const float4 *>(absmax) + i));
     for (uint64_t i = 4 * n4 + first; i < nblocks; i += stride)
         scale_codes[i] = (uint8_t)scale_code_exact(__ldg(absmax + i), max_scale);
+    publish_weight();
 }
 
 inline bool aligned32(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 31u) == 0; }
