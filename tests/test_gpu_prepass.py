@@ -1,0 +1,71 @@
+"""The pre-pass of the tensor-core path and the adapter gradients: pieces of K over a cluster, ragged rows and ranks."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+from gpu_util import DEV  # noqa: E402
+from unifur_b200 import _lib  # noqa: E402
+
+
+def layer(M, K, N, r, layout, dt, seed, x_std=1.0):
+    from unifur_b200.quantize import PackedNf4Tensor
+    from unifur_b200.qwennet import Nf4Linear, QloraLinear
+
+    gen = torch.Generator(device=DEV).manual_seed(seed)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=gen)  # noqa: E731
+    out_in = layout == _lib.LAYOUT_OUT_IN
+    a, b = ((r, K), (N, r)) if out_in else ((K, r), (r, N))
+    base = Nf4Linear(PackedNf4Tensor.quantize(rnd(K * N) * 0.02), K, N, None, layout)
+    q = QloraLinear(base, (rnd(*a) * 0.1).to(dt), (rnd(*b) * 0.1).to(dt), 1.5)
+    w = base.dequantized_weight().double()
+    w = w.t() if out_in else w                                       # [K, N]
+    A, B = q.lora_a.double(), q.lora_b.double()
+    A, B = (A.t(), B.t()) if out_in else (A, B)                      # [K, r], [r, N]
+    x = rnd(M, K) * x_std
+    x = x * torch.logspace(-12, 12, M, base=2.0, device=DEV)[:, None]  # rows far apart in magnitude
+    return q, w, A, B, x.to(dt), rnd
+
+
+def rel(got, ref):
+    return float((got.double() - ref).norm() / ref.norm())
+
+
+@pytest.mark.parametrize("M,K,N,r,layout,f32", [
+    (17, 64, 64, 8, 0, False),         # one stage of K, one CTA
+    (33, 320, 128, 16, 0, False),      # K pieces of unequal length, one row in the second tile
+    (100, 4096, 256, 64, 0, False),    # sixteen CTAs per tile
+    (300, 2112, 192, 72, 0, False),    # more than 64 ranks
+    (64, 704, 320, 24, 1, False),      # the factor [K, r] through transposing loads
+    (40, 1024, 128, 12, 0, True),      # f32: converted in place
+    (70, 4160, 64, 4, 1, True),
+    (20, 65536, 64, 8, 0, False),      # K in several pieces of shared memory
+    (18, 40960, 64, 8, 0, True),
+])
+def test_forward(M, K, N, r, layout, f32):
+    dt = torch.float32 if f32 else torch.bfloat16
+    q, w, A, B, x, _ = layer(M, K, N, r, layout, dt, M + K + N)
+    y = q.forward(x)
+    ref = x.double() @ w + 1.5 * (x.double() @ A) @ B
+    per_row = ((y.double() - ref).norm(dim=1) / ref.norm(dim=1)).max()
+    assert float(per_row) < (1e-3 if f32 else 4e-3)
+
+
+@pytest.mark.parametrize("M,K,N,r,layout", [
+    (1, 64, 128, 8, 0), (5, 200, 136, 5, 1), (16, 1024, 512, 16, 0),   # decode sizes: both intermediates by the product-only mode
+    (63, 256, 384, 16, 1), (513, 640, 200, 80, 0), (2049, 576, 1344, 64, 1),   # shares of the rows, ragged pieces of columns
+    (1100, 128, 32000, 8, 0),                                          # more pieces of columns than counters
+])
+def test_backward(M, K, N, r, layout):
+    q, w, A, B, x, rnd = layer(M, K, N, r, layout, torch.bfloat16, M + K + N)
+    x = torch.randn(M, K, device=DEV).bfloat16()
+    gy = (rnd(M, N) * 1e-3).bfloat16()
+    gx, ga, gb = q.backward(x, gy)
+    again = q.backward(x, gy)
+    assert all(torch.equal(u, v) for u, v in zip((gx, ga, gb), again))
+    X, G = x.double(), gy.double()
+    gA, gB = 1.5 * X.t() @ (G @ B.t()), 1.5 * (X @ A).t() @ G
+    gA, gB = (gA.t(), gB.t()) if layout == _lib.LAYOUT_OUT_IN else (gA, gB)
+    assert rel(gx, G @ w.t() + 1.5 * (G @ B.t()) @ A.t()) < 4e-3
+    assert rel(ga, gA) < 3e-3 and rel(gb, gB) < 3e-3

@@ -1,0 +1,259 @@
+// The adapter's gradients for bf16 tensors on warp MMAs:
+//   grad_A(k, j) = s sum_m x[m][k] U[m][j],   grad_B(j, n) = s sum_m T[m][j] grad_y[m][n],
+// T = x A, U = grad_y B^T from the pre-pass kernel as bf16 high and low halves (their f32 values survive:
+// two MMAs per tile).
+//
+// gradient_kernel: out(p, j) = s sum_m X[m][p] R[m][j] as D[p][j] += A[p][m] B[m][j] (m16n8k16).  A CTA takes
+// 128 columns p, 64 ranks and a share of the rows; 64 rows of X and R per stage come by 16-byte
+// asynchronous copies, three stages in flight, and both operands are transposing matrix loads of what lies
+// there.  Eight warps: four pieces of 32 columns, two halves of a stage's rows.  Rows are shared out so that
+// two CTAs run on every SM; the shares meet in the workspace, where the CTA that arrives last for a
+// piece of columns adds them in order.  Bound by reading X once: grad_B of 2048 rows x 14336 columns took
+// 96 us and grad_A of 4096 columns 64 with one CTA per 64 columns walking all rows through a
+// register transpose, without overlap.
+#include <cuda_bf16.h>
+
+#include "kernels.cuh"
+#include "ptx.cuh"
+
+namespace nf4 {
+namespace {
+
+constexpr uint32_t kThreads = 256, kCols = 128, kRowsStage = 64, kStages = 3;
+constexpr uint32_t kPitch = 272;                           // 256 bytes of a row and 16 of padding
+constexpr uint32_t kXStage = kRowsStage * kPitch, kStage = 2 * kXStage;
+constexpr uint32_t kSumPitch = 68;                         // floats
+constexpr uint32_t kCounterTiles = 248;                    // byte counters the flag words hold
+static_assert(kCols * kSumPitch * 4 <= kStages * kStage, "the sums reuse the stages");
+
+struct Params {
+    const __nv_bfloat16 *x, *r;   // [rows][P]; [rows][2 * 64 * chunks]: hi halves, then lo
+    __nv_bfloat16 *out;
+    float *partial;               // [chunk][share][tile][128][64]
+    uint32_t *counters;
+    uint32_t rows, P, rank, chunks, shares, stages_per_share, p_major;
+    float scale;
+};
+
+__global__ void __launch_bounds__(kThreads, 2) gradient_kernel(const Params p) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    __shared__ uint32_t last_s;
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    const uint32_t g = lane >> 2, t = lane & 3u, li = lane >> 3, lr = lane & 7u;
+    const uint32_t pw = warp & 3u, h = warp >> 2;
+    const uint32_t tile = blockIdx.x, share = blockIdx.y, p0 = tile * kCols;
+    const uint32_t st0 = share * p.stages_per_share;
+    const uint32_t all = (p.rows + kRowsStage - 1) / kRowsStage;
+    const uint32_t nst = st0 < all ? min(p.stages_per_share, all - st0) : 0u;
+    const uint32_t base = ptx::smem_addr(smem), ld_r = 128 * p.chunks;
+    float *sum = reinterpret_cast<float *>(smem);
+    ptx::pdl_launch_dependents();
+    ptx::pdl_wait();
+    for (uint32_t chunk = 0; chunk < p.chunks; ++chunk) {
+        const uint32_t ranks = min(64u, p.rank - chunk * 64), tiles16 = (ranks + 15) / 16;
+        auto load = [&](uint32_t st) {
+            if (st < nst) {
+                const uint32_t m0 = (st0 + st) * kRowsStage, dst = base + (st % kStages) * kStage;
+                #pragma unroll
+                for (uint32_t q = 0; q < 4; ++q) {  // X: 64 rows x 16 pieces of eight columns
+                    const uint32_t i = tid + q * kThreads, r = i >> 4, c = i & 15u;
+                    const bool real = m0 + r < p.rows && p0 + c * 8 < p.P;
+                    ptx::cp_async_16_or_zero(dst + r * kPitch + c * 16, p.x + (real ? (size_t)(m0 + r) * p.P + p0 + c * 8 : 0), real);
+                }
+                #pragma unroll
+                for (uint32_t q = 0; q < 4; ++q) {  // R: 64 rows x (8 pieces of hi, 8 of lo)
+                    const uint32_t i = tid + q * kThreads, r = i >> 4, c = i & 15u;
+                    if ((c & 7u) >= 2 * tiles16) continue;
+                    const bool real = m0 + r < p.rows;
+                    const size_t at = (size_t)(m0 + r) * ld_r + (c >> 3) * 64 * p.chunks + chunk * 64 + (c & 7u) * 8;
+                    ptx::cp_async_16_or_zero(dst + kXStage + r * kPitch + c * 16, p.r + (real ? at : 0), real);
+                }
+            }
+            ptx::cp_async_commit();
+        };
+        float acc[2][8][4];
+        #pragma unroll
+        for (int a = 0; a < 2; ++a)
+            #pragma unroll
+            for (int u = 0; u < 8; ++u) acc[a][u][0] = acc[a][u][1] = acc[a][u][2] = acc[a][u][3] = 0.0f;
+        load(0);
+        load(1);
+        for (uint32_t st = 0; st < nst; ++st) {
+            ptx::cp_async_wait<1>();
+            __syncthreads();
+            load(st + 2);
+            const uint32_t xs = base + (st % kStages) * kStage, rs = xs + kXStage;
+            #pragma unroll
+            for (uint32_t k2 = 0; k2 < 2; ++k2) {
+                const uint32_t m = (2 * h + k2) * 16;
+                uint32_t af[2][4];
+                #pragma unroll
+                for (int a = 0; a < 2; ++a)
+                    ptx::ldmatrix_x4_trans(af[a], xs + (m + (li >> 1) * 8 + lr) * kPitch + (pw * 32 + a * 16 + (li & 1u) * 8) * 2);
+                const uint32_t b_at = rs + (m + (li & 1u) * 8 + lr) * kPitch + (li >> 1) * 16;
+                #pragma unroll
+                for (uint32_t u = 0; u < 4; ++u) {
+                    if (u >= tiles16) break;
+                    #pragma unroll
+                    for (uint32_t half = 0; half < 2; ++half) {  // hi, then lo
+                        uint32_t bf[4];
+                        ptx::ldmatrix_x4_trans(bf, b_at + half * 128 + u * 32);
+                        #pragma unroll
+                        for (int a = 0; a < 2; ++a) {
+                            ptx::mma_16816_bf16(acc[a][2 * u], af[a][0], af[a][1], af[a][2], af[a][3], bf[0], bf[1]);
+                            ptx::mma_16816_bf16(acc[a][2 * u + 1], af[a][0], af[a][1], af[a][2], af[a][3], bf[2], bf[3]);
+                        }
+                    }
+                }
+            }
+        }
+        ptx::cp_async_wait<0>();
+        // the two halves of the rows, in order
+        for (uint32_t turn = 0; turn < 2; ++turn) {
+            __syncthreads();
+            if (h == turn) {
+                #pragma unroll
+                for (int a = 0; a < 2; ++a)
+                    #pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        float2 *lo = reinterpret_cast<float2 *>(sum + (pw * 32 + a * 16 + g) * kSumPitch + u * 8 + 2 * t);
+                        float2 *hi = reinterpret_cast<float2 *>(sum + (pw * 32 + a * 16 + g + 8) * kSumPitch + u * 8 + 2 * t);
+                        const float2 l = turn ? *lo : make_float2(0.0f, 0.0f), hh = turn ? *hi : make_float2(0.0f, 0.0f);
+                        *lo = make_float2(l.x + acc[a][u][0], l.y + acc[a][u][1]);
+                        *hi = make_float2(hh.x + acc[a][u][2], hh.y + acc[a][u][3]);
+                    }
+            }
+        }
+        __syncthreads();
+        if (p.shares > 1) {
+            float4 *mine = reinterpret_cast<float4 *>(p.partial) +
+                           (((size_t)chunk * p.shares + share) * gridDim.x + tile) * (kCols * 16);
+            for (uint32_t i = tid; i < kCols * 16; i += kThreads)
+                if ((i & 15u) < 4 * tiles16)
+                    __stcg(mine + i, *reinterpret_cast<const float4 *>(sum + (i >> 4) * kSumPitch + (i & 15u) * 4));
+            __syncthreads();
+            if (tid == 0) {
+                __threadfence();
+                const uint32_t sh = (tile & 3u) * 8u;
+                const uint32_t old = (atomicAdd(p.counters + (tile >> 2), 1u << sh) >> sh) & 0xffu;
+                if (old == p.shares - 1) atomicSub(p.counters + (tile >> 2), p.shares << sh);
+                last_s = old == p.shares - 1;
+            }
+            __syncthreads();
+            if (!last_s) continue;
+            __threadfence();
+            for (uint32_t i = tid; i < kCols * 16; i += kThreads) {
+                if ((i & 15u) >= 4 * tiles16) continue;
+                float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                #pragma unroll 4
+                for (uint32_t q = 0; q < p.shares; ++q) {
+                    const float4 o = __ldcg(reinterpret_cast<const float4 *>(p.partial) +
+                                            (((size_t)chunk * p.shares + q) * gridDim.x + tile) * (kCols * 16) + i);
+                    v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
+                }
+                *reinterpret_cast<float4 *>(sum + (i >> 4) * kSumPitch + (i & 15u) * 4) = v;
+            }
+            __syncthreads();
+        }
+        for (uint32_t i = tid; i < kCols * 64; i += kThreads) {
+            // p fastest for [rank][P] outputs, j fastest for [P][rank]
+            const uint32_t q = p.p_major ? i >> 6 : i & (kCols - 1), j = p.p_major ? i & 63u : i >> 7;
+            const uint32_t pp = p0 + q, jj = chunk * 64 + j;
+            if (pp < p.P && j < ranks)
+                p.out[p.p_major ? (size_t)pp * p.rank + jj : (size_t)jj * p.P + pp] = __float2bfloat16_rn(__fmul_rn(sum[q * kSumPitch + j], p.scale));
+        }
+        __syncthreads();  // (before the next chunk's stages)
+    }
+}
+
+uint32_t chunks_of(uint32_t rank) { return (rank + 63) / 64; }
+uint64_t up256(uint64_t v) { return (v + 255) / 256 * 256; }
+uint64_t intermediate_bytes(uint64_t rows, uint32_t rank) { return up256(rows * 2 * 64 * chunks_of(rank) * 2); }
+uint64_t tiles_of(uint64_t P) { return (P + kCols - 1) / kCols; }
+// Shares of the rows: two CTAs on every SM where a share keeps four stages (256 rows); one where the
+// pieces of columns alone fill the SMs, or are more than there are counters.
+uint64_t shares_of(uint64_t rows, uint64_t P) {
+    const uint64_t tiles = tiles_of(P);
+    if (tiles > kCounterTiles) return 1;
+    uint64_t shares = 2 * kNumSMs / tiles;
+    const uint64_t most = (rows + 4 * kRowsStage - 1) / (4 * kRowsStage);
+    if (shares > most) shares = most;
+    if (shares > 64) shares = 64;
+    return shares ? shares : 1;
+}
+uint64_t partial_bytes(uint64_t rows, uint64_t P, uint32_t rank) {
+    const uint64_t shares = shares_of(rows, P);
+    return shares > 1 ? shares * tiles_of(P) * kCols * 64 * 4 * chunks_of(rank) : 0;
+}
+
+int32_t gradient(const void *x, const void *r, void *out, uint64_t rows, uint64_t P, uint32_t rank, float scale, bool p_major,
+                 void *partial, uint32_t *counters, cudaStream_t s) {
+    Params p{};
+    p.x = static_cast<const __nv_bfloat16 *>(x);
+    p.r = static_cast<const __nv_bfloat16 *>(r);
+    p.out = static_cast<__nv_bfloat16 *>(out);
+    p.partial = static_cast<float *>(partial);
+    p.counters = counters;
+    p.rows = (uint32_t)rows;
+    p.P = (uint32_t)P;
+    p.rank = rank;
+    p.chunks = chunks_of(rank);
+    p.shares = (uint32_t)shares_of(rows, P);
+    const uint32_t all = (uint32_t)((rows + kRowsStage - 1) / kRowsStage);
+    p.stages_per_share = (all + p.shares - 1) / p.shares;
+    p.p_major = p_major;
+    p.scale = scale;
+    NF4_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(gradient_kernel), (int)(kStages * kStage)));
+    count_launch();
+    return launch_maybe_overlapped(gradient_kernel, dim3((unsigned)tiles_of(P), p.shares), dim3(kThreads), kStages * kStage, s, true, p);
+}
+
+}  // namespace
+
+bool adapter_grads_supported(const void *x, const void *gy, const void *a, const void *b, uint64_t rows, uint64_t d_in,
+                             uint64_t d_out, uint32_t rank) {
+    return d_in % 8 == 0 && d_out % 8 == 0 && rows < (1ull << 31) && d_in < (1ull << 31) && d_out < (1ull << 31) && rank <= 4096 &&
+           aligned16(x) && aligned16(gy) && (reinterpret_cast<uintptr_t>(a) & 1u) == 0 && (reinterpret_cast<uintptr_t>(b) & 1u) == 0;
+}
+
+// T | U | partial sums
+uint64_t adapter_grads_bytes(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t rank) {
+    if (!rank) return 0;
+    const uint64_t pa = partial_bytes(rows, d_in, rank), pb = partial_bytes(rows, d_out, rank);
+    return 2 * intermediate_bytes(rows, rank) + (pa > pb ? pa : pb);
+}
+
+void *adapter_grads_u(void *scratch, uint64_t rows, uint32_t rank) {
+    return static_cast<uint8_t *>(scratch) + intermediate_bytes(rows, rank);
+}
+
+int32_t adapter_grads(const void *x, const void *gy, const void *a, const void *b, uint64_t rows, uint64_t d_in,
+                      uint64_t d_out, uint32_t rank, float scale, int32_t layout, void *ga, void *gb, void *scratch,
+                      uint32_t *counters, bool u_ready, cudaStream_t s) {
+    const bool in_out = layout == NF4_LAYOUT_IN_OUT;
+    void *t = scratch, *u = adapter_grads_u(scratch, rows, rank);
+    void *partial = static_cast<uint8_t *>(u) + intermediate_bytes(rows, rank);
+    PrepassArgs q{};
+    q.M = (uint32_t)rows;
+    q.rank = rank;
+    if (!u_ready) {  // U = grad_y B^T, B [d_out][r] or [r][d_out]
+        q.x = gy;
+        q.K = (uint32_t)d_out;
+        q.a = b;
+        q.k_major = !in_out;
+        q.r_out = u;
+        NF4_TRY(activations_prepass(q, s));
+    }
+    q.x = x;             // T = x A, A [r][d_in] or [d_in][r]
+    q.K = (uint32_t)d_in;
+    q.a = a;
+    q.k_major = in_out;
+    q.r_out = t;
+    q.flags = counters;  // (zero by the workspace's contract; a host that clears them only for decode sizes need not care)
+    q.n_flags = kCounterTiles / 4;
+    NF4_TRY(activations_prepass(q, s));
+    NF4_TRY(gradient(x, u, ga, rows, d_in, rank, scale, in_out, partial, counters, s));
+    return gradient(gy, t, gb, rows, d_out, rank, scale, !in_out, partial, counters, s);
+}
+
+}  // namespace nf4

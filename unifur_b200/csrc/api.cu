@@ -453,25 +453,25 @@ uint64_t nf4_linear_workspace_bytes(uint64_t rows, uint64_t d_in, uint64_t d_out
     return need;
 }
 
-int32_t nf4_linear_forward_dev(const nf4_linear_args *args, void *stream) {
+// The kernel for a forward's shape.  *r_out (r_out may be null): where the adapter intermediate x A is wanted
+// beside the output; null afterwards if the kernel taken does not give it.
+static int32_t linear_forward(const nf4_linear_args *args, cudaStream_t s, void **r_out) {
     NF4_TRY(validate_linear(args));
     if (args->rows == 0) return NF4_OK;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    // rows <= 16: the warp-MMA kernel (d_in <= 4096, whole 256-slices), else the tcgen05 split-K
-    // kernel; more rows: the tcgen05 GEMM; whatever none of them takes: the CUDA-core kernel.
-    if (decode_supported(*args)) {
-        return decode_forward(*args, s);
-    }
-    if (decode2_supported(*args)) {
-        return decode2_forward(*args, s);
-    }
-    if (prefill_supported(*args) || prefill_in_out_supported(*args)) {
-        return prefill_forward(*args, s);
-    }
-    if (f32_rows_supported(*args)) {
-        return f32_rows_forward(*args, s);
-    }
+    // rows <= 16: the warp-MMA kernel (whole 64-blocks of d_in), else the tcgen05 split-K kernel; more
+    // rows: the tcgen05 GEMM; whatever none of them takes: the CUDA-core kernels.
+    const bool decode = decode_supported(*args);
+    if (!decode && !decode2_supported(*args) && (prefill_supported(*args) || prefill_in_out_supported(*args)))
+        return prefill_forward(*args, s, r_out ? *r_out : nullptr);
+    if (r_out) *r_out = nullptr;
+    if (decode) return decode_forward(*args, s);
+    if (decode2_supported(*args)) return decode2_forward(*args, s);
+    if (f32_rows_supported(*args)) return f32_rows_forward(*args, s);
     return generic_forward(*args, s);
+}
+
+int32_t nf4_linear_forward_dev(const nf4_linear_args *args, void *stream) {
+    return linear_forward(args, static_cast<cudaStream_t>(stream), nullptr);
 }
 
 // SMs the decode kernel leaves alone (see nf4_reserve_sms)
@@ -628,12 +628,12 @@ int32_t nf4_qlora_merge_dev(const uint8_t *packed, const float *absmax, const ui
 
 // ---- backward of the QLoRA linear (base weight frozen) -----------------------------------------
 
+// grad_x is a forward with d_in and d_out exchanged; then two [rows][rank] f32 intermediates, or what the
+// tensor-core gradients need
 uint64_t nf4_qlora_backward_workspace_bytes(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t lora_rank) {
-    // grad_x is a forward with d_in and d_out exchanged; then two [rows][rank] f32 intermediates
-    // ... and one adapter factor transposed (bf16)
-    const uint64_t widest = d_in > d_out ? d_in : d_out;
-    return nf4_linear_workspace_bytes(rows, d_out, d_in, lora_rank) + 2 * lora_workspace_bytes(rows, lora_rank) +
-           align_up((uint64_t)lora_rank * widest * 2, 256);
+    const uint64_t plain = 2 * lora_workspace_bytes(rows, lora_rank) + align_up((uint64_t)lora_rank * (d_in > d_out ? d_in : d_out) * 2, 256);
+    const uint64_t mma = adapter_grads_bytes(rows, d_in, d_out, lora_rank);
+    return nf4_linear_workspace_bytes(rows, d_out, d_in, lora_rank) + (plain > mma ? plain : mma);
 }
 
 int32_t nf4_qlora_backward_dev(const nf4_linear_args *fwd, const void *grad_y, void *grad_x, void *grad_a,
@@ -665,15 +665,20 @@ int32_t nf4_qlora_backward_dev(const nf4_linear_args *fwd, const void *grad_y, v
     g.lora_b = fwd->lora_a;
     const uint64_t fw = nf4_linear_workspace_bytes(fwd->rows, fwd->d_out, fwd->d_in, r);
     g.workspace_bytes = fw;
-    NF4_TRY(nf4_linear_forward_dev(&g, stream));
-    if (!r) return NF4_OK;
     uint8_t *ws = static_cast<uint8_t *>(fwd->workspace) + fw;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const bool mma = r && fwd->io_dtype == NF4_DTYPE_BF16 &&
+                     adapter_grads_supported(fwd->x, grad_y, fwd->lora_a, fwd->lora_b, fwd->rows, fwd->d_in, fwd->d_out, r);
+    void *u_out = mma ? adapter_grads_u(ws, fwd->rows, r) : nullptr;
+    NF4_TRY(linear_forward(&g, s, &u_out));
+    if (!r) return NF4_OK;
+    if (mma)
+        return adapter_grads(fwd->x, grad_y, fwd->lora_a, fwd->lora_b, fwd->rows, fwd->d_in, fwd->d_out, r, fwd->lora_scale,
+                             fwd->layout, grad_a, grad_b, ws, static_cast<uint32_t *>(fwd->workspace), u_out != nullptr, s);
     float *t = reinterpret_cast<float *>(ws);
     float *u = reinterpret_cast<float *>(ws + lora_workspace_bytes(fwd->rows, r));
-    void *factor_t = ws + 2 * lora_workspace_bytes(fwd->rows, r);
     return lora_grads(fwd->x, grad_y, fwd->lora_a, fwd->lora_b, fwd->rows, fwd->d_in, fwd->d_out, r,
-                      fwd->lora_scale, fwd->layout, fwd->io_dtype, grad_a, grad_b, t, u, factor_t,
-                      static_cast<cudaStream_t>(stream));
+                      fwd->lora_scale, fwd->layout, fwd->io_dtype, grad_a, grad_b, t, u, s);
 }
 
 // ---- column-sharded forward ------------------------------------------------------------------

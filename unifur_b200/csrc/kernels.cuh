@@ -38,7 +38,18 @@ int32_t lora_delta(const void *a, const void *b, const uint8_t *packed, const fl
                    uint32_t rank, float scale, int32_t layout, int32_t io_dtype, float *out, cudaStream_t s);
 int32_t lora_grads(const void *x, const void *gy, const void *a, const void *b, uint64_t rows, uint64_t d_in,
                    uint64_t d_out, uint32_t rank, float scale, int32_t layout, int32_t io_dtype, void *ga,
-                   void *gb, float *t, float *u, void *scratch, cudaStream_t s);
+                   void *gb, float *t, float *u, cudaStream_t s);
+
+// adapter_grads.cu: the same for bf16 tensors on warp MMAs.  `scratch` (256-byte aligned) holds R = x a and
+// grad_y b in the pre-pass's form and partial sums; `counters`: flag words, zero, left zero; u_ready:
+// adapter_grads_u(scratch, ...) already holds grad_y b (the pre-pass of grad_x left it there).
+bool adapter_grads_supported(const void *x, const void *gy, const void *a, const void *b, uint64_t rows, uint64_t d_in,
+                             uint64_t d_out, uint32_t rank);
+uint64_t adapter_grads_bytes(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t rank);
+void *adapter_grads_u(void *scratch, uint64_t rows, uint32_t rank);
+int32_t adapter_grads(const void *x, const void *gy, const void *a, const void *b, uint64_t rows, uint64_t d_in,
+                      uint64_t d_out, uint32_t rank, float scale, int32_t layout, void *ga, void *gb, void *scratch,
+                      uint32_t *counters, bool u_ready, cudaStream_t s);
 int32_t push_columns(void *const *y_full, uint32_t *const *arrive, uint32_t world, uint32_t rank, uint64_t rows,
                      uint64_t width_bytes, uint64_t ldy_bytes, bool signal, uint32_t *done, cudaStream_t s);
 int32_t gather_slabs(const void *slab, void *gathered, void *y, uint64_t rows, uint64_t width_bytes,
@@ -128,9 +139,33 @@ bool prefill_in_out_supported(const nf4_linear_args &a);
 uint64_t prefill_workspace_bytes(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t lora_rank);
 int32_t prefill_share_plan(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t cta, uint32_t *ctas,
                            uint32_t *segments, uint32_t cap);
-int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream);
-// t32[m][j] = sum_k x[m][k] F(k, j), bf16 operands on warp MMAs; NF4_ERR_UNSUPPORTED (no message) for shapes it declines
-int32_t adapter_intermediate_bf16(const void *x, const void *f, bool k_major, uint64_t rows, uint64_t k, uint32_t rank,
-                                  float *t32, void *scratch, cudaStream_t stream);
+// r_out: null, or where x A goes too (see PrepassArgs)
+int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_out = nullptr);
+
+// prepass.cu: the f16 copy of the activations with its rows' factors, and the adapter intermediate.
+// x [M][K] bf16 or f32 (K a multiple of 8, 16-byte aligned); a: the factor as [rank][K], or [K][rank]
+// (k_major), bf16, f16 for f32 x.  xh null: r_out alone (bf16 x).  t_out and r_out: [M][2 * 64 * ceil(rank / 64)]
+// bf16, hi halves then lo; t_out the scaled intermediate the GEMM adds, r_out (may be null) x a as it is.
+// beside_predecessor: the kernel ahead in the stream touches nothing that this one reads or writes; they may
+// run side by side, and this one completes after it.
+struct PrepassArgs {
+    const void *x;
+    bool x_f32;
+    uint32_t M, K;
+    const void *a;
+    uint32_t rank;
+    bool k_major;
+    float scale;
+    void *xh;
+    float *row_scale;
+    void *t_out, *r_out;
+    const float *absmax;
+    const uint8_t *scale_codes;
+    const float *scale_of_scales;
+    uint32_t *flags;
+    uint32_t n_flags;
+    bool beside_predecessor;
+};
+int32_t activations_prepass(const PrepassArgs &q, cudaStream_t stream);
 
 }  // namespace nf4

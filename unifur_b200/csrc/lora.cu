@@ -231,94 +231,6 @@ lora_xtr_tile_kernel(const T *__restrict__ x, const float *__restrict__ r, T *__
     }
 }
 
-// The same gradients for bf16 tensors on warp MMAs: out(p, j) = scale * sum_m X[m][p] R[m][j] as
-// D[p][j] += A[p][m] B[m][j] with m16n8k16.  A CTA takes 64 columns p and up to 64 ranks; pieces of
-// 64 rows m pass through shared memory transposed (X as it is; R split into bf16 high and low parts,
-// so that its f32 value survives: two MMAs per tile), which makes every fragment one 32-bit load;
-// warp w takes the 16 columns (w & 3) and the two k-steps (w >> 2) of a piece; the two halves meet
-// in a fixed order.  P must be even (pairs of columns are read as words).
-__global__ void __launch_bounds__(256)
-lora_xtr_mma_kernel(const __nv_bfloat16 *__restrict__ x, const float *__restrict__ r, __nv_bfloat16 *__restrict__ out,
-                    uint64_t rows, uint64_t P, uint32_t rank, float scale, int p_major) {
-    constexpr int kP = 64, kJ = 64, kM = 64, kS = 72;  // kS: halves per transposed row (fragment loads hit 32 banks)
-    __shared__ __align__(16) uint16_t xs_t[kP][kS];
-    __shared__ __align__(16) uint16_t rh[kJ][kS], rl[kJ][kS];
-    __shared__ float sum[kP][kJ + 1];
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, g = lane >> 2, t = lane & 3u;
-    const uint32_t pt = warp & 3u, h = warp >> 2;
-    const uint64_t p0 = (uint64_t)blockIdx.x * kP;
-    const uint32_t lo = threadIdx.x & 31u, hi = threadIdx.x >> 5;  // staging: 8 columns x 4 rows per warp and step
-    for (uint32_t j0 = 0; j0 < rank; j0 += kJ) {
-        float acc[8][4];
-        #pragma unroll
-        for (int jt = 0; jt < 8; ++jt) acc[jt][0] = acc[jt][1] = acc[jt][2] = acc[jt][3] = 0.0f;
-        for (uint64_t m0 = 0; m0 < rows; m0 += kM) {
-            __syncthreads();
-            #pragma unroll
-            for (int it = 0; it < 8; ++it) {   // X: 64 rows x 32 pairs of columns
-                const uint32_t hh = hi + 8 * it;  // 0 .. 63
-                const uint32_t pair = (lo & 7u) + 8 * (hh & 3u), m = (lo >> 3) + 4 * (hh >> 2);
-                uint32_t v = 0;
-                if (m0 + m < rows && p0 + 2 * pair < P)
-                    v = __ldg(reinterpret_cast<const uint32_t *>(x + (m0 + m) * P + p0 + 2 * pair));
-                xs_t[2 * pair][m] = (uint16_t)(v & 0xffffu);
-                xs_t[2 * pair + 1][m] = (uint16_t)(v >> 16);
-            }
-            #pragma unroll
-            for (int it = 0; it < 16; ++it) {  // R: 64 rows x 64 ranks
-                const uint32_t hh = hi + 8 * it;  // 0 .. 127
-                const uint32_t j = (lo & 7u) + 8 * (hh & 7u), m = (lo >> 3) + 4 * (hh >> 3);
-                float v = 0.0f;
-                if (m0 + m < rows && j0 + j < rank) v = __ldg(r + (m0 + m) * rank + j0 + j);
-                const __nv_bfloat16 vh = __float2bfloat16_rn(v);
-                const __nv_bfloat16 vl = __float2bfloat16_rn(v - __bfloat162float(vh));
-                rh[j][m] = __bfloat16_as_ushort(vh);
-                rl[j][m] = __bfloat16_as_ushort(vl);
-            }
-            __syncthreads();
-            #pragma unroll
-            for (int ks2 = 0; ks2 < 2; ++ks2) {
-                const uint32_t mb = (2 * h + ks2) * 16 + 2 * t;
-                const uint32_t a0 = *reinterpret_cast<const uint32_t *>(&xs_t[pt * 16 + g][mb]);
-                const uint32_t a1 = *reinterpret_cast<const uint32_t *>(&xs_t[pt * 16 + g + 8][mb]);
-                const uint32_t a2 = *reinterpret_cast<const uint32_t *>(&xs_t[pt * 16 + g][mb + 8]);
-                const uint32_t a3 = *reinterpret_cast<const uint32_t *>(&xs_t[pt * 16 + g + 8][mb + 8]);
-                #pragma unroll
-                for (int jt = 0; jt < 8; ++jt) {
-                    const uint32_t bh0 = *reinterpret_cast<const uint32_t *>(&rh[jt * 8 + g][mb]);
-                    const uint32_t bh1 = *reinterpret_cast<const uint32_t *>(&rh[jt * 8 + g][mb + 8]);
-                    const uint32_t bl0 = *reinterpret_cast<const uint32_t *>(&rl[jt * 8 + g][mb]);
-                    const uint32_t bl1 = *reinterpret_cast<const uint32_t *>(&rl[jt * 8 + g][mb + 8]);
-                    ptx::mma_16816_bf16(acc[jt], a0, a1, a2, a3, bh0, bh1);
-                    ptx::mma_16816_bf16(acc[jt], a0, a1, a2, a3, bl0, bl1);
-                }
-            }
-        }
-        // the two halves of the rows, in order
-        for (uint32_t turn = 0; turn < 2; ++turn) {
-            __syncthreads();
-            if (h == turn) {
-                #pragma unroll
-                for (int jt = 0; jt < 8; ++jt) {
-                    float *s0 = &sum[pt * 16 + g][jt * 8 + 2 * t], *s1 = &sum[pt * 16 + g + 8][jt * 8 + 2 * t];
-                    s0[0] = turn ? s0[0] + acc[jt][0] : acc[jt][0];
-                    s0[1] = turn ? s0[1] + acc[jt][1] : acc[jt][1];
-                    s1[0] = turn ? s1[0] + acc[jt][2] : acc[jt][2];
-                    s1[1] = turn ? s1[1] + acc[jt][3] : acc[jt][3];
-                }
-            }
-        }
-        __syncthreads();
-        for (uint32_t i = threadIdx.x; i < kP * kJ; i += 256) {
-            // p fastest for [rank][P] outputs, j fastest for [P][rank]
-            const uint32_t q = p_major ? i / kJ : i % kP, j = p_major ? i % kJ : i / kP;
-            const uint64_t pp = p0 + q;
-            if (pp < P && j0 + j < rank)
-                out[p_major ? pp * rank + j0 + j : (uint64_t)(j0 + j) * P + pp] = __float2bfloat16_rn(__fmul_rn(sum[q][j], scale));
-        }
-    }
-}
-
 // y[r][rank * width + c] = gathered[rank][r][c]: the ranks' slabs side by side.  16-byte pieces.
 __global__ void __launch_bounds__(256)
 place_slabs_kernel(const uint4 *__restrict__ gathered, uint4 *__restrict__ y, uint64_t rows, uint64_t pieces_per_row,
@@ -391,35 +303,20 @@ int32_t forward_t(const void *x, uint64_t rows, uint64_t d_in, uint64_t d_out, c
 template <class T>
 int32_t grads_t(const void *x, const void *gy, const void *a, const void *b, uint64_t rows, uint64_t d_in,
                 uint64_t d_out, uint32_t rank, float scale, int32_t layout, void *ga, void *gb, float *t,
-                float *u, void *scratch, cudaStream_t s) {
+                float *u, cudaStream_t s) {
     const T *xx = static_cast<const T *>(x), *gg = static_cast<const T *>(gy);
-    // T = x A (as in the forward) and U = grad_y B^T (B read as an "A" of the other orientation).
-    // bf16: on warp MMAs (products of bf16 values are exact in f32, so the sums differ from the
-    // CUDA-core kernels' only in their order); shapes that path declines, and f32, on CUDA cores.
+    // T = x A (as in the forward) and U = grad_y B^T (B read as an "A" of the other orientation)
     const int32_t other = layout == NF4_LAYOUT_OUT_IN ? NF4_LAYOUT_IN_OUT : NF4_LAYOUT_OUT_IN;
-    bool t_done = false, u_done = false;
-    if (sizeof(T) == 2) {
-        int32_t rc = adapter_intermediate_bf16(x, a, layout == NF4_LAYOUT_IN_OUT, rows, d_in, rank, t, scratch, s);
-        if (rc == NF4_OK) t_done = true;
-        else if (rc != NF4_ERR_UNSUPPORTED) return rc;
-        rc = adapter_intermediate_bf16(gy, b, other == NF4_LAYOUT_IN_OUT, rows, d_out, rank, u, scratch, s);
-        if (rc == NF4_OK) u_done = true;
-        else if (rc != NF4_ERR_UNSUPPORTED) return rc;
-    }
-    if (!t_done) launch_xa<T>(xx, static_cast<const T *>(a), t, rows, d_in, rank, layout, s);
-    if (!u_done) launch_xa<T>(gg, static_cast<const T *>(b), u, rows, d_out, rank, other, s);
+    launch_xa<T>(xx, static_cast<const T *>(a), t, rows, d_in, rank, layout, s);
+    launch_xa<T>(gg, static_cast<const T *>(b), u, rows, d_out, rank, other, s);
     // grad_A(k, j) = s sum_m x[m][k] U[m][j];  grad_B(j, n) = s sum_m T[m][j] grad_y[m][n]
     NF4_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(lora_xtr_tile_kernel<T>), (int)xtr_smem_bytes<T>()));
-    auto xtr = [&](const void *X, const float *R, void *out, uint64_t P, int p_major) {
-        if (sizeof(T) == 2 && P % 2 == 0 && (reinterpret_cast<uintptr_t>(X) & 3u) == 0)
-            lora_xtr_mma_kernel<<<(unsigned)((P + 63) / 64), 256, 0, s>>>(
-                static_cast<const __nv_bfloat16 *>(X), R, static_cast<__nv_bfloat16 *>(out), rows, P, rank, scale, p_major);
-        else
-            lora_xtr_tile_kernel<T><<<(unsigned)((P + kXtrP - 1) / kXtrP), 256, xtr_smem_bytes<T>(), s>>>(
-                static_cast<const T *>(X), R, static_cast<T *>(out), rows, P, rank, scale, p_major);
+    auto xtr = [&](const T *X, const float *R, void *out, uint64_t P, int p_major) {
+        lora_xtr_tile_kernel<T><<<(unsigned)((P + kXtrP - 1) / kXtrP), 256, xtr_smem_bytes<T>(), s>>>(
+            X, R, static_cast<T *>(out), rows, P, rank, scale, p_major);
     };
-    xtr(x, u, ga, d_in, layout == NF4_LAYOUT_IN_OUT);
-    xtr(gy, t, gb, d_out, layout == NF4_LAYOUT_OUT_IN);
+    xtr(xx, u, ga, d_in, layout == NF4_LAYOUT_IN_OUT);
+    xtr(gg, t, gb, d_out, layout == NF4_LAYOUT_OUT_IN);
     count_launch(4);
     return check_cuda(cudaGetLastError(), "lora gradient launch");
 }
@@ -496,16 +393,15 @@ int32_t lora_delta(const void *a, const void *b, const uint8_t *packed, const fl
     return check_cuda(cudaGetLastError(), "lora delta launch");
 }
 
-// grad_A and grad_B of y = x W + s (x A) B with W frozen; t and u are [rows][rank] f32 scratch,
-// `scratch` rank * max(d_in, d_out) * 2 bytes (a factor transposed; used one product at a time).
+// grad_A and grad_B of y = x W + s (x A) B with W frozen, on CUDA cores; t and u are [rows][rank] f32 scratch
 int32_t lora_grads(const void *x, const void *gy, const void *a, const void *b, uint64_t rows, uint64_t d_in,
                    uint64_t d_out, uint32_t rank, float scale, int32_t layout, int32_t io_dtype, void *ga,
-                   void *gb, float *t, float *u, void *scratch, cudaStream_t s) {
+                   void *gb, float *t, float *u, cudaStream_t s) {
     if (rows * rank >= (1ull << 40) || (d_in + d_out) * rank >= (1ull << 40))
         return fail(NF4_ERR_UNSUPPORTED, "lora gradients: shape too large");
     return io_dtype == NF4_DTYPE_F32
-               ? grads_t<float>(x, gy, a, b, rows, d_in, d_out, rank, scale, layout, ga, gb, t, u, scratch, s)
-               : grads_t<__nv_bfloat16>(x, gy, a, b, rows, d_in, d_out, rank, scale, layout, ga, gb, t, u, scratch, s);
+               ? grads_t<float>(x, gy, a, b, rows, d_in, d_out, rank, scale, layout, ga, gb, t, u, s)
+               : grads_t<__nv_bfloat16>(x, gy, a, b, rows, d_in, d_out, rank, scale, layout, ga, gb, t, u, s);
 }
 
 // All-gather of the ranks' [rows, width_bytes] slabs into `gathered` ([world][rows][width_bytes]),

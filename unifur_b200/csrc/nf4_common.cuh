@@ -157,6 +157,20 @@ __device__ __forceinline__ float dq_scale(uint32_t code, float scale_of_scales) 
     return __fmul_rn(__fdiv_rn((float)code, 255.0f), scale_of_scales);
 }
 
+// The tensor-core GEMM scales the expanded levels in f16, so block scales must sit inside f16's
+// normal range (6.1e-5 .. 65504).  It and its pre-pass therefore work with scales divided by 2^e, e the
+// exponent of the weight's first block scale (the scales of one weight lie within a few powers of
+// two of each other), and the outputs are multiplied back by 2^e: the pre-pass folds 2^e into the
+// rows' factors and 2^-e into the adapter intermediate.  Powers of two: every step is exact.
+__device__ __forceinline__ int weight_exponent(const float *absmax, const uint8_t *scale_codes,
+                                               const float *scale_of_scales) {
+    const float s0 = absmax ? __ldg(absmax) : dq_scale(__ldg(scale_codes), __ldg(scale_of_scales));
+    if (!(s0 > 0.0f) || s0 >= __int_as_float(0x7f800000)) return 0;
+    int e;
+    frexpf(s0, &e);  // s0 = f * 2^e, f in [0.5, 1)
+    return min(max(e, -100), 100);
+}
+
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 }  // namespace nf4

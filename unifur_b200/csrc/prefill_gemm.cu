@@ -286,23 +286,9 @@ __device__ __forceinline__ void expand_half_per_k(const LevelTables &t, const ui
 }
 
 struct RowStage {
-    uint4 c0, c1;  // the row's 64 packed codes of one k-stage
-    float scale;   // PERK: the bits of this lane's pair of f16 scales
+    uint4 c0, c1;    // the row's 64 packed codes of one k-stage
+    uint32_t scale;  // its scale as loaded: f32 bits, a u8 code, or (PERK) this lane's pair of f16 scales
 };
-
-// The tensor-core GEMM scales the expanded levels in f16, so block scales must sit inside f16's
-// normal range (6.1e-5 .. 65504).  Both kernels therefore work with scales divided by 2^e, e the
-// exponent of the weight's first block scale (the scales of one weight lie within a few powers of
-// two of each other), and the outputs are multiplied back by 2^e: the pre-pass folds 2^e into the
-// rows' factors and 2^-e into the adapter intermediate.  Powers of two: every step is exact.
-__device__ __forceinline__ int weight_exponent(const float *absmax, const uint8_t *scale_codes,
-                                               const float *scale_of_scales) {
-    const float s0 = absmax ? __ldg(absmax) : dq_scale(__ldg(scale_codes), __ldg(scale_of_scales));
-    if (!(s0 > 0.0f) || s0 >= __int_as_float(0x7f800000)) return 0;
-    int e;
-    frexpf(s0, &e);  // s0 = f * 2^e, f in [0.5, 1)
-    return min(max(e, -100), 100);
-}
 
 template <bool YF32, bool PERK>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -650,10 +636,13 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         const uint32_t group = (warp - kFirstExpanderWarp) >> 2;
         const uint32_t q = warp & 3u;
         const uint32_t row_in_tile = q * 32 + lane;
+        if (PERK) ptx::pdl_wait();  // the weight is repacked by a kernel that completes before the pre-pass does
         const LevelTables tables = make_level_tables();
-        const float sos = p.scale_codes ? __ldg(p.scale_of_scales) : 0.0f;
         // block scales are used divided by a power of two (see weight_exponent)
+        // ... and enter the product as f16: one multiplication from the loaded value.  (A u8 code's scale is
+        // (code / 255) * scale of scales; dividing once instead of per code moves it by an ulp of f32.)
         const float w_down = ldexpf(1.0f, -weight_exponent(p.absmax, p.scale_codes, p.scale_of_scales));
+        const float scale_unit = p.absmax ? w_down : __fdiv_rn(__ldg(p.scale_of_scales), 255.0f) * w_down;
         const uint32_t blocks_per_row = p.K / 64;
         const uint32_t total = (uint32_t)(wl.u1 - wl.u0) + p.dp_rounds * k_stages;  // main stages of this CTA
         const uint32_t lane_base = tmem_a + ((q * 32) << 16);
@@ -687,7 +676,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         };
         auto fetch = [&](const Pos &pos, RowStage &rs) {
             rs.c0 = rs.c1 = make_uint4(0, 0, 0, 0);
-            rs.scale = 0.0f;
+            rs.scale = 0;
             if (pos.cnt >= total) return;
             const uint32_t ks = pos.ks, n = pos.n;
             if (n >= p.N) return;
@@ -700,10 +689,13 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 // line of scales for the stage, a pair per lane
                 const uint32_t *line = reinterpret_cast<const uint32_t *>(
                     p.scales_t + (size_t)((n - lane) >> 6) * p.K + (size_t)ks * BK);
-                rs.scale = __uint_as_float(__ldg(line + lane));
+                rs.scale = __ldg(line + lane);
             } else {
+                // nothing is computed from the loaded value here: that would wait for the load, the
+                // latency the pipeline is there to hide (half of a dequantiser's time at few rows)
                 const size_t blk = (size_t)n * blocks_per_row + ks;
-                rs.scale = (p.absmax ? __ldg(p.absmax + blk) : dq_scale(__ldg(p.scale_codes + blk), sos)) * w_down;
+                if (p.absmax) rs.scale = __float_as_uint(__ldg(p.absmax + blk));
+                else rs.scale = __ldg(p.scale_codes + blk);
             }
         };
         auto emit = [&](const Pos &pos, const RowStage &rs) -> bool {
@@ -712,11 +704,12 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             const uint32_t dst = lane_base + s * kAStageCols;
             uint32_t lo[16], hi[16];
             if constexpr (PERK) {
-                expand_half_per_k(tables, rs.c0, __float_as_uint(rs.scale), 0, lo);
-                expand_half_per_k(tables, rs.c1, __float_as_uint(rs.scale), 16, hi);
+                expand_half_per_k(tables, rs.c0, rs.scale, 0, lo);
+                expand_half_per_k(tables, rs.c1, rs.scale, 16, hi);
             } else {
-                expand_half(tables, rs.c0, rs.scale, lo);
-                expand_half(tables, rs.c1, rs.scale, hi);
+                const float scale = (p.absmax ? __uint_as_float(rs.scale) : (float)rs.scale) * scale_unit;
+                expand_half(tables, rs.c0, scale, lo);
+                expand_half(tables, rs.c1, scale, hi);
             }
             if (!ptx::mbar_wait_suspended(bar(kBarAEmpty + s), ph ^ 1u)) return false;
             ptx::tc_fence_after();
@@ -766,211 +759,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     }
 }
 
-// ---- pre-pass: f16 activations, row scales and the LoRA intermediate ---------------------
-// One CTA per 16 rows of x, sixteen warps splitting K.  x is read once:
-//   1. xh[m][k] = f16(x[m][k]) is written at once (exact inside f16's range) while the row
-//      maxima are collected; row_scale[m] = 1, or the power of two that brings a row whose
-//      largest magnitude exceeds 32768 or lies below 2^-8 to [16384, 32768), in which case that
-//      row is converted again as f16(x / row_scale) at the end (rare).
-//   2. with an adapter: T = lora_scale * (x A^T) / row_scale, written as bf16 hi / lo halves:
-//      T[m][c] for c < 64*chunks holds bf16(T), T[m][64*chunks + c] holds bf16(T - bf16(T));
-//      columns beyond the rank are zero.  The same registers of x feed warp MMAs against A.
-// k is walked in 32-wide pieces; inside a piece thread t owns k = 8t .. 8t+7 so that both
-// operands are read with 16-byte loads (a consistent permutation of k on A and B).  The loads
-// of the next piece are in flight while a piece is multiplied.
-constexpr int kTThreads = 512;
-constexpr int kTWarps = kTThreads / 32;
-constexpr int kTPartStride = 72;  // floats per row of a warp's partial sums (64 + padding against bank conflicts)
-constexpr int kTPartBytes = kTWarps * 16 * kTPartStride * 4;
-
-struct PrepassPiece {
-    uint4 xa, xb;   // rows g and g + 8 of the slab
-    uint4 bv[8];    // rows 8u + g of this 64-rank chunk of A
-};
-
-// Running maxima of |bf16|, a pair at a time; a NaN leaves the maximum as it is (max.bf16x2
-// returns the other operand).
-__device__ __forceinline__ uint32_t bf16x2_absmax(uint32_t w, uint32_t mx) {
-    uint32_t d;
-    asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(w & 0x7fff7fffu), "r"(mx));
-    return d;
-}
-// The larger half of such a pair as an f32 pattern; 0 if only NaNs were seen.
-__device__ __forceinline__ uint32_t bf16x2_larger_bits(uint32_t mx) {
-    const uint32_t lo = mx << 16, hi = mx & 0xffff0000u;
-    const uint32_t a = lo <= 0x7f800000u ? lo : 0u, b = hi <= 0x7f800000u ? hi : 0u;
-    return max(a, b);
-}
-
-__device__ __forceinline__ uint4 bf16x8_to_f16x8(const uint4 &v, float is) {
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-    uint32_t o[4];
-    #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const __half2 h = __floats2half2_rn(__uint_as_float(w[q] << 16) * is,
-                                            __uint_as_float(w[q] & 0xffff0000u) * is);
-        o[q] = *reinterpret_cast<const uint32_t *>(&h);
-    }
-    return make_uint4(o[0], o[1], o[2], o[3]);
-}
-
-// MODE 1 (XH_READY): the activations arrive as the f16 copy itself (made, with the row scales, by
-// x_f32_to_f16_row) and the adapter factor as f16: only T is computed, with f16 MMAs.
-// MODE 2 (T_ONLY): the product alone, t32[m][j] = sum_k x[m][k] a[j][k] in f32, for callers outside
-// the GEMM (the adapter's gradients): no copy of x, no scales.
-template <int MODE>
-__global__ void __launch_bounds__(kTThreads)
-prefill_prepass_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ a,
-                       uint32_t M, uint32_t K, uint32_t rank, uint32_t chunks, float scale,
-                       __half *__restrict__ xh, float *__restrict__ row_scale,
-                       __nv_bfloat16 *__restrict__ t_out, const float *__restrict__ absmax,
-                       const uint8_t *__restrict__ scale_codes, const float *__restrict__ scale_of_scales,
-                       uint32_t *__restrict__ sk_flags, uint32_t n_flags, float *__restrict__ t32) {
-    constexpr bool XH_READY = MODE == 1, T_ONLY = MODE == 2;
-    // the warps' partial sums of T: [warp][16 rows][64 ranks, padded to 72], summed in warp order
-    extern __shared__ __align__(16) float part[];
-    __shared__ uint32_t row_max_bits[16];
-    __shared__ float inv_scale[16];
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const uint32_t g = lane >> 2, t = lane & 3u;
-    const uint32_t m0 = blockIdx.x * 16;
-    const uint32_t rows = min(16u, M - m0);
-    ptx::pdl_launch_dependents();  // the GEMM may set itself up and start on the weights
-    // the GEMM's CTAs raise these once this kernel has completed (their readers and writers wait for that)
-    if (blockIdx.x == 0)
-        for (uint32_t i = threadIdx.x; i < n_flags; i += kTThreads) sk_flags[i] = 0;
-    const int w_exp = T_ONLY ? 0 : weight_exponent(absmax, scale_codes, scale_of_scales);
-    const float w_up = ldexpf(1.0f, w_exp), w_down = ldexpf(1.0f, -w_exp);
-    const bool row_a = g < rows, row_b = g + 8 < rows;
-    const uint32_t pieces = (K + 31) / 32, n_it = (pieces + kTWarps - 1) / kTWarps;
-    const size_t off_a = (size_t)(m0 + g) * K, off_b = (size_t)(m0 + g + 8) * K;
-
-    if (threadIdx.x < 16) row_max_bits[threadIdx.x] = 0;
-    __syncthreads();
-    uint32_t mx_a = 0, mx_b = 0;
-
-    const uint32_t passes = chunks ? chunks : 1u;
-    for (uint32_t chunk = 0; chunk < passes; ++chunk) {
-        float acc[8][4];
-        #pragma unroll
-        for (int u = 0; u < 8; ++u) acc[u][0] = acc[u][1] = acc[u][2] = acc[u][3] = 0.0f;
-
-        // piece `it` of this warp starts at k = (warp + 16 it) * 32; this thread's 8 values at + 8t
-        auto k_of = [&](uint32_t it) { return (warp + kTWarps * it) * 32 + 8 * t; };
-        auto load = [&](PrepassPiece &pc, uint32_t it) {
-            const uint32_t k = k_of(it);
-            const bool in = it < n_it && k + 8 <= K && (!XH_READY || rank != 0);
-            pc.xa = pc.xb = make_uint4(0, 0, 0, 0);
-            if (in && row_a) pc.xa = __ldg(reinterpret_cast<const uint4 *>(x + off_a + k));
-            if (in && row_b) pc.xb = __ldg(reinterpret_cast<const uint4 *>(x + off_b + k));
-            #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const uint32_t j = chunk * 64 + 8 * u + g;
-                pc.bv[u] = make_uint4(0, 0, 0, 0);
-                if (in && j < rank) pc.bv[u] = __ldg(reinterpret_cast<const uint4 *>(a + (size_t)j * K + k));
-            }
-        };
-        auto process = [&](const PrepassPiece &pc, uint32_t it) {
-            const uint32_t k = k_of(it);
-            if (MODE == 0 && chunk == 0 && it < n_it && k + 8 <= K) {
-                if (row_a) {
-                    mx_a = bf16x2_absmax(pc.xa.x, bf16x2_absmax(pc.xa.y, mx_a));
-                    mx_a = bf16x2_absmax(pc.xa.z, bf16x2_absmax(pc.xa.w, mx_a));
-                    *reinterpret_cast<uint4 *>(xh + off_a + k) = bf16x8_to_f16x8(pc.xa, 1.0f);
-                }
-                if (row_b) {
-                    mx_b = bf16x2_absmax(pc.xb.x, bf16x2_absmax(pc.xb.y, mx_b));
-                    mx_b = bf16x2_absmax(pc.xb.z, bf16x2_absmax(pc.xb.w, mx_b));
-                    *reinterpret_cast<uint4 *>(xh + off_b + k) = bf16x8_to_f16x8(pc.xb, 1.0f);
-                }
-            }
-            if (rank) {
-                #pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    if (XH_READY) {
-                        ptx::mma_16816_f16(acc[u], pc.xa.x, pc.xb.x, pc.xa.y, pc.xb.y, pc.bv[u].x, pc.bv[u].y);
-                        ptx::mma_16816_f16(acc[u], pc.xa.z, pc.xb.z, pc.xa.w, pc.xb.w, pc.bv[u].z, pc.bv[u].w);
-                    } else {
-                        ptx::mma_16816_bf16(acc[u], pc.xa.x, pc.xb.x, pc.xa.y, pc.xb.y, pc.bv[u].x, pc.bv[u].y);
-                        ptx::mma_16816_bf16(acc[u], pc.xa.z, pc.xb.z, pc.xa.w, pc.xb.w, pc.bv[u].z, pc.bv[u].w);
-                    }
-                }
-            }
-        };
-        PrepassPiece p0, p1;
-        load(p0, 0);
-        for (uint32_t it = 0; it < n_it; it += 2) {
-            load(p1, it + 1);
-            process(p0, it);
-            load(p0, it + 2);
-            process(p1, it + 1);
-        }
-
-        if (MODE == 0 && chunk == 0) {
-            atomicMax(&row_max_bits[g], bf16x2_larger_bits(mx_a));
-            atomicMax(&row_max_bits[g + 8], bf16x2_larger_bits(mx_b));
-        }
-        if (rank) {
-            #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                float *mine = part + warp * (16 * kTPartStride);
-                *reinterpret_cast<float2 *>(mine + g * kTPartStride + 8 * u + 2 * t) = make_float2(acc[u][0], acc[u][1]);
-                *reinterpret_cast<float2 *>(mine + (g + 8) * kTPartStride + 8 * u + 2 * t) =
-                    make_float2(acc[u][2], acc[u][3]);
-            }
-        }
-        __syncthreads();
-        if (MODE != 0 && chunk == 0) {
-            if (threadIdx.x < 16) inv_scale[threadIdx.x] = 1.0f;  // the rows arrive scaled, or stay as they are
-            __syncthreads();
-        }
-        if (MODE == 0 && chunk == 0) {
-            if (threadIdx.x < 16) {
-                const float mx = __uint_as_float(row_max_bits[threadIdx.x]);
-                float sc = 1.0f;
-                if ((mx > 32768.0f || (mx < 0.00390625f && mx >= 1.1754944e-38f)) && mx < __int_as_float(0x7f800000)) {
-                    int e;
-                    frexpf(mx, &e);             // mx = f * 2^e with f in [0.5, 1)
-                    sc = ldexpf(1.0f, e - 15 < -100 ? -100 : e - 15);  // mx / sc lands in [16384, 32768)
-                }
-                inv_scale[threadIdx.x] = 1.0f / sc;  // exact: sc is a power of two
-                if (threadIdx.x < rows) row_scale[m0 + threadIdx.x] = sc * w_up;  // both factors of the outputs
-            }
-            __syncthreads();
-            // rows beyond f16's range: convert again, scaled
-            for (uint32_t r = 0; r < rows; ++r) {
-                const float is = inv_scale[r];
-                if (is == 1.0f) continue;
-                for (uint32_t c = threadIdx.x; c < K / 8; c += kTThreads) {
-                    const uint4 v = __ldg(reinterpret_cast<const uint4 *>(x + (size_t)(m0 + r) * K) + c);
-                    reinterpret_cast<uint4 *>(xh + (size_t)(m0 + r) * K)[c] = bf16x8_to_f16x8(v, is);
-                }
-            }
-        }
-        if (rank) {
-            const uint32_t ld_t = 2 * 64 * chunks;
-            for (uint32_t i = threadIdx.x; i < 16 * 64; i += kTThreads) {
-                const uint32_t r = i >> 6, c = i & 63u;
-                if (m0 + r < M) {
-                    float sum = 0.0f;
-                    #pragma unroll
-                    for (int w = 0; w < kTWarps; ++w) sum += part[w * (16 * kTPartStride) + r * kTPartStride + c];
-                    if (T_ONLY) {
-                        if (chunk * 64 + c < rank) t32[(size_t)(m0 + r) * rank + chunk * 64 + c] = sum;
-                        continue;
-                    }
-                    const float v = sum * scale * inv_scale[r] * w_down;
-                    const __nv_bfloat16 hi = __float2bfloat16_rn(v);
-                    const __nv_bfloat16 lo = __float2bfloat16_rn(v - __bfloat162float(hi));
-                    t_out[(size_t)(m0 + r) * ld_t + chunk * 64 + c] = hi;
-                    t_out[(size_t)(m0 + r) * ld_t + 64 * chunks + chunk * 64 + c] = lo;
-                }
-            }
-        }
-        __syncthreads();
-    }
-}
-
 // ---- weights in the other orientation: repacking before the GEMM ---------------------------
 // W [d_in][d_out] with the 64-blocks along d_out (the reference's Burn layout) is brought into the
 // form the GEMM's dequantisers read: codes_t[n][k / 2] (the same nibbles, transposed, so exact) and
@@ -991,10 +779,6 @@ struct RepackParams {
     uint32_t code_cols, code_rows, code_blocks;   // CTAs of the nibbles: columns of 128 n x groups of kRepackTiles k-tiles
     uint32_t scale_cols, scale_blocks;            // CTAs of the scales: 32 x 32 tiles
     uint32_t adapter_blocks;
-    const float *x32;           // f32 activations [x_rows][K] to convert, or null
-    __half *xh;
-    float *row_scale;
-    uint32_t x_rows;
 };
 constexpr uint32_t kRepackTiles = 4;  // 64-row tiles of nibbles one CTA walks, the next one's loads in flight
 
@@ -1063,7 +847,7 @@ __device__ __forceinline__ void repack_scales_block(const RepackParams &p, uint3
 
 // The adapter factors in the orientation and types the pre-pass and the GEMM read them in.
 // From A [d_in][r], B [r][d_out] of type T:
-//   bf16: a_t[j][k] = A[k][j], b_t[n][j] = B[j][n] (rank_out = r): exact.
+//   bf16: b_t[n][j] = B[j][n]: exact (the pre-pass reads A as it is).
 //   f32:  a_t[j][k] = a_t[r + j][k] = f16(A[k][j]); b_t[n][j] = bf16(B[j][n]), b_t[n][r + j] = the
 //         bf16 of what that rounding left: as an adapter of rank 2 r whose intermediate holds every
 //         column twice, B enters the product with sixteen bits of mantissa.
@@ -1073,16 +857,13 @@ __device__ __forceinline__ void repack_adapter_block(const RepackParams &p, uint
     const T *a = static_cast<const T *>(p.a), *b = static_cast<const T *>(p.b);
     const uint32_t r = p.r, rank_out = kF32 ? 2 * r : r;
     const uint64_t i = (uint64_t)block * blockDim.x + threadIdx.x;
-    const uint64_t na = (uint64_t)r * p.K, nb = (uint64_t)p.N * r;
+    const uint64_t na = kF32 ? (uint64_t)r * p.K : 0, nb = (uint64_t)p.N * r;
     if (i < na) {
-        const uint32_t j = (uint32_t)(i / p.K), k = (uint32_t)(i % p.K);
-        const size_t at = p.factors_out_in ? (size_t)j * p.K + k : (size_t)k * r + j;
         if constexpr (kF32) {
-            const __half h = __float2half_rn(a[at]);
+            const uint32_t j = (uint32_t)(i / p.K), k = (uint32_t)(i % p.K);
+            const __half h = __float2half_rn(a[p.factors_out_in ? (size_t)j * p.K + k : (size_t)k * r + j]);
             p.a_t[i] = __half_as_ushort(h);
             p.a_t[na + i] = __half_as_ushort(h);
-        } else {
-            p.a_t[i] = reinterpret_cast<const uint16_t *>(a)[at];
         }
     } else if (i < na + nb) {
         const uint64_t e = i - na;
@@ -1099,64 +880,18 @@ __device__ __forceinline__ void repack_adapter_block(const RepackParams &p, uint
     }
 }
 
-// f32 activations: xh[m][k] = f16(x[m][k] / sc), sc the power of two that brings the row's largest
-// finite magnitude into [16384, 32768) (any row, so small activations keep their bits too);
-// row_scale[m] = sc * 2^e with e the weight's exponent.  One CTA of 256 threads per row.
-__device__ __forceinline__ void x_f32_to_f16_row(const float *__restrict__ x, uint32_t m, uint32_t K,
-                                                 __half *__restrict__ xh, float *__restrict__ row_scale,
-                                                 const float *__restrict__ absmax,
-                                                 const uint8_t *__restrict__ scale_codes,
-                                                 const float *__restrict__ scale_of_scales, uint32_t *mx_bits) {
-    const float4 *row = reinterpret_cast<const float4 *>(x + (size_t)m * K);
-    if (threadIdx.x == 0) *mx_bits = 0;
-    __syncthreads();
-    uint32_t mx = 0;
-    for (uint32_t c = threadIdx.x; c < K / 4; c += 256) {
-        const float4 v = __ldg(row + c);
-        const uint32_t b[4] = {__float_as_uint(v.x) & 0x7fffffffu, __float_as_uint(v.y) & 0x7fffffffu,
-                               __float_as_uint(v.z) & 0x7fffffffu, __float_as_uint(v.w) & 0x7fffffffu};
-        #pragma unroll
-        for (int q = 0; q < 4; ++q)
-            if (b[q] < 0x7f800000u) mx = max(mx, b[q]);
-    }
-    #pragma unroll
-    for (int s = 16; s > 0; s >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, s));
-    if ((threadIdx.x & 31u) == 0) atomicMax(mx_bits, mx);
-    __syncthreads();
-    const float largest = __uint_as_float(*mx_bits);
-    float sc = 1.0f;
-    if (largest >= 1.1754944e-38f) {  // a normal number
-        int e;
-        frexpf(largest, &e);
-        e = e - 15 < -100 ? -100 : e - 15;  // 1 / sc stays finite
-        sc = ldexpf(1.0f, e);
-    }
-    const float is = 1.0f / sc;
-    if (threadIdx.x == 0)
-        row_scale[m] = sc * ldexpf(1.0f, weight_exponent(absmax, scale_codes, scale_of_scales));
-    uint2 *out = reinterpret_cast<uint2 *>(xh + (size_t)m * K);
-    for (uint32_t c = threadIdx.x; c < K / 4; c += 256) {
-        const float4 v = __ldg(row + c);
-        const __half2 lo = __floats2half2_rn(v.x * is, v.y * is), hi = __floats2half2_rn(v.z * is, v.w * is);
-        out[c] = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
-    }
-}
-
-// One launch for everything in front of the pre-pass: the first code_blocks CTAs take the nibbles,
-// the next scale_blocks the scales, the next adapter_blocks the adapter, the last x_rows one row of
-// f32 activations each.
+// One launch for everything the activations do not need: the first code_blocks CTAs take the nibbles,
+// the next scale_blocks the scales, the last adapter_blocks the adapter.  The pre-pass may run beside it.
 template <class T>
 __global__ void __launch_bounds__(256) repack_kernel(const RepackParams p) {
     __shared__ __align__(16) uint8_t smem[2 * 64 * 80];
+    ptx::pdl_launch_dependents();
     uint32_t b = blockIdx.x;
     if (b < p.code_blocks) return repack_codes_block(p, b, reinterpret_cast<uint8_t(*)[64][80]>(smem));
     b -= p.code_blocks;
     if (b < p.scale_blocks) return repack_scales_block(p, b, reinterpret_cast<float(*)[33]>(smem));
     b -= p.scale_blocks;
-    if (b < p.adapter_blocks) return repack_adapter_block<T>(p, b);
-    b -= p.adapter_blocks;
-    x_f32_to_f16_row(p.x32, b, p.K, p.xh, p.row_scale, p.absmax, p.scale_codes, p.scale_of_scales,
-                     reinterpret_cast<uint32_t *>(smem));
+    repack_adapter_block<T>(p, b);
 }
 
 // ---- host side -----------------------------------------------------------------------
@@ -1313,7 +1048,7 @@ bool prefill_in_out_supported(const nf4_linear_args &a) {
     return true;
 }
 
-int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream) {
+int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_out) {
     const bool repacked = a.layout == NF4_LAYOUT_IN_OUT;
     if (!(repacked ? prefill_in_out_supported(a) : prefill_supported(a)))
         return fail(NF4_ERR_UNSUPPORTED, "prefill_forward: unsupported shape");
@@ -1350,7 +1085,8 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream) {
     p.sk_flags = reinterpret_cast<uint32_t *>(ws + wl.off_flags);
     p.partial = reinterpret_cast<float *>(ws + wl.off_partial);
     const void *lora_a = a.lora_a, *lora_b = a.lora_b;
-    if (extra != kPlain) {  // the other orientation, f32 tensors, or both: one launch in front of the pre-pass
+    bool packing = false;
+    if (repacked || (x_f32 && p.rank)) {  // the other orientation, f32 factors, or both
         RepackParams rp{};
         rp.factors_out_in = !repacked;
         rp.codes = a.packed;
@@ -1372,17 +1108,11 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream) {
             rp.r = a.lora_rank;
             rp.a_t = reinterpret_cast<uint16_t *>(ws + wl.off_a_t);
             rp.b_t = reinterpret_cast<__nv_bfloat16 *>(ws + wl.off_b_t);
-            rp.adapter_blocks = (uint32_t)(((uint64_t)a.lora_rank * (p.K + p.N) + 255) / 256);
-            lora_a = rp.a_t;
+            rp.adapter_blocks = (uint32_t)(((uint64_t)a.lora_rank * ((x_f32 ? p.K : 0) + (uint64_t)p.N) + 255) / 256);
+            if (x_f32) lora_a = rp.a_t;
             lora_b = rp.b_t;
         }
-        if (x_f32) {
-            rp.x32 = static_cast<const float *>(a.x);
-            rp.xh = xh;
-            rp.row_scale = row_scale;
-            rp.x_rows = p.M;
-        }
-        const uint32_t blocks = rp.code_blocks + rp.scale_blocks + rp.adapter_blocks + rp.x_rows;
+        const uint32_t blocks = rp.code_blocks + rp.scale_blocks + rp.adapter_blocks;
         if (x_f32) repack_kernel<float><<<blocks, 256, 0, stream>>>(rp);
         else repack_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(rp);
         count_launch();
@@ -1391,22 +1121,29 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream) {
             p.scales_t = rp.scales_t;
         }
         NF4_CUDA_TRY(cudaGetLastError());
+        packing = true;
     }
-    NF4_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(prefill_prepass_kernel<1>), kTPartBytes));
-    NF4_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(prefill_prepass_kernel<0>), kTPartBytes));
-    if (x_f32) {
-        prefill_prepass_kernel<1><<<(p.M + 15) / 16, kTThreads, kTPartBytes, stream>>>(
-            reinterpret_cast<const __nv_bfloat16 *>(xh), static_cast<const __nv_bfloat16 *>(lora_a), p.M, p.K, p.rank,
-            p.lora_chunks, a.lora_scale, xh, row_scale, t, a.absmax, a.scale_codes, a.scale_of_scales, p.sk_flags,
-            sh.grid, nullptr);
-    } else {
-        prefill_prepass_kernel<0><<<(p.M + 15) / 16, kTThreads, kTPartBytes, stream>>>(
-            static_cast<const __nv_bfloat16 *>(a.x), static_cast<const __nv_bfloat16 *>(lora_a), p.M, p.K, p.rank,
-            p.lora_chunks, a.lora_scale, xh, row_scale, t, a.absmax, a.scale_codes, a.scale_of_scales, p.sk_flags,
-            sh.grid, nullptr);
-    }
-    count_launch();
-    NF4_CUDA_TRY(cudaGetLastError());
+    PrepassArgs pre{};
+    pre.x = a.x;
+    pre.x_f32 = x_f32;
+    pre.M = p.M;
+    pre.K = p.K;
+    pre.a = lora_a;
+    pre.rank = p.rank;
+    pre.k_major = repacked && !x_f32;
+    pre.scale = a.lora_scale;
+    pre.xh = xh;
+    pre.row_scale = row_scale;
+    pre.t_out = t;
+    pre.r_out = r_out;
+    pre.absmax = a.absmax;
+    pre.scale_codes = a.scale_codes;
+    pre.scale_of_scales = a.scale_of_scales;
+    pre.flags = p.sk_flags;
+    pre.n_flags = sh.grid;
+    // (f32 factors reach the pre-pass through the repacking launch: then it has to wait for it)
+    pre.beside_predecessor = packing && !(x_f32 && p.rank);
+    NF4_TRY(activations_prepass(pre, stream));
 
     CUtensorMap map_x, map_t, map_b, map_y;
     NF4_TRY(make_map(&map_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, xh, p.M, p.K, (uint64_t)p.K * 2, BN, BK,
@@ -1441,39 +1178,6 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream) {
     return check_cuda(cudaGetLastError(), "prefill_kernel launch");
 }
 
-
-namespace {
-// dst[j][k] = src[k][j] for a bf16 factor [K][r]
-__global__ void __launch_bounds__(256)
-transpose_factor_kernel(const uint16_t *__restrict__ src, uint16_t *__restrict__ dst, uint64_t K, uint32_t r) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= K * r) return;
-    const uint64_t j = i / K, k = i % K;
-    dst[i] = src[k * r + j];
-}
-}  // namespace
-
-// t32[m][j] = sum_k x[m][k] F(k, j) for bf16 x [rows][k] on the warp MMAs of the pre-pass; the factor is
-// f [rank][k] (`k_major` false) or f [k][rank], which is transposed into `scratch` (rank * k * 2 bytes)
-// first.  Declines shapes its 16-byte loads do not cover.
-int32_t adapter_intermediate_bf16(const void *x, const void *f, bool k_major, uint64_t rows, uint64_t k, uint32_t rank,
-                                  float *t32, void *scratch, cudaStream_t stream) {
-    if (k % 8 != 0 || rows == 0 || rows >= (1ull << 31) || k >= (1ull << 31) || rank == 0 || !aligned16(x) ||
-        (k_major ? !scratch || !aligned16(scratch) : !aligned16(f)))
-        return NF4_ERR_UNSUPPORTED;
-    if (k_major) {
-        transpose_factor_kernel<<<(unsigned)((k * rank + 255) / 256), 256, 0, stream>>>(
-            static_cast<const uint16_t *>(f), static_cast<uint16_t *>(scratch), k, rank);
-        count_launch();
-        f = scratch;
-    }
-    NF4_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(prefill_prepass_kernel<2>), kTPartBytes));
-    prefill_prepass_kernel<2><<<(unsigned)((rows + 15) / 16), kTThreads, kTPartBytes, stream>>>(
-        static_cast<const __nv_bfloat16 *>(x), static_cast<const __nv_bfloat16 *>(f), (uint32_t)rows, (uint32_t)k, rank,
-        lora_chunks_of(rank), 1.0f, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, t32);
-    count_launch();
-    return check_cuda(cudaGetLastError(), "adapter intermediate launch");
-}
 
 int32_t prefill_set_host_flag(int *mapped) {
     return check_cuda(cudaMemcpyToSymbol(g_prefill_error_host, &mapped, sizeof(mapped)), "setting the mapped failure word");

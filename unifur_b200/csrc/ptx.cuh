@@ -67,6 +67,8 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
 // back at once when the phase is not complete and the loop around it competes for issue).
 __device__ __forceinline__ bool mbar_wait_suspended(uint32_t bar, uint32_t parity,
                                                     uint32_t suspend_ns = 4000) {
+    // (the usual case first: reading the global timer takes longer than a wait that is already over)
+    if (mbar_try_wait(bar, parity)) return true;
     const uint64_t t0 = global_timer_ns();
     for (;;) {
         uint32_t ok;
@@ -102,6 +104,19 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst_smem, const void *src, uin
 // 16 bytes, L2 only (streaming data); both addresses 16-byte aligned.
 __device__ __forceinline__ void cp_async_16(uint32_t dst_smem, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
+}
+// The same, or sixteen zeros.
+__device__ __forceinline__ void cp_async_16_or_zero(uint32_t dst_smem, const void *src, bool real) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst_smem), "l"(src), "r"(real ? 16u : 0u) : "memory");
+}
+// Four 8 x 8 matrices of 16-bit values; lane 8i + r gives the address of row r of matrix i.
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
 // 4 bytes; both addresses 4-byte aligned.
 __device__ __forceinline__ void cp_async_4(uint32_t dst_smem, const void *src) {

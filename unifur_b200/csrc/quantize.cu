@@ -466,6 +466,7 @@ scale_max_cluster_kernel(const float4 *__restrict__ absmax4, const float *__rest
     constexpr uint32_t kStride = kClusterCtas * kClusterThreads, kInFlight = 8;
     ptx::pdl_wait();
     ptx::pdl_launch_dependents();
+    cluster.barrier_arrive();  // (waited for before another CTA's shared memory is touched)
     float m = 0.0f;
     for (uint32_t i = rank * kClusterThreads + tid; i < n4; i += kStride * kInFlight) {
         float4 v[kInFlight];
@@ -484,8 +485,9 @@ scale_max_cluster_kernel(const float4 *__restrict__ absmax4, const float *__rest
         m = s_warp[tid];
         #pragma unroll
         for (int s = 1; s < 32; s <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, s));
-        if (tid == 0) cluster.map_shared_rank(s_cta, 0)[rank] = m;
     }
+    cluster.barrier_wait();
+    if (tid == 0) cluster.map_shared_rank(s_cta, 0)[rank] = m;
     cluster.sync();
     if (rank == 0 && tid == 0) {
         m = s_cta[0];
