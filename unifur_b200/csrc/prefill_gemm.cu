@@ -3,33 +3,36 @@
 // bound, built on tcgen05.mma with the dequantised weight operand and the accumulator in
 // tensor memory (TMEM) and the activations in shared memory.
 //
-// Roles inside one persistent CTA (one per SM, 864 threads):
-//   warp 0      TMA producer: x tiles [256 rows x 64 k] (f16, 128B-swizzled, K-major) into a
-//               4-deep shared-memory ring; after the K loop the same ring carries the LoRA
-//               intermediate T (bf16 hi / lo halves) and a second small ring the matching
-//               128 x 64 tiles of LoRA B, so the adapter is just more k-steps (with both
+// Two CTAs of a cluster, one per SM, work on a tile of 256 weight rows x 256 activation rows together
+// (cta_group::2): each holds 128 weight rows and their accumulators in its tensor memory and half of the
+// activations in its shared memory, which halves what a shared memory is written and read per
+// multiplication.  Roles inside a CTA (persistent, 864 threads):
+//   warp 0      TMA producer: this CTA's half of the x tile [128 rows x 64 k] (f16, 128B-swizzled,
+//               K-major) into a 4-deep shared-memory ring; after the K loop the same ring carries the LoRA
+//               intermediate T (bf16 hi / lo halves) and one more place the matching
+//               128 x 64 tile of LoRA B, so the adapter is just more k-steps (with both
 //               operands in shared memory).
-//   warp 1      owns TMEM (alloc/dealloc); one of its threads issues the tcgen05.mma of the even
-//               k-stages, one thread of warp 6 those of the odd ones.  Issuing a stage's MMAs
-//               holds the thread for about as long as they run, and waits, fences and commits
-//               separate two batches; with two threads the second has done its waiting while
-//               the first issues, and only a short hand-over is left.
+//   warp 1      owns TMEM (alloc/dealloc); in the even CTA it issues the pair's tcgen05.mma.
+//   warp 6      asks for the packed codes: blocks of 128 weight rows x 256 codes by TMA, prefetched into L2.
 //   warps 2-5, 23-26  epilogue: TMEM -> registers -> (* row scale, + bias) -> bf16/f32 ->
 //               shared -> TMA store.
 //   warps 7-22  dequantisers, four groups of 128 threads taking every fourth k-stage.  A thread
 //               owns one weight row (= one TMEM lane; a warp may only touch the lane quarter its
-//               number names): it reads the row's 32 packed bytes and the block scale straight
-//               from global memory (L2), expands the nibbles with byte-permute lookups held in
-//               registers, multiplies by the scale in f16x2 and writes the 64 f16 values into
-//               its lane of an eight-deep ring of TMEM columns with tcgen05.st.
+//               number names): it takes the row's 32 packed bytes from shared memory, looks byte by
+//               byte a pair of levels up in a table, multiplies by the block's scale in f16x2 and writes the
+//               64 f16 values into its lane of an eight-deep ring of TMEM columns with tcgen05.st.
 //
-// Why the weight operand lives in TMEM.  An MMA of 128 x 256 x 16 with both operands in shared
-// memory reads 12 KB per 128 cycles, and the TMA and the dequantisers write as much again: more
-// than the 128 B/clk a shared memory delivers, so the k-stage was bound by shared-memory traffic.
-// With the 128-row operand in TMEM the shared memory carries only the activation tile (written
-// once, read once), and the dequantised weight never touches it.  The price: the accumulator
+// Why the weight operand lives in TMEM.  The table look-ups, the TMA and the MMA's reads of the
+// activations already take most of the 128 B/clk a shared memory delivers; the dequantised weight never
+// touches it.  The price: the accumulator
 // (256 columns) and the weight ring (8 x 32 columns) share the 512 TMEM columns, so there is one
 // accumulator and the MMAs of the next tile wait while the epilogue reads it out.
+//
+// What bounds it: for many rows the tensor pipe (512 cycles a stage and pair; 570 to 630 are taken, with
+// the read-outs), and the clock that the power limit leaves (1.55 GHz on random operands, 1.83 GHz on zeros).
+// 2048 x 4096 x 14336: 231 us with single CTAs, codes loaded by the dequantisers and two issuing threads; now
+// 178, of which the kernels before it take 15.  256 x 3584 x 18944: 45 -> 34 us.  What gave it: the pairs; codes
+// by TMA; one full and one done barrier per stage, both halves counted in the even CTA; the issuing warp together.
 //
 // The MMA computes D[n, m] = sum_k W[n, k] x[m, k]: weight rows are the MMA's M (TMEM lanes),
 // activation rows its N (256 accumulator columns).  Both operands are f16 with f32 accumulation:
@@ -64,30 +67,45 @@ __device__ int *g_prefill_error_host = nullptr;  // the same, in mapped host mem
 
 namespace {
 
-constexpr int BM = 128;        // weight rows per tile (MMA M, TMEM lanes)
-constexpr int BN = 256;        // activation rows per tile (MMA N, accumulator columns)
+constexpr int BM = 128;        // weight rows per CTA and tile (half of the pair's MMA M; TMEM lanes)
+constexpr int BN = 256;        // activation rows per tile (MMA N, accumulator columns); a CTA brings half of them
 constexpr int BK = 64;         // k per stage = one quantization block = one 128B swizzle row
 constexpr int kXStages = 4;    // shared-memory ring of activation tiles
-constexpr int kLoraStages = 2; // shared-memory ring of LoRA B tiles (adapter k-stages)
+constexpr int kCodeSlots = 2;  // shared-memory ring of packed weight codes, four k-stages each
+constexpr int kCodeStages = 4;
 constexpr int kAStages = 8;    // TMEM ring of dequantised weight stages
 constexpr int kAStageCols = BK / 2;  // 32 columns: two f16 per 32-bit cell
 constexpr int kAccCols = BN;   // the accumulator: columns [0, 256); the weight ring follows
 constexpr int kTmemCols = 512;
-constexpr int kXTileBytes = BN * BK * 2;   // 32 KB: activations, written by TMA
-constexpr int kLoraTileBytes = BM * BK * 2;  // 16 KB: 128 rows of LoRA B x 64 ranks, written by TMA
+constexpr int kXTileBytes = BN / 2 * BK * 2;   // 16 KB: this CTA's half of the activations, written by TMA
+constexpr int kLoraTileBytes = BM * BK * 2;    // 16 KB: 128 rows of LoRA B x 64 ranks, written by TMA
+constexpr int kCodeTileBytes = BM * 128;       // 16 KB: 128 weight rows x 256 codes, written by TMA (128B swizzle)
 
-constexpr int kEpiBytes = 64 * 1024;       // output staging: a whole tile of bf16, half a tile of f32
+constexpr int kEpiBytes = 32 * 1024;       // output staging: half a tile of bf16, a quarter of f32
 constexpr int kThreads = 27 * 32;
 constexpr int kFirstExpanderWarp = 7;      // sixteen warps
 constexpr int kFirstEpilogueWarpB = 23;    // the second set of four epilogue warps
+constexpr int kCodeWarp = 6;               // asks for the packed codes
+constexpr int kStageWarps = 8;             // warps that dequantise one stage: a group in each CTA
 constexpr int kExpanderGroups = 4;         // of four warps (one per TMEM lane quarter) each
 constexpr uint64_t kInOutMinRows = 17;     // the other weight orientation comes here from this many rows on
 
+// Places in the shared window.  The lookup table starts at 0x10000, so that one byte permute of the code
+// word with {4 lane, 0, 1, rank} is an entry's address.
+constexpr uint32_t kLoraAt = 0x800, kCodesAt = 0x4800, kBarsAt = 0xc800, kTmemSlotAt = 0xca00, kRowScalesAt = 0xcc00,
+                   kTableAt = 0x10000, kEpiAt = 0x20000, kXAt = 0x28000, kWindowEnd = kXAt + kXStages * kXTileBytes;
+constexpr uint32_t kDynamicSmem = kWindowEnd - 1024;   // the dynamic shared memory starts at 1024 or a little above
+static_assert(kLoraAt + kLoraTileBytes <= kCodesAt && kCodesAt + kCodeSlots * kCodeTileBytes <= kBarsAt && kEpiAt + kEpiBytes <= kXAt, "places overlap");
+static_assert(kDynamicSmem <= 227 * 1024, "shared memory");
+
 // barrier slots
-constexpr int kBarXFull = 0, kBarXEmpty = kBarXFull + kXStages, kBarAFull = kBarXEmpty + kXStages,
-              kBarAEmpty = kBarAFull + kAStages, kBarAccFull = kBarAEmpty + kAStages,
-              kBarAccEmpty = kBarAccFull + 1, kBarIssued = kBarAccEmpty + 1, kBarLEmpty = kBarIssued + 2,
-              kNumBars = kBarLEmpty + kLoraStages;
+// Full counts, in the even CTA, what a k-stage of the pair needs: both halves of the activations (or of an
+// adapter stage's operands) and the eight warps of both CTAs that dequantise its weights.  Done is a stage's
+// MMAs over, in both CTAs: whatever the stage's slots held is free.  Stages number on over a pair's segments,
+// the adapter's included; stage c has slot c % kXStages of the activations, c % kAStages of everything else.
+constexpr int kBarFull = 0, kBarDone = kBarFull + kAStages, kBarAccFull = kBarDone + kAStages, kBarAccEmpty = kBarAccFull + 1,
+              kBarCFull = kBarAccEmpty + 1, kBarCEmpty = kBarCFull + kCodeSlots, kNumBars = kBarCEmpty + kCodeSlots;
+static_assert(kBarsAt + kNumBars * 8 <= kTmemSlotAt, "barrier room");
 
 struct PrefillParams {
     const uint8_t *codes;
@@ -102,11 +120,12 @@ struct PrefillParams {
     const __half *scales_t;
     uint32_t M, N, K, rank;
     uint32_t lora_chunks;  // ceil(rank / 64); T is [M][2 * 64 * lora_chunks] (hi halves, then lo)
-    uint32_t m_tiles, n_tiles;
-    // Work of a CTA: first its share of the `sk_tiles` tiles whose k-stages all CTAs divide
-    // evenly between them (a tile can be split between neighbouring CTAs), then `dp_rounds`
-    // whole tiles.  A CTA that multiplies the leading stages of a tile leaves its accumulator
-    // in `partial` ([CTA][BN][BM] f32) and raises its word of `sk_flags`; the CTA that multiplies
+    uint32_t m_tiles;
+    // Work of a pair of CTAs (tiles of 256 weight rows x 256 activation rows, the even CTA the lower 128
+    // weight rows): first its share of the `sk_tiles` tiles whose k-stages all pairs divide
+    // evenly between them (a tile can be split between neighbouring pairs), then `dp_rounds`
+    // whole tiles.  A pair that multiplies the leading stages of a tile leaves its accumulators
+    // in `partial` ([CTA][BN][BM] f32) and raises its CTAs' words of `sk_flags`; the pair that multiplies
     // the last stages adds those and finishes the tile.
     uint32_t sk_tiles, dp_rounds;
     float *partial;
@@ -114,12 +133,12 @@ struct PrefillParams {
     uint32_t wait_ns;  // bound of the wait for a neighbour's flag
 };
 
-// This CTA's list of segments (tile, main k-stages [b, e)), in the order they are worked on: the
+// A pair's list of segments (tile, main k-stages [b, e)), in the order they are worked on: the
 // shared tiles from the last to the first -- a piece without a tile's last stage comes first and
 // waits for nobody; the piece with the last stage of a tile that a neighbour began comes last of
 // them -- then the whole tiles.
 struct WorkList {
-    uint64_t u0, u1;   // this CTA's range of main stages of the shared tiles
+    uint64_t u0, u1;   // this pair's range of main stages of the shared tiles
     uint32_t ks;       // main stages per tile
     uint32_t t_first, t_last, n_shared, n_seg, sk_tiles, cta, ctas;
 
@@ -201,137 +220,75 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&a)[16
         : "memory");
 }
 
-// ---- nibble -> f16 expansion with byte-permute lookups --------------------------------
-// The sixteen f16 levels are split into a table of high bytes and a table of low bytes, four
-// registers each.  One prmt looks four nibbles up in an 8-entry half table; a third prmt picks,
-// per nibble, the half its top bit names; a last pair interleaves high and low bytes.
-struct LevelTables {
-    uint32_t hi[4], lo[4];
-};
-
-__device__ __forceinline__ LevelTables make_level_tables() {
-    LevelTables t;
-    #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        uint32_t h = 0, l = 0;
-        #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint32_t bits = __half_as_ushort(
-                __float2half_rn(__uint_as_float(c_level_bits[4 * q + i])));
-            h |= (bits >> 8) << (8 * i);
-            l |= (bits & 0xffu) << (8 * i);
-        }
-        t.hi[q] = h;
-        t.lo[q] = l;
-    }
-    return t;
-}
-
-__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-
-// Four nibbles (bits 0..15 of `w4`) -> two f16x2 registers {e0,e1}, {e2,e3}.
-__device__ __forceinline__ void expand4(const LevelTables &t, uint32_t w4, uint32_t &out01,
-                                        uint32_t &out23) {
-    const uint32_t sel = w4 & 0x7777u;
-    const uint32_t pick = ((w4 & 0x8888u) >> 1) | 0x3210u;
-    const uint32_t h = prmt(prmt(t.hi[0], t.hi[1], sel), prmt(t.hi[2], t.hi[3], sel), pick);
-    const uint32_t l = prmt(prmt(t.lo[0], t.lo[1], sel), prmt(t.lo[2], t.lo[3], sel), pick);
-    out01 = prmt(l, h, 0x5140u);
-    out23 = prmt(l, h, 0x7362u);
-}
-
+// ---- nibble -> f16 expansion --------------------------------------------------------------
+// One packed byte (two codes) indexes a 256-entry table of half2 {level[lo], level[hi]} in shared memory,
+// replicated per lane (no bank conflicts; entries 256 bytes apart, half of that used): a permute, a load
+// and the multiplication by the scale per two weights.  (Byte-permute lookups in registers take four times
+// the instructions; the table's reads have room in the shared memory because a CTA of a pair moves half an
+// activation tile per stage.)
 __device__ __forceinline__ uint32_t hmul2(uint32_t a, uint32_t b) {
     uint32_t d;
     asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
     return d;
 }
-
-// Half a stage of one weight row: 16 packed bytes + scale -> 16 registers of f16x2.
-__device__ __forceinline__ void expand_half(const LevelTables &t, const uint4 &c, float scale,
-                                            uint32_t (&out)[16]) {
-    const __half2 s2 = __float2half2_rn(scale);
-    const uint32_t s = *reinterpret_cast<const uint32_t *>(&s2);
-    const uint32_t w[4] = {c.x, c.y, c.z, c.w};
-    #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        uint32_t a, b, c2, d;
-        expand4(t, w[i], a, b);
-        expand4(t, w[i] >> 16, c2, d);
-        out[4 * i + 0] = hmul2(a, s);
-        out[4 * i + 1] = hmul2(b, s);
-        out[4 * i + 2] = hmul2(c2, s);
-        out[4 * i + 3] = hmul2(d, s);
-    }
+__device__ __forceinline__ uint32_t level_pair(uint32_t word, int byte, uint32_t lane_word) {
+    const uint32_t at = __byte_perm(word, lane_word, 0x7604u | ((uint32_t)byte << 4));  // {4 lane, the byte, 1, rank}
+    uint32_t v;
+    asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(at));
+    return v;
 }
 
-// The same with a scale per k: lane j of the warp holds the f16 pair of scales of k = 2j, 2j + 1
-// of this stage (`pairs`); `first` is the pair that goes with out[0].
-__device__ __forceinline__ void expand_half_per_k(const LevelTables &t, const uint4 &c, uint32_t pairs,
-                                                  int first, uint32_t (&out)[16]) {
-    const uint32_t w[4] = {c.x, c.y, c.z, c.w};
+// Half a stage of one weight row: 16 packed bytes -> 16 registers of f16x2.  PERK (a scale per k): lane j
+// of the warp holds the f16 pair of scales of k = 2j, 2j + 1 of this stage; `first` is the pair of out[0].
+template <bool PERK>
+__device__ __forceinline__ void expand_half(const uint32_t *w, uint32_t scale2, int first, uint32_t lane_word, uint32_t (&out)[16]) {
     #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        uint32_t a, b, c2, d;
-        expand4(t, w[i], a, b);
-        expand4(t, w[i] >> 16, c2, d);
-        out[4 * i + 0] = hmul2(a, __shfl_sync(0xffffffffu, pairs, first + 4 * i + 0));
-        out[4 * i + 1] = hmul2(b, __shfl_sync(0xffffffffu, pairs, first + 4 * i + 1));
-        out[4 * i + 2] = hmul2(c2, __shfl_sync(0xffffffffu, pairs, first + 4 * i + 2));
-        out[4 * i + 3] = hmul2(d, __shfl_sync(0xffffffffu, pairs, first + 4 * i + 3));
+    for (int i = 0; i < 16; ++i) {
+        const uint32_t v = level_pair(w[i >> 2], i & 3, lane_word);
+        out[i] = hmul2(v, PERK ? __shfl_sync(0xffffffffu, scale2, first + i) : scale2);
     }
 }
-
-struct RowStage {
-    uint4 c0, c1;    // the row's 64 packed codes of one k-stage
-    uint32_t scale;  // its scale as loaded: f32 bits, a u8 code, or (PERK) this lane's pair of f16 scales
-};
 
 template <bool YF32, bool PERK>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_t,
                const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_y,
-               const PrefillParams p) {
+               const __grid_constant__ CUtensorMap tmap_w, const PrefillParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    // 1024-byte alignment for the swizzled operand tiles
-    uint8_t *smem = reinterpret_cast<uint8_t *>(
-        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t *x_ring = smem;                                   // kXStages activation tiles
-    uint8_t *lora_ring = x_ring + kXStages * kXTileBytes;     // kLoraStages tiles of LoRA B
-    uint8_t *epi = lora_ring + kLoraStages * kLoraTileBytes;  // output staging, 64 KB
+    // In a cluster a CTA's shared-memory addresses carry its rank in the top byte: `own`.
+    const uint32_t win = ptx::smem_addr(smem_raw), own = win & 0xff000000u;
+    auto at = [&](uint32_t place) { return smem_raw + ((own | place) - win); };
     constexpr int kStageRows = kEpiBytes / (BM * (YF32 ? 4 : 2));  // activation rows per staging pass
-    uint64_t *bars = reinterpret_cast<uint64_t *>(epi + kEpiBytes);
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + kNumBars);
-    float *row_scales = reinterpret_cast<float *>(bars + kNumBars + 2);  // BN factors of the tile's rows
+    uint8_t *epi = at(kEpiAt);
+    float *row_scales = reinterpret_cast<float *>(at(kRowScalesAt));  // BN factors of the tile's rows
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const uint32_t bar0 = ptx::smem_addr(bars);
-    auto bar = [&](int i) { return bar0 + 8u * i; };
+    const uint32_t rank = ptx::cluster_cta_rank(), pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    auto bar = [&](int i) { return (own | kBarsAt) + 8u * i; };
 
     const uint32_t k_stages = p.K / BK;
     const uint32_t lora_stages = 2 * p.lora_chunks;  // adapter k-stages per tile: hi and lo halves of T
     WorkList wl;
-    wl.init(p, k_stages, blockIdx.x, gridDim.x);
+    wl.init(p, k_stages, pair, pairs);
 
+    if (win - own > kLoraAt) {  // (both CTAs alike) the places below are not ours
+        if (threadIdx.x == 0) NF4_REPORT_FAILURE(g_prefill_error, g_prefill_error_host, 6);
+        return;
+    }
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kXStages; ++s) {
-            ptx::mbar_init(bar(kBarXFull + s), 1);
-            ptx::mbar_init(bar(kBarXEmpty + s), 1);
-        }
         for (int s = 0; s < kAStages; ++s) {
-            ptx::mbar_init(bar(kBarAFull + s), 4);  // the four warps writing the stage
-            ptx::mbar_init(bar(kBarAEmpty + s), 1);
+            ptx::mbar_init(bar(kBarFull + s), 1 + kStageWarps);
+            ptx::mbar_init(bar(kBarDone + s), 1);
         }
         ptx::mbar_init(bar(kBarAccFull), 1);
-        ptx::mbar_init(bar(kBarAccEmpty), 8);
-        ptx::mbar_init(bar(kBarIssued + 0), 1);
-        ptx::mbar_init(bar(kBarIssued + 1), 1);
-        for (int s = 0; s < kLoraStages; ++s) ptx::mbar_init(bar(kBarLEmpty + s), 1);
+        ptx::mbar_init(bar(kBarAccEmpty), 16);      // the epilogue warps of both CTAs (used in the even one)
+        for (int s = 0; s < kCodeSlots; ++s) {
+            ptx::mbar_init(bar(kBarCFull + s), 1);
+            ptx::mbar_init(bar(kBarCEmpty + s), 16);  // the dequantiser warps
+        }
         ptx::fence_mbar_init();
         ptx::fence_proxy_async();
+        ptx::prefetch_tmap(&tmap_w);
         ptx::prefetch_tmap(&tmap_x);
         ptx::prefetch_tmap(&tmap_y);
         if (p.lora_chunks) {
@@ -339,14 +296,22 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             ptx::prefetch_tmap(&tmap_b);
         }
     }
+    if (threadIdx.x >= 64 && threadIdx.x < 64 + 512) {
+        // thread (byte, half) writes sixteen lanes' copies, rotated so that a warp's stores spread over the banks
+        const uint32_t i = threadIdx.x - 64, byte = i >> 1, half = i & 1u;
+        const uint32_t e = c_level_f16_bits[byte & 15u] | (c_level_f16_bits[byte >> 4] << 16);
+        #pragma unroll
+        for (uint32_t q = 0; q < 4; ++q)
+            *reinterpret_cast<uint4 *>(at(kTableAt) + byte * 256u + half * 64u + ((q + byte) & 3u) * 16u) = make_uint4(e, e, e, e);
+    }
     if (warp == 1) {
-        ptx::tmem_alloc(ptx::smem_addr(tmem_slot), kTmemCols);
-        ptx::tmem_relinquish();
+        ptx::tmem_alloc_pair(own | kTmemSlotAt, kTmemCols);
+        ptx::tmem_relinquish_pair();
     }
     ptx::tc_fence_before();
-    __syncthreads();
+    ptx::cluster_sync_all();  // (a superset of __syncthreads) the barriers of both CTAs are in place
     ptx::tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = *reinterpret_cast<const uint32_t *>(at(kTmemSlotAt));
     const uint32_t tmem_acc = tmem_base;             // columns [0, 256)
     const uint32_t tmem_a = tmem_base + kAccCols;    // kAStages x 32 columns
 
@@ -358,124 +323,105 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             // the f16 activations and T come from the pre-pass, which may still be running: this
             // kernel is its programmatic dependent (the dequantisers start on the weights at once)
             ptx::pdl_wait();
-            uint32_t cnt = 0, lcnt = 0;
+            uint32_t cnt = 0;
+            int32_t b_read = -1;  // the last adapter stage so far
             for (uint32_t seg = 0; seg < wl.n_seg && ok; ++seg) {
                 uint32_t tile, kb, ke;
                 wl.get(seg, tile, kb, ke);
-                const uint32_t m0 = (tile % p.m_tiles) * BN, n0 = (tile / p.m_tiles) * BM;
+                const uint32_t m0 = (tile % p.m_tiles) * BN + rank * (BN / 2), n0 = ((tile / p.m_tiles) * 2 + rank) * BM;
                 // the adapter's stages follow a tile's last main stage
                 const uint32_t k_end = ke == k_stages ? k_stages + lora_stages : ke;
                 for (uint32_t ks = kb; ks < k_end; ++ks, ++cnt) {
-                    const uint32_t s = cnt % kXStages, ph = (cnt / kXStages) & 1u;
-                    if (!ptx::mbar_wait_suspended(bar(kBarXEmpty + s), ph ^ 1u)) {
+                    const bool main_stage = ks < k_stages;
+                    const uint32_t j = main_stage ? 0 : ks - k_stages;
+                    const bool new_b = !main_stage && (j & 1u) == 0;  // a chunk of B serves the hi and the lo half of T
+                    // the slot's last reader is done, and the last one of the B tile's only place
+                    int32_t last = (int32_t)cnt - kXStages;
+                    if (new_b && b_read > last) last = b_read;
+                    if (last >= 0 && !ptx::mbar_wait_suspended(bar(kBarDone + last % kAStages), ((uint32_t)last / kAStages) & 1u)) {
                         ok = false;
                         break;
                     }
-                    const uint32_t dst = ptx::smem_addr(x_ring + s * kXTileBytes);
-                    if (ks < k_stages) {
-                        ptx::mbar_arrive_expect_tx(bar(kBarXFull + s), kXTileBytes);
-                        ptx::tma_load_2d(dst, &tmap_x, (int32_t)(ks * BK), (int32_t)m0,
-                                         bar(kBarXFull + s));
+                    const uint32_t dst = (own | kXAt) + (cnt % kXStages) * kXTileBytes;
+                    const uint32_t full = bar(kBarFull + cnt % kAStages), pair_full = ptx::map_to_rank(full, 0);
+                    if (main_stage) {
+                        if (rank == 0) ptx::mbar_arrive_expect_tx(full, 2 * kXTileBytes);
+                        ptx::tma_load_2d_pair(dst, &tmap_x, (int32_t)(ks * BK), (int32_t)m0, pair_full);
                     } else {
-                        // adapter stage: a tile of T beside the activations' ring slot and the
+                        // adapter stage: a tile of T in the activations' ring slot and the
                         // matching 128 x 64 tile of LoRA B (ranks beyond the adapter's read as
                         // zero) as the MMA's other shared-memory operand
-                        const uint32_t j = ks - k_stages;
-                        const uint32_t ls = lcnt % kLoraStages, lph = (lcnt / kLoraStages) & 1u;
-                        ++lcnt;
-                        if (!ptx::mbar_wait_suspended(bar(kBarLEmpty + ls), lph ^ 1u)) {
-                            ok = false;
-                            break;
-                        }
-                        ptx::mbar_arrive_expect_tx(bar(kBarXFull + s), kXTileBytes + kLoraTileBytes);
-                        ptx::tma_load_2d(dst, &tmap_t, (int32_t)(j * BK), (int32_t)m0, bar(kBarXFull + s));
-                        ptx::tma_load_2d(ptx::smem_addr(lora_ring + ls * kLoraTileBytes), &tmap_b,
-                                         (int32_t)((j % p.lora_chunks) * BK), (int32_t)n0,
-                                         bar(kBarXFull + s));
+                        b_read = (int32_t)cnt;
+                        if (rank == 0) ptx::mbar_arrive_expect_tx(full, 2 * (kXTileBytes + (new_b ? kLoraTileBytes : 0)));
+                        ptx::tma_load_2d_pair(dst, &tmap_t, (int32_t)(((j & 1u) * p.lora_chunks + j / 2) * BK), (int32_t)m0, pair_full);
+                        if (new_b) ptx::tma_load_2d_pair(own | kLoraAt, &tmap_b, (int32_t)(j / 2 * BK), (int32_t)n0, pair_full);
                     }
                 }
             }
-            if (!ok) NF4_REPORT_FAILURE(g_prefill_error, g_prefill_error_host, 1);
+            if (!ok) {
+                NF4_REPORT_FAILURE(g_prefill_error, g_prefill_error_host, 1);
+                __nanosleep(1000000);  // the copies in flight (counted in the even CTA) end before the CTA does
+            }
         }
-    } else if (warp == 1 || warp == 6) {
-        // ============================= MMA issuers =============================
-        // Thread `me` (0: warp 1, 1: warp 6) issues the stages whose global counter has its
-        // parity.  Stage c may only be issued after stage c - 1 has been (hand-over barrier
-        // kBarIssued + parity of c - 1), which keeps the MMAs of the accumulator in order.
-        if (lane == 0) {
-            const uint32_t me = warp == 1 ? 0u : 1u;
-            constexpr uint32_t idesc_main = make_idesc(0, 0, BM, BN);  // f16 x f16
-            constexpr uint32_t idesc_lora = make_idesc(1, 1, BM, BN);  // bf16 x bf16
-            const uint32_t x_addr = ptx::smem_addr(x_ring);
-            uint32_t cnt = 0, a_next = 0, l_next = 0;  // stages, main stages, adapter stages so far
+    } else if (warp == 1) {
+        // ============================= MMA issuer =============================
+        // One thread of the even CTA issues the pair's MMAs: per stage one wait, four MMAs, one commit.  The
+        // warp stays together and elects the thread where it issues, so that addresses and descriptors are
+        // uniform registers; one lane on its own in a branch spent 77 cycles on each MMA, which takes 128.
+        if (rank == 0) {
+            constexpr uint32_t idesc_main = make_idesc(0, 0, 2 * BM, BN);  // f16 x f16
+            constexpr uint32_t idesc_lora = make_idesc(1, 1, 2 * BM, BN);  // bf16 x bf16
+            uint32_t cnt = 0;
             for (uint32_t seg = 0; seg < wl.n_seg && ok; ++seg) {
                 uint32_t tile, kb, ke;
                 wl.get(seg, tile, kb, ke);
-                const uint32_t k_end = ke == k_stages ? k_stages + lora_stages : ke;
-                for (uint32_t ks = kb; ks < k_end; ++ks, ++cnt) {
-                    // the weight ring counts main stages only, the LoRA ring adapter stages only
-                    const bool main_stage = ks < k_stages;
-                    const uint32_t acnt = a_next, lcnt = l_next;
-                    if (main_stage) ++a_next;
-                    else ++l_next;
-                    if ((cnt & 1u) != me) continue;
-                    const uint32_t sx = cnt % kXStages, phx = (cnt / kXStages) & 1u;
-                    const uint32_t sa = acnt % kAStages, pha = (acnt / kAStages) & 1u;
-                    const uint32_t ls = lcnt % kLoraStages;
-                    // the epilogue must have read the previous segment out of the accumulator
-                    if (ks == kb && !ptx::mbar_wait_suspended(bar(kBarAccEmpty), (seg & 1u) ^ 1u)) {
-                        ok = false;
-                        break;
-                    }
-                    if (!ptx::mbar_wait_suspended(bar(kBarXFull + sx), phx)) {
-                        ok = false;
-                        break;
-                    }
-                    if (main_stage && !ptx::mbar_wait_suspended(bar(kBarAFull + sa), pha)) {
-                        ok = false;
-                        break;
-                    }
-                    // hand-over: the other thread has issued stage cnt - 1 (its (cnt-1)/2-th)
-                    if (cnt > 0 &&
-                        !ptx::mbar_wait_suspended(bar(kBarIssued + (me ^ 1u)), ((cnt - 1) >> 1) & 1u)) {
-                        ok = false;
-                        break;
-                    }
+                // the epilogues must have read the previous segment out of the accumulators
+                ok = ptx::mbar_wait_suspended(bar(kBarAccEmpty), (seg & 1u) ^ 1u);
+                for (uint32_t ks = kb; ks < ke && ok; ++ks, ++cnt) {
+                    const uint32_t s = cnt % kAStages;
+                    const uint64_t bdesc = make_kmajor_sw128_desc(kXAt + (cnt % kXStages) * kXTileBytes);
+                    const uint32_t a_cols = tmem_a + s * kAStageCols;
+                    ok = ptx::mbar_wait_suspended(bar(kBarFull + s), (cnt / kAStages) & 1u);
+                    if (!ok) break;
                     ptx::tc_fence_after();
-                    const uint64_t bdesc = make_kmajor_sw128_desc(x_addr + sx * kXTileBytes);
-                    const uint32_t a_cols = tmem_a + sa * kAStageCols;
-                    if (main_stage) {
+                    if (ptx::elect_one()) {
                         // 16 k = 8 TMEM columns of the weight stage = 32 bytes inside the
                         // activation tile's swizzled row (+2 in the encoded address)
-                        ptx::mma_ts_f16(tmem_acc, a_cols, bdesc, idesc_main, ks != kb ? 1u : 0u);
-                        ptx::mma_ts_f16(tmem_acc, a_cols + 8, bdesc + 2, idesc_main, 1u);
-                        ptx::mma_ts_f16(tmem_acc, a_cols + 16, bdesc + 4, idesc_main, 1u);
-                        ptx::mma_ts_f16(tmem_acc, a_cols + 24, bdesc + 6, idesc_main, 1u);
-                    } else {
-                        const uint32_t chunk = (ks - k_stages) % p.lora_chunks;
-                        const uint32_t left = p.rank - chunk * 64;
-                        const uint32_t nk16 = ((left < 64 ? left : 64) + 15) / 16;
-                        const uint64_t adesc =
-                            make_kmajor_sw128_desc(ptx::smem_addr(lora_ring) + ls * kLoraTileBytes);
-                        for (uint32_t j = 0; j < nk16; ++j)
-                            ptx::mma_ss_f16(tmem_acc, adesc + 2 * j, bdesc + 2 * j, idesc_lora, 1u);
+                        ptx::mma_ts_f16_pair(tmem_acc, a_cols, bdesc, idesc_main, ks != kb ? 1u : 0u);
+                        ptx::mma_ts_f16_pair(tmem_acc, a_cols + 8, bdesc + 2, idesc_main, 1u);
+                        ptx::mma_ts_f16_pair(tmem_acc, a_cols + 16, bdesc + 4, idesc_main, 1u);
+                        ptx::mma_ts_f16_pair(tmem_acc, a_cols + 24, bdesc + 6, idesc_main, 1u);
+                        ptx::tc_commit_pair(bar(kBarDone + s));
                     }
-                    ptx::tc_fence_before();
-                    ptx::mbar_arrive(bar(kBarIssued + me));
-                    ptx::tc_commit(bar(kBarXEmpty + sx));
-                    ptx::tc_commit(main_stage ? bar(kBarAEmpty + sa) : bar(kBarLEmpty + ls));
-                    if (ks + 1 == k_end) ptx::tc_commit(bar(kBarAccFull));
+                    __syncwarp();
                 }
+                for (uint32_t j = 0; ke == k_stages && j < lora_stages && ok; ++j, ++cnt) {
+                    const uint32_t s = cnt % kAStages;
+                    const uint32_t left = p.rank - j / 2 * 64, nk16 = ((left < 64 ? left : 64) + 15) / 16;
+                    const uint64_t adesc = make_kmajor_sw128_desc(kLoraAt);
+                    const uint64_t bdesc = make_kmajor_sw128_desc(kXAt + (cnt % kXStages) * kXTileBytes);
+                    ok = ptx::mbar_wait_suspended(bar(kBarFull + s), (cnt / kAStages) & 1u);
+                    if (!ok) break;
+                    ptx::tc_fence_after();
+                    if (ptx::elect_one()) {
+                        for (uint32_t i = 0; i < nk16; ++i)
+                            ptx::mma_ss_f16_pair(tmem_acc, adesc + 2 * i, bdesc + 2 * i, idesc_lora, 1u);
+                        ptx::tc_commit_pair(bar(kBarDone + s));
+                    }
+                    __syncwarp();
+                }
+                if (ok && ptx::elect_one()) ptx::tc_commit_pair(bar(kBarAccFull));
+                __syncwarp();
             }
-            if (!ok) NF4_REPORT_FAILURE(g_prefill_error, g_prefill_error_host, 2);
+            if (!ok && lane == 0) NF4_REPORT_FAILURE(g_prefill_error, g_prefill_error_host, 2);
         }
     } else if (warp < 6 || warp >= kFirstEpilogueWarpB) {
         // ============================== epilogue ==============================
         // The MMAs of the next tile wait for the accumulator, so it is read out as fast as eight
         // warps can (two per TMEM lane quarter, each taking half of the columns): the whole tile
-        // (bf16) or half of it (f32) goes through one 64 KB staging buffer, two TMEM loads in
+        // (bf16) or half of it (f32) goes through one staging buffer, two TMEM loads in
         // flight per warp, and the accumulator is handed back before the last values are
-        // converted; the TMA store of the tile then overlaps the next tile's MMAs.
+        // converted; the TMA store of the last values then overlaps the next tile's MMAs.
         const uint32_t set = warp >= kFirstEpilogueWarpB ? 1u : 0u;
         const uint32_t q = warp & 3u;  // TMEM lane quarter this warp may touch
         const uint32_t row_in_tile = q * 32 + lane;
@@ -489,13 +435,14 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         auto col_of = [&](uint32_t k) {
             return (k / kPerPass) * kStageRows + set * kHalfRows + (k % kPerPass) * 16;
         };
+        const uint32_t acc_empty = ptx::map_to_rank(bar(kBarAccEmpty), 0);
         ptx::pdl_wait();  // the rows' factors come from the pre-pass, which also cleared the flags
         float *own_partial = p.partial + (size_t)blockIdx.x * (BM * BN) + row_in_tile;
         for (uint32_t seg = 0; seg < wl.n_seg && ok; ++seg) {
             const uint32_t i = seg;  // the accumulator's barriers alternate per segment
             uint32_t tile, kb, ke;
             wl.get(seg, tile, kb, ke);
-            const uint32_t n0 = (tile / p.m_tiles) * BM, m0 = (tile % p.m_tiles) * BN;
+            const uint32_t n0 = ((tile / p.m_tiles) * 2 + rank) * BM, m0 = (tile % p.m_tiles) * BN;
             const uint32_t n = n0 + row_in_tile;
             if (ke != k_stages) {
                 // The leading stages of a tile that a neighbour finishes: the raw sums go to this
@@ -515,7 +462,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 }
                 ptx::tc_fence_before();
                 __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(bar(kBarAccEmpty));
+                if (lane == 0) ptx::mbar_arrive_cluster(acc_empty);
                 asm volatile("bar.sync 1, 256;" ::: "memory");
                 if (epi_leader) {
                     __threadfence();
@@ -523,14 +470,14 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 }
                 continue;
             }
-            // a tile whose leading stages other CTAs multiplied: the CTAs before this one, back to
-            // the one that began the tile
-            uint32_t first_helper = blockIdx.x;
+            // a tile whose leading stages other pairs multiplied: the pairs before this one, back to
+            // the one that began the tile; a CTA's helpers have its own rank
+            uint32_t first_helper = pair;
             if (kb != 0) {
                 const uint64_t all = (uint64_t)wl.sk_tiles * k_stages, t0 = (uint64_t)tile * k_stages;
                 do {
                     --first_helper;
-                } while (first_helper > 0 && WorkList::range_begin(all, first_helper, gridDim.x) > t0);
+                } while (first_helper > 0 && WorkList::range_begin(all, first_helper, pairs) > t0);
             }
             const float bias = (p.bias && n < p.N) ? __ldg(p.bias + n) : 0.0f;
             // the rows' factors go to shared memory while the MMAs still run: a global load per
@@ -568,8 +515,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             };
             // the helpers' sums for sixteen activation rows of this thread's weight row
             auto add_helpers = [&](uint32_t (&v)[16], uint32_t col) {
-                for (uint32_t h = first_helper; h < blockIdx.x; ++h) {
-                    const float *src = p.partial + (size_t)h * (BM * BN) + (size_t)col * BM + row_in_tile;
+                for (uint32_t h = first_helper; h < pair; ++h) {
+                    const float *src = p.partial + (size_t)(2 * h + rank) * (BM * BN) + (size_t)col * BM + row_in_tile;
                     float part[16];
                     #pragma unroll
                     for (int r = 0; r < 16; ++r) part[r] = __ldcg(src + r * BM);
@@ -577,11 +524,11 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                     for (int r = 0; r < 16; ++r) v[r] = __float_as_uint(__uint_as_float(v[r]) + part[r]);
                 }
             };
-            if (first_helper != blockIdx.x && epi_leader) {
+            if (first_helper != pair && epi_leader) {
                 // bounded wait for the helpers' flags (they dumped before anything else they did)
                 const uint64_t t_begin = ptx::global_timer_ns();
-                for (uint32_t h = first_helper; h < blockIdx.x && ok; ++h) {
-                    while (ptx::ld_acquire_gpu_u32(p.sk_flags + h) == 0u) {
+                for (uint32_t h = first_helper; h < pair && ok; ++h) {
+                    while (ptx::ld_acquire_gpu_u32(p.sk_flags + 2 * h + rank) == 0u) {
                         if (ptx::global_timer_ns() - t_begin > (uint64_t)p.wait_ns) {
                             ok = false;
                             break;
@@ -600,25 +547,26 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 }
                 ptx::tmem_wait_ld();
                 tmem_ld16(acc_lane + col_of(k + 1), vb);
-                if (first_helper != blockIdx.x) add_helpers(va, col_of(k));
+                if (first_helper != pair) add_helpers(va, col_of(k));
                 stage_chunk(va, col_of(k));
                 ptx::tmem_wait_ld();
-                if (first_helper != blockIdx.x) add_helpers(vb, col_of(k + 1));
+                if (first_helper != pair) add_helpers(vb, col_of(k + 1));
                 if (k + 2 < kLoads) {
                     tmem_ld16(acc_lane + col_of(k + 2), va);
                 } else {
                     // this warp's part of the accumulator is read: hand it back to the MMA threads
                     ptx::tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) ptx::mbar_arrive(bar(kBarAccEmpty));
+                    if (lane == 0) ptx::mbar_arrive_cluster(acc_empty);
                 }
                 stage_chunk(vb, col_of(k + 1));
                 if ((k + 2) % kPerPass == 0) {
                     ptx::fence_proxy_async();
                     asm volatile("bar.sync 1, 256;" ::: "memory");
-                    if (epi_leader) {
-                        ptx::tma_store_2d(&tmap_y, ptx::smem_addr(epi), (int32_t)n0,
-                                          (int32_t)(m0 + (k / kPerPass) * kStageRows));
+                    // (an odd number of 128-row tiles: the last odd CTA's rows do not exist)
+                    const uint32_t m = m0 + (k / kPerPass) * kStageRows;
+                    if (epi_leader && n0 < p.N && m < p.M) {
+                        ptx::tma_store_2d(&tmap_y, own | kEpiAt, (int32_t)n0, (int32_t)m);
                         ptx::tma_store_commit();
                     }
                 }
@@ -637,125 +585,159 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         const uint32_t q = warp & 3u;
         const uint32_t row_in_tile = q * 32 + lane;
         if (PERK) ptx::pdl_wait();  // the weight is repacked by a kernel that completes before the pre-pass does
-        const LevelTables tables = make_level_tables();
+        const uint32_t lane_word = lane * 4u | kTableAt | own;  // bytes {4 lane, 0, 1, rank}: see level_pair
         // block scales are used divided by a power of two (see weight_exponent)
         // ... and enter the product as f16: one multiplication from the loaded value.  (A u8 code's scale is
         // (code / 255) * scale of scales; dividing once instead of per code moves it by an ulp of f32.)
         const float w_down = ldexpf(1.0f, -weight_exponent(p.absmax, p.scale_codes, p.scale_of_scales));
         const float scale_unit = p.absmax ? w_down : __fdiv_rn(__ldg(p.scale_of_scales), 255.0f) * w_down;
         const uint32_t blocks_per_row = p.K / 64;
-        const uint32_t total = (uint32_t)(wl.u1 - wl.u0) + p.dp_rounds * k_stages;  // main stages of this CTA
         const uint32_t lane_base = tmem_a + ((q * 32) << 16);
 
-        // Stage positions are walked, not divided out: a 64-bit division per stage costs more
-        // than the expansion itself.
+        // The scales of this group's next kDepth stages are in flight.  A position is walked, not divided out.
+        constexpr int kDepth = 3;
         struct Pos {
-            uint32_t cnt, seg, ks, ke, n;  // running main-stage number, segment, stage in tile, the segment's end, weight row
-        };
-        auto enter = [&](Pos &pos, uint32_t over) {  // to segment pos.seg, `over` stages in
-            uint32_t tile, kb, ke;
-            wl.get(pos.seg, tile, kb, ke);
-            pos.ks = kb + over;
-            pos.ke = ke;
-            pos.n = (tile / p.m_tiles) * BM + row_in_tile;
-        };
-        auto settle = [&](Pos &pos) {
-            while (pos.ks >= pos.ke) {
-                const uint32_t over = pos.ks - pos.ke;
-                if (++pos.seg >= wl.n_seg) {  // past the last segment
-                    pos.cnt = total;
+            uint32_t seg, ks, ke;  // segment, stage in tile, the segment's end
+            uint32_t before;       // stages before the segments after this one
+            size_t row;            // index of the weight row's first scale (PERK: of the pair for this lane)
+        } ahead{0, 0, 0, 0, 0};
+        auto enter = [&]() {  // the first main stage of this group in segment ahead.seg or a later one
+            for (; ahead.seg < wl.n_seg; ++ahead.seg) {
+                uint32_t tile, kb;
+                wl.get(ahead.seg, tile, kb, ahead.ke);
+                ahead.ks = kb + ((group - ahead.before) & (kExpanderGroups - 1u));
+                ahead.before += (ahead.ke - kb) + (ahead.ke == k_stages ? lora_stages : 0);
+                if (ahead.ks < ahead.ke) {
+                    // (rows beyond the last read its scales; nobody stores what comes of them)
+                    const uint32_t n0 = ((tile / p.m_tiles) * 2 + rank) * BM;
+                    ahead.row = PERK ? (size_t)(min(n0 + q * 32, p.N - 1) >> 6) * (p.K / 2) + lane
+                                     : (size_t)min(n0 + row_in_tile, p.N - 1) * blocks_per_row;
                     return;
                 }
-                enter(pos, over);
             }
         };
-        auto advance = [&](Pos &pos) {
-            pos.cnt += kExpanderGroups;
-            pos.ks += kExpanderGroups;
-            settle(pos);
-        };
-        auto fetch = [&](const Pos &pos, RowStage &rs) {
-            rs.c0 = rs.c1 = make_uint4(0, 0, 0, 0);
-            rs.scale = 0;
-            if (pos.cnt >= total) return;
-            const uint32_t ks = pos.ks, n = pos.n;
-            if (n >= p.N) return;
-            const uint4 *src = reinterpret_cast<const uint4 *>(
-                p.codes + (size_t)n * (p.K / 2) + (size_t)ks * 32);
-            rs.c0 = __ldg(src);
-            rs.c1 = __ldg(src + 1);
-            if constexpr (PERK) {
-                // the warp's 32 weight rows lie in one 64-block of the original rows: one 128-byte
-                // line of scales for the stage, a pair per lane
-                const uint32_t *line = reinterpret_cast<const uint32_t *>(
-                    p.scales_t + (size_t)((n - lane) >> 6) * p.K + (size_t)ks * BK);
-                rs.scale = __ldg(line + lane);
-            } else {
-                // nothing is computed from the loaded value here: that would wait for the load, the
-                // latency the pipeline is there to hide (half of a dequantiser's time at few rows)
-                const size_t blk = (size_t)n * blocks_per_row + ks;
-                if (p.absmax) rs.scale = __float_as_uint(__ldg(p.absmax + blk));
-                else rs.scale = __ldg(p.scale_codes + blk);
+        // The scale of the next stage as loaded: f32 bits, a u8 code, or (PERK: the warp's 32 weight rows lie in
+        // one 64-block of the original rows) this lane's pair of the stage's 128-byte line of f16 scales.
+        // Nothing is computed from it here: that would wait for the load, the latency the pipeline hides.
+        auto fetch = [&]() -> uint32_t {
+            if (ahead.seg >= wl.n_seg) return 0;
+            uint32_t v;
+            if constexpr (PERK) v = __ldg(reinterpret_cast<const uint32_t *>(p.scales_t) + ahead.row + (size_t)ahead.ks * (BK / 2));
+            else v = p.absmax ? __float_as_uint(__ldg(p.absmax + ahead.row + ahead.ks)) : __ldg(p.scale_codes + ahead.row + ahead.ks);
+            ahead.ks += kExpanderGroups;
+            if (ahead.ks >= ahead.ke) {
+                ++ahead.seg;
+                enter();
             }
+            return v;
         };
-        auto emit = [&](const Pos &pos, const RowStage &rs) -> bool {
-            const uint32_t cnt = pos.cnt;
-            const uint32_t s = cnt % kAStages, ph = (cnt / kAStages) & 1u;
-            const uint32_t dst = lane_base + s * kAStageCols;
-            uint32_t lo[16], hi[16];
-            if constexpr (PERK) {
-                expand_half_per_k(tables, rs.c0, rs.scale, 0, lo);
-                expand_half_per_k(tables, rs.c1, rs.scale, 16, hi);
-            } else {
-                const float scale = (p.absmax ? __uint_as_float(rs.scale) : (float)rs.scale) * scale_unit;
-                expand_half(tables, rs.c0, scale, lo);
-                expand_half(tables, rs.c1, scale, hi);
-            }
-            if (!ptx::mbar_wait_suspended(bar(kBarAEmpty + s), ph ^ 1u)) return false;
-            ptx::tc_fence_after();
-            tmem_st32(dst, lo, hi);
-            ptx::tmem_wait_st();
-            ptx::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(bar(kBarAFull + s));
-            return true;
-        };
-
-        // software pipeline over this group's stages (group, group + 4, group + 8, ...): the
-        // loads of a stage are in flight while the stages before it are expanded
-        constexpr int kDepth = 2;
-        Pos pe{group, 0, 0, 0, 0};
-        if (wl.n_seg == 0) pe.cnt = total;
-        else {
-            enter(pe, group);
-            settle(pe);
-        }
-        Pos pf = pe;
-        RowStage rs[kDepth];
+        enter();
+        uint32_t scales[kDepth];
         #pragma unroll
-        for (int d = 0; d < kDepth; ++d) {
-            fetch(pf, rs[d]);
-            advance(pf);
-        }
-        while (pe.cnt < total && ok) {
-            #pragma unroll
-            for (int d = 0; d < kDepth; ++d) {
-                if (ok && pe.cnt < total) {
-                    ok = emit(pe, rs[d]);
-                    advance(pe);
-                    fetch(pf, rs[d]);
-                    advance(pf);
+        for (int d = 0; d < kDepth; ++d) scales[d] = fetch();
+        // The codes come in blocks of four stages, one for each group (the first and the last block of a segment
+        // may lack some).  A group has every fourth stage, the adapter's included (nothing to write there, but its turn
+        // on the barriers): then it is never two rounds of Done ahead, where a parity would be the wrong round's.  Every warp goes through every block: it waits for it, takes its row's 32 bytes
+        // of its stage, and gives the slot back.
+        uint32_t before = 0, block = 0;  // stages before the segment, blocks so far
+        const uint32_t row_at = (own | kCodesAt) + row_in_tile * 128u;
+        const uint32_t full0 = ptx::map_to_rank(bar(kBarFull), 0);
+        for (uint32_t seg = 0; seg < wl.n_seg && ok; ++seg) {
+            uint32_t tile, kb, ke;
+            wl.get(seg, tile, kb, ke);
+            const uint32_t turn = (group + kb - before) & (kExpanderGroups - 1u);  // this group's stage of a block
+            const uint32_t chunk0 = row_at + (((turn * 2) ^ (row_in_tile & 7u)) << 4), chunk1 = row_at + (((turn * 2 + 1) ^ (row_in_tile & 7u)) << 4);
+            for (uint32_t ks = (kb & ~(kExpanderGroups - 1u)) + turn; (ks & ~(kExpanderGroups - 1u)) < ke; ks += kExpanderGroups, ++block) {
+                const uint32_t slot = block % kCodeSlots;
+                if (!ptx::mbar_wait_suspended(bar(kBarCFull + slot), (block / kCodeSlots) & 1u)) {
+                    ok = false;
+                    break;
                 }
+                const bool mine = ks >= kb && ks < ke;
+                uint32_t w[8];
+                if (mine) {
+                    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(chunk0 + slot * kCodeTileBytes));
+                    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                                 : "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "r"(chunk1 + slot * kCodeTileBytes));
+                }
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(bar(kBarCEmpty + slot));
+                if (!mine) continue;
+                const uint32_t cnt = before + ks - kb, s = cnt % kAStages;
+                uint32_t scale2 = scales[0];
+                if constexpr (!PERK) {
+                    const __half2 h = __float2half2_rn((p.absmax ? __uint_as_float(scale2) : (float)scale2) * scale_unit);
+                    scale2 = *reinterpret_cast<const uint32_t *>(&h);
+                }
+                #pragma unroll
+                for (int d = 0; d + 1 < kDepth; ++d) scales[d] = scales[d + 1];
+                scales[kDepth - 1] = fetch();
+                uint32_t lo[16], hi[16];
+                expand_half<PERK>(w, scale2, 0, lane_word, lo);
+                expand_half<PERK>(w + 4, scale2, 16, lane_word, hi);
+                if (cnt >= kAStages && !ptx::mbar_wait_suspended(bar(kBarDone + s), ((cnt / kAStages) & 1u) ^ 1u)) {
+                    ok = false;
+                    break;
+                }
+                ptx::tc_fence_after();
+                tmem_st32(lane_base + s * kAStageCols, lo, hi);
+                ptx::tmem_wait_st();
+                ptx::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive_cluster(full0 + 8u * s);
             }
+            before += ke - kb;
+            if (ke != k_stages) continue;
+            for (uint32_t cnt = before + ((group - before) & (kExpanderGroups - 1u)); cnt < before + lora_stages && ok; cnt += kExpanderGroups) {
+                const uint32_t s = cnt % kAStages;
+                ok = cnt < kAStages || ptx::mbar_wait_suspended(bar(kBarDone + s), ((cnt / kAStages) & 1u) ^ 1u);
+                __syncwarp();
+                if (ok && lane == 0) ptx::mbar_arrive_cluster(full0 + 8u * s);
+            }
+            before += lora_stages;
         }
         if (!ok && lane == 0) NF4_REPORT_FAILURE(g_prefill_error, g_prefill_error_host, 4);
     }
 
+    if (warp == kCodeWarp && lane == 0) {
+        // ========================= packed codes =========================
+        // Blocks of four k-stages of this CTA's 128 weight rows; the L2 is asked for a block a few ahead of
+        // its load (weights that nobody has touched yet come from HBM).
+        if (PERK) ptx::pdl_wait();
+        constexpr uint32_t kAhead = 6;
+        uint32_t block = 0;
+        for (uint32_t seg = 0; seg < wl.n_seg && ok; ++seg) {
+            uint32_t tile, kb, ke;
+            wl.get(seg, tile, kb, ke);
+            const int32_t n0 = (int32_t)(((tile / p.m_tiles) * 2 + rank) * BM);
+            const uint32_t b0 = kb / kCodeStages, b1 = (ke + kCodeStages - 1) / kCodeStages;
+            for (uint32_t b = b0; b < min(b1, b0 + kAhead); ++b) ptx::tma_prefetch_2d(&tmap_w, (int32_t)(b * 128), n0);
+            for (uint32_t b = b0; b < b1; ++b, ++block) {
+                const uint32_t slot = block % kCodeSlots;
+                if (b + kAhead < b1) ptx::tma_prefetch_2d(&tmap_w, (int32_t)((b + kAhead) * 128), n0);
+                if (!ptx::mbar_wait_suspended(bar(kBarCEmpty + slot), ((block / kCodeSlots) & 1u) ^ 1u)) {
+                    ok = false;
+                    break;
+                }
+                ptx::mbar_arrive_expect_tx(bar(kBarCFull + slot), kCodeTileBytes);
+                ptx::tma_load_2d((own | kCodesAt) + slot * kCodeTileBytes, &tmap_w, (int32_t)(b * 128), n0, bar(kBarCFull + slot));
+            }
+        }
+        if (!ok) {
+            for (uint32_t c = block > kCodeSlots ? block - kCodeSlots : 0; c < block; ++c)
+                ptx::mbar_wait_suspended(bar(kBarCFull + c % kCodeSlots), (c / kCodeSlots) & 1u);
+            NF4_REPORT_FAILURE(g_prefill_error, g_prefill_error_host, 7);
+        }
+    }
+
+    __syncwarp();
+    // neither CTA leaves, or gives its tensor memory back, while the other may still signal it
     ptx::tc_fence_before();
-    __syncthreads();
+    ptx::cluster_sync_all();
     if (warp == 1) {
         ptx::tc_fence_after();
-        ptx::tmem_dealloc(tmem_base, kTmemCols);
+        ptx::tmem_dealloc_pair(tmem_base, kTmemCols);
     }
 }
 
@@ -958,31 +940,31 @@ bool prefill_supported(const nf4_linear_args &a) {
 }
 
 namespace {
-// How the tiles are shared out: `grid` CTAs; the first `sk_tiles` tiles are divided by k-stages
-// (every CTA the same number of stages, a tile possibly split between neighbours), the other
-// grid * dp_rounds tiles go out whole.  With a tile count that is a multiple of the grid nothing
-// is split.  Otherwise the last round of whole tiles would leave most CTAs idle (896 tiles on 148
-// CTAs: seven rounds for 6.05 rounds of work), so the last full round and the remainder are
-// divided by stages instead.  Fewer tiles than SMs: divided as long as a CTA keeps 24 stages.
+// How the tiles are shared out between the pairs of CTAs: the first `sk_tiles` tiles are divided by k-stages
+// (every pair the same number of stages, a tile possibly split between neighbours), the other
+// pairs * dp_rounds tiles go out whole.  With a tile count that is a multiple of the pairs nothing
+// is split.  Otherwise the last round of whole tiles would leave most pairs idle, so the last full round and
+// the remainder are divided by stages instead.  Fewer tiles than pairs: divided as long as a pair keeps 24
+// stages.
 struct Sharing {
-    uint32_t grid, sk_tiles, dp_rounds;
+    uint32_t pairs, sk_tiles, dp_rounds;
 };
 Sharing share_tiles(uint64_t rows, uint64_t d_in, uint64_t d_out) {
-    const uint64_t tiles = ((rows + BN - 1) / BN) * ((d_out + BM - 1) / BM), ks = d_in / BK;
+    const uint64_t tiles = ((rows + BN - 1) / BN) * ((d_out + 2 * BM - 1) / (2 * BM)), ks = d_in / BK;
     Sharing sh;
-    uint64_t grid = kNumSMs;
-    if (tiles < grid) {
+    uint64_t pairs = kNumSMs / 2;
+    if (tiles < pairs) {
         const uint64_t by_stages = tiles * ks / 24;
-        grid = by_stages < grid ? by_stages : grid;
-        if (grid < tiles) grid = tiles;
+        pairs = by_stages < pairs ? by_stages : pairs;
+        if (pairs < tiles) pairs = tiles;
     }
-    sh.grid = (uint32_t)grid;
-    if (tiles % grid == 0) {
+    sh.pairs = (uint32_t)pairs;
+    if (tiles % pairs == 0) {
         sh.sk_tiles = 0;
-        sh.dp_rounds = (uint32_t)(tiles / grid);
+        sh.dp_rounds = (uint32_t)(tiles / pairs);
     } else {
-        sh.dp_rounds = tiles / grid >= 1 ? (uint32_t)(tiles / grid - 1) : 0u;
-        sh.sk_tiles = (uint32_t)(tiles - (uint64_t)sh.dp_rounds * grid);
+        sh.dp_rounds = tiles / pairs >= 1 ? (uint32_t)(tiles / pairs - 1) : 0u;
+        sh.sk_tiles = (uint32_t)(tiles - (uint64_t)sh.dp_rounds * pairs);
     }
     return sh;
 }
@@ -1004,8 +986,8 @@ WorkspaceLayout workspace_layout(uint64_t rows, uint64_t d_in, uint64_t d_out, u
     w.off_t = w.off_scale + up(rows * 4);
     w.off_flags = w.off_t + up(rows * 2ull * 64 * lora_chunks_of(lora_rank) * 2);
     const Sharing sh = share_tiles(rows, d_in, d_out);
-    w.off_partial = w.off_flags + up((uint64_t)sh.grid * 4);
-    w.bytes = w.off_partial + (sh.sk_tiles ? (uint64_t)sh.grid * BM * BN * 4 : 0);
+    w.off_partial = w.off_flags + up((uint64_t)sh.pairs * 8);
+    w.bytes = w.off_partial + (sh.sk_tiles ? (uint64_t)sh.pairs * 2 * BM * BN * 4 : 0);
     w.off_codes_t = w.off_scales_t = w.off_a_t = w.off_b_t = 0;
     if (extra >= kFactors) {  // `lora_rank` is the rank the GEMM sees (twice the adapter's for f32 factors)
         w.off_a_t = up(w.bytes);
@@ -1068,7 +1050,6 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_o
     if (x_f32) p.rank *= 2;  // see repack_adapter_block
     p.lora_chunks = lora_chunks_of(p.rank);
     p.m_tiles = (p.M + BN - 1) / BN;
-    p.n_tiles = (p.N + BM - 1) / BM;
     const uint64_t ldy = a.ldy ? a.ldy : a.d_out;
 
     const WorkspaceLayout wl = workspace_layout(p.M, p.K, p.N, p.rank, extra);
@@ -1140,18 +1121,19 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_o
     pre.scale_codes = a.scale_codes;
     pre.scale_of_scales = a.scale_of_scales;
     pre.flags = p.sk_flags;
-    pre.n_flags = sh.grid;
+    pre.n_flags = 2 * sh.pairs;
     // (f32 factors reach the pre-pass through the repacking launch: then it has to wait for it)
     pre.beside_predecessor = packing && !(x_f32 && p.rank);
     NF4_TRY(activations_prepass(pre, stream));
 
-    CUtensorMap map_x, map_t, map_b, map_y;
-    NF4_TRY(make_map(&map_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, xh, p.M, p.K, (uint64_t)p.K * 2, BN, BK,
+    CUtensorMap map_x, map_t, map_b, map_y, map_w;
+    NF4_TRY(make_map(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, p.codes, p.N, p.K / 2, p.K / 2, BM, 128, CU_TENSOR_MAP_SWIZZLE_128B));
+    NF4_TRY(make_map(&map_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, xh, p.M, p.K, (uint64_t)p.K * 2, BN / 2, BK,
                      CU_TENSOR_MAP_SWIZZLE_128B));
     map_t = map_b = map_x;
     if (p.rank) {
         const uint32_t ld_t = 2 * 64 * p.lora_chunks;
-        NF4_TRY(make_map(&map_t, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, t, p.M, ld_t, (uint64_t)ld_t * 2, BN,
+        NF4_TRY(make_map(&map_t, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, t, p.M, ld_t, (uint64_t)ld_t * 2, BN / 2,
                          BK, CU_TENSOR_MAP_SWIZZLE_128B));
         // LoRA B [N][rank]: columns beyond the rank and rows beyond N read as zero
         NF4_TRY(make_map(&map_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, lora_b, p.N, p.rank,
@@ -1164,13 +1146,10 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_o
         NF4_TRY(make_map(&map_y, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.y, p.M, p.N, ldy * 2, kEpiBytes / (BM * 2), BM,
                          CU_TENSOR_MAP_SWIZZLE_NONE));
 
-    const uint32_t grid = sh.grid;
-    const size_t smem = 1024 + kXStages * kXTileBytes + kLoraStages * kLoraTileBytes + kEpiBytes +
-                        kNumBars * 8 + 16 + BN * 4 + 64;
     auto go = [&](auto kernel) -> int32_t {
-        NF4_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), (int)smem));
-        return launch_maybe_overlapped(kernel, dim3(grid), dim3(kThreads), smem, stream, true, map_x, map_t, map_b,
-                                       map_y, p);
+        NF4_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), (int)kDynamicSmem));
+        return launch_maybe_overlapped(kernel, dim3(2 * sh.pairs), dim3(kThreads), kDynamicSmem, stream, true, map_x, map_t, map_b,
+                                       map_y, map_w, p);
     };
     if (repacked) NF4_TRY(y_f32 ? go(prefill_kernel<true, true>) : go(prefill_kernel<false, true>));
     else NF4_TRY(y_f32 ? go(prefill_kernel<true, false>) : go(prefill_kernel<false, false>));
@@ -1183,28 +1162,36 @@ int32_t prefill_set_host_flag(int *mapped) {
     return check_cuda(cudaMemcpyToSymbol(g_prefill_error_host, &mapped, sizeof(mapped)), "setting the mapped failure word");
 }
 
-// The sharing of the tiles as the kernel will see it, for inspection on the host: the number of
-// CTAs and, for CTA `cta`, its segments (tile, first main k-stage, one past the last) in the order
-// it works on them.  Returns the number of segments (at most `cap` are written), or -1.
+// The sharing of the tiles as the kernel will see it, for inspection on the host, in tiles of 128 weight rows x
+// 256 activation rows, one CTA's part of a pair's tile.  CTAs are counted with the even ones of all pairs
+// first: CTA `cta` is CTA cta / pairs of pair cta % pairs.  Returns the number of the CTA's segments (at
+// most `cap` are written), or -1.
 int32_t prefill_share_plan(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t cta, uint32_t *ctas,
                            uint32_t *segments, uint32_t cap) {
     if (rows <= 16 || d_in % BK != 0 || d_in == 0 || d_out == 0) return -1;
     const Sharing sh = share_tiles(rows, d_in, d_out);
-    if (ctas) *ctas = sh.grid;
-    if (cta >= sh.grid) return -1;
+    if (ctas) *ctas = 2 * sh.pairs;
+    if (cta >= 2 * sh.pairs) return -1;
+    const uint32_t rank = cta / sh.pairs, m_tiles = (uint32_t)((rows + BN - 1) / BN);
     PrefillParams p{};
     p.sk_tiles = sh.sk_tiles;
     p.dp_rounds = sh.dp_rounds;
     WorkList wl;
-    wl.init(p, (uint32_t)(d_in / BK), cta, sh.grid);
-    for (uint32_t j = 0; j < wl.n_seg && j < cap; ++j) {
+    wl.init(p, (uint32_t)(d_in / BK), cta % sh.pairs, sh.pairs);
+    uint32_t n = 0;
+    for (uint32_t j = 0; j < wl.n_seg; ++j) {
         uint32_t tile, b, e;
         wl.get(j, tile, b, e);
-        segments[3 * j] = tile;
-        segments[3 * j + 1] = b;
-        segments[3 * j + 2] = e;
+        const uint32_t n_tile = tile / m_tiles * 2 + rank;
+        if ((uint64_t)n_tile * BM >= d_out) continue;  // the odd CTA of the last pair of an odd number of tiles: no rows
+        if (n < cap) {
+            segments[3 * n] = n_tile * m_tiles + tile % m_tiles;
+            segments[3 * n + 1] = b;
+            segments[3 * n + 2] = e;
+        }
+        ++n;
     }
-    return (int32_t)wl.n_seg;
+    return (int32_t)n;
 }
 
 int32_t prefill_error_flag_ptr(int **dev_ptr) {

@@ -67,10 +67,10 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
 // back at once when the phase is not complete and the loop around it competes for issue).
 __device__ __forceinline__ bool mbar_wait_suspended(uint32_t bar, uint32_t parity,
                                                     uint32_t suspend_ns = 4000) {
-    // (the usual case first: reading the global timer takes longer than a wait that is already over)
+    // (the timer is read late: a read takes longer than most of the waits)
     if (mbar_try_wait(bar, parity)) return true;
-    const uint64_t t0 = global_timer_ns();
-    for (;;) {
+    uint64_t t0 = 0;
+    for (uint32_t i = 0;; ++i) {
         uint32_t ok;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -80,7 +80,8 @@ __device__ __forceinline__ bool mbar_wait_suspended(uint32_t bar, uint32_t parit
             : "r"(bar), "r"(parity), "r"(suspend_ns)
             : "memory");
         if (ok) return true;
-        if (global_timer_ns() - t0 > 1000000000ull) return false;
+        if (i == 8) t0 = global_timer_ns();
+        else if (i > 8 && global_timer_ns() - t0 > 1000000000ull) return false;
     }
 }
 
@@ -145,6 +146,18 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst_smem, const void *tmap,
         "[%0], [%1, {%2, %3}], [%4];"
         ::"r"(dst_smem), "l"(tmap), "r"(x), "r"(y), "r"(bar)
         : "memory");
+}
+// Half of a CTA pair's operand: into this CTA's shared memory, counted by a barrier of either CTA.
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst_smem, const void *tmap, int32_t x, int32_t y, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 "
+        "[%0], [%1, {%2, %3}], [%4];"
+        ::"r"(dst_smem), "l"(tmap), "r"(x), "r"(y), "r"(bar)
+        : "memory");
+}
+// Asks the L2 for a box that will be loaded later.
+__device__ __forceinline__ void tma_prefetch_2d(const void *tmap, int32_t x, int32_t y) {
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(tmap), "r"(x), "r"(y) : "memory");
 }
 __device__ __forceinline__ void tma_store_2d(const void *tmap, uint32_t src_smem, int32_t x,
                                              int32_t y) {
@@ -246,6 +259,64 @@ __device__ __forceinline__ void tmem_wait_ld() {
 }
 __device__ __forceinline__ void tmem_wait_st() {
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+// ---- CTA pairs ------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_cta_rank() {
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// Every thread of both CTAs; what was written before is visible after.
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The shared::cluster address of this CTA's shared-memory address `addr` in CTA `rank`.
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+// Arrive on a barrier of the other CTA.  No cluster-wide release: what the arrivals of the tensor-core
+// path announce (tensor memory read or written, bulk copies landed) is complete when they are made, and a
+// release at cluster scope took 1400 cycles each time.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+
+// tcgen05 for a pair: the CTAs' tensor memory holds the two halves of A's and D's 256 rows at the same
+// addresses, their shared memory the two halves of B's columns at the same offsets; one thread of the
+// even CTA issues.  Allocation is collective over the pair (one warp of each CTA).
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_smem, uint32_t ncols) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish_pair() {
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void mma_ts_f16_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void mma_ss_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// Arrive on the barrier at this offset in both CTAs once every pair operation issued so far by this thread is done.
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(bar), "h"((uint16_t)3)
+                 : "memory");
 }
 
 // Programmatic dependent launch: the pre-pass lets its dependent start early; the dependent
