@@ -654,16 +654,15 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                     break;
                 }
                 const bool mine = ks >= kb && ks < ke;
-                uint32_t w[8];
-                if (mine) {
-                    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-                                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(chunk0 + slot * kCodeTileBytes));
-                    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-                                 : "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "r"(chunk1 + slot * kCodeTileBytes));
+                if (!mine) {
+                    if (lane == 0) ptx::mbar_arrive(bar(kBarCEmpty + slot));
+                    continue;
                 }
-                __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(bar(kBarCEmpty + slot));
-                if (!mine) continue;
+                uint32_t w[8];
+                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                             : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(chunk0 + slot * kCodeTileBytes) : "memory");
+                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                             : "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "r"(chunk1 + slot * kCodeTileBytes) : "memory");
                 const uint32_t cnt = before + ks - kb, s = cnt % kAStages;
                 uint32_t scale2 = scales[0];
                 if constexpr (!PERK) {
@@ -685,7 +684,12 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 ptx::tmem_wait_st();
                 ptx::tc_fence_before();
                 __syncwarp();
-                if (lane == 0) ptx::mbar_arrive_cluster(full0 + 8u * s);
+                if (lane == 0) {
+                    ptx::mbar_arrive_cluster(full0 + 8u * s);
+                    // The slot goes back now that what was read from it has been used.  Right after the loads
+                    // were issued is too early: the next copy, of another proxy, was seen to overtake them.
+                    ptx::mbar_arrive(bar(kBarCEmpty + slot));
+                }
             }
             before += ke - kb;
             if (ke != k_stages) continue;
