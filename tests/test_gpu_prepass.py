@@ -42,6 +42,10 @@ def rel(got, ref):
     (70, 4160, 64, 4, 1, True),
     (20, 65536, 64, 8, 0, False),      # K in several pieces of shared memory
     (18, 40960, 64, 8, 0, True),
+    (513, 192, 136, 8, 0, False),      # 64 rows to a tile: one row in the last, stages of 128 k half empty
+    (600, 1088, 128, 20, 1, False),    # the same, the factor [K, r] in odd places
+    (545, 576, 64, 12, 0, True),       # f32, 64 rows to a tile
+    (1200, 2112, 64, 40, 1, True),
 ])
 def test_forward(M, K, N, r, layout, f32):
     dt = torch.float32 if f32 else torch.bfloat16

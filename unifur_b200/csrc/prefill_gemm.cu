@@ -1126,8 +1126,8 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_o
     pre.scale_of_scales = a.scale_of_scales;
     pre.flags = p.sk_flags;
     pre.n_flags = 2 * sh.pairs;
-    // (f32 factors reach the pre-pass through the repacking launch: then it has to wait for it)
-    pre.beside_predecessor = packing && !(x_f32 && p.rank);
+    pre.beside_predecessor = packing;
+    pre.factor_of_predecessor = x_f32 && p.rank;  // (f32 factors come through the repacking launch)
     NF4_TRY(activations_prepass(pre, stream));
 
     CUtensorMap map_x, map_t, map_b, map_y, map_w;
