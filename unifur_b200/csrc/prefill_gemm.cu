@@ -762,48 +762,67 @@ struct RepackParams {
     __nv_bfloat16 *b_t;
     uint32_t K, N, r;
     int32_t factors_out_in;     // the factors come as A [r][K], B [N][r] (else A [K][r], B [r][N])
-    uint32_t code_cols, code_rows, code_blocks;   // CTAs of the nibbles: columns of 128 n x groups of kRepackTiles k-tiles
+    uint32_t code_cols, code_blocks;              // CTAs of the nibbles: tiles of 128 n x 256 k
     uint32_t scale_cols, scale_blocks;            // CTAs of the scales: 32 x 32 tiles
-    uint32_t adapter_blocks;
+    uint32_t a_blocks, adapter_blocks;            // CTAs of the factors: 32 x 32 tiles, A's first
 };
-constexpr uint32_t kRepackTiles = 4;  // 64-row tiles of nibbles one CTA walks, the next one's loads in flight
 
-// Nibbles: 64 rows (k) x 128 columns (n) per tile through shared memory; a thread turns 16 rows of
-// one byte column (two n) into the 8 bytes each of those two weight rows gets.
-__device__ __forceinline__ void repack_codes_block(const RepackParams &p, uint32_t block, uint8_t (*tile)[64][80]) {
-    const uint32_t n0 = (block % p.code_cols) * 128, kt0 = (block / p.code_cols) * kRepackTiles, t = threadIdx.x;
-    const uint32_t k_tiles = p.K / 64;
-    const uint32_t n_it = min(kRepackTiles, k_tiles - kt0);
-    const uint32_t r = t >> 2, seg = t & 3u;  // loads: 16 bytes = 32 columns of row r per thread
-    const bool in = n0 + seg * 32 < p.N;
-    auto load = [&](uint32_t it) {
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (in)
-            v = __ldg(reinterpret_cast<const uint4 *>(p.codes + (size_t)((kt0 + it) * 64 + r) * (p.N / 2) + n0 / 2 +
-                                                      seg * 16));
-        return v;
-    };
-    const uint32_t bc = t & 63u, kq = t >> 6;  // byte column and quarter of the rows
-    uint4 v = load(0);
-    for (uint32_t it = 0; it < n_it; ++it) {
-        uint8_t(*cur)[80] = tile[it & 1u];
-        *reinterpret_cast<uint4 *>(&cur[r][seg * 16]) = v;
-        __syncthreads();
-        if (it + 1 < n_it) v = load(it + 1);
-        if (n0 + 2 * bc < p.N) {
-            uint32_t e0 = 0, e1 = 0, o0 = 0, o1 = 0;  // even column: k 0..7, 8..15 of the quarter; odd column
-            #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const uint32_t b0 = cur[kq * 16 + j][bc], b1 = cur[kq * 16 + 8 + j][bc];
-                e0 |= (b0 & 15u) << (4 * j);
-                o0 |= (b0 >> 4) << (4 * j);
-                e1 |= (b1 & 15u) << (4 * j);
-                o1 |= (b1 >> 4) << (4 * j);
-            }
-            const size_t at = (size_t)(n0 + 2 * bc) * (p.K / 2) + ((kt0 + it) * 64 + kq * 16) / 2;
-            *reinterpret_cast<uint2 *>(p.codes_t + at) = make_uint2(e0, e1);
-            *reinterpret_cast<uint2 *>(p.codes_t + at + p.K / 2) = make_uint2(o0, o1);
+// Nibbles.  A CTA turns 256 k x 128 n.  A thread takes eight words (8 k x 8 n) straight from global memory, all
+// loads of its two blocks in flight, transposes each in registers (halves and bytes by permutes, nibbles by masks: 32
+// operations for 32 bytes) and leaves the words in shared memory, from where whole 128-byte lines go out.  Bound by the
+// bytes; picking nibbles out of shared memory byte by byte, into 8-byte pieces of lines, took 33 us for 4096 x 14336 with its
+// scales and factors; now 15.
+__device__ __forceinline__ void transpose_nibbles(uint32_t (&w)[8]) {  // nibble c of word j <-> nibble j of word c
+    uint32_t h[8], b[8];
+    #pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        h[j] = __byte_perm(w[j], w[j + 4], 0x5410);      // columns 0-3 of rows j, j + 4
+        h[j + 4] = __byte_perm(w[j], w[j + 4], 0x7632);  // columns 4-7
+    }
+    #pragma unroll
+    for (int c = 0; c < 8; c += 4) {
+        #pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            b[c + j] = __byte_perm(h[c + j], h[c + j + 2], 0x6240);      // columns c, c + 1 of rows j, j + 2, j + 4, j + 6
+            b[c + j + 2] = __byte_perm(h[c + j], h[c + j + 2], 0x7351);  // columns c + 2, c + 3
         }
+    }
+    #pragma unroll
+    for (int c = 0; c < 8; c += 2) {
+        w[c] = (b[c] & 0x0f0f0f0fu) | ((b[c + 1] << 4) & 0xf0f0f0f0u);
+        w[c + 1] = ((b[c] >> 4) & 0x0f0f0f0fu) | (b[c + 1] & 0xf0f0f0f0u);
+    }
+}
+
+__device__ __forceinline__ void repack_codes_block(const RepackParams &p, uint32_t block, uint32_t *tile) {
+    const uint32_t n0 = (block % p.code_cols) * 128, k0 = (block / p.code_cols) * 256, t = threadIdx.x;
+    const uint32_t j = t & 15u, i0 = t >> 4;  // eight columns n0 + 8 j; eight rows k0 + 8 i, i = i0 and i0 + 16
+    const uint8_t *src = p.codes + (size_t)k0 * (p.N / 2) + n0 / 2 + j * 4;
+    uint32_t w[2][8];
+    #pragma unroll
+    for (uint32_t u = 0; u < 2; ++u) {
+        const uint32_t i = i0 + u * 16;
+        const bool in = n0 + j * 8 < p.N && k0 + i * 8 < p.K;  // (both are multiples of 64)
+        #pragma unroll
+        for (uint32_t q = 0; q < 8; ++q)
+            w[u][q] = in ? __ldg(reinterpret_cast<const uint32_t *>(src + (size_t)(i * 8 + q) * (p.N / 2))) : 0u;
+    }
+    // tile[n][i ^ 2 (n / 8)]: a warp's stores (sixteen j, two i) and its loads of pairs hit all banks
+    #pragma unroll
+    for (uint32_t u = 0; u < 2; ++u) {
+        transpose_nibbles(w[u]);
+        #pragma unroll
+        for (uint32_t c = 0; c < 8; ++c) tile[(j * 8 + c) * 32 + ((i0 + u * 16) ^ (2 * j))] = w[u][c];
+    }
+    __syncthreads();
+    const uint32_t pair = t & 15u;
+    if (k0 + pair * 16 >= p.K) return;
+    uint8_t *dst = p.codes_t + (size_t)n0 * (p.K / 2) + k0 / 2 + pair * 8;
+    #pragma unroll
+    for (uint32_t n = t >> 4; n < 128; n += 16) {
+        if (n0 + n >= p.N) break;
+        const uint2 v = *reinterpret_cast<const uint2 *>(tile + n * 32 + ((2 * pair) ^ (2 * (n >> 3))));
+        *reinterpret_cast<uint2 *>(dst + (size_t)n * (p.K / 2)) = v;
     }
 }
 
@@ -838,30 +857,35 @@ __device__ __forceinline__ void repack_scales_block(const RepackParams &p, uint3
 //         bf16 of what that rounding left: as an adapter of rank 2 r whose intermediate holds every
 //         column twice, B enters the product with sixteen bits of mantissa.
 template <class T>
-__device__ __forceinline__ void repack_adapter_block(const RepackParams &p, uint32_t block) {
+__device__ __forceinline__ void repack_adapter_block(const RepackParams &p, uint32_t block, float (*tile)[33]) {
     constexpr bool kF32 = sizeof(T) == 4;
-    const T *a = static_cast<const T *>(p.a), *b = static_cast<const T *>(p.b);
-    const uint32_t r = p.r, rank_out = kF32 ? 2 * r : r;
-    const uint64_t i = (uint64_t)block * blockDim.x + threadIdx.x;
-    const uint64_t na = kF32 ? (uint64_t)r * p.K : 0, nb = (uint64_t)p.N * r;
-    if (i < na) {
-        if constexpr (kF32) {
-            const uint32_t j = (uint32_t)(i / p.K), k = (uint32_t)(i % p.K);
-            const __half h = __float2half_rn(a[p.factors_out_in ? (size_t)j * p.K + k : (size_t)k * r + j]);
-            p.a_t[i] = __half_as_ushort(h);
-            p.a_t[na + i] = __half_as_ushort(h);
-        }
-    } else if (i < na + nb) {
-        const uint64_t e = i - na;
-        const uint32_t n = (uint32_t)(e / r), j = (uint32_t)(e % r);
-        const size_t at = p.factors_out_in ? (size_t)n * r + j : (size_t)j * p.N + n;
-        if constexpr (kF32) {
-            const float v = b[at];
-            const __nv_bfloat16 hi = __float2bfloat16_rn(v);
-            p.b_t[(size_t)n * rank_out + j] = hi;
-            p.b_t[(size_t)n * rank_out + r + j] = __float2bfloat16_rn(v - __bfloat162float(hi));
+    const bool is_a = block < p.a_blocks;
+    if (!is_a) block -= p.a_blocks;
+    // a tile of 32 x 32 of the result [rows][cols]: A's rows are ranks, B's columns
+    const T *src = static_cast<const T *>(is_a ? p.a : p.b);
+    const uint32_t rows = is_a ? p.r : p.N, cols = is_a ? p.K : p.r, col_tiles = (cols + 31) / 32;
+    const uint32_t r0 = block / col_tiles * 32, c0 = block % col_tiles * 32, tx = threadIdx.x & 31u, ty = threadIdx.x >> 5;
+    #pragma unroll
+    for (uint32_t q = ty; q < 32; q += 8) {
+        const uint32_t r = r0 + (p.factors_out_in ? q : tx), c = c0 + (p.factors_out_in ? tx : q);
+        float v = 0.0f;
+        if (r < rows && c < cols) v = (float)src[p.factors_out_in ? (size_t)r * cols + c : (size_t)c * rows + r];
+        tile[r - r0][c - c0] = v;
+    }
+    __syncthreads();
+    #pragma unroll
+    for (uint32_t q = ty; q < 32; q += 8) {
+        const uint32_t r = r0 + q, c = c0 + tx;
+        if (r >= rows || c >= cols) continue;
+        const float v = tile[q][tx];
+        if (is_a) {
+            const uint16_t h = __half_as_ushort(__float2half_rn(v));
+            p.a_t[(size_t)r * cols + c] = h;
+            p.a_t[(size_t)(rows + r) * cols + c] = h;
         } else {
-            p.b_t[(size_t)n * rank_out + j] = b[at];
+            const __nv_bfloat16 hi = __float2bfloat16_rn(v);
+            p.b_t[(size_t)r * (kF32 ? 2 * cols : cols) + c] = hi;
+            if (kF32) p.b_t[(size_t)r * 2 * cols + cols + c] = __float2bfloat16_rn(v - __bfloat162float(hi));
         }
     }
 }
@@ -870,14 +894,14 @@ __device__ __forceinline__ void repack_adapter_block(const RepackParams &p, uint
 // the next scale_blocks the scales, the last adapter_blocks the adapter.  The pre-pass may run beside it.
 template <class T>
 __global__ void __launch_bounds__(256) repack_kernel(const RepackParams p) {
-    __shared__ __align__(16) uint8_t smem[2 * 64 * 80];
+    __shared__ __align__(16) uint32_t smem[128 * 32];
     ptx::pdl_launch_dependents();
     uint32_t b = blockIdx.x;
-    if (b < p.code_blocks) return repack_codes_block(p, b, reinterpret_cast<uint8_t(*)[64][80]>(smem));
+    if (b < p.code_blocks) return repack_codes_block(p, b, smem);
     b -= p.code_blocks;
     if (b < p.scale_blocks) return repack_scales_block(p, b, reinterpret_cast<float(*)[33]>(smem));
     b -= p.scale_blocks;
-    repack_adapter_block<T>(p, b);
+    repack_adapter_block<T>(p, b, reinterpret_cast<float(*)[33]>(smem));
 }
 
 // ---- host side -----------------------------------------------------------------------
@@ -1083,8 +1107,7 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_o
         rp.K = p.K;
         rp.N = p.N;
         rp.code_cols = (p.N + 127) / 128;
-        rp.code_rows = (p.K / 64 + kRepackTiles - 1) / kRepackTiles;
-        rp.code_blocks = repacked ? rp.code_cols * rp.code_rows : 0;
+        rp.code_blocks = repacked ? rp.code_cols * ((p.K + 255) / 256) : 0;
         rp.scale_cols = (p.N / 64 + 31) / 32;
         rp.scale_blocks = repacked ? rp.scale_cols * ((p.K + 31) / 32) : 0;
         if (p.rank) {
@@ -1093,7 +1116,9 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_o
             rp.r = a.lora_rank;
             rp.a_t = reinterpret_cast<uint16_t *>(ws + wl.off_a_t);
             rp.b_t = reinterpret_cast<__nv_bfloat16 *>(ws + wl.off_b_t);
-            rp.adapter_blocks = (uint32_t)(((uint64_t)a.lora_rank * ((x_f32 ? p.K : 0) + (uint64_t)p.N) + 255) / 256);
+            const uint32_t rank_tiles = (a.lora_rank + 31) / 32;
+            rp.a_blocks = x_f32 ? rank_tiles * ((p.K + 31) / 32) : 0;
+            rp.adapter_blocks = rp.a_blocks + rank_tiles * ((p.N + 31) / 32);
             if (x_f32) lora_a = rp.a_t;
             lora_b = rp.b_t;
         }
