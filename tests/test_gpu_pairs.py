@@ -17,6 +17,9 @@ from test_gpu_linear import check_out_in, make_case  # noqa: E402
     (513, 832, 1160, 128, False, False),
     (257, 3008, 392, 256, True, True),  # eight adapter stages behind pieces of a few
     (600, 320, 5000, 256, False, False),  # whole tiles of five stages
+    (33, 2048, 520, 16, False, True),   # MMAs of 64 columns, split tiles with three of sixteen chunks of rows
+    (96, 4096, 264, 64, True, False),   # of 96, both sets of epilogue warps with and without rows
+    (479, 1536, 768, 8, False, False),  # of 224 in the second tile
 ])
 def test_uneven_pairs(oracle, M, K, N, r, dq, bias):
     c = make_case(oracle, 4000 + M + K + N, M, K, N, r, dq=dq, bias=bias)

@@ -174,6 +174,15 @@ struct WorkList {
     }
 };
 
+// Activation rows the MMAs of a tile beginning at row m0 take: all 256, or for the last, ragged tile the rows there are,
+// up to a multiple of 32 (each CTA brings half of them).  An MMA takes as long as it has columns: at 64 rows the
+// k-stage is then bound by the dequantisers (64 x 4096 x 4096, whole call: 41 -> 32 us with the rows that do not exist
+// left out of the split tiles' sums as well; 64 x 14336 x 4096: 54 -> 43).
+__device__ __forceinline__ uint32_t tile_columns(uint32_t M, uint32_t m0) {
+    const uint32_t left = M - m0;
+    return left < BN ? (left + 31) / 32 * 32 : BN;
+}
+
 // ---- descriptors -----------------------------------------------------------------
 // Shared-memory matrix descriptor, K-major operand, 128-byte swizzle: rows are 128 B apart,
 // 8-row groups 1024 B apart (SBO), version 1, layout type 2 (SWIZZLE_128B).
@@ -328,7 +337,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             for (uint32_t seg = 0; seg < wl.n_seg && ok; ++seg) {
                 uint32_t tile, kb, ke;
                 wl.get(seg, tile, kb, ke);
-                const uint32_t m0 = (tile % p.m_tiles) * BN + rank * (BN / 2), n0 = ((tile / p.m_tiles) * 2 + rank) * BM;
+                const uint32_t tile_m0 = (tile % p.m_tiles) * BN, n0 = ((tile / p.m_tiles) * 2 + rank) * BM;
+                const uint32_t m0 = tile_m0 + rank * (tile_columns(p.M, tile_m0) / 2);  // (the box is longer; the MMAs take what counts)
                 // the adapter's stages follow a tile's last main stage
                 const uint32_t k_end = ke == k_stages ? k_stages + lora_stages : ke;
                 for (uint32_t ks = kb; ks < k_end; ++ks, ++cnt) {
@@ -369,12 +379,13 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         // warp stays together and elects the thread where it issues, so that addresses and descriptors are
         // uniform registers; one lane on its own in a branch spent 77 cycles on each MMA, which takes 128.
         if (rank == 0) {
-            constexpr uint32_t idesc_main = make_idesc(0, 0, 2 * BM, BN);  // f16 x f16
-            constexpr uint32_t idesc_lora = make_idesc(1, 1, 2 * BM, BN);  // bf16 x bf16
             uint32_t cnt = 0;
             for (uint32_t seg = 0; seg < wl.n_seg && ok; ++seg) {
                 uint32_t tile, kb, ke;
                 wl.get(seg, tile, kb, ke);
+                const uint32_t columns = tile_columns(p.M, (tile % p.m_tiles) * BN);
+                const uint32_t idesc_main = make_idesc(0, 0, 2 * BM, columns);  // f16 x f16
+                const uint32_t idesc_lora = make_idesc(1, 1, 2 * BM, columns);  // bf16 x bf16
                 // the epilogues must have read the previous segment out of the accumulators
                 ok = ptx::mbar_wait_suspended(bar(kBarAccEmpty), (seg & 1u) ^ 1u);
                 for (uint32_t ks = kb; ks < ke && ok; ++ks, ++cnt) {
@@ -454,6 +465,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 ptx::tc_fence_after();
                 uint32_t v[16];
                 for (uint32_t k = 0; k < kLoads; ++k) {
+                    if (m0 + col_of(k) >= p.M) continue;  // rows that do not exist
                     tmem_ld16(acc_lane + col_of(k), v);
                     ptx::tmem_wait_ld();
                     float *dst = own_partial + (size_t)col_of(k) * BM;
@@ -513,8 +525,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                             __float2bfloat16_rn(f);
                 }
             };
-            // the helpers' sums for sixteen activation rows of this thread's weight row
             auto add_helpers = [&](uint32_t (&v)[16], uint32_t col) {
+                if (m0 + col >= p.M) return;
                 for (uint32_t h = first_helper; h < pair; ++h) {
                     const float *src = p.partial + (size_t)(2 * h + rank) * (BM * BN) + (size_t)col * BM + row_in_tile;
                     float part[16];
