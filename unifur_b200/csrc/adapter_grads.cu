@@ -6,11 +6,12 @@
 // gradient_kernel: out(p, j) = s sum_m X[m][p] R[m][j] as D[p][j] += A[p][m] B[m][j] (m16n8k16).  A CTA takes
 // 128 columns p, 64 ranks and a share of the rows; 64 rows of X and R per stage come by 16-byte
 // asynchronous copies, three stages in flight, and both operands are transposing matrix loads of what lies
-// there.  Eight warps: four pieces of 32 columns, two halves of a stage's rows.  Rows are shared out so that
-// two CTAs run on every SM; the shares meet in the workspace, where the CTA that arrives last for a
-// piece of columns adds them in order.  Bound by reading X once: grad_B of 2048 rows x 14336 columns took
-// 96 us and grad_A of 4096 columns 64 with one CTA per 64 columns walking all rows through a
-// register transpose, without overlap.
+// there.  Eight warps: four pieces of 32 columns, two halves of a stage's rows.  The CTAs that share a tile's
+// rows form a cluster: their sums meet through distributed shared memory, each adds (in rank order) and writes its part
+// of the columns.  Bound by reading X once and, at few columns, by the chain of a load, its stages and that
+// exchange; sums through the workspace, added by the CTA that arrived last, took 25 us for [2048, 4096] (now
+// 17) and 45 for [2048, 14336] (now 40) at rank 64.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
 #include "kernels.cuh"
@@ -23,25 +24,24 @@ constexpr uint32_t kThreads = 256, kCols = 128, kRowsStage = 64, kStages = 3;
 constexpr uint32_t kPitch = 272;                           // 256 bytes of a row and 16 of padding
 constexpr uint32_t kXStage = kRowsStage * kPitch, kStage = 2 * kXStage;
 constexpr uint32_t kSumPitch = 68;                         // floats
-constexpr uint32_t kCounterTiles = 248;                    // byte counters the flag words hold
+constexpr uint32_t kMaxShares = 16;
 static_assert(kCols * kSumPitch * 4 <= kStages * kStage, "the sums reuse the stages");
 
 struct Params {
     const __nv_bfloat16 *x, *r;   // [rows][P]; [rows][2 * 64 * chunks]: hi halves, then lo
     __nv_bfloat16 *out;
-    float *partial;               // [chunk][share][tile][128][64]
-    uint32_t *counters;
-    uint32_t rows, P, rank, chunks, shares, stages_per_share, p_major;
+    uint32_t rows, P, rank, chunks, stages_per_share, p_major;
     float scale;
 };
 
 __global__ void __launch_bounds__(kThreads, 2) gradient_kernel(const Params p) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ __align__(16) uint8_t smem[];
-    __shared__ uint32_t last_s;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const uint32_t g = lane >> 2, t = lane & 3u, li = lane >> 3, lr = lane & 7u;
     const uint32_t pw = warp & 3u, h = warp >> 2;
-    const uint32_t tile = blockIdx.x, share = blockIdx.y, p0 = tile * kCols;
+    const uint32_t shares = cluster.num_blocks(), share = cluster.block_rank(), p0 = blockIdx.x / shares * kCols;
     const uint32_t st0 = share * p.stages_per_share;
     const uint32_t all = (p.rows + kRowsStage - 1) / kRowsStage;
     const uint32_t nst = st0 < all ? min(p.stages_per_share, all - st0) : 0u;
@@ -124,45 +124,33 @@ __global__ void __launch_bounds__(kThreads, 2) gradient_kernel(const Params p) {
                     }
             }
         }
-        __syncthreads();
-        if (p.shares > 1) {
-            float4 *mine = reinterpret_cast<float4 *>(p.partial) +
-                           (((size_t)chunk * p.shares + share) * gridDim.x + tile) * (kCols * 16);
-            for (uint32_t i = tid; i < kCols * 16; i += kThreads)
-                if ((i & 15u) < 4 * tiles16)
-                    __stcg(mine + i, *reinterpret_cast<const float4 *>(sum + (i >> 4) * kSumPitch + (i & 15u) * 4));
-            __syncthreads();
-            if (tid == 0) {
-                __threadfence();
-                const uint32_t sh = (tile & 3u) * 8u;
-                const uint32_t old = (atomicAdd(p.counters + (tile >> 2), 1u << sh) >> sh) & 0xffu;
-                if (old == p.shares - 1) atomicSub(p.counters + (tile >> 2), p.shares << sh);
-                last_s = old == p.shares - 1;
-            }
-            __syncthreads();
-            if (!last_s) continue;
-            __threadfence();
-            for (uint32_t i = tid; i < kCols * 16; i += kThreads) {
+        if (shares > 1) cluster.sync();
+        else __syncthreads();
+        const uint32_t per = kCols / shares, per_log = __ffs(per) - 1, q0 = share * per;  // columns of this CTA's part
+        if (shares > 1) {  // (the others read their own parts of this CTA's sums: this one may be overwritten)
+            #pragma unroll 2
+            for (uint32_t i = tid; i < per * 16; i += kThreads) {
                 if ((i & 15u) >= 4 * tiles16) continue;
+                const uint32_t at = (q0 + (i >> 4)) * kSumPitch + (i & 15u) * 4;
                 float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                #pragma unroll 4
-                for (uint32_t q = 0; q < p.shares; ++q) {
-                    const float4 o = __ldcg(reinterpret_cast<const float4 *>(p.partial) +
-                                            (((size_t)chunk * p.shares + q) * gridDim.x + tile) * (kCols * 16) + i);
+                #pragma unroll 8
+                for (uint32_t c = 0; c < shares; ++c) {
+                    const float4 o = *reinterpret_cast<const float4 *>(cluster.map_shared_rank(sum, c) + at);
                     v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
                 }
-                *reinterpret_cast<float4 *>(sum + (i >> 4) * kSumPitch + (i & 15u) * 4) = v;
+                *reinterpret_cast<float4 *>(sum + at) = v;
             }
             __syncthreads();
         }
-        for (uint32_t i = tid; i < kCols * 64; i += kThreads) {
+        for (uint32_t i = tid; i < per * 64; i += kThreads) {
             // p fastest for [rank][P] outputs, j fastest for [P][rank]
-            const uint32_t q = p.p_major ? i >> 6 : i & (kCols - 1), j = p.p_major ? i & 63u : i >> 7;
+            const uint32_t q = q0 + (p.p_major ? i >> 6 : i & (per - 1)), j = p.p_major ? i & 63u : i >> per_log;
             const uint32_t pp = p0 + q, jj = chunk * 64 + j;
             if (pp < p.P && j < ranks)
                 p.out[p.p_major ? (size_t)pp * p.rank + jj : (size_t)jj * p.P + pp] = __float2bfloat16_rn(__fmul_rn(sum[q * kSumPitch + j], p.scale));
         }
-        __syncthreads();  // (before the next chunk's stages)
+        if (shares > 1) cluster.sync();
+        else __syncthreads();  // the sums have been read (before the next chunk's stages, and before a CTA leaves)
     }
 }
 
@@ -170,42 +158,49 @@ uint32_t chunks_of(uint32_t rank) { return (rank + 63) / 64; }
 uint64_t up256(uint64_t v) { return (v + 255) / 256 * 256; }
 uint64_t intermediate_bytes(uint64_t rows, uint32_t rank) { return up256(rows * 2 * 64 * chunks_of(rank) * 2); }
 uint64_t tiles_of(uint64_t P) { return (P + kCols - 1) / kCols; }
-// Shares of the rows: two CTAs on every SM where a share keeps four stages (256 rows); one where the
-// pieces of columns alone fill the SMs, or are more than there are counters.
-uint64_t shares_of(uint64_t rows, uint64_t P) {
+// Shares of the rows: as many as the chip holds clusters for at once, two CTAs on an SM (14 of sixteen, 33 of eight,
+// 71 of four), where a share keeps four stages (256 rows).
+uint32_t shares_of(uint64_t rows, uint64_t P) {
     const uint64_t tiles = tiles_of(P);
-    if (tiles > kCounterTiles) return 1;
-    uint64_t shares = 2 * kNumSMs / tiles;
-    const uint64_t most = (rows + 4 * kRowsStage - 1) / (4 * kRowsStage);
-    if (shares > most) shares = most;
-    if (shares > 64) shares = 64;
-    return shares ? shares : 1;
-}
-uint64_t partial_bytes(uint64_t rows, uint64_t P, uint32_t rank) {
-    const uint64_t shares = shares_of(rows, P);
-    return shares > 1 ? shares * tiles_of(P) * kCols * 64 * 4 * chunks_of(rank) : 0;
+    uint32_t shares = 1;
+    while (shares < kMaxShares && tiles <= (shares == 8 ? 14 : shares == 4 ? 33 : shares == 2 ? 71 : 148) && rows > shares * 4 * kRowsStage)
+        shares *= 2;
+    return shares;
 }
 
 int32_t gradient(const void *x, const void *r, void *out, uint64_t rows, uint64_t P, uint32_t rank, float scale, bool p_major,
-                 void *partial, uint32_t *counters, cudaStream_t s) {
+                 cudaStream_t s) {
     Params p{};
     p.x = static_cast<const __nv_bfloat16 *>(x);
     p.r = static_cast<const __nv_bfloat16 *>(r);
     p.out = static_cast<__nv_bfloat16 *>(out);
-    p.partial = static_cast<float *>(partial);
-    p.counters = counters;
     p.rows = (uint32_t)rows;
     p.P = (uint32_t)P;
     p.rank = rank;
     p.chunks = chunks_of(rank);
-    p.shares = (uint32_t)shares_of(rows, P);
+    const uint32_t shares = shares_of(rows, P);
     const uint32_t all = (uint32_t)((rows + kRowsStage - 1) / kRowsStage);
-    p.stages_per_share = (all + p.shares - 1) / p.shares;
+    p.stages_per_share = (all + shares - 1) / shares;
     p.p_major = p_major;
     p.scale = scale;
     NF4_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(gradient_kernel), (int)(kStages * kStage)));
+    if (shares > 8) NF4_TRY(allow_large_clusters(reinterpret_cast<const void *>(gradient_kernel)));
+    if (tiles_of(P) * shares >= (1ull << 31)) return fail(NF4_ERR_UNSUPPORTED, "gradient: too many columns");
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(tiles_of(P) * shares));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kStages * kStage;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = shares;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = shares > 1 ? 2 : 1;
     count_launch();
-    return launch_maybe_overlapped(gradient_kernel, dim3((unsigned)tiles_of(P), p.shares), dim3(kThreads), kStages * kStage, s, true, p);
+    return check_cuda(cudaLaunchKernelEx(&cfg, gradient_kernel, p), "gradient_kernel launch");
 }
 
 }  // namespace
@@ -216,11 +211,9 @@ bool adapter_grads_supported(const void *x, const void *gy, const void *a, const
            aligned16(x) && aligned16(gy) && (reinterpret_cast<uintptr_t>(a) & 1u) == 0 && (reinterpret_cast<uintptr_t>(b) & 1u) == 0;
 }
 
-// T | U | partial sums
-uint64_t adapter_grads_bytes(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t rank) {
-    if (!rank) return 0;
-    const uint64_t pa = partial_bytes(rows, d_in, rank), pb = partial_bytes(rows, d_out, rank);
-    return 2 * intermediate_bytes(rows, rank) + (pa > pb ? pa : pb);
+// T | U
+uint64_t adapter_grads_bytes(uint64_t rows, uint64_t, uint64_t, uint32_t rank) {
+    return rank ? 2 * intermediate_bytes(rows, rank) : 0;
 }
 
 void *adapter_grads_u(void *scratch, uint64_t rows, uint32_t rank) {
@@ -229,10 +222,9 @@ void *adapter_grads_u(void *scratch, uint64_t rows, uint32_t rank) {
 
 int32_t adapter_grads(const void *x, const void *gy, const void *a, const void *b, uint64_t rows, uint64_t d_in,
                       uint64_t d_out, uint32_t rank, float scale, int32_t layout, void *ga, void *gb, void *scratch,
-                      uint32_t *counters, bool u_ready, cudaStream_t s) {
+                      bool u_ready, cudaStream_t s) {
     const bool in_out = layout == NF4_LAYOUT_IN_OUT;
     void *t = scratch, *u = adapter_grads_u(scratch, rows, rank);
-    void *partial = static_cast<uint8_t *>(u) + intermediate_bytes(rows, rank);
     PrepassArgs q{};
     q.M = (uint32_t)rows;
     q.rank = rank;
@@ -249,11 +241,9 @@ int32_t adapter_grads(const void *x, const void *gy, const void *a, const void *
     q.a = a;
     q.k_major = in_out;
     q.r_out = t;
-    q.flags = counters;  // (zero by the workspace's contract; a host that clears them only for decode sizes need not care)
-    q.n_flags = kCounterTiles / 4;
     NF4_TRY(activations_prepass(q, s));
-    NF4_TRY(gradient(x, u, ga, rows, d_in, rank, scale, in_out, partial, counters, s));
-    return gradient(gy, t, gb, rows, d_out, rank, scale, !in_out, partial, counters, s);
+    NF4_TRY(gradient(x, u, ga, rows, d_in, rank, scale, in_out, s));
+    return gradient(gy, t, gb, rows, d_out, rank, scale, !in_out, s);
 }
 
 }  // namespace nf4

@@ -674,7 +674,7 @@ int32_t nf4_qlora_backward_dev(const nf4_linear_args *fwd, const void *grad_y, v
     if (!r) return NF4_OK;
     if (mma)
         return adapter_grads(fwd->x, grad_y, fwd->lora_a, fwd->lora_b, fwd->rows, fwd->d_in, fwd->d_out, r, fwd->lora_scale,
-                             fwd->layout, grad_a, grad_b, ws, static_cast<uint32_t *>(fwd->workspace), u_out != nullptr, s);
+                             fwd->layout, grad_a, grad_b, ws, u_out != nullptr, s);
     float *t = reinterpret_cast<float *>(ws);
     float *u = reinterpret_cast<float *>(ws + lora_workspace_bytes(fwd->rows, r));
     return lora_grads(fwd->x, grad_y, fwd->lora_a, fwd->lora_b, fwd->rows, fwd->d_in, fwd->d_out, r,

@@ -41,7 +41,7 @@ int32_t lora_grads(const void *x, const void *gy, const void *a, const void *b, 
                    void *gb, float *t, float *u, cudaStream_t s);
 
 // adapter_grads.cu: the same for bf16 tensors on warp MMAs.  `scratch` (256-byte aligned) holds R = x a and
-// grad_y b in the pre-pass's form and partial sums; `counters`: flag words, zero, left zero; u_ready:
+// grad_y b in the pre-pass's form; u_ready:
 // adapter_grads_u(scratch, ...) already holds grad_y b (the pre-pass of grad_x left it there).
 bool adapter_grads_supported(const void *x, const void *gy, const void *a, const void *b, uint64_t rows, uint64_t d_in,
                              uint64_t d_out, uint32_t rank);
@@ -49,7 +49,7 @@ uint64_t adapter_grads_bytes(uint64_t rows, uint64_t d_in, uint64_t d_out, uint3
 void *adapter_grads_u(void *scratch, uint64_t rows, uint32_t rank);
 int32_t adapter_grads(const void *x, const void *gy, const void *a, const void *b, uint64_t rows, uint64_t d_in,
                       uint64_t d_out, uint32_t rank, float scale, int32_t layout, void *ga, void *gb, void *scratch,
-                      uint32_t *counters, bool u_ready, cudaStream_t s);
+                      bool u_ready, cudaStream_t s);
 int32_t push_columns(void *const *y_full, uint32_t *const *arrive, uint32_t world, uint32_t rank, uint64_t rows,
                      uint64_t width_bytes, uint64_t ldy_bytes, bool signal, uint32_t *done, cudaStream_t s);
 int32_t gather_slabs(const void *slab, void *gathered, void *y, uint64_t rows, uint64_t width_bytes,
