@@ -603,6 +603,9 @@ struct Plan {
     uint32_t grid, smem_bytes;
     uint64_t off_counters, off_partials, ws_bytes;
 };
+// The workspace starts with the flag words of the other kernels (zero before a call and after it), which
+// this one has no use for: its counters are cleared by every call and T is written over whatever is there.
+constexpr uint64_t kOffT = 256;
 
 uint32_t round_up(uint32_t v, uint32_t a) { return (v + a - 1) / a * a; }
 
@@ -668,7 +671,7 @@ bool make_plan(uint64_t rows, uint64_t d_in, uint64_t d_out, bool dq, uint32_t r
     p.code_stages = stages;
     pl.smem_bytes = 1024 + p.off_ring + stages * kStageBytes;
     auto up = [](uint64_t v) { return (v + 255) / 256 * 256; };
-    pl.off_counters = up((uint64_t)16 * kMaxRank * 4);
+    pl.off_counters = kOffT + up((uint64_t)16 * kMaxRank * 4);
     pl.off_partials = pl.off_counters + up((uint64_t)p.row_tiles * 4);
     pl.ws_bytes = pl.off_partials + (uint64_t)(grid + p.row_tiles) * 16 * kRowsPerTile * 4;
     return true;
@@ -717,7 +720,7 @@ int32_t decode2_forward(const nf4_linear_args &a, cudaStream_t stream) {
         return fail(NF4_ERR_UNSUPPORTED, "decode2_forward: unsupported shape");
     Decode2Params &p = pl.p;
     uint8_t *ws = static_cast<uint8_t *>(a.workspace);
-    float *t = reinterpret_cast<float *>(ws);
+    float *t = reinterpret_cast<float *>(ws + kOffT);
     p.counters = reinterpret_cast<int *>(ws + pl.off_counters);
     p.partials = reinterpret_cast<float *>(ws + pl.off_partials);
     p.x = static_cast<const __nv_bfloat16 *>(a.x);
