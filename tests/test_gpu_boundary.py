@@ -218,6 +218,40 @@ def test_device_status_is_clean_and_a_bounded_wait_reports_a_timeout():
     assert float(t.sum().item()) == 4.0
 
 
+def test_a_failure_is_reported_once_and_not_to_later_host_pointer_calls(oracle):
+    # The kernels write their failure codes to a device flag and to host memory that the host-pointer forwards look
+    # at: what nf4_device_status has reported, or what came before a call, is not that call's failure.
+    L = lib()
+    rows, k, n = 3, 256, 64
+    rng = np.random.default_rng(4)
+    w, x = (rng.standard_normal((n, k)) * 0.02).astype(np.float32), rng.standard_normal((rows, k)).astype(np.float32)
+    h = ctypes.c_void_p()
+    _lib.check(L.nf4_weight_from_values_host(w.ctypes.data, k, n, _lib.LAYOUT_OUT_IN, 0, ctypes.byref(h)))
+    y = np.empty((rows, n), np.float32)
+    forward = lambda: L.nf4_weight_linear_forward_host(h, x.ctypes.data, rows, _lib.DTYPE_F32, None, None, None, 0, 0.0,  # noqa: E731
+                                                       y.ctypes.data)
+    try:
+        _lib.check(forward())  # (sets the host's words up)
+        want = y.copy()
+        for _ in range(2):
+            assert L.nf4_selftest_bounded_wait(1_000_000, None) == -5
+            y.fill(0.0)
+            _lib.check(forward())
+            assert y.tobytes() == want.tobytes()
+            assert L.nf4_device_status(None, None, None) == 0
+        # from another thread, whose calls begin after the failure as well
+        import threading
+
+        assert L.nf4_selftest_bounded_wait(1_000_000, None) == -5
+        got = []
+        t = threading.Thread(target=lambda: got.append(forward()))
+        t.start()
+        t.join()
+        assert got == [0]
+    finally:
+        L.nf4_weight_free(h)
+
+
 def _nccl():
     import os
 

@@ -151,13 +151,18 @@ struct Carver {
 };
 
 // ---- device-side failure flags ----------------------------------------------------
+int32_t current_device(int *dev) {
+    NF4_CUDA_TRY(cudaGetDevice(dev));
+    if (*dev < 0 || *dev >= 64) return fail(NF4_ERR_UNSUPPORTED, "device ordinal %d out of range", *dev);
+    return NF4_OK;
+}
+
 // Device addresses of the three kernels' flags, looked up once per device.
 int32_t flag_ptrs(int **out3) {
     static std::mutex mu;
     static int *cache[64][3] = {};
     int dev = 0;
-    NF4_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64) return fail(NF4_ERR_UNSUPPORTED, "device ordinal %d out of range", dev);
+    NF4_TRY(current_device(&dev));
     std::lock_guard<std::mutex> lock(mu);
     if (!cache[dev][0]) {
         int *p0 = nullptr, *p1 = nullptr, *p2 = nullptr;
@@ -189,15 +194,35 @@ int32_t report_flags(int *const *ptrs, const int *v) {
 
 // Three words of mapped host memory per device that the kernels' failure codes are written to
 // as well as to the device flags: the host-pointer entry points look at them after their final
-// synchronise, without a copy.  Set up at the first such call on a device.
-int32_t host_flag_words(volatile int **out) {
-    static std::mutex mu;
-    static int *words[64] = {};
+// synchronise, without a copy.  Codes found there are taken out and counted: several threads share the
+// words, and a call learns of a failure while it ran by the count having moved since it began, whoever
+// found the codes; one that came before the call (reported by then, or to be reported by
+// nf4_device_status) is not the call's.
+struct FailureWords {
+    volatile int *words = nullptr;
+    uint64_t found = 0;
+    int last[3] = {};  // the codes found last
+};
+std::mutex g_words_mu;
+FailureWords g_words[64];
+
+// (g_words_mu held)
+void take_failures(FailureWords &w) {
+    if (!w.words || !(w.words[0] | w.words[1] | w.words[2])) return;
+    for (int i = 0; i < 3; ++i) {
+        w.last[i] = w.words[i];
+        w.words[i] = 0;
+    }
+    ++w.found;
+}
+
+// Failures found on the current device so far; its words are set up at the first such call.  `last` may be null.
+int32_t failures_found(uint64_t *found, int *last) {
     int dev = 0;
-    NF4_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64) return fail(NF4_ERR_UNSUPPORTED, "device ordinal %d out of range", dev);
-    std::lock_guard<std::mutex> lock(mu);
-    if (!words[dev]) {
+    NF4_TRY(current_device(&dev));
+    std::lock_guard<std::mutex> lock(g_words_mu);
+    FailureWords &w = g_words[dev];
+    if (!w.words) {
         int *h = nullptr, *d = nullptr;
         NF4_CUDA_TRY(cudaHostAlloc(reinterpret_cast<void **>(&h), 3 * sizeof(int), cudaHostAllocMapped));
         h[0] = h[1] = h[2] = 0;
@@ -205,9 +230,11 @@ int32_t host_flag_words(volatile int **out) {
         NF4_TRY(decode_set_host_flag(d));
         NF4_TRY(decode2_set_host_flag(d + 1));
         NF4_TRY(prefill_set_host_flag(d + 2));
-        words[dev] = h;
+        w.words = h;
     }
-    *out = words[dev];
+    take_failures(w);
+    *found = w.found;
+    if (last) std::memcpy(last, w.last, sizeof(w.last));
     return NF4_OK;
 }
 
@@ -327,6 +354,12 @@ int32_t nf4_device_status(int32_t *decode, int32_t *decode_split_k, int32_t *pre
     int v[3] = {0, 0, 0};
     for (int i = 0; i < 3; ++i)
         NF4_CUDA_TRY(cudaMemcpy(&v[i], ptrs[i], sizeof(int), cudaMemcpyDeviceToHost));
+    int dev = 0;
+    NF4_TRY(current_device(&dev));
+    {  // what is reported here is not left for a later host-pointer call to find
+        std::lock_guard<std::mutex> lock(g_words_mu);
+        take_failures(g_words[dev]);
+    }
     if (decode) *decode = v[0];
     if (decode_split_k) *decode_split_k = v[1];
     if (prefill) *prefill = v[2];
@@ -1032,19 +1065,19 @@ int32_t nf4_weight_linear_forward_host(const nf4_weight *w, const void *x, uint6
     } else if (ws) {
         NF4_CUDA_TRY(cudaMemsetAsync(d_ws, 0, 256, kHostStream));
     }
-    volatile int *failed = nullptr;
-    NF4_TRY(host_flag_words(&failed));  // (before the launch: the kernels write their failure codes there too)
+    uint64_t before = 0, after = 0;
+    int codes[3];
+    NF4_TRY(failures_found(&before, nullptr));
     NF4_TRY(nf4_linear_forward_dev(&a, kHostStream));
     if (!y_mapped) NF4_CUDA_TRY(cudaMemcpyAsync(y, d_y, yb, cudaMemcpyDeviceToHost, kHostStream));
     NF4_TRY(check_cuda(cudaStreamSynchronize(kHostStream), "nf4_weight_linear_forward_host sync"));
     // ... and a wait that gave up in a kernel must not pass for a result
-    if (failed[0] | failed[1] | failed[2]) {
+    NF4_TRY(failures_found(&after, codes));
+    if (after != before) {
         int *ptrs[3];
         NF4_TRY(flag_ptrs(ptrs));
-        const int v[3] = {failed[0], failed[1], failed[2]};
-        failed[0] = failed[1] = failed[2] = 0;
         if (kept) (void)cudaMemset(kept, 0, 256);  // a kernel that gave up may have left its flag words set
-        return report_flags(ptrs, v);
+        return report_flags(ptrs, codes);
     }
     return NF4_OK;
 }
