@@ -355,7 +355,9 @@ NF4_API int32_t nf4_reserve_sms(int32_t count);
  *   wait_arrivals / wait_expected: if non-NULL, this forward's x is the output of a sharded
  *               layer: before reading x every CTA waits (bounded; NF4_ERR_TIMEOUT shows in
  *               nf4_device_status) until wait_expected arrivals -- one per rank and signal --
- *               are on this rank's own counter, and the launch takes them off it.
+ *               are on this rank's own counter, and the launch takes them off it -- also when
+ *               the wait gave up: the counter is signed, and late arrivals make up for what is
+ *               owed, so that later waits still count their own.
  * nf4_peer_arrivals_wait_dev is the wait on its own, for consumers that are not this library's
  * kernels: a one-thread kernel that waits (at most timeout_ns) until `expected` arrivals are on
  * the counter and takes them off; kernels behind it in the stream see all columns.

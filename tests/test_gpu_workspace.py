@@ -83,3 +83,34 @@ def test_flag_words_are_left_zero(route, backward):
     decode.y.zero_()
     assert torch.equal(decode.forward(ws), want)
     _lib.check(lib().nf4_device_status(None, None, None))
+
+
+def test_a_wait_for_arrivals_that_gives_up_leaves_the_counter_and_the_workspace_usable():
+    # One rank, whose counter nothing but this test adds to: the forwards wait out their second and say so.  An
+    # unsigned counter would wrap when the arrivals are taken off, and the next wait would pass without any.
+    L = lib()
+    rows, k, n, r = 4, 512, 256, 16
+    c = Call(rows, k, n, r, OUT_IN, BF16, seed=3)
+    want = c.forward(workspace(c.bytes())).clone()
+    ws, counters = workspace(c.bytes()), torch.zeros(2, dtype=torch.int32, device=DEV)
+    c.args.workspace, c.args.workspace_bytes = ws.data_ptr(), ws.numel()
+    y = torch.zeros(rows, n, dtype=BF16, device=DEV)
+    po = _lib.PeerOutputs()
+    po.struct_bytes, po.world, po.rank, po.ldy_full = ctypes.sizeof(po), 1, 0, n
+    po.y_full[0], po.arrivals[0], po.signal = y.data_ptr(), counters[1:].data_ptr(), 1
+    po.wait_arrivals, po.wait_expected = counters[:1].data_ptr(), 1
+    for step in (1, 2):
+        _lib.check(L.nf4_linear_forward_scatter_dev(ctypes.byref(c.args), ctypes.byref(po), None))
+        assert L.nf4_device_status(None, None, None) == -5
+        assert counters.tolist() == [-step, step]
+        assert int(ws[:256].count_nonzero()) == 0
+    counters[0] += 3  # both late arrivals and the next one
+    _lib.check(L.nf4_linear_forward_scatter_dev(ctypes.byref(c.args), ctypes.byref(po), None))
+    _lib.check(L.nf4_device_status(None, None, None))
+    assert counters.tolist() == [0, 3] and torch.equal(y, want)
+    # the wait by itself, a millisecond
+    _lib.check(L.nf4_peer_arrivals_wait_dev(counters.data_ptr(), 2, 1_000_000, None))
+    assert L.nf4_device_status(None, None, None) == -5
+    counters[0] += 2
+    assert counters.tolist() == [0, 3]
+    assert torch.equal(c.forward(ws), want)

@@ -208,6 +208,11 @@ __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t *p) {
     return v;
 }
 
+// Whether `expected` arrivals are on a counter that reads `v`.  The counter is signed: a wait takes its
+// arrivals off whether they came in time or not, so after one that gave up the counter is below zero by
+// what is owed, the late ones make that good, and the waits after it count their own.
+__device__ __forceinline__ bool arrived(uint32_t v, uint32_t expected) { return (int32_t)(v - expected) >= 0; }
+
 // How a launch gets its block scales.  d_in a multiple of 256 gives the scale rows a 16-byte pitch: f32
 // scales then come by TMA with the nibbles, u8 codes as one word per row and slice.  Other d_in (whole
 // blocks, but a pitch TMA does not take): lane t of a row's four lanes loads the scale of block t one
@@ -371,7 +376,7 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
             for (;;) {
                 uint32_t v;
                 asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(p.wait_on) : "memory");
-                if (v >= p.wait_expected) break;
+                if (arrived(v, p.wait_expected)) break;
                 if (ptx::global_timer_ns() - t0 > (uint64_t)p.wait_ns) {
                     NF4_REPORT_FAILURE(g_decode_error, g_decode_error_host, 7);
                     break;
@@ -846,7 +851,7 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
             __threadfence();
             if (atomicAdd(p.flags + 63, 1u) == nctas - 1) {
                 p.flags[63] = 0;
-                if (p.wait_on) atomicSub(p.wait_on, p.wait_expected);
+                if (p.wait_on) atomicAdd_system(p.wait_on, 0u - p.wait_expected);
                 if (p.signal) {
                     __threadfence_system();
                     for (uint32_t d = 0; d < p.n_dest; ++d) atomicAdd_system(p.arrive[d], 1u);
@@ -871,20 +876,20 @@ decode_kernel(const __grid_constant__ CUtensorMap tm_codes,
 
 // Waits (bounded) until `expected` CTAs of the ranks of a sharded layer have counted themselves in
 // on this rank's arrival counter, then takes them off the counter: the kernels behind it in the
-// stream find every rank's columns in this rank's output.
+// stream find every rank's columns in this rank's output (unless it gave up, which its flag says).
 __global__ void peer_wait_kernel(uint32_t *counter, uint32_t expected, uint32_t limit_ns) {
     const uint64_t t0 = ptx::global_timer_ns();
     for (;;) {
         uint32_t v;
         asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
-        if (v >= expected) break;
+        if (arrived(v, expected)) break;
         if (ptx::global_timer_ns() - t0 > (uint64_t)limit_ns) {
             NF4_REPORT_FAILURE(g_decode_error, g_decode_error_host, 7);
-            return;
+            break;
         }
         __nanosleep(100);
     }
-    atomicSub(counter, expected);
+    atomicAdd_system(counter, 0u - expected);
 }
 
 // Several forwards of the same activations (projections that share their input) in one launch:
