@@ -240,6 +240,12 @@ typedef struct nf4_linear_args {
 NF4_API uint64_t nf4_linear_workspace_bytes(uint64_t rows, uint64_t d_in, uint64_t d_out,
                                     uint32_t lora_rank);
 
+/* How many bytes at the start of its workspace the forward with these arguments relies on being zero: 256,
+ * or 0 where none of its kernels reads a flag word (most calls of more than 16 rows; what is there then
+ * stays as it is).  A host that allocates a workspace per call clears that much.  args->workspace and
+ * workspace_bytes are not read; all else is as for the call, the alignment of its pointers included. */
+NF4_API uint64_t nf4_linear_flag_bytes(const nf4_linear_args *args);
+
 NF4_API int32_t nf4_linear_forward_dev(const nf4_linear_args *args, void *stream);
 
 /* The adapter alone: y = ((x A) B) * lora_scale, the three operations in the reference's order,
@@ -282,6 +288,8 @@ NF4_API int32_t nf4_qlora_merge_dev(const uint8_t *packed, const float *absmax, 
  * bytes zero at the first use like any forward workspace (every call leaves them zero). */
 NF4_API uint64_t nf4_qlora_backward_workspace_bytes(uint64_t rows, uint64_t d_in, uint64_t d_out,
                                                     uint32_t lora_rank);
+/* nf4_linear_flag_bytes of the backward with these arguments. */
+NF4_API uint64_t nf4_qlora_backward_flag_bytes(const nf4_linear_args *fwd, const void *grad_y, const void *grad_x);
 NF4_API int32_t nf4_qlora_backward_dev(const nf4_linear_args *fwd, const void *grad_y, void *grad_x,
                                        void *grad_a, void *grad_b, void *stream);
 

@@ -89,6 +89,32 @@ def test_workspace_sizes_cover_every_route(lib):
     assert bw >= ws(2048, n, k, r) + 2 * 2048 * r * 4 + r * n * 2
 
 
+@pytest.mark.parametrize("rows,k,n,r,layout,f32,odd,want", [
+    (4, 512, 256, 16, 0, False, 0, 256), (16, 8192, 192, 0, 0, False, 0, 256),   # decode kernel
+    (5, 1024, 256, 24, 0, False, 0, 0),                                        # split-K kernel: counters of its own
+    (3, 512, 256, 8, 0, True, 0, 256), (2, 256, 320, 4, 1, True, 0, 256),        # f32 rows, strip kernel
+    (17, 512, 256, 16, 0, False, 0, 0), (64, 256, 192, 8, 1, True, 0, 0),        # tensor-core GEMM
+    (17, 320, 192, 3, 1, True, 0, 256), (64, 320, 192, 3, 1, True, 0, 256),      # strips: a rank the GEMM does not take
+    (64, 512, 256, 16, 1, False, 8, 256), (65, 512, 256, 16, 1, False, 8, 0),    # ... activations at an odd place
+    (65, 320, 192, 3, 1, True, 0, 0), (5, 200, 100, 5, 0, False, 0, 0),          # general kernel
+    (0, 512, 256, 16, 0, False, 0, 0),
+])
+def test_flag_bytes_follow_the_route(lib, rows, k, n, r, layout, f32, odd, want):
+    # host arithmetic only: the addresses are looked at for their alignment
+    from unifur_b200 import _lib
+
+    a = _lib.LinearArgs()
+    a.struct_bytes = ctypes.sizeof(a)
+    a.layout, a.io_dtype, a.rows, a.d_in, a.d_out = layout, int(f32), rows, k, n
+    a.x, a.y, a.packed, a.absmax = 4096 + odd, 4096, 4096, 4096
+    if r:
+        a.lora_a, a.lora_b, a.lora_rank = 4096, 4096, r
+    assert lib.nf4_linear_flag_bytes(ctypes.byref(a)) == want
+    # the backward's kernel is the forward's with the orientation and the dimensions exchanged
+    a.layout, a.d_in, a.d_out, a.x = 1 - layout, n, k, 4096
+    assert lib.nf4_qlora_backward_flag_bytes(ctypes.byref(a), 4096 + odd, 4096) == want
+
+
 def test_invalid_arguments_are_reported_not_fatal(lib):
     from unifur_b200 import _lib
 

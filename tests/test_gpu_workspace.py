@@ -85,6 +85,26 @@ def test_flag_words_are_left_zero(route, backward):
     _lib.check(lib().nf4_device_status(None, None, None))
 
 
+@pytest.mark.parametrize("backward", [False, True])
+@pytest.mark.parametrize("route", [r for r in ROUTES if r[:4] in (
+    (5, 1024, 256, 24), (2, 36864, 128, 12), (40, 256, 192, 16), (40, 256, 192, 8), (5, 200, 100, 5))])
+def test_routes_without_flag_words_run_on_any_workspace(route, backward):
+    c = Call(*route, seed=sum(route[:4]))
+    run = c.backward if backward else c.forward
+    c.args.y = c.y.data_ptr()
+    gx = torch.empty_like(c.x)
+    flags = lib().nf4_qlora_backward_flag_bytes(ctypes.byref(c.args), c.gy.data_ptr(), gx.data_ptr()) if backward else \
+        lib().nf4_linear_flag_bytes(ctypes.byref(c.args))
+    assert flags == (256 if backward and route[0] <= 16 and route[1] % 64 == 0 else 0)  # (strip kernel)
+    want = [t.clone() for t in run(workspace(c.bytes(backward)))]
+    ws = workspace(c.bytes(backward))
+    ws[flags:] = 0xAB
+    got = run(ws)
+    assert all(torch.equal(u, v) for u, v in zip(got, want))
+    assert torch.equal(ws[:256], torch.full_like(ws[:256], 0 if flags else 0xAB))
+    _lib.check(lib().nf4_device_status(None, None, None))
+
+
 def test_a_wait_for_arrivals_that_gives_up_leaves_the_counter_and_the_workspace_usable():
     # One rank, whose counter nothing but this test adds to: the forwards wait out their second and say so.  An
     # unsigned counter would wrap when the arrivals are taken off, and the next wait would pass without any.

@@ -92,6 +92,7 @@ SIGNATURES = {
     "nf4_quantize_dequantize_dev": (_i32, [_vp, _u64, _i32, _vp, _vp, _u64, _vp]),
     "nf4_quantize_dequantize_host": (_i32, [_vp, _u64, _i32, _vp]),
     "nf4_linear_workspace_bytes": (_u64, [_u64, _u64, _u64, _u32]),
+    "nf4_linear_flag_bytes": (_u64, [C.POINTER(LinearArgs)]),
     "nf4_linear_forward_dev": (_i32, [C.POINTER(LinearArgs), _vp]),
     "nf4_lora_workspace_bytes": (_u64, [_u64, _u32]),
     "nf4_lora_forward_dev": (_i32, [_vp, _u64, _u64, _u64, _vp, _vp, _u32, _f32, _i32, _i32, _vp, _u64, _vp,
@@ -99,6 +100,7 @@ SIGNATURES = {
     "nf4_lora_delta_weight_dev": (_i32, [_vp, _vp, _u64, _u64, _u32, _f32, _i32, _i32, _vp, _vp]),
     "nf4_qlora_merge_dev": (_i32, [_vp, _vp, _vp, _vp, _u64, _u64, _i32, _vp, _vp, _u32, _f32, _i32, _vp, _vp]),
     "nf4_qlora_backward_workspace_bytes": (_u64, [_u64, _u64, _u64, _u32]),
+    "nf4_qlora_backward_flag_bytes": (_u64, [C.POINTER(LinearArgs), _vp, _vp]),
     "nf4_qlora_backward_dev": (_i32, [C.POINTER(LinearArgs), _vp, _vp, _vp, _vp, _vp]),
     "nf4_sharded_gather_bytes": (_u64, [_u64, _u64, _i32, _i32, _i32]),
     "nf4_sharded_linear_forward_dev": (_i32, [C.POINTER(LinearArgs), _vp, _i32, _i32, _vp, _u64, _vp, _u64, _vp]),

@@ -134,6 +134,8 @@ struct ZeroScratch {
 };
 thread_local ZeroScratch t_zero_scratch;
 
+constexpr uint64_t kFlagWordBytes = 256;  // at the start of a workspace
+
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // Carves aligned sub-buffers out of the arena.
@@ -486,21 +488,46 @@ uint64_t nf4_linear_workspace_bytes(uint64_t rows, uint64_t d_in, uint64_t d_out
     return need;
 }
 
-// The kernel for a forward's shape.  *r_out (r_out may be null): where the adapter intermediate x A is wanted
-// beside the output; null afterwards if the kernel taken does not give it.
+// The kernels a forward goes to.  rows <= 16: the warp-MMA kernel (whole 64-blocks of d_in), else the tcgen05
+// split-K kernel; more rows: the tcgen05 GEMM; f32 rows with W [d_out, d_in] at up to 16 rows: the first two, as
+// bf16 halves; whatever none of them takes: the CUDA-core kernels.
+enum class Route { kDecode, kSplitK, kPrefill, kF32Rows, kGeneric };
+static Route route_of(const nf4_linear_args &a) {
+    if (decode_supported(a)) return Route::kDecode;
+    if (decode2_supported(a)) return Route::kSplitK;
+    if (prefill_supported(a) || prefill_in_out_supported(a)) return Route::kPrefill;
+    if (f32_rows_supported(a)) return Route::kF32Rows;
+    return Route::kGeneric;
+}
+
+// *r_out (r_out may be null): where the adapter intermediate x A is wanted beside the output; null afterwards
+// if the kernel taken does not give it.
 static int32_t linear_forward(const nf4_linear_args *args, cudaStream_t s, void **r_out) {
     NF4_TRY(validate_linear(args));
     if (args->rows == 0) return NF4_OK;
-    // rows <= 16: the warp-MMA kernel (whole 64-blocks of d_in), else the tcgen05 split-K kernel; more
-    // rows: the tcgen05 GEMM; whatever none of them takes: the CUDA-core kernels.
-    const bool decode = decode_supported(*args);
-    if (!decode && !decode2_supported(*args) && (prefill_supported(*args) || prefill_in_out_supported(*args)))
-        return prefill_forward(*args, s, r_out ? *r_out : nullptr);
+    const Route route = route_of(*args);
+    if (route == Route::kPrefill) return prefill_forward(*args, s, r_out ? *r_out : nullptr);
     if (r_out) *r_out = nullptr;
-    if (decode) return decode_forward(*args, s);
-    if (decode2_supported(*args)) return decode2_forward(*args, s);
-    if (f32_rows_supported(*args)) return f32_rows_forward(*args, s);
-    return generic_forward(*args, s);
+    switch (route) {
+        case Route::kDecode: return decode_forward(*args, s);
+        case Route::kSplitK: return decode2_forward(*args, s);
+        case Route::kF32Rows: return f32_rows_forward(*args, s);
+        default: return generic_forward(*args, s);
+    }
+}
+
+uint64_t nf4_linear_flag_bytes(const nf4_linear_args *args) {
+    if (!args || args->struct_bytes != sizeof(nf4_linear_args) || args->d_in == 0 || args->d_out == 0) return kFlagWordBytes;
+    if (args->rows == 0) return 0;
+    nf4_linear_args a = *args;  // with a workspace that fits, as the call will have
+    a.workspace = reinterpret_cast<void *>((uintptr_t)256);
+    a.workspace_bytes = nf4_linear_workspace_bytes(a.rows, a.d_in, a.d_out, a.lora_a ? a.lora_rank : 0);
+    switch (route_of(a)) {
+        case Route::kPrefill:
+        case Route::kSplitK: return 0;  // (its counters are cleared by every call)
+        case Route::kGeneric: return generic_reads_flags(a) ? kFlagWordBytes : 0;
+        default: return kFlagWordBytes;
+    }
 }
 
 int32_t nf4_linear_forward_dev(const nf4_linear_args *args, void *stream) {
@@ -669,6 +696,29 @@ uint64_t nf4_qlora_backward_workspace_bytes(uint64_t rows, uint64_t d_in, uint64
     return nf4_linear_workspace_bytes(rows, d_out, d_in, lora_rank) + (plain > mma ? plain : mma);
 }
 
+// grad_x = grad_y W^T + s (grad_y B^T) A^T: one more NF4 linear over the same packed bytes read
+// in the other orientation, the adapter factors exchanging roles
+static nf4_linear_args grad_x_args(const nf4_linear_args &fwd, const void *grad_y, void *grad_x) {
+    nf4_linear_args g = fwd;
+    g.layout = fwd.layout == NF4_LAYOUT_OUT_IN ? NF4_LAYOUT_IN_OUT : NF4_LAYOUT_OUT_IN;
+    g.d_in = fwd.d_out;
+    g.d_out = fwd.d_in;
+    g.x = grad_y;
+    g.y = grad_x;
+    g.ldy = 0;
+    g.y_f32 = 0;
+    g.bias = nullptr;
+    g.lora_a = fwd.lora_b;
+    g.lora_b = fwd.lora_a;
+    return g;
+}
+
+uint64_t nf4_qlora_backward_flag_bytes(const nf4_linear_args *fwd, const void *grad_y, const void *grad_x) {
+    if (!fwd) return kFlagWordBytes;
+    const nf4_linear_args g = grad_x_args(*fwd, grad_y, const_cast<void *>(grad_x));
+    return nf4_linear_flag_bytes(&g);  // (the adapter's gradients meet nowhere)
+}
+
 int32_t nf4_qlora_backward_dev(const nf4_linear_args *fwd, const void *grad_y, void *grad_x, void *grad_a,
                                void *grad_b, void *stream) {
     if (!fwd) return fail(NF4_ERR_INVALID_ARG, "nf4_qlora_backward_dev: null args");
@@ -683,19 +733,7 @@ int32_t nf4_qlora_backward_dev(const nf4_linear_args *fwd, const void *grad_y, v
     if (need && (!fwd->workspace || fwd->workspace_bytes < need || (reinterpret_cast<uintptr_t>(fwd->workspace) & 255u)))
         return fail(NF4_ERR_INVALID_ARG, "nf4_qlora_backward_dev: workspace smaller than "
                                          "nf4_qlora_backward_workspace_bytes or not 256-byte aligned");
-    // grad_x = grad_y W^T + s (grad_y B^T) A^T: one more NF4 linear over the same packed bytes read
-    // in the other orientation, the adapter factors exchanging roles
-    nf4_linear_args g = *fwd;
-    g.layout = fwd->layout == NF4_LAYOUT_OUT_IN ? NF4_LAYOUT_IN_OUT : NF4_LAYOUT_OUT_IN;
-    g.d_in = fwd->d_out;
-    g.d_out = fwd->d_in;
-    g.x = grad_y;
-    g.y = grad_x;
-    g.ldy = 0;
-    g.y_f32 = 0;
-    g.bias = nullptr;
-    g.lora_a = fwd->lora_b;
-    g.lora_b = fwd->lora_a;
+    nf4_linear_args g = grad_x_args(*fwd, grad_y, grad_x);
     const uint64_t fw = nf4_linear_workspace_bytes(fwd->rows, fwd->d_out, fwd->d_in, r);
     g.workspace_bytes = fw;
     uint8_t *ws = static_cast<uint8_t *>(fwd->workspace) + fw;

@@ -173,10 +173,13 @@ uint64_t generic_workspace_bytes(uint64_t rows, uint64_t d_in, uint64_t d_out, u
     return strips > need ? strips : need;
 }
 
+// whether generic_forward takes the strip kernel, whose runs meet on the flag words (nothing else here reads any)
+bool generic_reads_flags(const nf4_linear_args &a) { return a.rows <= kStripsMaxRows && strips_supported(a); }
+
 int32_t generic_forward(const nf4_linear_args &a, cudaStream_t stream) {
     if (a.d_out * 32 / 256 >= (1ull << 31) || a.rows * (a.lora_a ? a.lora_rank : 0) >= (1ull << 40))
         return fail(NF4_ERR_UNSUPPORTED, "generic_forward: shape too large");
-    if (a.rows <= kStripsMaxRows && strips_supported(a)) return strips_forward(a, stream);
+    if (generic_reads_flags(a)) return strips_forward(a, stream);
     GenericParams p{};
     p.x = a.x;
     p.lora_a = a.lora_a;

@@ -274,12 +274,12 @@ Rows flatten(const Tensor &x, uint64_t d_in) {
     return r;
 }
 
-// Up to 64 rows the kernels can meet on flag words; beyond, none of them reads any.
-constexpr uint64_t kMostRowsWithFlags = 64;
+// `bytes` of scratch whose first `flags` bytes have to be zero
+Tensor workspace(uint64_t bytes, uint64_t flags, const Place &at_, uint32_t slot = 0) {
+    return flags ? flagged_workspace(bytes, at_, slot) : empty({(int64_t)(bytes < 256 ? 256 : bytes)}, at::kByte, at_);
+}
 Tensor forward_workspace(const nf4_linear_args &a, const Place &at_, uint32_t slot = 0) {
-    const uint64_t bytes = nf4_linear_workspace_bytes(a.rows, a.d_in, a.d_out, a.lora_rank);
-    if (a.rows > kMostRowsWithFlags) return empty({(int64_t)(bytes < 256 ? 256 : bytes)}, at::kByte, at_);
-    return flagged_workspace(bytes, at_, slot);
+    return workspace(nf4_linear_workspace_bytes(a.rows, a.d_in, a.d_out, a.lora_rank), nf4_linear_flag_bytes(&a), at_, slot);
 }
 
 // linear_forward(x, d_in, layout, <projection>, out)
@@ -359,13 +359,12 @@ PyObject *qlora_backward(PyObject *, PyObject *const *v, Py_ssize_t n) {
         nf4_linear_args a = linear_args(r.x, r.rows, d_in, layout, p);
         Tensor gx = empty(r.shape, type, place);
         Tensor ga = empty(p.a.sizes(), type, place), gb = empty(p.b.sizes(), type, place);
-        const uint64_t bytes = nf4_qlora_backward_workspace_bytes(r.rows, d_in, p.d_out, a.lora_rank);
-        const Tensor ws = r.rows > kMostRowsWithFlags ? empty({(int64_t)(bytes < 256 ? 256 : bytes)}, at::kByte, place)
-                                                      : flagged_workspace(bytes, place, 0);
-        a.workspace = ws.mutable_data_ptr();
-        a.workspace_bytes = (uint64_t)ws.numel();
         void *px = gx.mutable_data_ptr(), *pa = ga.mutable_data_ptr(), *pb = gb.mutable_data_ptr();
         const void *pg = gy.const_data_ptr();
+        const Tensor ws = workspace(nf4_qlora_backward_workspace_bytes(r.rows, d_in, p.d_out, a.lora_rank),
+                                    nf4_qlora_backward_flag_bytes(&a, pg, px), place);
+        a.workspace = ws.mutable_data_ptr();
+        a.workspace_bytes = (uint64_t)ws.numel();
         check(unlocked([&] { return nf4_qlora_backward_dev(&a, pg, px, pa, pb, place.stream); }));
         return Py_BuildValue("NNN", THPVariable_Wrap(std::move(gx)), THPVariable_Wrap(std::move(ga)),
                              THPVariable_Wrap(std::move(gb)));

@@ -120,6 +120,7 @@ int32_t decode2_forward(const nf4_linear_args &a, cudaStream_t stream);
 
 // generic_linear.cu: any layout / dtype / shape on CUDA cores (exact f32 weights).
 uint64_t generic_workspace_bytes(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t lora_rank);
+bool generic_reads_flags(const nf4_linear_args &a);
 int32_t generic_forward(const nf4_linear_args &a, cudaStream_t stream);
 
 // in_out_strips.cu: NF4_LAYOUT_IN_OUT at few rows (sixteen per launch), d_out a multiple of 64, f32 arithmetic
