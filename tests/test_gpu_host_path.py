@@ -62,6 +62,35 @@ def test_kept_workspaces_serve_any_mix_of_calls(threads):
     _lib.check(_lib.load().nf4_device_status(None, None, None))
 
 
+def test_the_workspace_unused_longest_goes_first():
+    # sixteen are kept: a call on a seventeenth stream displaces the one whose last use is furthest back
+    x, p, k, n, layout, a, b = layers()[0]
+    out = torch.empty(x.shape[0], n, dtype=x.dtype, device=DEV)
+    streams, seen = [], set()
+    while len(streams) < 17:  # (torch hands its pool's streams out in turn)
+        s = torch.cuda.Stream()
+        if s.cuda_stream not in seen:
+            seen.add(s.cuda_stream)
+            streams.append(s)
+
+    def allocations(stream):
+        from unifur_b200.quantize import linear_forward
+
+        before = torch.cuda.memory_stats()["allocation.all.allocated"]
+        with torch.cuda.stream(stream):
+            linear_forward(x, p, k, n, layout, lora_a=a, lora_b=b, lora_scale=1.5, out=out)
+        torch.cuda.synchronize()
+        return torch.cuda.memory_stats()["allocation.all.allocated"] - before
+
+    _lib.host().release_workspaces()
+    assert [allocations(s) for s in streams[:16]] == [1] * 16
+    assert allocations(streams[0]) == 0                     # the oldest entry becomes the newest
+    assert allocations(streams[16]) == 1                    # displaces streams[1]'s
+    assert [allocations(s) for s in (streams[0], *streams[2:])] == [0] * 16
+    assert allocations(streams[1]) == 1
+    _lib.host().release_workspaces()
+
+
 def test_forward_under_capture_replays_beside_eager_calls():
     c = layers()[0]
     want = forward(*c)

@@ -9,10 +9,11 @@
 // Workspaces.  The decode and strip kernels meet on flag words at the start of the workspace that
 // must be zero at first use and are left zero.  A fresh workspace would need a fill kernel in front
 // of every call, which also breaks the overlap of a call's prologue with the call before it.  So a
-// host thread keeps the last kKeptMost workspaces it used, of at most kKeptBytes each, by stream (calls
-// on one stream are ordered; two threads never share one).  They live in torch's caching allocator and
-// go back to it when others have been used since, when the thread ends, and by release_workspaces().  Larger workspaces, and calls under stream capture (whose replays may run
-// on any stream later), are allocated per call.
+// host thread keeps the last kKeptMost workspaces it used, of at most kKeptBytes each, by stream
+// (calls on one stream are ordered; two threads never share one).  They live in torch's caching
+// allocator and go back to it when others have been used since, when the thread ends, and by
+// release_workspaces().  Larger workspaces, and calls under stream capture (whose replays may run on
+// any stream later), are allocated per call.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -24,6 +25,7 @@
 #include <cuda_runtime.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <algorithm>
 #include <cstring>
 #include <optional>
 #include <stdexcept>
@@ -171,7 +173,7 @@ Tensor flagged_workspace(uint64_t bytes, const Place &at_, uint32_t slot) {
     for (size_t i = t_kept.size(); i-- > 0;) {
         if (t_kept[i].device != dev || t_kept[i].stream != at_.stream || t_kept[i].slot != slot) continue;
         if ((uint64_t)t_kept[i].ws.numel() >= bytes) {
-            if (i + 1 != t_kept.size()) std::swap(t_kept[i], t_kept.back());
+            std::rotate(t_kept.begin() + (long)i, t_kept.begin() + (long)i + 1, t_kept.end());
             return t_kept.back().ws;
         }
         t_kept.erase(t_kept.begin() + (long)i);  // too small: replaced by a larger one below
