@@ -293,3 +293,21 @@ def test_load_path_quantize_of_the_transpose(oracle, rows, cols, bf16):
     o_sc, o_sos = oracle.double_quantize(o_absmax)
     assert np.array_equal(lin.packed().scale_codes.cpu().numpy(), o_sc)
     assert bits_equal(lin.packed().scale_of_scales.cpu().numpy(), np.asarray([o_sos], np.float32))
+
+
+def test_a_weight_from_an_odd_address_is_in_place_for_the_forward_behind_it():
+    # the forward asks for weights before it waits for the kernel ahead of it, here the quantizer of unaligned
+    # buffers, which writes them where the weight before last lay
+    from unifur_b200.quantize import PackedNf4Tensor, linear_forward
+
+    rows, k, n = 4, 4096, 2048
+    g = torch.Generator(device=DEV).manual_seed(12)
+    values = [torch.randn(n * k + 1, device=DEV, generator=g)[1:] * 0.02 for _ in range(2)]
+    values = [torch.cat([torch.zeros(1, device=DEV), v])[1:] for v in values]
+    assert all(v.data_ptr() % 16 == 4 and v.is_contiguous() for v in values)
+    x = torch.randn(rows, k, device=DEV, generator=g).bfloat16()
+    forward = lambda p: linear_forward(x, p, k, n, _lib.LAYOUT_OUT_IN)  # noqa: E731
+    want = [forward(PackedNf4Tensor.quantize(v.clone())) for v in values]
+    torch.cuda.synchronize()
+    got = [forward(PackedNf4Tensor.quantize(values[i % 2])) for i in range(100)]
+    assert all(torch.equal(y, want[i % 2]) for i, y in enumerate(got))

@@ -147,6 +147,7 @@ quantize_generic_kernel(const float *__restrict__ values, uint64_t len, uint64_t
         quantize_block_by_warp<PACKED>(values + blk * kBlock, left < kBlock ? (uint32_t)left : (uint32_t)kBlock,
                                        codes + blk * (PACKED ? kBlock / 2 : kBlock), absmax + blk);
     }
+    publish_weight();
 }
 
 // ---- dequantize -------------------------------------------------------------
