@@ -16,6 +16,12 @@
  *   - `*_host` entry points take HOST pointers; they copy in, run the same kernels,
  *     copy out and return when the result is in the caller's buffer.
  *   - Device buffers must be 16-byte aligned (anything cudaMalloc returns is).
+ *   - The forwards overlap their start with the end of the kernel ahead of them in the stream: what a
+ *     weight consists of (codes, scales, scale of scales) and an adapter's factors are read before that
+ *     kernel has completed.  This library's own writers of them allow for it.  Where a kernel of the
+ *     host's writes them directly ahead of a forward, it makes its writes visible before its blocks
+ *     end (__threadfence()), or a copy, a fill or an event wait stands between the two.  x, the bias
+ *     and everything else may come from any kernel ahead.
  *   - Read-only calls on one weight handle may run concurrently from several host
  *     threads (the reference moves modules across its block-executor threads,
  *     src/blockexec.rs:11-17); give each thread its own stream and workspace.

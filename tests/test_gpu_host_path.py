@@ -62,6 +62,29 @@ def test_kept_workspaces_serve_any_mix_of_calls(threads):
     _lib.check(_lib.load().nf4_device_status(None, None, None))
 
 
+@pytest.mark.parametrize("trained", [False, True])
+def test_factors_written_right_ahead_of_a_forward(trained):
+    # converted by the call itself, or by an optimizer's step before it: the decode kernel asks for factors early
+    from unifur_b200.quantize import linear_forward
+
+    x, p, k, n, layout, a, b = layers()[0]
+    want = [linear_forward(x, p, k, n, layout, lora_a=a * s, lora_b=b * s, lora_scale=1.5) for s in (1, -2)]
+    torch.cuda.synchronize()
+    if trained:
+        fa, fb = (torch.nn.Parameter(t.clone()) for t in (a, b))
+    got = []
+    for i in range(100):
+        s = (1, -2)[i % 2]
+        if trained:
+            with torch.no_grad():
+                torch.mul(a, s, out=fa.data)
+                torch.mul(b, s, out=fb.data)
+        else:
+            fa, fb = (a * s).float(), (b * s).float()
+        got.append(linear_forward(x, p, k, n, layout, lora_a=fa, lora_b=fb, lora_scale=1.5))
+    assert all(torch.equal(y, want[i % 2]) for i, y in enumerate(got))
+
+
 def test_the_workspace_unused_longest_goes_first():
     # sixteen are kept: a call on a seventeenth stream displaces the one whose last use is furthest back
     x, p, k, n, layout, a, b = layers()[0]

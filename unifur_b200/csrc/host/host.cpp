@@ -209,6 +209,7 @@ struct Projection {
     uint64_t d_out;
     Tensor bias, a, b;
     float scale;
+    bool just_written;  // the factors: by a conversion here, or perhaps by the optimizer that trains them
 };
 
 Projection projection(PyObject *const *v, at::ScalarType type) {
@@ -219,10 +220,13 @@ Projection projection(PyObject *const *v, at::ScalarType type) {
     p.absmax = p.scale_codes ? nullptr : tensor_or_none(v[1]);
     p.scale_of_scales = tensor_or_none(v[3]);
     p.d_out = size_arg(v[4]);
+    p.just_written = false;
     if (const Tensor *t = tensor_or_none(v[5])) p.bias = as_type(*t, at::kFloat);
     if (const Tensor *t = tensor_or_none(v[6])) {
+        const Tensor &b = tensor(v[7]);
         p.a = as_type(*t, type);
-        p.b = as_type(tensor(v[7]), type);
+        p.b = as_type(b, type);
+        p.just_written = !p.a.is_same(*t) || !p.b.is_same(b) || t->requires_grad() || b.requires_grad();
     }
     p.scale = (float)float_arg(v[8]);
     return p;
@@ -276,12 +280,18 @@ Rows flatten(const Tensor &x, uint64_t d_in) {
     return r;
 }
 
-// `bytes` of scratch whose first `flags` bytes have to be zero
-Tensor workspace(uint64_t bytes, uint64_t flags, const Place &at_, uint32_t slot = 0) {
-    return flags ? flagged_workspace(bytes, at_, slot) : empty({(int64_t)(bytes < 256 ? 256 : bytes)}, at::kByte, at_);
+// `bytes` of scratch whose first `flags` bytes have to be zero.  The kernels that meet on flag words take the
+// adapter's factors for constants, like the weight: they ask for them before the kernel ahead has completed.  One
+// that has just written them would have to publish them for that, which torch's do not: a fill of the
+// (zero) flag words between the two keeps them apart.
+Tensor workspace(uint64_t bytes, uint64_t flags, const Projection &p, const Place &at_, uint32_t slot = 0) {
+    if (!flags) return empty({(int64_t)(bytes < 256 ? 256 : bytes)}, at::kByte, at_);
+    Tensor ws = flagged_workspace(bytes, at_, slot);
+    if (p.just_written) zero_flags(ws, at_);
+    return ws;
 }
-Tensor forward_workspace(const nf4_linear_args &a, const Place &at_, uint32_t slot = 0) {
-    return workspace(nf4_linear_workspace_bytes(a.rows, a.d_in, a.d_out, a.lora_rank), nf4_linear_flag_bytes(&a), at_, slot);
+Tensor forward_workspace(const nf4_linear_args &a, const Projection &p, const Place &at_, uint32_t slot = 0) {
+    return workspace(nf4_linear_workspace_bytes(a.rows, a.d_in, a.d_out, a.lora_rank), nf4_linear_flag_bytes(&a), p, at_, slot);
 }
 
 // linear_forward(x, d_in, layout, <projection>, out)
@@ -299,7 +309,7 @@ PyObject *linear_forward(PyObject *, PyObject *const *v, Py_ssize_t n) {
         Tensor y = out ? *out : empty(r.shape, r.x.scalar_type(), place);
         a.y = y.mutable_data_ptr();
         a.ldy = out ? (uint64_t)out->stride(0) : p.d_out;
-        const Tensor ws = forward_workspace(a, place);
+        const Tensor ws = forward_workspace(a, p, place);
         a.workspace = ws.mutable_data_ptr();
         a.workspace_bytes = (uint64_t)ws.numel();
         check(unlocked([&] { return nf4_linear_forward_dev(&a, place.stream); }));
@@ -332,7 +342,7 @@ PyObject *linear_forward_grouped(PyObject *, PyObject *const *v, Py_ssize_t n) {
             ys.push_back(empty(r.shape, r.x.scalar_type(), place));
             a.y = ys.back().mutable_data_ptr();
             a.ldy = a.d_out;
-            scratch.push_back(forward_workspace(a, place, (uint32_t)i));
+            scratch.push_back(forward_workspace(a, ps.back(), place, (uint32_t)i));
             a.workspace = scratch.back().mutable_data_ptr();
             a.workspace_bytes = (uint64_t)scratch.back().numel();
         }
@@ -364,7 +374,7 @@ PyObject *qlora_backward(PyObject *, PyObject *const *v, Py_ssize_t n) {
         void *px = gx.mutable_data_ptr(), *pa = ga.mutable_data_ptr(), *pb = gb.mutable_data_ptr();
         const void *pg = gy.const_data_ptr();
         const Tensor ws = workspace(nf4_qlora_backward_workspace_bytes(r.rows, d_in, p.d_out, a.lora_rank),
-                                    nf4_qlora_backward_flag_bytes(&a, pg, px), place);
+                                    nf4_qlora_backward_flag_bytes(&a, pg, px), p, place);
         a.workspace = ws.mutable_data_ptr();
         a.workspace_bytes = (uint64_t)ws.numel();
         check(unlocked([&] { return nf4_qlora_backward_dev(&a, pg, px, pa, pb, place.stream); }));
