@@ -344,6 +344,12 @@ NF4_API int32_t nf4_decode_share_plan(uint32_t rows, uint32_t d_in, uint32_t d_o
 NF4_API int32_t nf4_prefill_share_plan(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t cta, uint32_t *ctas,
                                        uint32_t *segments, uint32_t capacity);
 
+/* How the kernels that share a tile's work out over a cluster of CTAs (the pre-pass of the tensor-core
+ * kernel, the adapter gradients) choose its size, computed on the host: 1, 2, 4, 8 or 16 CTAs for `tiles`
+ * tiles whose `length` is divided into pieces of `unit` or more.  room[i]: clusters of 2^i CTAs that the
+ * device holds at once (five entries; the library asks the driver).  For inspection and tests. */
+NF4_API int32_t nf4_cluster_share_plan(uint64_t tiles, uint64_t length, uint64_t unit, const uint32_t *room);
+
 /* The decode kernel puts one CTA on every SM (it needs a whole SM's shared memory), so a kernel
  * that runs beside it on another stream -- a collective gathering the previous step's outputs --
  * holds back whole CTAs of it.  A host that overlaps such work tells the library to leave `count`

@@ -86,3 +86,26 @@ def test_decode_kernel_shares_rows_and_k_exactly(rows, d_in, d_out, rank):
         assert ranges[0][0] == 0 and ranges[-1][1] == d_out
         assert all(a[1] == b[0] for a, b in zip(ranges, ranges[1:]))
     assert L.nf4_decode_share_plan(17, 4096, 64, 0, 0, out) < 0 and L.nf4_decode_share_plan(4, 100, 64, 0, 0, out) < 0
+
+
+def _clusters(tiles, length, unit, room):
+    return _lib.load().nf4_cluster_share_plan(tiles, length, unit, (ctypes.c_uint32 * 5)(*room))
+
+
+ROOM = (296, 148, 71, 33, 14)
+
+
+@pytest.mark.parametrize("tiles,length,unit,want", [
+    (1, 64, 64, 1), (1, 65, 64, 2), (4, 4096, 64, 16), (14, 4096, 64, 16), (15, 4096, 64, 8), (33, 4096, 64, 8),
+    (34, 4096, 64, 4), (71, 4096, 64, 4), (72, 4096, 64, 2), (148, 4096, 64, 2), (149, 4096, 64, 1),
+    (1, 1024, 64, 16), (1, 512, 64, 8), (8, 2048, 256, 8), (8, 2049, 256, 16), (112, 2048, 256, 2),
+])
+def test_clusters_fill_the_device_once(tiles, length, unit, want):
+    assert _clusters(tiles, length, unit, ROOM) == want
+
+
+def test_clusters_where_large_ones_have_no_place():
+    # what a device cannot place is not launched: the next smaller size is, down to a CTA by itself
+    assert [_clusters(4, 4096, 64, ROOM[:i] + (0,) * (5 - i)) for i in (5, 4, 3, 2, 1, 0)] == [16, 8, 4, 2, 1, 1]
+    assert _clusters(4, 4096, 64, (18, 9, 4, 2, 1)) == 4   # a slice of a device
+    assert _lib.load().nf4_cluster_share_plan(1, 1, 0, (ctypes.c_uint32 * 5)(*ROOM)) == -1

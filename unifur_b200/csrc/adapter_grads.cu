@@ -24,7 +24,6 @@ constexpr uint32_t kThreads = 256, kCols = 128, kRowsStage = 64, kStages = 3;
 constexpr uint32_t kPitch = 272;                           // 256 bytes of a row and 16 of padding
 constexpr uint32_t kXStage = kRowsStage * kPitch, kStage = 2 * kXStage;
 constexpr uint32_t kSumPitch = 68;                         // floats
-constexpr uint32_t kMaxShares = 16;
 static_assert(kCols * kSumPitch * 4 <= kStages * kStage, "the sums reuse the stages");
 
 struct Params {
@@ -158,16 +157,6 @@ uint32_t chunks_of(uint32_t rank) { return (rank + 63) / 64; }
 uint64_t up256(uint64_t v) { return (v + 255) / 256 * 256; }
 uint64_t intermediate_bytes(uint64_t rows, uint32_t rank) { return up256(rows * 2 * 64 * chunks_of(rank) * 2); }
 uint64_t tiles_of(uint64_t P) { return (P + kCols - 1) / kCols; }
-// Shares of the rows: as many as the chip holds clusters for at once, two CTAs on an SM (14 of sixteen, 33 of eight,
-// 71 of four), where a share keeps four stages (256 rows).
-uint32_t shares_of(uint64_t rows, uint64_t P) {
-    const uint64_t tiles = tiles_of(P);
-    uint32_t shares = 1;
-    while (shares < kMaxShares && tiles <= (shares == 8 ? 14 : shares == 4 ? 33 : shares == 2 ? 71 : 148) && rows > shares * 4 * kRowsStage)
-        shares *= 2;
-    return shares;
-}
-
 int32_t gradient(const void *x, const void *r, void *out, uint64_t rows, uint64_t P, uint32_t rank, float scale, bool p_major,
                  cudaStream_t s) {
     Params p{};
@@ -178,13 +167,15 @@ int32_t gradient(const void *x, const void *r, void *out, uint64_t rows, uint64_
     p.P = (uint32_t)P;
     p.rank = rank;
     p.chunks = chunks_of(rank);
-    const uint32_t shares = shares_of(rows, P);
+    // Shares of the rows: as many as the chip holds clusters for at once, where a share keeps four stages (256 rows)
+    const void *kernel = reinterpret_cast<const void *>(gradient_kernel);
+    ClusterRoom room;
+    NF4_TRY(cluster_room(kernel, kThreads, kStages * kStage, &room));
+    const uint32_t shares = cluster_ctas(tiles_of(P), rows, 4 * kRowsStage, room);
     const uint32_t all = (uint32_t)((rows + kRowsStage - 1) / kRowsStage);
     p.stages_per_share = (all + shares - 1) / shares;
     p.p_major = p_major;
     p.scale = scale;
-    NF4_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(gradient_kernel), (int)(kStages * kStage)));
-    if (shares > 8) NF4_TRY(allow_large_clusters(reinterpret_cast<const void *>(gradient_kernel)));
     if (tiles_of(P) * shares >= (1ull << 31)) return fail(NF4_ERR_UNSUPPORTED, "gradient: too many columns");
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(tiles_of(P) * shares));

@@ -65,8 +65,51 @@ int32_t ensure_dynamic_smem(const void *kernel, int bytes) {
     return set_once(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
-int32_t allow_large_clusters(const void *kernel) {
-    return set_once(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+int32_t cluster_room(const void *kernel, uint32_t threads, uint32_t smem, ClusterRoom *room) {
+    struct Asked {
+        const void *kernel;
+        int device;
+        ClusterRoom room;
+    };
+    static std::mutex mu;
+    static Asked asked[64];
+    static int n_asked = 0;
+    int dev = 0;
+    NF4_CUDA_TRY(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mu);
+    for (int i = 0; i < n_asked; ++i)
+        if (asked[i].kernel == kernel && asked[i].device == dev) {
+            *room = asked[i].room;
+            return NF4_OK;
+        }
+    NF4_TRY(ensure_dynamic_smem(kernel, (int)smem));
+    NF4_TRY(set_once(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    for (uint32_t i = 0; i < kClusterSizes; ++i) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(1u << i);
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = 1u << i;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+            (void)cudaGetLastError();  // (a size the device does not have)
+            n = 0;
+        }
+        room->of[i] = n > 0 ? (uint32_t)n : 0u;
+    }
+    if (n_asked < 64) asked[n_asked++] = Asked{kernel, dev, *room};
+    return NF4_OK;
+}
+
+uint32_t cluster_ctas(uint64_t tiles, uint64_t length, uint64_t unit, const ClusterRoom &room) {
+    uint32_t i = 0;
+    while (i + 1 < kClusterSizes && tiles <= room.of[i + 1] && length > (unit << i)) ++i;
+    return 1u << i;
 }
 
 void count_launch(uint64_t n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
@@ -628,6 +671,13 @@ int32_t nf4_prefill_share_plan(uint64_t rows, uint64_t d_in, uint64_t d_out, uin
     const int32_t n = prefill_share_plan(rows, d_in, d_out, cta, ctas, segments, capacity);
     if (n < 0) return fail(NF4_ERR_INVALID_ARG, "nf4_prefill_share_plan: not a shape of the tensor-core kernel, or no such CTA");
     return n;
+}
+
+int32_t nf4_cluster_share_plan(uint64_t tiles, uint64_t length, uint64_t unit, const uint32_t *room) {
+    if (!room || unit == 0) return fail(NF4_ERR_INVALID_ARG, "nf4_cluster_share_plan: null room or no unit");
+    ClusterRoom r;
+    std::memcpy(r.of, room, sizeof(r.of));
+    return (int32_t)cluster_ctas(tiles, length, unit, r);
 }
 
 uint64_t nf4_linear_noalloc_scratch_bytes(void) { return decode_static_scratch_bytes(); }

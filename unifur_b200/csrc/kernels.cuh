@@ -26,6 +26,18 @@ int32_t launch_maybe_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 block,
 // once per (kernel, device): the attribute belongs to the device a kernel is loaded on.
 int32_t ensure_dynamic_smem(const void *kernel, int bytes);
 
+// api.cu: how many clusters of 2^i CTAs of `kernel` the current device holds at once, by the driver's count (once
+// per kernel and device; 0: it has no place for one).  Sets the kernel's dynamic shared memory, and allows it clusters
+// of sixteen.  (A whole B200, two CTAs of 108 KB on an SM: 148 of two, 71 of four, 33 of eight, 14 of sixteen.)
+constexpr uint32_t kClusterSizes = 5;
+struct ClusterRoom {
+    uint32_t of[kClusterSizes];
+};
+int32_t cluster_room(const void *kernel, uint32_t threads, uint32_t smem, ClusterRoom *room);
+// CTAs to a cluster when each takes a piece of a tile's `length`: as many as leave the tiles' clusters in one wave and
+// every CTA a piece of more than half a unit, 1 at least.
+uint32_t cluster_ctas(uint64_t tiles, uint64_t length, uint64_t unit, const ClusterRoom &room);
+
 // lora.cu: the adapter alone, its dense update, the merge, and the gather of column slabs
 uint64_t lora_workspace_bytes(uint64_t rows, uint32_t rank);
 int32_t lora_forward(const void *x, uint64_t rows, uint64_t d_in, uint64_t d_out, const void *a, const void *b,

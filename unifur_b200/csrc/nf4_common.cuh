@@ -16,8 +16,6 @@ constexpr int kNumSMs = 148;            // B200
 int32_t fail(int32_t code, const char *fmt, ...);
 int32_t check_cuda(cudaError_t e, const char *what);
 void count_launch(uint64_t n = 1);
-// allows clusters of more than eight CTAs for `kernel` on the current device (once per kernel and device)
-int32_t allow_large_clusters(const void *kernel);
 
 #define NF4_CUDA_TRY(expr)                                         \
     do {                                                           \

@@ -31,7 +31,7 @@ namespace {
 
 constexpr uint32_t kThreads = 256;
 constexpr uint32_t kPartPitch = 68;  // floats
-constexpr uint32_t kMaxCluster = 16;
+constexpr uint32_t kMaxCluster = 1u << (kClusterSizes - 1);
 constexpr uint32_t kSmem = 108 * 1024;  // two CTAs on an SM
 // A stage: 128 k of bf16, 64 of f32.  Pitches are 16 bytes off a multiple of 128 (conflict-free matrix loads), for
 // the pairs of floats 32.
@@ -444,14 +444,9 @@ int32_t activations_prepass(const PrepassArgs &q, cudaStream_t stream) {
     p.scale = q.scale;
     p.wait = !q.beside_predecessor ? 0 : q.factor_of_predecessor ? 1 : 2;
     // 64 rows to a cluster beyond 512 rows, where the clusters of 32 no longer fit the chip at once, else 32 (half of the
-    // factor's traffic against more CTAs); then as many CTAs of K as the chip holds at once, two on an SM: it has room for
-    // 14 clusters of sixteen, 33 of eight, 71 of four (a second wave took 21 us where one takes 11)
+    // factor's traffic against more CTAs)
     const uint32_t rows = q.M > 512 ? 64 : 32;
     const uint64_t tiles = (q.M + rows - 1) / rows;
-    uint32_t cn = 1;
-    while (cn < kMaxCluster && tiles <= (cn == 8 ? 14 : cn == 4 ? 33 : cn == 2 ? 71 : 148) && q.K > cn * 64) cn *= 2;
-    p.piece = ((q.K + cn - 1) / cn + 63) / 64 * 64;
-    if (tiles * cn >= (1ull << 31)) return fail(NF4_ERR_UNSUPPORTED, "activations_prepass: too many rows");
     auto pick = [&](auto km) {
         constexpr bool k_major = decltype(km)::value;
         return rows == 64 ? (q.xh ? prepass_kernel<0, 64, k_major> : prepass_kernel<2, 64, k_major>)
@@ -461,8 +456,12 @@ int32_t activations_prepass(const PrepassArgs &q, cudaStream_t stream) {
     auto kernel = q.x_f32 ? (rows == 64 ? prepass_kernel<1, 64, false> : prepass_kernel<1, 32, false>)
                           : q.k_major ? pick(std::true_type{}) : pick(std::false_type{});
     const int smem = (int)(stages_of(q.x_f32, rows) * stage_bytes(q.x_f32, rows));
-    NF4_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), smem));
-    if (cn > 8) NF4_TRY(allow_large_clusters(reinterpret_cast<const void *>(kernel)));
+    // as many CTAs of K as the chip holds at once, two on an SM (a second wave took 21 us where one takes 11)
+    ClusterRoom room;
+    NF4_TRY(cluster_room(reinterpret_cast<const void *>(kernel), kThreads, (uint32_t)smem, &room));
+    const uint32_t cn = cluster_ctas(tiles, q.K, 64, room);
+    p.piece = ((q.K + cn - 1) / cn + 63) / 64 * 64;
+    if (tiles * cn >= (1ull << 31)) return fail(NF4_ERR_UNSUPPORTED, "activations_prepass: too many rows");
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(tiles * cn));
     cfg.blockDim = dim3(kThreads);

@@ -452,7 +452,7 @@ struct ScaleEncoder {
 // meet in distributed shared memory, so that no word has to be cleared first.  Sixteen SMs with eight
 // 16-byte loads in flight per thread read 3.7 MB (the scales of 14336 x 4096 weights) from the L2 in
 // about 2 us.  (Both passes in one cluster: 16 us, the encoding is too much work for sixteen SMs.)
-constexpr int kClusterCtas = 16, kClusterThreads = 1024;
+constexpr int kClusterCtas = 1 << (kClusterSizes - 1), kClusterThreads = 1024;
 constexpr uint64_t kClusterMaxBlocks = 1u << 20;
 
 __global__ void __launch_bounds__(kClusterThreads, 1)
@@ -498,7 +498,7 @@ scale_max_cluster_kernel(const float4 *__restrict__ absmax4, const float *__rest
     }
 }
 
-// More scales, or unaligned ones.  Pass 1: max over the (non-negative, never-NaN) block scales.  Their
+// More scales, unaligned ones, or a device that has no place for the cluster.  Pass 1: max over the (non-negative, never-NaN) block scales.  Their
 // f32 bit patterns order like unsigned integers, so one atomicMax on the bits per warp is exact.
 __global__ void __launch_bounds__(kThreads)
 scale_max_kernel(const float *__restrict__ absmax, uint64_t nblocks, uint32_t *max_bits) {
@@ -684,8 +684,9 @@ int32_t double_quantize(const float *absmax, uint64_t nblocks, uint8_t *scale_co
     if (!absmax || !scale_codes)
         return fail(NF4_ERR_INVALID_ARG, "nf4_double_quantize: null pointer");
     const bool whole = aligned16(absmax) && (reinterpret_cast<uintptr_t>(scale_codes) & 3u) == 0;
-    if (aligned16(absmax) && nblocks <= kClusterMaxBlocks) {
-        NF4_TRY(allow_large_clusters(reinterpret_cast<const void *>(scale_max_cluster_kernel)));
+    ClusterRoom room;
+    NF4_TRY(cluster_room(reinterpret_cast<const void *>(scale_max_cluster_kernel), kClusterThreads, 0, &room));
+    if (aligned16(absmax) && nblocks <= kClusterMaxBlocks && room.of[kClusterSizes - 1]) {
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(kClusterCtas);
         cfg.blockDim = dim3(kClusterThreads);
