@@ -84,9 +84,8 @@ NF4_API uint64_t nf4_kernel_launch_count(void);
  * Rust shim maps a non-zero status to anyhow::Error (src/lib.rs:16-32). */
 NF4_API int32_t nf4_device_status(int32_t *decode, int32_t *decode_split_k, int32_t *prefill);
 
-/* How many failures nf4_device_status and the `*_host` entry points have reported in this process.  A
- * kernel that gave up may have left its workspace's flag words set: a host that keeps a workspace
- * across calls clears its first 256 bytes again when this number has changed. */
+/* How many failures nf4_device_status and the `*_host` entry points have reported in this process (a
+ * host's log, a watchdog).  Workspaces need no care after one: see nf4_linear_args. */
 NF4_API uint64_t nf4_failure_count(void);
 
 /* Diagnostic: launches a one-thread kernel that waits on a barrier nobody signals, with the same
@@ -229,7 +228,8 @@ typedef struct nf4_linear_args {
     uint64_t ldy;               /* row stride of y in elements; 0 means d_out */
     void *workspace;            /* nf4_linear_workspace_bytes() bytes, 256-byte aligned; its first 256
                                    bytes must be zero at the first call that uses it (cudaMemset once
-                                   after allocating); every call leaves them zero */
+                                   after allocating); every call leaves them zero, one whose bounded wait
+                                   gave up included (nf4_device_status): it needs no clearing again */
     uint64_t workspace_bytes;
 } nf4_linear_args;
 

@@ -209,11 +209,12 @@ def test_device_status_is_clean_and_a_bounded_wait_reports_a_timeout():
     assert (d.value, d2.value, pf.value) == (0, 0, 0)
     # a wait that nothing will ever satisfy, with a one-millisecond limit: the kernel comes back,
     # the status says timeout, the flag is cleared and the context is usable afterwards
-    waited_ns = ctypes.c_uint64(0)
+    waited_ns, failures = ctypes.c_uint64(0), L.nf4_failure_count()
     st = L.nf4_selftest_bounded_wait(1_000_000, ctypes.byref(waited_ns))
     assert st == -5 and b"wait" in L.nf4_last_error()
     assert 1_000_000 <= waited_ns.value < 500_000_000
     assert L.nf4_device_status(None, None, None) == 0
+    assert L.nf4_failure_count() == failures + 1
     t = torch.ones(4, device=DEV)
     assert float(t.sum().item()) == 4.0
 

@@ -1145,11 +1145,10 @@ int32_t nf4_weight_linear_forward_host(const nf4_weight *w, const void *x, uint6
     a.ldy = w->d_out;
     a.workspace = ws ? d_ws : nullptr;
     a.workspace_bytes = ws;
-    void *kept = nullptr;
     if (ws && rows <= 16 && ws <= ZeroScratch::kMaxBytes) {
-        // the decode workspace starts with flag words that must be zero: a buffer kept for it
-        NF4_TRY(t_zero_scratch.get(&kept, ws));
-        a.workspace = kept;
+        // the decode workspace starts with flag words that must be zero: a buffer kept for it (every call, one that
+        // gives up included, leaves them zero)
+        NF4_TRY(t_zero_scratch.get(&a.workspace, ws));
     } else if (ws) {
         NF4_CUDA_TRY(cudaMemsetAsync(d_ws, 0, 256, kHostStream));
     }
@@ -1164,7 +1163,6 @@ int32_t nf4_weight_linear_forward_host(const nf4_weight *w, const void *x, uint6
     if (after != before) {
         int *ptrs[3];
         NF4_TRY(flag_ptrs(ptrs));
-        if (kept) (void)cudaMemset(kept, 0, 256);  // a kernel that gave up may have left its flag words set
         return report_flags(ptrs, codes);
     }
     return NF4_OK;

@@ -860,9 +860,11 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
         }
     }
     if (done_old == nctas - 1) {
-        // The last CTA to have read T re-arms the two flag words for the next launch: every other
-        // CTA read the first before it counted itself in on the second, and the next launch
-        // looks at them only after this one has completed, so no order is needed between them.
+        // The last CTA to have read T, or to have given up on it, re-arms the two flag words for the next
+        // launch: every other CTA read the first before it counted itself in on the second, a producer's two
+        // additions are one thread's, to one sector, and the next launch looks at the words only after this
+        // one has completed, so no order is needed between them.  Nothing a wait that gives up skips is
+        // counted: the words (the arrival counters and word 63 alike) are zero after every launch.
         *reinterpret_cast<uint2 *>(p.flags) = make_uint2(0u, 0u);
     }
 }

@@ -7,7 +7,7 @@
 // host work for 70 us of kernels).  Here a call costs about as much as its launch.
 //
 // Workspaces.  The decode and strip kernels meet on flag words at the start of the workspace that
-// must be zero at first use and are left zero.  A fresh workspace would need a fill kernel in front
+// must be zero at first use and are left zero, by calls whose waits gave up too.  A fresh workspace would need a fill kernel in front
 // of every call, which also breaks the overlap of a call's prologue with the call before it.  So a
 // host thread keeps the last kKeptMost workspaces it used, of at most kKeptBytes each, by stream
 // (calls on one stream are ordered; two threads never share one).  They live in torch's caching
@@ -154,7 +154,6 @@ struct Kept {
     Tensor ws;
 };
 thread_local std::vector<Kept> t_kept;  // most recently used last
-thread_local uint64_t t_failures = 0;   // failures of the library's kernels reported so far
 
 // `bytes` of scratch whose first 256 bytes are zero.  `slot`: which of a call's workspaces (the
 // projections of a grouped call have one each).
@@ -164,10 +163,6 @@ Tensor flagged_workspace(uint64_t bytes, const Place &at_, uint32_t slot) {
         Tensor ws = empty({(int64_t)bytes}, at::kByte, at_);
         zero_flags(ws, at_);
         return ws;
-    }
-    if (const uint64_t f = nf4_failure_count(); f != t_failures) {
-        t_kept.clear();  // a kernel that gave up may have left its flag words set
-        t_failures = f;
     }
     const int dev = at_.device.index();
     for (size_t i = t_kept.size(); i-- > 0;) {
