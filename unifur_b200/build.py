@@ -68,13 +68,14 @@ def _build_host(verbose: bool) -> None:
     inc = [*cpp_extension.include_paths(), sysconfig.get_paths()["include"],
            os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include")]
     libs = os.path.join(os.path.dirname(torch.__file__), "lib")
-    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *[f"-I{d}" for d in inc], HOST,
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           "-Wall", "-Wextra", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           *[a for d in inc for a in ("-isystem", d)], HOST,
            "-o", HOST_LIB, f"-L{HERE}", "-l:libnf4b200.so", f"-L{libs}", "-lc10", "-lc10_cuda", "-ltorch_cpu",
            "-ltorch_cuda", "-ltorch_python", f"-L{os.path.join(os.path.dirname(os.path.dirname(NVCC)), 'lib64')}",
            "-lcudart_static", "-ldl", "-lrt", "-lpthread", "-Wl,-rpath,$ORIGIN"]
     r = subprocess.run(cmd, capture_output=True, text=True)
-    if verbose or r.returncode != 0:
+    if verbose or r.returncode != 0 or r.stderr:
         sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
     if r.returncode != 0:
         raise RuntimeError("building the host extension failed")

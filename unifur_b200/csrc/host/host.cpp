@@ -119,7 +119,6 @@ Tensor as_type(const Tensor &t, at::ScalarType type) {
     return (t.scalar_type() == type ? t : t.to(type)).contiguous();
 }
 
-const void *ptr(const Tensor *t) { return t ? t->const_data_ptr() : nullptr; }
 template <class T>
 const T *ptr_as(const Tensor *t) { return t ? static_cast<const T *>(t->const_data_ptr()) : nullptr; }
 
