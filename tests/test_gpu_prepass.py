@@ -59,7 +59,7 @@ def test_forward(M, K, N, r, layout, f32):
 @pytest.mark.parametrize("M,K,N,r,layout", [
     (1, 64, 128, 8, 0), (5, 200, 136, 5, 1), (16, 1024, 512, 16, 0),   # decode sizes: both intermediates by the product-only mode
     (63, 256, 384, 16, 1), (513, 640, 200, 80, 0), (2049, 576, 1344, 64, 1),   # shares of the rows, ragged pieces of columns
-    (1100, 128, 32000, 8, 0),                                          # more pieces of columns than counters
+    (1100, 128, 32000, 8, 0),                                          # 250 tiles of columns by CTAs on their own, one by a cluster of eight
 ])
 def test_backward(M, K, N, r, layout):
     q, w, A, B, x, rnd = layer(M, K, N, r, layout, torch.bfloat16, M + K + N)

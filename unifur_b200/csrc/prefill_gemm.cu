@@ -936,16 +936,15 @@ EncodeTiledFn encode_fn() {
 }
 
 // 2-D row-major tensor [rows][cols] with row pitch `pitch_bytes`; box = [box_rows][box_cols].
-int32_t make_map(CUtensorMap *map, CUtensorMapDataType dt, uint32_t elem_bytes, const void *base,
-                 uint64_t rows, uint64_t cols, uint64_t pitch_bytes, uint32_t box_rows,
-                 uint32_t box_cols, CUtensorMapSwizzle swz) {
+int32_t make_map(CUtensorMap *map, CUtensorMapDataType dt, const void *base, uint64_t rows,
+                 uint64_t cols, uint64_t pitch_bytes, uint32_t box_rows, uint32_t box_cols,
+                 CUtensorMapSwizzle swz) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return fail(NF4_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     cuuint64_t dims[2] = {cols, rows};
     cuuint64_t strides[1] = {pitch_bytes};
     cuuint32_t box[2] = {box_cols, box_rows};
     cuuint32_t estr[2] = {1, 1};
-    (void)elem_bytes;
     CUresult r = fn(map, dt, 2, const_cast<void *>(base), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1168,23 +1167,23 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_o
     NF4_TRY(activations_prepass(pre, stream));
 
     CUtensorMap map_x, map_t, map_b, map_y, map_w;
-    NF4_TRY(make_map(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, p.codes, p.N, p.K / 2, p.K / 2, BM, 128, CU_TENSOR_MAP_SWIZZLE_128B));
-    NF4_TRY(make_map(&map_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, xh, p.M, p.K, (uint64_t)p.K * 2, BN / 2, BK,
+    NF4_TRY(make_map(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.codes, p.N, p.K / 2, p.K / 2, BM, 128, CU_TENSOR_MAP_SWIZZLE_128B));
+    NF4_TRY(make_map(&map_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, xh, p.M, p.K, (uint64_t)p.K * 2, BN / 2, BK,
                      CU_TENSOR_MAP_SWIZZLE_128B));
     map_t = map_b = map_x;
     if (p.rank) {
         const uint32_t ld_t = 2 * 64 * p.lora_chunks;
-        NF4_TRY(make_map(&map_t, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, t, p.M, ld_t, (uint64_t)ld_t * 2, BN / 2,
+        NF4_TRY(make_map(&map_t, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, t, p.M, ld_t, (uint64_t)ld_t * 2, BN / 2,
                          BK, CU_TENSOR_MAP_SWIZZLE_128B));
         // LoRA B [N][rank]: columns beyond the rank and rows beyond N read as zero
-        NF4_TRY(make_map(&map_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, lora_b, p.N, p.rank,
+        NF4_TRY(make_map(&map_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, lora_b, p.N, p.rank,
                          (uint64_t)p.rank * 2, BM, BK, CU_TENSOR_MAP_SWIZZLE_128B));
     }
     if (y_f32)
-        NF4_TRY(make_map(&map_y, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a.y, p.M, p.N, ldy * 4, kEpiBytes / (BM * 4), BM,
+        NF4_TRY(make_map(&map_y, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, a.y, p.M, p.N, ldy * 4, kEpiBytes / (BM * 4), BM,
                          CU_TENSOR_MAP_SWIZZLE_NONE));
     else
-        NF4_TRY(make_map(&map_y, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.y, p.M, p.N, ldy * 2, kEpiBytes / (BM * 2), BM,
+        NF4_TRY(make_map(&map_y, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a.y, p.M, p.N, ldy * 2, kEpiBytes / (BM * 2), BM,
                          CU_TENSOR_MAP_SWIZZLE_NONE));
 
     auto go = [&](auto kernel) -> int32_t {

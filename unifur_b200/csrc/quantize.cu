@@ -210,13 +210,13 @@ dequantize_full_kernel(const uint8_t *__restrict__ codes, uint32_t ngroups, uint
 
 template <bool PACKED>
 __global__ void __launch_bounds__(kThreads)
-dequantize_generic_kernel(const uint8_t *__restrict__ codes, uint64_t len, uint64_t first,
+dequantize_generic_kernel(const uint8_t *__restrict__ codes, uint64_t len,
                           const float *__restrict__ absmax,
                           const uint8_t *__restrict__ scale_codes,
                           const float *__restrict__ scale_of_scales, float *__restrict__ out) {
     const float sos = scale_of_scales ? __ldg(scale_of_scales) : 0.0f;
     const uint64_t stride = (uint64_t)gridDim.x * kThreads;
-    for (uint64_t i = first + (uint64_t)blockIdx.x * kThreads + threadIdx.x; i < len; i += stride) {
+    for (uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x; i < len; i += stride) {
         uint32_t c;
         if (PACKED) {
             const uint32_t byte = codes[i >> 1];
@@ -583,8 +583,8 @@ int32_t dequantize_impl(const uint8_t *codes, uint64_t len, const float *absmax,
         }
         return NF4_OK;
     }
-    dequantize_generic_kernel<PACKED><<<grid_for(len, kThreads, 8), kThreads, 0, stream>>>(codes, len, 0, absmax, scale_codes,
-                                                                                         scale_of_scales, out);
+    dequantize_generic_kernel<PACKED><<<grid_for(len, kThreads, 8), kThreads, 0, stream>>>(codes, len, absmax, scale_codes,
+                                                                                       scale_of_scales, out);
     count_launch();
     return check_cuda(cudaGetLastError(), "nf4_dequantize launch");
 }
