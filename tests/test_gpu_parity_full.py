@@ -139,23 +139,25 @@ def _decode_case(oracle, m, k, n, r, x_scale_rows, seed):
     check_out_in(oracle, c, m, k, n, 2.0)
 
 
-@pytest.mark.parametrize("m", [1, 5, 16])
-def test_decode_activations_far_outside_f16_range(oracle, m):
+@pytest.mark.parametrize("m,r", [(1, 16), (5, 16), (16, 16), (1, 24), (7, 24), (16, 24)])
+def test_decode_activations_far_outside_f16_range(oracle, m, r):
     # bf16 activations the f16 operand type cannot hold: rows scaled by 2^17 (overflow), by 2^-20
-    # (below f16's normal range) and mixed rows; the kernel rescales each warp's slice by a power
-    # of two, so the tolerance is the usual one
-    k, n, r = 4096, 1024, 16
+    # (below f16's normal range) and mixed rows; the kernels (rank 24: the split-K one) rescale a row of
+    # the slice they multiply by a power of two, so the tolerance is the usual one
+    k, n = 4096, 1024
     _decode_case(oracle, m, k, n, r, {i: 2.0 ** 17 for i in range(16)}, 71)
     _decode_case(oracle, m, k, n, r, {i: 2.0 ** -20 for i in range(16)}, 72)
     _decode_case(oracle, m, k, n, r, {0: 2.0 ** 17, 1: 2.0 ** -20, 3: 2.0 ** 30, 9: 2.0 ** -40}, 73)
 
 
-def test_decode_block_scales_at_both_ends(oracle):
-    # the decode kernel multiplies by the f32 block scale after the MMA: weights of any magnitude
+@pytest.mark.parametrize("r,dq", [(16, False), (24, False), (24, True)])
+def test_decode_block_scales_at_both_ends(oracle, r, dq):
+    # the decode kernel multiplies by the f32 block scale after the MMA, the split-K one (rank 24) divides the
+    # scales by a power of two of the weight before it: weights of any magnitude
     from test_gpu_linear import check_out_in, make_case
 
     for w_std, seed in ((1e-5, 81), (1e4, 82)):
-        c = make_case(oracle, seed, 4, 2048, 512, 16, w_std=w_std)
+        c = make_case(oracle, seed, 4, 2048, 512, r, dq=dq, w_std=w_std)
         check_out_in(oracle, c, 4, 2048, 512, 2.0)
 
 

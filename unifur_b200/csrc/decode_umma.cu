@@ -24,6 +24,10 @@
 // B = x from shared memory (16 columns, rows >= M are zero), D = f32 accumulators in TMEM (two
 // per issuer and segment, so consecutive MMAs of an issuer do not chain).
 //
+// f16's range.  The block scales enter divided by a power of two of the weight; a row of x whose largest
+// magnitude in the CTA's k-range is 2^16 or above, or below 2^-7, enters divided by one of its own (both
+// exact).  The CTA's sums are multiplied back before they leave it.
+//
 // Finish (four warps).  A segment that spans the whole K is finished in place (+bias, +LoRA, convert, store).
 // Otherwise its 128 x 16 partial goes to a scratch slot; the last CTA to arrive for a row-tile
 // (one counter per row-tile) adds the slots in a fixed order and finishes the tile, so results
@@ -33,6 +37,7 @@
 #include <cuda_fp16.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "kernels.cuh"
 #include "ptx.cuh"
@@ -76,6 +81,8 @@ struct Decode2Params {
     void *y;
     float *partials;   // [(grid + row_tiles)][16][128] f32
     int *counters;     // [row_tiles], zero at launch
+    const float *absmax;          // one of the two: for the weight's power of two (see weight_exponent)
+    const uint8_t *scale_codes;
     const float *scale_of_scales;
     uint64_t ldy;
     uint32_t y_f32;
@@ -129,6 +136,14 @@ __device__ __forceinline__ uint32_t hmul2(uint32_t a, uint32_t b) {
     uint32_t d;
     asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
     return d;
+}
+
+// The power of two a row is divided by, from the bits of its largest bf16 magnitude, which it brings to
+// [2^14, 2^15); 1 for ordinary rows and those with infinities.
+__device__ __forceinline__ float row_factor(uint32_t mx) {
+    const int ex = (int)(mx >> 7);  // biased exponent: 127 is 2^0, 255 is infinity
+    const bool odd = mx != 0u && ex != 255 && (ex > 142 || ex < 120);
+    return odd ? __int_as_float((127 + max(ex - 141, -100)) << 23) : 1.0f;
 }
 
 __device__ __forceinline__ uint64_t make_kmajor_sw128_desc(uint32_t smem_byte_addr) {
@@ -196,6 +211,8 @@ decode2_kernel(const __grid_constant__ CUtensorMap tmap_codes,
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kLutBytes);          // < 512 B
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + kLutBytes + 512);
     int *last_flag = reinterpret_cast<int *>(smem + kLutBytes + 520);
+    uint32_t *x_max = reinterpret_cast<uint32_t *>(smem + kLutBytes + 544);   // [4][16]: parts of the rows' largest magnitudes
+    float *x_factor = reinterpret_cast<float *>(smem + kLutBytes + 800);      // [16]
     float *t_s = reinterpret_cast<float *>(smem + kLutBytes + 1024);          // [16][64] f32
     uint8_t *x_s = smem + p.off_x;                                            // x_blocks * 2 KB
     uint8_t *ring = smem + p.off_ring;
@@ -260,42 +277,61 @@ decode2_kernel(const __grid_constant__ CUtensorMap tmap_codes,
         ptx::tmem_relinquish();
     } else if (warp < kExpanderWarps) {
         // ---- x's k-range -> f16, canonical K-major 128B-swizzled rows (16 rows per block) ----
-        // one 16-byte chunk (8 values) per thread and step, four loads in flight; rows >= M are zero
+        // one 16-byte chunk (8 values) per thread and step, four loads in flight; rows >= M are zero.
+        // (A thread's chunks all belong to one row.)
         const uint32_t chunks = p.x_blocks * 16 * 8;
         constexpr uint32_t nthreads = kExpanderWarps * 32;
+        const uint32_t row = (tid >> 3) & 15u;
         bool released = false;
-        for (uint32_t base = tid; base < chunks; base += 4 * nthreads) {
-            uint4 v[4];
-            #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const uint32_t i = base + u * nthreads;
-                const uint32_t slot = i >> 7, row = (i >> 3) & 15u, c = i & 7u;
-                uint32_t kb = slot + x_base;
-                if (kb >= p.kb) kb -= p.kb;
-                v[u] = make_uint4(0, 0, 0, 0);
-                if (i < chunks && row < p.M)
-                    v[u] = __ldg(reinterpret_cast<const uint4 *>(
-                        p.x + (size_t)row * p.K + (size_t)kb * 64 + c * 8));
-            }
-            if (!released) {  // first batch of loads is out: release the producer
-                asm volatile("bar.arrive 3, %0;" ::"n"((kExpanderWarps + 1) * 32) : "memory");
-                released = true;
-            }
-            #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const uint32_t i = base + u * nthreads;
-                if (i >= chunks) break;
-                const uint32_t slot = i >> 7, row = (i >> 3) & 15u, c = i & 7u;
-                const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
-                uint32_t h[4];
+        auto convert = [&](auto scaled, float down) {
+            __nv_bfloat162 mx2 = __float2bfloat162_rn(0.0f);  // the largest magnitudes, as pairs (NaNs are left out)
+            for (uint32_t base = tid; base < chunks; base += 4 * nthreads) {
+                uint4 v[4];
                 #pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    h[q] = pack_h2(__uint_as_float(w[q] << 16), __uint_as_float(w[q] & 0xffff0000u));
-                uint8_t *dst = x_s + slot * kXBlockBytes + (row >> 3) * 1024 + (row & 7u) * 128 +
-                               ((c ^ (row & 7u)) << 4);
-                *reinterpret_cast<uint4 *>(dst) = make_uint4(h[0], h[1], h[2], h[3]);
+                for (int u = 0; u < 4; ++u) {
+                    const uint32_t i = base + u * nthreads;
+                    const uint32_t slot = i >> 7, c = i & 7u;
+                    uint32_t kb = slot + x_base;
+                    if (kb >= p.kb) kb -= p.kb;
+                    v[u] = make_uint4(0, 0, 0, 0);
+                    if (i < chunks && row < p.M)
+                        v[u] = __ldg(reinterpret_cast<const uint4 *>(
+                            p.x + (size_t)row * p.K + (size_t)kb * 64 + c * 8));
+                }
+                if (!released) {  // first batch of loads is out: release the producer
+                    asm volatile("bar.arrive 3, %0;" ::"n"((kExpanderWarps + 1) * 32) : "memory");
+                    released = true;
+                }
+                #pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const uint32_t i = base + u * nthreads;
+                    if (i >= chunks) break;
+                    const uint32_t slot = i >> 7, c = i & 7u;
+                    const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+                    uint32_t h[4];
+                    #pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const float lo = __uint_as_float(w[q] << 16), hi = __uint_as_float(w[q] & 0xffff0000u);
+                        h[q] = scaled.value ? pack_h2(lo * down, hi * down) : pack_h2(lo, hi);
+                        mx2 = __hmax2(mx2, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&w[q])));
+                    }
+                    uint8_t *dst = x_s + slot * kXBlockBytes + (row >> 3) * 1024 + (row & 7u) * 128 +
+                                   ((c ^ (row & 7u)) << 4);
+                    *reinterpret_cast<uint4 *>(dst) = make_uint4(h[0], h[1], h[2], h[3]);
+                }
             }
-        }
+            const uint32_t pair = *reinterpret_cast<const uint32_t *>(&mx2);
+            return max(pair & 0xffffu, pair >> 16);  // non-negative bf16 values order like their bit patterns
+        };
+        // converted as they are, which serves nearly always; the other rows once more with their factor
+        uint32_t mx = convert(std::false_type{}, 1.0f);
+        #pragma unroll
+        for (int d = 1; d < 8; d *= 2) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, d));
+        if ((tid & 7u) == 0) x_max[(tid >> 7) * 16 + row] = mx;
+        asm volatile("bar.sync 4, %0;" ::"n"(kExpanderWarps * 32) : "memory");
+        const float factor = row_factor(max(max(x_max[row], x_max[16 + row]), max(x_max[32 + row], x_max[48 + row])));
+        if (tid < 128 && (tid & 7u) == 0) x_factor[row] = factor;
+        if (factor != 1.0f) convert(std::true_type{}, 1.0f / factor);
         if (!released) asm volatile("bar.arrive 3, %0;" ::"n"((kExpanderWarps + 1) * 32) : "memory");
         ptx::fence_proxy_async();  // x_s is read by the tensor core through the async proxy
     }
@@ -370,6 +406,7 @@ decode2_kernel(const __grid_constant__ CUtensorMap tmap_codes,
         const uint32_t q = warp & 3u, grp = warp >> 2;   // TMEM lane quarter, block within a tile
         const uint32_t row = q * 32 + lane;              // row inside the 128-row tile = TMEM lane
         const float sos = DQ ? __ldg(p.scale_of_scales) : 0.0f;
+        const float w_down = ldexpf(1.0f, -weight_exponent(p.absmax, p.scale_codes, p.scale_of_scales));
         const uint32_t *lut_lane = lut + lane;
         const uint32_t swz = row & 7u;
         uint32_t st = 0, bc_base = 0;
@@ -393,7 +430,7 @@ decode2_kernel(const __grid_constant__ CUtensorMap tmap_codes,
                         scale = dq_scale(stage[kCodeStageBytes + row * 16 + (kb & 15u)], sos);
                     else
                         scale = reinterpret_cast<const float *>(stage + kCodeStageBytes)[row * 4 + grp];
-                    const uint32_t s2 = pack_h2(scale, scale);
+                    const uint32_t s2 = pack_h2(scale * w_down, scale * w_down);
                     const uint32_t w[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
                     uint32_t out[32];
                     #pragma unroll
@@ -429,6 +466,7 @@ decode2_kernel(const __grid_constant__ CUtensorMap tmap_codes,
         const uint32_t row = q * 32 + lane;  // TMEM lane = row inside the 128-row tile
         const uint32_t ftid = (warp - kWarpFinish0) * 32 + lane;
         Segment sg;
+        const float w_up = ldexpf(1.0f, weight_exponent(p.absmax, p.scale_codes, p.scale_of_scales));
         // this thread's LoRA-B rows (one per segment) are fetched now, long before they are needed
         uint4 lbq[kMaxSegments][2];
         const bool lb_in_regs = p.rank == 16;
@@ -472,6 +510,8 @@ decode2_kernel(const __grid_constant__ CUtensorMap tmap_codes,
                     for (int m = 0; m < 16; ++m) v[m] += ok ? __uint_as_float(r[m]) : 0.0f;
                 }
             }
+            #pragma unroll
+            for (int m = 0; m < 16; ++m) v[m] = v[m] * x_factor[m] * w_up;  // (powers of two)
             const bool whole = sg.kb0 == 0 && sg.kb1 == p.kb;
             bool finish = whole;
             uint32_t c_first = cta, c_last = cta;
@@ -730,6 +770,8 @@ int32_t decode2_forward(const nf4_linear_args &a, cudaStream_t stream) {
     p.y_f32 = (uint32_t)a.y_f32;
     p.ldy = a.ldy ? a.ldy : a.d_out;
     p.lora_scale = a.lora_scale;
+    p.absmax = a.absmax;
+    p.scale_codes = a.scale_codes;
     p.scale_of_scales = a.scale_of_scales;
     NF4_CUDA_TRY(cudaMemsetAsync(p.counters, 0, (size_t)p.row_tiles * 4, stream));
     if (p.rank) {
