@@ -123,6 +123,12 @@ def test_invalid_arguments_are_reported_not_fatal(lib):
     st = lib.nf4_linear_forward_dev(ctypes.byref(a), None)
     assert st == -1 and b"struct_bytes" in lib.nf4_last_error()
     assert lib.nf4_linear_forward_dev(None, None) == -1
+    # the adapter's gradients read x, which the forward they begin with does not
+    a.struct_bytes, a.rows, a.d_in, a.d_out, a.lora_rank = ctypes.sizeof(a), 4, 64, 64, 8
+    a.packed = a.absmax = a.lora_a = a.lora_b = a.workspace = 4096
+    a.workspace_bytes = 1 << 30
+    grads = [4096] * 4
+    assert lib.nf4_qlora_backward_dev(ctypes.byref(a), *grads, None) == -1 and b"null x" in lib.nf4_last_error()
     out = ctypes.c_void_p()
     assert lib.nf4_weight_from_values_host(None, 4, 4, 0, 1, ctypes.byref(out)) == -1
     assert lib.nf4_quantize_host(None, 10, None, None) == -1

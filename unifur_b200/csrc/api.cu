@@ -779,6 +779,7 @@ int32_t nf4_qlora_backward_dev(const nf4_linear_args *fwd, const void *grad_y, v
     if (fwd->rows == 0) return NF4_OK;
     if (!grad_y || !grad_x || (r && (!grad_a || !grad_b)))
         return fail(NF4_ERR_INVALID_ARG, "nf4_qlora_backward_dev: null gradient buffer");
+    if (r && (!fwd->x || !fwd->lora_b)) return fail(NF4_ERR_INVALID_ARG, "nf4_qlora_backward_dev: null x or factor");
     const uint64_t need = nf4_qlora_backward_workspace_bytes(fwd->rows, fwd->d_in, fwd->d_out, r);
     if (need && (!fwd->workspace || fwd->workspace_bytes < need || (reinterpret_cast<uintptr_t>(fwd->workspace) & 255u)))
         return fail(NF4_ERR_INVALID_ARG, "nf4_qlora_backward_dev: workspace smaller than "
