@@ -1,4 +1,5 @@
-"""Quantize / dequantize of lengths that are no multiple of a block, on aligned buffers (one launch) and unaligned ones."""
+"""Quantize / dequantize of lengths that are no multiple of a block, on aligned buffers (one launch) and unaligned ones;
+forwards whose output is a part of a wider buffer."""
 import numpy as np
 import pytest
 
@@ -49,3 +50,21 @@ def test_double_quantization_of_any_length(oracle, nb):
     sc, sos = double_quantize_dev(s)
     o_sc, o_sos = oracle.double_quantize(s)
     assert sc.tobytes() == o_sc.tobytes() and np.float32(sos).tobytes() == np.float32(o_sos).tobytes()
+
+
+@pytest.mark.parametrize("rows", [1, 16, 17, 100, 361])
+@pytest.mark.parametrize("n,ld", [(41, 44), (43, 48), (47, 48), (65, 72), (130, 136), (300, 304), (300, 301), (192, 200), (1000, 1024)])
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+def test_a_row_s_padding_is_left_alone(rows, n, ld, dt):
+    # outputs that end inside a 16-byte piece, in buffers whose rows go on: a tensor map's store writes whole pieces
+    from unifur_b200.quantize import PackedNf4Tensor, linear_forward
+
+    k = 128
+    g = torch.Generator(device=DEV).manual_seed(rows + n)
+    p = PackedNf4Tensor.quantize(torch.randn(k * n, device=DEV, generator=g) * 0.02)
+    x = torch.randn(rows, k, device=DEV, generator=g).to(dt)
+    buf = torch.full((rows + 1, ld), 7.0, dtype=dt, device=DEV)
+    y = linear_forward(x, p, k, n, _lib.LAYOUT_OUT_IN, out=buf[:rows, :n])
+    ref = x.double() @ p.dequantize().view(n, k).t().double()
+    assert float((y.double() - ref).norm() / ref.norm()) < (1e-3 if dt == torch.float32 else 4e-3)
+    assert bool((buf[:, n:] == 7.0).all()) and bool((buf[rows] == 7.0).all())

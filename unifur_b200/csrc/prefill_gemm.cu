@@ -55,6 +55,7 @@
 #include <cuda_fp16.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "kernels.cuh"
 #include "ptx.cuh"
@@ -131,6 +132,10 @@ struct PrefillParams {
     float *partial;
     uint32_t *sk_flags;
     uint32_t wait_ns;  // bound of the wait for a neighbour's flag
+    // A TMA store writes whole 16-byte pieces: the piece that holds the last columns would reach beyond them into the
+    // row's padding, which is not the call's.  Where d_out ends inside a piece, the tiles at that end are stored plainly.
+    void *y_ragged;    // the output then, else null
+    uint64_t ldy;
 };
 
 // A pair's list of segments (tile, main k-stages [b, e)), in the order they are worked on: the
@@ -577,7 +582,14 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                     asm volatile("bar.sync 1, 256;" ::: "memory");
                     // (an odd number of 128-row tiles: the last odd CTA's rows do not exist)
                     const uint32_t m = m0 + (k / kPerPass) * kStageRows;
-                    if (epi_leader && n0 < p.N && m < p.M) {
+                    if (p.y_ragged && n0 + BM > p.N) {
+                        using Y = typename std::conditional<YF32, float, __nv_bfloat16>::type;
+                        #pragma unroll 1
+                        for (uint32_t e = epi_thread; e < kStageRows * BM; e += 256) {
+                            const uint32_t row = m + e / BM, col = n0 + e % BM;
+                            if (row < p.M && col < p.N) static_cast<Y *>(p.y_ragged)[row * p.ldy + col] = reinterpret_cast<const Y *>(epi)[e];
+                        }
+                    } else if (epi_leader && n0 < p.N && m < p.M) {
                         ptx::tma_store_2d(&tmap_y, own | kEpiAt, (int32_t)n0, (int32_t)m);
                         ptx::tma_store_commit();
                     }
@@ -1090,6 +1102,8 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_o
     p.lora_chunks = lora_chunks_of(p.rank);
     p.m_tiles = (p.M + BN - 1) / BN;
     const uint64_t ldy = a.ldy ? a.ldy : a.d_out;
+    if (p.N * (y_f32 ? 4u : 2u) % 16 != 0) p.y_ragged = a.y;
+    p.ldy = ldy;
 
     const WorkspaceLayout wl = workspace_layout(p.M, p.K, p.N, p.rank, extra);
     if (a.workspace_bytes < wl.bytes) return fail(NF4_ERR_INVALID_ARG, "prefill_forward: workspace too small");
