@@ -533,7 +533,7 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
     // the producers' count one tile early (the load is in flight while that tile is multiplied),
     // waits -- bounded -- only if the count is not there yet, then the warp issues asynchronous
     // copies that the end-of-pass wait collects.
-    bool lost = false;   // a wait of this warp ran out: results are void, the flag is set
+    bool lost = false;   // a wait of this warp ran out: results are void, the flag is set, no more tiles are asked for
     uint32_t seen = 0;   // lane 0 of warp 0: the producers' count as last read
     uint32_t done_old = 0xffffffffu;  // lane 0 of warp 0: CTAs that had read T before this one
     auto peek_t = [&]() {
@@ -552,7 +552,11 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
             }
         }
         ok = __shfl_sync(0xffffffffu, ok, 0);
-        if (!ok) lost = true;
+        if (!ok) {
+            lost = true;
+            req_j = my_tiles;
+            ptx::let_flights_land();
+        }
         const uint32_t n = SL * p.M * p.rank;
         const float *t_part = p.t_global + (size_t)part * n;  // this part's share of T
         if ((n & 3u) == 0) {
@@ -616,7 +620,9 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
             const uint32_t slot = use_j & (kRing - 1);
             if (!lost && !wait_phase(bar0 + 8 * slot, (use_j / kRing) & 1u, p.wait_ns)) {
                 lost = true;
+                req_j = my_tiles;  // a slot whose copy is still out takes no other, and the copies land before the CTA ends
                 if (lane == 0) NF4_REPORT_FAILURE(g_decode_error, g_decode_error_host, 5);
+                ptx::let_flights_land();
             }
             float acc[NT][4];
             #pragma unroll

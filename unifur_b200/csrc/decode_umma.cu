@@ -596,6 +596,7 @@ decode2_kernel(const __grid_constant__ CUtensorMap tmap_codes,
         if (!ok && lane == 0) NF4_REPORT_FAILURE(g_decode2_error, g_decode2_error_host, 4);
     }
 
+    if (!ok) ptx::let_flights_land();
     ptx::tc_fence_before();
     __syncthreads();
     if (warp == kWarpIssuer0) {

@@ -373,10 +373,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                     }
                 }
             }
-            if (!ok) {
-                NF4_REPORT_FAILURE(g_prefill_error, g_prefill_error_host, 1);
-                __nanosleep(1000000);  // the copies in flight (counted in the even CTA) end before the CTA does
-            }
+            if (!ok) NF4_REPORT_FAILURE(g_prefill_error, g_prefill_error_host, 1);
         }
     } else if (warp == 1) {
         // ============================= MMA issuer =============================
@@ -752,13 +749,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 ptx::tma_load_2d((own | kCodesAt) + slot * kCodeTileBytes, &tmap_w, (int32_t)(b * 128), n0, bar(kBarCFull + slot));
             }
         }
-        if (!ok) {
-            for (uint32_t c = block > kCodeSlots ? block - kCodeSlots : 0; c < block; ++c)
-                ptx::mbar_wait_suspended(bar(kBarCFull + c % kCodeSlots), (c / kCodeSlots) & 1u);
-            NF4_REPORT_FAILURE(g_prefill_error, g_prefill_error_host, 7);
-        }
+        if (!ok) NF4_REPORT_FAILURE(g_prefill_error, g_prefill_error_host, 7);
     }
 
+    if (!ok) ptx::let_flights_land();
     __syncwarp();
     // neither CTA leaves, or gives its tensor memory back, while the other may still signal it
     ptx::tc_fence_before();

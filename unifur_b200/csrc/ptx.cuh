@@ -85,6 +85,14 @@ __device__ __forceinline__ bool mbar_wait_suspended(uint32_t bar, uint32_t parit
     }
 }
 
+// For a thread that has given up on a barrier, before its CTA may end (and its shared and tensor memory go to the
+// next one): copies and MMAs in flight land within microseconds, but their barriers can no longer be relied on, so
+// it lets a millisecond pass by the clock (a sleep by itself may return at once).
+__device__ __forceinline__ void let_flights_land() {
+    const uint64_t t0 = global_timer_ns();
+    while (global_timer_ns() - t0 < 1000000ull) __nanosleep(10000);
+}
+
 __device__ __forceinline__ uint32_t ld_acquire_gpu_u32(const uint32_t *p) {
     uint32_t v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
