@@ -16,10 +16,12 @@ def layers():
 
     gen = torch.Generator(device=DEV).manual_seed(5)
     out = []
-    # decode with an adapter, K in parts, strip kernel, split-K, prefill (its workspace is larger), K in parts again
+    # decode with an adapter, K in parts, strip kernel, d_in no multiple of 256, prefill (its workspace is larger), K in
+    # parts again, the split-K kernel (a rank the decode kernel does not multiply)
     for rows, k, n, r, layout, dt in ((4, 512, 256, 16, 0, torch.bfloat16), (3, 8192, 192, 8, 0, torch.bfloat16),
                                       (2, 256, 320, 4, 1, torch.float32), (5, 320, 192, 8, 0, torch.bfloat16),
-                                      (40, 256, 192, 16, 0, torch.bfloat16), (16, 4352, 64, 64, 0, torch.bfloat16)):
+                                      (40, 256, 192, 16, 0, torch.bfloat16), (16, 4352, 64, 64, 0, torch.bfloat16),
+                                      (5, 1024, 192, 24, 0, torch.bfloat16)):
         rnd = lambda *s: torch.randn(*s, device=DEV, generator=gen)  # noqa: E731
         a, b = ((r, k), (n, r)) if layout == 0 else ((k, r), (r, n))
         out.append((rnd(rows, k).to(dt), PackedNf4Tensor.quantize(rnd(k * n) * 0.02), k, n, layout,

@@ -176,9 +176,9 @@ def test_general_kernel_in_out_layout_f32(oracle):
 @pytest.mark.parametrize("rows,d_in,d_out,r,dq,f32", [
     (1, 4096, 11008, 16, False, True),     # the decode configuration in the reference's orientation and types
     (4, 4096, 11008, 16, True, False),     # bf16 activations, double-quantized scales
-    (16, 1024, 4096, 8, False, True),      # two launches of eight activation rows
-    (40, 512, 320, 3, True, True),         # five launches (rank 3: not for the tensor-core path); strip narrower than 256 columns at the end
-    (3, 100, 64, 0, False, True),          # one strip, K shorter than two pieces
+    (16, 1024, 4096, 8, False, True),      # one launch of sixteen activation rows
+    (40, 512, 320, 3, True, True),         # three launches (rank 3: not for the tensor-core path); strip narrower than 256 columns at the end
+    (3, 100, 64, 0, False, True),          # one strip, K ends inside its second unit of 64 rows
     (8, 18944, 3584, 16, False, False),    # the block's down projection
 ])
 def test_reference_orientation_at_decode_sizes(oracle, rows, d_in, d_out, r, dq, f32):
@@ -290,7 +290,7 @@ def test_f32_tensors_at_prefill_sizes(oracle, rows, d_in, d_out, r, dq, bias):
     (5, 4096, 11008, 16, True, True),
     (16, 1024, 768, 12, False, True),      # two passes of eight rows; a rank the decode kernel itself would refuse
     (3, 18944, 512, 8, False, False),      # K in parts
-    (2, 320, 192, 4, False, True),         # d_in no multiple of 256: the split-K tensor-core kernel
+    (2, 320, 192, 4, False, True),         # d_in no multiple of 256: scales fetched block by block
 ])
 def test_f32_tensors_at_decode_sizes(oracle, rows, d_in, d_out, r, dq, bias):
     # W [d_out, d_in] with f32 activations and factors at up to 16 rows: every row goes through the
@@ -462,7 +462,7 @@ def test_qwen2_7b_block_decode_batch_8(oracle, dq):
     (520, 256, 304, 8, False, False),     # three activation tiles x three weight tiles, narrow adapter
     (512, 4096, 256, 16, False, True),    # four tiles over ten CTAs: a tile's k-stages split three ways
     (300, 3072, 200, 64, True, True),     # four ragged tiles over eight CTAs, adapter stages on the finishing CTA only
-    (768, 1536, 6400, 16, False, False),  # 150 tiles on 148 CTAs: every CTA takes a little more than one tile
+    (768, 1536, 6400, 16, False, False),  # 75 tiles on 74 pairs of CTAs: every pair takes a little more than one tile
 ])
 def test_prefill_shapes(oracle, M, K, N, r, dq, bias):
     c = make_case(oracle, 5000 + M + K + N, M, K, N, r, dq=dq, bias=bias)

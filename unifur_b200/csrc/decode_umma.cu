@@ -1,8 +1,8 @@
 // Decode path, tcgen05 version: y[M<=16, N] = x * dequant(W)^T (+bias) (+ s * (x A^T) B^T) with
 // W packed NF4 [N, K], 64-blocks along K.  HBM-bound; every byte of W is read once.
 //
-// Where it is used: shapes the warp-MMA decode kernel does not take (d_in above 4096, e.g. an
-// 18944-wide down projection).  Measured on B200, a tcgen05.mma whose A operand sits in TMEM
+// Where it is used: what the warp-MMA decode kernel does not take (adapter ranks up to 64 other than 8, 16, 32
+// and 64; d_in above 32768).  Measured on B200, a tcgen05.mma whose A operand sits in TMEM
 // costs ~130-150 cycles whatever N is, so one MMA per 2048 weights bounds this kernel near
 // 10 us for the 11008 x 4096 layer; the warp-MMA kernel is faster wherever both apply.
 //

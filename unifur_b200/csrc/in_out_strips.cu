@@ -15,8 +15,10 @@
 // word with {8 lane, 0, 1, 0} is the whole address; the 64-bit entry is an operand of a packed
 // multiply-add (fma.rn.f32x2) as it is.  Three instructions per two weights at one row (eight per weight
 // in the kernel before, which scaled every weight, added the table's base and multiplied single f32).
-// What bounds it: two shared-memory wavefronts per lookup (5 us for 45 M weights) and, at few rows, the
-// ends of the segments; from about eight rows on the f32 rate.  f32 x [M, 4096], W [4096, 11008], f32
+// What bounds it.  At one row neither pipe: of 15.7 us the lookups' shared-memory wavefronts are 5.9 (two per lookup)
+// and the instructions 4.4 (3.6 per weight with everything around the loop); the rest is latency at the ends of the
+// segments: the first codes from idle, the barriers around a piece of x, the meeting of a strip's segments.  From
+// about eight rows on the f32 rate.  f32 x [M, 4096], W [4096, 11008], f32
 // scales, calls back to back, before -> now: 29.8 -> 16.4 us at one row, 36.4 -> 21.2 at four, 49.1 -> 31.2 at
 // eight, 88.6 -> 55.9 at sixteen.
 //

@@ -98,8 +98,8 @@ __device__ __forceinline__ void quantize_block_by_warp(const float *values, uint
 // `ngroups` groups of eight values make up the full 64-blocks; a ragged last block (`rest` values) is one
 // more warp's work in the same launch.
 // The loads of a warp's next chunk are in flight while it encodes one: without that a warp's 1 KB
-// arrives, is encoded and only then replaced, and half of the time went to waiting (4096 x 4096:
-// 17.6 us; 22.8 with the slower code selection).
+// arrives, is encoded and only then replaced, and half of the time went to waiting (4096 x 4096 from
+// rotating buffers: 15.4 us; 22.8 with the slower code selection and without that).
 template <bool PACKED>
 __global__ void __launch_bounds__(kThreads, 6)
 quantize_full_kernel(const float *__restrict__ values, uint32_t ngroups, uint32_t rest,
@@ -236,9 +236,11 @@ dequantize_generic_kernel(const uint8_t *__restrict__ codes, uint64_t len,
 // c: a column segment of src.
 // Two lanes (kSplit) share a column of f32, or a pair of columns of bf16 (one 32-bit word per row):
 // each keeps 32 of the segment's 64 rows in registers, so a warp's load touches 64 bytes of two rows,
-// 32 loads are in flight per thread, a block's maximum is one shuffle and its codes leave as one sector.  No shared-memory transpose.  CTAs that are neighbours in launch order
-// take neighbouring row segments, so the sectors of an output line meet in the L2.
-// Bound by instruction issue (14 per value: half of them select the code) and the L2's tag lookups.
+// 32 loads are in flight per thread, a block's maximum is one shuffle and its codes leave as one
+// sector.  No shared-memory transpose.  CTAs that are neighbours in launch order take neighbouring row
+// segments, so the sectors of an output line meet in the L2.
+// Bound by instruction issue for a little over half of its time (14.7 per value, half of them to select
+// the code: 23 us) and by waiting for its loads (28 warps an SM) and for the fence at the end.
 // bf16 [14336, 4096]: 40 us; 92 through a 64 x 64 tile in shared memory with eight lanes per block; 49
 // with all 64 rows in one thread's registers (twenty warps per SM) and with sixteen rows per thread
 // (32-byte pieces of four rows per load: the L2 was busy with lookups).
