@@ -1,155 +1,167 @@
-// The adapter's gradients for bf16 tensors on warp MMAs:
+// The adapter's gradients for bf16 tensors on the tensor cores:
 //   grad_A(k, j) = s sum_m x[m][k] U[m][j],   grad_B(j, n) = s sum_m T[m][j] grad_y[m][n],
 // T = x A, U = grad_y B^T from the pre-pass kernel as bf16 high and low halves (their f32 values survive:
 // two MMAs per tile).
 //
-// gradient_kernel: out(p, j) = s sum_m X[m][p] R[m][j] as D[p][j] += A[p][m] B[m][j] (m16n8k16).  A CTA takes
-// 128 columns p, 64 ranks and a share of the rows; 64 rows of X and R per stage come by 16-byte
-// asynchronous copies, three stages in flight, and both operands are transposing matrix loads of what lies
-// there.  Eight warps: four pieces of 32 columns, two halves of a stage's rows.  The CTAs that share a tile's
-// rows form a cluster: their sums meet through distributed shared memory, each adds (in rank order) and writes its part
-// of the columns.  Bound by reading X once and, at few columns, by the chain of a load, its stages and that
-// exchange; sums through the workspace, added by the CTA that arrived last, took 25 us for [2048, 4096] (now
-// 17) and 45 for [2048, 14336] (now 40) at rank 64.
+// gradient_kernel: out(p, j) = s sum_m X[m][p] R[m][j] as D[p][j] += X^T R (tcgen05, both operands MN-major as they lie).  A
+// CTA takes 128 columns p, 64 ranks and a share of the rows; stages of 64 rows of X and of both halves of R (32 KB) come
+// by TMA, three in flight and two CTAs on an SM; one thread asks for them and one issues their MMAs.  The CTAs that share a
+// tile's rows form a cluster: their sums meet through distributed shared memory, each adds (in rank order) and writes its
+// part of the columns.  Bound by reading X once and R from the L2 for every 128 columns and, at few columns, by the chain
+// of a load, its stages and that exchange.  Warp MMAs behind transposing loads, whose pipe was half busy, took 40 us
+// for [2048, 14336] and 17 for [2048, 4096] at rank 64.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
 #include "kernels.cuh"
 #include "ptx.cuh"
+#include "tmap.cuh"
 
 namespace nf4 {
 namespace {
 
-constexpr uint32_t kThreads = 256, kCols = 128, kRowsStage = 64, kStages = 3;
-constexpr uint32_t kPitch = 272;                           // 256 bytes of a row and 16 of padding
-constexpr uint32_t kXStage = kRowsStage * kPitch, kStage = 2 * kXStage;
-constexpr uint32_t kSumPitch = 68;                         // floats
+constexpr uint32_t kThreads = 192, kCols = 128, kRowsStage = 64, kStages = 3;
+constexpr uint32_t kBox = kRowsStage * 128, kStage = 4 * kBox;  // X: two boxes of 64 columns; R: high and low halves
+constexpr uint32_t kSmem = kStages * kStage + 1024;
+constexpr uint32_t kSumPitch = 68;                              // floats
 static_assert(kCols * kSumPitch * 4 <= kStages * kStage, "the sums reuse the stages");
 
 struct Params {
-    const __nv_bfloat16 *x, *r;   // [rows][P]; [rows][2 * 64 * chunks]: hi halves, then lo
     __nv_bfloat16 *out;
     uint32_t rows, P, rank, chunks, stages_per_share, p_major;
     float scale;
 };
 
-__global__ void __launch_bounds__(kThreads, 2) gradient_kernel(const Params p) {
+__global__ void __launch_bounds__(kThreads, 2)
+gradient_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_r, const Params p, const FailureRef failure) {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
-    extern __shared__ __align__(16) uint8_t smem[];
+    extern __shared__ uint8_t smem_any[];
+    __shared__ __align__(8) uint64_t s_bars[2 * kStages + 1];
+    __shared__ uint32_t s_tmem;
+    uint8_t *const smem = smem_any + (1024u - (ptx::smem_addr(smem_any) & 1023u)) % 1024u;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-    const uint32_t g = lane >> 2, t = lane & 3u, li = lane >> 3, lr = lane & 7u;
-    const uint32_t pw = warp & 3u, h = warp >> 2;
-    const uint32_t shares = cluster.num_blocks(), share = cluster.block_rank(), p0 = blockIdx.x / shares * kCols;
+    const uint32_t shares = cluster.num_blocks(), share = cluster.block_rank(), p0 = blockIdx.x / shares * kCols, chunk = blockIdx.y;
     const uint32_t st0 = share * p.stages_per_share;
     const uint32_t all = (p.rows + kRowsStage - 1) / kRowsStage;
     const uint32_t nst = st0 < all ? min(p.stages_per_share, all - st0) : 0u;
-    const uint32_t base = ptx::smem_addr(smem), ld_r = 128 * p.chunks;
+    const uint32_t base = ptx::smem_addr(smem), full0 = ptx::smem_addr(s_bars), empty0 = full0 + 8 * kStages, acc_bar = empty0 + 8 * kStages;
+    const uint32_t ranks = min(64u, p.rank - chunk * 64), n16 = (ranks + 15) / 16 * 16;
     float *sum = reinterpret_cast<float *>(smem);
+    if (tid == 0) {
+        for (uint32_t s = 0; s < kStages; ++s) {
+            ptx::mbar_init(full0 + 8 * s, 1);
+            ptx::mbar_init(empty0 + 8 * s, 1);
+        }
+        ptx::mbar_init(acc_bar, 1);
+        ptx::fence_mbar_init();
+        ptx::fence_proxy_async();
+        ptx::prefetch_tmap(&tmap_x);
+        ptx::prefetch_tmap(&tmap_r);
+    }
+    if (warp == 1) {
+        ptx::tmem_alloc(ptx::smem_addr(&s_tmem), 64);
+        ptx::tmem_relinquish();
+    }
+    ptx::tc_fence_before();
+    __syncthreads();
+    ptx::tc_fence_after();
+    const uint32_t acc = s_tmem;
     ptx::pdl_launch_dependents();
     ptx::pdl_wait();
-    for (uint32_t chunk = 0; chunk < p.chunks; ++chunk) {
-        const uint32_t ranks = min(64u, p.rank - chunk * 64), tiles16 = (ranks + 15) / 16;
-        auto load = [&](uint32_t st) {
-            if (st < nst) {
-                const uint32_t m0 = (st0 + st) * kRowsStage, dst = base + (st % kStages) * kStage;
-                #pragma unroll
-                for (uint32_t q = 0; q < 4; ++q) {  // X: 64 rows x 16 pieces of eight columns
-                    const uint32_t i = tid + q * kThreads, r = i >> 4, c = i & 15u;
-                    const bool real = m0 + r < p.rows && p0 + c * 8 < p.P;
-                    ptx::cp_async_16_or_zero(dst + r * kPitch + c * 16, p.x + (real ? (size_t)(m0 + r) * p.P + p0 + c * 8 : 0), real);
-                }
-                #pragma unroll
-                for (uint32_t q = 0; q < 4; ++q) {  // R: 64 rows x (8 pieces of hi, 8 of lo)
-                    const uint32_t i = tid + q * kThreads, r = i >> 4, c = i & 15u;
-                    if ((c & 7u) >= 2 * tiles16) continue;
-                    const bool real = m0 + r < p.rows;
-                    const size_t at = (size_t)(m0 + r) * ld_r + (c >> 3) * 64 * p.chunks + chunk * 64 + (c & 7u) * 8;
-                    ptx::cp_async_16_or_zero(dst + kXStage + r * kPitch + c * 16, p.r + (real ? at : 0), real);
-                }
+    bool ok = true;
+    if (warp == 0) {
+        for (uint32_t st = 0; lane == 0 && st < nst; ++st) {
+            const uint32_t s = st % kStages, full = full0 + 8 * s, dst = base + s * kStage;
+            const int32_t m = (int32_t)((st0 + st) * kRowsStage);
+            if (st >= kStages && !ptx::mbar_wait_suspended(empty0 + 8 * s, (st / kStages + 1) & 1u)) {
+                ok = false;
+                NF4_REPORT_FAILURE(*failure.flag, *failure.host, 12);
+                break;
             }
-            ptx::cp_async_commit();
-        };
-        float acc[2][8][4];
-        #pragma unroll
-        for (int a = 0; a < 2; ++a)
-            #pragma unroll
-            for (int u = 0; u < 8; ++u) acc[a][u][0] = acc[a][u][1] = acc[a][u][2] = acc[a][u][3] = 0.0f;
-        load(0);
-        load(1);
+            ptx::mbar_arrive_expect_tx(full, kStage);
+            ptx::tma_load_2d(dst, &tmap_x, (int32_t)p0, m, full);
+            ptx::tma_load_2d(dst + kBox, &tmap_x, (int32_t)p0 + 64, m, full);
+            ptx::tma_load_2d(dst + 2 * kBox, &tmap_r, (int32_t)(chunk * 64), m, full);
+            ptx::tma_load_2d(dst + 3 * kBox, &tmap_r, (int32_t)((p.chunks + chunk) * 64), m, full);
+        }
+    } else if (warp == 1) {
+        const uint32_t idesc = ptx::f16_idesc(1, 128, n16, true, true);
         for (uint32_t st = 0; st < nst; ++st) {
-            ptx::cp_async_wait<1>();
-            __syncthreads();
-            load(st + 2);
-            const uint32_t xs = base + (st % kStages) * kStage, rs = xs + kXStage;
+            const uint32_t s = st % kStages;
+            ok = ptx::mbar_wait_suspended(full0 + 8 * s, (st / kStages) & 1u);
+            if (!ok) {
+                if (lane == 0) NF4_REPORT_FAILURE(*failure.flag, *failure.host, 13);
+                break;
+            }
+            ptx::tc_fence_after();
+            if (ptx::elect_one()) {
+                const uint64_t a = ptx::sw128_desc(base + s * kStage, kBox), hi = ptx::sw128_desc(base + s * kStage + 2 * kBox),
+                               lo = ptx::sw128_desc(base + s * kStage + 3 * kBox);
+                #pragma unroll
+                for (uint32_t i = 0; i < 4; ++i) {  // sixteen rows: 2 KB
+                    ptx::mma_ss_f16(acc, a + 128 * i, hi + 128 * i, idesc, (st | i) != 0);
+                    ptx::mma_ss_f16(acc, a + 128 * i, lo + 128 * i, idesc, 1);
+                }
+                ptx::tc_commit(empty0 + 8 * s);
+                if (st + 1 == nst) ptx::tc_commit(acc_bar);
+            }
+            __syncwarp();
+        }
+    }
+    if (!ok) ptx::let_flights_land();
+    __syncwarp();
+    __syncthreads();
+    if (warp >= 2) {  // a lane a column p; ranks that there are not are zeros
+        if (nst && !ptx::mbar_wait_suspended(acc_bar, 0)) {
+            if (lane == 0) NF4_REPORT_FAILURE(*failure.flag, *failure.host, 14);
+        }
+        ptx::tc_fence_after();
+        const uint32_t q = warp & 3u;
+        #pragma unroll
+        for (uint32_t c = 0; c < 64; c += 16) {
+            uint32_t v[16];
+            ptx::tmem_ld16(acc + ((q * 32) << 16) + c, v);
+            ptx::tmem_wait_ld();
+            const bool real = c < n16 && nst;
+            float4 *dst = reinterpret_cast<float4 *>(sum + (q * 32 + lane) * kSumPitch + c);
             #pragma unroll
-            for (uint32_t k2 = 0; k2 < 2; ++k2) {
-                const uint32_t m = (2 * h + k2) * 16;
-                uint32_t af[2][4];
-                #pragma unroll
-                for (int a = 0; a < 2; ++a)
-                    ptx::ldmatrix_x4_trans(af[a], xs + (m + (li >> 1) * 8 + lr) * kPitch + (pw * 32 + a * 16 + (li & 1u) * 8) * 2);
-                const uint32_t b_at = rs + (m + (li & 1u) * 8 + lr) * kPitch + (li >> 1) * 16;
-                #pragma unroll
-                for (uint32_t u = 0; u < 4; ++u) {
-                    if (u >= tiles16) break;
-                    #pragma unroll
-                    for (uint32_t half = 0; half < 2; ++half) {  // hi, then lo
-                        uint32_t bf[4];
-                        ptx::ldmatrix_x4_trans(bf, b_at + half * 128 + u * 32);
-                        #pragma unroll
-                        for (int a = 0; a < 2; ++a) {
-                            ptx::mma_16816_bf16(acc[a][2 * u], af[a][0], af[a][1], af[a][2], af[a][3], bf[0], bf[1]);
-                            ptx::mma_16816_bf16(acc[a][2 * u + 1], af[a][0], af[a][1], af[a][2], af[a][3], bf[2], bf[3]);
-                        }
-                    }
-                }
+            for (int i = 0; i < 4; ++i)
+                dst[i] = real ? make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]), __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]))
+                              : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+        ptx::tc_fence_before();
+    }
+    if (shares > 1) cluster.sync();
+    else __syncthreads();
+    const uint32_t per = kCols / shares, per_log = __ffs(per) - 1, q0 = share * per;  // columns of this CTA's part
+    if (shares > 1) {  // (the others read their own parts of this CTA's sums: this one may be overwritten)
+        #pragma unroll 2
+        for (uint32_t i = tid; i < per * 16; i += kThreads) {
+            if ((i & 15u) * 4 >= n16) continue;
+            const uint32_t at = (q0 + (i >> 4)) * kSumPitch + (i & 15u) * 4;
+            float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            #pragma unroll 8
+            for (uint32_t c = 0; c < shares; ++c) {
+                const float4 o = *reinterpret_cast<const float4 *>(cluster.map_shared_rank(sum, c) + at);
+                v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
             }
+            *reinterpret_cast<float4 *>(sum + at) = v;
         }
-        ptx::cp_async_wait<0>();
-        // the two halves of the rows, in order
-        for (uint32_t turn = 0; turn < 2; ++turn) {
-            __syncthreads();
-            if (h == turn) {
-                #pragma unroll
-                for (int a = 0; a < 2; ++a)
-                    #pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        float2 *lo = reinterpret_cast<float2 *>(sum + (pw * 32 + a * 16 + g) * kSumPitch + u * 8 + 2 * t);
-                        float2 *hi = reinterpret_cast<float2 *>(sum + (pw * 32 + a * 16 + g + 8) * kSumPitch + u * 8 + 2 * t);
-                        const float2 l = turn ? *lo : make_float2(0.0f, 0.0f), hh = turn ? *hi : make_float2(0.0f, 0.0f);
-                        *lo = make_float2(l.x + acc[a][u][0], l.y + acc[a][u][1]);
-                        *hi = make_float2(hh.x + acc[a][u][2], hh.y + acc[a][u][3]);
-                    }
-            }
-        }
-        if (shares > 1) cluster.sync();
-        else __syncthreads();
-        const uint32_t per = kCols / shares, per_log = __ffs(per) - 1, q0 = share * per;  // columns of this CTA's part
-        if (shares > 1) {  // (the others read their own parts of this CTA's sums: this one may be overwritten)
-            #pragma unroll 2
-            for (uint32_t i = tid; i < per * 16; i += kThreads) {
-                if ((i & 15u) >= 4 * tiles16) continue;
-                const uint32_t at = (q0 + (i >> 4)) * kSumPitch + (i & 15u) * 4;
-                float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                #pragma unroll 8
-                for (uint32_t c = 0; c < shares; ++c) {
-                    const float4 o = *reinterpret_cast<const float4 *>(cluster.map_shared_rank(sum, c) + at);
-                    v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
-                }
-                *reinterpret_cast<float4 *>(sum + at) = v;
-            }
-            __syncthreads();
-        }
-        for (uint32_t i = tid; i < per * 64; i += kThreads) {
-            // p fastest for [rank][P] outputs, j fastest for [P][rank]
-            const uint32_t q = q0 + (p.p_major ? i >> 6 : i & (per - 1)), j = p.p_major ? i & 63u : i >> per_log;
-            const uint32_t pp = p0 + q, jj = chunk * 64 + j;
-            if (pp < p.P && j < ranks)
-                p.out[p.p_major ? (size_t)pp * p.rank + jj : (size_t)jj * p.P + pp] = __float2bfloat16_rn(__fmul_rn(sum[q * kSumPitch + j], p.scale));
-        }
-        if (shares > 1) cluster.sync();
-        else __syncthreads();  // the sums have been read (before the next chunk's stages, and before a CTA leaves)
+        __syncthreads();
+    }
+    for (uint32_t i = tid; i < per * 64; i += kThreads) {
+        // p fastest for [rank][P] outputs, j fastest for [P][rank]
+        const uint32_t q = q0 + (p.p_major ? i >> 6 : i & (per - 1)), j = p.p_major ? i & 63u : i >> per_log;
+        const uint32_t pp = p0 + q, jj = chunk * 64 + j;
+        if (pp < p.P && j < ranks)
+            p.out[p.p_major ? (size_t)pp * p.rank + jj : (size_t)jj * p.P + pp] = __float2bfloat16_rn(__fmul_rn(sum[q * kSumPitch + j], p.scale));
+    }
+    if (shares > 1) cluster.sync();  // the sums have been read, before a CTA leaves
+    else __syncthreads();
+    if (warp == 1) {
+        ptx::tc_fence_after();
+        ptx::tmem_dealloc(acc, 64);
     }
 }
 
@@ -160,8 +172,6 @@ uint64_t tiles_of(uint64_t P) { return (P + kCols - 1) / kCols; }
 int32_t gradient(const void *x, const void *r, void *out, uint64_t rows, uint64_t P, uint32_t rank, float scale, bool p_major,
                  cudaStream_t s) {
     Params p{};
-    p.x = static_cast<const __nv_bfloat16 *>(x);
-    p.r = static_cast<const __nv_bfloat16 *>(r);
     p.out = static_cast<__nv_bfloat16 *>(out);
     p.rows = (uint32_t)rows;
     p.P = (uint32_t)P;
@@ -170,17 +180,23 @@ int32_t gradient(const void *x, const void *r, void *out, uint64_t rows, uint64_
     // Shares of the rows: as many as the chip holds clusters for at once, where a share keeps four stages (256 rows)
     const void *kernel = reinterpret_cast<const void *>(gradient_kernel);
     ClusterRoom room;
-    NF4_TRY(cluster_room(kernel, kThreads, kStages * kStage, &room));
+    NF4_TRY(cluster_room(kernel, kThreads, kSmem, &room));
     const uint32_t shares = cluster_ctas(tiles_of(P), rows, 4 * kRowsStage, room);
     const uint32_t all = (uint32_t)((rows + kRowsStage - 1) / kRowsStage);
     p.stages_per_share = (all + shares - 1) / shares;
     p.p_major = p_major;
     p.scale = scale;
     if (tiles_of(P) * shares >= (1ull << 31)) return fail(NF4_ERR_UNSUPPORTED, "gradient: too many columns");
+    CUtensorMap map_x, map_r;
+    const uint64_t ld_r = 2 * 64 * (uint64_t)p.chunks;
+    NF4_TRY(make_map(&map_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, x, rows, P, P * 2, kRowsStage, 64, CU_TENSOR_MAP_SWIZZLE_128B));
+    NF4_TRY(make_map(&map_r, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, r, rows, ld_r, ld_r * 2, kRowsStage, 64, CU_TENSOR_MAP_SWIZZLE_128B));
+    FailureRef failure;
+    NF4_TRY(prefill_failure_ref(&failure));
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(tiles_of(P) * shares));
+    cfg.gridDim = dim3((unsigned)(tiles_of(P) * shares), p.chunks);
     cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = kStages * kStage;
+    cfg.dynamicSmemBytes = kSmem;
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -191,7 +207,7 @@ int32_t gradient(const void *x, const void *r, void *out, uint64_t rows, uint64_
     cfg.attrs = attr;
     cfg.numAttrs = shares > 1 ? 2 : 1;
     count_launch();
-    return check_cuda(cudaLaunchKernelEx(&cfg, gradient_kernel, p), "gradient_kernel launch");
+    return check_cuda(cudaLaunchKernelEx(&cfg, gradient_kernel, map_x, map_r, p, failure), "gradient_kernel launch");
 }
 
 }  // namespace

@@ -122,6 +122,12 @@ int32_t decode_selftest_wait(uint32_t limit_ns, unsigned long long *waited_ns_de
 int32_t decode_error_flag_ptr(int **dev_ptr);
 int32_t decode2_error_flag_ptr(int **dev_ptr);
 int32_t prefill_error_flag_ptr(int **dev_ptr);
+// where the kernels around the tensor-core GEMM report a failure: its flag and the place of its host word (current device)
+struct FailureRef {
+    int *flag;
+    int **host;
+};
+int32_t prefill_failure_ref(FailureRef *ref);
 uint64_t decode_static_scratch_bytes();
 int32_t decode_forward_static_scratch(const nf4_linear_args &a, cudaStream_t stream);
 

@@ -59,6 +59,7 @@
 
 #include "kernels.cuh"
 #include "ptx.cuh"
+#include "tmap.cuh"
 
 namespace nf4 {
 
@@ -186,38 +187,6 @@ struct WorkList {
 __device__ __forceinline__ uint32_t tile_columns(uint32_t M, uint32_t m0) {
     const uint32_t left = M - m0;
     return left < BN ? (left + 31) / 32 * 32 : BN;
-}
-
-// ---- descriptors -----------------------------------------------------------------
-// Shared-memory matrix descriptor, K-major operand, 128-byte swizzle: rows are 128 B apart,
-// 8-row groups 1024 B apart (SBO), version 1, layout type 2 (SWIZZLE_128B).
-__device__ __forceinline__ uint64_t make_kmajor_sw128_desc(uint32_t smem_byte_addr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_byte_addr & 0x3FFFFu) >> 4);  // start address, bits [0,14)
-    d |= (uint64_t)1 << 16;                              // LBO (unused for swizzled K-major)
-    d |= (uint64_t)(1024 >> 4) << 32;                    // SBO, bits [32,46)
-    d |= (uint64_t)1 << 46;                              // descriptor version
-    d |= (uint64_t)2 << 61;                              // SWIZZLE_128B
-    return d;
-}
-
-// Instruction descriptor for kind::f16: f32 accumulate, K-major A and B.
-// a_fmt / b_fmt: 0 = f16, 1 = bf16.
-__host__ __device__ constexpr uint32_t make_idesc(uint32_t a_fmt, uint32_t b_fmt, uint32_t m,
-                                                  uint32_t n) {
-    return (1u << 4) | (a_fmt << 7) | (b_fmt << 10) | ((n >> 3) << 17) | ((m >> 4) << 24);
-}
-
-// ---- TMEM load (32 lanes x 32-bit, 16 consecutive columns) -------------------------------
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,"
-        "%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-          "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
 }
 
 // ---- TMEM store (32 lanes x 32-bit, 32 consecutive columns) ------------------------------
@@ -386,13 +355,13 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 uint32_t tile, kb, ke;
                 wl.get(seg, tile, kb, ke);
                 const uint32_t columns = tile_columns(p.M, (tile % p.m_tiles) * BN);
-                const uint32_t idesc_main = make_idesc(0, 0, 2 * BM, columns);  // f16 x f16
-                const uint32_t idesc_lora = make_idesc(1, 1, 2 * BM, columns);  // bf16 x bf16
+                const uint32_t idesc_main = ptx::f16_idesc(0, 2 * BM, columns, false, false);  // f16 x f16
+                const uint32_t idesc_lora = ptx::f16_idesc(1, 2 * BM, columns, false, false);  // bf16 x bf16
                 // the epilogues must have read the previous segment out of the accumulators
                 ok = ptx::mbar_wait_suspended(bar(kBarAccEmpty), (seg & 1u) ^ 1u);
                 for (uint32_t ks = kb; ks < ke && ok; ++ks, ++cnt) {
                     const uint32_t s = cnt % kAStages;
-                    const uint64_t bdesc = make_kmajor_sw128_desc(kXAt + (cnt % kXStages) * kXTileBytes);
+                    const uint64_t bdesc = ptx::sw128_desc(kXAt + (cnt % kXStages) * kXTileBytes);
                     const uint32_t a_cols = tmem_a + s * kAStageCols;
                     ok = ptx::mbar_wait_suspended(bar(kBarFull + s), (cnt / kAStages) & 1u);
                     if (!ok) break;
@@ -411,8 +380,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 for (uint32_t j = 0; ke == k_stages && j < lora_stages && ok; ++j, ++cnt) {
                     const uint32_t s = cnt % kAStages;
                     const uint32_t left = p.rank - j / 2 * 64, nk16 = ((left < 64 ? left : 64) + 15) / 16;
-                    const uint64_t adesc = make_kmajor_sw128_desc(kLoraAt);
-                    const uint64_t bdesc = make_kmajor_sw128_desc(kXAt + (cnt % kXStages) * kXTileBytes);
+                    const uint64_t adesc = ptx::sw128_desc(kLoraAt);
+                    const uint64_t bdesc = ptx::sw128_desc(kXAt + (cnt % kXStages) * kXTileBytes);
                     ok = ptx::mbar_wait_suspended(bar(kBarFull + s), (cnt / kAStages) & 1u);
                     if (!ok) break;
                     ptx::tc_fence_after();
@@ -468,7 +437,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 uint32_t v[16];
                 for (uint32_t k = 0; k < kLoads; ++k) {
                     if (m0 + col_of(k) >= p.M) continue;  // rows that do not exist
-                    tmem_ld16(acc_lane + col_of(k), v);
+                    ptx::tmem_ld16(acc_lane + col_of(k), v);
                     ptx::tmem_wait_ld();
                     float *dst = own_partial + (size_t)col_of(k) * BM;
                     #pragma unroll
@@ -502,7 +471,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             if (!ok) break;
             ptx::tc_fence_after();
             uint32_t va[16], vb[16];
-            tmem_ld16(acc_lane + col_of(0), va);
+            ptx::tmem_ld16(acc_lane + col_of(0), va);
             // staging layout: [kStageRows activation rows][BM weight rows]
             auto stage_chunk = [&](const uint32_t (&v)[16], uint32_t col) {
                 const uint32_t r0 = col % kStageRows;
@@ -560,13 +529,13 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                     asm volatile("bar.sync 1, 256;" ::: "memory");
                 }
                 ptx::tmem_wait_ld();
-                tmem_ld16(acc_lane + col_of(k + 1), vb);
+                ptx::tmem_ld16(acc_lane + col_of(k + 1), vb);
                 if (first_helper != pair) add_helpers(va, col_of(k));
                 stage_chunk(va, col_of(k));
                 ptx::tmem_wait_ld();
                 if (first_helper != pair) add_helpers(vb, col_of(k + 1));
                 if (k + 2 < kLoads) {
-                    tmem_ld16(acc_lane + col_of(k + 2), va);
+                    ptx::tmem_ld16(acc_lane + col_of(k + 2), va);
                 } else {
                     // this warp's part of the accumulator is read: hand it back to the MMA threads
                     ptx::tc_fence_before();
@@ -923,41 +892,6 @@ __global__ void __launch_bounds__(256) repack_kernel(const RepackParams p) {
 }
 
 // ---- host side -----------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
-                                  const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
-                                  const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(p);
-    });
-    return fn;
-}
-
-// 2-D row-major tensor [rows][cols] with row pitch `pitch_bytes`; box = [box_rows][box_cols].
-int32_t make_map(CUtensorMap *map, CUtensorMapDataType dt, const void *base, uint64_t rows,
-                 uint64_t cols, uint64_t pitch_bytes, uint32_t box_rows, uint32_t box_cols,
-                 CUtensorMapSwizzle swz) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return fail(NF4_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-    cuuint64_t dims[2] = {cols, rows};
-    cuuint64_t strides[1] = {pitch_bytes};
-    cuuint32_t box[2] = {box_cols, box_rows};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = fn(map, dt, 2, const_cast<void *>(base), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(NF4_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d", (int)r);
-    return NF4_OK;
-}
-
 uint32_t lora_chunks_of(uint32_t rank) { return (rank + 63) / 64; }
 
 }  // namespace
@@ -1245,6 +1179,24 @@ int32_t prefill_share_plan(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_
 int32_t prefill_error_flag_ptr(int **dev_ptr) {
     return check_cuda(cudaGetSymbolAddress(reinterpret_cast<void **>(dev_ptr), g_prefill_error),
                       "address of the prefill error flag");
+}
+
+int32_t prefill_failure_ref(FailureRef *ref) {
+    static std::mutex mu;
+    static FailureRef of_device[64] = {};
+    int dev = 0;
+    NF4_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return fail(NF4_ERR_UNSUPPORTED, "device ordinal %d out of range", dev);
+    std::lock_guard<std::mutex> lock(mu);
+    if (!of_device[dev].flag) {
+        void *host = nullptr;
+        int *flag = nullptr;
+        NF4_CUDA_TRY(cudaGetSymbolAddress(&host, g_prefill_error_host));
+        NF4_TRY(prefill_error_flag_ptr(&flag));
+        of_device[dev] = FailureRef{flag, static_cast<int **>(host)};
+    }
+    *ref = of_device[dev];
+    return NF4_OK;
 }
 
 }  // namespace nf4
