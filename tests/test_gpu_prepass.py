@@ -45,6 +45,9 @@ def rel(got, ref):
     (513, 192, 136, 8, 0, False),      # 64 rows to a tile: one row in the last, stages of 128 k half empty
     (600, 1088, 128, 20, 1, False),    # the same, the factor [K, r] in odd places
     (545, 576, 64, 12, 0, True),       # f32, 64 rows to a tile
+    (1029, 4160, 64, 24, 0, False),    # from four million values on the tcgen05 kernel: ragged rows, ranks and pieces of K
+    (2050, 2112, 64, 64, 1, False),    # the factor [K, r] as the MMA's MN-major operand
+    (16500, 256, 64, 8, 0, False),     # a CTA by itself
     (1200, 2112, 64, 40, 1, True),
 ])
 def test_forward(M, K, N, r, layout, f32):
@@ -54,6 +57,18 @@ def test_forward(M, K, N, r, layout, f32):
     ref = x.double() @ w + 1.5 * (x.double() @ A) @ B
     per_row = ((y.double() - ref).norm(dim=1) / ref.norm(dim=1)).max()
     assert float(per_row) < (1e-3 if f32 else 4e-3)
+
+
+@pytest.mark.parametrize("first,std", [(0.0, 1.0), (float("inf"), 1.0), (3e38, 1e-4), (1e-30, 1.0), (1e-3, 1e-3)])
+def test_rows_far_from_the_first_values(first, std):
+    # The copy's common factor follows the first row's first values; rows it does not suit get their own.
+    # (Row 0 itself may be infinite.)  8 bits of x and 11 of the weights: the bound of the other forwards.
+    q, w, A, B, x, _ = layer(1030, 4096, 64, 16, 0, torch.bfloat16, 7, x_std=std)
+    x[0] = first
+    y = q.forward(x)
+    ref = x.double() @ w + 1.5 * (x.double() @ A) @ B
+    per_row = (y[1:].double() - ref[1:]).norm(dim=1) / ref[1:].norm(dim=1)
+    assert float(per_row.max()) < 4e-3
 
 
 @pytest.mark.parametrize("M,K,N,r,layout", [

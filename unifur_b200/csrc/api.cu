@@ -84,14 +84,15 @@ int32_t cluster_room(const void *kernel, uint32_t threads, uint32_t smem, Cluste
         }
     NF4_TRY(ensure_dynamic_smem(kernel, (int)smem));
     NF4_TRY(set_once(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    for (uint32_t i = 0; i < kClusterSizes; ++i) {
+    room->any[0] = 0;
+    for (uint32_t i = 1; i <= 1u << (kClusterSizes - 1); ++i) {
         cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(1u << i);
+        cfg.gridDim = dim3(i);
         cfg.blockDim = dim3(threads);
         cfg.dynamicSmemBytes = smem;
         cudaLaunchAttribute attr{};
         attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = 1u << i;
+        attr.val.clusterDim.x = i;
         attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
@@ -100,8 +101,9 @@ int32_t cluster_room(const void *kernel, uint32_t threads, uint32_t smem, Cluste
             (void)cudaGetLastError();  // (a size the device does not have)
             n = 0;
         }
-        room->of[i] = n > 0 ? (uint32_t)n : 0u;
+        room->any[i] = n > 0 ? (uint32_t)n : 0u;
     }
+    for (uint32_t i = 0; i < kClusterSizes; ++i) room->of[i] = room->any[1u << i];
     if (n_asked < 64) asked[n_asked++] = Asked{kernel, dev, *room};
     return NF4_OK;
 }

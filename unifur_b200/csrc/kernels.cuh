@@ -26,12 +26,13 @@ int32_t launch_maybe_overlapped(void (*kernel)(KArgs...), dim3 grid, dim3 block,
 // once per (kernel, device): the attribute belongs to the device a kernel is loaded on.
 int32_t ensure_dynamic_smem(const void *kernel, int bytes);
 
-// api.cu: how many clusters of 2^i CTAs of `kernel` the current device holds at once, by the driver's count (once
-// per kernel and device; 0: it has no place for one).  Sets the kernel's dynamic shared memory, and allows it clusters
+// api.cu: how many clusters of 2^i CTAs (`any`: of i CTAs) of `kernel` the current device holds at once, by the driver's
+// count (once per kernel and device; 0: it has no place for one).  Sets the kernel's dynamic shared memory, and allows it clusters
 // of sixteen.  (A whole B200, two CTAs of 108 KB on an SM: 148 of two, 71 of four, 33 of eight, 14 of sixteen.)
 constexpr uint32_t kClusterSizes = 5;
 struct ClusterRoom {
     uint32_t of[kClusterSizes];
+    uint32_t any[(1u << (kClusterSizes - 1)) + 1];
 };
 int32_t cluster_room(const void *kernel, uint32_t threads, uint32_t smem, ClusterRoom *room);
 // CTAs to a cluster when each takes a piece of a tile's `length`: as many as leave the tiles' clusters in one wave and

@@ -25,6 +25,7 @@
 
 #include "kernels.cuh"
 #include "ptx.cuh"
+#include "tmap.cuh"
 
 namespace nf4 {
 namespace {
@@ -105,6 +106,22 @@ __device__ __forceinline__ float row_factor(float mx) {
     int e;
     frexpf(mx, &e);  // mx = f * 2^e with f in [0.5, 1)
     return ldexpf(1.0f, e - 15 < -100 ? -100 : e - 15);
+}
+
+// Four sums times f as bf16 high halves at out[at], low halves `lo` elements on; out may be null.
+__device__ __forceinline__ void put_halves(__nv_bfloat16 *out, const float (&sum)[4], float f, size_t at, uint32_t lo) {
+    if (!out) return;
+    uint32_t hi[2], low[2];
+    #pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const float v0 = sum[2 * h] * f, v1 = sum[2 * h + 1] * f;
+        const __nv_bfloat162 b = __floats2bfloat162_rn(v0, v1);
+        const __nv_bfloat162 l = __floats2bfloat162_rn(v0 - __low2float(b), v1 - __high2float(b));
+        hi[h] = *reinterpret_cast<const uint32_t *>(&b);
+        low[h] = *reinterpret_cast<const uint32_t *>(&l);
+    }
+    *reinterpret_cast<uint2 *>(out + at) = make_uint2(hi[0], hi[1]);
+    *reinterpret_cast<uint2 *>(out + at + lo) = make_uint2(low[0], low[1]);
 }
 
 // MODE 0: bf16 x (products with the bf16 factor are exact).  MODE 1: f32 x; the products use the scaled
@@ -399,26 +416,318 @@ prepass_kernel(const Params p) {
             }
             if (m >= p.M) continue;
             const size_t at = (size_t)m * ld + chunk * 64 + c;
-            auto put = [&](__nv_bfloat16 *out, float f) {
-                uint32_t hi[2], lo[2];
-                #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const float v0 = sum[2 * h] * f, v1 = sum[2 * h + 1] * f;
-                    const __nv_bfloat162 b = __floats2bfloat162_rn(v0, v1);
-                    const __nv_bfloat162 l = __floats2bfloat162_rn(v0 - __low2float(b), v1 - __high2float(b));
-                    hi[h] = *reinterpret_cast<const uint32_t *>(&b);
-                    lo[h] = *reinterpret_cast<const uint32_t *>(&l);
-                }
-                *reinterpret_cast<uint2 *>(out + at) = make_uint2(hi[0], hi[1]);
-                *reinterpret_cast<uint2 *>(out + at + 64 * p.chunks) = make_uint2(lo[0], lo[1]);
-            };
             // (MODE 1: the products were taken with the scaled rows)
-            if (MODE != 2) put(p.t_out, F32 ? p.scale * w_down : p.scale * s_inv[r] * w_down);
-            if (MODE == 2 || p.r_out) put(p.r_out, 1.0f);
+            if (MODE != 2) put_halves(p.t_out, sum, F32 ? p.scale * w_down : p.scale * s_inv[r] * w_down, at, 64 * p.chunks);
+            put_halves(p.r_out, sum, 1.0f, at, 64 * p.chunks);
         }
         cluster.sync();  // the sums have been read (before the next chunk's stages, and before a CTA leaves)
     }
     if (p.wait == 2) ptx::pdl_wait();
+}
+
+// ---- the same for bf16 x and a factor on tcgen05: up to 64 ranks, rows of 16-byte pieces -------------------------------
+// A cluster takes kRows (128, 64 or 32) rows of x, each CTA a piece of K in stages of 64 k.  One thread asks for a stage
+// of x and of the factor by TMA (128-byte swizzle, a ring of eight stages), another issues its four MMAs (x the A
+// operand as it lies, 128 rows whatever kRows is: the rows behind the tile are somebody else's bytes and nobody reads
+// what they give; the factor the B operand, K-major as [r][K], MN-major as [K][r]), eight warps write the f16 copy and
+// keep the maxima.  Nothing in the loop waits for the whole CTA: the kernel above, with warp MMAs, a barrier a stage
+// and two stages in flight, ran at a fifth of the DRAM rate ([2048, 14336] at rank 64: 48 us; [2048, 4096]: 17.6).
+constexpr uint32_t kTcThreads = 384, kTcStages = 8, kTcFactorStage = 8192;
+__host__ __device__ constexpr uint32_t tc_ring(uint32_t rows) { return kTcStages * (rows * 128 + kTcFactorStage); }
+
+template <int MODE, uint32_t kRows, bool k_major>
+__global__ void __launch_bounds__(kTcThreads, 1)
+prepass_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_a, const Params p, const FailureRef failure) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    constexpr uint32_t kStages = kTcStages, kXStage = kRows * 128;
+    // Eight warps convert: one a stage, two where it has 128 rows; a lane eight k of every fourth row.  A warp has the same
+    // place of the ring every time (or two): it waits for all the place's rounds, so that a parity names the round.
+    constexpr uint32_t kPerStage = kRows == 128 ? 2 : 1, kGroups = 8 / kPerStage, kWarpRows = kRows / kPerStage, kQuads = kWarpRows / 4;
+    static_assert(kStages % kGroups == 0, "a warp's stages keep their places");
+    constexpr bool kCopy = MODE == 0;
+    static_assert(kRows * kPartPitch * 4 <= tc_ring(kRows), "the sums reuse the stages");
+    static_assert((kStages - 1) * kXStage + 128 * 128 <= tc_ring(kRows), "an MMA reads 128 rows from the last stage's place");
+    extern __shared__ uint8_t smem_any[];
+    __shared__ uint32_t s_max[kMaxCluster][kRows];   // the CTAs' row maxima (f32 patterns)
+    __shared__ float s_inv[kRows];
+    __shared__ uint32_t s_own[kRows];
+    __shared__ float s_shift;
+    __shared__ int s_exp;
+    __shared__ __align__(8) uint64_t s_bars[2 * kStages + 1];
+    __shared__ uint32_t s_tmem;
+    uint8_t *const smem = smem_any + (1024u - (ptx::smem_addr(smem_any) & 1023u)) % 1024u;
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    const uint32_t cn = cluster.num_blocks(), rank_in = cluster.block_rank();
+    const uint32_t m0 = (blockIdx.x / cn) * kRows, k0 = min(rank_in * p.piece, p.K), k1 = min(k0 + p.piece, p.K);
+    const uint32_t stages = (k1 - k0 + 63) / 64, base = ptx::smem_addr(smem), factor0 = base + kStages * kXStage;
+    const uint32_t full0 = ptx::smem_addr(s_bars), empty0 = full0 + 8 * kStages, acc_bar = empty0 + 8 * kStages;
+    float *part = reinterpret_cast<float *>(smem);
+    const uint32_t n16 = (p.rank + 15) / 16 * 16;
+
+    cluster.barrier_arrive();      // (waited for before the first access to another CTA's shared memory)
+    auto request = [&](uint32_t st) {
+        const uint32_t s = st % kStages, full = full0 + 8 * s;
+        const int32_t k = (int32_t)(k0 + st * 64);
+        ptx::mbar_arrive_expect_tx(full, kXStage + (k_major ? kTcFactorStage : n16 * 128));
+        ptx::tma_load_2d(base + s * kXStage, &tmap_x, k, (int32_t)m0, full);
+        ptx::tma_load_2d(factor0 + s * kTcFactorStage, &tmap_a, k_major ? 0 : k, k_major ? k : 0, full);
+    };
+    if (tid == 256) {  // (its loads are on their way while the others set up)
+        for (uint32_t s = 0; s < kStages; ++s) {
+            ptx::mbar_init(full0 + 8 * s, 1);
+            ptx::mbar_init(empty0 + 8 * s, (kCopy ? kPerStage : 0) + 1);
+        }
+        ptx::mbar_init(acc_bar, 1);
+        ptx::fence_mbar_init();
+        ptx::fence_proxy_async();
+        ptx::prefetch_tmap(&tmap_x);
+        ptx::prefetch_tmap(&tmap_a);
+        if (p.wait == 0) ptx::pdl_wait();
+        for (uint32_t st = 0; st < min(stages, kStages); ++st) request(st);
+    }
+    if (kCopy && tid < kRows) s_own[tid] = 0;
+    if (warp == 9) {
+        ptx::tmem_alloc(ptx::smem_addr(&s_tmem), 64);
+        ptx::tmem_relinquish();
+    }
+    ptx::tc_fence_before();
+    __syncthreads();
+    ptx::tc_fence_after();
+    if (p.wait == 0) ptx::pdl_wait();
+    ptx::pdl_launch_dependents();  // (what for: see the kernel above)
+    if (blockIdx.x == 0)
+        for (uint32_t i = tid; i < p.n_flags; i += kTcThreads) p.flags[i] = 0;
+    const uint32_t acc = s_tmem;
+    bool ok = true;
+    if (warp == 11) {
+        const int e = kCopy ? weight_exponent(p.absmax, p.scale_codes, p.scale_of_scales) : 0;
+        if (lane == 0) s_exp = e;
+    }
+    if (kCopy && warp == 10) {
+        // x comes over times a power of two that brings the largest of its first 256 values to [2, 4), so that the rows
+        // of a tensor of small values (gradients of 1e-3) do not all need their own factor and a second writing
+        uint32_t w = 0;
+        if (lane * 8 < p.K) {
+            const uint4 v = __ldg(static_cast<const uint4 *>(p.x) + lane);
+            w = bf16x2_absmax(v.x, bf16x2_absmax(v.y, bf16x2_absmax(v.z, bf16x2_absmax(v.w, 0))));
+        }
+        const uint32_t m = __reduce_max_sync(0xffffffffu, bf16x2_larger_bits(w)), e = m >> 23;  // 128: [2, 4)
+        if (lane == 0) s_shift = e > 27 && e < 228 ? __uint_as_float((255 - e) << 23) : 1.0f;
+    }
+    if (kCopy && (warp == 10 || warp < 8)) asm volatile("bar.sync 1, 288;" ::: "memory");
+
+    if (warp == 8) {
+        if (lane == 0) {
+            for (uint32_t st = kStages; st < stages; ++st) {
+                if (!ptx::mbar_wait_suspended(empty0 + 8 * (st % kStages), (st / kStages + 1) & 1u)) {
+                    ok = false;
+                    break;
+                }
+                request(st);
+            }
+            if (!ok) NF4_REPORT_FAILURE(*failure.flag, *failure.host, 8);
+        }
+    } else if (warp == 9) {
+        const uint32_t idesc = ptx::f16_idesc(1, 128, n16, false, k_major);
+        for (uint32_t st = 0; st < stages; ++st) {
+            const uint32_t s = st % kStages;
+            ok = ptx::mbar_wait_suspended(full0 + 8 * s, (st / kStages) & 1u);
+            if (!ok) break;
+            ptx::tc_fence_after();
+            if (ptx::elect_one()) {
+                const uint64_t a = ptx::sw128_desc(base + s * kXStage), b = ptx::sw128_desc(factor0 + s * kTcFactorStage);
+                #pragma unroll
+                for (uint32_t i = 0; i < 4; ++i)  // 16 k: 32 bytes of a row, or sixteen rows
+                    ptx::mma_ss_f16(acc, a + 2 * i, b + (k_major ? 128 : 2) * i, idesc, (st | i) != 0);
+                ptx::tc_commit(empty0 + 8 * s);
+                if (st + 1 == stages) ptx::tc_commit(acc_bar);
+            }
+            __syncwarp();
+        }
+        if (!ok && lane == 0) NF4_REPORT_FAILURE(*failure.flag, *failure.host, 9);
+    } else if (kCopy && warp < 8) {
+        // Every warp has stages of its own: a stage is read, converted and written in one go of many loads, and the next
+        // ones are other warps' (eight warps to a stage waited for each link of its chain in turn: 30 us without the stores).
+        const uint32_t piece = lane & 7u, r0 = warp % kPerStage * kWarpRows + (lane >> 3);
+        uint32_t mx[kQuads] = {};
+        const float shift = s_shift;
+        for (uint32_t st = warp / kPerStage; st < stages; st += kGroups) {
+            const uint32_t s = st % kStages;
+            if (!ptx::mbar_wait_suspended(full0 + 8 * s, (st / kStages) & 1u)) {
+                ok = false;
+                break;
+            }
+            const uint32_t k = k0 + st * 64 + piece * 8, rows = k < k1 ? p.M - min(m0 + r0, p.M) : 0u;  // (from r0 on)
+            __half *out = p.xh + (size_t)(m0 + r0) * p.K + k;
+            constexpr uint32_t kBatch = 8;
+            #pragma unroll
+            for (uint32_t q0 = 0; q0 < kQuads; q0 += kBatch) {
+                uint4 v[kBatch];
+                #pragma unroll
+                for (uint32_t q = 0; q < kBatch; ++q) {
+                    const uint32_t r = r0 + (q0 + q) * 4;
+                    v[q] = *reinterpret_cast<const uint4 *>(smem + s * kXStage + r * 128 + ((piece ^ (r & 7u)) << 4));
+                }
+                #pragma unroll
+                for (uint32_t q = 0; q < kBatch; ++q, out += (size_t)4 * p.K) {
+                    const uint32_t w[4] = {v[q].x, v[q].y, v[q].z, v[q].w};
+                    #pragma unroll
+                    for (int i = 0; i < 4; ++i) mx[q0 + q] = bf16x2_absmax(w[i], mx[q0 + q]);
+                    if ((q0 + q) * 4 < rows) *reinterpret_cast<uint4 *>(out) = bf16x8_to_f16x8(v[q], shift);
+                }
+            }
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(empty0 + 8 * s);
+        }
+        #pragma unroll
+        for (uint32_t q = 0; q < kQuads; ++q) {  // (eight lanes hold a row's)
+            uint32_t m = bf16x2_larger_bits(mx[q]);
+            #pragma unroll
+            for (int d = 1; d < 8; d *= 2) m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
+            if (piece == 0) atomicMax(s_own + r0 + q * 4, m);
+        }
+        if (!ok && lane == 0) NF4_REPORT_FAILURE(*failure.flag, *failure.host, 10);
+    }
+    if (!ok) ptx::let_flights_land();
+    __syncwarp();
+    __syncthreads();
+
+    // The exchange.  Only the last four warps, which have written nothing to global memory, release what they do here: a
+    // release by the others would wait for the copy's stores.
+    if (warp >= 8 && warp - 8 < kRows / 32) {
+        // this CTA's sums, a lane a row; columns the factor does not have are zeros
+        const uint32_t q = warp - 8;
+        if (stages && !ptx::mbar_wait_suspended(acc_bar, 0)) {
+            if (lane == 0) NF4_REPORT_FAILURE(*failure.flag, *failure.host, 11);
+        }
+        ptx::tc_fence_after();
+        #pragma unroll
+        for (uint32_t c = 0; c < 64; c += 16) {
+            uint32_t v[16];
+            ptx::tmem_ld16(acc + ((q * 32) << 16) + c, v);
+            ptx::tmem_wait_ld();
+            const bool real = c < n16 && stages;
+            float4 *dst = reinterpret_cast<float4 *>(part + (q * 32 + lane) * kPartPitch + c);
+            #pragma unroll
+            for (int i = 0; i < 4; ++i)
+                dst[i] = real ? make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]), __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]))
+                              : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+        ptx::tc_fence_before();
+    }
+    cluster.barrier_wait();
+    if (kCopy && warp >= 8)
+        for (uint32_t i = tid - 256; i < kRows * cn; i += 128) cluster.map_shared_rank(&s_max[0][0], i / kRows)[rank_in * kRows + i % kRows] = s_own[i % kRows];
+    if (warp >= 8) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    else asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const int w_exp = s_exp;
+    if (kCopy) {
+        if (tid < kRows) {
+            uint32_t m = 0;
+            for (uint32_t c = 0; c < cn; ++c) m = max(m, s_max[c][tid]);
+            // the copy stays where its largest value is in f16's comfortable range (see row_factor), or is infinite
+            const float mx = __uint_as_float(m), copied = mx * s_shift;
+            const bool own = (copied > 32768.0f || copied < 0.00390625f) && mx < __int_as_float(0x7f800000) && mx >= 1.1754944e-38f;
+            const float sc = own ? row_factor<true>(mx) : 1.0f / s_shift;
+            s_inv[tid] = 1.0f / sc;  // exact: sc is a power of two
+            if (rank_in == 0 && m0 + tid < p.M) p.row_scale[m0 + tid] = sc * ldexpf(1.0f, w_exp);  // both factors of the outputs
+        }
+        __syncthreads();
+        for (uint32_t r = warp; r < kRows; r += kTcThreads / 32) {  // the rare rows with a factor of their own, again
+            const float is = s_inv[r];
+            if (is == s_shift || m0 + r >= p.M) continue;
+            for (uint32_t k = k0 + lane * 8; k < k1; k += 256) {
+                const size_t at = (size_t)(m0 + r) * p.K + k;
+                *reinterpret_cast<uint4 *>(p.xh + at) = bf16x8_to_f16x8(__ldg(reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(p.x) + at)), is);
+            }
+        }
+    }
+    const float w_down = ldexpf(1.0f, -w_exp);
+    const uint32_t per = (kRows + cn - 1) / cn;  // rows of this CTA's share
+    for (uint32_t i = tid; i < per * 16; i += kTcThreads) {
+        const uint32_t r = rank_in * per + (i >> 4), c = (i & 15u) * 4, m = m0 + r;
+        if (r >= kRows || m >= p.M) continue;
+        float sum[4] = {};
+        #pragma unroll 4
+        for (uint32_t q = 0; q < cn; ++q) {
+            const float4 w = *reinterpret_cast<const float4 *>(cluster.map_shared_rank(part, q) + r * kPartPitch + c);
+            sum[0] += w.x;
+            sum[1] += w.y;
+            sum[2] += w.z;
+            sum[3] += w.w;
+        }
+        put_halves(kCopy ? p.t_out : nullptr, sum, p.scale * (kCopy ? s_inv[r] : 1.0f) * w_down, (size_t)m * 128 + c, 64);
+        put_halves(p.r_out, sum, 1.0f, (size_t)m * 128 + c, 64);
+    }
+    ptx::tc_fence_before();
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");  // the sums have been read
+    if (warp == 9) {
+        ptx::tc_fence_after();
+        ptx::tmem_dealloc(acc, 64);
+    }
+    if (p.wait == 2) ptx::pdl_wait();
+}
+
+}  // namespace
+
+namespace {
+
+template <uint32_t kRows>
+auto tc_kernel(bool copy, bool k_major) {
+    return copy ? (k_major ? prepass_tc_kernel<0, kRows, true> : prepass_tc_kernel<0, kRows, false>)
+                : (k_major ? prepass_tc_kernel<2, kRows, true> : prepass_tc_kernel<2, kRows, false>);
+}
+
+int32_t launch_tc(const PrepassArgs &q, Params &p, cudaStream_t stream) {
+    // Rows to a cluster: what leaves an SM the least to fetch, its stages of x and the factor (an SM holds one CTA).
+    uint32_t rows = 0, cn = 1;
+    uint64_t least = 0;
+    decltype(tc_kernel<128>(true, true)) kernel = nullptr;
+    for (uint32_t r : {128u, 64u, 32u}) {
+        const bool copy = q.xh != nullptr;
+        auto k = r == 128 ? tc_kernel<128>(copy, q.k_major) : r == 64 ? tc_kernel<64>(copy, q.k_major) : tc_kernel<32>(copy, q.k_major);
+        ClusterRoom room;
+        NF4_TRY(cluster_room(reinterpret_cast<const void *>(k), kTcThreads, tc_ring(r) + 1024, &room));
+        const uint64_t tiles = (q.M + r - 1) / r;
+        for (uint32_t c = 1; c <= kMaxCluster && (c == 1 || (tiles <= room.any[c] && q.K > 64ull * (c - 1))); ++c) {
+            const uint64_t stages = (q.K + 64ull * c - 1) / (64ull * c), waves = (tiles * c + kNumSMs - 1) / kNumSMs;
+            const uint64_t cost = waves * stages * (r * 128 + kTcFactorStage);
+            if (kernel && cost >= least) continue;
+            least = cost;
+            rows = r;
+            cn = c;
+            kernel = k;
+        }
+    }
+    const uint64_t tiles = (q.M + rows - 1) / rows;
+    if (tiles * cn >= (1ull << 31)) return fail(NF4_ERR_UNSUPPORTED, "activations_prepass: too many rows");
+    p.piece = ((q.K + cn - 1) / cn + 63) / 64 * 64;
+    CUtensorMap map_x, map_a;
+    NF4_TRY(make_map(&map_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, q.x, q.M, q.K, (uint64_t)q.K * 2, rows, 64, CU_TENSOR_MAP_SWIZZLE_128B));
+    if (q.k_major)
+        NF4_TRY(make_map(&map_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, q.a, q.K, q.rank, (uint64_t)q.rank * 2, 64, 64, CU_TENSOR_MAP_SWIZZLE_128B));
+    else
+        NF4_TRY(make_map(&map_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, q.a, q.rank, q.K, (uint64_t)q.K * 2, (q.rank + 15) / 16 * 16, 64,
+                         CU_TENSOR_MAP_SWIZZLE_128B));
+    FailureRef failure;
+    NF4_TRY(prefill_failure_ref(&failure));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(tiles * cn));
+    cfg.blockDim = dim3(kTcThreads);
+    cfg.dynamicSmemBytes = tc_ring(rows) + 1024;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cn;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    count_launch();
+    return check_cuda(cudaLaunchKernelEx(&cfg, kernel, map_x, map_a, p, failure), "prepass_tc_kernel launch");
 }
 
 }  // namespace
@@ -443,6 +752,12 @@ int32_t activations_prepass(const PrepassArgs &q, cudaStream_t stream) {
     p.a_vec = aligned16(q.a) && (q.k_major ? q.rank : q.K) % 8 == 0;
     p.scale = q.scale;
     p.wait = !q.beside_predecessor ? 0 : q.factor_of_predecessor ? 1 : 2;
+    // The tcgen05 kernel, where its TMA takes the tensors: always for the product alone ([16, 11008] and [14, 768] the same
+    // time); with the copy from four million values on (whole forwards to 512 columns: [1024, 4096] at rank 64 42.7 -> 40.3 us,
+    // [4096, 1024] 23.7 -> 23.1, but [512, 2048] 27.5 -> 30.3 and [256, 4096] at rank 16 the other way too: an SM
+    // holds one of its CTAs and two of the other's), and never without a factor ([2048, 4096]: 39.2 -> 41.1).
+    const bool tc_shape = !q.x_f32 && q.rank && q.rank <= 64 && q.K % 8 == 0 && aligned16(q.x) && p.a_vec;
+    if (tc_shape && (!q.xh || (uint64_t)q.M * q.K >= 1u << 22)) return launch_tc(q, p, stream);
     // 64 rows to a cluster beyond 512 rows, where the clusters of 32 no longer fit the chip at once, else 32 (half of the
     // factor's traffic against more CTAs)
     const uint32_t rows = q.M > 512 ? 64 : 32;
