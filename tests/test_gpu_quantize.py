@@ -267,7 +267,9 @@ def test_embedding_gather_equals_dequantize_then_gather(oracle, n_embedding, d_m
 
 
 @pytest.mark.parametrize("rows,cols,bf16", [(64, 64, False), (128, 200, True), (256, 1024, True),
-                                            (192, 36, False), (100, 72, True), (65, 7, False)])
+                                            (192, 36, False), (100, 72, True), (65, 7, False),
+                                            (64, 8, True), (128, 68, True),      # rows TMA takes, and rows it does not
+                                            (2560, 4608, True), (2560, 2304, False)])  # warps that take a second tile
 def test_load_path_quantize_of_the_transpose(oracle, rows, cols, bf16):
     # src/qwennet.rs:1709-1711: transpose2d([out, in]) then PackedNf4Tensor::quantize (+ double
     # quantization).  The fused kernel (rows % 64 == 0) and the workspace route must both give
@@ -293,6 +295,35 @@ def test_load_path_quantize_of_the_transpose(oracle, rows, cols, bf16):
     o_sc, o_sos = oracle.double_quantize(o_absmax)
     assert np.array_equal(lin.packed().scale_codes.cpu().numpy(), o_sc)
     assert bits_equal(lin.packed().scale_of_scales.cpu().numpy(), np.asarray([o_sos], np.float32))
+
+
+def test_load_path_codes_of_every_quotient_of_bf16(oracle):
+    # The bf16 path decides without a margin: every quotient of two eight-bit significands down to 2^-8 of the block's
+    # scale, both signs, and blocks whose scale the reciprocal is not used for.
+    from unifur_b200.quantize import PackedNf4Tensor
+
+    sig = np.arange(128, 256, dtype=np.float64)
+    cols = []
+    for m in sig:
+        for k in range(9):
+            x = np.concatenate([s * sig * 2.0 ** -k for s in (1, -1)])
+            x = x[np.abs(x) <= m]
+            for i in range(0, len(x), 63):
+                c = np.zeros(64)
+                c[0], c[1:1 + len(x[i:i + 63])] = m, x[i:i + 63]
+                cols.append(c)
+    for scale in (0.0, 1e-38, 1e-33, 1e33, np.inf, np.nan):
+        c = np.tile(np.linspace(-1.0, 1.0, 64), (2, 1)) * (scale if np.isfinite(scale) else 1.0)
+        if not np.isfinite(scale):
+            c[:, 5] = scale
+            c[1, 9] = -np.inf
+        cols += list(c)
+    cols += [np.zeros(64)] * (-len(cols) % 8)
+    w = oracle.round_bf16(np.ascontiguousarray(np.stack(cols, axis=1)).astype(np.float32))
+    o_packed, o_absmax = oracle.quantize_packed(np.ascontiguousarray(w.T).reshape(-1))
+    p = PackedNf4Tensor.quantize_transposed(torch.from_numpy(w).to(DEV).bfloat16())
+    assert bits_equal(p.absmax.cpu().numpy(), o_absmax)
+    assert np.array_equal(p.codes.cpu().numpy(), o_packed)
 
 
 def test_a_weight_from_an_odd_address_is_in_place_for_the_forward_behind_it():

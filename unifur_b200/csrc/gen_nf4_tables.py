@@ -60,6 +60,22 @@ def threshold(i: int) -> np.float32:
 CELL_MARGIN = 2  # units of 2^-21 on either side of a threshold where the exact path decides (errors add up to < 1.4)
 
 
+def bf16_cut(t: np.float32) -> int:
+    """The integer (units of 2^-21) that splits the quotients of two bf16 numbers as the threshold t does.
+
+    There are few such quotients (two eight-bit significands and a power of two), so around every threshold they leave a gap, and
+    the kernel's approximation (within half a unit of rounding and a quarter for the reciprocal) stays on their side of
+    its middle: no value has to be looked at again."""
+    m = np.arange(128, 256, dtype=np.float64)
+    q = np.unique(np.concatenate([s * (m[:, None] / m[None, :]).ravel() * 2.0 ** -k for k in range(12) for s in (1, -1)] + [np.zeros(1)]))
+    q = q[np.abs(q) <= 1.0]
+    up = q.astype(np.float32) >= t  # the reference compares the quotient as f32
+    below, above = float(q[~up].max()), float(q[up].min())
+    last, first = np.floor(below * 2 ** 21 + 0.25 * abs(below) + 0.5), np.ceil(above * 2 ** 21 - 0.25 * abs(above) - 0.5)
+    assert first - last >= 2
+    return int((last + first + 1) // 2)
+
+
 def main():
     th = [threshold(i) for i in range(15)]
     lines = [
@@ -80,7 +96,7 @@ def main():
     # which are 0x4b400000 + round(v * 2^21); the cell's word W is such that the top four bits of bits - W
     # are the code and the low 28 bits are below 2 * MARGIN exactly when v is within MARGIN units of 2^-21 of
     # the threshold.  Padded to 64 words; the last one (a NaN's bits index it) is always "within".
-    cells = []
+    cells, cells_bf16 = [], []
     for c in range(33):
         lo, hi = (4 * c - 0.5) / 64.0 - 1.0, (4 * c + 3.5) / 64.0 - 1.0
         inside = [t for t in th if lo <= float(t) < hi]
@@ -91,11 +107,17 @@ def main():
             assert min(abs(float(t) - lo), abs(float(t) - hi)) > 1e-4
         units = int(round(float(inside[0]) * 2 ** 21)) if inside else 1 << 26  # out of reach: never within, never above
         cells.append((0x4B400000 + units - CELL_MARGIN - ((base + 1) << 28)) & 0xFFFFFFFF)
+        cut = bf16_cut(inside[0]) if inside else 1 << 26
+        cells_bf16.append((0x4B400000 + cut - ((base + 1) << 28)) & 0xFFFFFFFF)
     cells += [0x7FFFFFFF] * (64 - len(cells))
+    cells_bf16 += [0x7FFFFFFF] * (64 - len(cells_bf16))
     lines.append("// 33 cells of width 1/16 over [-1, 1], padded to 64 (see nf4_common.cuh: FastCodes)")
     lines.append("#define NF4_CELL_MARGIN %d" % CELL_MARGIN)
     lines.append("#define NF4_CELL_TABLE_LIST \\")
     lines.append("  " + ", ".join("0x%08xu" % c for c in cells))
+    lines.append("// the same for quotients of bf16 numbers, with cuts that need no margin (see nf4_common.cuh: codes_of_bf16)")
+    lines.append("#define NF4_CELL_BF16_TABLE_LIST \\")
+    lines.append("  " + ", ".join("0x%08xu" % c for c in cells_bf16))
     lines.append("// thresholds as decimals: " + ", ".join(repr(float(t)) for t in th))
     out = os.path.join(os.path.dirname(os.path.abspath(__file__)), "nf4_tables.inc")
     with open(out, "w") as f:

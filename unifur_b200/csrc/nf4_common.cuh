@@ -150,6 +150,21 @@ __device__ __forceinline__ uint32_t codes_of_group(const float (&x)[8], float ab
     return w;
 }
 
+// The same for eight bf16 values of a block whose scale is in [1e-30, 1e30], none of them a NaN: the quotients of two bf16
+// numbers leave gaps around the thresholds that are wider than the approximation's error, the cuts of `cells`
+// (c_cell_bf16_table) lie in their middle, and nothing is left to decide otherwise.
+static __device__ __constant__ const uint32_t c_cell_bf16_table[kCellWords] = {NF4_CELL_BF16_TABLE_LIST};
+__device__ __forceinline__ uint32_t codes_of_bf16(const float (&x)[8], float rcp_units, float rcp_cells, const uint32_t *cells) {
+    uint32_t codes = 0;
+    #pragma unroll
+    for (int i = 7; i >= 0; --i) {
+        const uint32_t u = __float_as_uint(fmaf(x[i], rcp_units, 12582912.0f));
+        const uint32_t at = __float_as_uint(fmaf(x[i], rcp_cells, 12582912.0f + 64.0f)) & 0xfcu;
+        codes = __funnelshift_l(u - *reinterpret_cast<const uint32_t *>(reinterpret_cast<const char *>(cells) + at), codes, 4);
+    }
+    return codes;
+}
+
 // Scale of a double-quantized block: divide first, then multiply (src/quantize.rs:348).
 __device__ __forceinline__ float dq_scale(uint32_t code, float scale_of_scales) {
     return __fmul_rn(__fdiv_rn((float)code, 255.0f), scale_of_scales);

@@ -10,6 +10,7 @@
 
 #include "kernels.cuh"
 #include "ptx.cuh"
+#include "tmap.cuh"
 
 namespace nf4 {
 
@@ -301,6 +302,129 @@ quantize_transposed_kernel(const uint32_t *__restrict__ src, uint32_t segments, 
     publish_weight();
 }
 static_assert(kSplitRows == 32, "a lane stores four words of codes per block");
+
+// The same where TMA takes the matrix (rows of whole 16-byte pieces): a warp takes a 64-block's rows of 32 words (64 columns of
+// bf16, 32 of f32), a lane the 64 rows of a word.  The 8 KB come by TMA into the warp's own place in shared memory, pass into
+// registers, and the next ones are asked for before these are encoded: the loads of sixteen warps, 128 KB an SM, are in flight
+// while the codes of 128 values a lane are computed, where the kernel above loads, waits and computes in turn.  bf16 needs no
+// look at the threshold's neighbourhood (see codes_of_bf16): 9 instructions a value.
+constexpr int kTmaWarps = 8, kTmaThreads = kTmaWarps * 32, kTmaTile = kBlock * 128;  // two CTAs on an SM
+constexpr uint32_t kTmaSmem = kTmaWarps * kTmaTile + 1024;
+
+template <bool SRC_BF16>
+__global__ void __launch_bounds__(kTmaThreads, 2)
+quantize_transposed_tma_kernel(const __grid_constant__ CUtensorMap tmap, uint32_t segments, uint32_t octets, uint32_t words_per_row, uint32_t tiles,
+                               uint8_t *__restrict__ codes, float *__restrict__ absmax, bool wide, bool wide_scales, const FailureRef failure) {
+    extern __shared__ uint8_t smem_any[];
+    __shared__ uint32_t s_cells[kCellWords];
+    __shared__ __align__(8) uint64_t s_bars[kTmaWarps];
+    constexpr int kCols = SRC_BF16 ? 2 : 1;  // of a word
+    __shared__ float s_max[2][kTmaWarps][32 * kCols];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    uint8_t *const place = smem_any + (1024u - (ptx::smem_addr(smem_any) & 1023u)) % 1024u + warp * kTmaTile;
+    const uint32_t bar = ptx::smem_addr(s_bars + warp), stride = gridDim.x;
+    if (threadIdx.x < kCellWords) s_cells[threadIdx.x] = SRC_BF16 ? c_cell_bf16_table[threadIdx.x] : c_cell_table[threadIdx.x];
+    if (lane == 0) {
+        ptx::mbar_init(bar, 1);
+        ptx::fence_mbar_init();
+        ptx::fence_proxy_async();
+        if (warp == 0) ptx::prefetch_tmap(&tmap);
+    }
+    __syncthreads();
+    ptx::pdl_wait();
+    // A tile of the CTA: 32 words of eight segments, one a warp, so that a column's block scales are a sector and its codes two
+    // lines.  The segments run fastest over the grid.
+    auto request = [&](uint32_t tile) {
+        const uint32_t group = tile / octets, seg = (tile - group * octets) * kTmaWarps + warp;
+        if (seg >= segments) return;
+        ptx::mbar_arrive_expect_tx(bar, kTmaTile);
+        ptx::tma_load_2d(ptx::smem_addr(place), &tmap, (int32_t)(group * 32), (int32_t)(seg * kBlock), bar);
+    };
+    uint32_t parity = 0, turn = 0;
+    bool lost = false;
+    if (lane == 0 && blockIdx.x < tiles) request(blockIdx.x);
+    for (uint32_t tile = blockIdx.x; tile < tiles; tile += stride, turn ^= 1u) {
+        const uint32_t group = tile / octets, seg0 = (tile - group * octets) * kTmaWarps, seg = seg0 + warp, word = group * 32 + lane;
+        const bool mine = seg < segments && !lost;  // (the last tile of a group may have fewer segments)
+        if (mine && !ptx::mbar_wait_suspended(bar, parity)) {
+            lost = true;  // its codes are void, and no more tiles are asked for
+            if (lane == 0) NF4_REPORT_FAILURE(*failure.flag, *failure.host, 15);
+            ptx::let_flights_land();
+        }
+        if (mine) parity ^= 1u;
+        uint32_t w[kBlock];
+        #pragma unroll
+        for (int r = 0; r < kBlock; ++r) w[r] = *reinterpret_cast<const uint32_t *>(place + r * 128 + lane * 4);
+        uint32_t mx = 0;  // both columns' maxima of |bf16| as a pair (a NaN stays one), or the f32 column's (NaNs drop out)
+        #pragma unroll
+        for (int r = 0; r < kBlock; ++r) {
+            if (SRC_BF16) asm("max.NaN.xorsign.abs.bf16x2 %0, %0, %1;" : "+r"(mx) : "r"(w[r]));
+            else mx = __float_as_uint(fmaxf(__uint_as_float(mx), fabsf(__uint_as_float(w[r]))));
+        }
+        __syncwarp();  // every value has been used: the place may be filled again
+        if (lane == 0 && tile + stride < tiles && !lost) request(tile + stride);
+        #pragma unroll 1  // (unrolled, both columns' values would be kept in registers at once)
+        for (int h = mine && word < words_per_row ? 0 : kCols; h < kCols; ++h) {
+            const uint32_t half = h == 0 ? 0x1044u : 0x3244u;
+            auto value = [&](uint32_t bits) { return __uint_as_float(SRC_BF16 ? __byte_perm(bits, 0u, half) : bits); };
+            float m = fabsf(value(mx));
+            const uint64_t blk = (uint64_t)(word * kCols + h) * segments + seg;  // the block's number in the result
+            uint32_t out[kBlock / 8];
+            if (SRC_BF16 && m >= 1e-30f && m <= 1e30f) {
+                const float rcp = approx_rcp(m), rcp_units = rcp * 2097152.0f, rcp_cells = rcp * 64.0f;
+                #pragma unroll
+                for (int g = 0; g < kBlock / 8; ++g) {
+                    float v[8];
+                    #pragma unroll
+                    for (int i = 0; i < 8; ++i) v[i] = value(w[8 * g + i]);
+                    out[g] = codes_of_bf16(v, rcp_units, rcp_cells, s_cells);
+                }
+            } else if (SRC_BF16) {  // NaNs among them, or a scale the reciprocal is not used for
+                m = 0.0f;
+                #pragma unroll
+                for (int r = 0; r < kBlock; ++r) m = fmaxf(m, fabsf(value(w[r])));
+                #pragma unroll
+                for (int g = 0; g < kBlock / 8; ++g) {
+                    out[g] = 0;
+                    #pragma unroll
+                    for (int i = 0; i < 8; ++i) out[g] |= code_of_exact(value(w[8 * g + i]), m) << (4 * i);
+                }
+            } else {
+                #pragma unroll
+                for (int g = 0; g < kBlock / 8; ++g) {
+                    float v[8];
+                    #pragma unroll
+                    for (int i = 0; i < 8; ++i) v[i] = value(w[8 * g + i]);
+                    out[g] = codes_of_group(v, m, s_cells);
+                }
+            }
+            uint32_t *dst = reinterpret_cast<uint32_t *>(codes + blk * (kBlock / 2));
+            if (wide) {
+                asm volatile("st.global.v8.b32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};" ::"r"(out[0]), "r"(out[1]), "r"(out[2]), "r"(out[3]),
+                             "r"(out[4]), "r"(out[5]), "r"(out[6]), "r"(out[7]), "l"(dst) : "memory");
+            } else {  // codes only 4-byte aligned
+                #pragma unroll
+                for (int g = 0; g < kBlock / 8; ++g) dst[g] = out[g];
+            }
+            s_max[turn][warp][lane * kCols + h] = m;
+        }
+        // The block scales of the tile: eight segments of a column by a thread, in one sector where they are whole.  (The next
+        // tile's go to the other half, and nobody writes this one before all have passed the barrier of that tile.)
+        __syncthreads();
+        const uint32_t c = threadIdx.x, col = group * 32 * kCols + c;
+        if (c < 32 * kCols && col < words_per_row * kCols) {
+            float *dst = absmax + (uint64_t)col * segments + seg0;
+            if (wide_scales) {
+                asm volatile("st.global.v8.f32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};" ::"f"(s_max[turn][0][c]), "f"(s_max[turn][1][c]),
+                             "f"(s_max[turn][2][c]), "f"(s_max[turn][3][c]), "f"(s_max[turn][4][c]), "f"(s_max[turn][5][c]),
+                             "f"(s_max[turn][6][c]), "f"(s_max[turn][7][c]), "l"(dst) : "memory");
+            } else {
+                for (uint32_t i = 0; i < min((uint32_t)kTmaWarps, segments - seg0); ++i) dst[i] = s_max[turn][i][c];
+            }
+        }
+    }
+    publish_weight();
+}
 
 // Any shape: the transpose written out as f32 (then quantized by the flat kernels).
 template <bool SRC_BF16>
@@ -629,6 +753,18 @@ int32_t quantize_transposed(const void *src, bool src_bf16, uint64_t rows, uint6
             return fail(NF4_ERR_UNSUPPORTED, "nf4_quantize_transposed: matrix too large");
         const uint32_t *w = static_cast<const uint32_t *>(src);
         count_launch();
+        if (words % 4 == 0) {  // (always for f32)
+            auto kernel = src_bf16 ? quantize_transposed_tma_kernel<true> : quantize_transposed_tma_kernel<false>;
+            const uint64_t segments = rows / kBlock, octets = (segments + kTmaWarps - 1) / kTmaWarps, tiles = octets * ((words + 31) / 32);
+            CUtensorMap map;
+            NF4_TRY(make_map(&map, CU_TENSOR_MAP_DATA_TYPE_UINT32, src, rows, words, words * 4, kBlock, 32, CU_TENSOR_MAP_SWIZZLE_NONE));
+            FailureRef failure;
+            NF4_TRY(prefill_failure_ref(&failure));
+            NF4_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), (int)kTmaSmem));
+            return launch_maybe_overlapped(kernel, dim3((unsigned)(tiles < 2 * kNumSMs ? tiles : 2 * kNumSMs)), dim3(kTmaThreads), kTmaSmem, stream, true,
+                                           map, (uint32_t)segments, (uint32_t)octets, (uint32_t)words, (uint32_t)tiles, packed, absmax, aligned32(packed),
+                                           aligned32(absmax) && segments % kTmaWarps == 0, failure);
+        }
         return launch_maybe_overlapped(src_bf16 ? quantize_transposed_kernel<true> : quantize_transposed_kernel<false>,
                                        dim3((unsigned)ctas), dim3(kTThreads), 0, stream, true, w, (uint32_t)(rows / kBlock), (uint32_t)words, packed, absmax,
                                        aligned16(packed));
