@@ -40,7 +40,7 @@ def test_any_length_and_alignment(oracle, n, shift, packed):
     assert (rest == 123.0).all()
 
 
-@pytest.mark.parametrize("nb", [1, 3, 4, 63, 4096 + 1, 131072 * 4 + 7, (1 << 20) + 5])  # one cluster, and beyond its range
+@pytest.mark.parametrize("nb", [1, 3, 4, 63, 4096 + 1, 131072, 131073, 131072 * 4 + 7, (1 << 20) + 5])  # one launch, one cluster, and beyond
 def test_double_quantization_of_any_length(oracle, nb):
     from gpu_util import double_quantize_dev
 
@@ -50,6 +50,9 @@ def test_double_quantization_of_any_length(oracle, nb):
     sc, sos = double_quantize_dev(s)
     o_sc, o_sos = oracle.double_quantize(s)
     assert sc.tobytes() == o_sc.tobytes() and np.float32(sos).tobytes() == np.float32(o_sos).tobytes()
+    d, out, m = torch.from_numpy(s).to(DEV), torch.full((nb + 2,), 77, dtype=torch.uint8, device=DEV), torch.zeros(1, device=DEV)
+    _lib.check(_lib.load().nf4_double_quantize_dev(d.data_ptr(), nb, out.data_ptr() + 1, m.data_ptr(), None))  # codes at an odd address
+    assert out[1:-1].cpu().numpy().tobytes() == o_sc.tobytes() and out[0] == 77 and out[-1] == 77
 
 
 @pytest.mark.parametrize("rows", [1, 16, 17, 100, 361])
