@@ -41,6 +41,38 @@ def test_reference_orientation_in_f32(M, K, N, r):
     assert float((y.double() - ref).norm() / ref.norm()) < 1e-3
 
 
+@pytest.mark.parametrize("M,K,N,ld,f32,in_out", [
+    (17, 1792, 64, 64, False, False),    # 28 stages in three or four parts
+    (19, 4160, 43, 48, False, False),    # the last columns are no whole pieces
+    (300, 3008, 392, 400, False, True),  # parts of unequal length, two tiles of rows, the last odd CTA without weight rows
+    (65, 20288, 130, 136, True, False),  # two tiles of columns in the most parts
+    (257, 2560, 448, 448, True, True),   # one row in the second tile
+])
+def test_tiles_of_several_pairs(M, K, N, ld, f32, in_out):
+    # f16 weights and f32 sums: 1e-3 for f32 results, bf16's own rounding for the others
+    from unifur_b200 import _lib
+    from unifur_b200.quantize import PackedNf4Tensor, linear_forward
+
+    g = torch.Generator(device="cuda").manual_seed(M + K + N)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    dt, r = torch.float32 if f32 else torch.bfloat16, 8
+    p = PackedNf4Tensor.quantize(rnd(K * N) * 0.02)
+    a, b = rnd(K, r) * 0.05, rnd(r, N) * 0.05
+    x, bias, a, b = rnd(M, K).to(dt), rnd(N), a.to(dt), b.to(dt)
+    la, lb = (a, b) if in_out else (a.t().contiguous(), b.t().contiguous())
+    w = p.dequantize().double()
+    w = w.view(K, N) if in_out else w.view(N, K).t()
+    ref = x.double() @ w + bias.double() + 1.5 * (x.double() @ a.double()) @ b.double()
+    buf = torch.full((M + 1, ld), 7.0, dtype=dt, device="cuda")
+    layout = _lib.LAYOUT_IN_OUT if in_out else _lib.LAYOUT_OUT_IN
+    for _ in range(2):
+        y = linear_forward(x, p, K, N, layout, bias=bias, lora_a=la, lora_b=lb, lora_scale=1.5, out=buf[:M, :N])
+        assert float((y.double() - ref).norm() / ref.norm()) < (1e-3 if f32 else 4e-3)
+    first = y.clone()
+    assert torch.equal(first, linear_forward(x, p, K, N, layout, bias=bias, lora_a=la, lora_b=lb, lora_scale=1.5, out=buf[:M, :N]))
+    assert bool((buf[:, N:] == 7.0).all()) and bool((buf[M] == 7.0).all())
+
+
 def test_repeated_calls_agree():
     # several tiles to a pair, so that the epilogue's traffic runs beside the dequantisers': a slot of the rings given
     # back too early shows as a few weight rows that differ from call to call

@@ -13,6 +13,8 @@ SHAPES = [
     (4096, 3584, 3584), (4096, 3584, 512), (4096, 3584, 18944), (4096, 18944, 3584),   # the block's projections
     (4096, 18944, 1792), (4096, 18944, 896), (4096, 18944, 448), (4096, 3584, 64),     # and their shards
     (2048, 4096, 7168), (2048, 4096, 1792),
+    (99, 20288, 512), (512, 4096, 4096), (2514, 15104, 320),   # fewer tiles than pairs: several pairs to a tile
+    (600, 16384, 10240),                                       # ... divided by stages
     (512, 4096, 256), (300, 3072, 200), (768, 1536, 6400), (17, 64, 8), (40, 64, 40000), (257, 192, 136),
 ]
 

@@ -129,7 +129,9 @@ struct PrefillParams {
     // whole tiles.  A pair that multiplies the leading stages of a tile leaves its accumulators
     // in `partial` ([CTA][BN][BM] f32) and raises its CTAs' words of `sk_flags`; the pair that multiplies
     // the last stages adds those and finishes the tile.
-    uint32_t sk_tiles, dp_rounds;
+    // split > 1 (fewer tiles than pairs): a tile is `split` pairs' instead, an equal part of its stages each; all leave
+    // their accumulators in `partial`, and a kernel of its own adds them (sum_parts_kernel).
+    uint32_t sk_tiles, dp_rounds, split;
     float *partial;
     uint32_t *sk_flags;
     uint32_t wait_ns;  // bound of the wait for a neighbour's flag
@@ -156,6 +158,10 @@ struct WorkList {
         const uint64_t all = (uint64_t)p.sk_tiles * ks;
         u0 = all * cta / ctas;
         u1 = all * (cta + 1) / ctas;
+        if (p.split > 1) {  // (sk_tiles * split == ctas: a part lies in one tile)
+            u0 = (uint64_t)(cta / p.split) * ks + (uint64_t)ks * (cta % p.split) / p.split;
+            u1 = (uint64_t)(cta / p.split) * ks + (uint64_t)ks * (cta % p.split + 1) / p.split;
+        }
         n_shared = 0;
         t_first = t_last = 0;
         if (u1 > u0) {
@@ -254,6 +260,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     WorkList wl;
     wl.init(p, k_stages, pair, pairs);
 
+    if (p.split > 1) ptx::pdl_launch_dependents();  // the kernel that adds the parts: it waits for this one to complete
     if (win - own > kLoraAt) {  // (both CTAs alike) the places below are not ours
         if (threadIdx.x == 0) NF4_REPORT_FAILURE(g_prefill_error, g_prefill_error_host, 6);
         return;
@@ -426,8 +433,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             wl.get(seg, tile, kb, ke);
             const uint32_t n0 = ((tile / p.m_tiles) * 2 + rank) * BM, m0 = (tile % p.m_tiles) * BN;
             const uint32_t n = n0 + row_in_tile;
-            if (ke != k_stages) {
-                // The leading stages of a tile that a neighbour finishes: the raw sums go to this
+            if (ke != k_stages || p.split > 1) {
+                // The leading stages of a tile that a neighbour finishes, or a part of one: the raw sums go to this
                 // CTA's place in global memory ([activation row][weight row]: a warp's stores are
                 // whole lines; a thread's values 64 bytes in a row were measured 15 % slower over
                 // the whole GEMM), then the flag goes up.
@@ -447,7 +454,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 __syncwarp();
                 if (lane == 0) ptx::mbar_arrive_cluster(acc_empty);
                 asm volatile("bar.sync 1, 256;" ::: "memory");
-                if (epi_leader) {
+                if (epi_leader && p.split <= 1) {
                     __threadfence();
                     atomicExch(p.sk_flags + blockIdx.x, 1u);
                 }
@@ -732,6 +739,61 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     }
 }
 
+// ---- the sums of a tile whose stages several pairs shared --------------------------------------------------
+// y[m][n] = (sum over the parts, in order, of partial[part][m][n]) * row factor + bias.  A warp takes one activation row of a
+// CTA's 128 weight rows, a lane four of them.  One pair that collected the others' sums in its read-out, a helper and
+// sixteen columns at a time, took 10 us (300 x 3584 x 3584), 14 (512 x 4096 x 4096, f32) and 23 (99 x 20288 x 512, twelve
+// helpers); a launch of its own has all SMs' loads in flight, and no CTA waits for another one.
+template <bool YF32>
+__global__ void __launch_bounds__(256)
+sum_parts_kernel(const float *__restrict__ partial, uint32_t split, uint32_t m_tiles, uint32_t M, uint32_t N, const float *__restrict__ row_scale,
+                 const float *__restrict__ bias, void *__restrict__ y, uint64_t ldy) {
+    ptx::pdl_wait();
+    const uint32_t lane = threadIdx.x & 31u, col = blockIdx.x * 8 + (threadIdx.x >> 5);  // of the tile's activation rows
+    const uint32_t tile = blockIdx.y >> 1, rank = blockIdx.y & 1u;
+    const uint32_t m = tile % m_tiles * BN + col, n = (tile / m_tiles * 2 + rank) * BM + lane * 4;
+    if (m >= M || n >= N) return;
+    const float4 *src = reinterpret_cast<const float4 *>(partial + ((size_t)(tile * split * 2 + rank) * BN + col) * BM) + lane;
+    constexpr size_t kPart = 2 * (size_t)BN * BM / 4;  // a pair's parts, in float4
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    constexpr uint32_t kInFlight = 8;
+    for (uint32_t s = 0; s < split; s += kInFlight) {
+        float4 p[kInFlight];
+        #pragma unroll
+        for (uint32_t i = 0; i < kInFlight; ++i)
+            p[i] = s + i < split ? __ldcg(src + (s + i) * kPart) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        #pragma unroll
+        for (uint32_t i = 0; i < kInFlight; ++i) {
+            if (s + i >= split) break;
+            v.x += p[i].x;
+            v.y += p[i].y;
+            v.z += p[i].z;
+            v.w += p[i].w;
+        }
+    }
+    const float rs = __ldg(row_scale + m);
+    float o[4] = {v.x, v.y, v.z, v.w};
+    #pragma unroll
+    for (int i = 0; i < 4; ++i) o[i] = fmaf(o[i], rs, bias && n + i < N ? __ldg(bias + n + i) : 0.0f);
+    const size_t at = (size_t)m * ldy + n;
+    if (n + 3 < N) {  // (rows and n are whole 16-byte pieces of f32, 8-byte ones of bf16)
+        if (YF32) {
+            *reinterpret_cast<float4 *>(static_cast<float *>(y) + at) = make_float4(o[0], o[1], o[2], o[3]);
+        } else {
+            const __nv_bfloat162 a = __floats2bfloat162_rn(o[0], o[1]), b = __floats2bfloat162_rn(o[2], o[3]);
+            *reinterpret_cast<uint2 *>(static_cast<__nv_bfloat16 *>(y) + at) =
+                make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
+        }
+        return;
+    }
+    #pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (n + i >= N) break;
+        if (YF32) static_cast<float *>(y)[at + i] = o[i];
+        else static_cast<__nv_bfloat16 *>(y)[at + i] = __float2bfloat16_rn(o[i]);
+    }
+}
+
 // ---- weights in the other orientation: repacking before the GEMM ---------------------------
 // W [d_in][d_out] with the 64-blocks along d_out (the reference's Burn layout) is brought into the
 // form the GEMM's dequantisers read: codes_t[n][k / 2] (the same nibbles, transposed, so exact) and
@@ -923,19 +985,44 @@ namespace {
 // (every pair the same number of stages, a tile possibly split between neighbours), the other
 // pairs * dp_rounds tiles go out whole.  With a tile count that is a multiple of the pairs nothing
 // is split.  Otherwise the last round of whole tiles would leave most pairs idle, so the last full round and
-// the remainder are divided by stages instead.  Fewer tiles than pairs: divided as long as a pair keeps 24
-// stages.
+// the remainder are divided by stages instead.  Fewer tiles than pairs: what of three takes the shortest by the times
+// measured (a stage 0.28 us however many columns it has): whole tiles, read out in 3 us; `split` pairs to a tile, whose
+// sums a kernel of its own adds (dump 3.5, launch and sum 4.5 us); or divided by stages, every pair 24 at least, with a tile's last
+// pair collecting (3 us of dump, and 2 a helper).
 struct Sharing {
-    uint32_t pairs, sk_tiles, dp_rounds;
+    uint32_t pairs, sk_tiles, dp_rounds, split;
 };
 Sharing share_tiles(uint64_t rows, uint64_t d_in, uint64_t d_out) {
     const uint64_t tiles = ((rows + BN - 1) / BN) * ((d_out + 2 * BM - 1) / (2 * BM)), ks = d_in / BK;
     Sharing sh;
+    sh.split = 1;
     uint64_t pairs = kNumSMs / 2;
     if (tiles < pairs) {
-        const uint64_t by_stages = tiles * ks / 24;
-        pairs = by_stages < pairs ? by_stages : pairs;
-        if (pairs < tiles) pairs = tiles;
+        constexpr uint64_t kStage = 280, kReadOut = 3000, kDump = 3500, kSum = 4500, kHelper = 2000;  // ns
+        const uint64_t by_stages = tiles * ks / 24, shared = by_stages < pairs ? by_stages : pairs;
+        uint64_t least = ks * kStage + kReadOut, most = pairs / tiles;
+        if (shared > tiles) {
+            const uint64_t cost = tiles * ks * kStage / shared + 2 * kReadOut + (shared + tiles - 1) / tiles * kHelper;
+            if (cost < least) {
+                least = cost;
+                sh.split = 0;
+            }
+        }
+        for (uint64_t s = 2; s <= most && s * 4 <= ks; ++s) {
+            const uint64_t cost = (ks + s - 1) / s * kStage + kDump + kSum;
+            if (cost < least) {
+                least = cost;
+                sh.split = (uint32_t)s;
+            }
+        }
+        pairs = sh.split ? tiles * sh.split : shared;
+        if (sh.split > 1) {
+            sh.pairs = (uint32_t)pairs;
+            sh.sk_tiles = (uint32_t)tiles;
+            sh.dp_rounds = 0;
+            return sh;
+        }
+        sh.split = 1;
     }
     sh.pairs = (uint32_t)pairs;
     if (tiles % pairs == 0) {
@@ -1038,6 +1125,7 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_o
     const Sharing sh = share_tiles(p.M, p.K, p.N);
     p.sk_tiles = sh.sk_tiles;
     p.dp_rounds = sh.dp_rounds;
+    p.split = sh.split;
     p.wait_ns = 1000000000u;
     uint8_t *ws = static_cast<uint8_t *>(a.workspace);
     __half *xh = reinterpret_cast<__half *>(ws + wl.off_xh);
@@ -1136,7 +1224,12 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_o
     if (repacked) NF4_TRY(y_f32 ? go(prefill_kernel<true, true>) : go(prefill_kernel<false, true>));
     else NF4_TRY(y_f32 ? go(prefill_kernel<true, false>) : go(prefill_kernel<false, false>));
     count_launch();
-    return check_cuda(cudaGetLastError(), "prefill_kernel launch");
+    NF4_TRY(check_cuda(cudaGetLastError(), "prefill_kernel launch"));
+    if (sh.split <= 1) return NF4_OK;
+    const uint32_t columns = p.M < (uint32_t)BN ? p.M : (uint32_t)BN;
+    count_launch();
+    return launch_maybe_overlapped(y_f32 ? sum_parts_kernel<true> : sum_parts_kernel<false>, dim3((columns + 7) / 8, sh.pairs / sh.split * 2), dim3(256), 0,
+                                   stream, true, p.partial, p.split, p.m_tiles, p.M, p.N, p.row_scale, p.bias, a.y, ldy);
 }
 
 
@@ -1158,6 +1251,7 @@ int32_t prefill_share_plan(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_
     PrefillParams p{};
     p.sk_tiles = sh.sk_tiles;
     p.dp_rounds = sh.dp_rounds;
+    p.split = sh.split;
     WorkList wl;
     wl.init(p, (uint32_t)(d_in / BK), cta % sh.pairs, sh.pairs);
     uint32_t n = 0;
