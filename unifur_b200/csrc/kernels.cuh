@@ -166,8 +166,8 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_o
 // x [M][K] bf16 or f32 (K a multiple of 8, 16-byte aligned); a: the factor as [rank][K], or [K][rank]
 // (k_major), bf16, f16 for f32 x.  xh null: r_out alone (bf16 x).  t_out and r_out: [M][2 * 64 * ceil(rank / 64)]
 // bf16, hi halves then lo; t_out the scaled intermediate the GEMM adds, r_out (may be null) x a as it is.
-// beside_predecessor: the kernel ahead in the stream touches nothing that this one reads or writes; they may
-// run side by side, and this one completes after it.  factor_of_predecessor: it writes the factor, nothing else of this.
+// factor_of_predecessor: the kernel ahead in the stream writes the factor and touches nothing else of this one's; they
+// run side by side up to there.
 struct PrepassArgs {
     const void *x;
     bool x_f32;
@@ -184,7 +184,7 @@ struct PrepassArgs {
     const float *scale_of_scales;
     uint32_t *flags;
     uint32_t n_flags;
-    bool beside_predecessor, factor_of_predecessor;
+    bool factor_of_predecessor;
 };
 int32_t activations_prepass(const PrepassArgs &q, cudaStream_t stream);
 

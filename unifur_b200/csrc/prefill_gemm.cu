@@ -814,6 +814,7 @@ struct RepackParams {
     uint32_t code_cols, code_blocks;              // CTAs of the nibbles: tiles of 128 n x 256 k
     uint32_t scale_cols, scale_blocks;            // CTAs of the scales: 32 x 32 tiles
     uint32_t a_blocks, adapter_blocks;            // CTAs of the factors: 32 x 32 tiles, A's first
+    uint32_t wait_last;         // for the kernel ahead: at the end (else at the start)
 };
 
 // Nibbles.  A CTA turns 256 k x 128 n.  A thread takes eight words (8 k x 8 n) straight from global memory, all
@@ -939,18 +940,20 @@ __device__ __forceinline__ void repack_adapter_block(const RepackParams &p, uint
     }
 }
 
-// One launch for everything the activations do not need: the first code_blocks CTAs take the nibbles,
-// the next scale_blocks the scales, the last adapter_blocks the adapter.  The pre-pass may run beside it.
+// The first code_blocks CTAs take the nibbles, the next scale_blocks the scales, the last adapter_blocks the adapter.  The
+// weight's launch runs beside the pre-pass ahead of it, which it shares nothing with (wait_last): one CTA waits for that at
+// the end, so that whoever waits for this kernel finds both complete.  (Weight first, pre-pass beside it: the pre-pass's CTAs
+// found no room until the many small ones were through.)
 template <class T>
 __global__ void __launch_bounds__(256) repack_kernel(const RepackParams p) {
     __shared__ __align__(16) uint32_t smem[128 * 32];
+    if (!p.wait_last) ptx::pdl_wait();
     ptx::pdl_launch_dependents();
-    uint32_t b = blockIdx.x;
-    if (b < p.code_blocks) return repack_codes_block(p, b, smem);
-    b -= p.code_blocks;
-    if (b < p.scale_blocks) return repack_scales_block(p, b, reinterpret_cast<float(*)[33]>(smem));
-    b -= p.scale_blocks;
-    repack_adapter_block<T>(p, b, reinterpret_cast<float(*)[33]>(smem));
+    const uint32_t b = blockIdx.x;
+    if (b < p.code_blocks) repack_codes_block(p, b, smem);
+    else if (b < p.code_blocks + p.scale_blocks) repack_scales_block(p, b - p.code_blocks, reinterpret_cast<float(*)[33]>(smem));
+    else repack_adapter_block<T>(p, b - p.code_blocks - p.scale_blocks, reinterpret_cast<float(*)[33]>(smem));
+    if (p.wait_last && b == 0) ptx::pdl_wait();
 }
 
 // ---- host side -----------------------------------------------------------------------
@@ -1135,9 +1138,20 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_o
     p.sk_flags = reinterpret_cast<uint32_t *>(ws + wl.off_flags);
     p.partial = reinterpret_cast<float *>(ws + wl.off_partial);
     const void *lora_a = a.lora_a, *lora_b = a.lora_b;
-    bool packing = false;
-    if (repacked || (x_f32 && p.rank)) {  // the other orientation, f32 factors, or both
-        RepackParams rp{};
+    RepackParams rp{};
+    auto repack = [&](bool weight, bool a, bool b, bool wait_last) -> int32_t {
+        RepackParams part = rp;
+        if (!weight) part.code_blocks = part.scale_blocks = 0;
+        const uint32_t b_blocks = rp.adapter_blocks - rp.a_blocks;
+        part.a_blocks = a ? rp.a_blocks : 0;
+        part.adapter_blocks = part.a_blocks + (b ? b_blocks : 0);
+        part.wait_last = wait_last;
+        const uint32_t blocks = part.code_blocks + part.scale_blocks + part.adapter_blocks;
+        count_launch();
+        return launch_maybe_overlapped(x_f32 ? repack_kernel<float> : repack_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, true, part);
+    };
+    const bool factors_first = x_f32 && p.rank;  // the pre-pass reads a converted factor
+    if (repacked || factors_first) {  // the other orientation, f32 factors, or both
         rp.factors_out_in = !repacked;
         rp.codes = a.packed;
         rp.absmax = a.absmax;
@@ -1163,16 +1177,11 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_o
             if (x_f32) lora_a = rp.a_t;
             lora_b = rp.b_t;
         }
-        const uint32_t blocks = rp.code_blocks + rp.scale_blocks + rp.adapter_blocks;
-        if (x_f32) repack_kernel<float><<<blocks, 256, 0, stream>>>(rp);
-        else repack_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(rp);
-        count_launch();
         if (repacked) {
             p.codes = rp.codes_t;
             p.scales_t = rp.scales_t;
         }
-        NF4_CUDA_TRY(cudaGetLastError());
-        packing = true;
+        if (factors_first) NF4_TRY(repack(false, true, true, false));
     }
     PrepassArgs pre{};
     pre.x = a.x;
@@ -1192,9 +1201,9 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_o
     pre.scale_of_scales = a.scale_of_scales;
     pre.flags = p.sk_flags;
     pre.n_flags = 2 * sh.pairs;
-    pre.beside_predecessor = packing;
-    pre.factor_of_predecessor = x_f32 && p.rank;  // (f32 factors come through the repacking launch)
+    pre.factor_of_predecessor = factors_first;
     NF4_TRY(activations_prepass(pre, stream));
+    if (repacked) NF4_TRY(repack(true, false, !factors_first, true));
 
     CUtensorMap map_x, map_t, map_b, map_y, map_w;
     NF4_TRY(make_map(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.codes, p.N, p.K / 2, p.K / 2, BM, 128, CU_TENSOR_MAP_SWIZZLE_128B));

@@ -58,7 +58,7 @@ struct Params {
     uint32_t a_vec;        // the factor's rows are 16-byte aligned
     uint32_t piece;        // k per CTA, a multiple of 64
     float scale;
-    uint32_t wait;         // for the kernel ahead: 0 first of all, 1 before the factor is read, 2 at the end
+    uint32_t wait;         // for the kernel ahead: 0 first of all, 1 before the factor is read
 };
 
 // Running maxima of |bf16|, a pair at a time (the sign bits mean nothing); a NaN leaves the maximum as
@@ -422,7 +422,6 @@ prepass_kernel(const Params p) {
         }
         cluster.sync();  // the sums have been read (before the next chunk's stages, and before a CTA leaves)
     }
-    if (p.wait == 2) ptx::pdl_wait();
 }
 
 // ---- the same for bf16 x and a factor on tcgen05: up to 64 ranks, rows of 16-byte pieces -------------------------------
@@ -667,7 +666,6 @@ prepass_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         ptx::tc_fence_after();
         ptx::tmem_dealloc(acc, 64);
     }
-    if (p.wait == 2) ptx::pdl_wait();
 }
 
 }  // namespace
@@ -751,7 +749,7 @@ int32_t activations_prepass(const PrepassArgs &q, cudaStream_t stream) {
     p.chunks = (q.rank + 63) / 64;
     p.a_vec = aligned16(q.a) && (q.k_major ? q.rank : q.K) % 8 == 0;
     p.scale = q.scale;
-    p.wait = !q.beside_predecessor ? 0 : q.factor_of_predecessor ? 1 : 2;
+    p.wait = q.factor_of_predecessor ? 1 : 0;
     // The tcgen05 kernel, where its TMA takes the tensors: always for the product alone ([16, 11008] and [14, 768] the same
     // time); with the copy from four million values on (whole forwards to 512 columns: [1024, 4096] at rank 64 42.7 -> 40.3 us,
     // [4096, 1024] 23.7 -> 23.1, but [512, 2048] 27.5 -> 30.3 and [256, 4096] at rank 16 the other way too: an SM
