@@ -127,3 +127,51 @@ def test_forward_under_capture_replays_beside_eager_calls():
         again = forward(*c)
     torch.cuda.synchronize()
     assert torch.equal(y, want) and torch.equal(again, want)
+
+
+@pytest.mark.parametrize("rows,k,n,r", [
+    (1, 256, 16, 0),         # one CTA fetches x and is the last as well
+    (16, 20480, 1024, 8),    # more of x than the first CTAs fetch at a time, K in parts
+    (3, 4352, 96, 16),
+    (5, 320, 192, 8),        # d_in the kernel does not fetch for: copies and the stream's synchronise
+])
+def test_page_locked_calls_give_the_same_bits(rows, k, n, r):
+    # x fetched by the kernel and its word to the host, against copies of pageable memory; new values every call, from two
+    # threads at a time
+    import ctypes
+    import threading
+
+    from unifur_b200.quantize import PackedNf4Tensor
+
+    L, g = _lib.load(), torch.Generator(device="cuda").manual_seed(k + n)
+    p = PackedNf4Tensor.quantize(torch.randn(k * n, device="cuda", generator=g) * 0.02)
+    codes, absmax = p.codes.cpu(), p.absmax.cpu()
+    a, b = (torch.randn(*s, device="cuda", generator=g).bfloat16().cpu() * 0.05 for s in ((max(r, 1), k), (n, max(r, 1))))
+    h = ctypes.c_void_p()
+    _lib.check(L.nf4_weight_from_packed_host(codes.data_ptr(), absmax.data_ptr(), None, 0.0, k, n, _lib.LAYOUT_OUT_IN, ctypes.byref(h)))
+    if r:
+        _lib.check(L.nf4_weight_attach_lora_host(h, a.data_ptr(), b.data_ptr(), r, 1.5, _lib.DTYPE_BF16))
+    call = lambda x, y: _lib.check(L.nf4_weight_linear_forward_host(  # noqa: E731
+        h, x.data_ptr(), rows, _lib.DTYPE_BF16, None, None, None, 0, 0.0, y.data_ptr()))
+    wrong = []
+
+    def work(seed):
+        gen = torch.Generator().manual_seed(seed)
+        xl, yl = torch.empty(rows, k, dtype=torch.bfloat16).pin_memory(), torch.empty(rows, n, dtype=torch.bfloat16).pin_memory()
+        for _ in range(25):
+            x, y = torch.randn(rows, k, generator=gen).bfloat16(), torch.empty(rows, n, dtype=torch.bfloat16)
+            xl.copy_(x)
+            yl.fill_(7.0)
+            call(xl, yl)
+            got = yl.clone()
+            call(x, y)
+            if not torch.equal(got, y):
+                wrong.append(seed)
+
+    try:
+        threads = [threading.Thread(target=work, args=(s,)) for s in (1, 2)]
+        [t.start() for t in threads]
+        [t.join() for t in threads]
+        assert not wrong
+    finally:
+        L.nf4_weight_free(h)

@@ -179,6 +179,48 @@ struct ZeroScratch {
 };
 thread_local ZeroScratch t_zero_scratch;
 
+// A word of mapped host memory per host thread that a kernel writes when its results are in place, and the value
+// the thread's last such call waited for.
+struct DoneWord {
+    volatile uint32_t *host = nullptr;
+    uint32_t *device = nullptr;
+    uint32_t value = 0;
+    int32_t get() {
+        if (host) return NF4_OK;
+        uint32_t *h = nullptr;
+        NF4_CUDA_TRY(cudaHostAlloc(reinterpret_cast<void **>(&h), sizeof(uint32_t), cudaHostAllocMapped | cudaHostAllocPortable));
+        *h = 0;
+        NF4_CUDA_TRY(cudaHostGetDevicePointer(reinterpret_cast<void **>(&device), h, 0));
+        host = h;
+        return NF4_OK;
+    }
+    // Until the word has the value, or the stream has an error or nothing left to do.
+    int32_t wait(cudaStream_t stream) const {
+        for (uint32_t i = 1; *host != value; ++i) {
+#if defined(__x86_64__)
+            __builtin_ia32_pause();
+#endif
+            if (i % 4096 != 0) continue;
+            const cudaError_t e = cudaStreamQuery(stream);
+            if (e != cudaErrorNotReady) return check_cuda(e, "waiting for the kernel's word");
+        }
+        std::atomic_thread_fence(std::memory_order_acquire);
+        return NF4_OK;
+    }
+    ~DoneWord() {
+        if (host) cudaFreeHost(const_cast<uint32_t *>(host));
+    }
+};
+thread_local DoneWord t_done;
+
+// The device's address of page-locked host memory it can reach, or null.
+void *device_view(const void *host) {
+    cudaPointerAttributes attr{};
+    if (cudaPointerGetAttributes(&attr, host) == cudaSuccess && attr.type == cudaMemoryTypeHost) return attr.devicePointer;
+    (void)cudaGetLastError();  // pageable memory is reported as an error by older drivers: not one here
+    return nullptr;
+}
+
 constexpr uint64_t kFlagWordBytes = 256;  // at the start of a workspace
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
@@ -1093,7 +1135,8 @@ int32_t nf4_weight_linear_forward_host(const nf4_weight *w, const void *x, uint6
         lora_scale = w->lora_scale;
     }
     const uint32_t r = (lora_a || resident) ? lora_rank : 0;
-    const uint64_t ws = nf4_linear_workspace_bytes(rows, w->d_in, w->d_out, r);
+    uint64_t ws = nf4_linear_workspace_bytes(rows, w->d_in, w->d_out, r);
+    if (rows <= 16 && ws < kFlagWordBytes) ws = kFlagWordBytes;  // (the words a call that fetches x itself meets on)
     const size_t xb = rows * w->d_in * eb, yb = rows * w->d_out * eb;
     const size_t ab = resident ? 0 : (size_t)r * w->d_in * eb;
     const size_t bb = resident ? 0 : (size_t)r * w->d_out * eb;
@@ -1106,7 +1149,15 @@ int32_t nf4_weight_linear_forward_host(const nf4_weight *w, const void *x, uint6
     uint8_t *d_b = cv.take<uint8_t>(bb);
     float *d_bias = cv.take<float>(w->d_out);
     uint8_t *d_ws = cv.take<uint8_t>(ws);
-    NF4_CUDA_TRY(cudaMemcpyAsync(d_x, x, xb, cudaMemcpyHostToDevice, kHostStream));
+    // x and y of a decode-sized call that are page-locked memory the device can address (cudaHostAlloc, cudaHostRegister
+    // with the mapped flag) need no copy operation: the kernel stores its results to y itself, and where it also
+    // fetches x, the host waits for its word instead of the stream.  (Not for the tensor-core GEMM of more rows, which stores
+    // through a tensor map, and where the copies do not matter.)
+    void *const y_mapped = rows <= 16 ? device_view(y) : nullptr;
+    const bool fetches = w->layout == NF4_LAYOUT_OUT_IN && io_dtype == NF4_DTYPE_BF16 && w->d_in % 256 == 0;  // the decode kernel
+    void *const x_mapped = y_mapped && fetches ? device_view(x) : nullptr;
+    auto copy_x = [&] { return check_cuda(cudaMemcpyAsync(d_x, x, xb, cudaMemcpyHostToDevice, kHostStream), "copy of x"); };
+    if (!x_mapped) NF4_TRY(copy_x());
     if (r && !resident) {
         NF4_CUDA_TRY(cudaMemcpyAsync(d_a, lora_a, ab, cudaMemcpyHostToDevice, kHostStream));
         NF4_CUDA_TRY(cudaMemcpyAsync(d_b, lora_b, bb, cudaMemcpyHostToDevice, kHostStream));
@@ -1131,19 +1182,6 @@ int32_t nf4_weight_linear_forward_host(const nf4_weight *w, const void *x, uint6
     a.lora_rank = r;
     a.lora_scale = lora_scale;
     a.y = d_y;
-    // At decode sizes the two copies are half of the call's latency.  When y is page-locked memory
-    // the device can address (cudaHostAlloc, cudaHostRegister with the mapped flag), the kernel
-    // stores its results there itself: the copy back, a separate operation of some ten microseconds, goes.
-    // (Not for the tensor-core GEMM of more rows, which stores through a tensor map, and where the
-    // copies do not matter.)
-    void *y_mapped = nullptr;
-    if (rows <= 16) {
-        cudaPointerAttributes attr{};
-        if (cudaPointerGetAttributes(&attr, y) == cudaSuccess && attr.type == cudaMemoryTypeHost && attr.devicePointer)
-            y_mapped = attr.devicePointer;
-        else
-            (void)cudaGetLastError();  // pageable memory is reported as an error by older drivers: not one here
-    }
     if (y_mapped) a.y = y_mapped;
     a.ldy = w->d_out;
     a.workspace = ws ? d_ws : nullptr;
@@ -1158,9 +1196,20 @@ int32_t nf4_weight_linear_forward_host(const nf4_weight *w, const void *x, uint6
     uint64_t before = 0, after = 0;
     int codes[3];
     NF4_TRY(failures_found(&before, nullptr));
-    NF4_TRY(nf4_linear_forward_dev(&a, kHostStream));
-    if (!y_mapped) NF4_CUDA_TRY(cudaMemcpyAsync(y, d_y, yb, cudaMemcpyDeviceToHost, kHostStream));
-    NF4_TRY(check_cuda(cudaStreamSynchronize(kHostStream), "nf4_weight_linear_forward_host sync"));
+    bool taken = false;
+    if (x_mapped) {
+        NF4_TRY(t_done.get());
+        NF4_TRY(decode_forward_host(a, x_mapped, t_done.device, t_done.value + 1, kHostStream, &taken));
+        if (taken) ++t_done.value;
+        else NF4_TRY(copy_x());
+    }
+    if (taken) {
+        NF4_TRY(t_done.wait(kHostStream));
+    } else {
+        NF4_TRY(nf4_linear_forward_dev(&a, kHostStream));
+        if (!y_mapped) NF4_CUDA_TRY(cudaMemcpyAsync(y, d_y, yb, cudaMemcpyDeviceToHost, kHostStream));
+        NF4_TRY(check_cuda(cudaStreamSynchronize(kHostStream), "nf4_weight_linear_forward_host sync"));
+    }
     // ... and a wait that gave up in a kernel must not pass for a result
     NF4_TRY(failures_found(&after, codes));
     if (after != before) {

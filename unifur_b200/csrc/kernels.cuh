@@ -114,6 +114,7 @@ int32_t decode_forward(const nf4_linear_args &a, cudaStream_t stream);
 int32_t decode_forward_scatter(const nf4_linear_args &a, void *const *dest, uint32_t *const *arrive, uint32_t world,
                                uint32_t rank, uint64_t ldy, bool signal, uint32_t *wait_on, uint32_t wait_expected,
                                cudaStream_t stream);
+int32_t decode_forward_host(const nf4_linear_args &a, const void *x_host, uint32_t *host_done, uint32_t value, cudaStream_t stream, bool *taken);
 int32_t decode_peer_wait(uint32_t *counter, uint32_t expected, uint32_t limit_ns, cudaStream_t stream);
 int32_t decode_share_plan(uint32_t rows, uint32_t d_in, uint32_t d_out, uint32_t rank, uint32_t cta, uint32_t *out4);
 int32_t decode_forward_grouped(const nf4_linear_args *a, uint32_t count, cudaStream_t stream, bool *taken);
