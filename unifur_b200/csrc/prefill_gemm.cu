@@ -83,7 +83,7 @@ constexpr int kXTileBytes = BN / 2 * BK * 2;   // 16 KB: this CTA's half of the 
 constexpr int kLoraTileBytes = BM * BK * 2;    // 16 KB: 128 rows of LoRA B x 64 ranks, written by TMA
 constexpr int kCodeTileBytes = BM * 128;       // 16 KB: 128 weight rows x 256 codes, written by TMA (128B swizzle)
 
-constexpr int kEpiBytes = 32 * 1024;       // output staging: half a tile of bf16, a quarter of f32
+constexpr int kEpiBytes = 32 * 1024;       // output staging: half a tile of bf16 (as two swizzled boxes), a quarter of f32
 constexpr int kThreads = 27 * 32;
 constexpr int kFirstExpanderWarp = 7;      // sixteen warps
 constexpr int kFirstEpilogueWarpB = 23;    // the second set of four epilogue warps
@@ -407,10 +407,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     } else if (warp < 6 || warp >= kFirstEpilogueWarpB) {
         // ============================== epilogue ==============================
         // The MMAs of the next tile wait for the accumulator, so it is read out as fast as eight
-        // warps can (two per TMEM lane quarter, each taking half of the columns): the whole tile
-        // (bf16) or half of it (f32) goes through one staging buffer, two TMEM loads in
-        // flight per warp, and the accumulator is handed back before the last values are
-        // converted; the TMA store of the last values then overlaps the next tile's MMAs.
+        // warps can (two per TMEM lane quarter, each taking half of the columns): half of the tile
+        // (bf16) or a quarter of it (f32) goes through one staging buffer at a time, and the accumulator is
+        // handed back before the last values are stored; their TMA store then overlaps the next tile's MMAs.
         const uint32_t set = warp >= kFirstEpilogueWarpB ? 1u : 0u;
         const uint32_t q = warp & 3u;  // TMEM lane quarter this warp may touch
         const uint32_t row_in_tile = q * 32 + lane;
@@ -469,7 +468,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                     --first_helper;
                 } while (first_helper > 0 && WorkList::range_begin(all, first_helper, pairs) > t0);
             }
-            const float bias = (p.bias && n < p.N) ? __ldg(p.bias + n) : 0.0f;
             // the rows' factors go to shared memory while the MMAs still run: a global load per
             // value inside the read-out would wait for L2 every time (the L1 left beside 227 KB
             // of shared memory is small and the dequantisers stream through it)
@@ -477,43 +475,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             ok = ptx::mbar_wait_suspended(bar(kBarAccFull), i & 1u);
             if (!ok) break;
             ptx::tc_fence_after();
-            uint32_t va[16], vb[16];
-            ptx::tmem_ld16(acc_lane + col_of(0), va);
-            // staging layout: [kStageRows activation rows][BM weight rows]
-            auto stage_chunk = [&](const uint32_t (&v)[16], uint32_t col) {
-                const uint32_t r0 = col % kStageRows;
-                // the factors first, as vectors: a load per value between the stores could not be
-                // moved ahead of them (both are shared memory) and each would wait out its latency
-                float rs[16];
-                #pragma unroll
-                for (int r4 = 0; r4 < 4; ++r4) {
-                    const float4 f4 = reinterpret_cast<const float4 *>(row_scales + col)[r4];
-                    rs[4 * r4 + 0] = f4.x;
-                    rs[4 * r4 + 1] = f4.y;
-                    rs[4 * r4 + 2] = f4.z;
-                    rs[4 * r4 + 3] = f4.w;
-                }
-                #pragma unroll
-                for (int r = 0; r < 16; ++r) {
-                    const float f = fmaf(__uint_as_float(v[r]), rs[r], bias);
-                    if (YF32)
-                        reinterpret_cast<float *>(epi)[(r0 + r) * BM + row_in_tile] = f;
-                    else
-                        reinterpret_cast<__nv_bfloat16 *>(epi)[(r0 + r) * BM + row_in_tile] =
-                            __float2bfloat16_rn(f);
-                }
-            };
-            auto add_helpers = [&](uint32_t (&v)[16], uint32_t col) {
-                if (m0 + col >= p.M) return;
-                for (uint32_t h = first_helper; h < pair; ++h) {
-                    const float *src = p.partial + (size_t)(2 * h + rank) * (BM * BN) + (size_t)col * BM + row_in_tile;
-                    float part[16];
-                    #pragma unroll
-                    for (int r = 0; r < 16; ++r) part[r] = __ldcg(src + r * BM);
-                    #pragma unroll
-                    for (int r = 0; r < 16; ++r) v[r] = __float_as_uint(__uint_as_float(v[r]) + part[r]);
-                }
-            };
             if (first_helper != pair && epi_leader) {
                 // bounded wait for the helpers' flags (they dumped before anything else they did)
                 const uint64_t t_begin = ptx::global_timer_ns();
@@ -529,43 +490,176 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 if (!ok) NF4_REPORT_FAILURE(g_prefill_error, g_prefill_error_host, 5);  // the sums are wrong; the flag says so
                 ok = true;  // the read-out goes on (every role must finish its segments)
             }
-            for (uint32_t k = 0; k < kLoads; k += 2) {
-                if (k % kPerPass == 0) {
-                    // the TMA store that last read the staging buffer must be done with it
+            if constexpr (YF32) {
+                const float bias = (p.bias && n < p.N) ? __ldg(p.bias + n) : 0.0f;
+                uint32_t va[16], vb[16];
+                ptx::tmem_ld16(acc_lane + col_of(0), va);
+                // staging layout: [kStageRows activation rows][BM weight rows]
+                auto stage_chunk = [&](const uint32_t (&v)[16], uint32_t col) {
+                    const uint32_t r0 = col % kStageRows;
+                    // the factors first, as vectors: a load per value between the stores could not be
+                    // moved ahead of them (both are shared memory) and each would wait out its latency
+                    float rs[16];
+                    #pragma unroll
+                    for (int r4 = 0; r4 < 4; ++r4) {
+                        const float4 f4 = reinterpret_cast<const float4 *>(row_scales + col)[r4];
+                        rs[4 * r4 + 0] = f4.x;
+                        rs[4 * r4 + 1] = f4.y;
+                        rs[4 * r4 + 2] = f4.z;
+                        rs[4 * r4 + 3] = f4.w;
+                    }
+                    #pragma unroll
+                    for (int r = 0; r < 16; ++r) {
+                        const float f = fmaf(__uint_as_float(v[r]), rs[r], bias);
+                        reinterpret_cast<float *>(epi)[(r0 + r) * BM + row_in_tile] = f;
+                    }
+                };
+                auto add_helpers = [&](uint32_t (&v)[16], uint32_t col) {
+                    if (m0 + col >= p.M) return;
+                    for (uint32_t h = first_helper; h < pair; ++h) {
+                        const float *src = p.partial + (size_t)(2 * h + rank) * (BM * BN) + (size_t)col * BM + row_in_tile;
+                        float part[16];
+                        #pragma unroll
+                        for (int r = 0; r < 16; ++r) part[r] = __ldcg(src + r * BM);
+                        #pragma unroll
+                        for (int r = 0; r < 16; ++r) v[r] = __float_as_uint(__uint_as_float(v[r]) + part[r]);
+                    }
+                };
+                for (uint32_t k = 0; k < kLoads; k += 2) {
+                    if (k % kPerPass == 0) {
+                        // the TMA store that last read the staging buffer must be done with it
+                        if (epi_leader) ptx::tma_store_wait_read<0>();
+                        asm volatile("bar.sync 1, 256;" ::: "memory");
+                    }
+                    ptx::tmem_wait_ld();
+                    ptx::tmem_ld16(acc_lane + col_of(k + 1), vb);
+                    if (first_helper != pair) add_helpers(va, col_of(k));
+                    stage_chunk(va, col_of(k));
+                    ptx::tmem_wait_ld();
+                    if (first_helper != pair) add_helpers(vb, col_of(k + 1));
+                    if (k + 2 < kLoads) {
+                        ptx::tmem_ld16(acc_lane + col_of(k + 2), va);
+                    } else {
+                        // this warp's part of the accumulator is read: hand it back to the MMA threads
+                        ptx::tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) ptx::mbar_arrive_cluster(acc_empty);
+                    }
+                    stage_chunk(vb, col_of(k + 1));
+                    if ((k + 2) % kPerPass == 0) {
+                        ptx::fence_proxy_async();
+                        asm volatile("bar.sync 1, 256;" ::: "memory");
+                        // (an odd number of 128-row tiles: the last odd CTA's rows do not exist)
+                        const uint32_t m = m0 + (k / kPerPass) * kStageRows;
+                        if (p.y_ragged && n0 + BM > p.N) {
+                            #pragma unroll 1
+                            for (uint32_t e = epi_thread; e < kStageRows * BM; e += 256) {
+                                const uint32_t row = m + e / BM, col = n0 + e % BM;
+                                if (row < p.M && col < p.N) static_cast<float *>(p.y_ragged)[row * p.ldy + col] = reinterpret_cast<const float *>(epi)[e];
+                            }
+                        } else if (epi_leader && n0 < p.N && m < p.M) {
+                            ptx::tma_store_2d(&tmap_y, own | kEpiAt, (int32_t)n0, (int32_t)m);
+                            ptx::tma_store_commit();
+                        }
+                    }
+                }
+            } else {
+                // bf16: fragments of 16 weight rows x 32 columns, so that two neighbouring columns are converted to one
+                // register and a transposing matrix store puts eight weight rows of a column side by side: 16 two-byte
+                // stores for 16 columns took 400 cycles (700 x 4096 x 14336: 89.4 -> 86.8 us, 1000 x 8192 x 8192 129 -> 126,
+                // 2048 x 4096 x 14336, at the power limit, 209 -> 206).  The first half of the columns goes to the staging
+                // buffer and out; half of the second is in registers when the buffer is free again.
+                const uint32_t fn = lane >> 2, fm = 2u * (lane & 3u), mi = lane & 7u, mq = lane >> 3;
+                const uint32_t nq = n0 + q * 32 + fn;
+                auto bias_of = [&](uint32_t row) { return p.bias && row < p.N ? __ldg(p.bias + row) : 0.0f; };
+                auto convert = [&](uint32_t col, uint32_t half, uint32_t *w) {  // -> eight registers
+                    uint32_t v[16];
+                    ptx::tmem_ld_fragments(acc_lane + ((half * 16) << 16) + col, v);
+                    const float b0 = bias_of(nq + half * 16), b1 = bias_of(nq + half * 16 + 8);
+                    ptx::tmem_wait_ld();
+                    if (m0 + col < p.M)
+                        for (uint32_t h = first_helper; h < pair; ++h) {
+                            const float *src = p.partial + (size_t)(2 * h + rank) * (BM * BN) + (size_t)(col + fm) * BM + q * 32 + half * 16 + fn;
+                            #pragma unroll
+                            for (int j = 0; j < 4; j += 2) {
+                                float part[8];
+                                #pragma unroll
+                                for (int r = 0; r < 8; ++r) part[r] = __ldcg(src + (8 * (j + (r >> 2)) + (r & 1)) * BM + ((r >> 1) & 1) * 8);
+                                #pragma unroll
+                                for (int r = 0; r < 8; ++r) v[4 * j + r] = __float_as_uint(__uint_as_float(v[4 * j + r]) + part[r]);
+                            }
+                        }
+                    #pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float2 rs = *reinterpret_cast<const float2 *>(row_scales + col + 8 * j + fm);
+                        #pragma unroll
+                        for (int r = 0; r < 2; ++r) {
+                            const __nv_bfloat162 o = __floats2bfloat162_rn(fmaf(__uint_as_float(v[4 * j + 2 * r]), rs.x, r ? b1 : b0),
+                                                                          fmaf(__uint_as_float(v[4 * j + 2 * r + 1]), rs.y, r ? b1 : b0));
+                            w[2 * j + r] = *reinterpret_cast<const uint32_t *>(&o);
+                        }
+                    }
+                };
+                // staging: two boxes of 64 weight rows, [128 activation rows][128 bytes] with the store's swizzle
+                auto stage = [&](uint32_t col, uint32_t half, const uint32_t *w) {
+                    const uint32_t oct = q * 4 + half * 2 + (mq & 1u);
+                    #pragma unroll
+                    for (uint32_t j = 0; j < 4; j += 2) {
+                        const uint32_t row = col + (j + (mq >> 1)) * 8 + mi;
+                        ptx::stmatrix_x4_trans((own | kEpiAt) + (oct >> 3) * (kEpiBytes / 2) + row * 128 + (((oct & 7u) ^ (row & 7u)) << 4),
+                                               w[2 * j], w[2 * j + 1], w[2 * j + 2], w[2 * j + 3]);
+                    }
+                };
+                auto send = [&](uint32_t m) {  // the staged 128 activation rows from m on (an odd last CTA has no weight rows)
+                    ptx::fence_proxy_async();
+                    asm volatile("bar.sync 1, 256;" ::: "memory");
+                    if (p.y_ragged && n0 + BM > p.N) {
+                        #pragma unroll 1
+                        for (uint32_t e = epi_thread; e < kStageRows * BM; e += 256) {
+                            const uint32_t r = e / BM, c = e % BM;
+                            if (m + r < p.M && n0 + c < p.N)
+                                static_cast<__nv_bfloat16 *>(p.y_ragged)[(size_t)(m + r) * p.ldy + n0 + c] = *reinterpret_cast<const __nv_bfloat16 *>(
+                                    epi + (c >> 6) * (kEpiBytes / 2) + r * 128 + ((((c >> 3) & 7u) ^ (r & 7u)) << 4) + (c & 7u) * 2);
+                        }
+                    } else if (epi_leader) {
+                        if (n0 < p.N) ptx::tma_store_2d(&tmap_y, own | kEpiAt, (int32_t)n0, (int32_t)m);
+                        if (n0 + 64 < p.N) ptx::tma_store_2d(&tmap_y, (own | kEpiAt) + kEpiBytes / 2, (int32_t)n0 + 64, (int32_t)m);
+                        ptx::tma_store_commit();
+                    }
+                };
+                auto buffer_free = [&]() {
                     if (epi_leader) ptx::tma_store_wait_read<0>();
                     asm volatile("bar.sync 1, 256;" ::: "memory");
-                }
-                ptx::tmem_wait_ld();
-                ptx::tmem_ld16(acc_lane + col_of(k + 1), vb);
-                if (first_helper != pair) add_helpers(va, col_of(k));
-                stage_chunk(va, col_of(k));
-                ptx::tmem_wait_ld();
-                if (first_helper != pair) add_helpers(vb, col_of(k + 1));
-                if (k + 2 < kLoads) {
-                    ptx::tmem_ld16(acc_lane + col_of(k + 2), va);
-                } else {
-                    // this warp's part of the accumulator is read: hand it back to the MMA threads
+                };
+                auto hand_back = [&]() {  // this warp's part of the accumulator is read
                     ptx::tc_fence_before();
                     __syncwarp();
                     if (lane == 0) ptx::mbar_arrive_cluster(acc_empty);
+                };
+                const uint32_t at = set * 64;  // a set's columns of a half: four pieces of 16 weight rows x 32 columns
+                uint32_t w[2][8];
+                buffer_free();
+                #pragma unroll
+                for (uint32_t c = 0; c < 4; ++c) {
+                    convert(at + (c >> 1) * 32, c & 1u, w[0]);
+                    stage(at + (c >> 1) * 32, c & 1u, w[0]);
                 }
-                stage_chunk(vb, col_of(k + 1));
-                if ((k + 2) % kPerPass == 0) {
-                    ptx::fence_proxy_async();
-                    asm volatile("bar.sync 1, 256;" ::: "memory");
-                    // (an odd number of 128-row tiles: the last odd CTA's rows do not exist)
-                    const uint32_t m = m0 + (k / kPerPass) * kStageRows;
-                    if (p.y_ragged && n0 + BM > p.N) {
-                        using Y = typename std::conditional<YF32, float, __nv_bfloat16>::type;
-                        #pragma unroll 1
-                        for (uint32_t e = epi_thread; e < kStageRows * BM; e += 256) {
-                            const uint32_t row = m + e / BM, col = n0 + e % BM;
-                            if (row < p.M && col < p.N) static_cast<Y *>(p.y_ragged)[row * p.ldy + col] = reinterpret_cast<const Y *>(epi)[e];
-                        }
-                    } else if (epi_leader && n0 < p.N && m < p.M) {
-                        ptx::tma_store_2d(&tmap_y, own | kEpiAt, (int32_t)n0, (int32_t)m);
-                        ptx::tma_store_commit();
+                send(m0);
+                if (m0 + kStageRows < p.M) {
+                    #pragma unroll
+                    for (uint32_t c = 0; c < 2; ++c) convert(kStageRows + at, c, w[c]);
+                    buffer_free();
+                    #pragma unroll
+                    for (uint32_t c = 0; c < 2; ++c) stage(at, c, w[c]);
+                    #pragma unroll
+                    for (uint32_t c = 0; c < 2; ++c) {
+                        convert(kStageRows + at + 32, c, w[0]);
+                        if (c == 1) hand_back();
+                        stage(at + 32, c, w[0]);
                     }
+                    send(m0 + kStageRows);
+                } else {
+                    hand_back();
                 }
             }
         }
@@ -1222,8 +1316,8 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_o
         NF4_TRY(make_map(&map_y, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, a.y, p.M, p.N, ldy * 4, kEpiBytes / (BM * 4), BM,
                          CU_TENSOR_MAP_SWIZZLE_NONE));
     else
-        NF4_TRY(make_map(&map_y, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a.y, p.M, p.N, ldy * 2, kEpiBytes / (BM * 2), BM,
-                         CU_TENSOR_MAP_SWIZZLE_NONE));
+        NF4_TRY(make_map(&map_y, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a.y, p.M, p.N, ldy * 2, kEpiBytes / (BM * 2), BM / 2,
+                         CU_TENSOR_MAP_SWIZZLE_128B));
 
     auto go = [&](auto kernel) -> int32_t {
         NF4_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), (int)kDynamicSmem));

@@ -256,6 +256,22 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         : "r"(taddr)
         : "memory");
 }
+// 16 lanes x 32 consecutive 32-bit columns as an MMA's accumulator fragments: thread t has, of every eight columns, lane
+// t / 4 (r[4j], r[4j + 1]) and t / 4 + 8 (r[4j + 2], r[4j + 3]) of columns 8j + 2 (t % 4) and the next.
+__device__ __forceinline__ void tmem_ld_fragments(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,"
+        "%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+          "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
+// Four 8 x 8 matrices of 16-bit values, transposed: lane 8i + c gives the address of column c of matrix i.
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
 // Shared-memory matrix descriptor, 128-byte swizzle, version 1, rows of 128 bytes, eight of them 1024 bytes apart (SBO).
 // K-major operands: a row is 64 k of one M or N.  MN-major operands: a row is 64 M or N of one k; the next 64 are
 // `block` bytes on (LBO).
