@@ -18,6 +18,10 @@ from unifur_b200 import _lib  # noqa: E402
     (6, 8192, 64, 64, True, True),
     (8, 640, 11008, 16, False, True),    # CTAs with the end of one strip and the start of the next
     (13, 4160, 1344, 32, True, True),    # activations of K in several pieces
+    (2, 300, 2304, 4, False, True),      # a cluster to a strip, a unit to a CTA, the last one short
+    (1, 4096, 10944, 0, True, True),     # clusters of three with unequal parts, the last strip three quarters full
+    (7, 3072, 8192, 16, False, False),
+    (11, 1536, 6976, 24, True, True),
     (16, 20480, 128, 8, False, False),
     (37, 100, 192, 3, False, True),      # d_in the tensor-core path does not take: sixteen rows per launch
     (5, 64, 63552, 0, True, False),      # more strips than counters: whole strips per CTA

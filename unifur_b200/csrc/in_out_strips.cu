@@ -15,17 +15,20 @@
 // word with {8 lane, 0, 1, 0} is the whole address; the 64-bit entry is an operand of a packed
 // multiply-add (fma.rn.f32x2) as it is.  Three instructions per two weights at one row (eight per weight
 // in the kernel before, which scaled every weight, added the table's base and multiplied single f32).
-// What bounds it.  At one row neither pipe: of 15.7 us the lookups' shared-memory wavefronts are 5.9 (two per lookup)
+// What bounds it.  At one row neither pipe: of 15.7 us (runs) the lookups' shared-memory wavefronts are 5.9 (two per lookup)
 // and the instructions 4.4 (3.6 per weight with everything around the loop); the rest is latency at the ends of the
 // segments: the first codes from idle, the barriers around a piece of x, the meeting of a strip's segments.  From
 // about eight rows on the f32 rate.  f32 x [M, 4096], W [4096, 11008], f32
 // scales, calls back to back, before -> now: 29.8 -> 16.4 us at one row, 36.4 -> 21.2 at four, 49.1 -> 31.2 at
 // eight, 88.6 -> 55.9 at sixteen.
+// Where there are few strips, a strip is a cluster's instead (template parameter CLUSTER): every CTA has one segment, and the
+// strip's sums meet through distributed shared memory, in order, each CTA finishing a share of the columns (cluster_parts).
 //
 // Sums.  Lanes with the same columns meet by shuffles, the warps in shared memory, segments that share a
 // strip in global memory, where the CTA that arrives last for a strip (a byte counter per strip in the
 // workspace's flag words, zero at first use, left zero) adds them in the order of the runs: every sum has
 // a fixed order.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
 #include "kernels.cuh"
@@ -56,6 +59,7 @@ struct StripParams {
     float lora_scale;
     uint32_t units_per_strip, total_units;
     uint32_t whole_strips;  // runs are whole strips (more strips than counters)
+    uint32_t parts;         // CLUSTER: a strip is a cluster's of so many CTAs, an equal part of its units each one's
     uint32_t x_rows;        // rows of W whose activations are in shared memory at a time
     uint32_t f32, y_f32, y_vec;
 };
@@ -123,7 +127,7 @@ __device__ __forceinline__ void finish4(const StripParams &p, uint32_t m, uint32
     }
 }
 
-template <int MR, int CPL, int THREADS, int D, bool DQ>
+template <int MR, int CPL, int THREADS, int D, bool DQ, bool CLUSTER>
 __global__ void __launch_bounds__(THREADS, 1) in_out_strip_kernel(const StripParams p) {
     constexpr uint32_t kWarps = THREADS / 32, LPR = kStripCols / CPL, RS = 32 / LPR, kStep = kWarps * RS;
     constexpr int kWords = CPL / 8;
@@ -133,9 +137,9 @@ __global__ void __launch_bounds__(THREADS, 1) in_out_strip_kernel(const StripPar
     extern __shared__ __align__(16) uint8_t dyn[];
     __shared__ uint32_t last_s;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-    const uint32_t win = ptx::smem_addr(dyn);
+    const uint32_t win = ptx::smem_addr(dyn), own = CLUSTER ? win & 0xff000000u : 0u;  // (a cluster's CTAs have their rank in the top byte)
     float *xs = reinterpret_cast<float *>(dyn);                             // [row of the piece][MR]
-    uint8_t *table = dyn + (kTableAt - win);
+    uint8_t *table = dyn + ((own | kTableAt) - win);
     float *red = reinterpret_cast<float *>(table + 0x10000);                // [warp][MG][256]
     {
         // thread (byte, part) writes the copies of 32 * 256 / THREADS lanes, rotated over the banks
@@ -148,13 +152,16 @@ __global__ void __launch_bounds__(THREADS, 1) in_out_strip_kernel(const StripPar
     }
     const float sos = DQ ? __ldg(p.scale_of_scales) : 0.0f;
     const uint32_t sub = lane / LPR, in_row = lane % LPR;
-    const uint32_t lane_word = (lane * 8u) | 0x00010000u;  // bytes {8 lane, 0, 1, 0}
+    const uint32_t lane_word = (lane * 8u) | kTableAt | own;  // bytes {8 lane, 0, 1, rank}
     const uint32_t blocks_per_row = p.N / kBlock;
     const uint32_t ctas = gridDim.x;
     uint32_t u = p.whole_strips ? run_begin(p.total_units / p.units_per_strip, blockIdx.x, ctas) * p.units_per_strip
                                 : run_begin(p.total_units, blockIdx.x, ctas);
-    const uint32_t u_end = p.whole_strips ? run_begin(p.total_units / p.units_per_strip, blockIdx.x + 1, ctas) * p.units_per_strip
+    const uint32_t run_end = p.whole_strips ? run_begin(p.total_units / p.units_per_strip, blockIdx.x + 1, ctas) * p.units_per_strip
                                           : run_begin(p.total_units, blockIdx.x + 1, ctas);
+    const uint32_t cluster_strip = CLUSTER ? blockIdx.x / p.parts : 0u, cluster_part = CLUSTER ? blockIdx.x - cluster_strip * p.parts : 0u;
+    const uint32_t u_end = CLUSTER ? cluster_strip * p.units_per_strip + run_begin(p.units_per_strip, cluster_part + 1, p.parts) : run_end;
+    if (CLUSTER) u = cluster_strip * p.units_per_strip + run_begin(p.units_per_strip, cluster_part, p.parts);
     const uint32_t u_begin = u;
     bool first = true;
     while (u < u_end) {
@@ -298,7 +305,7 @@ __global__ void __launch_bounds__(THREADS, 1) in_out_strip_kernel(const StripPar
         const uint32_t group = CPL == 32 ? in_row * 4 + ((lane >> 4) & 1u) * 2 + ((lane >> 3) & 1u)
                                : CPL == 16 ? in_row * 2 + (lane >> 4) : lane;
         auto place = [](uint32_t q) { return q ^ ((q >> 3) & 7u); };
-        const bool whole = b == 0 && e == p.units_per_strip;
+        const bool whole = !CLUSTER && b == 0 && e == p.units_per_strip;
         // (a CTA shares its first strip and its last one at most)
         float *slot = p.partial + (size_t)(2 * blockIdx.x + (u == u_begin ? 0 : 1)) * (MR * kStripCols);
         #pragma unroll
@@ -320,9 +327,30 @@ __global__ void __launch_bounds__(THREADS, 1) in_out_strip_kernel(const StripPar
                     s.x += o.x; s.y += o.y; s.z += o.z; s.w += o.w;
                 }
                 const uint32_t n = strip * kStripCols + 4 * q;
-                if (!whole) __stcg(reinterpret_cast<float4 *>(slot + (mg + m) * kStripCols) + q, s);
+                if (CLUSTER) reinterpret_cast<float4 *>(xs + (mg + m) * kStripCols)[q] = s;  // (the activations have been used)
+                else if (!whole) __stcg(reinterpret_cast<float4 *>(slot + (mg + m) * kStripCols) + q, s);
                 else if (mg + m < p.rows && n < p.N) finish4(p, mg + m, n, s);
             }
+        }
+        if (CLUSTER) {
+            // the cluster's sums, in the order of the parts; every CTA finishes a share of the outputs
+            namespace cg = cooperative_groups;
+            cg::cluster_group cluster = cg::this_cluster();
+            const uint32_t part = cluster.block_rank();
+            cluster.sync();
+            for (uint32_t i = tid * p.parts + part; i < MR * (kStripCols / 4); i += THREADS * p.parts) {
+                const uint32_t m = i / (kStripCols / 4), n = strip * kStripCols + 4 * (i % (kStripCols / 4));
+                if (m >= p.rows || n >= p.N) continue;
+                float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                #pragma unroll 4
+                for (uint32_t c = 0; c < p.parts; ++c) {
+                    const float4 o = reinterpret_cast<const float4 *>(cluster.map_shared_rank(xs, c))[i];
+                    s.x += o.x; s.y += o.y; s.z += o.z; s.w += o.w;
+                }
+                finish4(p, m, n, s);
+            }
+            cluster.sync();  // nobody leaves while its sums are being read
+            return;
         }
         if (!whole) {
             const uint32_t c0 = cta_of(strip * p.units_per_strip, p.total_units, ctas);
@@ -410,6 +438,24 @@ struct Runs {
     uint32_t ctas, units_per_strip, total;
     bool whole_strips;
 };
+// CTAs to a strip's cluster: 1 where runs over all strips are the better division.  A unit takes about 0.27 us at one row; a run's
+// meeting through global memory costs six of them, the ends of the second segments where runs do not divide the strips evenly
+// six more, a cluster's meeting four and half a unit for every CTA.  (More rows: longer units, and longer ends as well.)  1 x 4096 x 11008 15.7 -> 12.6 us in clusters of three, 1 x 512 x 11008 5.8 -> 5.0; in clusters of sixteen
+// 1 x 4096 x 2048 went from 6.2 to 7.0.
+uint32_t cluster_parts(const Runs &r, const ClusterRoom &room) {
+    const uint32_t strips = r.total / r.units_per_strip;
+    const uint32_t run = (r.total + r.ctas - 1) / r.ctas;
+    const bool equal = r.total % r.ctas == 0, whole = equal && run % r.units_per_strip == 0, even = equal && r.units_per_strip % run == 0;
+    uint32_t best = 1, least = run + (whole ? 0 : even ? 6 : 12);
+    for (uint32_t c = 2; c <= 8 && c <= r.units_per_strip; ++c) {
+        const uint32_t cost = (r.units_per_strip + c - 1) / c + 4 + c / 2;
+        if (strips <= room.any[c] && strips * c <= persistent_ctas() && (cost < least || (cost == least && best > 1))) {
+            least = cost;
+            best = c;
+        }
+    }
+    return best;
+}
 // A run keeps four units at least (256 rows of W: beyond that, what a strip's segments cost to meet
 // outweighs the parallelism), and one CTA per SM at most.
 bool deal_out(uint64_t K, uint64_t N, Runs &r) {
@@ -434,10 +480,35 @@ int32_t launch_as(StripParams &p, uint32_t ctas, cudaStream_t stream) {
     constexpr uint32_t kStep = THREADS / 32 * (32 / (kStripCols / CPL));
     p.x_rows = kXBytes / (4 * x_stride(MR)) / (D * kStep) * (D * kStep);
     const int smem = (int)(kTableAt + 0x10000 + kRedBytes - 1024);
-    auto kernel = in_out_strip_kernel<MR, CPL, THREADS, D, DQ>;
-    NF4_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), smem));
+    auto kernel = in_out_strip_kernel<MR, CPL, THREADS, D, DQ, true>;
+    ClusterRoom room;
+    NF4_TRY(cluster_room(reinterpret_cast<const void *>(kernel), THREADS, (uint32_t)smem, &room));
+    Runs r;
+    r.ctas = ctas;
+    r.units_per_strip = p.units_per_strip;
+    r.total = p.total_units;
+    p.parts = cluster_parts(r, room);
+    if (p.parts > 1) {
+        ctas = p.total_units / p.units_per_strip * p.parts;
+    } else {
+        kernel = in_out_strip_kernel<MR, CPL, THREADS, D, DQ, false>;
+        NF4_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), smem));
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = p.parts;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = p.parts > 1 ? 2 : 1;
     count_launch();
-    return launch_maybe_overlapped(kernel, dim3(ctas), dim3(THREADS), (size_t)smem, stream, true, p);
+    return check_cuda(cudaLaunchKernelEx(&cfg, kernel, p), "in_out_strip_kernel launch");
 }
 
 template <bool DQ>
