@@ -7,9 +7,10 @@
 // CTA takes 128 columns p, 64 ranks and a share of the rows; stages of 64 rows of X and of both halves of R (32 KB) come
 // by TMA, three in flight and two CTAs on an SM; one thread asks for them and one issues their MMAs.  The CTAs that share a
 // tile's rows form a cluster: their sums meet through distributed shared memory, each adds (in rank order) and writes its
-// part of the columns.  Bound by reading X once and R from the L2 for every 128 columns and, at few columns, by the chain
-// of a load, its stages and that exchange.  Warp MMAs behind transposing loads, whose pipe was half busy, took 40 us
-// for [2048, 14336] and 17 for [2048, 4096] at rank 64.
+// part of the columns.  Both gradients are one launch: the tiles of x with U, then those of grad_y with T.  Bound by reading X
+// once and R from the L2 for every 128 columns and, at few columns, by the chain of a load, its stages and that exchange.
+// Warp MMAs behind transposing loads, whose pipe was half busy, took 40 us for [2048, 14336] and 17 for [2048, 4096] at
+// rank 64; in a launch each these tiles take 21 and 12 us, together 22.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
@@ -27,13 +28,16 @@ constexpr uint32_t kSumPitch = 68;                              // floats
 static_assert(kCols * kSumPitch * 4 <= kStages * kStage, "the sums reuse the stages");
 
 struct Params {
-    __nv_bfloat16 *out;
-    uint32_t rows, P, rank, chunks, stages_per_share, p_major;
+    __nv_bfloat16 *out[2];        // of x (times U), of grad_y (times T)
+    uint32_t P[2], p_major[2];
+    uint32_t tiles0;              // tiles of the first
+    uint32_t rows, rank, chunks, stages_per_share;
     float scale;
 };
 
 __global__ void __launch_bounds__(kThreads, 2)
-gradient_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_r, const Params p, const FailureRef failure) {
+gradient_kernel(const __grid_constant__ CUtensorMap tmap_x0, const __grid_constant__ CUtensorMap tmap_r0, const __grid_constant__ CUtensorMap tmap_x1,
+                const __grid_constant__ CUtensorMap tmap_r1, const Params p, const FailureRef failure) {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ uint8_t smem_any[];
@@ -41,7 +45,11 @@ gradient_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
     __shared__ uint32_t s_tmem;
     uint8_t *const smem = smem_any + (1024u - (ptx::smem_addr(smem_any) & 1023u)) % 1024u;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-    const uint32_t shares = cluster.num_blocks(), share = cluster.block_rank(), p0 = blockIdx.x / shares * kCols, chunk = blockIdx.y;
+    const uint32_t shares = cluster.num_blocks(), share = cluster.block_rank(), tile = blockIdx.x / shares, chunk = blockIdx.y;
+    const uint32_t job = tile < p.tiles0 ? 0u : 1u, p0 = (tile - (job ? p.tiles0 : 0u)) * kCols;
+    const uint32_t P = job ? p.P[1] : p.P[0], p_major = job ? p.p_major[1] : p.p_major[0];
+    const CUtensorMap *const tmap_x = job ? &tmap_x1 : &tmap_x0, *const tmap_r = job ? &tmap_r1 : &tmap_r0;
+    __nv_bfloat16 *const out = job ? p.out[1] : p.out[0];
     const uint32_t st0 = share * p.stages_per_share;
     const uint32_t all = (p.rows + kRowsStage - 1) / kRowsStage;
     const uint32_t nst = st0 < all ? min(p.stages_per_share, all - st0) : 0u;
@@ -56,8 +64,8 @@ gradient_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
         ptx::mbar_init(acc_bar, 1);
         ptx::fence_mbar_init();
         ptx::fence_proxy_async();
-        ptx::prefetch_tmap(&tmap_x);
-        ptx::prefetch_tmap(&tmap_r);
+        ptx::prefetch_tmap(tmap_x);
+        ptx::prefetch_tmap(tmap_r);
     }
     if (warp == 1) {
         ptx::tmem_alloc(ptx::smem_addr(&s_tmem), 64);
@@ -80,10 +88,10 @@ gradient_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
                 break;
             }
             ptx::mbar_arrive_expect_tx(full, kStage);
-            ptx::tma_load_2d(dst, &tmap_x, (int32_t)p0, m, full);
-            ptx::tma_load_2d(dst + kBox, &tmap_x, (int32_t)p0 + 64, m, full);
-            ptx::tma_load_2d(dst + 2 * kBox, &tmap_r, (int32_t)(chunk * 64), m, full);
-            ptx::tma_load_2d(dst + 3 * kBox, &tmap_r, (int32_t)((p.chunks + chunk) * 64), m, full);
+            ptx::tma_load_2d(dst, tmap_x, (int32_t)p0, m, full);
+            ptx::tma_load_2d(dst + kBox, tmap_x, (int32_t)p0 + 64, m, full);
+            ptx::tma_load_2d(dst + 2 * kBox, tmap_r, (int32_t)(chunk * 64), m, full);
+            ptx::tma_load_2d(dst + 3 * kBox, tmap_r, (int32_t)((p.chunks + chunk) * 64), m, full);
         }
     } else if (warp == 1) {
         const uint32_t idesc = ptx::f16_idesc(1, 128, n16, true, true);
@@ -152,10 +160,10 @@ gradient_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
     }
     for (uint32_t i = tid; i < per * 64; i += kThreads) {
         // p fastest for [rank][P] outputs, j fastest for [P][rank]
-        const uint32_t q = q0 + (p.p_major ? i >> 6 : i & (per - 1)), j = p.p_major ? i & 63u : i >> per_log;
+        const uint32_t q = q0 + (p_major ? i >> 6 : i & (per - 1)), j = p_major ? i & 63u : i >> per_log;
         const uint32_t pp = p0 + q, jj = chunk * 64 + j;
-        if (pp < p.P && j < ranks)
-            p.out[p.p_major ? (size_t)pp * p.rank + jj : (size_t)jj * p.P + pp] = __float2bfloat16_rn(__fmul_rn(sum[q * kSumPitch + j], p.scale));
+        if (pp < P && j < ranks)
+            out[p_major ? (size_t)pp * p.rank + jj : (size_t)jj * P + pp] = __float2bfloat16_rn(__fmul_rn(sum[q * kSumPitch + j], p.scale));
     }
     if (shares > 1) cluster.sync();  // the sums have been read, before a CTA leaves
     else __syncthreads();
@@ -169,32 +177,43 @@ uint32_t chunks_of(uint32_t rank) { return (rank + 63) / 64; }
 uint64_t up256(uint64_t v) { return (v + 255) / 256 * 256; }
 uint64_t intermediate_bytes(uint64_t rows, uint32_t rank) { return up256(rows * 2 * 64 * chunks_of(rank) * 2); }
 uint64_t tiles_of(uint64_t P) { return (P + kCols - 1) / kCols; }
-int32_t gradient(const void *x, const void *r, void *out, uint64_t rows, uint64_t P, uint32_t rank, float scale, bool p_major,
-                 cudaStream_t s) {
+// ga (p-major as `ga_p_major`) of x [rows][d_in] and u, gb of gy [rows][d_out] and t
+int32_t gradients(const void *x, const void *u, void *ga, bool ga_p_major, uint64_t d_in, const void *gy, const void *t, void *gb, bool gb_p_major,
+                  uint64_t d_out, uint64_t rows, uint32_t rank, float scale, cudaStream_t s) {
     Params p{};
-    p.out = static_cast<__nv_bfloat16 *>(out);
+    p.out[0] = static_cast<__nv_bfloat16 *>(ga);
+    p.out[1] = static_cast<__nv_bfloat16 *>(gb);
+    p.P[0] = (uint32_t)d_in;
+    p.P[1] = (uint32_t)d_out;
+    p.p_major[0] = ga_p_major;
+    p.p_major[1] = gb_p_major;
     p.rows = (uint32_t)rows;
-    p.P = (uint32_t)P;
     p.rank = rank;
     p.chunks = chunks_of(rank);
+    p.scale = scale;
+    p.tiles0 = (uint32_t)tiles_of(d_in);
+    const uint64_t tiles = tiles_of(d_in) + tiles_of(d_out);
     // Shares of the rows: as many as the chip holds clusters for at once, where a share keeps four stages (256 rows)
     const void *kernel = reinterpret_cast<const void *>(gradient_kernel);
     ClusterRoom room;
     NF4_TRY(cluster_room(kernel, kThreads, kSmem, &room));
-    const uint32_t shares = cluster_ctas(tiles_of(P), rows, 4 * kRowsStage, room);
+    const uint32_t shares = cluster_ctas(tiles, rows, 4 * kRowsStage, room);
     const uint32_t all = (uint32_t)((rows + kRowsStage - 1) / kRowsStage);
     p.stages_per_share = (all + shares - 1) / shares;
-    p.p_major = p_major;
-    p.scale = scale;
-    if (tiles_of(P) * shares >= (1ull << 31)) return fail(NF4_ERR_UNSUPPORTED, "gradient: too many columns");
-    CUtensorMap map_x, map_r;
+    if (tiles * shares >= (1ull << 31)) return fail(NF4_ERR_UNSUPPORTED, "gradients: too many columns");
+    CUtensorMap map_x0, map_r0, map_x1, map_r1;
     const uint64_t ld_r = 2 * 64 * (uint64_t)p.chunks;
-    NF4_TRY(make_map(&map_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, x, rows, P, P * 2, kRowsStage, 64, CU_TENSOR_MAP_SWIZZLE_128B));
-    NF4_TRY(make_map(&map_r, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, r, rows, ld_r, ld_r * 2, kRowsStage, 64, CU_TENSOR_MAP_SWIZZLE_128B));
+    auto of = [&](CUtensorMap *map, const void *v, uint64_t cols) {
+        return make_map(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, v, rows, cols, cols * 2, kRowsStage, 64, CU_TENSOR_MAP_SWIZZLE_128B);
+    };
+    NF4_TRY(of(&map_x0, x, d_in));
+    NF4_TRY(of(&map_r0, u, ld_r));
+    NF4_TRY(of(&map_x1, gy, d_out));
+    NF4_TRY(of(&map_r1, t, ld_r));
     FailureRef failure;
     NF4_TRY(prefill_failure_ref(&failure));
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(tiles_of(P) * shares), p.chunks);
+    cfg.gridDim = dim3((unsigned)(tiles * shares), p.chunks);
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = kSmem;
     cfg.stream = s;
@@ -207,7 +226,7 @@ int32_t gradient(const void *x, const void *r, void *out, uint64_t rows, uint64_
     cfg.attrs = attr;
     cfg.numAttrs = shares > 1 ? 2 : 1;
     count_launch();
-    return check_cuda(cudaLaunchKernelEx(&cfg, gradient_kernel, map_x, map_r, p, failure), "gradient_kernel launch");
+    return check_cuda(cudaLaunchKernelEx(&cfg, gradient_kernel, map_x0, map_r0, map_x1, map_r1, p, failure), "gradient_kernel launch");
 }
 
 }  // namespace
@@ -249,8 +268,7 @@ int32_t adapter_grads(const void *x, const void *gy, const void *a, const void *
     q.k_major = in_out;
     q.r_out = t;
     NF4_TRY(activations_prepass(q, s));
-    NF4_TRY(gradient(x, u, ga, rows, d_in, rank, scale, in_out, s));
-    return gradient(gy, t, gb, rows, d_out, rank, scale, !in_out, s);
+    return gradients(x, u, ga, in_out, d_in, gy, t, gb, !in_out, d_out, rows, rank, scale, s);
 }
 
 }  // namespace nf4
