@@ -4,15 +4,19 @@
 // between them), the decode kernel multiplies the 2 m rows with f32 outputs, and one more kernel
 // adds the two halves, the bias and the adapter term s (x A^T) B^T, which is computed in f32 from
 // the f32 factors as the reference does.  At most eight rows per pass (sixteen for the kernel).
+// 9 x 9728 x 18240 at rank 32: 160 us with T by CTAs of many columns (38 of it) and a thread per output that walked its row of B
+// value by value (29), now 115; 4 x 4096 x 11008 at rank 16 28.7, now 16.7; 16 x 4096 x 4096 at rank 64 54.6, now 34.9.
 #include <cuda_bf16.h>
 
 #include "kernels.cuh"
+#include "ptx.cuh"
 
 namespace nf4 {
 namespace {
 
 __global__ void __launch_bounds__(256)
 split_rows_kernel(const float *__restrict__ x, __nv_bfloat16 *__restrict__ xs, uint32_t m, uint64_t K) {
+    ptx::pdl_wait();
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (uint64_t)m * K) return;
     const float v = x[i];
@@ -23,22 +27,46 @@ split_rows_kernel(const float *__restrict__ x, __nv_bfloat16 *__restrict__ xs, u
     xs[(uint64_t)m * K + i] = __float2bfloat16_rn(rest);
 }
 
-// y[r][n] = yy[r][n] + yy[m + r][n] (+ bias[n]) (+ scale * sum_j t[r][j] * B[n][j])
-__global__ void __launch_bounds__(256)
+// y[r][n] = yy[r][n] + yy[m + r][n] (+ bias[n]) (+ scale * sum_j t[r][j] * B[n][j]).  A thread has a column n of two
+// rows: its row of B is read four values at a time where they are whole (`wide`), T comes from shared memory.
+constexpr uint32_t kCombineThreads = 128, kPassRows = 8, kThreadRows = 2, kCombineCols = kCombineThreads / (kPassRows / kThreadRows), kMaxRankHeld = 256;
+__global__ void __launch_bounds__(kCombineThreads)
 combine_rows_kernel(const float *__restrict__ yy, const float *__restrict__ bias, const float *__restrict__ t,
                     const float *__restrict__ b, float *__restrict__ y, uint32_t m, uint64_t N, uint64_t ldy,
-                    uint32_t rank, float scale) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (uint64_t)m * N) return;
-    const uint64_t r = i / N, n = i % N;
-    float v = yy[i] + yy[(uint64_t)m * N + i];
-    if (rank) {
-        float acc = 0.0f;
-        for (uint32_t j = 0; j < rank; ++j) acc = fmaf(t[r * rank + j], b[n * rank + j], acc);
-        v += __fmul_rn(acc, scale);
+                    uint32_t rank, float scale, bool wide) {
+    __shared__ float s_t[kPassRows * kMaxRankHeld];
+    const bool held = rank <= kMaxRankHeld;
+    for (uint32_t i = threadIdx.x; held && i < m * rank; i += kCombineThreads) s_t[i] = t[i];
+    __syncthreads();
+    const float *tt = held ? s_t : t;
+    const uint64_t n = (uint64_t)blockIdx.x * kCombineCols + threadIdx.x % kCombineCols;
+    const uint32_t r0 = threadIdx.x / kCombineCols * kThreadRows;
+    if (n >= N || r0 >= m) return;
+    float acc[kThreadRows] = {};
+    uint32_t j = 0;
+    #pragma unroll 4
+    for (; wide && j + 4 <= rank; j += 4) {
+        const float4 v = __ldg(reinterpret_cast<const float4 *>(b + n * rank + j));
+        #pragma unroll
+        for (uint32_t r = 0; r < kThreadRows; ++r) {
+            const float *row = tt + min(r0 + r, m - 1) * rank + j;
+            acc[r] = fmaf(row[3], v.w, fmaf(row[2], v.z, fmaf(row[1], v.y, fmaf(row[0], v.x, acc[r]))));
+        }
     }
-    if (bias) v += bias[n];
-    y[r * ldy + n] = v;
+    for (; j < rank; ++j) {
+        const float v = __ldg(b + n * rank + j);
+        #pragma unroll
+        for (uint32_t r = 0; r < kThreadRows; ++r) acc[r] = fmaf(tt[min(r0 + r, m - 1) * rank + j], v, acc[r]);
+    }
+    const float add = bias ? __ldg(bias + n) : 0.0f;
+    #pragma unroll
+    for (uint32_t i = 0; i < kThreadRows; ++i) {
+        const uint32_t r = r0 + i;
+        if (r >= m) break;
+        float v = yy[r * N + n] + yy[(uint64_t)(m + r) * N + n];
+        if (rank) v += __fmul_rn(acc[i], scale);
+        y[r * ldy + n] = bias ? v + add : v;
+    }
 }
 
 inline uint64_t up256(uint64_t v) { return (v + 255) / 256 * 256; }
@@ -102,21 +130,22 @@ int32_t f32_rows_forward(const nf4_linear_args &a, cudaStream_t stream) {
     const float *x = static_cast<const float *>(a.x);
     float *y = static_cast<float *>(a.y);
     if (rank)  // T = x A^T for all the rows, in f32
-        NF4_TRY(lora_intermediate(a.x, a.lora_a, t, a.rows, a.d_in, rank, NF4_LAYOUT_OUT_IN, NF4_DTYPE_F32, stream));
-    for (uint64_t r0 = 0; r0 < a.rows; r0 += 8) {
-        const uint32_t m = (uint32_t)(a.rows - r0 < 8 ? a.rows - r0 : 8);
-        split_rows_kernel<<<(unsigned)((m * a.d_in + 255) / 256), 256, 0, stream>>>(x + r0 * a.d_in, xs, m, a.d_in);
+        NF4_TRY(small_lora_t(a.x, a.lora_a, t, a.rows, a.d_in, rank, true, true, stream));
+    for (uint64_t r0 = 0; r0 < a.rows; r0 += kPassRows) {
+        const uint32_t m = (uint32_t)(a.rows - r0 < kPassRows ? a.rows - r0 : kPassRows);
         count_launch();
-        NF4_CUDA_TRY(cudaGetLastError());
+        NF4_TRY(launch_maybe_overlapped(split_rows_kernel, dim3((unsigned)((m * a.d_in + 255) / 256)), dim3(256), 0, stream, true, x + r0 * a.d_in, xs,
+                                        m, a.d_in));
         nf4_linear_args h = halves_args(a, m, xs, yy);
         h.workspace_bytes = sc.off_xs;
         if (decode_supported(h)) NF4_TRY(decode_forward(h, stream));
         else NF4_TRY(decode2_forward(h, stream));
-        combine_rows_kernel<<<(unsigned)((m * a.d_out + 255) / 256), 256, 0, stream>>>(
-            yy, a.bias, t + r0 * rank, static_cast<const float *>(a.lora_b), y + r0 * ldy, m, a.d_out, ldy, rank,
-            a.lora_scale);
+        // (an ordinary launch: as the decode kernel's programmatic dependent this one took 16 x 4096 x 4096 from 35 to 70 us)
+        const bool wide = rank % 4 == 0 && aligned16(a.lora_b);
         count_launch();
-        NF4_CUDA_TRY(cudaGetLastError());
+        NF4_TRY(launch_maybe_overlapped(combine_rows_kernel, dim3((unsigned)((a.d_out + kCombineCols - 1) / kCombineCols)), dim3(kCombineThreads), 0,
+                                        stream, false, static_cast<const float *>(yy), a.bias, static_cast<const float *>(t + r0 * rank),
+                                        static_cast<const float *>(a.lora_b), y + r0 * ldy, m, a.d_out, ldy, rank, a.lora_scale, wide));
     }
     return NF4_OK;
 }

@@ -525,6 +525,16 @@ int32_t launch(StripParams &p, uint32_t ctas, bool wide, cudaStream_t stream) {
 
 }  // namespace
 
+int32_t small_lora_t(const void *x, const void *a, float *t, uint64_t rows, uint64_t K, uint32_t rank, bool f32, bool out_in, cudaStream_t stream) {
+    const dim3 grid((unsigned)(rows * rank));
+    count_launch();
+    if (f32)
+        return launch_maybe_overlapped(strip_lora_t_kernel<float>, grid, dim3(256), 0, stream, true, static_cast<const float *>(x),
+                                       static_cast<const float *>(a), t, (uint32_t)K, rank, out_in);
+    return launch_maybe_overlapped(strip_lora_t_kernel<__nv_bfloat16>, grid, dim3(256), 0, stream, true, static_cast<const __nv_bfloat16 *>(x),
+                                   static_cast<const __nv_bfloat16 *>(a), t, (uint32_t)K, rank, out_in);
+}
+
 // flag words | T | two partial results per CTA (sized for sixteen rows where a call has more than one pass)
 uint64_t strips_workspace_bytes(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t lora_rank) {
     Runs r;
@@ -546,17 +556,7 @@ int32_t strips_forward(const nf4_linear_args &a, cudaStream_t stream) {
     uint8_t *ws = static_cast<uint8_t *>(a.workspace);
     float *t = reinterpret_cast<float *>(ws + 256);
     const bool f32 = a.io_dtype == NF4_DTYPE_F32;
-    if (rank) {
-        const dim3 grid((unsigned)(a.rows * rank));
-        count_launch();
-        if (f32)
-            NF4_TRY(launch_maybe_overlapped(strip_lora_t_kernel<float>, grid, dim3(256), 0, stream, true, static_cast<const float *>(a.x),
-                                            static_cast<const float *>(a.lora_a), t, (uint32_t)a.d_in, rank, false));
-        else
-            NF4_TRY(launch_maybe_overlapped(strip_lora_t_kernel<__nv_bfloat16>, grid, dim3(256), 0, stream, true,
-                                            static_cast<const __nv_bfloat16 *>(a.x), static_cast<const __nv_bfloat16 *>(a.lora_a), t,
-                                            (uint32_t)a.d_in, rank, false));
-    }
+    if (rank) NF4_TRY(small_lora_t(a.x, a.lora_a, t, a.rows, a.d_in, rank, f32, false, stream));
     const uint64_t ldy = a.ldy ? a.ldy : a.d_out;
     const size_t xb = f32 ? 4 : 2, yb = f32 || a.y_f32 ? 4 : 2;
     for (uint64_t m0 = 0; m0 < a.rows; m0 += 16) {  // sixteen activation rows per launch

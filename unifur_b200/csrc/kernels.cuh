@@ -147,6 +147,8 @@ int32_t generic_forward(const nf4_linear_args &a, cudaStream_t stream);
 bool strips_supported(const nf4_linear_args &a);
 uint64_t strips_workspace_bytes(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t lora_rank);
 int32_t strips_forward(const nf4_linear_args &a, cudaStream_t stream);
+// T = x A in f32, [rows][rank], a CTA to a value: for few rows.  a: [d_in][r], or [r][d_in] (out_in)
+int32_t small_lora_t(const void *x, const void *a, float *t, uint64_t rows, uint64_t K, uint32_t rank, bool f32, bool out_in, cudaStream_t stream);
 
 // f32_rows.cu: f32 tensors, NF4_LAYOUT_OUT_IN, rows <= 16: rows split into bf16 halves for the decode kernels
 bool f32_rows_supported(const nf4_linear_args &a);
