@@ -44,19 +44,22 @@ namespace {
 int32_t set_once(const void *kernel, cudaFuncAttribute what, int value) {
     struct Done {
         const void *kernel;
-        int device;
         cudaFuncAttribute what;
     };
+    constexpr int kDevices = 64, kMost = 256;
     static std::mutex mu;
-    static Done done[256];
-    static int n_done = 0;
+    static Done done_on[kDevices][kMost];
+    static int n_done_on[kDevices] = {};
     int dev = 0;
     NF4_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= kDevices) return fail(NF4_ERR_UNSUPPORTED, "device ordinal %d out of range", dev);
     std::lock_guard<std::mutex> lock(mu);
+    Done *const done = done_on[dev];
+    int &n_done = n_done_on[dev];
     for (int i = 0; i < n_done; ++i)
-        if (done[i].kernel == kernel && done[i].device == dev && done[i].what == what) return NF4_OK;
+        if (done[i].kernel == kernel && done[i].what == what) return NF4_OK;
     NF4_CUDA_TRY(cudaFuncSetAttribute(kernel, what, value));
-    if (n_done < 256) done[n_done++] = Done{kernel, dev, what};
+    if (n_done < kMost) done[n_done++] = Done{kernel, what};
     return NF4_OK;
 }
 }  // namespace
@@ -68,17 +71,20 @@ int32_t ensure_dynamic_smem(const void *kernel, int bytes) {
 int32_t cluster_room(const void *kernel, uint32_t threads, uint32_t smem, ClusterRoom *room) {
     struct Asked {
         const void *kernel;
-        int device;
         ClusterRoom room;
     };
+    constexpr int kDevices = 64, kKernels = 64;  // (some forty kernels ask)
     static std::mutex mu;
-    static Asked asked[64];
-    static int n_asked = 0;
+    static Asked asked_of[kDevices][kKernels];
+    static int n_asked_of[kDevices] = {};
     int dev = 0;
     NF4_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= kDevices) return fail(NF4_ERR_UNSUPPORTED, "device ordinal %d out of range", dev);
     std::lock_guard<std::mutex> lock(mu);
+    Asked *const asked = asked_of[dev];
+    int &n_asked = n_asked_of[dev];
     for (int i = 0; i < n_asked; ++i)
-        if (asked[i].kernel == kernel && asked[i].device == dev) {
+        if (asked[i].kernel == kernel) {
             *room = asked[i].room;
             return NF4_OK;
         }
@@ -104,7 +110,7 @@ int32_t cluster_room(const void *kernel, uint32_t threads, uint32_t smem, Cluste
         room->any[i] = n > 0 ? (uint32_t)n : 0u;
     }
     for (uint32_t i = 0; i < kClusterSizes; ++i) room->of[i] = room->any[1u << i];
-    if (n_asked < 64) asked[n_asked++] = Asked{kernel, dev, *room};
+    if (n_asked < kKernels) asked[n_asked++] = Asked{kernel, *room};
     return NF4_OK;
 }
 

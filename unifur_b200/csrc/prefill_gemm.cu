@@ -43,7 +43,7 @@
 // produces the LoRA intermediate.
 //
 // The other orientation (W [K][N] with the 64-blocks along N, the reference's own; f32 or bf16
-// activations) comes through the same GEMM at more than 16 rows: three small kernels first write the
+// activations) comes through the same GEMM at more than 16 rows: small kernels beside the pre-pass write the
 // transposed nibbles, the scales as f16 [N / 64][K] and the adapter factors in this kernel's
 // orientation into the workspace (the nibbles exactly; the scales with the rounding the dequantisers
 // apply anyway).  A weight row's scale then changes with every k: a lane loads the pair of scales of
