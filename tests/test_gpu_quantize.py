@@ -269,7 +269,8 @@ def test_embedding_gather_equals_dequantize_then_gather(oracle, n_embedding, d_m
 @pytest.mark.parametrize("rows,cols,bf16", [(64, 64, False), (128, 200, True), (256, 1024, True),
                                             (192, 36, False), (100, 72, True), (65, 7, False),
                                             (64, 8, True), (128, 68, True),      # rows TMA takes, and rows it does not
-                                            (2560, 4608, True), (2560, 2304, False)])  # warps that take a second tile
+                                            (2560, 4608, True), (2560, 2304, False),  # warps that take a second tile
+                                            (1984, 68, False), (1600, 100, False)])  # a last tile of seven segments; more missing: the other kernel
 def test_load_path_quantize_of_the_transpose(oracle, rows, cols, bf16):
     # src/qwennet.rs:1709-1711: transpose2d([out, in]) then PackedNf4Tensor::quantize (+ double
     # quantization).  The fused kernel (rows % 64 == 0) and the workspace route must both give

@@ -817,9 +817,10 @@ int32_t quantize_transposed(const void *src, bool src_bf16, uint64_t rows, uint6
             return fail(NF4_ERR_UNSUPPORTED, "nf4_quantize_transposed: matrix too large");
         const uint32_t *w = static_cast<const uint32_t *>(src);
         count_launch();
-        // bf16 wherever TMA takes it; f32, bound by its bytes, where every tile has its eight segments ([7936, 7424] 57.4 -> 55.1 us,
-        // but [4352, 2688] 18.5 -> 19.2)
-        if (words % 4 == 0 && (src_bf16 || rows / kBlock % kTmaWarps == 0)) {
+        // bf16 wherever TMA takes it; f32, bound by its bytes, where no more than a twenty-fifth of the tiles' eight segments
+        // are missing ([7936, 7424], 124 segments: 57.4 -> 55.1 us; but [4352, 2688], 68: 18.5 -> 19.2, [4416, 2688], 69: 18.3 -> 19.5)
+        const uint64_t whole = (rows / kBlock + kTmaWarps - 1) / kTmaWarps * kTmaWarps;
+        if (words % 4 == 0 && (src_bf16 || whole * 24 <= rows / kBlock * 25)) {
             auto kernel = src_bf16 ? quantize_transposed_tma_kernel<true> : quantize_transposed_tma_kernel<false>;
             const uint64_t segments = rows / kBlock, octets = (segments + kTmaWarps - 1) / kTmaWarps, tiles = octets * ((words + 31) / 32);
             CUtensorMap map;
