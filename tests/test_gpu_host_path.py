@@ -175,3 +175,48 @@ def test_page_locked_calls_give_the_same_bits(rows, k, n, r):
         assert not wrong
     finally:
         L.nf4_weight_free(h)
+
+
+def test_a_host_call_behind_the_kernel_that_writes_its_x():
+    # Stream order holds on the stream the host calls work on: a forward there writes page-locked memory, and the host
+    # call that takes it as x follows without a synchronise.  Forwards of few CTAs ahead, so that the host call's could start
+    # beside them; the one right ahead writes other values every time.
+    import ctypes
+
+    from unifur_b200.quantize import PackedNf4Tensor
+
+    L, g, bf16 = _lib.load(), torch.Generator(device="cuda").manual_seed(3), torch.bfloat16
+    rows, k0, k, n = 16, 4096, 256, 512
+    first, second = (PackedNf4Tensor.quantize(torch.randn(a * b, device="cuda", generator=g) * 0.02) for a, b in ((k0, k), (k, n)))
+    codes, absmax = second.codes.cpu(), second.absmax.cpu()
+    h = ctypes.c_void_p()
+    _lib.check(L.nf4_weight_from_packed_host(codes.data_ptr(), absmax.data_ptr(), None, 0.0, k, n, _lib.LAYOUT_OUT_IN, ctypes.byref(h)))
+    xs = [torch.randn(rows, k0, device="cuda", generator=g).to(bf16) for _ in range(2)]
+    mid, y = torch.empty(rows, k, dtype=bf16).pin_memory(), torch.empty(rows, n, dtype=bf16).pin_memory()
+    per_thread = ctypes.c_void_p(2)  # cudaStreamPerThread
+    scratch = torch.zeros(L.nf4_linear_workspace_bytes(rows, k0, k, 0), dtype=torch.uint8, device="cuda")
+
+    def ahead(x):
+        a = _lib.LinearArgs(struct_bytes=ctypes.sizeof(_lib.LinearArgs), layout=_lib.LAYOUT_OUT_IN, io_dtype=_lib.DTYPE_BF16, rows=rows,
+                            d_in=k0, d_out=k, x=x.data_ptr(), packed=first.codes.data_ptr(), absmax=first.absmax.data_ptr(),
+                            y=mid.data_ptr(), ldy=k, workspace=scratch.data_ptr(), workspace_bytes=scratch.numel())
+        _lib.check(L.nf4_linear_forward_dev(ctypes.byref(a), per_thread))
+
+    def host():
+        _lib.check(L.nf4_weight_linear_forward_host(h, mid.data_ptr(), rows, _lib.DTYPE_BF16, None, None, None, 0, 0.0, y.data_ptr()))
+        return y.clone()
+
+    torch.cuda.synchronize()
+    try:
+        want = []
+        for x in xs:
+            ahead(x)
+            torch.cuda.synchronize()
+            want.append(host())
+        assert not torch.equal(*want)
+        for i in range(60):
+            for j in range(7):
+                ahead(xs[(i + j) % 2])  # (the last one's x: i % 2)
+            assert torch.equal(host(), want[i % 2])
+    finally:
+        L.nf4_weight_free(h)

@@ -248,12 +248,16 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
         if (tid == 0) NF4_REPORT_FAILURE(g_decode_error, g_decode_error_host, 4);
         return;
     }
-    // The CTAs that bring x from the host are those that start first, and wait for nobody: the ones that wait are sure of
-    // them.  Their loads cross the bus while the table is built.
+    // The CTAs that bring x from the host are those that start first, and wait for no other CTA: the ones that wait are sure
+    // of them.  x may come from the kernel ahead in the stream (a forward that wrote page-locked memory), so they wait for
+    // that first; behind an empty stream it costs nothing, and their loads cross the bus while the table is built.
     const bool fetcher = PEERS && p.x_host && bid < p.wait_expected;
     const uint32_t x_at = (bid * kThreads + tid) * 16u;
     uint4 x_first = make_uint4(0, 0, 0, 0);
-    if (fetcher && x_at < p.x_bytes) x_first = __ldcv(reinterpret_cast<const uint4 *>(p.x_host + x_at));
+    if (fetcher) {
+        ptx::pdl_wait();
+        if (x_at < p.x_bytes) x_first = __ldcv(reinterpret_cast<const uint4 *>(p.x_host + x_at));
+    }
     if (lane == 0) {  // the descriptors are on their way while the table is built
         ptx::prefetch_tmap(tm_codes);
         if (TMA_SCALES) ptx::prefetch_tmap(tm_scales);
