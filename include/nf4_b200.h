@@ -468,8 +468,11 @@ NF4_API int32_t nf4_weight_attach_lora_host(nf4_weight *w, const void *lora_a, c
  * `io_dtype`.  `lora_a`/`lora_b` (host, may be NULL) use the layout's orientation; when they are NULL and
  * an adapter of the same element type is attached to the weight, that adapter is used.  Any host
  * memory serves; with up to 16 rows a page-locked y that the device can address (cudaHostAlloc, or
- * cudaHostRegister with the mapped flag) is written by the kernel itself, which saves the copy
- * back (a quarter of the call's latency at these sizes). */
+ * cudaHostRegister with the mapped flag) is written by the kernel itself, which saves the copy back.
+ * Where x is page-locked too (16-byte aligned, bf16, NF4_LAYOUT_OUT_IN, d_in a multiple of 256 up to
+ * 32768, an adapter of rank 0, 8, 16, 32 or 64) the kernel also fetches x, behind the work ahead of it on
+ * cudaStreamPerThread, and the calling thread polls for the results instead of synchronising with the stream --
+ * unless the device's flags say cudaDeviceScheduleBlockingSync or cudaDeviceScheduleYield: then it waits that way. */
 NF4_API int32_t nf4_weight_linear_forward_host(const nf4_weight *w, const void *x, uint64_t rows,
                                        int32_t io_dtype, const float *bias, const void *lora_a,
                                        const void *lora_b, uint32_t lora_rank, float lora_scale,

@@ -220,3 +220,39 @@ def test_a_host_call_behind_the_kernel_that_writes_its_x():
             assert torch.equal(host(), want[i % 2])
     finally:
         L.nf4_weight_free(h)
+
+
+BLOCKING_CHILD = """
+import ctypes, sys, time
+drv = ctypes.CDLL("libcuda.so.1")
+assert drv.cuInit(0) == 0 and drv.cuDevicePrimaryCtxSetFlags_v2(0, int(sys.argv[1])) == 0
+import torch
+from unifur_b200 import _lib
+L, rows, k, n = _lib.load(), 4, 512, 256
+codes, absmax = torch.zeros(k * n // 2, dtype=torch.uint8), torch.ones(k * n // 64)
+h = ctypes.c_void_p()
+torch.cuda.init()
+_lib.check(L.nf4_weight_from_packed_host(codes.data_ptr(), absmax.data_ptr(), None, 0.0, k, n, _lib.LAYOUT_OUT_IN, ctypes.byref(h)))
+x, y = torch.ones(rows, k, dtype=torch.bfloat16).pin_memory(), torch.empty(rows, n, dtype=torch.bfloat16).pin_memory()
+call = lambda: _lib.check(L.nf4_weight_linear_forward_host(h, x.data_ptr(), rows, _lib.DTYPE_BF16, None, None, None, 0, 0.0, y.data_ptr()))
+call()
+with torch.cuda.stream(torch.cuda.ExternalStream(2)):  # the calls' stream has a tenth of a second to do first
+    torch.cuda._sleep(200_000_000)
+wall, cpu = time.perf_counter(), time.thread_time()
+call()
+print(time.perf_counter() - wall, time.thread_time() - cpu, bool((y == -k).all()))
+"""
+
+
+@pytest.mark.parametrize("schedule", [2, 4])  # CU_CTX_SCHED_YIELD, CU_CTX_SCHED_BLOCKING_SYNC
+def test_a_waiting_host_call_waits_as_the_process_chose(schedule):
+    # page-locked buffers, so that the call's kernel has a word for the host: it is polled only where nothing was chosen
+    import subprocess
+    import sys
+
+    out = subprocess.run([sys.executable, "-c", BLOCKING_CHILD, str(schedule)], capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0, out.stderr
+    wall, cpu, right = out.stdout.split()
+    assert right == "True" and float(wall) > 0.05
+    if schedule == 4:
+        assert float(cpu) < 0.2 * float(wall)  # (a poll takes all of it)

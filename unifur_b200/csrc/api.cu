@@ -200,8 +200,14 @@ struct DoneWord {
         host = h;
         return NF4_OK;
     }
-    // Until the word has the value, or the stream has an error or nothing left to do.
+    // Until the word has the value, or the stream has an error or nothing left to do.  A process that has chosen to sleep or
+    // to yield while it waits for the device (cudaSetDeviceFlags) does so here too, for the grid's end instead of the word.
     int32_t wait(cudaStream_t stream) const {
+        unsigned flags = 0;
+        NF4_CUDA_TRY(cudaGetDeviceFlags(&flags));
+        const unsigned schedule = flags & cudaDeviceScheduleMask;
+        if (schedule == cudaDeviceScheduleBlockingSync || schedule == cudaDeviceScheduleYield)
+            return check_cuda(cudaStreamSynchronize(stream), "waiting for the kernel");
         for (uint32_t i = 1; *host != value; ++i) {
 #if defined(__x86_64__)
             __builtin_ia32_pause();
@@ -1157,7 +1163,7 @@ int32_t nf4_weight_linear_forward_host(const nf4_weight *w, const void *x, uint6
     uint8_t *d_ws = cv.take<uint8_t>(ws);
     // x and y of a decode-sized call that are page-locked memory the device can address (cudaHostAlloc, cudaHostRegister
     // with the mapped flag) need no copy operation: the kernel stores its results to y itself, and where it also
-    // fetches x, the host waits for its word instead of the stream.  (Not for the tensor-core GEMM of more rows, which stores
+    // fetches x, the host polls a word of it instead of waiting for the stream (DoneWord::wait).  (Not for the tensor-core GEMM of more rows, which stores
     // through a tensor map, and where the copies do not matter.)
     void *const y_mapped = rows <= 16 ? device_view(y) : nullptr;
     const bool fetches = w->layout == NF4_LAYOUT_OUT_IN && io_dtype == NF4_DTYPE_BF16 && w->d_in % 256 == 0;  // the decode kernel
