@@ -71,6 +71,36 @@ def test_rows_far_from_the_first_values(first, std):
     assert float(per_row.max()) < 4e-3
 
 
+@pytest.mark.parametrize("first", [1000.0, 1e-30, 0.0, 0.5])
+@pytest.mark.parametrize("big", [1.0, 3e4, 1e5, 2.0 ** -9])
+def test_a_row_does_not_depend_on_the_first_row(first, big):
+    # Rows of small values around one large one that meets a zero weight (and a zero of the factor): what the outputs are
+    # made of lies 2^-16 below the row's maximum, where a copy with a factor that suits other rows keeps few of its bits.
+    # The bound of the other forwards, and the same bits whatever stands in row 0.
+    from unifur_b200.quantize import PackedNf4Tensor
+    from unifur_b200.qwennet import Nf4Linear, QloraLinear
+
+    M, K, N, r = 1030, 4096, 64, 16
+    gen = torch.Generator(device=DEV).manual_seed(11)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=gen)  # noqa: E731
+    W, A, B = rnd(N, K) * 0.02, (rnd(r, K) * 0.1).bfloat16(), (rnd(N, r) * 0.1).bfloat16()
+    W[:, 300] = 0
+    A[:, 300] = 0
+    base = Nf4Linear(PackedNf4Tensor.quantize(W.flatten()), K, N, None, _lib.LAYOUT_OUT_IN)
+    q = QloraLinear(base, A, B, 1.5)
+    w = base.dequantized_weight().double().t()
+    assert not w[300].any()
+    x = (rnd(M, K) * big * 2.0 ** -16).bfloat16()
+    x[:, 300] = big
+    x[0] = first
+    y = q.forward(x)
+    ref = x.double() @ w + 1.5 * (x.double() @ A.double().t()) @ B.double().t()
+    per_row = (y[1:].double() - ref[1:]).norm(dim=1) / ref[1:].norm(dim=1)
+    assert float(per_row.max()) < 4e-3
+    x[0] = 1.0
+    assert torch.equal(q.forward(x)[1:], y[1:])
+
+
 @pytest.mark.parametrize("M,K,N,r,layout", [
     (1, 64, 128, 8, 0), (5, 200, 136, 5, 1), (16, 1024, 512, 16, 0),   # decode sizes: both intermediates by the product-only mode
     (63, 256, 384, 16, 1), (513, 640, 200, 80, 0), (2049, 576, 1344, 64, 1),   # shares of the rows, ragged pieces of columns

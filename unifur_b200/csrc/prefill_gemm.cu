@@ -38,8 +38,9 @@
 // activation rows its N (256 accumulator columns).  Both operands are f16 with f32 accumulation:
 // rounding the dequantised weight to bf16 instead would cost ~1.6e-3 relative error, above the
 // 1e-3 parity bar, while f16 costs ~3e-4.  The bf16 activations are converted to f16 by a
-// pre-pass (exact for every value inside f16's range; a row whose largest magnitude exceeds 32768
-// or lies below 2^-8 is divided by a power of two that the epilogue multiplies back), which also
+// pre-pass, divided by a power of two that the epilogue multiplies back: exact where f16 holds the value's
+// eight bits, which is down to 2^-31 of the row's largest magnitude where the row has its own power of two,
+// and down to 2^-17 where it has none (the pre-pass says which rows that is).  It also
 // produces the LoRA intermediate.
 //
 // The other orientation (W [K][N] with the 64-blocks along N, the reference's own; f32 or bf16

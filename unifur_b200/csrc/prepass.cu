@@ -75,6 +75,13 @@ __device__ __forceinline__ uint32_t bf16x2_larger_bits(uint32_t mx) {
     return max(a, b);
 }
 
+// Running minima of the nonzero |bf16|, a pair at a time: 2 |v| - 2 as 16 unsigned bits, which puts a zero on top of all.
+// (The sign below and the borrow of a zero below reach the upper half: it may come out one lower.  The smallest subnormals
+// may wrap; no power of two used here brings them into f16's range.)
+__device__ __forceinline__ uint32_t bf16x2_absmin(uint32_t w, uint32_t mn) { return __vminu2(mn, w * 2u - 0x00020002u); }
+// The smaller half as an f32 pattern at or just below the least nonzero value.
+__device__ __forceinline__ uint32_t bf16x2_smaller_bits(uint32_t mn) { return (min(mn & 0xffffu, mn >> 16) >> 1) << 16; }
+
 __device__ __forceinline__ uint4 bf16x8_to_f16x8(const uint4 &v) {
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
     uint32_t o[4];
@@ -448,9 +455,9 @@ prepass_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     static_assert(kRows * kPartPitch * 4 <= tc_ring(kRows), "the sums reuse the stages");
     static_assert((kStages - 1) * kXStage + 128 * 128 <= tc_ring(kRows), "an MMA reads 128 rows from the last stage's place");
     extern __shared__ uint8_t smem_any[];
-    __shared__ uint32_t s_max[kMaxCluster][kRows];   // the CTAs' row maxima (f32 patterns)
+    __shared__ uint32_t s_seen[kMaxCluster][kRows];  // the CTAs' row maxima (bf16 patterns) above their nonzero minima
     __shared__ float s_inv[kRows];
-    __shared__ uint32_t s_own[kRows];
+    __shared__ uint32_t s_most[kRows], s_least[kRows];  // this CTA's, as f32 patterns
     __shared__ float s_shift;
     __shared__ int s_exp;
     __shared__ __align__(8) uint64_t s_bars[2 * kStages + 1];
@@ -485,7 +492,10 @@ prepass_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         if (p.wait == 0) ptx::pdl_wait();
         for (uint32_t st = 0; st < min(stages, kStages); ++st) request(st);
     }
-    if (kCopy && tid < kRows) s_own[tid] = 0;
+    if (kCopy && tid < kRows) {
+        s_most[tid] = 0;
+        s_least[tid] = 0x7fff0000u;
+    }
     if (warp == 9) {
         ptx::tmem_alloc(ptx::smem_addr(&s_tmem), 64);
         ptx::tmem_relinquish();
@@ -504,15 +514,16 @@ prepass_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         if (lane == 0) s_exp = e;
     }
     if (kCopy && warp == 10) {
-        // x comes over times a power of two that brings the largest of its first 256 values to [2, 4), so that the rows
-        // of a tensor of small values (gradients of 1e-3) do not all need their own factor and a second writing
+        // x comes over times a power of two that brings the largest of its first 256 values to [512, 1024): rows up to 32
+        // times as large stay below 32768, and what is not exact in f16 then lies 2^-26 below those values, so that hardly
+        // a row of ordinary values or of gradients needs to be written a second time (see below).
         uint32_t w = 0;
         if (lane * 8 < p.K) {
             const uint4 v = __ldg(static_cast<const uint4 *>(p.x) + lane);
             w = bf16x2_absmax(v.x, bf16x2_absmax(v.y, bf16x2_absmax(v.z, bf16x2_absmax(v.w, 0))));
         }
-        const uint32_t m = __reduce_max_sync(0xffffffffu, bf16x2_larger_bits(w)), e = m >> 23;  // 128: [2, 4)
-        if (lane == 0) s_shift = e > 27 && e < 228 ? __uint_as_float((255 - e) << 23) : 1.0f;
+        const uint32_t m = __reduce_max_sync(0xffffffffu, bf16x2_larger_bits(w)), e = m >> 23;  // 136: [512, 1024)
+        if (lane == 0) s_shift = e > 35 && e < 228 ? __uint_as_float((263 - e) << 23) : 1.0f;
     }
     if (kCopy && (warp == 10 || warp < 8)) asm volatile("bar.sync 1, 288;" ::: "memory");
 
@@ -549,7 +560,9 @@ prepass_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         // Every warp has stages of its own: a stage is read, converted and written in one go of many loads, and the next
         // ones are other warps' (eight warps to a stage waited for each link of its chain in turn: 30 us without the stores).
         const uint32_t piece = lane & 7u, r0 = warp % kPerStage * kWarpRows + (lane >> 3);
-        uint32_t mx[kQuads] = {};
+        uint32_t mx[kQuads] = {}, mn[kQuads];
+        #pragma unroll
+        for (uint32_t q = 0; q < kQuads; ++q) mn[q] = ~0u;
         const float shift = s_shift;
         for (uint32_t st = warp / kPerStage; st < stages; st += kGroups) {
             const uint32_t s = st % kStages;
@@ -572,7 +585,10 @@ prepass_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                 for (uint32_t q = 0; q < kBatch; ++q, out += (size_t)4 * p.K) {
                     const uint32_t w[4] = {v[q].x, v[q].y, v[q].z, v[q].w};
                     #pragma unroll
-                    for (int i = 0; i < 4; ++i) mx[q0 + q] = bf16x2_absmax(w[i], mx[q0 + q]);
+                    for (int i = 0; i < 4; ++i) {
+                        mx[q0 + q] = bf16x2_absmax(w[i], mx[q0 + q]);
+                        mn[q0 + q] = bf16x2_absmin(w[i], mn[q0 + q]);
+                    }
                     if ((q0 + q) * 4 < rows) *reinterpret_cast<uint4 *>(out) = bf16x8_to_f16x8(v[q], shift);
                 }
             }
@@ -581,10 +597,16 @@ prepass_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         }
         #pragma unroll
         for (uint32_t q = 0; q < kQuads; ++q) {  // (eight lanes hold a row's)
-            uint32_t m = bf16x2_larger_bits(mx[q]);
+            uint32_t m = bf16x2_larger_bits(mx[q]), n = bf16x2_smaller_bits(mn[q]);
             #pragma unroll
-            for (int d = 1; d < 8; d *= 2) m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
-            if (piece == 0) atomicMax(s_own + r0 + q * 4, m);
+            for (int d = 1; d < 8; d *= 2) {
+                m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
+                n = min(n, __shfl_xor_sync(0xffffffffu, n, d));
+            }
+            if (piece == 0) {
+                atomicMax(s_most + r0 + q * 4, m);
+                atomicMin(s_least + r0 + q * 4, n);
+            }
         }
         if (!ok && lane == 0) NF4_REPORT_FAILURE(*failure.flag, *failure.host, 10);
     }
@@ -617,19 +639,26 @@ prepass_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     }
     cluster.barrier_wait();
     if (kCopy && warp >= 8)
-        for (uint32_t i = tid - 256; i < kRows * cn; i += 128) cluster.map_shared_rank(&s_max[0][0], i / kRows)[rank_in * kRows + i % kRows] = s_own[i % kRows];
+        for (uint32_t i = tid - 256; i < kRows * cn; i += 128)
+            cluster.map_shared_rank(&s_seen[0][0], i / kRows)[rank_in * kRows + i % kRows] = s_most[i % kRows] | s_least[i % kRows] >> 16;
     if (warp >= 8) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     else asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     const int w_exp = s_exp;
     if (kCopy) {
         if (tid < kRows) {
-            uint32_t m = 0;
-            for (uint32_t c = 0; c < cn; ++c) m = max(m, s_max[c][tid]);
-            // the copy stays where its largest value is in f16's comfortable range (see row_factor), or is infinite
-            const float mx = __uint_as_float(m), copied = mx * s_shift;
-            const bool own = (copied > 32768.0f || copied < 0.00390625f) && mx < __int_as_float(0x7f800000) && mx >= 1.1754944e-38f;
-            const float sc = own ? row_factor<true>(mx) : 1.0f / s_shift;
+            uint32_t most = 0, least = 0x7fffu;
+            for (uint32_t c = 0; c < cn; ++c) {
+                most = max(most, s_seen[c][tid] >> 16);
+                least = min(least, s_seen[c][tid] & 0xffffu);
+            }
+            // A row's own factor brings its largest value to [16384, 32768); one with an infinity has none.  The copy is
+            // left as it is where it holds every value exactly: nothing too large, and nothing below 2^-17 (eight bits
+            // down to f16's last, 2^-24).  The row's own copy is then exact as well, so that what the GEMM sees of a row
+            // does not depend on the values the common factor came from.
+            const float mx = __uint_as_float(most << 16);
+            const bool exact = mx * s_shift <= 32768.0f && __uint_as_float(min(least, 0x7f80u) << 16) * s_shift >= 7.62939453125e-6f;
+            const float sc = exact ? 1.0f / s_shift : mx < __int_as_float(0x7f800000) ? row_factor<true>(mx) : 1.0f;
             s_inv[tid] = 1.0f / sc;  // exact: sc is a power of two
             if (rank_in == 0 && m0 + tid < p.M) p.row_scale[m0 + tid] = sc * ldexpf(1.0f, w_exp);  // both factors of the outputs
         }
