@@ -237,11 +237,18 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
     constexpr int NC = SL * kSliceChunks;  // 64-blocks of K a warp owns
     constexpr bool DQ = SC == kScalesU8Words || SC == kScalesU8, TMA_SCALES = SC == kScalesTma;
     extern __shared__ __align__(1024) uint8_t smem[];
-    // (the warp's number through a shuffle: the compiler then knows that it is the same in all lanes, and keeps what follows
-    // from it in uniform registers; with the requests by an elected lane 4 x 4096 x 11008 8.84 -> 8.60 us, the block 54.2 -> 52.6.
-    // The other forms, with more in their registers, lose a little by it, 4 x 4096 x 11008 with u8 scales 9.41 -> 9.62; the
-    // elected lane by itself helps those of 16 columns, 16 x 4096 x 11008 11.68 -> 11.31.)
-    constexpr bool kUniformWarp = NT == 1 && SC == kScalesTma, kElects = NT == 2 || SC == kScalesTma;
+    // kUniformWarp: the warp's number comes through a shuffle; the compiler then knows that it is the same in all lanes, and
+    // keeps what follows from it in uniform registers.  kElects: an elected lane asks for the loop's tiles, else the first one.
+    // Which of them helps depends on what a form has in its registers (us, back to back, without -> with):
+    //   up to 8 rows, scales by TMA: both, 4 x 4096 x 11008 8.84 -> 8.60, the block 54.2 -> 52.6; the other forms lose by them
+    //     (u8 scales 9.41 -> 9.62)
+    //   9 to 16 rows, scales by TMA: elected, at rank 16 16 x 4096 x 11008 12.45 -> 12.28, x 3584 x 18944 18.1 -> 17.9 (but
+    //     16 x 3584 x 512 without an adapter, a tile a warp, 4.99 -> 5.03); uniform as well 9 x 4096 x 4096 7.09 -> 7.28
+    //   9 to 16 rows, u8 words: neither, elected 16 x 4096 x 4096 7.43 -> 7.63, 16 x 11008 x 4096 17.5 -> 17.6 (but
+    //     16 x 3584 x 18944 at rank 16 18.6 -> 18.4)
+    //   9 to 16 rows, d_in no multiple of 256: both, 9 x 4160 x 8192 15.9 -> 15.6, u8 scales 16.2 -> 16.0
+    constexpr bool kUniformWarp = NT == 1 ? SC == kScalesTma : SC == kScalesF32 || SC == kScalesU8;
+    constexpr bool kElects = NT == 1 ? SC == kScalesTma : SC != kScalesU8Words;
     const uint32_t tid = threadIdx.x, warp = kUniformWarp ? __shfl_sync(0xffffffffu, tid >> 5, 0) : tid >> 5, lane = tid & 31u;
     if (ptx::smem_addr(smem) != kWin0) {
         // the table's base is an immediate of the lookups: nothing can run from another address
@@ -698,7 +705,7 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
                         fetch_scales(use_j);
                         __syncwarp();
                         if (req_j < my_tiles) {
-                            if (kElects ? ptx::elect_one() != 0 : lane < nsl) request(req_j, kElects ? 0 : lane);
+                            if (kElects ? ptx::elect_one() != 0 : lane < (NT == 1 ? nsl : 1u)) request(req_j, NT == 1 && !kElects ? lane : 0);
                             ++req_j;
                         }
                     }
