@@ -269,8 +269,13 @@ def test_embedding_gather_equals_dequantize_then_gather(oracle, n_embedding, d_m
 @pytest.mark.parametrize("rows,cols,bf16", [(64, 64, False), (128, 200, True), (256, 1024, True),
                                             (192, 36, False), (100, 72, True), (65, 7, False),
                                             (64, 8, True), (128, 68, True),      # rows TMA takes, and rows it does not
-                                            (2560, 4608, True), (2560, 2304, False),  # warps that take a second tile
-                                            (1984, 68, False), (1600, 100, False)])  # a last tile of seven segments; more missing: the other kernel
+                                            (2560, 4608, True), (2560, 2304, False),
+                                            (1984, 68, False), (1600, 100, False),
+                                            # the TMA kernel: a tile an SM, the last of 12 words; seven segments; two tiles a
+                                            # warp, both ends ragged; scales by fours; f32 whole and ragged
+                                            (512, 7064, True), (448, 7104, True), (1984, 9224, True), (1792, 4160, True),
+                                            (512, 32740, False), (1984, 14020, False),
+                                            (512, 9536, True), (512, 30720, False)])  # just short of it: the other kernel
 def test_load_path_quantize_of_the_transpose(oracle, rows, cols, bf16):
     # src/qwennet.rs:1709-1711: transpose2d([out, in]) then PackedNf4Tensor::quantize (+ double
     # quantization).  The fused kernel (rows % 64 == 0) and the workspace route must both give
@@ -298,7 +303,8 @@ def test_load_path_quantize_of_the_transpose(oracle, rows, cols, bf16):
     assert bits_equal(lin.packed().scale_of_scales.cpu().numpy(), np.asarray([o_sos], np.float32))
 
 
-def test_load_path_codes_of_every_quotient_of_bf16(oracle):
+@pytest.mark.parametrize("copies", [1, 32])  # 32: enough for the TMA kernel
+def test_load_path_codes_of_every_quotient_of_bf16(oracle, copies):
     # The bf16 path decides without a margin: every quotient of two eight-bit significands down to 2^-8 of the block's
     # scale, both signs, and blocks whose scale the reciprocal is not used for.
     from unifur_b200.quantize import PackedNf4Tensor
@@ -320,7 +326,7 @@ def test_load_path_codes_of_every_quotient_of_bf16(oracle):
             c[1, 9] = -np.inf
         cols += list(c)
     cols += [np.zeros(64)] * (-len(cols) % 8)
-    w = oracle.round_bf16(np.ascontiguousarray(np.stack(cols, axis=1)).astype(np.float32))
+    w = oracle.round_bf16(np.ascontiguousarray(np.tile(np.stack(cols, axis=1), (copies, 1))).astype(np.float32))
     o_packed, o_absmax = oracle.quantize_packed(np.ascontiguousarray(w.T).reshape(-1))
     p = PackedNf4Tensor.quantize_transposed(torch.from_numpy(w).to(DEV).bfloat16())
     assert bits_equal(p.absmax.cpu().numpy(), o_absmax)

@@ -817,12 +817,20 @@ int32_t quantize_transposed(const void *src, bool src_bf16, uint64_t rows, uint6
             return fail(NF4_ERR_UNSUPPORTED, "nf4_quantize_transposed: matrix too large");
         const uint32_t *w = static_cast<const uint32_t *>(src);
         count_launch();
-        // bf16 wherever TMA takes it; f32, bound by its bytes, where no more than a twenty-fifth of the tiles' eight segments
-        // are missing ([7936, 7424], 124 segments: 57.4 -> 55.1 us; but [4352, 2688], 68: 18.5 -> 19.2, [4416, 2688], 69: 18.3 -> 19.5)
-        const uint64_t whole = (rows / kBlock + kTmaWarps - 1) / kTmaWarps * kTmaWarps;
-        if (words % 4 == 0 && (src_bf16 || whole * 24 <= rows / kBlock * 25)) {
+        // The TMA kernel gains where its CTAs have enough to do for its later start and even shares of it; a tile is eight
+        // segments of 32 words, those beyond the last segment included (back to back, cold, the other kernel's time first).
+        // bf16: from 7/4 of the SMs in tiles on ([2048, 4096], 256 tiles: 9.7, 9.6 us; [4096, 4096] 15.9, 15.0; [14336, 7424]
+        // 74, 57), and where most SMs have a tile and none two ([4096, 1024], 128: 7.2, 6.9; [3072, 1024], 96: 6.5, 6.6; [256, 4096]
+        // 4.7, 5.3; [1536, 4096], 192: 8.4, 9.2), unless a fifth of the segments is missing ([1088, 11008], 17 of 24: 12.5, 13.4).
+        // f32, bound by its bytes: 13/16 of the other kernel's time a segment and 2.6 us of start ([4096, 4096]: 19.5, 19.3;
+        // [14336, 7424] 99, 84; [3584, 4096] 17.4, 17.5; [1024, 1024] 4.5, 6.3), more where the scales leave in less than sectors
+        // ([4352, 7424], 68 segments: 31.8, 30.8; [4416, 4096], 69: 19.9, 20.7).
+        const uint64_t segments = rows / kBlock, octets = (segments + kTmaWarps - 1) / kTmaWarps, strips = (words + 31) / 32, tiles = octets * strips;
+        const bool even = tiles <= kNumSMs ? tiles * 4 >= kNumSMs * 3 : tiles * 4 >= kNumSMs * 7;
+        const int64_t saved = (int64_t)strips * ((int64_t)segments * 16 - (int64_t)octets * kTmaWarps * 13);
+        const bool gains = src_bf16 ? even && segments * 5 >= octets * kTmaWarps * 4 : saved >= (segments % 8 ? 35000 : 24576);
+        if (words % 4 == 0 && gains) {
             auto kernel = src_bf16 ? quantize_transposed_tma_kernel<true> : quantize_transposed_tma_kernel<false>;
-            const uint64_t segments = rows / kBlock, octets = (segments + kTmaWarps - 1) / kTmaWarps, tiles = octets * ((words + 31) / 32);
             CUtensorMap map;
             NF4_TRY(make_map(&map, CU_TENSOR_MAP_DATA_TYPE_UINT32, src, rows, words, words * 4, kBlock, 32, CU_TENSOR_MAP_SWIZZLE_NONE));
             FailureRef failure;
