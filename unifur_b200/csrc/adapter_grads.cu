@@ -5,8 +5,8 @@
 //
 // gradient_kernel: out(p, j) = s sum_m X[m][p] R[m][j] as D[p][j] += X^T R (tcgen05, both operands MN-major as they lie).  A
 // CTA takes 128 columns p, 64 ranks and a share of the rows; stages of 64 rows of X and of both halves of R (32 KB) come
-// by TMA, three in flight (an SM holds one CTA, by the driver's count; 61 of its L2 port's bytes a nanosecond
-// arrive); one thread asks for them and one issues their MMAs.  The CTAs that share a
+// by TMA, three in flight (an SM holds one CTA: the driver counts one, although shared memory and registers would do for
+// two; 61 of its L2 port's bytes a nanosecond arrive); one thread asks for them and one issues their MMAs.  The CTAs that share a
 // tile's rows form a cluster: their sums meet through distributed shared memory, each adds (in rank order) and writes its
 // part of the columns.  Both gradients are one launch: the tiles of x with U, then those of grad_y with T.  Bound by reading X
 // once and R from the L2 for every 128 columns and, at few columns, by the chain of a load, its stages and that exchange.
@@ -36,7 +36,7 @@ struct Params {
     float scale;
 };
 
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kThreads, 2)  // (registers for two)
 gradient_kernel(const __grid_constant__ CUtensorMap tmap_x0, const __grid_constant__ CUtensorMap tmap_r0, const __grid_constant__ CUtensorMap tmap_x1,
                 const __grid_constant__ CUtensorMap tmap_r1, const Params p, const FailureRef failure) {
     namespace cg = cooperative_groups;

@@ -1302,7 +1302,7 @@ int32_t decode_forward_scatter(const nf4_linear_args &a, void *const *dest, uint
 // memory it can write.  `host_done` becomes `value` once y is complete.  False in `taken`: not this kernel's call.
 // The kernel starts at once, sets itself up and asks for its first weights while x crosses the bus, and the host sees its
 // word before the grid has drained: with a copy operation ahead of the kernel and a stream's synchronise behind it the
-// call of 4 x 4096 x 11008 took 30.0 us, now 25.6 (the caller 3.4 and the launch 3 of them, 4 until it runs, x 3 after that,
+// call of 4 x 4096 x 11008 took 29.9 us, now 23.8 (the caller 3.4 and the launch 3 of them, 4 until it runs, x 3 after that,
 // the tiles 7, the results' way over the bus 4).
 int32_t decode_forward_host(const nf4_linear_args &a, const void *x_host, uint32_t *host_done, uint32_t value, cudaStream_t stream, bool *taken) {
     *taken = false;

@@ -5,7 +5,7 @@
 // adds the two halves, the bias and the adapter term s (x A^T) B^T, which is computed in f32 from
 // the f32 factors as the reference does.  At most eight rows per pass (sixteen for the kernel).
 // 9 x 9728 x 18240 at rank 32: 160 us with T by CTAs of many columns (38 of it) and a thread per output that walked its row of B
-// value by value (29), now 115; 4 x 4096 x 11008 at rank 16 28.7, now 16.7; 16 x 4096 x 4096 at rank 64 54.6, now 34.9.
+// value by value (29), now 108; 4 x 4096 x 11008 at rank 16 28.7, now 16.7; 16 x 4096 x 4096 at rank 64 54.6, now 34.9.
 #include <cuda_bf16.h>
 
 #include "kernels.cuh"

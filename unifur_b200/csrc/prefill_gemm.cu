@@ -676,7 +676,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         const uint32_t group = (warp - kFirstExpanderWarp) >> 2;
         const uint32_t q = warp & 3u;
         const uint32_t row_in_tile = q * 32 + lane;
-        if (PERK) ptx::pdl_wait();  // the weight is repacked by a kernel that completes before the pre-pass does
+        if (PERK) ptx::pdl_wait();  // the kernel ahead repacks the weight, and completes after the pre-pass
         const uint32_t lane_word = lane * 4u | kTableAt | own;  // bytes {4 lane, 0, 1, rank}: see level_pair
         // block scales are used divided by a power of two (see weight_exponent)
         // ... and enter the product as f16: one multiplication from the loaded value.  (A u8 code's scale is

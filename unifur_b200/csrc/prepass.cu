@@ -437,7 +437,7 @@ prepass_kernel(const Params p) {
 // operand as it lies, 128 rows whatever kRows is: the rows behind the tile are somebody else's bytes and nobody reads
 // what they give; the factor the B operand, K-major as [r][K], MN-major as [K][r]), eight warps write the f16 copy and
 // keep the maxima.  Nothing in the loop waits for the whole CTA: the kernel above, with warp MMAs, a barrier a stage
-// and two stages in flight, ran at a fifth of the DRAM rate ([2048, 14336] at rank 64: 48 us; [2048, 4096]: 17.6).
+// and two stages in flight, ran at a fifth of the DRAM rate ([2048, 14336] at rank 64: 48 us, now 29, two of them for the rows' least values).
 constexpr uint32_t kTcThreads = 384, kTcStages = 8, kTcFactorStage = 8192;
 __host__ __device__ constexpr uint32_t tc_ring(uint32_t rows) { return kTcStages * (rows * 128 + kTcFactorStage); }
 
@@ -489,7 +489,7 @@ prepass_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         ptx::fence_proxy_async();
         ptx::prefetch_tmap(&tmap_x);
         ptx::prefetch_tmap(&tmap_a);
-        if (p.wait == 0) ptx::pdl_wait();
+        ptx::pdl_wait();  // (p.wait is 0: only f32 x has a factor that the kernel ahead writes)
         for (uint32_t st = 0; st < min(stages, kStages); ++st) request(st);
     }
     if (kCopy && tid < kRows) {
@@ -503,7 +503,7 @@ prepass_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
-    if (p.wait == 0) ptx::pdl_wait();
+    ptx::pdl_wait();
     ptx::pdl_launch_dependents();  // (what for: see the kernel above)
     if (blockIdx.x == 0)
         for (uint32_t i = tid; i < p.n_flags; i += kTcThreads) p.flags[i] = 0;
