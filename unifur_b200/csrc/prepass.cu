@@ -75,12 +75,24 @@ __device__ __forceinline__ uint32_t bf16x2_larger_bits(uint32_t mx) {
     return max(a, b);
 }
 
-// Running minima of the nonzero |bf16|, a pair at a time: 2 |v| - 2 as 16 unsigned bits, which puts a zero on top of all.
-// (The sign below and the borrow of a zero below reach the upper half: it may come out one lower.  The smallest subnormals
-// may wrap; no power of two used here brings them into f16's range.)
-__device__ __forceinline__ uint32_t bf16x2_absmin(uint32_t w, uint32_t mn) { return __vminu2(mn, w * 2u - 0x00020002u); }
-// The smaller half as an f32 pattern at or just below the least nonzero value.
-__device__ __forceinline__ uint32_t bf16x2_smaller_bits(uint32_t mn) { return (min(mn & 0xffffu, mn >> 16) >> 1) << 16; }
+// Running minima of the nonzero |bf16|, a pair at a time, as patterns one or two below them: taking one off turns a zero into
+// a NaN, which the minimum leaves out.  (A zero's borrow reaches the upper half, where it may make a NaN of the smallest
+// subnormal; no power of two used here brings that one into f16's range.)
+__device__ __forceinline__ uint32_t bf16x2_absmin(uint32_t w, uint32_t mn) {
+    uint32_t d;
+    asm("min.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(w - 0x00010001u), "r"(mn));
+    return d;
+}
+// What was seen of a row as one word: its largest value above the negative of its least nonzero one (infinity: it has none),
+// both as bf16, so that words join by one maximum of pairs.
+__device__ __forceinline__ uint32_t row_seen(uint32_t mx, uint32_t mn) {
+    return bf16x2_larger_bits(mx) | 0x8000u | min(min(mn & 0x7fffu, (mn >> 16) & 0x7fffu), 0x7f80u);
+}
+__device__ __forceinline__ uint32_t join_seen(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
 
 __device__ __forceinline__ uint4 bf16x8_to_f16x8(const uint4 &v) {
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
@@ -455,9 +467,9 @@ prepass_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     static_assert(kRows * kPartPitch * 4 <= tc_ring(kRows), "the sums reuse the stages");
     static_assert((kStages - 1) * kXStage + 128 * 128 <= tc_ring(kRows), "an MMA reads 128 rows from the last stage's place");
     extern __shared__ uint8_t smem_any[];
-    __shared__ uint32_t s_seen[kMaxCluster][kRows];  // the CTAs' row maxima (bf16 patterns) above their nonzero minima
+    __shared__ uint32_t s_seen[kMaxCluster][kRows];  // the CTAs' rows (see row_seen)
+    __shared__ uint32_t s_part[kGroups][kRows];      // this CTA's, by the warps
     __shared__ float s_inv[kRows];
-    __shared__ uint32_t s_most[kRows], s_least[kRows];  // this CTA's, as f32 patterns
     __shared__ float s_shift;
     __shared__ int s_exp;
     __shared__ __align__(8) uint64_t s_bars[2 * kStages + 1];
@@ -491,10 +503,6 @@ prepass_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         ptx::prefetch_tmap(&tmap_a);
         ptx::pdl_wait();  // (p.wait is 0: only f32 x has a factor that the kernel ahead writes)
         for (uint32_t st = 0; st < min(stages, kStages); ++st) request(st);
-    }
-    if (kCopy && tid < kRows) {
-        s_most[tid] = 0;
-        s_least[tid] = 0x7fff0000u;
     }
     if (warp == 9) {
         ptx::tmem_alloc(ptx::smem_addr(&s_tmem), 64);
@@ -597,16 +605,10 @@ prepass_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         }
         #pragma unroll
         for (uint32_t q = 0; q < kQuads; ++q) {  // (eight lanes hold a row's)
-            uint32_t m = bf16x2_larger_bits(mx[q]), n = bf16x2_smaller_bits(mn[q]);
+            uint32_t seen = row_seen(mx[q], mn[q]);
             #pragma unroll
-            for (int d = 1; d < 8; d *= 2) {
-                m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
-                n = min(n, __shfl_xor_sync(0xffffffffu, n, d));
-            }
-            if (piece == 0) {
-                atomicMax(s_most + r0 + q * 4, m);
-                atomicMin(s_least + r0 + q * 4, n);
-            }
+            for (int d = 1; d < 8; d *= 2) seen = join_seen(seen, __shfl_xor_sync(0xffffffffu, seen, d));
+            if (piece == 0) s_part[warp / kPerStage][r0 + q * 4] = seen;
         }
         if (!ok && lane == 0) NF4_REPORT_FAILURE(*failure.flag, *failure.host, 10);
     }
@@ -638,26 +640,27 @@ prepass_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         ptx::tc_fence_before();
     }
     cluster.barrier_wait();
-    if (kCopy && warp >= 8)
-        for (uint32_t i = tid - 256; i < kRows * cn; i += 128)
-            cluster.map_shared_rank(&s_seen[0][0], i / kRows)[rank_in * kRows + i % kRows] = s_most[i % kRows] | s_least[i % kRows] >> 16;
+    if (kCopy && warp >= 8) {
+        const uint32_t r = (tid - 256) % kRows;
+        uint32_t seen = s_part[0][r];
+        #pragma unroll
+        for (uint32_t g = 1; g < kGroups; ++g) seen = join_seen(seen, s_part[g][r]);
+        for (uint32_t c = (tid - 256) / kRows; c < cn; c += 128 / kRows) cluster.map_shared_rank(&s_seen[0][0], c)[rank_in * kRows + r] = seen;
+    }
     if (warp >= 8) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     else asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     const int w_exp = s_exp;
     if (kCopy) {
         if (tid < kRows) {
-            uint32_t most = 0, least = 0x7fffu;
-            for (uint32_t c = 0; c < cn; ++c) {
-                most = max(most, s_seen[c][tid] >> 16);
-                least = min(least, s_seen[c][tid] & 0xffffu);
-            }
+            uint32_t seen = s_seen[0][tid];
+            for (uint32_t c = 1; c < cn; ++c) seen = join_seen(seen, s_seen[c][tid]);
             // A row's own factor brings its largest value to [16384, 32768); one with an infinity has none.  The copy is
             // left as it is where it holds every value exactly: nothing too large, and nothing below 2^-17 (eight bits
             // down to f16's last, 2^-24).  The row's own copy is then exact as well, so that what the GEMM sees of a row
             // does not depend on the values the common factor came from.
-            const float mx = __uint_as_float(most << 16);
-            const bool exact = mx * s_shift <= 32768.0f && __uint_as_float(min(least, 0x7f80u) << 16) * s_shift >= 7.62939453125e-6f;
+            const float mx = __uint_as_float(seen & 0xffff0000u), least = __uint_as_float((seen & 0x7fffu) << 16);
+            const bool exact = mx * s_shift <= 32768.0f && least * s_shift >= 7.62939453125e-6f;
             const float sc = exact ? 1.0f / s_shift : mx < __int_as_float(0x7f800000) ? row_factor<true>(mx) : 1.0f;
             s_inv[tid] = 1.0f / sc;  // exact: sc is a power of two
             if (rank_in == 0 && m0 + tid < p.M) p.row_scale[m0 + tid] = sc * ldexpf(1.0f, w_exp);  // both factors of the outputs
