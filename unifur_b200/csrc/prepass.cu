@@ -449,7 +449,7 @@ prepass_kernel(const Params p) {
 // operand as it lies, 128 rows whatever kRows is: the rows behind the tile are somebody else's bytes and nobody reads
 // what they give; the factor the B operand, K-major as [r][K], MN-major as [K][r]), eight warps write the f16 copy and
 // keep the maxima.  Nothing in the loop waits for the whole CTA: the kernel above, with warp MMAs, a barrier a stage
-// and two stages in flight, ran at a fifth of the DRAM rate ([2048, 14336] at rank 64: 48 us, now 29, two of them for the rows' least values).
+// and two stages in flight, ran at a fifth of the DRAM rate ([2048, 14336] at rank 64: 48 us, now 27).
 constexpr uint32_t kTcThreads = 384, kTcStages = 8, kTcFactorStage = 8192;
 __host__ __device__ constexpr uint32_t tc_ring(uint32_t rows) { return kTcStages * (rows * 128 + kTcFactorStage); }
 
