@@ -339,7 +339,9 @@ NF4_API int32_t nf4_decode_share_plan(uint32_t rows, uint32_t d_in, uint32_t d_o
  * receives, for CTA `cta`, up to `capacity` triples (tile, first main k-stage, one past the last)
  * in the order the CTA works on them.  Returns the number of the CTA's segments, or a negative
  * status.  Tiles that appear with a partial range of k-stages are split between neighbouring
- * pairs of CTAs (the one with the last stages finishes the tile).  For inspection and tests; the
+ * pairs of CTAs (the one with the last stages finishes the tile).  Up to 128 rows the tiles have 128
+ * activation rows.  Where more rows make few tiles, a forward may instead give each of up to 74 pairs one whole
+ * tile of 128 activation rows; the plan is then the one it would follow with tiles of 256.  For inspection and tests; the
  * reference has no counterpart. */
 NF4_API int32_t nf4_prefill_share_plan(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t cta, uint32_t *ctas,
                                        uint32_t *segments, uint32_t capacity);

@@ -6,21 +6,22 @@
 // Two CTAs of a cluster, one per SM, work on a tile of 256 weight rows x 256 activation rows together
 // (cta_group::2): each holds 128 weight rows and their accumulators in its tensor memory and half of the
 // activations in its shared memory, which halves what a shared memory is written and read per
-// multiplication.  Roles inside a CTA (persistent, 864 threads):
-//   warp 0      TMA producer: this CTA's half of the x tile [128 rows x 64 k] (f16, 128B-swizzled,
-//               K-major) into a 4-deep shared-memory ring; after the K loop the same ring carries the LoRA
-//               intermediate T (bf16 hi / lo halves) and one more place the matching
-//               128 x 64 tile of LoRA B, so the adapter is just more k-steps (with both
+// multiplication.  Few rows take tiles of 128 activation rows (share_tiles).  K goes in steps of two stages of 64; what warps
+// hand to one another they hand over a step at a time.  Roles inside a CTA (persistent, 864 threads):
+//   warp 0      TMA producer: this CTA's half of a step's x tiles [128 rows x 64 k] (f16, 128B-swizzled,
+//               K-major) into a 96 KB ring of steps; after the K loop the same ring carries the LoRA
+//               intermediate T (bf16 hi / lo halves) and, a slot before it, the matching
+//               128 x 64 tile of LoRA B, so the adapter is just more steps (with both
 //               operands in shared memory).
 //   warp 1      owns TMEM (alloc/dealloc); in the even CTA it issues the pair's tcgen05.mma.
-//   warp 6      asks for the packed codes: blocks of 128 weight rows x 256 codes by TMA, prefetched into L2.
+//   warp 6      asks for the packed codes, 128 weight rows x 128 a step by TMA, prefetched into L2, and for their scales.
 //   warps 2-5, 23-26  epilogue: TMEM -> registers -> (* row scale, + bias) -> bf16/f32 ->
 //               shared -> TMA store.
-//   warps 7-22  dequantisers, four groups of 128 threads taking every fourth k-stage.  A thread
+//   warps 7-22  dequantisers, four groups of 128 threads, two to a step in turn.  A thread
 //               owns one weight row (= one TMEM lane; a warp may only touch the lane quarter its
-//               number names): it takes the row's 32 packed bytes from shared memory, looks byte by
+//               number names): it takes the row's 32 packed bytes of a stage from shared memory, looks byte by
 //               byte a pair of levels up in a table, multiplies by the block's scale in f16x2 and writes the
-//               64 f16 values into its lane of an eight-deep ring of TMEM columns with tcgen05.st.
+//               64 f16 values into its lane of a ring of four steps of TMEM columns with tcgen05.st.
 //
 // Why the weight operand lives in TMEM.  The table look-ups, the TMA and the MMA's reads of the
 // activations already take most of the 128 B/clk a shared memory delivers; the dequantised weight never
@@ -28,11 +29,14 @@
 // (256 columns) and the weight ring (8 x 32 columns) share the 512 TMEM columns, so there is one
 // accumulator and the MMAs of the next tile wait while the epilogue reads it out.
 //
-// What bounds it: for many rows the tensor pipe (512 cycles a stage and pair; 570 to 630 are taken, with
-// the read-outs), and the clock that the power limit leaves (1.55 GHz on random operands, 1.83 GHz on zeros).
-// 2048 x 4096 x 14336: 231 us with single CTAs, codes loaded by the dequantisers and two issuing threads; now
-// 178, of which the kernels before it take 15.  256 x 3584 x 18944: 45 -> 34 us.  What gave it: the pairs; codes
-// by TMA; one full and one done barrier per stage, both halves counted in the even CTA; the issuing warp together.
+// What bounds it: a wide tile's MMAs, 1024 cycles a step of 256 columns (893 measured for the 896 of 224), and for many rows
+// the clock that the power limit leaves (1.4 GHz on random operands).  A narrow tile's step is the dequantisers' latency, 0.4 us.
+// With a stage at a time the skeleton alone, no look-ups, no stores, a quarter of the MMAs, took 0.29 us a stage: the one lane that
+// asked for the activations spent 300 to 440 cycles on each, and scales loaded by the threads another 0.05 us.  Before ->
+// now, whole calls: 64 x 4096 x 4096 20.6 -> 16.5 us, 128 x 8192 x 8192 37.7 -> 28.6, 203 x 3584 x 18944 36.8 -> 34.7, 512 x 4096 x 4096
+// 32.0 -> 25.9, 2048 x 4096 x 14336 209.9 -> 208.0; the GEMM of a backward over 2048 x 4096 x 14336 167 -> 151.
+// The start counts for few rows: most CTAs start when the pre-pass's end, so the codes of the first steps are asked for
+// before anything else is set up, and the CTAs of a pair meet without a release (1.2 us): 512 x 4096 x 4096 19.4 -> 16.8 us.
 //
 // The MMA computes D[n, m] = sum_k W[n, k] x[m, k]: weight rows are the MMA's M (TMEM lanes),
 // activation rows its N (256 accumulator columns).  Both operands are f16 with f32 accumulation:
@@ -47,9 +51,8 @@
 // activations) comes through the same GEMM at more than 16 rows: small kernels beside the pre-pass write the
 // transposed nibbles, the scales as f16 [N / 64][K] and the adapter factors in this kernel's
 // orientation into the workspace (the nibbles exactly; the scales with the rounding the dequantisers
-// apply anyway).  A weight row's scale then changes with every k: a lane loads the pair of scales of
-// k = 2 lane, 2 lane + 1 of its stage (one 128-byte line per warp) and the warp hands them round
-// with shuffles while it multiplies (template parameter PERK).  f32 activations are converted to f16
+// apply anyway).  A weight row's scale then changes with every k, and is the same for 64 rows: a step's scales come by TMA
+// beside its codes, and every lane reads the same pairs (kScalesPerK).  f32 activations are converted to f16
 // directly, every row divided by its own power of two.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -67,46 +70,66 @@ namespace nf4 {
 __device__ int g_prefill_error = 0;  // set when a bounded wait gives up
 __device__ int *g_prefill_error_host = nullptr;  // the same, in mapped host memory (set by the host-pointer entry points)
 
-
 namespace {
 
 constexpr int BM = 128;        // weight rows per CTA and tile (half of the pair's MMA M; TMEM lanes)
-constexpr int BN = 256;        // activation rows per tile (MMA N, accumulator columns); a CTA brings half of them
 constexpr int BK = 64;         // k per stage = one quantization block = one 128B swizzle row
-constexpr int kXStages = 4;    // shared-memory ring of activation tiles
-constexpr int kCodeSlots = 2;  // shared-memory ring of packed weight codes, four k-stages each
-constexpr int kCodeStages = 4;
-constexpr int kAStages = 8;    // TMEM ring of dequantised weight stages
-constexpr int kAStageCols = BK / 2;  // 32 columns: two f16 per 32-bit cell
-constexpr int kAccCols = BN;   // the accumulator: columns [0, 256); the weight ring follows
+constexpr int kASteps = 4;     // TMEM ring of dequantised weights: steps of two stages
+constexpr int kStageCols = BK / 2;  // 32 columns: two f16 per 32-bit cell
+constexpr int kAccCols = 256;  // the accumulator: columns [0, 256); the weight ring follows
 constexpr int kTmemCols = 512;
-constexpr int kXTileBytes = BN / 2 * BK * 2;   // 16 KB: this CTA's half of the activations, written by TMA
+constexpr int kBarRing = 8;    // steps whose barriers are told apart (more than the deepest ring of activations holds)
+constexpr int kCodeSlots = 3;  // shared-memory ring of packed weight codes, a step each
+constexpr int kCodeTileBytes = BM * 64;        // 8 KB: 128 weight rows x 128 codes, written by TMA (64B swizzle)
+constexpr int kScaleTileBytes = BM * 16;       // 2 KB: the same rows' scales of four stages (f32) or sixteen (u8), by TMA
+constexpr int kPerKBytes = BM / 64 * 2 * BK * 2;  // 512 bytes: a scale for every k of a step and 64-block of rows
 constexpr int kLoraTileBytes = BM * BK * 2;    // 16 KB: 128 rows of LoRA B x 64 ranks, written by TMA
-constexpr int kCodeTileBytes = BM * 128;       // 16 KB: 128 weight rows x 256 codes, written by TMA (128B swizzle)
 
-constexpr int kEpiBytes = 32 * 1024;       // output staging: half a tile of bf16 (as two swizzled boxes), a quarter of f32
+constexpr int kEpiBytes = 32 * 1024;       // output staging: half a wide tile of bf16 (as two swizzled boxes), a quarter of f32
 constexpr int kThreads = 27 * 32;
 constexpr int kFirstExpanderWarp = 7;      // sixteen warps
 constexpr int kFirstEpilogueWarpB = 23;    // the second set of four epilogue warps
 constexpr int kCodeWarp = 6;               // asks for the packed codes
-constexpr int kStageWarps = 8;             // warps that dequantise one stage: a group in each CTA
+constexpr int kStepWarps = 16;             // warps that dequantise a step: two groups in each CTA
 constexpr int kExpanderGroups = 4;         // of four warps (one per TMEM lane quarter) each
 constexpr uint64_t kInOutMinRows = 17;     // the other weight orientation comes here from this many rows on
 
 // Places in the shared window.  The lookup table starts at 0x10000, so that one byte permute of the code
-// word with {4 lane, 0, 1, rank} is an entry's address.
-constexpr uint32_t kLoraAt = 0x800, kCodesAt = 0x4800, kBarsAt = 0xc800, kTmemSlotAt = 0xca00, kRowScalesAt = 0xcc00,
-                   kTableAt = 0x10000, kEpiAt = 0x20000, kXAt = 0x28000, kWindowEnd = kXAt + kXStages * kXTileBytes;
+// word with {4 lane, 0, 1, rank} is an entry's address; the first third of the ring of activations lies below it.
+constexpr uint32_t kBarsAt = 0x800, kTmemSlotAt = 0xa00, kRowScalesAt = 0xc00, kCodesAt = 0x1000, kXAt = 0x8000, kTableAt = 0x10000,
+                   kEpiAt = 0x20000, kXRestAt = 0x28000, kScalesRestAt = kXRestAt + 2 * (kTableAt - kXAt), kScalesAt = kCodesAt + kCodeSlots * kCodeTileBytes,
+                   kWindowEnd = kScalesRestAt + kScaleTileBytes;
 constexpr uint32_t kDynamicSmem = kWindowEnd - 1024;   // the dynamic shared memory starts at 1024 or a little above
-static_assert(kLoraAt + kLoraTileBytes <= kCodesAt && kCodesAt + kCodeSlots * kCodeTileBytes <= kBarsAt && kEpiAt + kEpiBytes <= kXAt, "places overlap");
+static_assert(kScalesAt + (kCodeSlots - 1) * kScaleTileBytes <= kXAt && kEpiAt + kEpiBytes <= kXRestAt, "places overlap");
 static_assert(kDynamicSmem <= 227 * 1024, "shared memory");
 
+// The ring of activations, in slots of a step: this CTA's half of two stages' tiles of BN rows.  96 KB of 32 or 16 KB each.
+template <int BN>
+struct XRing {
+    static constexpr uint32_t kTile = BN / 2 * BK * 2, kSlot = 2 * kTile, kBelow = (kTableAt - kXAt) / kSlot, kSlots = 3 * kBelow;
+    static_assert(kSlot >= kLoraTileBytes && kSlots < kBarRing, "the adapter's tile takes a slot; a parity names a step's round");
+    __device__ static __forceinline__ uint32_t place(uint32_t slot) {
+        return kXAt + slot * kSlot + (slot >= kBelow ? kXRestAt - kTableAt : 0u);
+    }
+    __device__ static __forceinline__ uint32_t next(uint32_t slot) { return slot + 1 == kSlots ? 0u : slot + 1; }
+};
+
+// How the dequantisers get a row's scale of a stage: loaded by the thread, three of its stages ahead; by TMA, sixteen bytes of every row
+// with the codes of a step; or, for weights in the other orientation, a scale for every k, a step's 128 pairs of each of the CTA's two
+// 64-blocks of rows (handed round with shuffles, 32 a stage beside as many lookups, a narrow tile's stage took 0.31 us).  A warp's
+// loads of 32 rows' scales are 32 sectors for four bytes of each, and its walk to the next one some forty instructions: 64 x 16384 x
+// 18944 67 us with them, 55 without scales.  TMA takes rows of whole 16-byte pieces only: d_in a multiple of 256 (u8: 1024).
+enum ScaleSource : int { kScalesLoaded = 0, kScalesTma = 1, kScalesPerK = 2 };
+__device__ __forceinline__ uint32_t scales_place(uint32_t slot) {
+    return slot + 1 == kCodeSlots ? kScalesRestAt : kScalesAt + slot * kScaleTileBytes;
+}
+
 // barrier slots
-// Full counts, in the even CTA, what a k-stage of the pair needs: both halves of the activations (or of an
-// adapter stage's operands) and the eight warps of both CTAs that dequantise its weights.  Done is a stage's
-// MMAs over, in both CTAs: whatever the stage's slots held is free.  Stages number on over a pair's segments,
-// the adapter's included; stage c has slot c % kXStages of the activations, c % kAStages of everything else.
-constexpr int kBarFull = 0, kBarDone = kBarFull + kAStages, kBarAccFull = kBarDone + kAStages, kBarAccEmpty = kBarAccFull + 1,
+// Full counts, in the even CTA, what a step of the pair needs: both halves of the activations (or of an
+// adapter step's operands) and the sixteen warps of both CTAs that dequantise its weights.  Done is a step's
+// MMAs over, in both CTAs: whatever the step's slots held is free.  Steps number on over a pair's segments,
+// the adapter's included; step c has barriers c % kBarRing and weight columns c % kASteps.
+constexpr int kBarFull = 0, kBarDone = kBarFull + kBarRing, kBarAccFull = kBarDone + kBarRing, kBarAccEmpty = kBarAccFull + 1,
               kBarCFull = kBarAccEmpty + 1, kBarCEmpty = kBarCFull + kCodeSlots, kNumBars = kBarCEmpty + kCodeSlots;
 static_assert(kBarsAt + kNumBars * 8 <= kTmemSlotAt, "barrier room");
 
@@ -124,7 +147,8 @@ struct PrefillParams {
     uint32_t M, N, K, rank;
     uint32_t lora_chunks;  // ceil(rank / 64); T is [M][2 * 64 * lora_chunks] (hi halves, then lo)
     uint32_t m_tiles;
-    // Work of a pair of CTAs (tiles of 256 weight rows x 256 activation rows, the even CTA the lower 128
+    uint32_t box_rows;     // activation rows a CTA brings of a tile
+    // Work of a pair of CTAs (tiles of 256 weight rows x BN activation rows, the even CTA the lower 128
     // weight rows): first its share of the `sk_tiles` tiles whose k-stages all pairs divide
     // evenly between them (a tile can be split between neighbouring pairs), then `dp_rounds`
     // whole tiles.  A pair that multiplies the leading stages of a tile leaves its accumulators
@@ -133,6 +157,8 @@ struct PrefillParams {
     // split > 1 (fewer tiles than pairs): a tile is `split` pairs' instead, an equal part of its stages each; all leave
     // their accumulators in `partial`, and a kernel of its own adds them (sum_parts_kernel).
     uint32_t sk_tiles, dp_rounds, split;
+    uint32_t share_r;      // main stages of the shared tiles beyond share_q for every pair (a division in 64 bits takes the
+    uint64_t share_q;      // kernel's start 0.2 us)
     float *partial;
     uint32_t *sk_flags;
     uint32_t wait_ns;  // bound of the wait for a neighbour's flag
@@ -156,23 +182,30 @@ struct WorkList {
         cta = cta_;
         ctas = ctas_;
         sk_tiles = p.sk_tiles;
-        const uint64_t all = (uint64_t)p.sk_tiles * ks;
-        u0 = all * cta / ctas;
-        u1 = all * (cta + 1) / ctas;
         if (p.split > 1) {  // (sk_tiles * split == ctas: a part lies in one tile)
-            u0 = (uint64_t)(cta / p.split) * ks + (uint64_t)ks * (cta % p.split) / p.split;
-            u1 = (uint64_t)(cta / p.split) * ks + (uint64_t)ks * (cta % p.split + 1) / p.split;
+            const uint64_t t0 = (uint64_t)(cta / p.split) * ks;
+            u0 = t0 + part_begin(0, ks, cta % p.split, p.split);
+            u1 = t0 + part_begin(0, ks, cta % p.split + 1, p.split);
+        } else {
+            u0 = part_begin(p.share_q, p.share_r, cta, ctas);
+            u1 = part_begin(p.share_q, p.share_r, cta + 1, ctas);
         }
         n_shared = 0;
         t_first = t_last = 0;
         if (u1 > u0) {
-            t_first = (uint32_t)(u0 / ks);
-            t_last = (uint32_t)((u1 - 1) / ks);
+            t_first = tile_of(u0);
+            t_last = tile_of(u1 - 1);
             n_shared = t_last - t_first + 1;
         }
         n_seg = n_shared + p.dp_rounds;
     }
-    __host__ __device__ static uint64_t range_begin(uint64_t all, uint32_t c, uint32_t n) { return all * c / n; }
+    __host__ __device__ uint32_t tile_of(uint64_t stage) const { return stage >> 32 ? (uint32_t)(stage / ks) : (uint32_t)stage / ks; }
+    // Where part c of n begins, when each has q stages and r more are shared out (c r below 2^32): at a whole step of two
+    // stages, if tiles consist of whole steps.
+    __host__ __device__ uint64_t part_begin(uint64_t q, uint32_t r, uint32_t c, uint32_t n) const {
+        const uint64_t u = q * c + r * c / n;
+        return ks & 1u ? u : u & ~1ull;
+    }
     __host__ __device__ void get(uint32_t j, uint32_t &tile, uint32_t &b, uint32_t &e) const {
         if (j < n_shared) {
             tile = t_last - j;
@@ -187,11 +220,12 @@ struct WorkList {
     }
 };
 
-// Activation rows the MMAs of a tile beginning at row m0 take: all 256, or for the last, ragged tile the rows there are,
+// Activation rows the MMAs of a tile beginning at row m0 take: all BN, or for the last, ragged tile the rows there are,
 // up to a multiple of 32 (each CTA brings half of them).  An MMA takes as long as it has columns: at 64 rows the
 // k-stage is then bound by the dequantisers (64 x 4096 x 4096, whole call: 41 -> 32 us with the rows that do not exist
 // left out of the split tiles' sums as well; 64 x 14336 x 4096: 54 -> 43).
-__device__ __forceinline__ uint32_t tile_columns(uint32_t M, uint32_t m0) {
+template <int BN>
+__host__ __device__ __forceinline__ uint32_t tile_columns(uint32_t M, uint32_t m0) {
     const uint32_t left = M - m0;
     return left < BN ? (left + 31) / 32 * 32 : BN;
 }
@@ -228,22 +262,30 @@ __device__ __forceinline__ uint32_t level_pair(uint32_t word, int byte, uint32_t
     return v;
 }
 
-// Half a stage of one weight row: 16 packed bytes -> 16 registers of f16x2.  PERK (a scale per k): lane j
-// of the warp holds the f16 pair of scales of k = 2j, 2j + 1 of this stage; `first` is the pair of out[0].
+// Half a stage of one weight row: 16 packed bytes -> 16 registers of f16x2.  `scale`: the block's, twice; PERK: where the pairs of
+// scales of the sixteen pairs of k lie, the same for the whole warp.
 template <bool PERK>
-__device__ __forceinline__ void expand_half(const uint32_t *w, uint32_t scale2, int first, uint32_t lane_word, uint32_t (&out)[16]) {
+__device__ __forceinline__ void expand_half(const uint32_t *w, uint32_t scale, uint32_t lane_word, uint32_t (&out)[16]) {
     #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const uint32_t v = level_pair(w[i >> 2], i & 3, lane_word);
-        out[i] = hmul2(v, PERK ? __shfl_sync(0xffffffffu, scale2, first + i) : scale2);
+    for (int i = 0; i < 16; i += 4) {
+        uint32_t s[4] = {scale, scale, scale, scale};
+        if (PERK) asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3]) : "r"(scale + i * 4u) : "memory");
+        #pragma unroll
+        for (int j = 0; j < 4; ++j) out[i + j] = hmul2(level_pair(w[i >> 2], j, lane_word), s[j]);
     }
 }
 
-template <bool YF32, bool PERK>
+// The sixteen f16 levels, for plain loads when the table is built (constant memory is read one index at a time).
+__device__ const uint32_t g_level_f16[16] = {NF4_LEVEL_F16_BITS_LIST};
+
+template <int BN, bool YF32, int SCALES>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_t,
                const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_y,
-               const __grid_constant__ CUtensorMap tmap_w, const PrefillParams p) {
+               const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_ahead,
+               const __grid_constant__ CUtensorMap tmap_s, const PrefillParams p) {
+    using X = XRing<BN>;
+    constexpr bool PERK = SCALES == kScalesPerK;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // In a cluster a CTA's shared-memory addresses carry its rank in the top byte: `own`.
     const uint32_t win = ptx::smem_addr(smem_raw), own = win & 0xff000000u;
@@ -257,29 +299,53 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     auto bar = [&](int i) { return (own | kBarsAt) + 8u * i; };
 
     const uint32_t k_stages = p.K / BK;
-    const uint32_t lora_stages = 2 * p.lora_chunks;  // adapter k-stages per tile: hi and lo halves of T
+    // A tile's steps: two stages each (an odd last one has one), then one for each chunk of the adapter (T's hi and lo halves).
     WorkList wl;
     wl.init(p, k_stages, pair, pairs);
 
     if (p.split > 1) ptx::pdl_launch_dependents();  // the kernel that adds the parts: it waits for this one to complete
-    if (win - own > kLoraAt) {  // (both CTAs alike) the places below are not ours
+    if (win - own > kBarsAt) {  // (both CTAs alike) the places below are not ours
         if (threadIdx.x == 0) NF4_REPORT_FAILURE(g_prefill_error, g_prefill_error_host, 6);
         return;
     }
+    // A step's codes (and scales) go to a slot of their ring; the L2 is asked for eight stages at a time, some twenty
+    // ahead of their loads (weights that nobody has touched yet come from HBM).
+    constexpr uint32_t kAhead = 3, kUnit = 8;  // requests to the L2 ahead, and stages of each
+    auto ask_codes = [&](uint32_t ks, int32_t n0, uint32_t slot) {
+        ptx::mbar_arrive_expect_tx(bar(kBarCFull + slot), kCodeTileBytes + (PERK ? kPerKBytes : SCALES == kScalesTma ? kScaleTileBytes : 0));
+        ptx::tma_load_2d((own | kCodesAt) + slot * kCodeTileBytes, &tmap_w, (int32_t)(ks * (BK / 2)), n0, bar(kBarCFull + slot));
+        if (SCALES == kScalesTma)
+            ptx::tma_load_2d(own | scales_place(slot), &tmap_s, (int32_t)(p.absmax ? ks & ~3u : ks & ~15u), n0, bar(kBarCFull + slot));
+        if (PERK) ptx::tma_load_2d(own | scales_place(slot), &tmap_s, (int32_t)(ks * BK), n0 / 64, bar(kBarCFull + slot));
+    };
+    auto ask_l2 = [&](uint32_t ks, int32_t n0) { ptx::tma_prefetch_2d(&tmap_ahead, (int32_t)(ks * (BK / 2)), n0); };
+    uint32_t asked = 0;  // steps of the first segment whose codes are on their way before anything else is in place
+    if (warp == kCodeWarp) {
+        uint32_t tile = 0, kb = 0, ke = 0;
+        if (!PERK && wl.n_seg) wl.get(0, tile, kb, ke);
+        asked = min((ke - kb + 1) / 2, (uint32_t)kCodeSlots);
+        if (ptx::elect_one()) {
+            for (int s = 0; s < kCodeSlots; ++s) {
+                ptx::mbar_init(bar(kBarCFull + s), 1);
+                ptx::mbar_init(bar(kBarCEmpty + s), 8);   // the warps that dequantise a step
+            }
+            ptx::fence_mbar_init();
+            ptx::fence_proxy_async();
+            const int32_t n0 = (int32_t)(((tile / p.m_tiles) * 2 + rank) * BM);
+            for (uint32_t i = 0; i < asked; ++i) ask_codes(kb + 2 * i, n0, i);
+            for (uint32_t k = kb; k < min(ke, kb + kAhead * kUnit); k += kUnit) ask_l2(k, n0);
+        }
+        __syncwarp();
+    }
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kAStages; ++s) {
-            ptx::mbar_init(bar(kBarFull + s), 1 + kStageWarps);
+        for (int s = 0; s < kBarRing; ++s) {
+            ptx::mbar_init(bar(kBarFull + s), 1 + kStepWarps);
             ptx::mbar_init(bar(kBarDone + s), 1);
         }
         ptx::mbar_init(bar(kBarAccFull), 1);
         ptx::mbar_init(bar(kBarAccEmpty), 16);      // the epilogue warps of both CTAs (used in the even one)
-        for (int s = 0; s < kCodeSlots; ++s) {
-            ptx::mbar_init(bar(kBarCFull + s), 1);
-            ptx::mbar_init(bar(kBarCEmpty + s), 16);  // the dequantiser warps
-        }
         ptx::fence_mbar_init();
         ptx::fence_proxy_async();
-        ptx::prefetch_tmap(&tmap_w);
         ptx::prefetch_tmap(&tmap_x);
         ptx::prefetch_tmap(&tmap_y);
         if (p.lora_chunks) {
@@ -287,10 +353,61 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             ptx::prefetch_tmap(&tmap_b);
         }
     }
-    if (threadIdx.x >= 64 && threadIdx.x < 64 + 512) {
-        // thread (byte, half) writes sixteen lanes' copies, rotated so that a warp's stores spread over the banks
-        const uint32_t i = threadIdx.x - 64, byte = i >> 1, half = i & 1u;
-        const uint32_t e = c_level_f16_bits[byte & 15u] | (c_level_f16_bits[byte >> 4] << 16);
+    // The scales of this group's next kDepth stages are in flight.  A position is walked, not divided out.
+    constexpr int kDepth = 3;
+    struct Pos {
+        uint32_t seg, ks, ke;  // segment, stage in tile, the segment's end
+        uint32_t before;       // steps before the segments after this one
+        size_t row;            // index of the weight row's first scale
+    } ahead{0, 0, 0, 0, 0};
+    const uint32_t group = (warp - kFirstExpanderWarp) >> 2, odd = group >> 1, half = group & 1u;  // (of a dequantiser)
+    const uint32_t q = warp & 3u, row_in_tile = q * 32 + lane;  // the TMEM lane quarter this warp may touch
+    const uint32_t blocks_per_row = p.K / 64;
+    auto enter = [&]() {  // the first main stage of this group in segment ahead.seg or a later one
+        for (; ahead.seg < wl.n_seg; ++ahead.seg) {
+            uint32_t tile, kb;
+            wl.get(ahead.seg, tile, kb, ahead.ke);
+            ahead.ks = kb + 2 * ((odd - ahead.before) & 1u) + half;
+            ahead.before += (ahead.ke - kb + 1) / 2 + (ahead.ke == k_stages ? p.lora_chunks : 0);
+            if (ahead.ks < ahead.ke) {
+                // (rows beyond the last read its scales; nobody stores what comes of them)
+                const uint32_t n0 = ((tile / p.m_tiles) * 2 + rank) * BM;
+                ahead.row = (size_t)min(n0 + row_in_tile, p.N - 1) * blocks_per_row;
+                return;
+            }
+        }
+    };
+    // The scale of the next stage as loaded: f32 bits or a u8 code.
+    // Nothing is computed from it here: that would wait for the load, the latency the pipeline hides.
+    auto fetch = [&]() -> uint32_t {
+        if (SCALES != kScalesLoaded || ahead.seg >= wl.n_seg) return 0;
+        const uint32_t v = p.absmax ? __float_as_uint(__ldg(p.absmax + ahead.row + ahead.ks)) : __ldg(p.scale_codes + ahead.row + ahead.ks);
+        ahead.ks += kExpanderGroups;
+        if (ahead.ks >= ahead.ke) {
+            ++ahead.seg;
+            enter();
+        }
+        return v;
+    };
+    uint32_t scales[kDepth] = {};
+    const bool dequantiser = threadIdx.x >= kFirstExpanderWarp * 32 && threadIdx.x < kFirstEpilogueWarpB * 32;
+    if (SCALES == kScalesLoaded && dequantiser) {
+        enter();
+        #pragma unroll
+        for (int d = 0; d < kDepth; ++d) scales[d] = fetch();
+    }
+    // Block scales are used divided by a power of two (see weight_exponent)
+    // ... and enter the product as f16: one multiplication from the loaded value.  (A u8 code's scale is
+    // (code / 255) * scale of scales; dividing once instead of per code moves it by an ulp of f32.)
+    float scale_unit = 1.0f;
+    if (dequantiser) {
+        // dequantiser (byte, half) writes sixteen lanes' copies, rotated so that a warp's stores spread over the banks
+        const uint32_t i = threadIdx.x - kFirstExpanderWarp * 32, byte = i >> 1, half = i & 1u;
+        const uint32_t e = __ldg(g_level_f16 + (byte & 15u)) | (__ldg(g_level_f16 + (byte >> 4)) << 16);
+        if (!PERK) {
+            const float w_down = ldexpf(1.0f, -weight_exponent(p.absmax, p.scale_codes, p.scale_of_scales));
+            scale_unit = p.absmax ? w_down : __fdiv_rn(__ldg(p.scale_of_scales), 255.0f) * w_down;
+        }
         #pragma unroll
         for (uint32_t q = 0; q < 4; ++q)
             *reinterpret_cast<uint4 *>(at(kTableAt) + byte * 256u + half * 64u + ((q + byte) & 3u) * 16u) = make_uint4(e, e, e, e);
@@ -299,104 +416,125 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         ptx::tmem_alloc_pair(own | kTmemSlotAt, kTmemCols);
         ptx::tmem_relinquish_pair();
     }
+    // The barriers of both CTAs are in place (their initialisation is fenced for the cluster by the threads that made it; a
+    // release by all threads took 1.2 us), and this CTA's table.
+    ptx::cluster_arrive_relaxed();
     ptx::tc_fence_before();
-    ptx::cluster_sync_all();  // (a superset of __syncthreads) the barriers of both CTAs are in place
+    __syncthreads();
+    ptx::cluster_wait();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *reinterpret_cast<const uint32_t *>(at(kTmemSlotAt));
     const uint32_t tmem_acc = tmem_base;             // columns [0, 256)
-    const uint32_t tmem_a = tmem_base + kAccCols;    // kAStages x 32 columns
+    const uint32_t tmem_a = tmem_base + kAccCols;    // kASteps x 2 x 32 columns
 
     bool ok = true;
+    auto step_done = [&](uint32_t step) { return ptx::mbar_wait_suspended(bar(kBarDone + step % kBarRing), (step / kBarRing) & 1u); };
 
     if (warp == 0) {
         // ============================ TMA producer ============================
-        if (lane == 0) {
-            // the f16 activations and T come from the pre-pass, which may still be running: this
-            // kernel is its programmatic dependent (the dequantisers start on the weights at once)
-            ptx::pdl_wait();
-            uint32_t cnt = 0;
-            int32_t b_read = -1;  // the last adapter stage so far
-            for (uint32_t seg = 0; seg < wl.n_seg && ok; ++seg) {
-                uint32_t tile, kb, ke;
-                wl.get(seg, tile, kb, ke);
-                const uint32_t tile_m0 = (tile % p.m_tiles) * BN, n0 = ((tile / p.m_tiles) * 2 + rank) * BM;
-                const uint32_t m0 = tile_m0 + rank * (tile_columns(p.M, tile_m0) / 2);  // (the box is longer; the MMAs take what counts)
-                // the adapter's stages follow a tile's last main stage
-                const uint32_t k_end = ke == k_stages ? k_stages + lora_stages : ke;
-                for (uint32_t ks = kb; ks < k_end; ++ks, ++cnt) {
-                    const bool main_stage = ks < k_stages;
-                    const uint32_t j = main_stage ? 0 : ks - k_stages;
-                    const bool new_b = !main_stage && (j & 1u) == 0;  // a chunk of B serves the hi and the lo half of T
-                    // the slot's last reader is done, and the last one of the B tile's only place
-                    int32_t last = (int32_t)cnt - kXStages;
-                    if (new_b && b_read > last) last = b_read;
-                    if (last >= 0 && !ptx::mbar_wait_suspended(bar(kBarDone + last % kAStages), ((uint32_t)last / kAStages) & 1u)) {
-                        ok = false;
-                        break;
-                    }
-                    const uint32_t dst = (own | kXAt) + (cnt % kXStages) * kXTileBytes;
-                    const uint32_t full = bar(kBarFull + cnt % kAStages), pair_full = ptx::map_to_rank(full, 0);
-                    if (main_stage) {
-                        if (rank == 0) ptx::mbar_arrive_expect_tx(full, 2 * kXTileBytes);
-                        ptx::tma_load_2d_pair(dst, &tmap_x, (int32_t)(ks * BK), (int32_t)m0, pair_full);
-                    } else {
-                        // adapter stage: a tile of T in the activations' ring slot and the
-                        // matching 128 x 64 tile of LoRA B (ranks beyond the adapter's read as
-                        // zero) as the MMA's other shared-memory operand
-                        b_read = (int32_t)cnt;
-                        if (rank == 0) ptx::mbar_arrive_expect_tx(full, 2 * (kXTileBytes + (new_b ? kLoraTileBytes : 0)));
-                        ptx::tma_load_2d_pair(dst, &tmap_t, (int32_t)(((j & 1u) * p.lora_chunks + j / 2) * BK), (int32_t)m0, pair_full);
-                        if (new_b) ptx::tma_load_2d_pair(own | kLoraAt, &tmap_b, (int32_t)(j / 2 * BK), (int32_t)n0, pair_full);
-                    }
+        // The warp stays together and elects the thread that asks (see the issuer): a lane on its own in a branch took 300 to
+        // 440 cycles a stage for its waits, arrivals and requests, which made this warp what every stage waited for.
+        // The f16 activations and T come from the pre-pass, which may still be running: this
+        // kernel is its programmatic dependent (the dequantisers start on the weights at once).
+        ptx::pdl_wait();
+        uint32_t step = 0, slot = 0;
+        uint32_t user[X::kSlots];  // of the slots from the next one on: the last step that used it, plus one
+        #pragma unroll
+        for (uint32_t i = 0; i < X::kSlots; ++i) user[i] = 0;
+        auto take = [&]() -> uint32_t {  // the next slot, once its last user is done
+            if (user[0]) ok = step_done(user[0] - 1);
+            #pragma unroll
+            for (uint32_t i = 0; i + 1 < X::kSlots; ++i) user[i] = user[i + 1];
+            user[X::kSlots - 1] = step + 1;
+            const uint32_t at = own | X::place(slot);
+            slot = X::next(slot);
+            return at;
+        };
+        const uint32_t full0 = bar(kBarFull), pair_full0 = ptx::map_to_rank(full0, 0), tile_bytes = p.box_rows * (BK * 2);
+        for (uint32_t seg = 0; seg < wl.n_seg && ok; ++seg) {
+            uint32_t tile, kb, ke;
+            wl.get(seg, tile, kb, ke);
+            const uint32_t tile_m0 = (tile % p.m_tiles) * BN, n0 = ((tile / p.m_tiles) * 2 + rank) * BM;
+            const uint32_t m0 = tile_m0 + rank * (tile_columns<BN>(p.M, tile_m0) / 2);  // (the box may be longer; the MMAs take what counts)
+            for (uint32_t ks = kb; ks < ke && ok; ks += 2, ++step) {
+                const uint32_t dst = take();
+                if (!ok) break;
+                const bool two = ks + 1 < ke;
+                const uint32_t b = 8u * (step % kBarRing);
+                if (ptx::elect_one()) {
+                    if (rank == 0) ptx::mbar_arrive_expect_tx(full0 + b, (two ? 4u : 2u) * tile_bytes);
+                    ptx::tma_load_2d_pair(dst, &tmap_x, (int32_t)(ks * BK), (int32_t)m0, pair_full0 + b);
+                    if (two) ptx::tma_load_2d_pair(dst + X::kTile, &tmap_x, (int32_t)((ks + 1) * BK), (int32_t)m0, pair_full0 + b);
                 }
+                __syncwarp();
             }
-            if (!ok) NF4_REPORT_FAILURE(g_prefill_error, g_prefill_error_host, 1);
+            // the adapter's steps follow a tile's last main step: a slot for the 128 x 64 tile of LoRA B (ranks beyond the
+            // adapter's read as zero), one for the halves of T
+            for (uint32_t j = 0; ke == k_stages && j < p.lora_chunks && ok; ++j, ++step) {
+                const uint32_t dst_b = take(), dst = ok ? take() : 0u;
+                if (!ok) break;
+                const uint32_t b = 8u * (step % kBarRing);
+                if (ptx::elect_one()) {
+                    if (rank == 0) ptx::mbar_arrive_expect_tx(full0 + b, 2 * (2 * tile_bytes + kLoraTileBytes));
+                    ptx::tma_load_2d_pair(dst_b, &tmap_b, (int32_t)(j * BK), (int32_t)n0, pair_full0 + b);
+                    ptx::tma_load_2d_pair(dst, &tmap_t, (int32_t)(j * BK), (int32_t)m0, pair_full0 + b);
+                    ptx::tma_load_2d_pair(dst + X::kTile, &tmap_t, (int32_t)((p.lora_chunks + j) * BK), (int32_t)m0, pair_full0 + b);
+                }
+                __syncwarp();
+            }
         }
+        if (!ok && lane == 0) NF4_REPORT_FAILURE(g_prefill_error, g_prefill_error_host, 1);
     } else if (warp == 1) {
         // ============================= MMA issuer =============================
-        // One thread of the even CTA issues the pair's MMAs: per stage one wait, four MMAs, one commit.  The
+        // One thread of the even CTA issues the pair's MMAs: per step one wait, eight MMAs, one commit.  The
         // warp stays together and elects the thread where it issues, so that addresses and descriptors are
         // uniform registers; one lane on its own in a branch spent 77 cycles on each MMA, which takes 128.
         if (rank == 0) {
-            uint32_t cnt = 0;
+            uint32_t step = 0, slot = 0;
+            auto step_full = [&]() { return ptx::mbar_wait_suspended(bar(kBarFull + step % kBarRing), (step / kBarRing) & 1u); };
             for (uint32_t seg = 0; seg < wl.n_seg && ok; ++seg) {
                 uint32_t tile, kb, ke;
                 wl.get(seg, tile, kb, ke);
-                const uint32_t columns = tile_columns(p.M, (tile % p.m_tiles) * BN);
+                const uint32_t columns = tile_columns<BN>(p.M, (tile % p.m_tiles) * BN);
                 const uint32_t idesc_main = ptx::f16_idesc(0, 2 * BM, columns, false, false);  // f16 x f16
                 const uint32_t idesc_lora = ptx::f16_idesc(1, 2 * BM, columns, false, false);  // bf16 x bf16
                 // the epilogues must have read the previous segment out of the accumulators
                 ok = ptx::mbar_wait_suspended(bar(kBarAccEmpty), (seg & 1u) ^ 1u);
-                for (uint32_t ks = kb; ks < ke && ok; ++ks, ++cnt) {
-                    const uint32_t s = cnt % kAStages;
-                    const uint64_t bdesc = ptx::sw128_desc(kXAt + (cnt % kXStages) * kXTileBytes);
-                    const uint32_t a_cols = tmem_a + s * kAStageCols;
-                    ok = ptx::mbar_wait_suspended(bar(kBarFull + s), (cnt / kAStages) & 1u);
+                for (uint32_t ks = kb; ks < ke && ok; ks += 2, ++step, slot = X::next(slot)) {
+                    const uint64_t bdesc = ptx::sw128_desc(X::place(slot));
+                    const uint32_t a_cols = tmem_a + step % kASteps * (2 * kStageCols);
+                    ok = step_full();
                     if (!ok) break;
                     ptx::tc_fence_after();
                     if (ptx::elect_one()) {
                         // 16 k = 8 TMEM columns of the weight stage = 32 bytes inside the
                         // activation tile's swizzled row (+2 in the encoded address)
                         ptx::mma_ts_f16_pair(tmem_acc, a_cols, bdesc, idesc_main, ks != kb ? 1u : 0u);
-                        ptx::mma_ts_f16_pair(tmem_acc, a_cols + 8, bdesc + 2, idesc_main, 1u);
-                        ptx::mma_ts_f16_pair(tmem_acc, a_cols + 16, bdesc + 4, idesc_main, 1u);
-                        ptx::mma_ts_f16_pair(tmem_acc, a_cols + 24, bdesc + 6, idesc_main, 1u);
-                        ptx::tc_commit_pair(bar(kBarDone + s));
+                        #pragma unroll
+                        for (uint32_t i = 1; i < 4; ++i) ptx::mma_ts_f16_pair(tmem_acc, a_cols + 8 * i, bdesc + 2 * i, idesc_main, 1u);
+                        if (ks + 1 < ke) {
+                            #pragma unroll
+                            for (uint32_t i = 0; i < 4; ++i)
+                                ptx::mma_ts_f16_pair(tmem_acc, a_cols + kStageCols + 8 * i, bdesc + (X::kTile >> 4) + 2 * i, idesc_main, 1u);
+                        }
+                        ptx::tc_commit_pair(bar(kBarDone + step % kBarRing));
                     }
                     __syncwarp();
                 }
-                for (uint32_t j = 0; ke == k_stages && j < lora_stages && ok; ++j, ++cnt) {
-                    const uint32_t s = cnt % kAStages;
-                    const uint32_t left = p.rank - j / 2 * 64, nk16 = ((left < 64 ? left : 64) + 15) / 16;
-                    const uint64_t adesc = ptx::sw128_desc(kLoraAt);
-                    const uint64_t bdesc = ptx::sw128_desc(kXAt + (cnt % kXStages) * kXTileBytes);
-                    ok = ptx::mbar_wait_suspended(bar(kBarFull + s), (cnt / kAStages) & 1u);
+                for (uint32_t j = 0; ke == k_stages && j < p.lora_chunks && ok; ++j, ++step) {
+                    const uint32_t left = p.rank - j * 64, nk16 = ((left < 64 ? left : 64) + 15) / 16;
+                    const uint64_t adesc = ptx::sw128_desc(X::place(slot));
+                    slot = X::next(slot);
+                    const uint64_t bdesc = ptx::sw128_desc(X::place(slot));
+                    slot = X::next(slot);
+                    ok = step_full();
                     if (!ok) break;
                     ptx::tc_fence_after();
                     if (ptx::elect_one()) {
+                        for (uint32_t i = 0; i < nk16; ++i) ptx::mma_ss_f16_pair(tmem_acc, adesc + 2 * i, bdesc + 2 * i, idesc_lora, 1u);
                         for (uint32_t i = 0; i < nk16; ++i)
-                            ptx::mma_ss_f16_pair(tmem_acc, adesc + 2 * i, bdesc + 2 * i, idesc_lora, 1u);
-                        ptx::tc_commit_pair(bar(kBarDone + s));
+                            ptx::mma_ss_f16_pair(tmem_acc, adesc + 2 * i, bdesc + (X::kTile >> 4) + 2 * i, idesc_lora, 1u);
+                        ptx::tc_commit_pair(bar(kBarDone + step % kBarRing));
                     }
                     __syncwarp();
                 }
@@ -412,8 +550,6 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         // (bf16) or a quarter of it (f32) goes through one staging buffer at a time, and the accumulator is
         // handed back before the last values are stored; their TMA store then overlaps the next tile's MMAs.
         const uint32_t set = warp >= kFirstEpilogueWarpB ? 1u : 0u;
-        const uint32_t q = warp & 3u;  // TMEM lane quarter this warp may touch
-        const uint32_t row_in_tile = q * 32 + lane;
         const uint32_t epi_thread = set * 128 + (warp - (set ? kFirstEpilogueWarpB : 2)) * 32 + lane;
         const uint32_t epi_leader = (warp == 2 && lane == 0);
         const uint32_t acc_lane = tmem_acc + ((q * 32) << 16);
@@ -429,6 +565,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         float *own_partial = p.partial + (size_t)blockIdx.x * (BM * BN) + row_in_tile;
         for (uint32_t seg = 0; seg < wl.n_seg && ok; ++seg) {
             const uint32_t i = seg;  // the accumulator's barriers alternate per segment
+            const bool more = seg + 1 < wl.n_seg;  // (what nobody waits for must not be under way when the other CTA ends)
             uint32_t tile, kb, ke;
             wl.get(seg, tile, kb, ke);
             const uint32_t n0 = ((tile / p.m_tiles) * 2 + rank) * BM, m0 = (tile % p.m_tiles) * BN;
@@ -452,7 +589,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 }
                 ptx::tc_fence_before();
                 __syncwarp();
-                if (lane == 0) ptx::mbar_arrive_cluster(acc_empty);
+                if (lane == 0 && more) ptx::mbar_arrive_cluster(acc_empty);
                 asm volatile("bar.sync 1, 256;" ::: "memory");
                 if (epi_leader && p.split <= 1) {
                     __threadfence();
@@ -464,15 +601,15 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             // the one that began the tile; a CTA's helpers have its own rank
             uint32_t first_helper = pair;
             if (kb != 0) {
-                const uint64_t all = (uint64_t)wl.sk_tiles * k_stages, t0 = (uint64_t)tile * k_stages;
+                const uint64_t t0 = (uint64_t)tile * k_stages;
                 do {
                     --first_helper;
-                } while (first_helper > 0 && WorkList::range_begin(all, first_helper, pairs) > t0);
+                } while (first_helper > 0 && wl.part_begin(p.share_q, p.share_r, first_helper, pairs) > t0);
             }
             // the rows' factors go to shared memory while the MMAs still run: a global load per
             // value inside the read-out would wait for L2 every time (the L1 left beside 227 KB
             // of shared memory is small and the dequantisers stream through it)
-            row_scales[epi_thread] = m0 + epi_thread < p.M ? __ldg(p.row_scale + m0 + epi_thread) : 1.0f;
+            if (epi_thread < BN) row_scales[epi_thread] = m0 + epi_thread < p.M ? __ldg(p.row_scale + m0 + epi_thread) : 1.0f;
             ok = ptx::mbar_wait_suspended(bar(kBarAccFull), i & 1u);
             if (!ok) break;
             ptx::tc_fence_after();
@@ -544,7 +681,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                         // this warp's part of the accumulator is read: hand it back to the MMA threads
                         ptx::tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) ptx::mbar_arrive_cluster(acc_empty);
+                        if (lane == 0 && more) ptx::mbar_arrive_cluster(acc_empty);
                     }
                     stage_chunk(vb, col_of(k + 1));
                     if ((k + 2) % kPerPass == 0) {
@@ -635,7 +772,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 auto hand_back = [&]() {  // this warp's part of the accumulator is read
                     ptx::tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) ptx::mbar_arrive_cluster(acc_empty);
+                    if (lane == 0 && more) ptx::mbar_arrive_cluster(acc_empty);
                 };
                 const uint32_t at = set * 64;  // a set's columns of a half: four pieces of 16 weight rows x 32 columns
                 uint32_t w[2][8];
@@ -646,7 +783,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                     stage(at + (c >> 1) * 32, c & 1u, w[0]);
                 }
                 send(m0);
-                if (m0 + kStageRows < p.M) {
+                if (BN > kStageRows && m0 + kStageRows < p.M) {
                     #pragma unroll
                     for (uint32_t c = 0; c < 2; ++c) convert(kStageRows + at, c, w[c]);
                     buffer_free();
@@ -664,90 +801,44 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 }
             }
         }
-        if (epi_leader) ptx::tma_store_wait<0>();
+        if (epi_leader) ptx::tma_store_wait_read<0>();  // (what was read is on its way; the kernel's end waits for it)
         if (!ok && lane == 0) NF4_REPORT_FAILURE(g_prefill_error, g_prefill_error_host, 3);
     } else if (warp >= kFirstExpanderWarp && warp < kFirstEpilogueWarpB) {
         // ============================ dequantisers ============================
-        // Four groups of four warps; group g takes the main stages (adapter stages need no
-        // dequantiser) whose running number over this CTA's tiles is g modulo 4.
+        // Four groups of four warps; groups 0 and 1 take the two stages of the even steps (counted over this CTA's tiles),
+        // groups 2 and 3 those of the odd ones.
         // Within a group the warp's number modulo 4 names the TMEM lane quarter it may write, and
         // the lane the weight row: 32 packed bytes + the scale in, 64 f16 values out, stored as
-        // 32 TMEM columns (two f16 per cell, even k in the low half) of the stage's ring slot.
-        const uint32_t group = (warp - kFirstExpanderWarp) >> 2;
-        const uint32_t q = warp & 3u;
-        const uint32_t row_in_tile = q * 32 + lane;
-        if (PERK) ptx::pdl_wait();  // the kernel ahead repacks the weight, and completes after the pre-pass
+        // 32 TMEM columns (two f16 per cell, even k in the low half) of the stage's place in the ring.
         const uint32_t lane_word = lane * 4u | kTableAt | own;  // bytes {4 lane, 0, 1, rank}: see level_pair
-        // block scales are used divided by a power of two (see weight_exponent)
-        // ... and enter the product as f16: one multiplication from the loaded value.  (A u8 code's scale is
-        // (code / 255) * scale of scales; dividing once instead of per code moves it by an ulp of f32.)
-        const float w_down = ldexpf(1.0f, -weight_exponent(p.absmax, p.scale_codes, p.scale_of_scales));
-        const float scale_unit = p.absmax ? w_down : __fdiv_rn(__ldg(p.scale_of_scales), 255.0f) * w_down;
-        const uint32_t blocks_per_row = p.K / 64;
         const uint32_t lane_base = tmem_a + ((q * 32) << 16);
 
-        // The scales of this group's next kDepth stages are in flight.  A position is walked, not divided out.
-        constexpr int kDepth = 3;
-        struct Pos {
-            uint32_t seg, ks, ke;  // segment, stage in tile, the segment's end
-            uint32_t before;       // stages before the segments after this one
-            size_t row;            // index of the weight row's first scale (PERK: of the pair for this lane)
-        } ahead{0, 0, 0, 0, 0};
-        auto enter = [&]() {  // the first main stage of this group in segment ahead.seg or a later one
-            for (; ahead.seg < wl.n_seg; ++ahead.seg) {
-                uint32_t tile, kb;
-                wl.get(ahead.seg, tile, kb, ahead.ke);
-                ahead.ks = kb + ((group - ahead.before) & (kExpanderGroups - 1u));
-                ahead.before += (ahead.ke - kb) + (ahead.ke == k_stages ? lora_stages : 0);
-                if (ahead.ks < ahead.ke) {
-                    // (rows beyond the last read its scales; nobody stores what comes of them)
-                    const uint32_t n0 = ((tile / p.m_tiles) * 2 + rank) * BM;
-                    ahead.row = PERK ? (size_t)(min(n0 + q * 32, p.N - 1) >> 6) * (p.K / 2) + lane
-                                     : (size_t)min(n0 + row_in_tile, p.N - 1) * blocks_per_row;
-                    return;
-                }
-            }
-        };
-        // The scale of the next stage as loaded: f32 bits, a u8 code, or (PERK: the warp's 32 weight rows lie in
-        // one 64-block of the original rows) this lane's pair of the stage's 128-byte line of f16 scales.
-        // Nothing is computed from it here: that would wait for the load, the latency the pipeline hides.
-        auto fetch = [&]() -> uint32_t {
-            if (ahead.seg >= wl.n_seg) return 0;
-            uint32_t v;
-            if constexpr (PERK) v = __ldg(reinterpret_cast<const uint32_t *>(p.scales_t) + ahead.row + (size_t)ahead.ks * (BK / 2));
-            else v = p.absmax ? __float_as_uint(__ldg(p.absmax + ahead.row + ahead.ks)) : __ldg(p.scale_codes + ahead.row + ahead.ks);
-            ahead.ks += kExpanderGroups;
-            if (ahead.ks >= ahead.ke) {
-                ++ahead.seg;
-                enter();
-            }
-            return v;
-        };
-        enter();
-        uint32_t scales[kDepth];
-        #pragma unroll
-        for (int d = 0; d < kDepth; ++d) scales[d] = fetch();
-        // The codes come in blocks of four stages, one for each group (the first and the last block of a segment
-        // may lack some).  A group has every fourth stage, the adapter's included (nothing to write there, but its turn
-        // on the barriers): then it is never two rounds of Done ahead, where a parity would be the wrong round's.  Every warp goes through every block: it waits for it, takes its row's 32 bytes
-        // of its stage, and gives the slot back.
-        uint32_t before = 0, block = 0;  // stages before the segment, blocks so far
-        const uint32_t row_at = (own | kCodesAt) + row_in_tile * 128u;
+        // A group has every other step, the adapter's and the missing half of an odd last one included (nothing to write
+        // there, but its turn on the barriers): then it is never two rounds of Done ahead, where a parity would be the wrong
+        // round's.
+        uint32_t before = 0, blocks = 0;  // steps, and main ones, before the segment
+        const uint32_t swizzle = (row_in_tile >> 1) & 3u, row_at = (own | kCodesAt) + row_in_tile * 64u;
+        const uint32_t chunk0 = row_at + (((half * 2) ^ swizzle) << 4), chunk1 = row_at + (((half * 2 + 1) ^ swizzle) << 4);
         const uint32_t full0 = ptx::map_to_rank(bar(kBarFull), 0);
+        auto columns_free = [&](uint32_t step) { return step < kASteps || step_done(step - kASteps); };
+        auto nothing = [&](uint32_t step) {
+            ok = columns_free(step);
+            __syncwarp();
+            if (ok && lane == 0) ptx::mbar_arrive_cluster(full0 + 8u * (step % kBarRing));
+        };
         for (uint32_t seg = 0; seg < wl.n_seg && ok; ++seg) {
             uint32_t tile, kb, ke;
             wl.get(seg, tile, kb, ke);
-            const uint32_t turn = (group + kb - before) & (kExpanderGroups - 1u);  // this group's stage of a block
-            const uint32_t chunk0 = row_at + (((turn * 2) ^ (row_in_tile & 7u)) << 4), chunk1 = row_at + (((turn * 2 + 1) ^ (row_in_tile & 7u)) << 4);
-            for (uint32_t ks = (kb & ~(kExpanderGroups - 1u)) + turn; (ks & ~(kExpanderGroups - 1u)) < ke; ks += kExpanderGroups, ++block) {
-                const uint32_t slot = block % kCodeSlots;
+            const uint32_t steps = (ke - kb + 1) / 2;
+            for (uint32_t j = (odd - before) & 1u; j < steps && ok; j += 2) {
+                const uint32_t step = before + j, block = blocks + j, slot = block % kCodeSlots;
                 if (!ptx::mbar_wait_suspended(bar(kBarCFull + slot), (block / kCodeSlots) & 1u)) {
                     ok = false;
                     break;
                 }
-                const bool mine = ks >= kb && ks < ke;
-                if (!mine) {
+                if (kb + 2 * j + half >= ke) {  // an odd last step's second half
                     if (lane == 0) ptx::mbar_arrive(bar(kBarCEmpty + slot));
+                    nothing(step);
                     continue;
                 }
                 uint32_t w[8];
@@ -755,79 +846,91 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                              : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(chunk0 + slot * kCodeTileBytes) : "memory");
                 asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
                              : "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "r"(chunk1 + slot * kCodeTileBytes) : "memory");
-                const uint32_t cnt = before + ks - kb, s = cnt % kAStages;
                 uint32_t scale2 = scales[0];
+                if constexpr (SCALES == kScalesTma) {
+                    const uint32_t ks = kb + 2 * j + half, at = (own | scales_place(slot)) + row_in_tile * 16u;
+                    if (p.absmax) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(scale2) : "r"(at + (ks & 3u) * 4u) : "memory");
+                    else asm volatile("ld.shared.u8 %0, [%1];" : "=r"(scale2) : "r"(at + (ks & 15u)) : "memory");
+                }
+                if constexpr (PERK) scale2 = (own | scales_place(slot)) + (q >> 1) * (2 * BK * 2) + half * (BK * 2);
                 if constexpr (!PERK) {
                     const __half2 h = __float2half2_rn((p.absmax ? __uint_as_float(scale2) : (float)scale2) * scale_unit);
                     scale2 = *reinterpret_cast<const uint32_t *>(&h);
                 }
-                #pragma unroll
-                for (int d = 0; d + 1 < kDepth; ++d) scales[d] = scales[d + 1];
-                scales[kDepth - 1] = fetch();
+                if constexpr (SCALES == kScalesLoaded) {
+                    #pragma unroll
+                    for (int d = 0; d + 1 < kDepth; ++d) scales[d] = scales[d + 1];
+                    scales[kDepth - 1] = fetch();
+                }
                 uint32_t lo[16], hi[16];
-                expand_half<PERK>(w, scale2, 0, lane_word, lo);
-                expand_half<PERK>(w + 4, scale2, 16, lane_word, hi);
-                if (cnt >= kAStages && !ptx::mbar_wait_suspended(bar(kBarDone + s), ((cnt / kAStages) & 1u) ^ 1u)) {
+                expand_half<PERK>(w, scale2, lane_word, lo);
+                expand_half<PERK>(w + 4, scale2 + (PERK ? BK : 0), lane_word, hi);
+                if (!columns_free(step)) {
                     ok = false;
                     break;
                 }
                 ptx::tc_fence_after();
-                tmem_st32(lane_base + s * kAStageCols, lo, hi);
+                tmem_st32(lane_base + (step % kASteps * 2 + half) * kStageCols, lo, hi);
                 ptx::tmem_wait_st();
                 ptx::tc_fence_before();
                 __syncwarp();
                 if (lane == 0) {
-                    ptx::mbar_arrive_cluster(full0 + 8u * s);
+                    ptx::mbar_arrive_cluster(full0 + 8u * (step % kBarRing));
                     // The slot goes back now that what was read from it has been used.  Right after the loads
                     // were issued is too early: the next copy, of another proxy, was seen to overtake them.
                     ptx::mbar_arrive(bar(kBarCEmpty + slot));
                 }
             }
-            before += ke - kb;
+            before += steps;
+            blocks += steps;
             if (ke != k_stages) continue;
-            for (uint32_t cnt = before + ((group - before) & (kExpanderGroups - 1u)); cnt < before + lora_stages && ok; cnt += kExpanderGroups) {
-                const uint32_t s = cnt % kAStages;
-                ok = cnt < kAStages || ptx::mbar_wait_suspended(bar(kBarDone + s), ((cnt / kAStages) & 1u) ^ 1u);
-                __syncwarp();
-                if (ok && lane == 0) ptx::mbar_arrive_cluster(full0 + 8u * s);
-            }
-            before += lora_stages;
+            for (uint32_t j = (odd - before) & 1u; j < p.lora_chunks && ok; j += 2) nothing(before + j);
+            before += p.lora_chunks;
         }
         if (!ok && lane == 0) NF4_REPORT_FAILURE(g_prefill_error, g_prefill_error_host, 4);
     }
 
-    if (warp == kCodeWarp && lane == 0) {
+    if (warp == kCodeWarp) {
         // ========================= packed codes =========================
-        // Blocks of four k-stages of this CTA's 128 weight rows; the L2 is asked for a block a few ahead of
-        // its load (weights that nobody has touched yet come from HBM).
         if (PERK) ptx::pdl_wait();
-        constexpr uint32_t kAhead = 6;
-        uint32_t block = 0;
+        uint32_t slot = asked % kCodeSlots, round = asked / kCodeSlots;
         for (uint32_t seg = 0; seg < wl.n_seg && ok; ++seg) {
             uint32_t tile, kb, ke;
             wl.get(seg, tile, kb, ke);
             const int32_t n0 = (int32_t)(((tile / p.m_tiles) * 2 + rank) * BM);
-            const uint32_t b0 = kb / kCodeStages, b1 = (ke + kCodeStages - 1) / kCodeStages;
-            for (uint32_t b = b0; b < min(b1, b0 + kAhead); ++b) ptx::tma_prefetch_2d(&tmap_w, (int32_t)(b * 128), n0);
-            for (uint32_t b = b0; b < b1; ++b, ++block) {
-                const uint32_t slot = block % kCodeSlots;
-                if (b + kAhead < b1) ptx::tma_prefetch_2d(&tmap_w, (int32_t)((b + kAhead) * 128), n0);
-                if (!ptx::mbar_wait_suspended(bar(kBarCEmpty + slot), ((block / kCodeSlots) & 1u) ^ 1u)) {
-                    ok = false;
-                    break;
+            if ((PERK || seg) && ptx::elect_one())
+                for (uint32_t k = kb; k < min(ke, kb + kAhead * kUnit); k += kUnit) ask_l2(k, n0);
+            __syncwarp();
+            for (uint32_t ks = kb; ks < ke; ks += 2) {
+                const uint32_t ahead = ks + kAhead * kUnit;
+                const bool to_l2 = (ks - kb) % kUnit == 0 && ahead < ke;
+                if (seg == 0 && ks < kb + 2 * asked) {
+                    if (to_l2 && ptx::elect_one()) ask_l2(ahead, n0);
+                    __syncwarp();
+                    continue;
                 }
-                ptx::mbar_arrive_expect_tx(bar(kBarCFull + slot), kCodeTileBytes);
-                ptx::tma_load_2d((own | kCodesAt) + slot * kCodeTileBytes, &tmap_w, (int32_t)(b * 128), n0, bar(kBarCFull + slot));
+                ok = ptx::mbar_wait_suspended(bar(kBarCEmpty + slot), (round & 1u) ^ 1u);
+                if (!ok) break;
+                if (ptx::elect_one()) {
+                    ask_codes(ks, n0, slot);
+                    if (to_l2) ask_l2(ahead, n0);
+                }
+                __syncwarp();
+                if (++slot == kCodeSlots) {
+                    slot = 0;
+                    ++round;
+                }
             }
         }
-        if (!ok) NF4_REPORT_FAILURE(g_prefill_error, g_prefill_error_host, 7);
+        if (!ok && lane == 0) NF4_REPORT_FAILURE(g_prefill_error, g_prefill_error_host, 7);
     }
 
     if (!ok) ptx::let_flights_land();
     __syncwarp();
     // neither CTA leaves, or gives its tensor memory back, while the other may still signal it
     ptx::tc_fence_before();
-    ptx::cluster_sync_all();
+    ptx::cluster_arrive_relaxed();
+    ptx::cluster_wait();
     if (warp == 1) {
         ptx::tc_fence_after();
         ptx::tmem_dealloc_pair(tmem_base, kTmemCols);
@@ -839,7 +942,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
 // CTA's 128 weight rows, a lane four of them.  One pair that collected the others' sums in its read-out, a helper and
 // sixteen columns at a time, took 10 us (300 x 3584 x 3584), 14 (512 x 4096 x 4096, f32) and 23 (99 x 20288 x 512, twelve
 // helpers); a launch of its own has all SMs' loads in flight, and no CTA waits for another one.
-template <bool YF32>
+template <int BN, bool YF32>
 __global__ void __launch_bounds__(256)
 sum_parts_kernel(const float *__restrict__ partial, uint32_t split, uint32_t m_tiles, uint32_t M, uint32_t N, const float *__restrict__ row_scale,
                  const float *__restrict__ bias, void *__restrict__ y, uint64_t ldy) {
@@ -1084,19 +1187,23 @@ namespace {
 // pairs * dp_rounds tiles go out whole.  With a tile count that is a multiple of the pairs nothing
 // is split.  Otherwise the last round of whole tiles would leave most pairs idle, so the last full round and
 // the remainder are divided by stages instead.  Fewer tiles than pairs: what of three takes the shortest by the times
-// measured (a stage 0.28 us however many columns it has): whole tiles, read out in 3 us; `split` pairs to a tile, whose
-// sums a kernel of its own adds (dump 3.5, launch and sum 4.5 us); or divided by stages, every pair 24 at least, with a tile's last
-// pair collecting (3 us of dump, and 2 a helper).
+// measured (a stage 0.28 us in wide tiles, 0.2 in narrow ones, however many columns it has): whole tiles, read out in 3 us; `split` pairs
+// to a tile, whose sums a kernel of its own adds (dump 3.5, launch and sum 4.5 us); or divided by stages, every pair 24 at least, with a
+// tile's last pair collecting (3 us of dump, and 2 a helper).
 struct Sharing {
+    uint32_t bn;  // activation rows of a tile
     uint32_t pairs, sk_tiles, dp_rounds, split;
+    uint64_t cost;  // ns, if there are fewer tiles than pairs
 };
-Sharing share_tiles(uint64_t rows, uint64_t d_in, uint64_t d_out) {
-    const uint64_t tiles = ((rows + BN - 1) / BN) * ((d_out + 2 * BM - 1) / (2 * BM)), ks = d_in / BK;
-    Sharing sh;
+Sharing share_tiles_of(uint32_t bn, uint64_t rows, uint64_t d_in, uint64_t d_out) {
+    const uint64_t tiles = ((rows + bn - 1) / bn) * ((d_out + 2 * BM - 1) / (2 * BM)), ks = d_in / BK;
+    Sharing sh{};
+    sh.bn = bn;
     sh.split = 1;
     uint64_t pairs = kNumSMs / 2;
     if (tiles < pairs) {
-        constexpr uint64_t kStage = 280, kReadOut = 3000, kDump = 3500, kSum = 4500, kHelper = 2000;  // ns
+        const bool narrow = bn < 256;
+        const uint64_t kStage = narrow ? 200 : 280, kReadOut = narrow ? 2000 : 3000, kDump = narrow ? 2500 : 3500, kSum = 4500, kHelper = 2000;
         const uint64_t by_stages = tiles * ks / 24, shared = by_stages < pairs ? by_stages : pairs;
         uint64_t least = ks * kStage + kReadOut, most = pairs / tiles;
         if (shared > tiles) {
@@ -1113,13 +1220,13 @@ Sharing share_tiles(uint64_t rows, uint64_t d_in, uint64_t d_out) {
                 sh.split = (uint32_t)s;
             }
         }
-        pairs = sh.split ? tiles * sh.split : shared;
+        sh.cost = least;
         if (sh.split > 1) {
-            sh.pairs = (uint32_t)pairs;
+            sh.pairs = (uint32_t)(tiles * sh.split);
             sh.sk_tiles = (uint32_t)tiles;
-            sh.dp_rounds = 0;
             return sh;
         }
+        pairs = sh.split ? tiles : shared;
         sh.split = 1;
     }
     sh.pairs = (uint32_t)pairs;
@@ -1130,6 +1237,20 @@ Sharing share_tiles(uint64_t rows, uint64_t d_in, uint64_t d_out) {
         sh.dp_rounds = tiles / pairs >= 1 ? (uint32_t)(tiles / pairs - 1) : 0u;
         sh.sk_tiles = (uint32_t)(tiles - (uint64_t)sh.dp_rounds * pairs);
     }
+    return sh;
+}
+// Up to 128 rows there is one narrow tile where there would be a wide one.  More rows take narrow tiles where a pair gets one whole
+// tile at most and that is the shorter way: 512 x 4096 x 4096 in 64 whole tiles instead of 32, two pairs to each and their sums added.
+Sharing share_tiles(uint64_t rows, uint64_t d_in, uint64_t d_out, bool wide_only = false) {
+    if (rows <= 128) return share_tiles_of(128, rows, d_in, d_out);
+    const Sharing wide = share_tiles_of(256, rows, d_in, d_out);
+    if (wide_only || !wide.cost) return wide;
+    const uint64_t tiles = ((rows + 127) / 128) * ((d_out + 2 * BM - 1) / (2 * BM)), cost = d_in / BK * 200 + 2000;
+    if (tiles > kNumSMs / 2 || cost >= wide.cost) return wide;
+    Sharing sh{};
+    sh.bn = 128;
+    sh.split = sh.dp_rounds = 1;
+    sh.pairs = (uint32_t)tiles;
     return sh;
 }
 
@@ -1151,7 +1272,7 @@ WorkspaceLayout workspace_layout(uint64_t rows, uint64_t d_in, uint64_t d_out, u
     w.off_flags = w.off_t + up(rows * 2ull * 64 * lora_chunks_of(lora_rank) * 2);
     const Sharing sh = share_tiles(rows, d_in, d_out);
     w.off_partial = w.off_flags + up((uint64_t)sh.pairs * 8);
-    w.bytes = w.off_partial + (sh.sk_tiles ? (uint64_t)sh.pairs * 2 * BM * BN * 4 : 0);
+    w.bytes = w.off_partial + (sh.sk_tiles ? (uint64_t)sh.pairs * 2 * BM * sh.bn * 4 : 0);
     w.off_codes_t = w.off_scales_t = w.off_a_t = w.off_b_t = 0;
     if (extra >= kFactors) {  // `lora_rank` is the rank the GEMM sees (twice the adapter's for f32 factors)
         w.off_a_t = up(w.bytes);
@@ -1213,17 +1334,21 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_o
     p.rank = a.lora_a ? a.lora_rank : 0;
     if (x_f32) p.rank *= 2;  // see repack_adapter_block
     p.lora_chunks = lora_chunks_of(p.rank);
-    p.m_tiles = (p.M + BN - 1) / BN;
+    const Sharing sh = share_tiles(p.M, p.K, p.N);
+    p.m_tiles = (p.M + sh.bn - 1) / sh.bn;
+    // (the last tile's rows, if there is no other; of several tiles the last one's box is longer than it need be)
+    p.box_rows = (p.m_tiles > 1 ? sh.bn : (p.M + 31) / 32 * 32) / 2;
     const uint64_t ldy = a.ldy ? a.ldy : a.d_out;
     if (p.N * (y_f32 ? 4u : 2u) % 16 != 0) p.y_ragged = a.y;
     p.ldy = ldy;
 
     const WorkspaceLayout wl = workspace_layout(p.M, p.K, p.N, p.rank, extra);
     if (a.workspace_bytes < wl.bytes) return fail(NF4_ERR_INVALID_ARG, "prefill_forward: workspace too small");
-    const Sharing sh = share_tiles(p.M, p.K, p.N);
     p.sk_tiles = sh.sk_tiles;
     p.dp_rounds = sh.dp_rounds;
     p.split = sh.split;
+    p.share_q = (uint64_t)sh.sk_tiles * (p.K / BK) / sh.pairs;
+    p.share_r = (uint32_t)((uint64_t)sh.sk_tiles * (p.K / BK) % sh.pairs);
     p.wait_ns = 1000000000u;
     uint8_t *ws = static_cast<uint8_t *>(a.workspace);
     __half *xh = reinterpret_cast<__half *>(ws + wl.off_xh);
@@ -1300,14 +1425,22 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_o
     NF4_TRY(activations_prepass(pre, stream));
     if (repacked) NF4_TRY(repack(true, false, !factors_first, true));
 
-    CUtensorMap map_x, map_t, map_b, map_y, map_w;
-    NF4_TRY(make_map(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.codes, p.N, p.K / 2, p.K / 2, BM, 128, CU_TENSOR_MAP_SWIZZLE_128B));
-    NF4_TRY(make_map(&map_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, xh, p.M, p.K, (uint64_t)p.K * 2, BN / 2, BK,
+    CUtensorMap map_x, map_t, map_b, map_y, map_w, map_ahead, map_s;
+    NF4_TRY(make_map(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.codes, p.N, p.K / 2, p.K / 2, BM, BK, CU_TENSOR_MAP_SWIZZLE_64B));
+    NF4_TRY(make_map(&map_ahead, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.codes, p.N, p.K / 2, p.K / 2, BM, 4 * BK, CU_TENSOR_MAP_SWIZZLE_NONE));
+    const bool tma_scales = !repacked && (p.absmax ? p.K % 256 == 0 && aligned16(p.absmax) : p.K % 1024 == 0 && aligned16(p.scale_codes));
+    map_s = map_w;
+    if (repacked) NF4_TRY(make_map(&map_s, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, p.scales_t, p.N / 64, p.K, (uint64_t)p.K * 2, BM / 64, 2 * BK, CU_TENSOR_MAP_SWIZZLE_NONE));
+    if (tma_scales && p.absmax)
+        NF4_TRY(make_map(&map_s, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, p.absmax, p.N, p.K / 64, p.K / 16, BM, 4, CU_TENSOR_MAP_SWIZZLE_NONE));
+    else if (tma_scales)
+        NF4_TRY(make_map(&map_s, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.scale_codes, p.N, p.K / 64, p.K / 64, BM, 16, CU_TENSOR_MAP_SWIZZLE_NONE));
+    NF4_TRY(make_map(&map_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, xh, p.M, p.K, (uint64_t)p.K * 2, p.box_rows, BK,
                      CU_TENSOR_MAP_SWIZZLE_128B));
     map_t = map_b = map_x;
     if (p.rank) {
         const uint32_t ld_t = 2 * 64 * p.lora_chunks;
-        NF4_TRY(make_map(&map_t, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, t, p.M, ld_t, (uint64_t)ld_t * 2, BN / 2,
+        NF4_TRY(make_map(&map_t, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, t, p.M, ld_t, (uint64_t)ld_t * 2, p.box_rows,
                          BK, CU_TENSOR_MAP_SWIZZLE_128B));
         // LoRA B [N][rank]: columns beyond the rank and rows beyond N read as zero
         NF4_TRY(make_map(&map_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, lora_b, p.N, p.rank,
@@ -1323,16 +1456,25 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_o
     auto go = [&](auto kernel) -> int32_t {
         NF4_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(kernel), (int)kDynamicSmem));
         return launch_maybe_overlapped(kernel, dim3(2 * sh.pairs), dim3(kThreads), kDynamicSmem, stream, true, map_x, map_t, map_b,
-                                       map_y, map_w, p);
+                                       map_y, map_w, map_ahead, map_s, p);
     };
-    if (repacked) NF4_TRY(y_f32 ? go(prefill_kernel<true, true>) : go(prefill_kernel<false, true>));
-    else NF4_TRY(y_f32 ? go(prefill_kernel<true, false>) : go(prefill_kernel<false, false>));
+    auto pick = [&](auto bn) -> int32_t {
+        constexpr int BN = decltype(bn)::value;
+        if (repacked) return y_f32 ? go(prefill_kernel<BN, true, kScalesPerK>) : go(prefill_kernel<BN, false, kScalesPerK>);
+        if (tma_scales) return y_f32 ? go(prefill_kernel<BN, true, kScalesTma>) : go(prefill_kernel<BN, false, kScalesTma>);
+        return y_f32 ? go(prefill_kernel<BN, true, kScalesLoaded>) : go(prefill_kernel<BN, false, kScalesLoaded>);
+    };
+    using Wide = std::integral_constant<int, 256>;
+    using Narrow = std::integral_constant<int, 128>;
+    NF4_TRY(sh.bn == 128 ? pick(Narrow{}) : pick(Wide{}));
     count_launch();
     NF4_TRY(check_cuda(cudaGetLastError(), "prefill_kernel launch"));
     if (sh.split <= 1) return NF4_OK;
-    const uint32_t columns = p.M < (uint32_t)BN ? p.M : (uint32_t)BN;
+    const uint32_t columns = p.M < sh.bn ? p.M : sh.bn;
     count_launch();
-    return launch_maybe_overlapped(y_f32 ? sum_parts_kernel<true> : sum_parts_kernel<false>, dim3((columns + 7) / 8, sh.pairs / sh.split * 2), dim3(256), 0,
+    auto sum = sh.bn == 128 ? (y_f32 ? sum_parts_kernel<128, true> : sum_parts_kernel<128, false>)
+                            : (y_f32 ? sum_parts_kernel<256, true> : sum_parts_kernel<256, false>);
+    return launch_maybe_overlapped(sum, dim3((columns + 7) / 8, sh.pairs / sh.split * 2), dim3(256), 0,
                                    stream, true, p.partial, p.split, p.m_tiles, p.M, p.N, p.row_scale, p.bias, a.y, ldy);
 }
 
@@ -1348,14 +1490,16 @@ int32_t prefill_set_host_flag(int *mapped) {
 int32_t prefill_share_plan(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t cta, uint32_t *ctas,
                            uint32_t *segments, uint32_t cap) {
     if (rows <= 16 || d_in % BK != 0 || d_in == 0 || d_out == 0) return -1;
-    const Sharing sh = share_tiles(rows, d_in, d_out);
+    const Sharing sh = share_tiles(rows, d_in, d_out, true);
     if (ctas) *ctas = 2 * sh.pairs;
     if (cta >= 2 * sh.pairs) return -1;
-    const uint32_t rank = cta / sh.pairs, m_tiles = (uint32_t)((rows + BN - 1) / BN);
+    const uint32_t rank = cta / sh.pairs, m_tiles = (uint32_t)((rows + sh.bn - 1) / sh.bn);
     PrefillParams p{};
     p.sk_tiles = sh.sk_tiles;
     p.dp_rounds = sh.dp_rounds;
     p.split = sh.split;
+    p.share_q = (uint64_t)sh.sk_tiles * (d_in / BK) / sh.pairs;
+    p.share_r = (uint32_t)((uint64_t)sh.sk_tiles * (d_in / BK) % sh.pairs);
     WorkList wl;
     wl.init(p, (uint32_t)(d_in / BK), cta % sh.pairs, sh.pairs);
     uint32_t n = 0;
