@@ -166,11 +166,10 @@ int32_t prefill_share_plan(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_
 int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_out = nullptr);
 
 // prepass.cu: the f16 copy of the activations with its rows' factors, and the adapter intermediate.
-// x [M][K] bf16 or f32 (K a multiple of 8, 16-byte aligned); a: the factor as [rank][K], or [K][rank]
-// (k_major), bf16, f16 for f32 x.  xh null: r_out alone (bf16 x).  t_out and r_out: [M][2 * 64 * ceil(rank / 64)]
+// x [M][K] bf16 or f32 (K a multiple of 8, of 64 for f32, 16-byte aligned); a: the factor as [rank][K], or [K][rank]
+// (k_major), of x's type.  xh null: r_out alone (bf16 x).  t_out and r_out: [M][2 * 64 * ceil(rank / 64)]
 // bf16, hi halves then lo; t_out the scaled intermediate the GEMM adds, r_out (may be null) x a as it is.
-// factor_of_predecessor: the kernel ahead in the stream writes the factor and touches nothing else of this one's; they
-// run side by side up to there.
+// f32: r_out null, rank <= 128 and a multiple of four; t_out holds every column twice, as an adapter's of twice the rank.
 struct PrepassArgs {
     const void *x;
     bool x_f32;
@@ -187,7 +186,6 @@ struct PrepassArgs {
     const float *scale_of_scales;
     uint32_t *flags;
     uint32_t n_flags;
-    bool factor_of_predecessor;
 };
 int32_t activations_prepass(const PrepassArgs &q, cudaStream_t stream);
 

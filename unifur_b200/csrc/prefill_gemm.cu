@@ -418,6 +418,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     }
     // The barriers of both CTAs are in place (their initialisation is fenced for the cluster by the threads that made it; a
     // release by all threads took 1.2 us), and this CTA's table.
+    __syncwarp();
     ptx::cluster_arrive_relaxed();
     ptx::tc_fence_before();
     __syncthreads();
@@ -1002,17 +1003,15 @@ struct RepackParams {
     const float *absmax;
     const uint8_t *scale_codes;
     const float *scale_of_scales;
-    const void *a, *b;          // adapter factors A [K][r], B [r][N], or null
+    const void *b;              // adapter factor B [r][N], or null
     uint8_t *codes_t;
     __half *scales_t;
-    uint16_t *a_t;
     __nv_bfloat16 *b_t;
     uint32_t K, N, r;
-    int32_t factors_out_in;     // the factors come as A [r][K], B [N][r] (else A [K][r], B [r][N])
+    int32_t factor_out_in;      // the factor comes as [N][r]
     uint32_t code_cols, code_blocks;              // CTAs of the nibbles: tiles of 128 n x 256 k
     uint32_t scale_cols, scale_blocks;            // CTAs of the scales: 32 x 32 tiles
-    uint32_t a_blocks, adapter_blocks;            // CTAs of the factors: 32 x 32 tiles, A's first
-    uint32_t wait_last;         // for the kernel ahead: at the end (else at the start)
+    uint32_t adapter_blocks;                      // CTAs of the factor: 32 x 32 tiles
 };
 
 // Nibbles.  A CTA turns 256 k x 128 n.  A thread takes eight words (8 k x 8 n) straight from global memory, all
@@ -1098,26 +1097,23 @@ __device__ __forceinline__ void repack_scales_block(const RepackParams &p, uint3
     }
 }
 
-// The adapter factors in the orientation and types the pre-pass and the GEMM read them in.
-// From A [d_in][r], B [r][d_out] of type T:
-//   bf16: b_t[n][j] = B[j][n]: exact (the pre-pass reads A as it is).
-//   f32:  a_t[j][k] = a_t[r + j][k] = f16(A[k][j]); b_t[n][j] = bf16(B[j][n]), b_t[n][r + j] = the
-//         bf16 of what that rounding left: as an adapter of rank 2 r whose intermediate holds every
-//         column twice, B enters the product with sixteen bits of mantissa.
+// The adapter factor in the orientation and type the GEMM reads it in (the pre-pass reads the other one as it is).
+// From B of type T:
+//   bf16: b_t[n][j] = B[j][n]: exact.
+//   f32:  b_t[n][j] = bf16(B[j][n]), b_t[n][r + j] = the bf16 of what that rounding left: as an adapter of rank 2 r
+//         whose intermediate holds every column twice, B enters the product with sixteen bits of mantissa.
 template <class T>
 __device__ __forceinline__ void repack_adapter_block(const RepackParams &p, uint32_t block, float (*tile)[33]) {
     constexpr bool kF32 = sizeof(T) == 4;
-    const bool is_a = block < p.a_blocks;
-    if (!is_a) block -= p.a_blocks;
-    // a tile of 32 x 32 of the result [rows][cols]: A's rows are ranks, B's columns
-    const T *src = static_cast<const T *>(is_a ? p.a : p.b);
-    const uint32_t rows = is_a ? p.r : p.N, cols = is_a ? p.K : p.r, col_tiles = (cols + 31) / 32;
+    // a tile of 32 x 32 of the result [N][r]
+    const T *src = static_cast<const T *>(p.b);
+    const uint32_t rows = p.N, cols = p.r, col_tiles = (cols + 31) / 32;
     const uint32_t r0 = block / col_tiles * 32, c0 = block % col_tiles * 32, tx = threadIdx.x & 31u, ty = threadIdx.x >> 5;
     #pragma unroll
     for (uint32_t q = ty; q < 32; q += 8) {
-        const uint32_t r = r0 + (p.factors_out_in ? q : tx), c = c0 + (p.factors_out_in ? tx : q);
+        const uint32_t r = r0 + (p.factor_out_in ? q : tx), c = c0 + (p.factor_out_in ? tx : q);
         float v = 0.0f;
-        if (r < rows && c < cols) v = (float)src[p.factors_out_in ? (size_t)r * cols + c : (size_t)c * rows + r];
+        if (r < rows && c < cols) v = (float)src[p.factor_out_in ? (size_t)r * cols + c : (size_t)c * rows + r];
         tile[r - r0][c - c0] = v;
     }
     __syncthreads();
@@ -1126,32 +1122,26 @@ __device__ __forceinline__ void repack_adapter_block(const RepackParams &p, uint
         const uint32_t r = r0 + q, c = c0 + tx;
         if (r >= rows || c >= cols) continue;
         const float v = tile[q][tx];
-        if (is_a) {
-            const uint16_t h = __half_as_ushort(__float2half_rn(v));
-            p.a_t[(size_t)r * cols + c] = h;
-            p.a_t[(size_t)(rows + r) * cols + c] = h;
-        } else {
-            const __nv_bfloat16 hi = __float2bfloat16_rn(v);
-            p.b_t[(size_t)r * (kF32 ? 2 * cols : cols) + c] = hi;
-            if (kF32) p.b_t[(size_t)r * 2 * cols + cols + c] = __float2bfloat16_rn(v - __bfloat162float(hi));
-        }
+        const __nv_bfloat16 hi = __float2bfloat16_rn(v);
+        p.b_t[(size_t)r * (kF32 ? 2 * cols : cols) + c] = hi;
+        if (kF32) p.b_t[(size_t)r * 2 * cols + cols + c] = __float2bfloat16_rn(v - __bfloat162float(hi));
     }
 }
 
 // The first code_blocks CTAs take the nibbles, the next scale_blocks the scales, the last adapter_blocks the adapter.  The
-// weight's launch runs beside the pre-pass ahead of it, which it shares nothing with (wait_last): one CTA waits for that at
-// the end, so that whoever waits for this kernel finds both complete.  (Weight first, pre-pass beside it: the pre-pass's CTAs
-// found no room until the many small ones were through.)
+// launch runs beside the pre-pass ahead of it, which it shares nothing with (and which lets it start once the kernels
+// before have completed): one CTA waits for that at the end, so that whoever waits for this kernel finds both complete.
+// (Weight first, pre-pass beside it: the pre-pass's CTAs found no room until the many small ones were through.  Both in one
+// launch, whose CTAs have the pre-pass's registers: 512 x 4096 x 4096 in f32 32.9 to 33.9 us instead of 32.6.)
 template <class T>
 __global__ void __launch_bounds__(256) repack_kernel(const RepackParams p) {
     __shared__ __align__(16) uint32_t smem[128 * 32];
-    if (!p.wait_last) ptx::pdl_wait();
     ptx::pdl_launch_dependents();
     const uint32_t b = blockIdx.x;
     if (b < p.code_blocks) repack_codes_block(p, b, smem);
     else if (b < p.code_blocks + p.scale_blocks) repack_scales_block(p, b - p.code_blocks, reinterpret_cast<float(*)[33]>(smem));
     else repack_adapter_block<T>(p, b - p.code_blocks - p.scale_blocks, reinterpret_cast<float(*)[33]>(smem));
-    if (p.wait_last && b == 0) ptx::pdl_wait();
+    if (b == 0) ptx::pdl_wait();
 }
 
 // ---- host side -----------------------------------------------------------------------
@@ -1256,10 +1246,10 @@ Sharing share_tiles(uint64_t rows, uint64_t d_in, uint64_t d_out, bool wide_only
 
 struct WorkspaceLayout {
     uint64_t off_xh, off_scale, off_t, off_flags, off_partial, bytes;
-    uint64_t off_a_t, off_b_t;             // the adapter factors as the GEMM reads them (f32 factors, other orientation)
+    uint64_t off_b_t;                      // the adapter factor as the GEMM reads it (f32, other orientation)
     uint64_t off_codes_t, off_scales_t;    // the repacked weight (other orientation)
 };
-enum Extra { kPlain = 0, kFactors = 1, kFactorsAndWeight = 2 };
+enum Extra { kPlain = 0, kFactor = 1, kFactorAndWeight = 2 };
 // f16 copy of x | row scales | T (bf16 hi/lo) | flags and partial sums of the split tiles; d_in is
 // bounded so that rows * d_in * 2 fits
 WorkspaceLayout workspace_layout(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t lora_rank,
@@ -1273,13 +1263,12 @@ WorkspaceLayout workspace_layout(uint64_t rows, uint64_t d_in, uint64_t d_out, u
     const Sharing sh = share_tiles(rows, d_in, d_out);
     w.off_partial = w.off_flags + up((uint64_t)sh.pairs * 8);
     w.bytes = w.off_partial + (sh.sk_tiles ? (uint64_t)sh.pairs * 2 * BM * sh.bn * 4 : 0);
-    w.off_codes_t = w.off_scales_t = w.off_a_t = w.off_b_t = 0;
-    if (extra >= kFactors) {  // `lora_rank` is the rank the GEMM sees (twice the adapter's for f32 factors)
-        w.off_a_t = up(w.bytes);
-        w.off_b_t = w.off_a_t + up((uint64_t)lora_rank * d_in * 2);
+    w.off_codes_t = w.off_scales_t = w.off_b_t = 0;
+    if (extra >= kFactor) {  // `lora_rank` is the rank the GEMM sees (twice the adapter's for f32 factors)
+        w.off_b_t = up(w.bytes);
         w.bytes = w.off_b_t + up(d_out * (uint64_t)lora_rank * 2);
     }
-    if (extra >= kFactorsAndWeight) {
+    if (extra >= kFactorAndWeight) {
         w.off_codes_t = up(w.bytes);
         w.off_scales_t = w.off_codes_t + up(d_in * d_out / 2);
         w.bytes = w.off_scales_t + up((d_out / 64) * d_in * 2);
@@ -1291,7 +1280,7 @@ WorkspaceLayout workspace_layout(uint64_t rows, uint64_t d_in, uint64_t d_out, u
 uint64_t prefill_workspace_bytes(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t lora_rank) {
     if (rows <= 16 || d_in % 64 != 0 || d_in == 0 || d_out == 0) return 0;
     // f32 factors at worst; the other orientation where its shapes allow it
-    return workspace_layout(rows, d_in, d_out, 2 * lora_rank, d_out % 64 == 0 ? kFactorsAndWeight : kFactors).bytes;
+    return workspace_layout(rows, d_in, d_out, 2 * lora_rank, d_out % 64 == 0 ? kFactorAndWeight : kFactor).bytes;
 }
 
 // The reference's orientation (W [d_in][d_out], blocks along d_out) at more than 16 rows: repacked
@@ -1321,7 +1310,7 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_o
         return fail(NF4_ERR_UNSUPPORTED, "prefill_forward: unsupported shape");
     const bool x_f32 = a.io_dtype == NF4_DTYPE_F32;
     const bool y_f32 = a.y_f32 || x_f32;
-    const Extra extra = repacked ? kFactorsAndWeight : x_f32 ? kFactors : kPlain;
+    const Extra extra = repacked ? kFactorAndWeight : x_f32 ? kFactor : kPlain;
     PrefillParams p{};
     p.codes = a.packed;
     p.absmax = a.absmax;
@@ -1357,60 +1346,40 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_o
     p.row_scale = row_scale;
     p.sk_flags = reinterpret_cast<uint32_t *>(ws + wl.off_flags);
     p.partial = reinterpret_cast<float *>(ws + wl.off_partial);
-    const void *lora_a = a.lora_a, *lora_b = a.lora_b;
+    const void *lora_b = a.lora_b;
     RepackParams rp{};
-    auto repack = [&](bool weight, bool a, bool b, bool wait_last) -> int32_t {
-        RepackParams part = rp;
-        if (!weight) part.code_blocks = part.scale_blocks = 0;
-        const uint32_t b_blocks = rp.adapter_blocks - rp.a_blocks;
-        part.a_blocks = a ? rp.a_blocks : 0;
-        part.adapter_blocks = part.a_blocks + (b ? b_blocks : 0);
-        part.wait_last = wait_last;
-        const uint32_t blocks = part.code_blocks + part.scale_blocks + part.adapter_blocks;
-        count_launch();
-        return launch_maybe_overlapped(x_f32 ? repack_kernel<float> : repack_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, true, part);
-    };
-    const bool factors_first = x_f32 && p.rank;  // the pre-pass reads a converted factor
-    if (repacked || factors_first) {  // the other orientation, f32 factors, or both
-        rp.factors_out_in = !repacked;
+    if (repacked) {  // the other orientation
         rp.codes = a.packed;
         rp.absmax = a.absmax;
         rp.scale_codes = a.scale_codes;
         rp.scale_of_scales = a.scale_of_scales;
         rp.codes_t = ws + wl.off_codes_t;
         rp.scales_t = reinterpret_cast<__half *>(ws + wl.off_scales_t);
-        rp.K = p.K;
-        rp.N = p.N;
         rp.code_cols = (p.N + 127) / 128;
-        rp.code_blocks = repacked ? rp.code_cols * ((p.K + 255) / 256) : 0;
+        rp.code_blocks = rp.code_cols * ((p.K + 255) / 256);
         rp.scale_cols = (p.N / 64 + 31) / 32;
-        rp.scale_blocks = repacked ? rp.scale_cols * ((p.K + 31) / 32) : 0;
-        if (p.rank) {
-            rp.a = a.lora_a;
-            rp.b = a.lora_b;
-            rp.r = a.lora_rank;
-            rp.a_t = reinterpret_cast<uint16_t *>(ws + wl.off_a_t);
-            rp.b_t = reinterpret_cast<__nv_bfloat16 *>(ws + wl.off_b_t);
-            const uint32_t rank_tiles = (a.lora_rank + 31) / 32;
-            rp.a_blocks = x_f32 ? rank_tiles * ((p.K + 31) / 32) : 0;
-            rp.adapter_blocks = rp.a_blocks + rank_tiles * ((p.N + 31) / 32);
-            if (x_f32) lora_a = rp.a_t;
-            lora_b = rp.b_t;
-        }
-        if (repacked) {
-            p.codes = rp.codes_t;
-            p.scales_t = rp.scales_t;
-        }
-        if (factors_first) NF4_TRY(repack(false, true, true, false));
+        rp.scale_blocks = rp.scale_cols * ((p.K + 31) / 32);
+        p.codes = rp.codes_t;
+        p.scales_t = rp.scales_t;
     }
+    if (p.rank && (repacked || x_f32)) {
+        rp.b = a.lora_b;
+        rp.r = a.lora_rank;
+        rp.factor_out_in = !repacked;
+        rp.b_t = reinterpret_cast<__nv_bfloat16 *>(ws + wl.off_b_t);
+        rp.adapter_blocks = (a.lora_rank + 31) / 32 * ((p.N + 31) / 32);
+        lora_b = rp.b_t;
+    }
+    rp.K = p.K;
+    rp.N = p.N;
     PrepassArgs pre{};
     pre.x = a.x;
     pre.x_f32 = x_f32;
     pre.M = p.M;
     pre.K = p.K;
-    pre.a = lora_a;
-    pre.rank = p.rank;
-    pre.k_major = repacked && !x_f32;
+    pre.a = a.lora_a;
+    pre.rank = a.lora_a ? a.lora_rank : 0;
+    pre.k_major = repacked;
     pre.scale = a.lora_scale;
     pre.xh = xh;
     pre.row_scale = row_scale;
@@ -1421,9 +1390,11 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_o
     pre.scale_of_scales = a.scale_of_scales;
     pre.flags = p.sk_flags;
     pre.n_flags = 2 * sh.pairs;
-    pre.factor_of_predecessor = factors_first;
     NF4_TRY(activations_prepass(pre, stream));
-    if (repacked) NF4_TRY(repack(true, false, !factors_first, true));
+    if (const uint32_t blocks = rp.code_blocks + rp.scale_blocks + rp.adapter_blocks) {
+        count_launch();
+        NF4_TRY(launch_maybe_overlapped(x_f32 ? repack_kernel<float> : repack_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, true, rp));
+    }
 
     CUtensorMap map_x, map_t, map_b, map_y, map_w, map_ahead, map_s;
     NF4_TRY(make_map(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.codes, p.N, p.K / 2, p.K / 2, BM, BK, CU_TENSOR_MAP_SWIZZLE_64B));

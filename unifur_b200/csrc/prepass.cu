@@ -5,18 +5,17 @@
 //   R = x A^T likewise, unscaled (the operand of the gradient kernel).
 //
 // Split.  A cluster of CTAs takes 64 or 32 rows of x, each CTA a piece of K, which streams through shared
-// memory in stages of 128 k (f32: 64) of x and of the adapter factor (16-byte asynchronous copies, two to five
+// memory in stages of 128 k of x and of the adapter factor (16-byte asynchronous copies, two or three
 // stages in flight): a stage is converted, written out and multiplied where it lies.  bf16 rows are nearly always
 // converted as they are, so the copy does not wait for the row's maximum; a row that needs a power of
-// two after all is written once more.  f32 rows need theirs first: x is read for the maxima, then (from L2) again.
+// two after all is written once more.  (f32 rows need theirs first: a kernel of their own below.)
 // The CTAs' maxima and partial sums of T meet through distributed shared memory, in rank order
 // (results do not depend on timing), after which each writes its share of the rows' T.  The factor
 // [r][K] is the MMA's B operand as it lies, [K][r] goes through transposing matrix loads.
 //
 // Bound by the bytes of x in and xh out, and for few rows by the chain of a load, a stage and one exchange.  Pieces
 // loaded whole, with an exchange of the maxima before anything was written and 32 rows to a factor tile, before:
-// [2048, 4096] at rank 64 30 us, now 19; [2048, 14336] 93, now 52; product alone, [2048, 4096], 21, now 15.  f32 beside
-// the repacking launch: the maxima are read while it runs, only the factor waits for it.
+// [2048, 4096] at rank 64 30 us, now 19; [2048, 14336] 93, now 52; product alone, [2048, 4096], 21, now 15.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -34,18 +33,16 @@ constexpr uint32_t kThreads = 256;
 constexpr uint32_t kPartPitch = 68;  // floats
 constexpr uint32_t kMaxCluster = 1u << (kClusterSizes - 1);
 constexpr uint32_t kSmem = 108 * 1024;  // two CTAs on an SM
-// A stage: 128 k of bf16, 64 of f32.  Pitches are 16 bytes off a multiple of 128 (conflict-free matrix loads), for
-// the pairs of floats 32.
-__host__ __device__ constexpr uint32_t stage_k(bool f32) { return f32 ? 64 : 128; }
-__host__ __device__ constexpr uint32_t x_pitch(bool f32) { return f32 ? 288 : 272; }
-__host__ __device__ constexpr uint32_t factor_pitch(bool f32, bool k_major) { return k_major || f32 ? 144 : 272; }
-__host__ __device__ constexpr uint32_t factor_bytes(bool f32) { return (f32 ? 64 : 128) * 144; }  // the larger orientation
-__host__ __device__ constexpr uint32_t stage_bytes(bool f32, uint32_t rows) { return rows * x_pitch(f32) + factor_bytes(f32); }
-__host__ __device__ constexpr uint32_t stages_of(bool f32, uint32_t rows) { return kSmem / stage_bytes(f32, rows); }
+// A stage: 128 k.  Pitches are 16 bytes off a multiple of 128 (conflict-free matrix loads).
+constexpr uint32_t kStageK = 128, kPitch = 272;
+__host__ __device__ constexpr uint32_t factor_pitch(bool k_major) { return k_major ? 144 : 272; }
+constexpr uint32_t kFactorBytes = 128 * 144;  // the larger orientation
+__host__ __device__ constexpr uint32_t stage_bytes(uint32_t rows) { return rows * kPitch + kFactorBytes; }
+__host__ __device__ constexpr uint32_t stages_of(uint32_t rows) { return kSmem / stage_bytes(rows); }
 
 struct Params {
     const void *x;
-    const void *a;         // factor, bf16 (f16 for MODE 1)
+    const void *a;         // factor, of x's type
     __half *xh;
     float *row_scale;
     __nv_bfloat16 *t_out, *r_out;  // [M][2 * 64 * chunks]: hi halves, then lo; or null
@@ -58,7 +55,6 @@ struct Params {
     uint32_t a_vec;        // the factor's rows are 16-byte aligned
     uint32_t piece;        // k per CTA, a multiple of 64
     float scale;
-    uint32_t wait;         // for the kernel ahead: 0 first of all, 1 before the factor is read
 };
 
 // Running maxima of |bf16|, a pair at a time (the sign bits mean nothing); a NaN leaves the maximum as
@@ -143,16 +139,13 @@ __device__ __forceinline__ void put_halves(__nv_bfloat16 *out, const float (&sum
     *reinterpret_cast<uint2 *>(out + at + lo) = make_uint2(low[0], low[1]);
 }
 
-// MODE 0: bf16 x (products with the bf16 factor are exact).  MODE 1: f32 x; the products use the scaled
-// f16 copy and an f16 factor.  MODE 2: the product R alone, bf16.
+// bf16 x (products with the bf16 factor are exact).  MODE 0: the copy, and T (or R).  MODE 2: the product R alone.
 template <int MODE, uint32_t kRows, bool k_major>
 __global__ void __launch_bounds__(kThreads, 2)
 prepass_kernel(const Params p) {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
-    constexpr bool F32 = MODE == 1;
-    constexpr uint32_t kStageK = stage_k(F32), kHalves = kStageK / 64;
-    constexpr uint32_t kElem = F32 ? 4 : 2, kPitch = x_pitch(F32), kStage = stage_bytes(F32, kRows), kStages = stages_of(F32, kRows);
+    constexpr uint32_t kHalves = kStageK / 64, kElem = 2, kStage = stage_bytes(kRows), kStages = stages_of(kRows);
     constexpr uint32_t kRowTiles = kRows / 32;  // 16-row tiles of a warp
     static_assert(4 * kRows * kPartPitch * 4 <= kStages * kStage, "the sums reuse the stages");
     extern __shared__ __align__(16) uint8_t smem[];
@@ -167,7 +160,7 @@ prepass_kernel(const Params p) {
     cluster.barrier_arrive();      // (waited for before the first access to another CTA's shared memory)
     // the GEMM may set itself up and start on the weights, which are in place once the kernels before this
     // one have completed (a repacked weight it waits for itself)
-    if (p.wait == 0) ptx::pdl_wait();
+    ptx::pdl_wait();
     ptx::pdl_launch_dependents();
     // the GEMM's CTAs raise these once this kernel has completed (their readers and writers wait for that)
     if (blockIdx.x == 0)
@@ -206,7 +199,6 @@ prepass_kernel(const Params p) {
                 for (uint32_t q = 0; q < kRowTiles; ++q) {
                     const uint32_t at = next_at + (tr + q * 32) * kPitch + (tk + h * 64) * kElem;
                     ptx::cp_async_16_or_zero(at, xsrc[q] + h * 64 * kElem, in ? xsize[q] : 0);
-                    if (F32) ptx::cp_async_16_or_zero(at + 16, xsrc[q] + 16, in ? xsize[q] : 0);
                 }
             }
             #pragma unroll
@@ -219,7 +211,7 @@ prepass_kernel(const Params p) {
                     for (uint32_t q = 0; q < 2; ++q) {
                         const uint32_t r = tr + q * 32;
                         const bool in = next_k + h * 64 + (k_major ? r : tk) < k1;
-                        const uint32_t at = fdst + (k_major ? (r + h * 64) * 144 + tk * 2 : r * factor_pitch(F32, false) + (tk + h * 64) * 2);
+                        const uint32_t at = fdst + (k_major ? (r + h * 64) * 144 + tk * 2 : r * factor_pitch(false) + (tk + h * 64) * 2);
                         ptx::cp_async_16_or_zero(at, fsrc[q] + h * (k_major ? 64 * p.rank : 64), in ? fsize[q] : 0);
                     }
                 }
@@ -230,7 +222,7 @@ prepass_kernel(const Params p) {
                     const uint32_t c = k_major ? i & 63u : i % kStageK, r = k_major ? i >> 6 : i / kStageK;
                     const uint32_t k = next_k + (k_major ? r : c), j = chunk * 64 + (k_major ? c : r);
                     const uint16_t v = k < k1 && j < p.rank ? __ldg(a + (k_major ? (size_t)k * p.rank + j : (size_t)j * p.K + k)) : (uint16_t)0;
-                    *reinterpret_cast<uint16_t *>(smem + (fdst - base) + r * factor_pitch(F32, k_major) + c * 2) = v;
+                    *reinterpret_cast<uint16_t *>(smem + (fdst - base) + r * factor_pitch(k_major) + c * 2) = v;
                 }
             }
             next_k += kStageK;
@@ -247,7 +239,7 @@ prepass_kernel(const Params p) {
     auto send_maxima = [&]() {
         #pragma unroll
         for (uint32_t q = 0; q < kRowTiles; ++q) {
-            uint32_t m = F32 ? mx[q] : bf16x2_larger_bits(mx[q]);
+            uint32_t m = bf16x2_larger_bits(mx[q]);
             #pragma unroll
             for (int d = 1; d < 8; d *= 2) m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
             for (uint32_t c = tid & 7u; c < cn; c += 8) cluster.map_shared_rank(&s_max[0][0], c)[rank_in * kRows + tr + q * 32] = m;
@@ -257,7 +249,7 @@ prepass_kernel(const Params p) {
         if (tid < kRows) {
             uint32_t m = 0;
             for (uint32_t c = 0; c < cn; ++c) m = max(m, s_max[c][tid]);
-            const float sc = row_factor<F32>(__uint_as_float(m));
+            const float sc = row_factor<false>(__uint_as_float(m));
             s_inv[tid] = 1.0f / sc;  // exact: sc is a power of two
             if (rank_in == 0 && m0 + tid < p.M) p.row_scale[m0 + tid] = sc * ldexpf(1.0f, w_exp);  // both factors of the outputs
         }
@@ -265,40 +257,13 @@ prepass_kernel(const Params p) {
     };
     const int w_exp = MODE == 2 ? 0 : weight_exponent(p.absmax, p.scale_codes, p.scale_of_scales);
 
-    if (F32) {
-        #pragma unroll
-        for (uint32_t q = 0; q < kRowTiles; ++q) {
-            const uint32_t r = tr + q * 32;
-            const float4 *row = reinterpret_cast<const float4 *>(static_cast<const float *>(p.x) + (size_t)(m0 + r) * p.K);
-            if (m0 + r < p.M) {
-                #pragma unroll 8
-                for (uint32_t k = k0 / 4 + (tid & 7u); k < k1 / 4; k += 8) {
-                    const float4 v = __ldg(row + k);
-                    const uint32_t w[4] = {__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w)};
-                    #pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        if ((w[i] & 0x7fffffffu) < 0x7f800000u) mx[q] = max(mx[q], w[i] & 0x7fffffffu);
-                }
-            }
-        }
-        if (p.wait != 1) begin(0);
-        cluster.barrier_wait();
-        send_maxima();
-        cluster.sync();
-        factors(w_exp);
-        if (p.wait == 1) {
-            ptx::pdl_wait();
-            begin(0);
-        }
-    } else {
-        begin(0);
-    }
+    begin(0);
 
     // ---- the stages: the f16 copy, and per stage a warp has half of the rows and 16 k, 64 ranks at a time ----
     const uint32_t rh = warp & 1u, kq = warp >> 1, g = lane >> 2, t = lane & 3u, li = lane >> 3, lr = lane & 7u;
     const float w_down = ldexpf(1.0f, -w_exp);
     const uint32_t per = kRows / cn, ld = 2 * 64 * p.chunks;
-    constexpr uint32_t kSteps = kStageK / 64, kFactorPitch = factor_pitch(F32, k_major);  // 16 k each; of the factor's rows
+    constexpr uint32_t kSteps = kStageK / 64, kFactorPitch = factor_pitch(k_major);  // 16 k each; of the factor's rows
     const uint32_t a_at = rh * kRowTiles * 16 * kPitch + ((li & 1u) * 8 + lr) * kPitch + (kq * kSteps * 16 + (li >> 1) * 8) * 2;
     const uint32_t b_at = kRows * kPitch + (k_major ? (kq * kSteps * 16 + (li & 1u) * 8 + lr) * kFactorPitch + (li >> 1) * 16
                                                     : ((li >> 1) * 8 + lr) * kFactorPitch + (kq * kSteps * 16 + (li & 1u) * 8) * 2);
@@ -322,21 +287,10 @@ prepass_kernel(const Params p) {
                     for (uint32_t h = 0; h < kHalves; ++h) {
                         const uint4 *in = reinterpret_cast<const uint4 *>(smem + at + r * kPitch + (tk + h * 64) * kElem);
                         uint4 o = in[0];
-                        if (F32) {
-                            const float is = s_inv[r];
-                            const uint4 o2 = in[1];
-                            const __half2 h0 = __floats2half2_rn(__uint_as_float(o.x) * is, __uint_as_float(o.y) * is);
-                            const __half2 h1 = __floats2half2_rn(__uint_as_float(o.z) * is, __uint_as_float(o.w) * is);
-                            const __half2 h2 = __floats2half2_rn(__uint_as_float(o2.x) * is, __uint_as_float(o2.y) * is);
-                            const __half2 h3 = __floats2half2_rn(__uint_as_float(o2.z) * is, __uint_as_float(o2.w) * is);
-                            o = make_uint4(*reinterpret_cast<const uint32_t *>(&h0), *reinterpret_cast<const uint32_t *>(&h1),
-                                           *reinterpret_cast<const uint32_t *>(&h2), *reinterpret_cast<const uint32_t *>(&h3));
-                        } else {
-                            const uint32_t w[4] = {o.x, o.y, o.z, o.w};
-                            #pragma unroll
-                            for (int i = 0; i < 4; ++i) mx[q] = bf16x2_absmax(w[i], mx[q]);
-                            o = bf16x8_to_f16x8(o);
-                        }
+                        const uint32_t w[4] = {o.x, o.y, o.z, o.w};
+                        #pragma unroll
+                        for (int i = 0; i < 4; ++i) mx[q] = bf16x2_absmax(w[i], mx[q]);
+                        o = bf16x8_to_f16x8(o);
                         if (m0 + r < p.M && ks + tk + h * 64 < k1) *reinterpret_cast<uint4 *>(out[q] + h * 64) = o;
                     }
                     out[q] += kStageK;
@@ -348,18 +302,7 @@ prepass_kernel(const Params p) {
                 uint32_t af[kRowTiles][4];
                 #pragma unroll
                 for (uint32_t q = 0; q < kRowTiles; ++q) {
-                    if (F32) {
-                        #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const uint32_t r = (rh * kRowTiles + q) * 16 + g + (i & 1) * 8;
-                            const float2 f = *reinterpret_cast<const float2 *>(smem + at + r * kPitch + (kq * 16 + 2 * t + (i >> 1) * 8) * 4);
-                            const float is = s_inv[r];
-                            const __half2 h = __floats2half2_rn(f.x * is, f.y * is);
-                            af[q][i] = *reinterpret_cast<const uint32_t *>(&h);
-                        }
-                    } else {
-                        ptx::ldmatrix_x4(af[q], base + at + a_at + q * 16 * kPitch + step * 32);
-                    }
+                    ptx::ldmatrix_x4(af[q], base + at + a_at + q * 16 * kPitch + step * 32);
                 }
                 #pragma unroll
                 for (uint32_t u = 0; u < 4; ++u) {
@@ -369,13 +312,8 @@ prepass_kernel(const Params p) {
                     else ptx::ldmatrix_x4(bf, base + at + b_at + u * 16 * kFactorPitch + step * 32);
                     #pragma unroll
                     for (uint32_t q = 0; q < kRowTiles; ++q) {
-                        if (F32) {
-                            ptx::mma_16816_f16(acc[q][2 * u], af[q][0], af[q][1], af[q][2], af[q][3], bf[0], bf[1]);
-                            ptx::mma_16816_f16(acc[q][2 * u + 1], af[q][0], af[q][1], af[q][2], af[q][3], bf[2], bf[3]);
-                        } else {
-                            ptx::mma_16816_bf16(acc[q][2 * u], af[q][0], af[q][1], af[q][2], af[q][3], bf[0], bf[1]);
-                            ptx::mma_16816_bf16(acc[q][2 * u + 1], af[q][0], af[q][1], af[q][2], af[q][3], bf[2], bf[3]);
-                        }
+                        ptx::mma_16816_bf16(acc[q][2 * u], af[q][0], af[q][1], af[q][2], af[q][3], bf[0], bf[1]);
+                        ptx::mma_16816_bf16(acc[q][2 * u + 1], af[q][0], af[q][1], af[q][2], af[q][3], bf[2], bf[3]);
                     }
                 }
             }
@@ -405,7 +343,7 @@ prepass_kernel(const Params p) {
                 *at = v;
             }
         }
-        if (chunk == 0 && !F32) {
+        if (chunk == 0) {
             cluster.barrier_wait();
             if (MODE == 0) send_maxima();
         }
@@ -435,12 +373,242 @@ prepass_kernel(const Params p) {
             }
             if (m >= p.M) continue;
             const size_t at = (size_t)m * ld + chunk * 64 + c;
-            // (MODE 1: the products were taken with the scaled rows)
-            if (MODE != 2) put_halves(p.t_out, sum, F32 ? p.scale * w_down : p.scale * s_inv[r] * w_down, at, 64 * p.chunks);
+            if (MODE != 2) put_halves(p.t_out, sum, p.scale * s_inv[r] * w_down, at, 64 * p.chunks);
             put_halves(p.r_out, sum, 1.0f, at, 64 * p.chunks);
         }
         cluster.sync();  // the sums have been read (before the next chunk's stages, and before a CTA leaves)
     }
+}
+
+// ---- f32 x ------------------------------------------------------------------------------------------------------------
+// T's products use the scaled f16 copy and the factor rounded to f16.  A cluster takes 32 rows, a CTA a piece of K: 32 k
+// at a time a warp, whose lanes hold eight k of four rows each, as the MMA's A operand wants them (in an order of k
+// that the factor's lanes share).  Up to 512 k, the usual case, the values stay in registers while the rows' maxima meet, so that x
+// is read once, all of it in flight together, and the factor's values are on their way beside it; of longer pieces all but the last 512 k are read again.
+// The factor comes as it is stored, f32 in either orientation.  T appears twice, in columns j and rank + j: the GEMM
+// multiplies it with the bf16 high and low halves of the other factor.
+// Bound by the chain of the loads, the maxima's exchange, the copy and the sums' exchange.  Before, with x read twice (the
+// second time behind the exchange, through shared memory) and a launch ahead that converted both factors, the two took 14 us of
+// the 36.5 of 512 x 4096 x 4096 at rank 16; now 9 of 32.7.  [2048, 4096] at rank 64 43 us and 6 for the factors, now 34;
+// [4096, 14336] at rank 8 133 and 6, now 121.  (The copy with a factor from the row's first values, without the maxima's
+// exchange, and T in tf32 from registers, both factors converted where they are used: 512 x 4096 x 4096 36.9.)
+constexpr uint32_t kUnits = 2, kPieceF32 = 8 * kUnits * 32, kGroupRanks = 16, kMostRanks = 128, kPartRow = 20, kSumRow = kMostRanks + 4;
+
+template <bool k_major>
+__global__ void __launch_bounds__(kThreads, 2)
+prepass_f32_kernel(const Params p) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    constexpr uint32_t kRows = 32;
+    __shared__ uint32_t s_warp[8][kRows], s_max[kMaxCluster][kRows];  // row maxima: of the warps, of the CTAs (f32 patterns)
+    __shared__ float s_inv[kRows];
+    __shared__ __align__(16) float s_part[8][kRows][kPartRow];  // the warps' sums of sixteen ranks
+    __shared__ __align__(16) float s_sum[kRows][kSumRow];       // this CTA's of all
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, g = lane >> 2, t = lane & 3u;
+    const uint32_t cn = cluster.num_blocks(), rank_in = cluster.block_rank();
+    const uint32_t m0 = (blockIdx.x / cn) * kRows, k0 = min(rank_in * p.piece, p.K), k1 = min(k0 + p.piece, p.K);
+
+    ptx::pdl_wait();
+    ptx::pdl_launch_dependents();  // (what for: see the kernel above)
+    cluster.barrier_arrive();  // (waited for before the first access to another CTA's shared memory)
+    if (blockIdx.x == 0)
+        for (uint32_t i = tid; i < p.n_flags; i += kThreads) p.flags[i] = 0;
+
+    // A lane's values of a unit of 32 k: rows q * 8 + g, k 16 s + 4 t and the three after it (K and the pieces are
+    // multiples of 64: a unit is whole or empty).
+    float4 v[kUnits][4][2];
+    auto load = [&](uint32_t kp) {
+        #pragma unroll
+        for (uint32_t u = 0; u < kUnits; ++u) {
+            const uint32_t k = kp + (u * 8 + warp) * 32 + 4 * t;
+            #pragma unroll
+            for (uint32_t q = 0; q < 4; ++q) {
+                const uint32_t m = m0 + q * 8 + g;
+                const float4 *src = reinterpret_cast<const float4 *>(static_cast<const float *>(p.x) + (size_t)m * p.K + k);
+                const bool in = m < p.M && k < k1;
+                #pragma unroll
+                for (uint32_t s = 0; s < 2; ++s) v[u][q][s] = in ? __ldg(src + 4 * s) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+        }
+    };
+    // The factor's values of the same k, ranks group * 16 + 8 n + g, as the MMA's B operand.
+    uint32_t b[kUnits][2][2][2];
+    auto load_factor = [&](uint32_t kp, uint32_t group) {
+        #pragma unroll
+        for (uint32_t u = 0; u < kUnits; ++u) {
+            #pragma unroll
+            for (uint32_t s = 0; s < 2; ++s) {
+                const uint32_t k = kp + (u * 8 + warp) * 32 + 16 * s + 4 * t;
+                #pragma unroll
+                for (uint32_t n = 0; n < 2; ++n) {
+                    const uint32_t j = group * kGroupRanks + 8 * n + g;
+                    float4 f = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (j < p.rank && k < k1) {
+                        const float *src = static_cast<const float *>(p.a) + (k_major ? (size_t)k * p.rank + j : (size_t)j * p.K + k);
+                        const size_t step = k_major ? p.rank : 1;
+                        if (!k_major && p.a_vec) f = __ldg(reinterpret_cast<const float4 *>(src));
+                        else f = make_float4(__ldg(src), __ldg(src + step), __ldg(src + 2 * step), __ldg(src + 3 * step));
+                    }
+                    const __half2 h0 = __floats2half2_rn(f.x, f.y), h1 = __floats2half2_rn(f.z, f.w);
+                    b[u][s][n][0] = *reinterpret_cast<const uint32_t *>(&h0);
+                    b[u][s][n][1] = *reinterpret_cast<const uint32_t *>(&h1);
+                }
+            }
+        }
+    };
+
+    // ---- the rows' maxima (values that are not finite drop out) and factors ----
+    uint32_t mx[4] = {};
+    const uint32_t k_last = k0 + (max(k1, k0 + 1) - k0 - 1) / kPieceF32 * kPieceF32;  // the last part of the piece
+    for (uint32_t kp = k0; kp <= k_last; kp += kPieceF32) {
+        load(kp);
+        if (kp == k_last) load_factor(kp, 0);
+        #pragma unroll
+        for (uint32_t u = 0; u < kUnits; ++u) {
+            #pragma unroll
+            for (uint32_t q = 0; q < 4; ++q) {
+                #pragma unroll
+                for (uint32_t s = 0; s < 2; ++s) {
+                    const uint32_t w[4] = {__float_as_uint(v[u][q][s].x), __float_as_uint(v[u][q][s].y), __float_as_uint(v[u][q][s].z), __float_as_uint(v[u][q][s].w)};
+                    #pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if ((w[i] & 0x7fffffffu) < 0x7f800000u) mx[q] = max(mx[q], w[i] & 0x7fffffffu);
+                }
+            }
+        }
+    }
+    const int w_exp = weight_exponent(p.absmax, p.scale_codes, p.scale_of_scales);
+    #pragma unroll
+    for (uint32_t q = 0; q < 4; ++q) {
+        mx[q] = max(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], 1));
+        mx[q] = max(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], 2));
+        if (t == 0) s_warp[warp][q * 8 + g] = mx[q];
+    }
+    __syncthreads();
+    cluster.barrier_wait();
+    {
+        uint32_t m = 0;
+        #pragma unroll
+        for (uint32_t w = 0; w < 8; ++w) m = max(m, s_warp[w][lane]);
+        for (uint32_t c = warp; c < cn; c += 8) cluster.map_shared_rank(&s_max[0][0], c)[rank_in * kRows + lane] = m;
+    }
+    cluster.sync();
+    if (tid < kRows) {
+        uint32_t m = 0;
+        for (uint32_t c = 0; c < cn; ++c) m = max(m, s_max[c][tid]);
+        const float sc = row_factor<true>(__uint_as_float(m));
+        s_inv[tid] = 1.0f / sc;  // exact: sc is a power of two
+        if (rank_in == 0 && m0 + tid < p.M) p.row_scale[m0 + tid] = sc * ldexpf(1.0f, w_exp);  // both factors of the outputs
+    }
+    __syncthreads();
+
+    // ---- the products, and the copy ----
+    // (The last piece's copy is written behind the arrival at the sums' exchange, whose release would wait for the stores.)
+    uint32_t h[kUnits][4][2][2];
+    auto copy = [&](uint32_t kp) {
+        #pragma unroll
+        for (uint32_t u = 0; u < kUnits; ++u) {
+            const uint32_t k = kp + (u * 8 + warp) * 32 + 4 * t;
+            #pragma unroll
+            for (uint32_t q = 0; q < 4; ++q) {
+                const uint32_t m = m0 + q * 8 + g;
+                #pragma unroll
+                for (uint32_t s = 0; s < 2; ++s)
+                    if (m < p.M && k < k1) *reinterpret_cast<uint2 *>(p.xh + (size_t)m * p.K + k + 16 * s) = make_uint2(h[u][q][s][0], h[u][q][s][1]);
+            }
+        }
+    };
+    uint32_t kp = k_last;  // (first, as its values are still there)
+    for (;;) {
+        #pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) {
+            const float is = s_inv[q * 8 + g];
+            #pragma unroll
+            for (uint32_t u = 0; u < kUnits; ++u) {
+                #pragma unroll
+                for (uint32_t s = 0; s < 2; ++s) {
+                    const __half2 lo = __floats2half2_rn(v[u][q][s].x * is, v[u][q][s].y * is), hi = __floats2half2_rn(v[u][q][s].z * is, v[u][q][s].w * is);
+                    h[u][q][s][0] = *reinterpret_cast<const uint32_t *>(&lo);
+                    h[u][q][s][1] = *reinterpret_cast<const uint32_t *>(&hi);
+                }
+            }
+        }
+        for (uint32_t group = 0; group * kGroupRanks < p.rank; ++group) {
+            if (group || kp != k_last) load_factor(kp, group);
+            float acc[2][2][4] = {};  // of sixteen rows, of eight ranks
+            #pragma unroll
+            for (uint32_t u = 0; u < kUnits; ++u) {
+                #pragma unroll
+                for (uint32_t s = 0; s < 2; ++s) {
+                    #pragma unroll
+                    for (uint32_t q = 0; q < 2; ++q) {
+                        #pragma unroll
+                        for (uint32_t n = 0; n < 2; ++n)
+                            ptx::mma_16816_f16(acc[q][n], h[u][2 * q][s][0], h[u][2 * q + 1][s][0], h[u][2 * q][s][1], h[u][2 * q + 1][s][1],
+                                               b[u][s][n][0], b[u][s][n][1]);
+                    }
+                }
+            }
+            #pragma unroll
+            for (uint32_t q = 0; q < 2; ++q) {
+                #pragma unroll
+                for (uint32_t n = 0; n < 2; ++n) {
+                    *reinterpret_cast<float2 *>(&s_part[warp][q * 16 + g][8 * n + 2 * t]) = make_float2(acc[q][n][0], acc[q][n][1]);
+                    *reinterpret_cast<float2 *>(&s_part[warp][q * 16 + 8 + g][8 * n + 2 * t]) = make_float2(acc[q][n][2], acc[q][n][3]);
+                }
+            }
+            __syncthreads();
+            {
+                const uint32_t r = tid >> 3, c = (tid & 7u) * 2;
+                float2 *const to = reinterpret_cast<float2 *>(&s_sum[r][group * kGroupRanks + c]);
+                float2 sum = kp == k_last ? make_float2(0.0f, 0.0f) : *to;
+                #pragma unroll
+                for (uint32_t w = 0; w < 8; ++w) {  // in order
+                    const float2 o = *reinterpret_cast<const float2 *>(&s_part[w][r][c]);
+                    sum.x += o.x;
+                    sum.y += o.y;
+                }
+                *to = sum;
+            }
+            __syncthreads();
+        }
+        const uint32_t next = kp == k_last ? k0 : kp + kPieceF32;
+        if (next == k_last) break;
+        copy(kp);
+        kp = next;
+        load(kp);
+    }
+    if (!p.rank) {
+        copy(kp);
+        return;
+    }
+
+    // ---- the CTAs' sums, each CTA a share of the rows; columns the adapter does not have are zeros ----
+    cluster.barrier_arrive();
+    copy(kp);
+    cluster.barrier_wait();
+    const float w_down = ldexpf(1.0f, -w_exp);
+    const uint32_t per = (kRows + cn - 1) / cn, quads = 16 * p.chunks, ld = 2 * 64 * p.chunks;
+    for (uint32_t i = tid; i < per * quads; i += kThreads) {
+        const uint32_t r = rank_in * per + i / quads, c = i % quads * 4, m = m0 + r;
+        if (r >= kRows || m >= p.M || (c >= p.rank && c < 2 * p.rank)) continue;  // (the rank is a multiple of four)
+        float sum[4] = {};
+        if (c < p.rank) {
+            #pragma unroll 4
+            for (uint32_t q = 0; q < cn; ++q) {
+                const float4 w = *reinterpret_cast<const float4 *>(cluster.map_shared_rank(&s_sum[0][0], q) + r * kSumRow + c);
+                sum[0] += w.x;
+                sum[1] += w.y;
+                sum[2] += w.z;
+                sum[3] += w.w;
+            }
+        }
+        // (the products were taken with the scaled rows)
+        put_halves(p.t_out, sum, p.scale * w_down, (size_t)m * ld + c, 64 * p.chunks);
+        if (c < p.rank) put_halves(p.t_out, sum, p.scale * w_down, (size_t)m * ld + p.rank + c, 64 * p.chunks);
+    }
+    __syncwarp();  // (lanes come from loops of different length)
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");  // the sums have been read
 }
 
 // ---- the same for bf16 x and a factor on tcgen05: up to 64 ranks, rows of 16-byte pieces -------------------------------
@@ -501,7 +669,7 @@ prepass_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         ptx::fence_proxy_async();
         ptx::prefetch_tmap(&tmap_x);
         ptx::prefetch_tmap(&tmap_a);
-        ptx::pdl_wait();  // (p.wait is 0: only f32 x has a factor that the kernel ahead writes)
+        ptx::pdl_wait();
         for (uint32_t st = 0; st < min(stages, kStages); ++st) request(st);
     }
     if (warp == 9) {
@@ -693,6 +861,7 @@ prepass_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         put_halves(p.r_out, sum, 1.0f, (size_t)m * 128 + c, 64);
     }
     ptx::tc_fence_before();
+    __syncwarp();  // (lanes come from loops of different length)
     asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");  // the sums have been read
     if (warp == 9) {
         ptx::tc_fence_after();
@@ -763,6 +932,8 @@ int32_t launch_tc(const PrepassArgs &q, Params &p, cudaStream_t stream) {
 }  // namespace
 
 int32_t activations_prepass(const PrepassArgs &q, cudaStream_t stream) {
+    if (q.x_f32 && (!q.xh || q.r_out || q.rank > kMostRanks || q.rank % 4))
+        return fail(NF4_ERR_UNSUPPORTED, "activations_prepass: f32 with the copy, without r_out, and at most %u ranks", kMostRanks);
     Params p{};
     p.x = q.x;
     p.a = q.a;
@@ -778,10 +949,9 @@ int32_t activations_prepass(const PrepassArgs &q, cudaStream_t stream) {
     p.M = q.M;
     p.K = q.K;
     p.rank = q.rank;
-    p.chunks = (q.rank + 63) / 64;
+    p.chunks = ((q.x_f32 ? 2 * q.rank : q.rank) + 63) / 64;
     p.a_vec = aligned16(q.a) && (q.k_major ? q.rank : q.K) % 8 == 0;
     p.scale = q.scale;
-    p.wait = q.factor_of_predecessor ? 1 : 0;
     // The tcgen05 kernel, where its TMA takes the tensors: always for the product alone ([16, 11008] and [14, 768] the same
     // time); with the copy from four million values on (whole forwards to 512 columns: [1024, 4096] at rank 64 42.7 -> 40.3 us,
     // [4096, 1024] 23.7 -> 23.1, but [512, 2048] 27.5 -> 30.3 and [256, 4096] at rank 16 the other way too: an SM
@@ -790,18 +960,18 @@ int32_t activations_prepass(const PrepassArgs &q, cudaStream_t stream) {
     if (tc_shape && (!q.xh || (uint64_t)q.M * q.K >= 1u << 22)) return launch_tc(q, p, stream);
     // 64 rows to a cluster beyond 512 rows, where the clusters of 32 no longer fit the chip at once, else 32 (half of the
     // factor's traffic against more CTAs)
-    const uint32_t rows = q.M > 512 ? 64 : 32;
+    const uint32_t rows = !q.x_f32 && q.M > 512 ? 64 : 32;
     const uint64_t tiles = (q.M + rows - 1) / rows;
     auto pick = [&](auto km) {
         constexpr bool k_major = decltype(km)::value;
+        if (q.x_f32) return prepass_f32_kernel<k_major>;
         return rows == 64 ? (q.xh ? prepass_kernel<0, 64, k_major> : prepass_kernel<2, 64, k_major>)
                           : (q.xh ? prepass_kernel<0, 32, k_major> : prepass_kernel<2, 32, k_major>);
     };
-    if (q.x_f32 && q.k_major) return fail(NF4_ERR_UNSUPPORTED, "activations_prepass: f32 factors come as [r][K]");
-    auto kernel = q.x_f32 ? (rows == 64 ? prepass_kernel<1, 64, false> : prepass_kernel<1, 32, false>)
-                          : q.k_major ? pick(std::true_type{}) : pick(std::false_type{});
-    const int smem = (int)(stages_of(q.x_f32, rows) * stage_bytes(q.x_f32, rows));
-    // as many CTAs of K as the chip holds at once, two on an SM (a second wave took 21 us where one takes 11)
+    auto kernel = q.k_major ? pick(std::true_type{}) : pick(std::false_type{});
+    const int smem = q.x_f32 ? 0 : (int)(stages_of(rows) * stage_bytes(rows));
+    // as many CTAs of K as the chip holds at once, two on an SM (a second wave took 21 us where one takes 11; of f32 [4096, 4096]
+    // two CTAs to a cluster 40 us, eight, whose pieces are read once, 45; [4096, 14336] 121 and, sixteen, 154)
     ClusterRoom room;
     NF4_TRY(cluster_room(reinterpret_cast<const void *>(kernel), kThreads, (uint32_t)smem, &room));
     const uint32_t cn = cluster_ctas(tiles, q.K, 64, room);
