@@ -5,13 +5,14 @@
 //
 // gradient_kernel: out(p, j) = s sum_m X[m][p] R[m][j] as D[p][j] += X^T R (tcgen05, both operands MN-major as they lie).  A
 // CTA takes 128 columns p, 64 ranks and a share of the rows; stages of 64 rows of X and of both halves of R (32 KB) come
-// by TMA, three in flight (an SM holds one CTA: the driver counts one, although shared memory and registers would do for
-// two; 61 of its L2 port's bytes a nanosecond arrive); one thread asks for them and one issues their MMAs.  The CTAs that share a
+// by TMA, six in flight where an SM has one CTA, three where there are more CTAs than SMs and it holds two; one thread asks
+// for them and one issues their MMAs.  The CTAs that share a
 // tile's rows form a cluster: their sums meet through distributed shared memory, each adds (in rank order) and writes its
 // part of the columns.  Both gradients are one launch: the tiles of x with U, then those of grad_y with T.  Bound by reading X
 // once and R from the L2 for every 128 columns and, at few columns, by the chain of a load, its stages and that exchange.
 // Warp MMAs behind transposing loads, whose pipe was half busy, took 40 us for [2048, 14336] and 17 for [2048, 4096] at
-// rank 64; in a launch each these tiles take 21 and 12 us, together 22.
+// rank 64; in a launch each these tiles took 21 and 12 us, together 22, and 19.7 with six stages in flight.  (Tiles of 256
+// columns and half of the rows, which read R half as often, 22.)
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
@@ -22,11 +23,11 @@
 namespace nf4 {
 namespace {
 
-constexpr uint32_t kThreads = 192, kCols = 128, kRowsStage = 64, kStages = 3;
+constexpr uint32_t kThreads = 192, kCols = 128, kRowsStage = 64;
 constexpr uint32_t kBox = kRowsStage * 128, kStage = 4 * kBox;  // X: two boxes of 64 columns; R: high and low halves
-constexpr uint32_t kSmem = kStages * kStage + 1024;
+constexpr uint32_t smem_of(uint32_t stages) { return stages * kStage + 1024; }
 constexpr uint32_t kSumPitch = 68;                              // floats
-static_assert(kCols * kSumPitch * 4 <= kStages * kStage, "the sums reuse the stages");
+static_assert(kCols * kSumPitch * 4 <= 3 * kStage, "the sums reuse the stages");
 
 struct Params {
     __nv_bfloat16 *out[2];        // of x (times U), of grad_y (times T)
@@ -36,6 +37,7 @@ struct Params {
     float scale;
 };
 
+template <uint32_t kStages>
 __global__ void __launch_bounds__(kThreads, 2)  // (registers for two)
 gradient_kernel(const __grid_constant__ CUtensorMap tmap_x0, const __grid_constant__ CUtensorMap tmap_r0, const __grid_constant__ CUtensorMap tmap_x1,
                 const __grid_constant__ CUtensorMap tmap_r1, const Params p, const FailureRef failure) {
@@ -195,10 +197,12 @@ int32_t gradients(const void *x, const void *u, void *ga, bool ga_p_major, uint6
     p.tiles0 = (uint32_t)tiles_of(d_in);
     const uint64_t tiles = tiles_of(d_in) + tiles_of(d_out);
     // Shares of the rows: as many as the chip holds clusters for at once, where a share keeps four stages (256 rows)
-    const void *kernel = reinterpret_cast<const void *>(gradient_kernel);
     ClusterRoom room;
-    NF4_TRY(cluster_room(kernel, kThreads, kSmem, &room));
+    NF4_TRY(cluster_room(reinterpret_cast<const void *>(gradient_kernel<6>), kThreads, smem_of(6), &room));
     const uint32_t shares = cluster_ctas(tiles, rows, 4 * kRowsStage, room);
+    // Three stages in flight leave room for a second CTA on an SM, six ask for what one SM's port brings: columns of 128 in all,
+    // 144 tiles of 2048 rows 22.0 and 19.5 us, 64 of 4096 14.0 and 12.8, but 251 tiles of 1100 rows 18.9 and 26.3.
+    const bool deep = tiles * shares * p.chunks <= kNumSMs;
     const uint32_t all = (uint32_t)((rows + kRowsStage - 1) / kRowsStage);
     p.stages_per_share = (all + shares - 1) / shares;
     if (tiles * shares >= (1ull << 31)) return fail(NF4_ERR_UNSUPPORTED, "gradients: too many columns");
@@ -216,7 +220,7 @@ int32_t gradients(const void *x, const void *u, void *ga, bool ga_p_major, uint6
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(tiles * shares), p.chunks);
     cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = kSmem;
+    cfg.dynamicSmemBytes = smem_of(deep ? 6 : 3);
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -227,7 +231,9 @@ int32_t gradients(const void *x, const void *u, void *ga, bool ga_p_major, uint6
     cfg.attrs = attr;
     cfg.numAttrs = shares > 1 ? 2 : 1;
     count_launch();
-    return check_cuda(cudaLaunchKernelEx(&cfg, gradient_kernel, map_x0, map_r0, map_x1, map_r1, p, failure), "gradient_kernel launch");
+    auto kernel = deep ? gradient_kernel<6> : gradient_kernel<3>;
+    if (!deep) NF4_TRY(cluster_room(reinterpret_cast<const void *>(kernel), kThreads, smem_of(3), &room));
+    return check_cuda(cudaLaunchKernelEx(&cfg, kernel, map_x0, map_r0, map_x1, map_r1, p, failure), "gradient_kernel launch");
 }
 
 }  // namespace
