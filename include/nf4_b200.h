@@ -167,6 +167,14 @@ NF4_API int32_t nf4_quantize_transposed_dev(const void *src, int32_t src_dtype, 
                                     uint8_t *packed, float *absmax, void *workspace,
                                     uint64_t workspace_bytes, void *stream);
 
+/* nf4_quantize_transposed_dev and nf4_double_quantize_dev in one, with the same results: a checkpoint's matrix to a
+ * double-quantized weight.  `absmax` (a float per block) holds the f32 scales afterwards; `workspace` is always needed
+ * (4-byte aligned). */
+NF4_API uint64_t nf4_quantize_transposed_double_workspace_bytes(uint64_t rows, uint64_t cols);
+NF4_API int32_t nf4_quantize_transposed_double_dev(const void *src, int32_t src_dtype, uint64_t rows, uint64_t cols,
+                                    uint8_t *packed, float *absmax, uint8_t *scale_codes, float *scale_of_scales,
+                                    void *workspace, uint64_t workspace_bytes, void *stream);
+
 /* Rows of a packed [n_embedding, d_model] table selected by `ids` (int64, device memory),
  * dequantized: out[t][j] = level[code] * block scale of element ids[t] * d_model + j, bit-exact
  * with dequantizing the whole table and gathering.  Replaces the body of Nf4Embedding::forward,

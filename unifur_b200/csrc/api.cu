@@ -528,6 +528,18 @@ int32_t nf4_quantize_transposed_dev(const void *src, int32_t src_dtype, uint64_t
                                workspace_bytes, static_cast<cudaStream_t>(stream));
 }
 
+uint64_t nf4_quantize_transposed_double_workspace_bytes(uint64_t rows, uint64_t cols) {
+    return quantize_transposed_double_workspace_bytes(rows, cols);
+}
+
+int32_t nf4_quantize_transposed_double_dev(const void *src, int32_t src_dtype, uint64_t rows, uint64_t cols, uint8_t *packed, float *absmax,
+                                           uint8_t *scale_codes, float *scale_of_scales, void *workspace, uint64_t workspace_bytes, void *stream) {
+    if (src_dtype != NF4_DTYPE_F32 && src_dtype != NF4_DTYPE_BF16)
+        return fail(NF4_ERR_INVALID_ARG, "nf4_quantize_transposed_double_dev: src_dtype must be NF4_DTYPE_F32 or NF4_DTYPE_BF16");
+    return quantize_transposed_double(src, src_dtype == NF4_DTYPE_BF16, rows, cols, packed, absmax, scale_codes, scale_of_scales, workspace,
+                                      workspace_bytes, static_cast<cudaStream_t>(stream));
+}
+
 int32_t nf4_embedding_gather_dev(const uint8_t *packed, const float *absmax,
                                  const uint8_t *scale_codes, const float *scale_of_scales,
                                  uint64_t n_embedding, uint64_t d_model, const int64_t *ids,

@@ -407,8 +407,8 @@ PyObject *quantize(PyObject *, PyObject *const *v, Py_ssize_t n) {
     });
 }
 
-// quantize_transposed(weight) -> (codes, absmax)
-PyObject *quantize_transposed(PyObject *, PyObject *const *v, Py_ssize_t n) {
+// quantize_transposed(weight) -> (codes, absmax); quantize_transposed_double(weight) -> (codes, scale_codes, scale_of_scales)
+PyObject *quantize_transposed_as(PyObject *const *v, Py_ssize_t n, bool twice) {
     return guarded([&]() -> PyObject * {
         expect(n, 1);
         const Tensor &t = tensor(v[0]);
@@ -421,7 +421,7 @@ PyObject *quantize_transposed(PyObject *, PyObject *const *v, Py_ssize_t n) {
         const uint64_t rows = (uint64_t)w.size(0), cols = (uint64_t)w.size(1);
         Tensor codes = empty({(len + 1) / 2}, at::kByte, place);
         Tensor absmax = empty({blocks_of(len)}, at::kFloat, place);
-        const uint64_t bytes = nf4_quantize_transposed_workspace_bytes(rows, cols);
+        const uint64_t bytes = twice ? nf4_quantize_transposed_double_workspace_bytes(rows, cols) : nf4_quantize_transposed_workspace_bytes(rows, cols);
         Tensor ws;
         if (bytes) ws = empty({(int64_t)bytes}, at::kByte, place);
         const void *pw = w.const_data_ptr();
@@ -429,12 +429,23 @@ PyObject *quantize_transposed(PyObject *, PyObject *const *v, Py_ssize_t n) {
         float *pa = static_cast<float *>(absmax.mutable_data_ptr());
         void *ps = bytes ? ws.mutable_data_ptr() : nullptr;
         const int32_t type = io_dtype(w.scalar_type());
+        if (twice) {
+            Tensor sc = empty({blocks_of(len)}, at::kByte, place), sos = empty({1}, at::kFloat, place);
+            uint8_t *psc = static_cast<uint8_t *>(sc.mutable_data_ptr());
+            float *psos = static_cast<float *>(sos.mutable_data_ptr());
+            check(unlocked([&] {
+                return nf4_quantize_transposed_double_dev(pw, type, rows, cols, pc, pa, psc, psos, ps, bytes, place.stream);
+            }));
+            return Py_BuildValue("NNN", THPVariable_Wrap(std::move(codes)), THPVariable_Wrap(std::move(sc)), THPVariable_Wrap(std::move(sos)));
+        }
         check(unlocked([&] {
             return nf4_quantize_transposed_dev(pw, type, rows, cols, pc, pa, ps, bytes, place.stream);
         }));
         return pair(std::move(codes), std::move(absmax));
     });
 }
+PyObject *quantize_transposed(PyObject *, PyObject *const *v, Py_ssize_t n) { return quantize_transposed_as(v, n, false); }
+PyObject *quantize_transposed_double(PyObject *, PyObject *const *v, Py_ssize_t n) { return quantize_transposed_as(v, n, true); }
 
 // double_quantize(absmax, num_blocks) -> (scale_codes, scale_of_scales)
 PyObject *double_quantize(PyObject *, PyObject *const *v, Py_ssize_t n) {
@@ -528,6 +539,7 @@ PyObject *release_workspaces(PyObject *, PyObject *) {
     { #name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(name)), METH_FASTCALL, nullptr }
 PyMethodDef kMethods[] = {
     FAST(linear_forward), FAST(linear_forward_grouped), FAST(qlora_backward), FAST(quantize), FAST(quantize_transposed),
+    FAST(quantize_transposed_double),
     FAST(double_quantize), FAST(dequantize), FAST(quantize_dequantize), FAST(embedding),
     {"release_workspaces", release_workspaces, METH_NOARGS, "Give the calling thread's kept workspaces back."},
     {nullptr, nullptr, 0, nullptr}};

@@ -74,6 +74,12 @@ class PackedNf4Tensor:
         codes, absmax = _lib.host().quantize_transposed(weight)
         return PackedNf4Tensor(codes, weight.numel(), absmax)
 
+    @staticmethod
+    def _from_checkpoint(weight: torch.Tensor) -> "PackedNf4Tensor":
+        """``quantize_transposed(weight).with_double_quantization()`` in one call."""
+        codes, sc, sos = _lib.host().quantize_transposed_double(weight)
+        return PackedNf4Tensor(codes, weight.numel(), None, sc, sos)
+
     def with_double_quantization(self) -> "PackedNf4Tensor":
         """src/quantize.rs:284-309; idempotent."""
         if self.is_double_quantized():

@@ -49,7 +49,7 @@ class Nf4Linear:
         ``[in, out]`` NF4 linear with double quantization, as its loader builds it
         (src/qwennet.rs:1687-1726): transpose and quantize fused on the device."""
         rows, cols = weight.shape
-        packed = PackedNf4Tensor.quantize_transposed(weight).with_double_quantization()
+        packed = PackedNf4Tensor._from_checkpoint(weight)
         return Nf4Linear(packed, cols, rows, None, LAYOUT_IN_OUT)
 
     def d_input(self) -> int:
