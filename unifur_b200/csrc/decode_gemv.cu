@@ -239,16 +239,19 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
     extern __shared__ __align__(1024) uint8_t smem[];
     // kUniformWarp: the warp's number comes through a shuffle; the compiler then knows that it is the same in all lanes, and
     // keeps what follows from it in uniform registers.  kElects: an elected lane asks for the loop's tiles, else the first one.
+    // kCarries: the tile loop keeps shared-memory addresses, its tiles' row and the number of T's tile in registers, and starts
+    // its sums with a product; without it works them out for every tile (18 of 315 instructions a warp and tile, up to 8 rows).
     // Which of them helps depends on what a form has in its registers (us, back to back, without -> with):
-    //   up to 8 rows, scales by TMA: both, 4 x 4096 x 11008 8.84 -> 8.60, the block 54.2 -> 52.6; the other forms lose by them
-    //     (u8 scales 9.41 -> 9.62)
-    //   9 to 16 rows, scales by TMA: elected, at rank 16 16 x 4096 x 11008 12.45 -> 12.28, x 3584 x 18944 18.1 -> 17.9 (but
-    //     16 x 3584 x 512 without an adapter, a tile a warp, 4.99 -> 5.03); uniform as well 9 x 4096 x 4096 7.09 -> 7.28
-    //   9 to 16 rows, u8 words: neither, elected 16 x 4096 x 4096 7.43 -> 7.63, 16 x 11008 x 4096 17.5 -> 17.6 (but
-    //     16 x 3584 x 18944 at rank 16 18.6 -> 18.4)
-    //   9 to 16 rows, d_in no multiple of 256: both, 9 x 4160 x 8192 15.9 -> 15.6, u8 scales 16.2 -> 16.0
-    constexpr bool kUniformWarp = NT == 1 ? SC == kScalesTma : SC == kScalesF32 || SC == kScalesU8;
-    constexpr bool kElects = NT == 1 ? SC == kScalesTma : SC != kScalesU8Words;
+    //   up to 8 rows, scales by TMA: all, 4 x 4096 x 11008 8.84 -> 8.60 by the first two, -> 8.22 by the third, 8 x 3584 x
+    //     18944 11.9 -> 11.6; the other forms the third alone (1 x 4096 x 11008 with u8 scales 9.08 -> 8.85, 4 x 4160 x 8192
+    //     12.3 -> 11.6)
+    //   9 to 16 rows, scales by TMA and u8 scales without words: uniform and carried, 16 x 20480 x 20480 98.9 -> 96.7,
+    //     16 x 4160 x 4096 11.3 -> 10.9; elected as well 16 x 3584 x 512 without an adapter 5.0 -> 5.2
+    //   9 to 16 rows, u8 words: none, with the third 9 x 4096 x 4096 without an adapter 6.7 -> 6.9 and more
+    //   9 to 16 rows, f32 scales of a d_in that is no multiple of 256: the first two, with the third 9 x 4160 x 8192 16.4 -> 16.7
+    constexpr bool kUniformWarp = NT == 1 ? SC == kScalesTma : SC != kScalesU8Words;
+    constexpr bool kElects = NT == 1 ? SC == kScalesTma : SC == kScalesF32;
+    constexpr bool kCarries = NT == 1 || SC == kScalesTma || SC == kScalesU8;
     const uint32_t tid = threadIdx.x, warp = kUniformWarp ? __shfl_sync(0xffffffffu, tid >> 5, 0) : tid >> 5, lane = tid & 31u;
     if (ptx::smem_addr(smem) != kWin0) {
         // the table's base is an immediate of the lookups: nothing can run from another address
@@ -306,22 +309,13 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
     const uint32_t bar0 = kWin0 + C::kOffBars + warp * kRing * 8u;
     const uint32_t codes0 = kWin0 + C::kOffCodes + warp * kRing * C::kCodesTile;
     const uint32_t scales0 = kWin0 + C::kOffScales + warp * kRing * C::kScaleTile;
-    const uint8_t *codes_ring = smem + C::kOffCodes + warp * kRing * C::kCodesTile;
-    const uint8_t *scales_ring = smem + C::kOffScales + warp * kRing * C::kScaleTile;
 
     // ---- this warp's barriers and its first tiles (nothing here depends on the predecessor):
-    // lane (slot, slice) asks for its box, so the requests of all slots leave in one instruction ----
-    auto request = [&](uint32_t j, uint32_t sl) {
-        // K-slice sl of this warp's tile number j goes to slot j % kRing
-        const uint32_t slot = j & (kRing - 1);
-        const int32_t row0 = (int32_t)(n0 + (rg + j * rw) * kTileRows);
-        const uint32_t bar = bar0 + 8 * slot;
+    // a lane asks for a slot's boxes, so the requests of all slots leave in one instruction ----
+    auto ask = [&](uint32_t bar, uint32_t slot, int32_t row0) {  // a tile of this warp's K-slice
         ptx::mbar_arrive_expect_tx(bar, TMA_SCALES ? kCodesSlot + kScaleSlot : kCodesSlot);
-        ptx::tma_load_2d(codes0 + slot * C::kCodesTile + sl * kCodesSlot, tm_codes,
-                         (int32_t)((slice0 + sl) * 128u), row0, bar);
-        if (TMA_SCALES)
-            ptx::tma_load_2d(scales0 + slot * C::kScaleTile + sl * kScaleSlot, tm_scales,
-                             (int32_t)((slice0 + sl) * 4u), row0, bar);
+        ptx::tma_load_2d(codes0 + slot * C::kCodesTile, tm_codes, (int32_t)(slice0 * 128u), row0, bar);
+        if (TMA_SCALES) ptx::tma_load_2d(scales0 + slot * C::kScaleTile, tm_scales, (int32_t)(slice0 * 4u), row0, bar);
     };
     if (active && nsl == 0) {
         #pragma unroll 1
@@ -366,9 +360,9 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
             ptx::fence_mbar_init();
         }
         __syncwarp();
-        if (lane < (uint32_t)(kRing * SL)) {
-            const uint32_t j = lane / SL, sl = lane % SL;
-            if (j < my_tiles && sl < nsl) request(j, sl);
+        if (lane < (uint32_t)kRing) {
+            const uint32_t j = lane, slot = j & (kRing - 1);
+            if (j < my_tiles) ask(bar0 + 8 * slot, slot, (int32_t)(n0 + (rg + j * rw) * kTileRows));
         }
     }
     uint32_t req_j = my_tiles < (uint32_t)kRing ? my_tiles : (uint32_t)kRing;  // tiles requested so far
@@ -644,6 +638,10 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
     fetch_scales(0);
 
     uint32_t use_j = 0;  // tiles consumed so far
+    // The tile in the ring's first slot: this lane's rows of it and their scales.  (A slot is a multiple of 1024 bytes from
+    // here, so that the block's number changes bits 5 and 6 of the sum as it does of the offset.)
+    const uint32_t at_lo = codes0 + off_lo, at_hi = codes0 + off_hi, at_scales = scales0 + g * 32u;
+    int32_t req_row = (int32_t)(n0 + (rg + req_j * rw) * kTileRows);  // first row of the next tile to ask for
 
     #pragma unroll 1
     for (uint32_t tile0 = 0; tile0 < max_tiles; tile0 += p.pass_tiles) {  // a pass: tiles tile0 ... of every warp
@@ -653,10 +651,11 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
         if (t_pass && mine < 2) peek_t();
         if (t_pass && mine == 0) fetch_t();
 
+        const uint32_t fetch_at = t_pass ? mine - 1 : ~0u;  // the tile before which T is fetched (none in the other warps and passes)
         #pragma unroll 1
         for (uint32_t q = 0; q < mine; ++q) {
             if (t_pass && q + 2 == mine) peek_t();
-            if (t_pass && q + 1 == mine) fetch_t();
+            if (kCarries ? q == fetch_at : t_pass && q + 1 == mine) fetch_t();
             const uint32_t slot = use_j & (kRing - 1);
             if (!lost && !wait_phase(bar0 + 8 * slot, (use_j / kRing) & 1u, p.wait_ns)) {
                 lost = true;
@@ -665,17 +664,20 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
                 ptx::let_flights_land();
             }
             float acc[NT][4];
-            #pragma unroll
-            for (int u = 0; u < NT; ++u) acc[u][0] = acc[u][1] = acc[u][2] = acc[u][3] = 0.0f;
-            #pragma unroll
-            for (int sl = 0; sl < SL; ++sl) {
-                if ((uint32_t)sl < nsl) {
-                    const uint8_t *cs = codes_ring + slot * C::kCodesTile + sl * kCodesSlot;
+            if (!kCarries) {  // (else the first block's products start them)
+                #pragma unroll
+                for (int u = 0; u < NT; ++u) acc[u][0] = acc[u][1] = acc[u][2] = acc[u][3] = 0.0f;
+            }
+            {
+                constexpr int sl = 0;
+                if (kCarries || (uint32_t)sl < nsl) {
+                    const uint32_t lo = at_lo + slot * C::kCodesTile, hi = at_hi + slot * C::kCodesTile;
+                    const uint8_t *cs = smem + (codes0 - kWin0) + slot * C::kCodesTile;
                     uint2 w0[kSliceChunks], w1[kSliceChunks];
                     #pragma unroll
                     for (int c = 0; c < kSliceChunks; ++c) {
-                        w0[c] = *reinterpret_cast<const uint2 *>(cs + (off_lo ^ ((uint32_t)c << 5)));
-                        w1[c] = *reinterpret_cast<const uint2 *>(cs + (off_hi ^ ((uint32_t)c << 5)));
+                        w0[c] = kCarries ? ptx::ld_shared_v2(lo ^ ((uint32_t)c << 5)) : *reinterpret_cast<const uint2 *>(cs + (off_lo ^ ((uint32_t)c << 5)));
+                        w1[c] = kCarries ? ptx::ld_shared_v2(hi ^ ((uint32_t)c << 5)) : *reinterpret_cast<const uint2 *>(cs + (off_hi ^ ((uint32_t)c << 5)));
                     }
                     float s_lo[kSliceChunks], s_hi[kSliceChunks];
                     if (SC == kScalesU8Words) {
@@ -693,9 +695,8 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
                             s_hi[c] = __shfl_sync(0xffffffffu, hi, (lane & ~3u) | c);
                         }
                     } else {
-                        const uint8_t *ss = scales_ring + slot * C::kScaleTile + sl * kScaleSlot + g * 32u;
-                        const float4 a = *reinterpret_cast<const float4 *>(ss);
-                        const float4 b = *reinterpret_cast<const float4 *>(ss + 16u);
+                        const uint32_t ss = at_scales + slot * C::kScaleTile;
+                        const float4 a = ptx::ld_shared_f4(ss), b = ptx::ld_shared_f4(ss + 16u);
                         s_lo[0] = a.x; s_lo[1] = a.y; s_lo[2] = a.z; s_lo[3] = a.w;
                         s_hi[0] = b.x; s_hi[1] = b.y; s_hi[2] = b.z; s_hi[3] = b.w;
                     }
@@ -705,8 +706,12 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
                         fetch_scales(use_j);
                         __syncwarp();
                         if (req_j < my_tiles) {
-                            if (kElects ? ptx::elect_one() != 0 : lane < (NT == 1 ? nsl : 1u)) request(req_j, NT == 1 && !kElects ? lane : 0);
+                            // (it takes the slot that has just been read: its number's)
+                            const uint32_t to = kCarries ? slot : req_j & (kRing - 1);
+                            if (kElects ? ptx::elect_one() != 0 : lane == 0)
+                                ask(bar0 + 8 * to, to, kCarries ? req_row : (int32_t)(n0 + (rg + req_j * rw) * kTileRows));
                             ++req_j;
+                            if (kCarries) req_row += (int32_t)(rw * kTileRows);
                         }
                     }
 
@@ -732,7 +737,7 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
                         for (int u = 0; u < NT; ++u) {
                             #pragma unroll
                             for (int r = 0; r < 4; ++r)
-                                acc[u][r] = fmaf(blk[u][r], r < 2 ? s_lo[c] : s_hi[c], acc[u][r]);
+                                acc[u][r] = c || !kCarries ? fmaf(blk[u][r], r < 2 ? s_lo[c] : s_hi[c], acc[u][r]) : blk[u][r] * (r < 2 ? s_lo[c] : s_hi[c]);
                         }
                     }
                 }
