@@ -34,9 +34,10 @@
 // With a stage at a time the skeleton alone, no look-ups, no stores, a quarter of the MMAs, took 0.29 us a stage: the one lane that
 // asked for the activations spent 300 to 440 cycles on each, and scales loaded by the threads another 0.05 us.  Before ->
 // now, whole calls: 64 x 4096 x 4096 20.6 -> 16.5 us, 128 x 8192 x 8192 37.7 -> 28.6, 203 x 3584 x 18944 36.8 -> 34.7, 512 x 4096 x 4096
-// 32.0 -> 25.9, 2048 x 4096 x 14336 209.9 -> 208.0; the GEMM of a backward over 2048 x 4096 x 14336 167 -> 151.
+// 32.0 -> 26.8, 2048 x 4096 x 14336 209.9 -> 208.0; the GEMM of a backward over 2048 x 4096 x 14336 167 -> 151.
 // The start counts for few rows: most CTAs start when the pre-pass's end, so the codes of the first steps are asked for
-// before anything else is set up, and the CTAs of a pair meet without a release (1.2 us): 512 x 4096 x 4096 19.4 -> 16.8 us.
+// before anything else is set up: 512 x 4096 x 4096 19.4 -> 17.6 us.  The CTAs of a pair meet with a release and an acquire by
+// all threads, at the start and at the end (relaxed arrivals would save 0.5 us at each).
 //
 // The MMA computes D[n, m] = sum_k W[n, k] x[m, k]: weight rows are the MMA's M (TMEM lanes),
 // activation rows its N (256 accumulator columns).  Both operands are f16 with f32 accumulation:
@@ -416,13 +417,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         ptx::tmem_alloc_pair(own | kTmemSlotAt, kTmemCols);
         ptx::tmem_relinquish_pair();
     }
-    // The barriers of both CTAs are in place (their initialisation is fenced for the cluster by the threads that made it; a
-    // release by all threads took 1.2 us), and this CTA's table.
-    __syncwarp();
-    ptx::cluster_arrive_relaxed();
+    // The barriers and the tensor memory of both CTAs are in place, and this CTA's table.
     ptx::tc_fence_before();
-    __syncthreads();
-    ptx::cluster_wait();
+    __syncwarp();
+    ptx::cluster_sync_all();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *reinterpret_cast<const uint32_t *>(at(kTmemSlotAt));
     const uint32_t tmem_acc = tmem_base;             // columns [0, 256)
@@ -930,8 +928,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     __syncwarp();
     // neither CTA leaves, or gives its tensor memory back, while the other may still signal it
     ptx::tc_fence_before();
-    ptx::cluster_arrive_relaxed();
-    ptx::cluster_wait();
+    ptx::cluster_sync_all();
     if (warp == 1) {
         ptx::tc_fence_after();
         ptx::tmem_dealloc_pair(tmem_base, kTmemCols);

@@ -318,9 +318,6 @@ __device__ __forceinline__ uint32_t cluster_cta_rank() {
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// The same in halves, without a release: for what a fence of its own orders (barriers' initialisation), or nothing.
-__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // The shared::cluster address of this CTA's shared-memory address `addr` in CTA `rank`.
 __device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
     uint32_t r;
