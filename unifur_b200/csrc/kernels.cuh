@@ -44,8 +44,6 @@ uint64_t lora_workspace_bytes(uint64_t rows, uint32_t rank);
 int32_t lora_forward(const void *x, uint64_t rows, uint64_t d_in, uint64_t d_out, const void *a, const void *b,
                      uint32_t rank, float scale, int32_t layout, int32_t io_dtype, void *y, uint64_t ldy,
                      float *t, cudaStream_t s);
-int32_t lora_intermediate(const void *x, const void *a, float *t, uint64_t rows, uint64_t d_in, uint32_t rank,
-                          int32_t layout, int32_t io_dtype, cudaStream_t s);
 int32_t lora_delta(const void *a, const void *b, const uint8_t *packed, const float *absmax,
                    const uint8_t *scale_codes, const float *scale_of_scales, uint64_t d_in, uint64_t d_out,
                    uint32_t rank, float scale, int32_t layout, int32_t io_dtype, float *out, cudaStream_t s);
