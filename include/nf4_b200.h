@@ -354,6 +354,11 @@ NF4_API int32_t nf4_decode_share_plan(uint32_t rows, uint32_t d_in, uint32_t d_o
 NF4_API int32_t nf4_prefill_share_plan(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t cta, uint32_t *ctas,
                                        uint32_t *segments, uint32_t capacity);
 
+/* Where that kernel puts the packed codes of a pair's main step number `block` (two k-stages each, numbered over its segments): the
+ * slot of its shared-memory ring, the barrier that counts their landing, and the parity of that barrier's round.  Returns
+ * the ring's slots.  For inspection and tests; the reference has no counterpart. */
+NF4_API int32_t nf4_prefill_code_place(uint32_t block, uint32_t slot_full_parity[3]);
+
 /* How the kernels that share a tile's work out over a cluster of CTAs (the pre-pass of the tensor-core
  * kernel, the adapter gradients) choose its size, computed on the host: 1, 2, 4, 8 or 16 CTAs for `tiles`
  * tiles whose `length` is divided into pieces of `unit` or more.  room[i]: clusters of 2^i CTAs that the

@@ -50,3 +50,30 @@ def test_steps(M, K, N, r, layout, f32, double):
     per_column = ((y - ref).norm(dim=0) / ref.norm(dim=0)).max()
     assert float(per_column) < (1e-3 if f32 else 4e-3)
     assert torch.equal(y, base.forward(x).double())  # results do not depend on timing
+
+
+@pytest.mark.parametrize("M,K,N,r,layout,f32,double", [
+    (100, 4096, 4096, 16, 0, False, False),   # narrow tiles: scales by TMA, a chunk of the adapter
+    (64, 3584, 9472, 136, 0, False, True),    # u8 scales loaded, three chunks
+    (48, 2048, 20480, 8, 0, False, True),     # u8 scales by TMA, more tiles than pairs
+    (128, 4160, 4096, 136, 1, False, False),  # a scale for every k, three chunks, an odd last step
+    (100, 1024, 20480, 8, 1, True, False),    # the same of f32 tensors, tiles divided between pairs
+    (600, 4096, 10240, 64, 0, False, False),  # wide tiles
+])
+def test_codes_that_come_late(M, K, N, r, layout, f32, double):
+    # the codes' copies land from a cold L2 and in no order; the ring's protocol is tests/test_code_ring.py's
+    from unifur_b200.quantize import PackedNf4Tensor
+    from unifur_b200.qwennet import Nf4Linear, QloraLinear
+
+    dt = torch.float32 if f32 else torch.bfloat16
+    gen = torch.Generator(device=DEV).manual_seed(M + N)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=gen)  # noqa: E731
+    packed = PackedNf4Tensor.quantize(rnd(K * N) * 0.02)
+    base = Nf4Linear(packed.with_double_quantization() if double else packed, K, N, None, layout)
+    a, b = ((r, K), (N, r)) if layout == 0 else ((K, r), (r, N))
+    q = QloraLinear(base, (rnd(*a) * 0.1).to(dt), (rnd(*b) * 0.1).to(dt), 1.5)
+    x, flush = rnd(M, K).to(dt), torch.empty(1 << 28, dtype=torch.uint8, device=DEV)
+    first = q.forward(x)
+    for i in range(20):
+        flush.fill_(i)
+        assert torch.equal(q.forward(x), first)

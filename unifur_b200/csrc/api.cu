@@ -733,6 +733,11 @@ int32_t nf4_decode_share_plan(uint32_t rows, uint32_t d_in, uint32_t d_out, uint
     return n;
 }
 
+int32_t nf4_prefill_code_place(uint32_t block, uint32_t slot_full_parity[3]) {
+    if (!slot_full_parity) return fail(NF4_ERR_INVALID_ARG, "nf4_prefill_code_place: null output");
+    return prefill_code_place(block, slot_full_parity);
+}
+
 int32_t nf4_prefill_share_plan(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t cta, uint32_t *ctas,
                                uint32_t *segments, uint32_t capacity) {
     if (!segments && capacity) return fail(NF4_ERR_INVALID_ARG, "nf4_prefill_share_plan: null segments");

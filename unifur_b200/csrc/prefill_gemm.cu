@@ -131,8 +131,21 @@ __device__ __forceinline__ uint32_t scales_place(uint32_t slot) {
 // MMAs over, in both CTAs: whatever the step's slots held is free.  Steps number on over a pair's segments,
 // the adapter's included; step c has barriers c % kBarRing and weight columns c % kASteps.
 constexpr int kBarFull = 0, kBarDone = kBarFull + kBarRing, kBarAccFull = kBarDone + kBarRing, kBarAccEmpty = kBarAccFull + 1,
-              kBarCFull = kBarAccEmpty + 1, kBarCEmpty = kBarCFull + kCodeSlots, kNumBars = kBarCEmpty + kCodeSlots;
+              kBarCFull = kBarAccEmpty + 1, kBarCEmpty = kBarCFull + 2 * kCodeSlots, kNumBars = kBarCEmpty + kCodeSlots;
 static_assert(kBarsAt + kNumBars * 8 <= kTmemSlotAt, "barrier room");
+
+// Where the codes of a main step go.  Blocks number on over a pair's segments, without the adapter's steps.  A slot's rounds are told
+// apart by two barriers in turn: a warp that dequantises takes every other step, so that it does not see every round of a slot, and
+// with one barrier a slot a wait for block b passed at once, with the parity of b - 6, while b - 3 was still under way.  The barrier of
+// block b had block b - 6 before; that one has landed whenever a warp comes to wait for b: at its turn before this one, two steps
+// back, it waited for the MMAs of the step four before that.
+struct CodePlace {
+    uint32_t slot, full, parity;  // of the ring, its barrier among the kBarCFull ones, the parity of the block's round on it
+};
+__host__ __device__ __forceinline__ CodePlace code_place(uint32_t block) {
+    const uint32_t round = block / kCodeSlots, slot = block - round * kCodeSlots;
+    return {slot, slot + (round & 1u) * kCodeSlots, (round >> 1) & 1u};
+}
 
 struct PrefillParams {
     const uint8_t *codes;
@@ -312,12 +325,13 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     // A step's codes (and scales) go to a slot of their ring; the L2 is asked for eight stages at a time, some twenty
     // ahead of their loads (weights that nobody has touched yet come from HBM).
     constexpr uint32_t kAhead = 3, kUnit = 8;  // requests to the L2 ahead, and stages of each
-    auto ask_codes = [&](uint32_t ks, int32_t n0, uint32_t slot) {
-        ptx::mbar_arrive_expect_tx(bar(kBarCFull + slot), kCodeTileBytes + (PERK ? kPerKBytes : SCALES == kScalesTma ? kScaleTileBytes : 0));
-        ptx::tma_load_2d((own | kCodesAt) + slot * kCodeTileBytes, &tmap_w, (int32_t)(ks * (BK / 2)), n0, bar(kBarCFull + slot));
+    auto ask_codes = [&](uint32_t ks, int32_t n0, const CodePlace &c) {
+        const uint32_t full = bar(kBarCFull + c.full);
+        ptx::mbar_arrive_expect_tx(full, kCodeTileBytes + (PERK ? kPerKBytes : SCALES == kScalesTma ? kScaleTileBytes : 0));
+        ptx::tma_load_2d((own | kCodesAt) + c.slot * kCodeTileBytes, &tmap_w, (int32_t)(ks * (BK / 2)), n0, full);
         if (SCALES == kScalesTma)
-            ptx::tma_load_2d(own | scales_place(slot), &tmap_s, (int32_t)(p.absmax ? ks & ~3u : ks & ~15u), n0, bar(kBarCFull + slot));
-        if (PERK) ptx::tma_load_2d(own | scales_place(slot), &tmap_s, (int32_t)(ks * BK), n0 / 64, bar(kBarCFull + slot));
+            ptx::tma_load_2d(own | scales_place(c.slot), &tmap_s, (int32_t)(p.absmax ? ks & ~3u : ks & ~15u), n0, full);
+        if (PERK) ptx::tma_load_2d(own | scales_place(c.slot), &tmap_s, (int32_t)(ks * BK), n0 / 64, full);
     };
     auto ask_l2 = [&](uint32_t ks, int32_t n0) { ptx::tma_prefetch_2d(&tmap_ahead, (int32_t)(ks * (BK / 2)), n0); };
     uint32_t asked = 0;  // steps of the first segment whose codes are on their way before anything else is in place
@@ -326,14 +340,12 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         if (!PERK && wl.n_seg) wl.get(0, tile, kb, ke);
         asked = min((ke - kb + 1) / 2, (uint32_t)kCodeSlots);
         if (ptx::elect_one()) {
-            for (int s = 0; s < kCodeSlots; ++s) {
-                ptx::mbar_init(bar(kBarCFull + s), 1);
-                ptx::mbar_init(bar(kBarCEmpty + s), 8);   // the warps that dequantise a step
-            }
+            for (int s = 0; s < 2 * kCodeSlots; ++s) ptx::mbar_init(bar(kBarCFull + s), 1);
+            for (int s = 0; s < kCodeSlots; ++s) ptx::mbar_init(bar(kBarCEmpty + s), 8);   // the warps that dequantise a step
             ptx::fence_mbar_init();
             ptx::fence_proxy_async();
             const int32_t n0 = (int32_t)(((tile / p.m_tiles) * 2 + rank) * BM);
-            for (uint32_t i = 0; i < asked; ++i) ask_codes(kb + 2 * i, n0, i);
+            for (uint32_t i = 0; i < asked; ++i) ask_codes(kb + 2 * i, n0, code_place(i));
             for (uint32_t k = kb; k < min(ke, kb + kAhead * kUnit); k += kUnit) ask_l2(k, n0);
         }
         __syncwarp();
@@ -814,7 +826,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
 
         // A group has every other step, the adapter's and the missing half of an odd last one included (nothing to write
         // there, but its turn on the barriers): then it is never two rounds of Done ahead, where a parity would be the wrong
-        // round's.
+        // round's, nor of the codes' barriers (see code_place).
         uint32_t before = 0, blocks = 0;  // steps, and main ones, before the segment
         const uint32_t swizzle = (row_in_tile >> 1) & 3u, row_at = (own | kCodesAt) + row_in_tile * 64u;
         const uint32_t chunk0 = row_at + (((half * 2) ^ swizzle) << 4), chunk1 = row_at + (((half * 2 + 1) ^ swizzle) << 4);
@@ -830,8 +842,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             wl.get(seg, tile, kb, ke);
             const uint32_t steps = (ke - kb + 1) / 2;
             for (uint32_t j = (odd - before) & 1u; j < steps && ok; j += 2) {
-                const uint32_t step = before + j, block = blocks + j, slot = block % kCodeSlots;
-                if (!ptx::mbar_wait_suspended(bar(kBarCFull + slot), (block / kCodeSlots) & 1u)) {
+                const uint32_t step = before + j;
+                const CodePlace c = code_place(blocks + j);
+                const uint32_t slot = c.slot;
+                if (!ptx::mbar_wait_suspended(bar(kBarCFull + c.full), c.parity)) {
                     ok = false;
                     break;
                 }
@@ -892,7 +906,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     if (warp == kCodeWarp) {
         // ========================= packed codes =========================
         if (PERK) ptx::pdl_wait();
-        uint32_t slot = asked % kCodeSlots, round = asked / kCodeSlots;
+        uint32_t block = asked;
         for (uint32_t seg = 0; seg < wl.n_seg && ok; ++seg) {
             uint32_t tile, kb, ke;
             wl.get(seg, tile, kb, ke);
@@ -908,17 +922,16 @@ prefill_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                     __syncwarp();
                     continue;
                 }
-                ok = ptx::mbar_wait_suspended(bar(kBarCEmpty + slot), (round & 1u) ^ 1u);
+                // (every block in turn: a round of the slot's Empty is never passed by)
+                const CodePlace c = code_place(block);
+                ok = ptx::mbar_wait_suspended(bar(kBarCEmpty + c.slot), (block / kCodeSlots & 1u) ^ 1u);
                 if (!ok) break;
                 if (ptx::elect_one()) {
-                    ask_codes(ks, n0, slot);
+                    ask_codes(ks, n0, c);
                     if (to_l2) ask_l2(ahead, n0);
                 }
                 __syncwarp();
-                if (++slot == kCodeSlots) {
-                    slot = 0;
-                    ++round;
-                }
+                ++block;
             }
         }
         if (!ok && lane == 0) NF4_REPORT_FAILURE(g_prefill_error, g_prefill_error_host, 7);
@@ -1449,6 +1462,14 @@ int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_o
 
 int32_t prefill_set_host_flag(int *mapped) {
     return check_cuda(cudaMemcpyToSymbol(g_prefill_error_host, &mapped, sizeof(mapped)), "setting the mapped failure word");
+}
+
+int32_t prefill_code_place(uint32_t block, uint32_t *slot_full_parity) {
+    const CodePlace c = code_place(block);
+    slot_full_parity[0] = c.slot;
+    slot_full_parity[1] = c.full;
+    slot_full_parity[2] = c.parity;
+    return kCodeSlots;
 }
 
 // The sharing of the tiles as the kernel will see it, for inspection on the host, in tiles of 128 weight rows x
