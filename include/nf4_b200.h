@@ -341,18 +341,21 @@ NF4_API int32_t nf4_decode_share_plan(uint32_t rows, uint32_t d_in, uint32_t d_o
                                       uint32_t *k0_k1_n0_n1);
 
 /* How the tensor-core kernel (more than 16 rows) shares a forward's tiles out between its
- * CTAs, computed on the host (no GPU needed).  Two CTAs work on 256 weight rows x 256 activation rows
+ * CTAs where it takes tiles of 256 activation rows, computed on the host (no GPU needed).  Two CTAs work on 256 weight rows x 256 activation rows
  * together, 128 of the weight rows each; tiles are counted here in those halves, CTAs with the first
  * of every pair before the second ones.  *ctas receives the number of CTAs; segments
  * receives, for CTA `cta`, up to `capacity` triples (tile, first main k-stage, one past the last)
  * in the order the CTA works on them.  Returns the number of the CTA's segments, or a negative
  * status.  Tiles that appear with a partial range of k-stages are split between neighbouring
  * pairs of CTAs (the one with the last stages finishes the tile).  Up to 128 rows the tiles have 128
- * activation rows.  Where more rows make few tiles, a forward may instead give each of up to 74 pairs one whole
- * tile of 128 activation rows; the plan is then the one it would follow with tiles of 256.  For inspection and tests; the
- * reference has no counterpart. */
+ * activation rows.  Where more rows make few tiles, a forward may take tiles of 128 rows as well: the plan that it
+ * follows is nf4_prefill_forward_plan's.  For inspection and tests; the reference has no counterpart. */
 NF4_API int32_t nf4_prefill_share_plan(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t cta, uint32_t *ctas,
                                        uint32_t *segments, uint32_t capacity);
+
+/* The same as a forward of this shape has it: *tile_rows receives the activation rows of a tile, 128 or 256. */
+NF4_API int32_t nf4_prefill_forward_plan(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t cta, uint32_t *tile_rows, uint32_t *ctas,
+                                         uint32_t *segments, uint32_t capacity);
 
 /* Where that kernel puts the packed codes of a pair's main step number `block` (two k-stages each, numbered over its segments): the
  * slot of its shared-memory ring, the barrier that counts their landing, and the parity of that barrier's round.  Returns

@@ -56,6 +56,50 @@ def test_every_stage_once_and_neighbours_share(rows, d_in, d_out):
     assert max(loads) - min(loads) <= ks             # nobody has a whole tile more than anybody else
 
 
+NARROW = [  # more than 128 rows in tiles of 128
+    (512, 4096, 4096), (2050, 2112, 64), (129, 1024, 9472), (200, 64, 8), (640, 3584, 3584), (224, 3584, 9472), (300, 1088, 640),
+]
+
+
+def _forward_plan(rows, d_in, d_out):
+    L = _lib.load()
+    ctas, height, cap = ctypes.c_uint32(0), ctypes.c_uint32(0), 4096
+    seg = (ctypes.c_uint32 * (3 * cap))()
+    assert L.nf4_prefill_forward_plan(rows, d_in, d_out, 0, ctypes.byref(height), ctypes.byref(ctas), seg, cap) >= 0
+    assert 1 <= ctas.value <= 148
+    out = []
+    for c in range(ctas.value):
+        n = L.nf4_prefill_forward_plan(rows, d_in, d_out, c, None, None, seg, cap)
+        assert 0 <= n <= cap
+        out.append([(seg[3 * j], seg[3 * j + 1], seg[3 * j + 2]) for j in range(n)])
+    return height.value, out
+
+
+@pytest.mark.parametrize("rows,d_in,d_out", SHAPES + NARROW)
+def test_what_a_forward_follows(rows, d_in, d_out):
+    height, plan = _forward_plan(rows, d_in, d_out)
+    if (rows, d_in, d_out) in NARROW or rows <= 128:
+        assert height == 128
+    ks = d_in // 64
+    tiles = ((rows + height - 1) // height) * ((d_out + 127) // 128)
+    pieces = {}
+    for c, segs in enumerate(plan):
+        unfinished = [j for j, (_t, _b, e) in enumerate(segs) if e != ks]
+        assert len(unfinished) <= 1 and (not unfinished or unfinished[0] == 0)
+        for tile, b, e in segs:
+            assert tile < tiles and 0 <= b < e <= ks
+            assert ks % 2 or (b % 2 == 0 and e % 2 == 0)   # whole steps of two stages, where a tile consists of them
+            pieces.setdefault(tile, []).append((b, e, c))
+    assert sorted(pieces) == list(range(tiles))
+    for ps in pieces.values():
+        ps.sort()
+        assert ps[0][0] == 0 and ps[-1][1] == ks
+        for (_b0, e0, c0), (b1, _e1, c1) in zip(ps, ps[1:]):
+            assert e0 == b1 and c1 == c0 + 1
+    if rows > 128 and height == 128:
+        assert all(len(segs) <= 1 and (not segs or segs[0][1:] == (0, ks)) for segs in plan)  # one whole tile at most
+
+
 def test_rejects_what_the_kernel_does_not_take():
     L = _lib.load()
     seg = (ctypes.c_uint32 * 3)()

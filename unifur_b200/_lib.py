@@ -110,6 +110,7 @@ SIGNATURES = {
     "nf4_linear_forward_grouped_dev": (_i32, [C.POINTER(LinearArgs), _u32, _vp]),
     "nf4_reserve_sms": (_i32, [_i32]),
     "nf4_decode_share_plan": (_i32, [_u32, _u32, _u32, _u32, _u32, C.POINTER(_u32)]),
+    "nf4_prefill_forward_plan": (_i32, [_u64, _u64, _u64, _u32, C.POINTER(_u32), C.POINTER(_u32), C.POINTER(_u32), _u32]),
     "nf4_prefill_code_place": (_i32, [_u32, C.POINTER(_u32)]),
     "nf4_prefill_share_plan": (_i32, [_u64, _u64, _u64, _u32, C.POINTER(_u32), C.POINTER(_u32), _u32]),
     "nf4_cluster_share_plan": (_i32, [_u64, _u64, _u64, C.POINTER(_u32)]),

@@ -741,8 +741,16 @@ int32_t nf4_prefill_code_place(uint32_t block, uint32_t slot_full_parity[3]) {
 int32_t nf4_prefill_share_plan(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t cta, uint32_t *ctas,
                                uint32_t *segments, uint32_t capacity) {
     if (!segments && capacity) return fail(NF4_ERR_INVALID_ARG, "nf4_prefill_share_plan: null segments");
-    const int32_t n = prefill_share_plan(rows, d_in, d_out, cta, ctas, segments, capacity);
+    const int32_t n = prefill_share_plan(rows, d_in, d_out, true, cta, nullptr, ctas, segments, capacity);
     if (n < 0) return fail(NF4_ERR_INVALID_ARG, "nf4_prefill_share_plan: not a shape of the tensor-core kernel, or no such CTA");
+    return n;
+}
+
+int32_t nf4_prefill_forward_plan(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t cta, uint32_t *tile_rows, uint32_t *ctas,
+                                 uint32_t *segments, uint32_t capacity) {
+    if (!segments && capacity) return fail(NF4_ERR_INVALID_ARG, "nf4_prefill_forward_plan: null segments");
+    const int32_t n = prefill_share_plan(rows, d_in, d_out, false, cta, tile_rows, ctas, segments, capacity);
+    if (n < 0) return fail(NF4_ERR_INVALID_ARG, "nf4_prefill_forward_plan: not a shape of the tensor-core kernel, or no such CTA");
     return n;
 }
 

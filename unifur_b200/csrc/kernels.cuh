@@ -163,7 +163,7 @@ bool prefill_supported(const nf4_linear_args &a);
 bool prefill_in_out_supported(const nf4_linear_args &a);
 uint64_t prefill_workspace_bytes(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t lora_rank);
 int32_t prefill_code_place(uint32_t block, uint32_t *slot_full_parity);
-int32_t prefill_share_plan(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t cta, uint32_t *ctas,
+int32_t prefill_share_plan(uint64_t rows, uint64_t d_in, uint64_t d_out, bool wide_only, uint32_t cta, uint32_t *tile_rows, uint32_t *ctas,
                            uint32_t *segments, uint32_t cap);
 // r_out: null, or where x A goes too (see PrepassArgs)
 int32_t prefill_forward(const nf4_linear_args &a, cudaStream_t stream, void *r_out = nullptr);

@@ -1472,14 +1472,15 @@ int32_t prefill_code_place(uint32_t block, uint32_t *slot_full_parity) {
     return kCodeSlots;
 }
 
-// The sharing of the tiles as the kernel will see it, for inspection on the host, in tiles of 128 weight rows x
-// 256 activation rows, one CTA's part of a pair's tile.  CTAs are counted with the even ones of all pairs
-// first: CTA `cta` is CTA cta / pairs of pair cta % pairs.  Returns the number of the CTA's segments (at
-// most `cap` are written), or -1.
-int32_t prefill_share_plan(uint64_t rows, uint64_t d_in, uint64_t d_out, uint32_t cta, uint32_t *ctas,
+// The sharing of the tiles, for inspection on the host, in tiles of 128 weight rows x *tile_rows activation rows, one CTA's part of a
+// pair's tile: as a forward has it, or (wide_only) as it would be with 256 rows to a tile wherever there are more than 128.  CTAs are
+// counted with the even ones of all pairs first: CTA `cta` is CTA cta / pairs of pair cta % pairs.  Returns the number of the CTA's
+// segments (at most `cap` are written), or -1.
+int32_t prefill_share_plan(uint64_t rows, uint64_t d_in, uint64_t d_out, bool wide_only, uint32_t cta, uint32_t *tile_rows, uint32_t *ctas,
                            uint32_t *segments, uint32_t cap) {
     if (rows <= 16 || d_in % BK != 0 || d_in == 0 || d_out == 0) return -1;
-    const Sharing sh = share_tiles(rows, d_in, d_out, true);
+    const Sharing sh = share_tiles(rows, d_in, d_out, wide_only);
+    if (tile_rows) *tile_rows = sh.bn;
     if (ctas) *ctas = 2 * sh.pairs;
     if (cta >= 2 * sh.pairs) return -1;
     const uint32_t rank = cta / sh.pairs, m_tiles = (uint32_t)((rows + sh.bn - 1) / sh.bn);
