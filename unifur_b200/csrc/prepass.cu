@@ -404,6 +404,7 @@ prepass_f32_kernel(const Params p) {
     __shared__ float s_inv[kRows];
     __shared__ __align__(16) float s_part[8][kRows][kPartRow];  // the warps' sums of sixteen ranks
     __shared__ __align__(16) float s_sum[kRows][kSumRow];       // this CTA's of all
+    extern __shared__ __align__(16) float s_all[];              // the CTAs', of this one's share of the rows [cn][32 / cn][kSumRow]
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, g = lane >> 2, t = lane & 3u;
     const uint32_t cn = cluster.num_blocks(), rank_in = cluster.block_rank();
     const uint32_t m0 = (blockIdx.x / cn) * kRows, k0 = min(rank_in * p.piece, p.K), k1 = min(k0 + p.piece, p.K);
@@ -584,19 +585,29 @@ prepass_f32_kernel(const Params p) {
     }
 
     // ---- the CTAs' sums, each CTA a share of the rows; columns the adapter does not have are zeros ----
+    // A row's sums go to the CTA whose share it is in, so that one meeting does: behind it nobody touches another CTA's memory.  (The
+    // sums read from where they are, with a second meeting before a CTA leaves: 512 x 4096 x 4096 at rank 16 33.6 us instead of 32.8.)
+    const uint32_t per = kRows / cn, rank_quads = p.rank / 4;  // (the rank is a multiple of four)
+    for (uint32_t i = tid; i < kRows * rank_quads; i += kThreads) {
+        const uint32_t r = i / rank_quads, c = i % rank_quads * 4;
+        float *const to = cluster.map_shared_rank(s_all, r / per) + (rank_in * per + r % per) * kSumRow + c;
+        *reinterpret_cast<float4 *>(to) = *reinterpret_cast<const float4 *>(&s_sum[r][c]);
+    }
+    __syncwarp();  // (lanes come from loops of different length)
     cluster.barrier_arrive();
     copy(kp);
+    __syncwarp();
     cluster.barrier_wait();
     const float w_down = ldexpf(1.0f, -w_exp);
-    const uint32_t per = (kRows + cn - 1) / cn, quads = 16 * p.chunks, ld = 2 * 64 * p.chunks;
+    const uint32_t quads = 16 * p.chunks, ld = 2 * 64 * p.chunks;
     for (uint32_t i = tid; i < per * quads; i += kThreads) {
-        const uint32_t r = rank_in * per + i / quads, c = i % quads * 4, m = m0 + r;
-        if (r >= kRows || m >= p.M || (c >= p.rank && c < 2 * p.rank)) continue;  // (the rank is a multiple of four)
+        const uint32_t r = i / quads, c = i % quads * 4, m = m0 + rank_in * per + r;
+        if (m >= p.M || (c >= p.rank && c < 2 * p.rank)) continue;
         float sum[4] = {};
         if (c < p.rank) {
             #pragma unroll 4
             for (uint32_t q = 0; q < cn; ++q) {
-                const float4 w = *reinterpret_cast<const float4 *>(cluster.map_shared_rank(&s_sum[0][0], q) + r * kSumRow + c);
+                const float4 w = *reinterpret_cast<const float4 *>(s_all + (q * per + r) * kSumRow + c);
                 sum[0] += w.x;
                 sum[1] += w.y;
                 sum[2] += w.z;
@@ -607,8 +618,6 @@ prepass_f32_kernel(const Params p) {
         put_halves(p.t_out, sum, p.scale * w_down, (size_t)m * ld + c, 64 * p.chunks);
         if (c < p.rank) put_halves(p.t_out, sum, p.scale * w_down, (size_t)m * ld + p.rank + c, 64 * p.chunks);
     }
-    __syncwarp();  // (lanes come from loops of different length)
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");  // the sums have been read
 }
 
 // ---- the same for bf16 x and a factor on tcgen05: up to 64 ranks, rows of 16-byte pieces -------------------------------
@@ -862,7 +871,7 @@ prepass_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     }
     ptx::tc_fence_before();
     __syncwarp();  // (lanes come from loops of different length)
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");  // the sums have been read
+    ptx::cluster_sync_all();  // the sums have been read, before a CTA leaves (a relaxed arrival would not say so)
     if (warp == 9) {
         ptx::tc_fence_after();
         ptx::tmem_dealloc(acc, 64);
@@ -969,7 +978,7 @@ int32_t activations_prepass(const PrepassArgs &q, cudaStream_t stream) {
                           : (q.xh ? prepass_kernel<0, 32, k_major> : prepass_kernel<2, 32, k_major>);
     };
     auto kernel = q.k_major ? pick(std::true_type{}) : pick(std::false_type{});
-    const int smem = q.x_f32 ? 0 : (int)(stages_of(rows) * stage_bytes(rows));
+    const int smem = (int)(q.x_f32 ? rows * kSumRow * sizeof(float) : stages_of(rows) * stage_bytes(rows));
     // as many CTAs of K as the chip holds at once, two on an SM (a second wave took 21 us where one takes 11; of f32 [4096, 4096]
     // two CTAs to a cluster 40 us, eight, whose pieces are read once, 45; [4096, 14336] 121 and, sixteen, 154)
     ClusterRoom room;
