@@ -1186,14 +1186,35 @@ namespace {
 // (every pair the same number of stages, a tile possibly split between neighbours), the other
 // pairs * dp_rounds tiles go out whole.  With a tile count that is a multiple of the pairs nothing
 // is split.  Otherwise the last round of whole tiles would leave most pairs idle, so the last full round and
-// the remainder are divided by stages instead.  Fewer tiles than pairs: what of three takes the shortest by the times
-// measured (a stage 0.28 us in wide tiles, 0.2 in narrow ones, however many columns it has): whole tiles, read out in 3 us; `split` pairs
-// to a tile, whose sums a kernel of its own adds (dump 3.5, launch and sum 4.5 us); or divided by stages, every pair 24 at least, with a
-// tile's last pair collecting (3 us of dump, and 2 a helper).
+// the remainder are divided by stages instead.  Fewer tiles than pairs: what of three takes the shortest (SharingCost): whole tiles;
+// `split` pairs to a tile, whose sums a kernel of its own adds; or divided by stages, every pair 24 at least, with a tile's last pair
+// collecting.
 struct Sharing {
     uint32_t bn;  // activation rows of a tile
     uint32_t pairs, sk_tiles, dp_rounds, split;
     uint64_t cost;  // ns, if there are fewer tiles than pairs
+};
+// What a way to share fewer tiles than pairs takes, in ns, beside what all have in common: fitted to 3200 calls, back to back, of 450
+// sizes from 17 x 256 x 256 to 1200 x 20480 x 20480 in both orientations and types, each in up to eight ways.  A stage is the dequantisers'
+// time, or in a tile of many columns the MMAs'.  A read-out, or a dump, and the sums' launch grow with a tile's columns, the sums with
+// all pairs' columns; and the more pairs, the fewer of their CTAs find an SM beside the pre-pass, to set themselves up in its shadow.
+// Before, with 200 or 280 ns a stage whatever the columns and no word of the pairs -> now: 146 x 2176 x 1024 16.4 -> 15.4 us, 117 x 7680 x
+// 704 24.2 -> 16.9, 62 x 1792 x 640 in the other orientation 16.3 -> 14.9, 1155 x 5888 x 2560 49.6 -> 43.2.  Of the 450 sizes 77 gain more
+// than 2 %, 1.35 % on average; 15 lose more than 2 %, the most 10 % (22.2 -> 24.5 us).
+struct SharingCost {
+    uint64_t columns, stage;  // of a tile
+    SharingCost(uint32_t bn, uint64_t rows) : columns(rows > bn ? bn : (rows + 31) / 32 * 32), stage(165) {
+        if (bn > 128 && columns * 275 / 256 > stage) stage = columns * 275 / 256;
+    }
+    uint64_t work(uint64_t stages, uint64_t pairs) const { return stages * stage + pairs * 2100 / (kNumSMs / 2); }
+    uint64_t read_out() const { return columns * 8400 / 256; }
+    uint64_t whole(uint64_t ks, uint64_t tiles) const { return work(ks, tiles) + read_out(); }
+    uint64_t split(uint64_t ks, uint64_t tiles, uint64_t s) const {
+        return work((ks + s - 1) / s, tiles * s) + 2700 + columns * 5900 / 256 + tiles * s * columns * 2700 / (kNumSMs / 2 * 256);
+    }
+    uint64_t by_stages(uint64_t ks, uint64_t tiles, uint64_t pairs) const {
+        return work(tiles * ks / pairs, pairs) + read_out() + 4000 + (pairs + tiles - 1) / tiles * 2200;
+    }
 };
 Sharing share_tiles_of(uint32_t bn, uint64_t rows, uint64_t d_in, uint64_t d_out) {
     const uint64_t tiles = ((rows + bn - 1) / bn) * ((d_out + 2 * BM - 1) / (2 * BM)), ks = d_in / BK;
@@ -1202,19 +1223,18 @@ Sharing share_tiles_of(uint32_t bn, uint64_t rows, uint64_t d_in, uint64_t d_out
     sh.split = 1;
     uint64_t pairs = kNumSMs / 2;
     if (tiles < pairs) {
-        const bool narrow = bn < 256;
-        const uint64_t kStage = narrow ? 200 : 280, kReadOut = narrow ? 2000 : 3000, kDump = narrow ? 2500 : 3500, kSum = 4500, kHelper = 2000;
+        const SharingCost cost_of(bn, rows);
         const uint64_t by_stages = tiles * ks / 24, shared = by_stages < pairs ? by_stages : pairs;
-        uint64_t least = ks * kStage + kReadOut, most = pairs / tiles;
+        uint64_t least = cost_of.whole(ks, tiles), most = pairs / tiles;
         if (shared > tiles) {
-            const uint64_t cost = tiles * ks * kStage / shared + 2 * kReadOut + (shared + tiles - 1) / tiles * kHelper;
+            const uint64_t cost = cost_of.by_stages(ks, tiles, shared);
             if (cost < least) {
                 least = cost;
                 sh.split = 0;
             }
         }
         for (uint64_t s = 2; s <= most && s * 4 <= ks; ++s) {
-            const uint64_t cost = (ks + s - 1) / s * kStage + kDump + kSum;
+            const uint64_t cost = cost_of.split(ks, tiles, s);
             if (cost < least) {
                 least = cost;
                 sh.split = (uint32_t)s;
@@ -1245,8 +1265,8 @@ Sharing share_tiles(uint64_t rows, uint64_t d_in, uint64_t d_out, bool wide_only
     if (rows <= 128) return share_tiles_of(128, rows, d_in, d_out);
     const Sharing wide = share_tiles_of(256, rows, d_in, d_out);
     if (wide_only || !wide.cost) return wide;
-    const uint64_t tiles = ((rows + 127) / 128) * ((d_out + 2 * BM - 1) / (2 * BM)), cost = d_in / BK * 200 + 2000;
-    if (tiles > kNumSMs / 2 || cost >= wide.cost) return wide;
+    const uint64_t tiles = ((rows + 127) / 128) * ((d_out + 2 * BM - 1) / (2 * BM));
+    if (tiles > kNumSMs / 2 || SharingCost(128, rows).whole(d_in / BK, tiles) >= wide.cost) return wide;
     Sharing sh{};
     sh.bn = 128;
     sh.split = sh.dp_rounds = 1;
