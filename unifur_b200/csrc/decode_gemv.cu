@@ -237,22 +237,24 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
     constexpr int NC = SL * kSliceChunks;  // 64-blocks of K a warp owns
     constexpr bool DQ = SC == kScalesU8Words || SC == kScalesU8, TMA_SCALES = SC == kScalesTma;
     extern __shared__ __align__(1024) uint8_t smem[];
-    // kUniformWarp: the warp's number comes through a shuffle; the compiler then knows that it is the same in all lanes, and
-    // keeps what follows from it in uniform registers.  kElects: an elected lane asks for the loop's tiles, else the first one.
+    // kUniform: the warp's number comes through a shuffle, so that the compiler knows it to be the same in all lanes and keeps what
+    // follows from it in uniform registers, and an elected lane asks for the loop's tiles, else the first one.
     // kCarries: the tile loop keeps shared-memory addresses, its tiles' row and the number of T's tile in registers, and starts
     // its sums with a product; without it works them out for every tile (18 of 315 instructions a warp and tile, up to 8 rows).
-    // Which of them helps depends on what a form has in its registers (us, back to back, without -> with):
-    //   up to 8 rows, scales by TMA: all, 4 x 4096 x 11008 8.84 -> 8.60 by the first two, -> 8.22 by the third, 8 x 3584 x
-    //     18944 11.9 -> 11.6; the other forms the third alone (1 x 4096 x 11008 with u8 scales 9.08 -> 8.85, 4 x 4160 x 8192
-    //     12.3 -> 11.6)
-    //   9 to 16 rows, scales by TMA and u8 scales without words: uniform and carried, 16 x 20480 x 20480 98.9 -> 96.7,
-    //     16 x 4160 x 4096 11.3 -> 10.9; elected as well 16 x 3584 x 512 without an adapter 5.0 -> 5.2
-    //   9 to 16 rows, u8 words: none, with the third 9 x 4096 x 4096 without an adapter 6.7 -> 6.9 and more
-    //   9 to 16 rows, f32 scales of a d_in that is no multiple of 256: the first two, with the third 9 x 4160 x 8192 16.4 -> 16.7
-    constexpr bool kUniformWarp = NT == 1 ? SC == kScalesTma : SC != kScalesU8Words;
-    constexpr bool kElects = NT == 1 ? SC == kScalesTma : SC == kScalesF32;
+    // Which of them helps depends on what a form has in its registers.  us, back to back in a graph, weights of 250 MB in turn
+    // (from the L2), neither -> as it is:
+    //   up to 8 rows, scales by TMA: both, 4 x 4096 x 11008 at rank 16 8.85 (8.32) -> 8.66 (7.98), 8 x 3584 x 18944 11.8 (11.4) -> 11.5
+    //     (11.1); the launches of a tile a warp gain without an adapter and lose with one, 8 x 3584 x 512 3.69 -> 3.50, 5.23 -> 5.45
+    //   up to 8 rows, other forms: carried, 1 x 4096 x 11008 with u8 scales 9.66 (9.48) -> 9.11 (9.11), 4 x 4160 x 8192 12.3 -> 11.6
+    //   9 to 16 rows, scales by TMA: both, at rank 16 9 x 11008 x 4096 16.1 -> 15.6, 9 x 20480 x 20480 89.8 -> 85.5, 16 x 4096 x 11008
+    //     11.63 -> 11.52, without an adapter 15.7 -> 15.2 for 16 x 3584 x 18944; a tile a warp 6.9 -> 7.0, at rank 64 7.1 -> 7.4.  (With
+    //     the first lane asking the adapter's calls lost 1 to 4 % of that from HBM, 9 x 3584 x 18944 16.5 -> 17.2)
+    //   9 to 16 rows, u8 scales without words: both, 16 x 4160 x 8192 18.2 -> 17.9
+    //   9 to 16 rows, u8 words: none, carried 9 x 4096 x 4096 without an adapter 6.7 -> 6.9 and more
+    //   9 to 16 rows, f32 scales of a d_in that is no multiple of 256: uniform, carried as well 9 x 4160 x 8192 16.4 -> 16.7
+    constexpr bool kUniform = NT == 1 ? SC == kScalesTma : SC != kScalesU8Words;
     constexpr bool kCarries = NT == 1 || SC == kScalesTma || SC == kScalesU8;
-    const uint32_t tid = threadIdx.x, warp = kUniformWarp ? __shfl_sync(0xffffffffu, tid >> 5, 0) : tid >> 5, lane = tid & 31u;
+    const uint32_t tid = threadIdx.x, warp = kUniform ? __shfl_sync(0xffffffffu, tid >> 5, 0) : tid >> 5, lane = tid & 31u;
     if (ptx::smem_addr(smem) != kWin0) {
         // the table's base is an immediate of the lookups: nothing can run from another address
         if (tid == 0) NF4_REPORT_FAILURE(g_decode_error, g_decode_error_host, 4);
@@ -708,7 +710,7 @@ __device__ __forceinline__ void decode_body(const CUtensorMap *tm_codes, const C
                         if (req_j < my_tiles) {
                             // (it takes the slot that has just been read: its number's)
                             const uint32_t to = kCarries ? slot : req_j & (kRing - 1);
-                            if (kElects ? ptx::elect_one() != 0 : lane == 0)
+                            if (kUniform ? ptx::elect_one() != 0 : lane == 0)
                                 ask(bar0 + 8 * to, to, kCarries ? req_row : (int32_t)(n0 + (rg + req_j * rw) * kTileRows));
                             ++req_j;
                             if (kCarries) req_row += (int32_t)(rw * kTileRows);
