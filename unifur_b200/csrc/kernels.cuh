@@ -51,7 +51,7 @@ int32_t lora_grads(const void *x, const void *gy, const void *a, const void *b, 
                    uint64_t d_out, uint32_t rank, float scale, int32_t layout, int32_t io_dtype, void *ga,
                    void *gb, float *t, float *u, cudaStream_t s);
 
-// adapter_grads.cu: the same for bf16 tensors on warp MMAs.  `scratch` (256-byte aligned) holds R = x a and
+// adapter_grads.cu: the same for bf16 tensors on tcgen05.  `scratch` (256-byte aligned) holds R = x a and
 // grad_y b in the pre-pass's form; u_ready:
 // adapter_grads_u(scratch, ...) already holds grad_y b (the pre-pass of grad_x left it there).
 bool adapter_grads_supported(const void *x, const void *gy, const void *a, const void *b, uint64_t rows, uint64_t d_in,
