@@ -33,11 +33,13 @@
 // the clock that the power limit leaves (1.4 GHz on random operands).  A narrow tile's step is the dequantisers' latency, 0.4 us.
 // With a stage at a time the skeleton alone, no look-ups, no stores, a quarter of the MMAs, took 0.29 us a stage: the one lane that
 // asked for the activations spent 300 to 440 cycles on each, and scales loaded by the threads another 0.05 us.  Before ->
-// now, whole calls: 64 x 4096 x 4096 20.6 -> 16.5 us, 128 x 8192 x 8192 37.7 -> 28.6, 203 x 3584 x 18944 36.8 -> 34.7, 512 x 4096 x 4096
-// 32.0 -> 26.8, 2048 x 4096 x 14336 209.9 -> 208.0; the GEMM of a backward over 2048 x 4096 x 14336 167 -> 151.
+// now, whole calls, weights and inputs in turn: 64 x 4096 x 4096 20.5 -> 18.0 us, 128 x 8192 x 8192 38.3 -> 31.3, 203 x 3584 x 18944 35.7 ->
+// 34.3, 512 x 4096 x 4096 31.6 -> 26.8, 64 x 14336 x 4096 36.0 -> 31.0; 256 x 4096 x 4096 25.0 -> 25.5; 2048 x 4096 x 14336 within what runs
+// differ (205 to 210); the GEMM of a backward over 2048 x 4096 x 14336 167 -> 147.  What got slower: few stages a tile in several rounds of
+// tiles with u8 scales loaded by the threads, 3216 x 512 x 4160 34.1 -> 35.1, 531 x 512 x 19200 36.1 -> 37.2.
 // The start counts for few rows: most CTAs start when the pre-pass's end, so the codes of the first steps are asked for
-// before anything else is set up: 512 x 4096 x 4096 19.4 -> 17.6 us.  The CTAs of a pair meet with a release and an acquire by
-// all threads, at the start and at the end (relaxed arrivals would save 0.5 us at each).
+// before anything else is set up: 512 x 4096 x 4096 19.4 -> 17.6 us of the kernel.  The CTAs of a pair meet with a release and an acquire by
+// all threads, at the start and at the end (relaxed arrivals took 0.5 to 0.9 us a call less).
 //
 // The MMA computes D[n, m] = sum_k W[n, k] x[m, k]: weight rows are the MMA's M (TMEM lanes),
 // activation rows its N (256 accumulator columns).  Both operands are f16 with f32 accumulation:
@@ -235,9 +237,9 @@ struct WorkList {
 };
 
 // Activation rows the MMAs of a tile beginning at row m0 take: all BN, or for the last, ragged tile the rows there are,
-// up to a multiple of 32 (each CTA brings half of them).  An MMA takes as long as it has columns: at 64 rows the
-// k-stage is then bound by the dequantisers (64 x 4096 x 4096, whole call: 41 -> 32 us with the rows that do not exist
-// left out of the split tiles' sums as well; 64 x 14336 x 4096: 54 -> 43).
+// up to a multiple of 32 (each CTA brings half of them).  An MMA takes as long as it has columns: at 64 rows the step is then
+// bound by the dequantisers.  (With single stages, all 256 columns and the rows that do not exist in the split tiles' sums -> without,
+// 64 x 4096 x 4096 41 -> 32 us, 64 x 14336 x 4096 54 -> 43; 18.0 and 31.0 now.)
 template <int BN>
 __host__ __device__ __forceinline__ uint32_t tile_columns(uint32_t M, uint32_t m0) {
     const uint32_t left = M - m0;
@@ -1142,7 +1144,7 @@ __device__ __forceinline__ void repack_adapter_block(const RepackParams &p, uint
 // launch runs beside the pre-pass ahead of it, which it shares nothing with (and which lets it start once the kernels
 // before have completed): one CTA waits for that at the end, so that whoever waits for this kernel finds both complete.
 // (Weight first, pre-pass beside it: the pre-pass's CTAs found no room until the many small ones were through.  Both in one
-// launch, whose CTAs have the pre-pass's registers: 512 x 4096 x 4096 in f32 32.9 to 33.9 us instead of 32.6.)
+// launch, whose CTAs have the pre-pass's registers: 512 x 4096 x 4096 in f32 0.3 to 1.3 us longer.)
 template <class T>
 __global__ void __launch_bounds__(256) repack_kernel(const RepackParams p) {
     __shared__ __align__(16) uint32_t smem[128 * 32];

@@ -389,9 +389,10 @@ prepass_kernel(const Params p) {
 // multiplies it with the bf16 high and low halves of the other factor.
 // Bound by the chain of the loads, the maxima's exchange, the copy and the sums' exchange.  Before, with x read twice (the
 // second time behind the exchange, through shared memory) and a launch ahead that converted both factors, the two took 14 us of
-// the 36.5 of 512 x 4096 x 4096 at rank 16; now 9 of 32.7.  [2048, 4096] at rank 64 43 us and 6 for the factors, now 34;
-// [4096, 14336] at rank 8 133 and 6, now 121.  (The copy with a factor from the row's first values, without the maxima's
-// exchange, and T in tf32 from registers, both factors converted where they are used: 512 x 4096 x 4096 36.9.)
+// the 42.2 of 512 x 4096 x 4096 at rank 16; now 9 of 33.1.  [2048, 4096] at rank 64 43 us and 6 for the factors, now 31;
+// [4096, 14336] at rank 8 133 and 6, now 124.  (The copy with a factor from the row's first values, without the maxima's
+// exchange, and T in tf32 from registers, both factors converted where they are used: 512 x 4096 x 4096 36.9
+// where the present way took 32.6.)
 constexpr uint32_t kUnits = 2, kPieceF32 = 8 * kUnits * 32, kGroupRanks = 16, kMostRanks = 128, kPartRow = 20, kSumRow = kMostRanks + 4;
 
 template <bool k_major>
@@ -586,7 +587,8 @@ prepass_f32_kernel(const Params p) {
 
     // ---- the CTAs' sums, each CTA a share of the rows; columns the adapter does not have are zeros ----
     // A row's sums go to the CTA whose share it is in, so that one meeting does: behind it nobody touches another CTA's memory.  (The
-    // sums read from where they are, with a second meeting before a CTA leaves: 512 x 4096 x 4096 at rank 16 33.6 us instead of 32.8.)
+    // sums read from where they are, with a second meeting before a CTA leaves: 512 x 4096 x 4096 at rank 16 33.6 us instead of 32.8, 200 x
+    // 8192 x 1024 at rank 64 33.7 instead of 32.1.)
     const uint32_t per = kRows / cn, rank_quads = p.rank / 4;  // (the rank is a multiple of four)
     for (uint32_t i = tid; i < kRows * rank_quads; i += kThreads) {
         const uint32_t r = i / rank_quads, c = i % rank_quads * 4;
